@@ -1,4 +1,5 @@
-"""ctypes bindings of the aclnn entry points exported by libopsnn_b200.so, plus torch-tensor conveniences.
+"""Bindings of the aclnn entry points exported by libopsnn_b200.so, plus torch-tensor conveniences: the matmuls and the quantiser, which
+a program calls once per layer, through a CPython module (csrc/python/native.cpp), everything else through ctypes.
 
 Mirrors the reference's operator interface (names, argument order and meaning, status codes):
   aclnnQuantMatmulV5[GetWorkspaceSize]            matmul/quant_batch_matmul_v4/op_host/op_api/aclnn_quant_matmul_v5.h:43-60
@@ -15,6 +16,7 @@ from ctypes import POINTER, byref, c_bool, c_char_p, c_int, c_int32, c_int64, c_
 
 _HERE = os.path.dirname(os.path.abspath(__file__))
 LIB_PATH = os.path.join(_HERE, "lib", "libopsnn_b200.so")
+NATIVE_PATH = os.path.join(_HERE, "lib", "_opsnn_native.so")
 
 ACLNN_SUCCESS = 0
 ACLNN_ERR_PARAM_NULLPTR = 161001
@@ -171,56 +173,41 @@ class AclnnError(RuntimeError):
         super().__init__("%s returned %s (%d): %s" % (api, STATUS_NAMES.get(status, "?"), status, last_error()))
 
 
-class Tensor:
-    """An aclTensor descriptor. `data` is a device address (int) or a torch tensor whose storage backs the view."""
+_native = None
 
-    def __init__(self, shape, dtype, data=0, strides=None, offset=0, fmt=ACL_FORMAT_ND, storage_shape=None):
-        self.shape = tuple(int(s) for s in shape)
-        self.dtype = DTYPE_BY_NAME[dtype] if isinstance(dtype, str) else int(dtype)
-        self._keep = data
-        ptr = data if isinstance(data, int) else (data.data_ptr() if data is not None else 0)
-        n = len(self.shape)
-        dims = (c_int64 * max(n, 1))(*self.shape)
-        st = None if strides is None else (c_int64 * max(n, 1))(*[int(s) for s in strides])
-        sshape = self.shape if storage_shape is None else tuple(storage_shape)
-        sd = (c_int64 * max(len(sshape), 1))(*sshape)
-        self.handle = lib().aclCreateTensor(dims, n, self.dtype, st, int(offset), int(fmt), sd, len(sshape), c_void_p(ptr))
-        if not self.handle:
-            raise ValueError("aclCreateTensor rejected the arguments")
 
-    def __del__(self):
-        try:
-            if getattr(self, "handle", None):
-                lib().aclDestroyTensor(c_void_p(self.handle))
-                self.handle = None
-        except Exception:
-            pass
+def native():
+    """The CPython module with the per-call work (csrc/python/native.cpp). Raises if it has not been built."""
+    global _native
+    if _native is None:
+        import importlib.util
+
+        import torch  # noqa: F401  (the module is linked against torch's libraries)
+
+        lib()
+        if not os.path.exists(NATIVE_PATH):
+            raise RuntimeError("%s is not built; run `python ops-nn_b200/build.py`" % NATIVE_PATH)
+        spec = importlib.util.spec_from_file_location("_opsnn_native", NATIVE_PATH)
+        mod = importlib.util.module_from_spec(spec)
+        spec.loader.exec_module(mod)
+        mod.init(DTYPE_BY_NAME, AclnnError)
+        _native = mod
+    return _native
+
+
+def __getattr__(name):
+    # Tensor(shape, dtype, data=0, strides=None, offset=0, fmt=ACL_FORMAT_ND, storage_shape=None): an aclTensor descriptor
+    # from_torch(t, dtype=None, shape=None, strides=None): descriptor over a torch tensor's memory (None for None). `dtype` / `shape`
+    # override the torch view for types torch lacks (e.g. a uint8 tensor of packed fp4 described as ACL_FLOAT4_E2M1 with twice the
+    # inner extent)
+    if name in ("Tensor", "from_torch"):
+        globals()[name] = getattr(native(), name)
+        return globals()[name]
+    raise AttributeError(name)
 
 
 def _h(t):
     return None if t is None else c_void_p(t.handle)
-
-
-def _torch_dtype_code(t):
-    import torch
-
-    m = {torch.float32: ACL_FLOAT, torch.float16: ACL_FLOAT16, torch.bfloat16: ACL_BF16, torch.int8: ACL_INT8,
-         torch.int32: ACL_INT32, torch.uint8: ACL_UINT8, torch.int64: ACL_INT64}
-    for name, code in (("float8_e4m3fn", ACL_FLOAT8_E4M3FN), ("float8_e5m2", ACL_FLOAT8_E5M2), ("uint64", ACL_UINT64)):
-        if hasattr(torch, name):
-            m[getattr(torch, name)] = code
-    return m[t.dtype]
-
-
-def from_torch(t, dtype=None, shape=None, strides=None):
-    """Descriptor over a torch tensor's memory. `dtype`/`shape` override the torch view for types torch lacks
-    (e.g. a uint8 tensor of packed fp4 described as ACL_FLOAT4_E2M1 with twice the inner extent)."""
-    if t is None:
-        return None
-    code = _torch_dtype_code(t) if dtype is None else (DTYPE_BY_NAME[dtype] if isinstance(dtype, str) else dtype)
-    if shape is None:
-        shape, strides = tuple(t.shape), tuple(t.stride())
-    return Tensor(shape, code, t, strides)
 
 
 def _stream():
@@ -304,39 +291,16 @@ def quant_matmul_v5(x1, x2, x1_scale, x2_scale, out, bias=None, transpose_x1=Fal
                     x2_offset=None, workspace=None, y_scale=None, weight_nz=False):
     """Runs aclnnQuantMatmulV5 (aclnnQuantMatmulWeightNz with weight_nz: x2 described as FRACTAL_NZ) on the current torch CUDA
     stream. Arguments are `Tensor` descriptors over device memory; `out` is written in place. Returns the workspace size used."""
-    st, ws_size, ex = quant_matmul_v5_get_workspace_size(x1, x2, x1_scale, x2_scale, y_scale, None, x2_offset, None, bias,
-                                                         transpose_x1, transpose_x2, group_size, out, weight_nz)
-    if st != ACLNN_SUCCESS:
-        raise AclnnError("aclnnQuantMatmul%sGetWorkspaceSize" % ("WeightNz" if weight_nz else "V5"), st)
-    if workspace is not None and workspace.numel() >= ws_size:
-        keep, wp = workspace, c_void_p(workspace.data_ptr())
-    else:
-        keep, wp = _workspace(ws_size, out._keep)
-    run = lib().aclnnQuantMatmulWeightNz if weight_nz else lib().aclnnQuantMatmulV5
-    st = run(wp, c_uint64(ws_size if keep is None else keep.numel()), ex, _stream())
-    if st != ACLNN_SUCCESS:
-        raise AclnnError("aclnnQuantMatmul%s" % ("WeightNz" if weight_nz else "V5"), st)
-    return ws_size
+    return native().quant_matmul_v5(x1, x2, x1_scale, x2_scale, out, bias, transpose_x1, transpose_x2, group_size, x2_offset, workspace,
+                                    y_scale, weight_nz)
 
 
 def weight_quant_batch_matmul(x, weight, antiquant_scale, y, antiquant_offset=None, bias=None, antiquant_group_size=0,
                               inner_precise=None, workspace=None):
     """Runs aclnnWeightQuantBatchMatmulV2 (V3 when `inner_precise` is 0 / 1, the Nz entry point when it is "nz") on the current
     torch CUDA stream."""
-    st, ws_size, ex = weight_quant_batch_matmul_get_workspace_size(x, weight, antiquant_scale, antiquant_offset, None, None,
-                                                                   bias, antiquant_group_size, y, inner_precise)
-    api = "aclnnWeightQuantBatchMatmulNz" if inner_precise == "nz" else (
-        "aclnnWeightQuantBatchMatmulV2" if inner_precise is None else "aclnnWeightQuantBatchMatmulV3")
-    if st != ACLNN_SUCCESS:
-        raise AclnnError(api + "GetWorkspaceSize", st)
-    if workspace is not None and workspace.numel() >= ws_size:
-        keep, wp = workspace, c_void_p(workspace.data_ptr())
-    else:
-        keep, wp = _workspace(ws_size, y._keep)
-    st = getattr(lib(), api)(wp, c_uint64(ws_size if keep is None else keep.numel()), ex, _stream())
-    if st != ACLNN_SUCCESS:
-        raise AclnnError(api, st)
-    return ws_size
+    return native().weight_quant_batch_matmul(x, weight, antiquant_scale, y, antiquant_offset, bias, antiquant_group_size, inner_precise,
+                                              workspace)
 
 
 def convert_weight_to_int4_pack_get_workspace_size(weight, weight_int4_pack):
@@ -357,15 +321,7 @@ def convert_weight_to_int4_pack(weight, weight_int4_pack):
 
 
 def dynamic_mx_quant(x, y_out, mxscale_out, dst_type, axis=-1, round_mode=b"rint", blocksize=32, scale_alg=0):
-    ws, ex = c_uint64(0), c_void_p(0)
-    code = DTYPE_BY_NAME[dst_type] if isinstance(dst_type, str) else dst_type
-    st = lib().aclnnDynamicMxQuantGetWorkspaceSize(_h(x), int(axis), round_mode, int(code), int(blocksize), int(scale_alg),
-                                                   _h(y_out), _h(mxscale_out), byref(ws), byref(ex))
-    if st != ACLNN_SUCCESS:
-        raise AclnnError("aclnnDynamicMxQuantGetWorkspaceSize", st)
-    st = lib().aclnnDynamicMxQuant(c_void_p(0), c_uint64(0), ex, _stream())
-    if st != ACLNN_SUCCESS:
-        raise AclnnError("aclnnDynamicMxQuant", st)
+    native().dynamic_mx_quant(x, y_out, mxscale_out, dst_type, axis, round_mode, blocksize, scale_alg)
 
 
 # ---- prepare-once weights (include/opsnn_b200_prepare.h) ----------------------------------------------------------

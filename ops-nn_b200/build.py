@@ -17,6 +17,7 @@ CSRC = os.path.join(HERE, "csrc")
 OUT_DIR = os.path.join(HERE, "lib")
 OBJ_DIR = os.path.join(OUT_DIR, "obj")
 LIB = os.path.join(OUT_DIR, "libopsnn_b200.so")
+NATIVE = os.path.join(OUT_DIR, "_opsnn_native.so")
 
 NVCC = os.environ.get("NVCC", "/usr/local/cuda/bin/nvcc")
 COMMON = [
@@ -42,9 +43,9 @@ def sources():
     return out
 
 
-def _headers_digest():
+def _headers_digest(bases=(os.path.join(ROOT, "include"), CSRC)):
     h = hashlib.sha1()
-    for base in (os.path.join(ROOT, "include"), CSRC):
+    for base in bases:
         for dp, _, fs in sorted(os.walk(base)):
             for f in sorted(fs):
                 if f.endswith((".h", ".cuh", ".hpp")):
@@ -84,7 +85,35 @@ def build(force=False, verbose=False):
         res = subprocess.run(cmd, capture_output=True, text=True)
         if res.returncode != 0:
             raise RuntimeError("link failed:\n%s\n%s" % (res.stdout, res.stderr))
+    build_native(force)
     return LIB
+
+
+def build_native(force=False):
+    """The CPython module of the Python package (csrc/python): links the library beside it and the torch that will load it."""
+    import sysconfig
+
+    import torch
+
+    hdr = _headers_digest((os.path.join(ROOT, "include"), os.path.join(CSRC, "host")))
+    src = os.path.join(CSRC, "python", "native.cpp")
+    troot = os.path.dirname(torch.__file__)
+    cmd = [os.environ.get("CXX", "g++"), "-O2", "-std=c++17", "-fPIC", "-shared", "-fvisibility=hidden", "-Wall", "-Wno-missing-field-initializers",
+           "-D_GLIBCXX_USE_CXX11_ABI=%d" % int(torch._C._GLIBCXX_USE_CXX11_ABI), "-I" + os.path.join(ROOT, "include"),
+           "-I" + os.path.join(CSRC, "host"), "-isystem", os.path.join(troot, "include"), "-isystem",
+           os.path.join(troot, "include", "torch", "csrc", "api", "include"), "-isystem", sysconfig.get_paths()["include"], "-isystem",
+           os.path.join(os.path.dirname(os.path.dirname(NVCC)), "include"), src, "-o", NATIVE, "-L" + OUT_DIR, "-l:libopsnn_b200.so",
+           "-Wl,-rpath,$ORIGIN", "-L" + os.path.join(troot, "lib"), "-lc10", "-lc10_cuda", "-ltorch_cpu", "-ltorch_cuda", "-ltorch_python"]
+    with open(src, "rb") as fh:
+        digest = hashlib.sha1(fh.read() + hdr.encode() + torch.__version__.encode() + " ".join(cmd).encode()).hexdigest()
+    stamp = os.path.join(OBJ_DIR, "native.sha1")
+    if not force and os.path.exists(NATIVE) and os.path.exists(stamp) and open(stamp).read() == digest:
+        return
+    res = subprocess.run(cmd, capture_output=True, text=True)
+    if res.returncode != 0:
+        raise RuntimeError("building %s failed:\n%s\n%s" % (NATIVE, res.stdout, res.stderr))
+    with open(stamp, "w") as fh:
+        fh.write(digest)
 
 
 if __name__ == "__main__":

@@ -10,6 +10,7 @@
 #include <atomic>
 
 #include "aclnn_compat/acl_base.h"
+#include "env.h"
 #include "opsnn_b200_kernels.h"
 
 namespace opsnn {

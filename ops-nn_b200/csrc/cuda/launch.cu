@@ -57,7 +57,7 @@ int32_t wqbmm_decode_tma_launch(const OpsnnWqbmmParams* p, cudaStream_t stream, 
 // swizzled stages, else the per-warp cp.async ring. OPSNN_WQ_DECODE_PATH=ring forces the second.
 static int32_t decode_stream_launch(const OpsnnWqbmmParams* p, cudaStream_t stream, bool exact)
 {
-    const char* e = getenv("OPSNN_WQ_DECODE_PATH");
+    const char* e = env("OPSNN_WQ_DECODE_PATH");
     const bool ring_only = e != nullptr && e[0] == 'r';
     if (!ring_only && wqbmm_decode_tma_eligible(p)) return wqbmm_decode_tma_launch(p, stream, exact);
     return wqbmm_decode_ring_launch(p, stream, exact);
@@ -168,7 +168,7 @@ static bool decode_in_chunks(const OpsnnWqbmmParams* p, OpsnnWqbmmParams* chunk)
     // m = 32 and 63 against 89 at m = 48. Two launches pay from 2^24 weights on, three from 3 x 2^24.
     // OPSNN_WQ_CHUNK_MIN_LOG2 replaces both thresholds by 2^value (tuning).
     int64_t min_kn = (p->m <= 32 ? 1 : 3) * ((int64_t)1 << 24);
-    if (const char* e = getenv("OPSNN_WQ_CHUNK_MIN_LOG2")) {
+    if (const char* e = env("OPSNN_WQ_CHUNK_MIN_LOG2")) {
         const int v = atoi(e);
         if (v > 0 && v < 62) min_kn = (int64_t)1 << v;
     }
@@ -178,8 +178,8 @@ static bool decode_in_chunks(const OpsnnWqbmmParams* p, OpsnnWqbmmParams* chunk)
     if (wqbmm_decode_eligible(chunk)) return true;
     // the 8-bit kernels and the (n,k) int4 kernel the same way: three launches of 55-65 us still beat the 0.3 ms of
     // dequantise-then-matmul on such a weight
-    if (wqbmm_decode8_eligible(chunk) && getenv("OPSNN_WQ_NO_DECODE8") == nullptr) return true;
-    return wqbmm_decode_tma_nk_eligible(chunk) && getenv("OPSNN_WQ_NO_DECODE_NK") == nullptr;
+    if (wqbmm_decode8_eligible(chunk) && env("OPSNN_WQ_NO_DECODE8") == nullptr) return true;
+    return wqbmm_decode_tma_nk_eligible(chunk) && env("OPSNN_WQ_NO_DECODE_NK") == nullptr;
 }
 
 // One decode launch per 16 rows; `fast` = the group-wise kernel of inner_precise = 1.
@@ -195,7 +195,7 @@ static int32_t decode_chunk_launches(const OpsnnWqbmmParams* p, cudaStream_t str
         if (q.w_dtype == ACL_INT8 || q.w_dtype == ACL_FLOAT8_E4M3FN) rc = wqbmm_decode8_launch(&q, stream);
         else if (q.trans_w != 0) rc = wqbmm_decode_tma_launch(&q, stream, true);
         else if (which == OPSNN_WQ_KERNEL_DECODE_FAST) rc = decode_stream_launch(&q, stream, false);
-        else if (wqbmm_decode_fast_eligible(&q) && getenv("OPSNN_WQ_DECODE_LEGACY") == nullptr) rc = decode_stream_launch(&q, stream, true);
+        else if (wqbmm_decode_fast_eligible(&q) && env("OPSNN_WQ_DECODE_LEGACY") == nullptr) rc = decode_stream_launch(&q, stream, true);
         else rc = wqbmm_decode_launch(&q, stream);
         if (rc != 0) return rc;
     }
@@ -213,14 +213,14 @@ int32_t opsnn_wqbmm_select_kernel(const OpsnnWqbmmParams* p)
     if (p->inner_precise == 1 && wqbmm_decode_fast_eligible(p)) return OPSNN_WQ_KERNEL_DECODE_FAST;
     if (wqbmm_decode_eligible(p)) return OPSNN_WQ_KERNEL_DECODE;
     // 8-bit weights (int8, e4m3) at small m: their own streaming kernel once the weight is large enough to be worth a k-split grid
-    if (wqbmm_decode8_eligible(p) && p->k * p->n >= ((int64_t)1 << 20) && getenv("OPSNN_WQ_NO_DECODE8") == nullptr) return OPSNN_WQ_KERNEL_DECODE;
+    if (wqbmm_decode8_eligible(p) && p->k * p->n >= ((int64_t)1 << 20) && env("OPSNN_WQ_NO_DECODE8") == nullptr) return OPSNN_WQ_KERNEL_DECODE;
     // 4-bit weights stored (n,k) at small m: the (n,k) form of the bulk-copy decode kernel, same threshold
-    if (wqbmm_decode_tma_nk_eligible(p) && p->k * p->n >= ((int64_t)1 << 20) && getenv("OPSNN_WQ_NO_DECODE_NK") == nullptr) return OPSNN_WQ_KERNEL_DECODE;
+    if (wqbmm_decode_tma_nk_eligible(p) && p->k * p->n >= ((int64_t)1 << 20) && env("OPSNN_WQ_NO_DECODE_NK") == nullptr) return OPSNN_WQ_KERNEL_DECODE;
     // a weight prepared for the prefill path (dequantised once, kept by the caller): beyond the decode range the tensor-core matmul
     // alone beats streaming the packed weight once per 16 rows
     if (p->prep_w != nullptr && p->m > 16 && wqbmm_prefill_eligible(p)) return OPSNN_WQ_KERNEL_PREFILL;
     OpsnnWqbmmParams chunk;
-    if (getenv("OPSNN_WQ_NO_CHUNKS") == nullptr && decode_in_chunks(p, &chunk))
+    if (env("OPSNN_WQ_NO_CHUNKS") == nullptr && decode_in_chunks(p, &chunk))
         return (p->inner_precise == 1 && wqbmm_decode_fast_eligible(&chunk)) ? OPSNN_WQ_KERNEL_DECODE_FAST : OPSNN_WQ_KERNEL_DECODE;
     // m beyond the decode range: dequantise once, multiply on the tensor cores; tiny problems stay on the one-launch coverage kernel
     // (also small m when no streaming decode kernel takes the layout - fp4 weights, unaligned pitches, odd group sizes - and the
@@ -293,11 +293,11 @@ int32_t opsnn_wqbmm_launch(const OpsnnWqbmmParams* p, int32_t kernel_choice, voi
         // decode kernels only; a call that would run elsewhere must not silently skip that.
         PeerBinding pb;
         if (lookup_peer_binding(p->y, &pb)) {
-            const char* e = getenv("OPSNN_WQ_DECODE_PATH");
+            const char* e = env("OPSNN_WQ_DECODE_PATH");
             const bool ring_only = e != nullptr && e[0] == 'r';
             const bool tma4 = (kernel_choice == OPSNN_WQ_KERNEL_DECODE || kernel_choice == OPSNN_WQ_KERNEL_DECODE_FAST) && p->w_dtype != ACL_INT8 &&
                               p->m <= 16 && !ring_only && wqbmm_decode_fast_eligible(p) && wqbmm_decode_tma_eligible(p) &&
-                              getenv("OPSNN_WQ_DECODE_LEGACY") == nullptr;
+                              env("OPSNN_WQ_DECODE_LEGACY") == nullptr;
             const bool tma8 = kernel_choice == OPSNN_WQ_KERNEL_DECODE && wqbmm_decode8_eligible(p);
             const bool tma4nk = kernel_choice == OPSNN_WQ_KERNEL_DECODE && wqbmm_decode_tma_nk_eligible(p);
             if (!tma4 && !tma8 && !tma4nk) {
@@ -325,7 +325,7 @@ int32_t opsnn_wqbmm_launch(const OpsnnWqbmmParams* p, int32_t kernel_choice, voi
         if (!wqbmm_decode_eligible(p)) return (int32_t)cudaErrorInvalidValue;
         // same arithmetic, two data paths: shared-memory ring + ldmatrix where the layout allows it (32-column pieces, 16-byte
         // aligned rows, groups of whole step pairs), register prefetch otherwise
-        if (wqbmm_decode_fast_eligible(p) && getenv("OPSNN_WQ_DECODE_LEGACY") == nullptr)
+        if (wqbmm_decode_fast_eligible(p) && env("OPSNN_WQ_DECODE_LEGACY") == nullptr)
             return decode_stream_launch(p, static_cast<cudaStream_t>(stream), true);
         return wqbmm_decode_launch(p, static_cast<cudaStream_t>(stream));
     }

@@ -288,7 +288,7 @@ int32_t mx_quant_launch(const OpsnnMxQuantParams* p, cudaStream_t stream)
     const int64_t total = p->rows * scale_row;
     if (total == 0) return 0;
     const bool stream_ok = p->k % 32 == 0 && (reinterpret_cast<uintptr_t>(p->x) & 15) == 0 && (reinterpret_cast<uintptr_t>(p->y) & 7) == 0 &&
-                           getenv("OPSNN_MXQ_GENERIC") == nullptr;
+                           env("OPSNN_MXQ_GENERIC") == nullptr;
     if (stream_ok) {
         const int64_t pieces = p->rows * blocks_per_row * 4;
         int64_t g2 = (pieces + 255) / 256;

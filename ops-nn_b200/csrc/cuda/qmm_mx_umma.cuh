@@ -264,7 +264,7 @@ inline void fp4_transpose(const uint8_t* src, uint8_t* dst, int64_t R, int64_t C
 {
     const bool whole = R % 64 == 0 && C % 128 == 0 && src_pitch % 16 == 0 && src_bs % 16 == 0 && dst_pitch % 4 == 0 && dst_bs % 4 == 0 &&
                        (reinterpret_cast<uintptr_t>(src) & 15) == 0 && (reinterpret_cast<uintptr_t>(dst) & 3) == 0 &&
-                       getenv("OPSNN_FP4_TRANSPOSE_SIMPLE") == nullptr;
+                       env("OPSNN_FP4_TRANSPOSE_SIMPLE") == nullptr;
     if (whole)
         fp4_transpose_tiles_kernel<<<dim3((unsigned)(C / 128), (unsigned)(R / 64), (unsigned)nb), 256, 0, stream>>>(src, dst, src_pitch, dst_pitch,
                                                                                                                    src_bs, dst_bs);
@@ -565,7 +565,7 @@ struct MxPlan {
 // Host tile selection: 224-column tiles (less operand traffic per flop) whenever they still give every SM a tile.
 int mx_pick_bn(const OpsnnQmmParams* p)
 {
-    if (const char* e = getenv("OPSNN_QMM_MX_BN")) {
+    if (const char* e = env("OPSNN_QMM_MX_BN")) {
         const int v = atoi(e);
         if (v == 128 || v == 224) return v;
     }
@@ -599,7 +599,7 @@ MxPlan mx_plan(const OpsnnQmmParams* p)
     q.tiles_n = (p->n + q.bn - 1) / q.bn;
     // CTA pairs (256 x 224 tiles, each CTA loading half of B) when there is a tile for about every pair of SMs
     q.pair = q.bn == 224 && p->m >= 256 && p->batch * ((p->m + 255) / 256) * q.tiles_n >= 74;
-    if (const char* e = getenv("OPSNN_QMM_PAIR")) q.pair = atoi(e) != 0 && q.bn == 224;
+    if (const char* e = env("OPSNN_QMM_PAIR")) q.pair = atoi(e) != 0 && q.bn == 224;
     q.kstages = (p->k + k_per_stage - 1) / k_per_stage;
     q.kblocks32 = (p->k + 31) / 32;
     q.kq = (p->k + 63) / 64;
@@ -607,7 +607,7 @@ MxPlan mx_plan(const OpsnnQmmParams* p)
     q.nb_b = p->sb_bs != 0 ? (uint64_t)p->batch : 1;
     q.tr_a = q.f4 && p->trans_a != 0;
     q.tr_b = q.f4 && p->trans_b == 0;
-    if (!q.f4 && p->trans_b == 0 && getenv("OPSNN_MX_NO_TRANSPOSE") == nullptr)
+    if (!q.f4 && p->trans_b == 0 && env("OPSNN_MX_NO_TRANSPOSE") == nullptr)
         q.tr_b = q.bn == 224 && p->m * (p->b_bs == 0 ? p->batch : 1) >= 4096 && (p->b_bs == 0 || p->batch <= 65535) && p->k / 64 < 65535;
     q.tr_a_bytes = q.tr_a ? (uint64_t)(p->a_bs != 0 ? p->batch : 1) * (uint64_t)p->m * (uint64_t)(p->k / 2) : 0;
     q.tr_b_bytes = q.tr_b ? (uint64_t)(p->b_bs != 0 ? p->batch : 1) * (uint64_t)p->n * (uint64_t)(q.f4 ? p->k / 2 : p->k) : 0;
@@ -672,7 +672,7 @@ uint64_t qmm_mx_umma_workspace_size(const OpsnnQmmParams* p0)
 static void mx_relayout_sfb(const OpsnnQmmParams* p, const MxPlan& q, int scale_b_k_major, uint8_t* dst, cudaStream_t stream)
 {
     const int64_t gb = (int64_t)q.nb_b * q.tiles_n * q.row_atoms;
-    if (getenv("OPSNN_MX_SF_SIMPLE") == nullptr && gb < 0x7FFFFFFF) {
+    if (env("OPSNN_MX_SF_SIMPLE") == nullptr && gb < 0x7FFFFFFF) {
         mx_sf_relayout_tiled_kernel<<<(unsigned)gb, 256, 0, stream>>>(reinterpret_cast<const uint8_t*>(p->scale_b), dst, p->n, q.kblocks32, q.kq,
                                                                       scale_b_k_major, q.tiles_n, q.kstages, q.atoms, p->sb_bs, q.bn, q.row_atoms);
     } else {
@@ -751,7 +751,7 @@ int32_t qmm_mx_umma_launch(const OpsnnQmmParams* p0, cudaStream_t stream)
         const int64_t ga = (int64_t)q.nb_a * q.tiles_m, gb = (int64_t)q.nb_b * q.tiles_n * q.row_atoms;
         (void)wb;
         (void)gb;
-        if (getenv("OPSNN_MX_SF_SIMPLE") == nullptr && ga < 0x7FFFFFFF) {
+        if (env("OPSNN_MX_SF_SIMPLE") == nullptr && ga < 0x7FFFFFFF) {
             mx_sf_relayout_tiled_kernel<<<(unsigned)ga, 256, 0, stream>>>(reinterpret_cast<const uint8_t*>(p->scale_a), sfa, p->m, q.kblocks32,
                                                                           q.kq, p->trans_a ? 1 : 0, q.tiles_m, q.kstages, q.atoms, p->sa_bs, BM, 1);
         } else {

@@ -699,7 +699,7 @@ bool is_fp8(int dt) { return dt == ACL_FLOAT8_E4M3FN || dt == ACL_FLOAT8_E5M2; }
 // Host tile selection: the widest N tile that still yields about one tile per SM.
 int pick_bn(const OpsnnQmmParams* p)
 {
-    if (const char* e = getenv("OPSNN_QMM_BN")) {
+    if (const char* e = env("OPSNN_QMM_BN")) {
         int v = atoi(e);
         if (v == 32 || v == 64 || v == 128 || v == 256) return v;
     }
@@ -723,7 +723,7 @@ int pick_ksplit(const OpsnnQmmParams* p, int bn, int kblocks)
 {
     (void)bn;
     if (p->mode != OPSNN_QMM_DEQ) return 1;
-    if (const char* e = getenv("OPSNN_QMM_KSPLIT")) {
+    if (const char* e = env("OPSNN_QMM_KSPLIT")) {
         const int v = atoi(e);
         return (v >= 1 && v <= 8 && v * 2 <= kblocks) ? v : 1;
     }
@@ -776,7 +776,7 @@ int32_t launch_pb(int bn, const CUtensorMap& ma, const CUtensorMap& mb, UmmaArgs
 {
     if (bn == 256) return launch_one<256, true, KIND, 8>(ma, mb, a, stream);
     int ew = KIND == ptx::MmaKind::kI8 ? 8 : 4;
-    if (const char* e = getenv("OPSNN_QMM_PB_EW")) ew = atoi(e);
+    if (const char* e = env("OPSNN_QMM_PB_EW")) ew = atoi(e);
     if (ew == 8) return launch_one<128, true, KIND, 8>(ma, mb, a, stream);
     return launch_one<128, true, KIND, 4>(ma, mb, a, stream);
 }
@@ -804,7 +804,7 @@ int32_t launch_bn(int bn, const CUtensorMap& ma, const CUtensorMap& mb, UmmaArgs
 
 bool qmm_umma_eligible(const OpsnnQmmParams* p)
 {
-    if (getenv("OPSNN_QMM_NO_UMMA")) return false;
+    if (env("OPSNN_QMM_NO_UMMA")) return false;
     if (p->mode == OPSNN_QMM_MX) return qmm_mx_umma_eligible(p);
     const bool i8 = p->a_dtype == ACL_INT8 && p->b_dtype == ACL_INT8;
     const bool f8 = is_fp8(p->a_dtype) && is_fp8(p->b_dtype);
@@ -820,7 +820,7 @@ bool qmm_umma_eligible(const OpsnnQmmParams* p)
     } else if (p->mode == OPSNN_QMM_PERGROUP_ASYM) {
         // INT4 x INT4 asymmetric per-group, operands already widened to INT8: groups of two 128-deep k-blocks on the pair kernel
         if (!i8 || p->group_k != 256 || p->batch != 1 || p->b_offset == nullptr || p->scale_a == nullptr || p->bias != nullptr) return false;
-        if (getenv("OPSNN_QMM_ASYM_GENERIC")) return false;
+        if (env("OPSNN_QMM_ASYM_GENERIC")) return false;
     } else {
         return false;
     }
@@ -928,9 +928,9 @@ int32_t qmm_umma_launch(const OpsnnQmmParams* p, cudaStream_t stream)
             a.ks_nonce = next_ks_nonce();
         }
     }
-    if (const char* e = getenv("OPSNN_TEST_UMMA_STALL_KBLOCK")) {  // tests of the give-up path only (single-CTA kernels)
+    if (const char* e = env("OPSNN_TEST_UMMA_STALL_KBLOCK")) {  // tests of the give-up path only (single-CTA kernels)
         a.test_stall_kblock = atoi(e);
-        const char* pl = getenv("OPSNN_TEST_UMMA_POLL_LIMIT");
+        const char* pl = env("OPSNN_TEST_UMMA_POLL_LIMIT");
         const uint32_t limit = pl != nullptr ? (uint32_t)atoi(pl) : 20000u;
         cudaMemcpyToSymbolAsync(ptx::g_spin_limit, &limit, sizeof(limit), 0, cudaMemcpyHostToDevice, stream);
     }

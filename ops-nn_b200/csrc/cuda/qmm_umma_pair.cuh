@@ -231,7 +231,7 @@ int32_t launch_pair(const CUtensorMap& ma, const CUtensorMap& mb, UmmaArgs& a, c
 // Pairs pay off when there is a 256 x 256 tile for about every pair of SMs; small problems keep the single-CTA kernel.
 bool pair_worthwhile(const OpsnnQmmParams* p)
 {
-    if (const char* e = getenv("OPSNN_QMM_PAIR")) return atoi(e) != 0;
+    if (const char* e = env("OPSNN_QMM_PAIR")) return atoi(e) != 0;
     if (p->mode != OPSNN_QMM_DEQ) return false;
     const int64_t tiles = p->batch * ((p->m + 255) / 256) * ((p->n + 255) / 256);
     return p->m >= 256 && p->n >= 256 && tiles >= 74;

@@ -504,7 +504,7 @@ __global__ void row_sums_kernel(const int8_t* __restrict__ x1, int64_t ld, int t
 bool pair_pb_worthwhile(const OpsnnQmmParams* p)
 {
     if (p->mode != OPSNN_QMM_PERBLOCK) return false;
-    if (const char* e = getenv("OPSNN_QMM_PAIR")) return atoi(e) != 0;
+    if (const char* e = env("OPSNN_QMM_PAIR")) return atoi(e) != 0;
     const int64_t tiles = p->batch * ((p->m + 255) / 256) * ((p->n + 127) / 128);
     return p->m >= 256 && tiles >= 74;
 }
@@ -514,7 +514,7 @@ bool pair_pb_worthwhile(const OpsnnQmmParams* p)
 // OPSNN_QMM_PB_BN=128|256 fixes it.
 int pair_pb_bn(const OpsnnQmmParams* p)
 {
-    if (const char* e = getenv("OPSNN_QMM_PB_BN")) return atoi(e) == 256 ? 256 : 128;
+    if (const char* e = env("OPSNN_QMM_PB_BN")) return atoi(e) == 256 ? 256 : 128;
     const int64_t tiles = p->batch * ((p->m + 255) / 256) * ((p->n + 255) / 256);
     return tiles >= sm_count() / 2 ? 256 : 128;
 }

@@ -557,7 +557,7 @@ int32_t opsnn_comm_arrive_and_wait(void* comm, void* stream)
     cfg.attrs = &attr;
     cfg.numAttrs = 1;
     unsigned int limit = 4u * 1000u * 1000u;
-    if (const char* e = getenv("OPSNN_COMM_POLL_LIMIT")) {  // tests of the give-up path: a shorter wait
+    if (const char* e = env("OPSNN_COMM_POLL_LIMIT")) {  // tests of the give-up path: a shorter wait
         const long v = atol(e);
         if (v > 0 && v < (long)limit) limit = (unsigned int)v;
     }
@@ -610,7 +610,7 @@ int32_t opsnn_comm_allgather_columns(void* comm, const void* y_local, int64_t y_
         return (int32_t)cudaErrorNotSupported;
     }
     unsigned int limit = 4u * 1000u * 1000u;
-    if (const char* e = getenv("OPSNN_COMM_POLL_LIMIT")) {
+    if (const char* e = env("OPSNN_COMM_POLL_LIMIT")) {
         const long v = atol(e);
         if (v > 0 && v < (long)limit) limit = (unsigned int)v;
     }

@@ -283,7 +283,7 @@ int32_t wqbmm_decode_launch(const OpsnnWqbmmParams* p, cudaStream_t stream)
     }
     // host tile selection: as many equal k ranges per strip as keep every CTA resident at once
     int64_t splits = resident / a.strips;
-    if (const char* e = getenv("OPSNN_WQ_DECODE_SPLITS")) {
+    if (const char* e = env("OPSNN_WQ_DECODE_SPLITS")) {
         int v = atoi(e);
         if (v > 0) splits = v;
     }

@@ -693,7 +693,7 @@ cudaError_t d8_configure_variant(int variant)
 
 cudaError_t d8_launch_variant(int variant, int grid, int cluster_policy, const CUtensorMap& mw, const CUtensorMap& mx, const D8Args& ta, cudaStream_t stream)
 {
-    const char* pe = getenv("OPSNN_WQ_PDL");
+    const char* pe = env("OPSNN_WQ_PDL");
     cudaLaunchConfig_t cfg{};
     cfg.gridDim = dim3((unsigned)grid, 1, 1);
     cfg.blockDim = dim3(kThreads, 1, 1);
@@ -782,8 +782,8 @@ int32_t wqbmm_decode8_launch(const OpsnnWqbmmParams* p, cudaStream_t stream)
     cudaError_t crc = d8_configure_variant(variant);
     if (crc != cudaSuccess) return (int32_t)crc;
     int64_t splits = (2 * (int64_t)current_sm_count()) / a.strips;
-    const char* se = getenv("OPSNN_WQ_DECODE_SPLITS");
-    const char* ce = getenv("OPSNN_WQ_DECODE_CLUSTER");
+    const char* se = env("OPSNN_WQ_DECODE_SPLITS");
+    const char* ce = env("OPSNN_WQ_DECODE_CLUSTER");
     if (se != nullptr && atoi(se) > 0) splits = atoi(se);
     if (splits > ta.total_stages) splits = ta.total_stages;
     if (splits * a.strips > k8MaxGrid) splits = k8MaxGrid / a.strips;

@@ -435,7 +435,7 @@ int32_t wqbmm_decode_ring_launch(const OpsnnWqbmmParams* p, cudaStream_t stream,
         default: resident = fast_grid<true, true, true>(7); break;
     }
     int64_t splits = resident / a.strips;
-    if (const char* e = getenv("OPSNN_WQ_DECODE_SPLITS")) {
+    if (const char* e = env("OPSNN_WQ_DECODE_SPLITS")) {
         int v = atoi(e);
         if (v > 0) splits = v;
     }
@@ -453,7 +453,7 @@ int32_t wqbmm_decode_ring_launch(const OpsnnWqbmmParams* p, cudaStream_t stream,
     const uint64_t tag_bytes = (((uint64_t)kFastMaxGrid * 8 + 255) / 256) * 256;
     // Opt-in (OPSNN_WQ_DECODE_CLUSTER=1): measured equal to the workspace combine on the benchmark shape (the tail is set by the
     // slowest CTA's main loop, not by the combination), so the path that needs no cluster scheduling stays the default.
-    const bool want_cluster = splits >= 2 && splits <= 8 && getenv("OPSNN_WQ_DECODE_CLUSTER") != nullptr;
+    const bool want_cluster = splits >= 2 && splits <= 8 && env("OPSNN_WQ_DECODE_CLUSTER") != nullptr;
     if (splits > 1 && !want_cluster && (p->workspace == nullptr || p->workspace_size < wqbmm_decode_workspace_size(p)))
         return (int32_t)cudaErrorInvalidValue;
     a.tags = reinterpret_cast<unsigned long long*>(p->workspace);

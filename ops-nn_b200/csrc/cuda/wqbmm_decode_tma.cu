@@ -750,7 +750,7 @@ cudaError_t configure_variant(int variant)
 cudaError_t launch_variant(int variant, int grid, int cluster_policy, const CUtensorMap& mw, const CUtensorMap& mx, const TmaArgs& ta, cudaStream_t stream)
 {
     // launched as a programmatic dependent of whatever precedes it in the stream (OPSNN_WQ_PDL=0: an ordinary launch)
-    const char* pe = getenv("OPSNN_WQ_PDL");
+    const char* pe = env("OPSNN_WQ_PDL");
     cudaLaunchConfig_t cfg{};
     cfg.gridDim = dim3((unsigned)grid, 1, 1);
     cfg.blockDim = dim3(kThreads, 1, 1);
@@ -769,7 +769,7 @@ cudaError_t launch_variant(int variant, int grid, int cluster_policy, const CUte
         attr[na].val.clusterDim.y = 1;
         attr[na].val.clusterDim.z = 1;
         ++na;
-        if (const char* pol = getenv("OPSNN_WQ_CLUSTER_POLICY")) cluster_policy = atoi(pol);  // experiments: 1 spread, 2 load balancing
+        if (const char* pol = env("OPSNN_WQ_CLUSTER_POLICY")) cluster_policy = atoi(pol);  // experiments: 1 spread, 2 load balancing
         if (cluster_policy == 1 || cluster_policy == 2) {
             attr[na].id = cudaLaunchAttributeClusterSchedulingPolicyPreference;
             attr[na].val.clusterSchedulingPolicyPreference = static_cast<cudaClusterSchedulingPolicy>(cluster_policy);
@@ -846,9 +846,9 @@ int32_t wqbmm_decode_tma_launch(const OpsnnWqbmmParams* p, cudaStream_t stream, 
     const int stage_steps = nk ? kNkStageRows / 16 : kStageSteps;
     ta.total_stages = (int32_t)((a.ksteps + stage_steps - 1) / stage_steps);
     ta.test_stall_stage = -1;
-    if (const char* e = getenv("OPSNN_TEST_DECODE_STALL_STAGE")) {  // tests of the give-up path only
+    if (const char* e = env("OPSNN_TEST_DECODE_STALL_STAGE")) {  // tests of the give-up path only
         ta.test_stall_stage = atoi(e);
-        const char* pl = getenv("OPSNN_TEST_DECODE_POLL_LIMIT");
+        const char* pl = env("OPSNN_TEST_DECODE_POLL_LIMIT");
         const uint32_t limit = pl != nullptr ? (uint32_t)atoi(pl) : 4096u;
         cudaMemcpyToSymbolAsync(g_wq_tma_poll_limit, &limit, sizeof(limit), 0, cudaMemcpyHostToDevice, stream);
     }
@@ -862,8 +862,8 @@ int32_t wqbmm_decode_tma_launch(const OpsnnWqbmmParams* p, cudaStream_t stream, 
     if (crc != cudaSuccess) return (int32_t)crc;
     const int resident = 2 * current_sm_count();
     int64_t splits = resident / a.strips;
-    const char* se = getenv("OPSNN_WQ_DECODE_SPLITS");
-    const char* ce = getenv("OPSNN_WQ_DECODE_CLUSTER");
+    const char* se = env("OPSNN_WQ_DECODE_SPLITS");
+    const char* ce = env("OPSNN_WQ_DECODE_CLUSTER");
     if (se != nullptr && atoi(se) > 0) splits = atoi(se);
     if (splits > ta.total_stages) splits = ta.total_stages;
     if (splits * a.strips > kTmaMaxGrid) splits = kTmaMaxGrid / a.strips;
@@ -887,13 +887,13 @@ int32_t wqbmm_decode_tma_launch(const OpsnnWqbmmParams* p, cudaStream_t stream, 
                 splits = s_pick;
                 a.cluster = 1;
             }
-        } else if (a.strips > kClusterMaxStrips && splits >= 2 && splits <= 16 && getenv("OPSNN_WQ_CLUSTER_POLICY") == nullptr) {
+        } else if (a.strips > kClusterMaxStrips && splits >= 2 && splits <= 16 && env("OPSNN_WQ_CLUSTER_POLICY") == nullptr) {
             // Wide outputs, two CTAs per SM: a cluster per strip pays when the hardware may pack the clusters' CTAs two to an SM
             // (the load-balancing scheduling policy; with the default, spreading one, a second wave forms: 74 us on the
             // benchmark shape) and every strip's cluster is resident at once. 56 strips x 5: 53.5 -> 49.8 us; 64 x 4: 61.7 -> 58.9;
             // cluster sizes that do not pack (6, 7, 9 CTAs: 47.6 -> 67 us) are what the occupancy question filters out.
             const int act = max_active_clusters(tma_kernel(variant), kThreads, kTmaSmem, (int)splits, (int)cudaClusterSchedulingPolicyLoadBalancing);
-            if (getenv("OPSNN_DEBUG_PLAN")) fprintf(stderr, "[opsnn] decode plan: strips %lld splits %lld active clusters (load balancing) %d\n", (long long)a.strips, (long long)splits, act);
+            if (env("OPSNN_DEBUG_PLAN")) fprintf(stderr, "[opsnn] decode plan: strips %lld splits %lld active clusters (load balancing) %d\n", (long long)a.strips, (long long)splits, act);
             if ((int64_t)act >= a.strips) {
                 a.cluster = 1;
                 cluster_policy = (int)cudaClusterSchedulingPolicyLoadBalancing;

@@ -369,7 +369,7 @@ uint64_t wqbmm_prefill_workspace_size(const OpsnnWqbmmParams* p) { return p->pre
 
 bool wqbmm_prefill_eligible(const OpsnnWqbmmParams* p)
 {
-    if (getenv("OPSNN_WQ_NO_PREFILL")) return false;
+    if (env("OPSNN_WQ_NO_PREFILL")) return false;
     if (p->x_dtype != ACL_BF16 && p->x_dtype != ACL_FLOAT16) return false;
     if (p->w_dtype != ACL_INT4 && p->w_dtype != ACL_INT8 && p->w_dtype != ACL_FLOAT8_E4M3FN && p->w_dtype != ACL_FLOAT8_E5M2 &&
         p->w_dtype != ACL_FLOAT4_E2M1)
@@ -397,12 +397,12 @@ int32_t wqbmm_prefill_prepass(const OpsnnWqbmmParams* p, uint8_t* ws, cudaStream
     const bool pairs = p->w_dtype == ACL_INT4 && !p->trans_w && p->w_ld % 8 == 0 && p->n % 8 == 0 &&
                        (reinterpret_cast<uintptr_t>(p->w) & 3) == 0 && (p->group_size == 0 || p->group_size % 8 == 0) &&
                        p->scale_dtype != ACL_FLOAT8_E8M0 &&
-                       getenv("OPSNN_WQ_PREFILL_SIMPLE") == nullptr;
+                       env("OPSNN_WQ_PREFILL_SIMPLE") == nullptr;
     const bool four = p->w_dtype == ACL_INT4 || p->w_dtype == ACL_FLOAT4_E2M1;
     const int per = four ? 8 : 4;
     const bool rows_path = p->trans_w && p->k % per == 0 && p->w_ld % per == 0 && (p->group_size == 0 || p->group_size % per == 0) &&
                            p->scale_dtype != ACL_FLOAT8_E8M0 && (reinterpret_cast<uintptr_t>(p->w) & 3) == 0 &&
-                           getenv("OPSNN_WQ_PREFILL_SIMPLE") == nullptr;
+                           env("OPSNN_WQ_PREFILL_SIMPLE") == nullptr;
     if (rows_path) {
         const int64_t work = p->n * (p->k / per);
         int64_t grid = (work + NT - 1) / NT;
@@ -428,7 +428,7 @@ int32_t wqbmm_prefill_prepass(const OpsnnWqbmmParams* p, uint8_t* ws, cudaStream
     } else if ((p->w_dtype == ACL_INT8 || p->w_dtype == ACL_FLOAT8_E4M3FN || p->w_dtype == ACL_FLOAT8_E5M2) && !p->trans_w &&
                p->n % 4 == 0 && p->w_ld % 4 == 0 && (reinterpret_cast<uintptr_t>(p->w) & 3) == 0 &&
                (p->group_size == 0 || p->group_size % 4 == 0) && p->scale_dtype != ACL_FLOAT8_E8M0 &&
-               getenv("OPSNN_WQ_PREFILL_SIMPLE") == nullptr) {
+               env("OPSNN_WQ_PREFILL_SIMPLE") == nullptr) {
         if (bf) wq_dequant_nk_bytes_kernel<true><<<(unsigned)tiles, NT, 0, stream>>>(*p, wdeq, kp, one);
         else wq_dequant_nk_bytes_kernel<false><<<(unsigned)tiles, NT, 0, stream>>>(*p, wdeq, kp, one);
     } else if (bf && fast) wq_dequant_nk_words_kernel<true><<<(unsigned)tiles, NT, 0, stream>>>(*p, wdeq, kp, one);

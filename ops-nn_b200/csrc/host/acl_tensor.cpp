@@ -12,7 +12,7 @@ static thread_local std::string g_last_err;
 int log_level()
 {
     static int lvl = [] {
-        const char* e = std::getenv("OPSNN_LOG_LEVEL");
+        const char* e = env("OPSNN_LOG_LEVEL");
         return e ? std::atoi(e) : 0;
     }();
     return lvl;

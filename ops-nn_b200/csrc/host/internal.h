@@ -1,14 +1,16 @@
 // Host-side object model shared by the aclnn entry points: tensor descriptor, executor (plan), error text.
 #pragma once
 
+#include <algorithm>
 #include <cstdarg>
 #include <cstdint>
+#include <initializer_list>
 #include <string>
-#include <vector>
 
 #include <nvtx3/nvToolsExt.h>
 
 #include "aclnn_compat/acl_base.h"
+#include "env.h"
 #include "opsnn_b200_kernels.h"
 
 // An NVTX range around each phase of every entry point (the reference brackets its entry points with L2_DFX_PHASE_1 / _2,
@@ -17,19 +19,71 @@ namespace opsnn {
 struct DfxRange {
     explicit DfxRange(const char* name) { nvtxRangePushA(name); }
     ~DfxRange() { nvtxRangePop(); }
+    EnvScope env;  // the call's tuning switches are looked for once
     DfxRange(const DfxRange&) = delete;
     DfxRange& operator=(const DfxRange&) = delete;
 };
 }  // namespace opsnn
 #define OPSNN_DFX_RANGE(name) ::opsnn::DfxRange opsnn_dfx_range_(name)
 
+namespace opsnn {
+// The extents or strides of a view, in place: a call describes half a dozen tensors and copies most of them once or twice while it
+// plans; with a heap vector for each of their three lists that was some sixty allocations a call, on the only path that small calls
+// (5 us from Python to the last launch) have.
+struct Dims {
+    static constexpr size_t kMax = 12;  // aclCreateTensor takes 8; an MX scale adds a dim to its operand's, a planning stand-in up to 3
+    int64_t v[kMax];
+    size_t n = 0;
+
+    Dims() = default;
+    Dims(std::initializer_list<int64_t> l) { assign(l.begin(), l.end()); }
+    Dims(const int64_t* b, const int64_t* e) { assign(b, e); }
+    Dims(const Dims& o) { assign(o.begin(), o.end()); }
+    Dims& operator=(const Dims& o)
+    {
+        if (this != &o) assign(o.begin(), o.end());
+        return *this;
+    }
+    void assign(const int64_t* b, const int64_t* e)
+    {
+        n = std::min<size_t>((size_t)(e - b), kMax);
+        for (size_t i = 0; i < n; ++i) v[i] = b[i];
+    }
+    void assign(size_t count, int64_t value)
+    {
+        n = std::min(count, kMax);
+        for (size_t i = 0; i < n; ++i) v[i] = value;
+    }
+    void resize(size_t count)
+    {
+        count = std::min(count, kMax);
+        for (size_t i = n; i < count; ++i) v[i] = 0;
+        n = count;
+    }
+    void push_back(int64_t value)
+    {
+        if (n < kMax) v[n++] = value;
+    }
+    void clear() { n = 0; }
+    size_t size() const { return n; }
+    int64_t* begin() { return v; }
+    int64_t* end() { return v + n; }
+    const int64_t* begin() const { return v; }
+    const int64_t* end() const { return v + n; }
+    int64_t& operator[](size_t i) { return v[i]; }
+    const int64_t& operator[](size_t i) const { return v[i]; }
+    int64_t& back() { return v[n - 1]; }
+    bool operator==(const Dims& o) const { return n == o.n && std::equal(begin(), end(), o.begin()); }
+    bool operator!=(const Dims& o) const { return !(*this == o); }
+};
+}  // namespace opsnn
 
 // Tensor descriptor. Mirrors what the reference's aclTensor carries (docs/zh/context/non_contiguous_tensor.md of
 // the reference): view shape, strides and offset in elements, storage shape, format, dtype, device address.
 struct aclTensor {
-    std::vector<int64_t> shape;
-    std::vector<int64_t> strides;
-    std::vector<int64_t> storage_shape;
+    opsnn::Dims shape;
+    opsnn::Dims strides;
+    opsnn::Dims storage_shape;
     int64_t offset = 0;
     aclDataType dtype = ACL_FLOAT;
     aclFormat format = ACL_FORMAT_ND;

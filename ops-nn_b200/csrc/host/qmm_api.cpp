@@ -328,7 +328,7 @@ bool check_shape(const Ctx& c)
         }
     }
     // output batch inference (:854-877)
-    std::vector<int64_t> batch;
+    Dims batch;
     int64_t batch_prod = 1;
     {
         size_t r1 = c.x1.rank(), r2 = c.x2.rank(), ro = std::max(r1, r2), off = ro - std::min(r1, r2);
@@ -424,7 +424,7 @@ aclnnStatus check_a8w4_float(const Ctx& c, const aclTensor* x1Scale, int64_t gro
 }
 
 // Batch stride (elements) of an operand whose leading dims either equal the output batch dims or are absent/1.
-bool operand_batch(const aclTensor& t, size_t core_rank, const std::vector<int64_t>& out_batch, int64_t core_elems,
+bool operand_batch(const aclTensor& t, size_t core_rank, const Dims& out_batch, int64_t core_elems,
                    int64_t* bs)
 {
     size_t nb = t.rank() - core_rank;
@@ -483,7 +483,7 @@ void make_hint(const aclTensor* x2, const aclTensor* x2Scale, bool transposeX2, 
 {
     const size_t r = x2->rank();
     const int64_t k = transposeX2 ? x2->dim(-1) : x2->dim(-2), n = transposeX2 ? x2->dim(-2) : x2->dim(-1);
-    std::vector<int64_t> batch(x2->shape.begin(), x2->shape.begin() + (r >= 2 ? r - 2 : 0));
+    Dims batch(x2->shape.begin(), x2->shape.begin() + (r >= 2 ? r - 2 : 0));
     auto contiguous = [](aclTensor* t) {
         t->strides.assign(t->shape.size(), 1);
         for (int i = (int)t->shape.size() - 2; i >= 0; --i) t->strides[i] = t->strides[i + 1] * t->shape[i + 1];
@@ -704,7 +704,7 @@ aclnnStatus aclnnQuantMatmulV5GetWorkspaceSize(const aclTensor* x1, const aclTen
             p.scale_b_len = c.n;
         }
         exec->kernel_choice = OPSNN_KERNEL_AUTO;
-        if (const char* e = std::getenv("OPSNN_QMM_KERNEL")) exec->kernel_choice = std::atoi(e);
+        if (const char* e = env("OPSNN_QMM_KERNEL")) exec->kernel_choice = std::atoi(e);
         if (!exec->unsupported) {
             if (exec->kernel_choice == OPSNN_KERNEL_AUTO) exec->kernel_choice = opsnn_qmm_select_kernel(&p);
             exec->workspace_size = opsnn_qmm_workspace_size(&p, exec->kernel_choice);
@@ -773,7 +773,7 @@ aclnnStatus aclnnQuantMatmulV5GetWorkspaceSize(const aclTensor* x1, const aclTen
     p.m = c.m;
     p.n = c.n;
     p.k = c.k1;
-    std::vector<int64_t> ob(c.out.shape.begin(), c.out.shape.end() - 2);
+    Dims ob(c.out.shape.begin(), c.out.shape.end() - 2);
     if (c.out.rank() == 3 && c.x1.rank() == 2 && c.x2.rank() == 2 && c.out.shape[1] == 1 && c.m != 1) ob.clear();
     p.batch = 1;
     for (auto d : ob) p.batch *= d;
@@ -859,7 +859,7 @@ aclnnStatus aclnnQuantMatmulV5GetWorkspaceSize(const aclTensor* x1, const aclTen
         if (c.fp8_in() && !c.has_x1s && float_bias) p.deq_flags |= OPSNN_DEQ_FBIAS_BEFORE_SCALE;
     }
     exec->kernel_choice = OPSNN_KERNEL_AUTO;
-    if (const char* e = std::getenv("OPSNN_QMM_KERNEL")) exec->kernel_choice = std::atoi(e);
+    if (const char* e = env("OPSNN_QMM_KERNEL")) exec->kernel_choice = std::atoi(e);
     if (!exec->unsupported) {
         if (exec->kernel_choice == OPSNN_KERNEL_AUTO) exec->kernel_choice = opsnn_qmm_select_kernel(&p);
         if (exec->kernel_choice == OPSNN_KERNEL_UMMA) attach_prepared(&p);  // an x2 registered by opsnnQuantMatmulPrepareX2

@@ -228,7 +228,7 @@ aclnnStatus wq_common(const char* api, const aclTensor* x, const aclTensor* weig
     if (nz_k0 != 0 && trans_w) no_kernel("a FRACTAL_NZ weight must be the plain (k,n) view");
     attach_prepared_w(&p);
     exec->kernel_choice = OPSNN_WQ_KERNEL_AUTO;
-    if (const char* e = std::getenv("OPSNN_WQ_KERNEL")) exec->kernel_choice = std::atoi(e);
+    if (const char* e = env("OPSNN_WQ_KERNEL")) exec->kernel_choice = std::atoi(e);
     if (!exec->unsupported) {
         // eligibility depends on pointer alignment, which needs real addresses; phase 1 may run without them
         // (unit tests pass NULL), so size the workspace for the decode kernel whenever the shapes allow it.
@@ -421,7 +421,7 @@ aclnnStatus aclnnDynamicMxQuantGetWorkspaceSize(const aclTensor* x, int64_t axis
     if ((dstType == ACL_FLOAT4_E2M1 || dstType == ACL_FLOAT4_E1M2) && (x->dim(-1) % 2 != 0)) WQ_INVALID("%s: fp4 output needs an even last dimension", api);
     {
         // mxscaleOut: x's shape with the axis replaced by ceil(ceil(k/32)/2), plus a trailing 2
-        std::vector<int64_t> want = x->shape;
+        Dims want = x->shape;
         want[ax] = ceil_div(ceil_div(kdim, 32), 2);
         want.push_back(2);
         if (mxscaleOut->shape != want) WQ_INVALID("%s: mxscaleOut has the wrong shape", api);
