@@ -72,6 +72,10 @@ int32_t wqbmm_prefill_launch(const OpsnnWqbmmParams* p, cudaStream_t stream);
 uint64_t wqbmm_prefill_image_size(const OpsnnWqbmmParams* p);
 int32_t wqbmm_prefill_prepass(const OpsnnWqbmmParams* p, uint8_t* ws, cudaStream_t stream);
 
+bool wqbmm_mixed_eligible(const OpsnnWqbmmParams* p);
+uint64_t wqbmm_mixed_workspace_size(const OpsnnWqbmmParams* p);
+int32_t wqbmm_mixed_launch(const OpsnnWqbmmParams* p, cudaStream_t stream);
+
 uint64_t wq_nz_bytes(const OpsnnWqbmmParams* p);
 void wq_nz_view(const OpsnnWqbmmParams* p, OpsnnWqbmmParams* q, void* dst);
 int32_t wq_nz_launch(const OpsnnWqbmmParams* p, void* dst, cudaStream_t stream);
@@ -202,6 +206,17 @@ static int32_t decode_chunk_launches(const OpsnnWqbmmParams* p, cudaStream_t str
     return 0;
 }
 
+// A call with m > 16 that was planned as decode launches or as dequantise-then-matmul runs on the fused kernel instead (wqbmm_mixed.cu:
+// the packed weight dequantised into tensor memory, once for up to 128 rows of x) where that is the faster form.
+static bool mixed_instead(const OpsnnWqbmmParams* p, int32_t kernel_choice)
+{
+    if (p->m <= 16 || (kernel_choice != OPSNN_WQ_KERNEL_DECODE && kernel_choice != OPSNN_WQ_KERNEL_PREFILL)) return false;
+    if (kernel_choice == OPSNN_WQ_KERNEL_PREFILL && (p->prep_w != nullptr || p->k * p->n <= ((int64_t)1 << 22))) return false;
+    int64_t max_m = 1024;
+    if (const char* e = env("OPSNN_WQ_MIXED_MAX_M")) max_m = atoi(e);
+    return p->m <= max_m && wqbmm_mixed_eligible(p);
+}
+
 int32_t opsnn_wqbmm_select_kernel(const OpsnnWqbmmParams* p)
 {
     if (p == nullptr) return OPSNN_WQ_KERNEL_GENERIC;
@@ -239,6 +254,7 @@ uint64_t opsnn_wqbmm_workspace_size(const OpsnnWqbmmParams* p, int32_t kernel_ch
         wq_nz_view(p, &nd, reinterpret_cast<void*>(uintptr_t(256)));
         return pre + opsnn_wqbmm_workspace_size(&nd, kernel_choice);
     }
+    if (mixed_instead(p, kernel_choice)) return wqbmm_mixed_workspace_size(p);
     if (kernel_choice == OPSNN_WQ_KERNEL_PREFILL) return wqbmm_prefill_workspace_size(p);
     return (kernel_choice == OPSNN_WQ_KERNEL_DECODE || kernel_choice == OPSNN_WQ_KERNEL_DECODE_FAST) ? wqbmm_decode_workspace_size(p) : 0;
 }
@@ -307,6 +323,7 @@ int32_t opsnn_wqbmm_launch(const OpsnnWqbmmParams* p, int32_t kernel_choice, voi
             }
         }
     }
+    if (mixed_instead(p, kernel_choice)) return wqbmm_mixed_launch(p, static_cast<cudaStream_t>(stream));
     OpsnnWqbmmParams chunk;
     if (p->m > 16 && (kernel_choice == OPSNN_WQ_KERNEL_DECODE || kernel_choice == OPSNN_WQ_KERNEL_DECODE_FAST)) {
         if (!decode_in_chunks(p, &chunk)) return (int32_t)cudaErrorInvalidValue;

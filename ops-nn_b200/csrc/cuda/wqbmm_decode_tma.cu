@@ -936,6 +936,11 @@ extern "C" __attribute__((visibility("default"))) int32_t opsnn_wqbmm_decode_tim
 }
 #endif
 
+namespace opsnn {
+uint32_t wqbmm_decode8_status(int reset);
+uint32_t wqbmm_mixed_status(int reset);
+}  // namespace opsnn
+
 // Error word of the bulk-copy decode kernels on the current device: 0 when every bounded wait inside them completed. Synchronises the
 // device; reset != 0 clears the word after reading it.
 extern "C" __attribute__((visibility("default"))) uint32_t opsnn_wqbmm_decode_status(int32_t reset)
@@ -948,5 +953,6 @@ extern "C" __attribute__((visibility("default"))) uint32_t opsnn_wqbmm_decode_st
         const uint32_t limit = opsnn::kWaitPolls;  // a test may have shortened the waits: back to the normal limit
         cudaMemcpyToSymbol(opsnn::g_wq_tma_poll_limit, &limit, sizeof(limit));
     }
-    return v;
+    const uint32_t v8 = opsnn::wqbmm_decode8_status(reset), vm = opsnn::wqbmm_mixed_status(reset);
+    return v != 0 ? v : (v8 != 0 ? v8 : vm);
 }

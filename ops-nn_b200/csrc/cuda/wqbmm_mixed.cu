@@ -1,0 +1,817 @@
+// Weight-only quant matmul for 16 < m: the packed weight is dequantised straight into tensor memory and multiplied there
+// (tcgen05 kind::f16 with A in TMEM), one pass over the weight for up to 128 rows of x. No 16-bit image of the weight in HBM.
+//
+// Reference: weight_quant_batch_matmul_v2/op_kernel/arch35/weight_quant_batch_matmul_v2_reg_base_common.h:164-286 (vector cores
+// dequantise tile by tile, the cube unit multiplies in bf16 / fp16); arithmetic of the golden wqbmmv2_kernel_golden.py:199-297:
+//   w' = rn_x(rn_x(w + offset) * scale),  y = rn_x(sum_k x * w' (fp32) + bias)
+//
+// Orientation: D^T = W'^T x^T. The MMA's 128 rows are weight columns, its N is the rows of x (16 ... 128 of them, a multiple of 16), so
+// the tensor core's work shrinks with m while the dequantisation - what bounds this kernel - is done once whatever m is.
+//   CTA tile: 256 weight columns (two M = 128 accumulators) x N rows of x; persistent, one CTA per SM (all 512 TMEM columns).
+//   Work is cut stream-k: the (tile, k stage) pairs in one line, every CTA an equal contiguous piece. A tile that several CTAs share is
+//   combined through workspace in CTA order by whichever of them arrives last (deterministic; nobody waits for anybody).
+//   warps 0-15   dequantise. Warp w serves TMEM lanes 32 (w % 4) .. (a hardware rule), accumulator half (w / 4) % 2, and every other
+//                64-row unit of k (w / 8). packed words -> registers (ldmatrix.trans for (k,n) storage: a register then holds nibbles /
+//                bytes of k rows 2q, 2q + 1, already the pair that a TMEM cell of A wants; a row per lane for (n,k) storage) ->
+//                the decode kernels' pair arithmetic -> tcgen05.st.
+//   warps 16-19  epilogue, overlapped with the next tile's main loop.
+//   warp 20      TMA producer (packed weight, x, scale / offset rows), warp 21 MMA issuer.
+// A operand buffers: four units of 64 k x 256 columns (64 TMEM columns each) at columns 256-511; accumulators at 0-255 (two sets while
+// N <= 64).
+// Every wait is bounded; a wait that gives up raises the CTA's abort flag, records a code and the CTA tears down (TMEM freed).
+#include <cstdio>
+
+#include "common.cuh"
+#include "sm100_ptx.cuh"
+#include "wqbmm_decode_common.cuh"
+
+namespace opsnn {
+
+namespace {
+
+constexpr int kMixTileN = 256;
+constexpr int kMixDqWarps = 16, kMixEpWarps = 4;
+constexpr int kMixThreads = (kMixDqWarps + kMixEpWarps + 2) * 32;
+constexpr int kMixMaxRows = 128;   // rows of x per pass over the weight
+constexpr int kMixABufs = 4;
+constexpr uint32_t kMixACol = 256;  // first TMEM column of the A buffers
+constexpr int kMixMaxStages = 16;
+constexpr int kMixSmemMax = 225 * 1024;
+
+struct MixArgs {
+    int32_t m, n_tiles, t_tiles, rows;  // rows: rows of x per tile (N of the MMA)
+    int64_t n, k;
+    int32_t kb;          // k stages per tile
+    int32_t stages, stage_bytes, x_off, sc_off;
+    int32_t grid;
+    int64_t units;       // n_tiles * t_tiles * kb
+    const void* scale;
+    const void* offset;
+    int64_t scale_sg, scale_sn;
+    int32_t group;       // rows of k per group; 0: one group
+    const void* bias;
+    int32_t bias_dtype;
+    void* y;
+    int64_t y_ld;
+    float* part;                   // [2 grid][2][rows / 4][128] float4
+    unsigned long long* count;     // [tiles] (nonce << 8) | arrivals
+    unsigned long long nonce;
+    uint32_t idesc;
+};
+
+__device__ unsigned int g_mix_status = 0;
+
+__device__ __forceinline__ void mix_report(volatile uint32_t* abort_flag, unsigned int code)
+{
+    *abort_flag = 1u;
+    atomicCAS(&g_mix_status, 0u, code);
+}
+
+__device__ __forceinline__ void mix_tma_2d(uint32_t smem_dst, const CUtensorMap* map, uint32_t bar_addr, int32_t c0, int32_t c1)
+{
+    asm volatile("cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4}], [%2];" ::"r"(smem_dst),
+                 "l"(reinterpret_cast<uint64_t>(map)), "r"(bar_addr), "r"(c0), "r"(c1)
+                 : "memory");
+}
+__device__ __forceinline__ void mix_arrive(uint32_t bar_addr)
+{
+    asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(bar_addr) : "memory");
+}
+// Bounded wait with one answer for the warp: what follows it is .sync.aligned.
+__device__ __forceinline__ bool mix_wait(uint32_t bar_addr, uint32_t parity, volatile uint32_t* abort_flag)
+{
+    return __all_sync(0xffffffffu, ptx::mbar_wait_a(bar_addr, parity, abort_flag));
+}
+__device__ __forceinline__ void mix_init(uint32_t bar_addr, uint32_t count)
+{
+    asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(bar_addr), "r"(count) : "memory");
+}
+__device__ __forceinline__ void mix_ldsm4_trans(uint32_t addr, uint32_t (&r)[4])
+{
+    asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0,%1,%2,%3}, [%4];"
+                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3])
+                 : "r"(addr)
+                 : "memory");
+}
+__device__ __forceinline__ uint4 mix_lds128(uint32_t addr)
+{
+    uint4 v;
+    asm volatile("ld.shared.v4.u32 {%0,%1,%2,%3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "r"(addr) : "memory");
+    return v;
+}
+// 16 TMEM lanes x 16 columns: register pairs (2c, 2c + 1) hold, in lane (g, q), rows g and g + 8 of columns 4c + q
+__device__ __forceinline__ void tmem_st_16x128b_x4(uint32_t taddr, const uint32_t (&r)[8])
+{
+    asm volatile("tcgen05.st.sync.aligned.16x128b.x4.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" ::"r"(taddr), "r"(r[0]), "r"(r[1]), "r"(r[2]),
+                 "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7])
+                 : "memory");
+}
+// 32 TMEM lanes x 8 columns, a lane's columns in its registers
+__device__ __forceinline__ void tmem_st_32x32b_x8(uint32_t taddr, const uint32_t (&r)[8])
+{
+    asm volatile("tcgen05.st.sync.aligned.32x32b.x8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" ::"r"(taddr), "r"(r[0]), "r"(r[1]), "r"(r[2]),
+                 "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7])
+                 : "memory");
+}
+__device__ __forceinline__ void tmem_st_wait() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
+// kind::f16, A (128 x 16) in tensor memory, B in shared memory
+__device__ __forceinline__ void umma_f16_ta(uint32_t d_tmem, uint32_t a_tmem, uint64_t bdesc, uint32_t idesc, uint32_t accumulate)
+{
+    asm volatile(
+        "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\ttcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n\t}" ::"r"(d_tmem),
+        "r"(a_tmem), "l"(bdesc), "r"(idesc), "r"(accumulate)
+        : "memory");
+}
+
+enum class MixW { kInt4, kInt8, kE4m3 };
+
+template <MixW kW, bool kNK>
+struct MixCfg {
+    static constexpr int kBits = kW == MixW::kInt4 ? 4 : 8;
+    static constexpr int kBK = kNK ? 128 : 64;  // k rows per stage: rows of 128 (or, int4 (n,k), 64) bytes for the copies
+    static constexpr int kUnits = kBK / 64;
+    static constexpr int kWBytes = kMixTileN * kBK * kBits / 8;
+    static constexpr int kEmptyArrivals = (kNK ? kMixDqWarps : kMixDqWarps / 2) + 1;
+};
+
+// A pair of weights, codes in the low bits of the two halves (other bits arbitrary), to the 16-bit type, exactly (int4: the caller has
+// shifted the nibble down). e4m3's two NaN codes read as +-480 here; fix_nan below puts that right.
+template <MixW kW, bool kBf16>
+__device__ __forceinline__ uint32_t mix_exact(uint32_t p)
+{
+    using N = Num<kBf16>;
+    uint32_t v;
+    if (kW == MixW::kInt4) {
+        asm("lop3.b32 %0, %1, %2, %3, 0x6A;" : "=r"(v) : "r"(p), "n"(0x000F000F), "n"(N::kMagic));  // (nibble ^ 8) | magic
+        return N::sub(v, N::kBias);
+    }
+    if (kW == MixW::kInt8) {
+        if (kBf16) {  // (128 + low seven bits) - (128 or 256)
+            uint32_t s;
+            asm("lop3.b32 %0, %1, %2, %3, 0xEA;" : "=r"(v) : "r"(p), "n"(0x007F007F), "n"(0x43004300));
+            asm("lop3.b32 %0, %1, %2, %3, 0xEA;" : "=r"(s) : "r"(p), "n"(0x00800080), "n"(0x43004300));
+            return N::sub(v, s);
+        }
+        asm("lop3.b32 %0, %1, %2, %3, 0x6A;" : "=r"(v) : "r"(p), "n"(0x00FF00FF), "n"(0x64806480));  // 1024 + (byte ^ 0x80)
+        return N::sub(v, 0x64806480u);
+    }
+    constexpr uint32_t kMag = kBf16 ? 0x07F007F0u : 0x3F803F80u, kRebias = kBf16 ? 0x7B807B80u : 0x5C005C00u;
+    v = (p << (kBf16 ? 4 : 7)) & kMag;  // the magnitude under the wider type's sign bit reads as w * 2^-120 (bf16) / 2^-8 (fp16)
+    asm("lop3.b32 %0, %1, %2, %3, 0xEA;" : "=r"(v) : "r"(p << 8), "n"(0x80008000), "r"(v));
+    return N::mul(v, kRebias);
+}
+
+template <bool kBf16, bool kOff>
+__device__ __forceinline__ uint32_t mix_scale(uint32_t v, uint32_t sc, uint32_t of)
+{
+    using N = Num<kBf16>;
+    if (kOff) v = N::add(v, of);
+    return N::mul(v, sc);
+}
+
+// Any of the four bytes an e4m3 NaN (low seven bits all set)?
+__device__ __forceinline__ uint32_t has_nan8(uint32_t r) { return ((r & 0x7F7F7F7Fu) + 0x01010101u) & 0x80808080u; }
+// Replaces the halves of `v` whose code byte (bytes 0 and 2 of p) is a NaN code.
+__device__ __forceinline__ uint32_t fix_nan(uint32_t v, uint32_t p)
+{
+    if ((p & 0x7Fu) == 0x7Fu) v |= 0x00007FFFu;
+    if ((p & 0x7F0000u) == 0x7F0000u) v |= 0x7FFF0000u;
+    return v;
+}
+
+// TMEM lane (within a warp's 32) -> weight column (within the warp's 32)
+template <MixW kW, bool kNK>
+__device__ __forceinline__ int mix_col_of_lane(int l)
+{
+    if (kNK) return l;
+    return kW == MixW::kInt4 ? 4 * (l & 7) + (l >> 3) : 16 * (l >> 4) + 2 * (l & 7) + ((l >> 3) & 1);
+}
+
+// A CTA's contiguous piece of the (tile, stage) line.
+__device__ __forceinline__ int64_t mix_begin(const MixArgs& a, int64_t c) { return c * a.units / a.grid; }
+
+template <MixW kW, bool kNK, bool kBf16, bool kOff>
+__global__ void __launch_bounds__(kMixThreads, 1)
+wqbmm_mixed_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUtensorMap map_x, const MixArgs a)
+{
+    using C = MixCfg<kW, kNK>;
+    const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0);
+    const int lane = threadIdx.x & 31;
+    extern __shared__ uint8_t dyn_raw[];
+    const uint32_t smem0 = (ptx::smem_u32(dyn_raw) + 1023u) & ~1023u;
+    __shared__ __align__(8) uint64_t s_bars[2 * kMixMaxStages + 2 * kMixABufs + 4];
+    __shared__ uint32_t s_tmem;
+    __shared__ volatile uint32_t s_abort;
+    __shared__ uint32_t s_last;
+    const uint32_t full0 = ptx::smem_u32(s_bars), empty0 = full0 + 8u * kMixMaxStages;
+    const uint32_t afull0 = empty0 + 8u * kMixMaxStages, aempty0 = afull0 + 8u * kMixABufs;
+    const uint32_t dfull0 = aempty0 + 8u * kMixABufs, dempty0 = dfull0 + 16u;
+    volatile uint32_t* abort_flag = &s_abort;
+
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    if (threadIdx.x == 0) {
+        s_abort = 0u;
+        for (int i = 0; i < a.stages; ++i) {
+            mix_init(full0 + 8u * i, 1u);
+            mix_init(empty0 + 8u * i, (uint32_t)C::kEmptyArrivals);
+        }
+        for (int i = 0; i < kMixABufs; ++i) {
+            mix_init(afull0 + 8u * i, kMixDqWarps / 2);
+            mix_init(aempty0 + 8u * i, 1u);
+        }
+        for (int i = 0; i < 2; ++i) {
+            mix_init(dfull0 + 8u * i, 1u);
+            mix_init(dempty0 + 8u * i, kMixEpWarps);
+        }
+        ptx::fence_mbar_init();
+        ptx::fence_proxy_async();
+    }
+    if (warp == kMixDqWarps + kMixEpWarps + 1) ptx::tmem_alloc(&s_tmem, 512);
+    ptx::tc_fence_before();
+    __syncthreads();
+    ptx::tc_fence_after();
+    const uint32_t tmem = s_tmem;
+    asm volatile("griddepcontrol.wait;" ::: "memory");  // nothing another kernel may have written is read before this
+
+    const int64_t u_begin = mix_begin(a, blockIdx.x), u_end = mix_begin(a, (int64_t)blockIdx.x + 1);
+    const uint32_t stages = (uint32_t)a.stages, stage_bytes = (uint32_t)a.stage_bytes;
+    const uint32_t xunit = (uint32_t)a.rows * 128u;  // bytes of x per 64-row unit of k
+    const bool two_d = a.rows <= 64;                 // two accumulator sets
+
+    if (warp == kMixDqWarps + kMixEpWarps) {
+        // ======================= TMA producer =======================
+        if (lane == 0) {
+            ptx::tma_prefetch_desc(&map_w);
+            ptx::tma_prefetch_desc(&map_x);
+        }
+        __syncwarp();
+        uint32_t s = 0, par = 0;
+        int64_t t = u_begin / a.kb;
+        int32_t kb = (int32_t)(u_begin - t * a.kb);
+        for (int64_t u = u_begin; u < u_end; ++u) {
+            if (!mix_wait(empty0 + 8u * s, par ^ 1u, abort_flag)) {
+                mix_report(abort_flag, (1u << 8) | 1u);
+                break;
+            }
+            if (ptx::elect_one()) {
+                const int32_t tn = (int32_t)(t / a.t_tiles), tt = (int32_t)(t - (int64_t)tn * a.t_tiles);
+                const int32_t n0 = tn * kMixTileN, k0 = kb * C::kBK;
+                const uint32_t fb = full0 + 8u * s, dst = smem0 + s * stage_bytes;
+                uint32_t sc_bytes = 0;
+                if (!kNK) sc_bytes = (uint32_t)min((int64_t)(kMixTileN * 2), (a.n - n0) * 2);
+                ptx::mbar_expect_tx_a(fb, (uint32_t)C::kWBytes + xunit * C::kUnits + sc_bytes * (kOff ? 2u : 1u));
+                if (kNK) {
+                    mix_tma_2d(dst, &map_w, fb, k0 * C::kBits / 8, n0);
+                } else {
+                    mix_tma_2d(dst, &map_w, fb, n0 * C::kBits / 8, k0);
+                    if (C::kBits == 8) mix_tma_2d(dst + C::kWBytes / 2, &map_w, fb, n0 + 128, k0);
+                }
+#pragma unroll
+                for (int i = 0; i < C::kUnits; ++i) mix_tma_2d(dst + a.x_off + i * xunit, &map_x, fb, (k0 + 64 * i) * 2, tt * a.rows);
+                if (!kNK) {
+                    const int64_t g = a.group > 0 ? min((int64_t)k0, a.k - 1) / a.group : 0;
+                    const int64_t at = g * a.scale_sg + n0;
+                    ptx::bulk_load_a(dst + a.sc_off, reinterpret_cast<const uint16_t*>(a.scale) + at, sc_bytes, fb);
+                    if (kOff) ptx::bulk_load_a(dst + a.sc_off + kMixTileN * 2, reinterpret_cast<const uint16_t*>(a.offset) + at, sc_bytes, fb);
+                }
+            }
+            __syncwarp();
+            if (++s == stages) { s = 0; par ^= 1u; }
+            if (++kb == a.kb) { kb = 0; ++t; }
+        }
+    } else if (warp == kMixDqWarps + kMixEpWarps + 1) {
+        // ======================= MMA issuer =======================
+        const uint64_t db = ptx::make_smem_desc(smem0 + a.x_off, 0, 1024, 2);
+        const uint32_t b_lo = (uint32_t)db;
+        const uint64_t b_hi = db & 0xFFFFFFFF00000000ull;
+        uint32_t s = 0, par = 0, ab = 0, apar = 0, seg = 0;
+        bool ok = true;
+        int64_t u = u_begin;
+        int32_t kb = (int32_t)(u_begin % a.kb);
+        while (u < u_end && ok) {
+            const int32_t cnt = (int32_t)min((int64_t)(a.kb - kb), u_end - u);
+            const uint32_t dbuf = two_d ? (seg & 1u) : 0u, dpar = two_d ? ((seg >> 1) & 1u) : (seg & 1u);
+            if (!mix_wait(dempty0 + 8u * dbuf, dpar ^ 1u, abort_flag)) {
+                mix_report(abort_flag, (2u << 8) | 1u);
+                break;
+            }
+            const uint32_t d0 = tmem + dbuf * 2u * (uint32_t)a.rows;
+            uint32_t acc = 0u;
+            for (int32_t i = 0; i < cnt && ok; ++i) {
+                if (!mix_wait(full0 + 8u * s, par, abort_flag)) {
+                    mix_report(abort_flag, (2u << 8) | 2u);
+                    ok = false;
+                    break;
+                }
+#pragma unroll
+                for (int un = 0; un < C::kUnits; ++un) {
+                    if (!mix_wait(afull0 + 8u * ab, apar, abort_flag)) {
+                        mix_report(abort_flag, (2u << 8) | 3u);
+                        ok = false;
+                        break;
+                    }
+                    ptx::tc_fence_after();
+                    if (ptx::elect_one()) {
+                        const uint32_t bl = b_lo + ((s * stage_bytes + un * xunit) >> 4);
+                        const uint32_t a0 = tmem + kMixACol + ab * 64u;
+#pragma unroll
+                        for (int kk = 0; kk < 4; ++kk) {
+#pragma unroll
+                            for (int h = 0; h < 2; ++h)
+                                umma_f16_ta(d0 + h * (uint32_t)a.rows, a0 + h * 32 + kk * 8, b_hi | (uint64_t)(bl + 2u * kk), a.idesc,
+                                            kk == 0 ? acc : 1u);
+                        }
+                        ptx::umma_commit_a(aempty0 + 8u * ab);
+                        if (un == C::kUnits - 1) ptx::umma_commit_a(empty0 + 8u * s);
+                    }
+                    __syncwarp();
+                    acc = 1u;
+                    if (++ab == kMixABufs) { ab = 0; apar ^= 1u; }
+                }
+                if (++s == stages) { s = 0; par ^= 1u; }
+            }
+            if (!ok) break;
+            if (ptx::elect_one()) ptx::umma_commit_a(dfull0 + 8u * dbuf);
+            __syncwarp();
+            ++seg;
+            u += cnt;
+            kb = 0;
+        }
+    } else if (warp < kMixDqWarps) {
+        // ======================= dequantisation =======================
+        const int qd = warp & 3, h = (warp >> 2) & 1;
+        const uint32_t grp = (uint32_t)warp >> 3;
+        const int g = lane >> 2;
+        const uint32_t tlane = (uint32_t)(qd * 32) << 16;
+        const int wcol = h * 128 + qd * 32;  // the warp's first column in the tile
+        uint32_t s = 0, par = 0;
+        if (!kNK) {  // units alternate between the two groups of eight warps
+            s = grp;
+            if (s >= stages) { s -= stages; par ^= 1u; }
+        }
+        uint32_t ab = grp, apar = 0;
+        // (n,k) storage: the lane's own scale and offset, a stage's worth ahead
+        const int64_t u0 = u_begin + (kNK ? 0 : grp);
+        int64_t t = u0 / a.kb;
+        int32_t kb = (int32_t)(u0 - t * a.kb);
+        uint32_t sc_next = 0, of_next = 0;
+        auto fetch = [&](int64_t tile, int32_t stage) {
+            const int64_t n = min((tile / a.t_tiles) * kMixTileN + wcol + lane, a.n - 1);
+            const int64_t kk = min((int64_t)stage * C::kBK + 64 * grp, a.k - 1);
+            const int64_t at = (a.group > 0 ? kk / a.group : 0) * a.scale_sg + n * a.scale_sn;
+            sc_next = __ldg(reinterpret_cast<const uint16_t*>(a.scale) + at);
+            if (kOff) of_next = __ldg(reinterpret_cast<const uint16_t*>(a.offset) + at);
+        };
+        if (kNK && u0 < u_end) fetch(t, kb);
+        for (int64_t u = u0; u < u_end; u += kNK ? 1 : 2) {
+            uint32_t sc[4], of[4];
+            if (kNK) {
+                sc[0] = sc_next | (sc_next << 16);
+                of[0] = of_next | (of_next << 16);
+                if (++kb == a.kb) { kb = 0; ++t; }
+                if (u + 1 < u_end) fetch(t, kb);
+            }
+            if (!mix_wait(full0 + 8u * s, par, abort_flag)) {
+                mix_report(abort_flag, (3u << 8) | 1u);
+                break;
+            }
+            const uint32_t base = smem0 + s * stage_bytes;
+            if (!kNK) {  // int4: columns 4g .. 4g + 3; int8: 2g, 2g + 1 of each 16
+                const uint32_t at = base + a.sc_off + 2u * wcol;
+                uint32_t r0, r1, o0 = 0, o1 = 0;
+                const uint32_t p0 = kW == MixW::kInt4 ? at + 8u * g : at + 4u * g, p1 = kW == MixW::kInt4 ? p0 + 4u : p0 + 32u;
+                asm volatile("ld.shared.u32 %0, [%1];" : "=r"(r0) : "r"(p0) : "memory");
+                asm volatile("ld.shared.u32 %0, [%1];" : "=r"(r1) : "r"(p1) : "memory");
+                if (kOff) {
+                    asm volatile("ld.shared.u32 %0, [%1];" : "=r"(o0) : "r"(p0 + kMixTileN * 2) : "memory");
+                    asm volatile("ld.shared.u32 %0, [%1];" : "=r"(o1) : "r"(p1 + kMixTileN * 2) : "memory");
+                }
+                sc[0] = prmt(r0, r0, 0x1010); sc[1] = prmt(r0, r0, 0x3232); sc[2] = prmt(r1, r1, 0x1010); sc[3] = prmt(r1, r1, 0x3232);
+                of[0] = prmt(o0, o0, 0x1010); of[1] = prmt(o0, o0, 0x3232); of[2] = prmt(o1, o1, 0x1010); of[3] = prmt(o1, o1, 0x3232);
+            }
+            bool waited = false, dead = false;
+            const uint32_t abase = tmem + kMixACol + ab * 64u + h * 32u + tlane;
+            auto need_buffer = [&]() {  // the MMAs that read this A buffer's previous contents are done
+                if (waited) return;
+                waited = true;
+                if (!mix_wait(aempty0 + 8u * ab, apar ^ 1u, abort_flag)) {
+                    mix_report(abort_flag, (3u << 8) | 2u);
+                    dead = true;
+                }
+                ptx::tc_fence_after();
+            };
+            if constexpr (!kNK) {
+                const int r = lane & 7, j = lane >> 3;
+                if constexpr (kW == MixW::kInt4) {
+                    // 64 rows of 128 bytes; matrix j of an ldmatrix = rows 8 j .. of a half of 32, the warp's 16 bytes of the row
+                    const uint32_t at = base + (uint32_t)(8 * j + r) * 128u + (uint32_t)(((h * 4 + qd) ^ r) << 4);
+                    uint32_t w[2][4];
+                    mix_ldsm4_trans(at, w[0]);
+                    mix_ldsm4_trans(at + 32 * 128, w[1]);
+                    __syncwarp();
+#pragma unroll
+                    for (int half = 0; half < 2; ++half) {
+                        uint32_t o[2][8];
+#pragma unroll
+                        for (int i = 0; i < 4; ++i)
+#pragma unroll
+                            for (int b = 0; b < 4; ++b)
+                                o[b >> 1][2 * i + (b & 1)] = mix_scale<kBf16, kOff>(mix_exact<kW, kBf16>(w[half][i] >> (4 * b)), sc[b], of[b]);
+                        need_buffer();
+                        tmem_st_16x128b_x4(abase + half * 16, o[0]);
+                        tmem_st_16x128b_x4(abase + half * 16 + (16u << 16), o[1]);
+                    }
+                } else {
+                    const uint32_t box = base + h * (C::kWBytes / 2) + (uint32_t)(8 * j + r) * 128u;
+#pragma unroll
+                    for (int half = 0; half < 2; ++half) {
+#pragma unroll
+                        for (int cc = 0; cc < 2; ++cc) {
+                            uint32_t w[4], o[8];
+                            mix_ldsm4_trans(box + half * 32 * 128 + (uint32_t)(((2 * qd + cc) ^ r) << 4), w);
+#pragma unroll
+                            for (int i = 0; i < 4; ++i)
+#pragma unroll
+                                for (int b = 0; b < 2; ++b)
+                                    o[2 * i + b] = mix_scale<kBf16, kOff>(mix_exact<kW, kBf16>(w[i] >> (8 * b)), sc[2 * cc + b], of[2 * cc + b]);
+                            if (kW == MixW::kE4m3) {
+                                const uint32_t any = has_nan8(w[0]) | has_nan8(w[1]) | has_nan8(w[2]) | has_nan8(w[3]);
+                                if (any != 0u) {
+#pragma unroll
+                                    for (int i = 0; i < 4; ++i) {
+                                        o[2 * i] = fix_nan(o[2 * i], w[i]);
+                                        o[2 * i + 1] = fix_nan(o[2 * i + 1], w[i] >> 8);
+                                    }
+                                }
+                                __syncwarp();
+                            }
+                            need_buffer();
+                            tmem_st_16x128b_x4(abase + half * 16 + ((uint32_t)(16 * cc) << 16), o);
+                        }
+                    }
+                }
+            } else {
+                const int row = wcol + lane;
+                if constexpr (kW == MixW::kInt4) {
+                    const uint32_t rb = base + (uint32_t)row * 64u;
+                    const uint32_t x = (uint32_t)(row >> 1) & 3u;  // 64-byte swizzle
+#pragma unroll
+                    for (int c = 0; c < 2; ++c) {
+                        const uint4 v = mix_lds128(rb + (((2u * grp + c) ^ x) << 4));
+                        const uint32_t w[4] = {v.x, v.y, v.z, v.w};
+#pragma unroll
+                        for (int hh = 0; hh < 2; ++hh) {
+                            uint32_t o[8];
+#pragma unroll
+                            for (int i = 0; i < 2; ++i) {
+                                const uint32_t lo = w[2 * hh + i], hi = lo >> 4;
+#pragma unroll
+                                for (int b = 0; b < 4; ++b)  // nibbles 2 b and 2 b + 1: byte b of the word and of the word shifted by four
+                                    o[4 * i + b] = mix_scale<kBf16, kOff>(mix_exact<kW, kBf16>(prmt(lo, hi, (uint32_t)(b | ((4 + b) << 8)))), sc[0], of[0]);
+                            }
+                            need_buffer();
+                            tmem_st_32x32b_x8(abase + c * 16 + hh * 8, o);
+                        }
+                    }
+                } else {
+                    const uint32_t rb = base + (uint32_t)row * 128u;
+                    const uint32_t x = (uint32_t)row & 7u;  // 128-byte swizzle
+#pragma unroll
+                    for (int c = 0; c < 4; ++c) {
+                        const uint4 v = mix_lds128(rb + (((4u * grp + c) ^ x) << 4));
+                        const uint32_t w[4] = {v.x, v.y, v.z, v.w};
+                        uint32_t o[8];
+#pragma unroll
+                        for (int i = 0; i < 4; ++i) {
+                            o[2 * i] = mix_scale<kBf16, kOff>(mix_exact<kW, kBf16>(prmt(w[i], 0u, 0x4140)), sc[0], of[0]);
+                            o[2 * i + 1] = mix_scale<kBf16, kOff>(mix_exact<kW, kBf16>(prmt(w[i], 0u, 0x4342)), sc[0], of[0]);
+                        }
+                        if (kW == MixW::kE4m3) {
+                            const uint32_t any = has_nan8(w[0]) | has_nan8(w[1]) | has_nan8(w[2]) | has_nan8(w[3]);
+                            if (any != 0u) {
+#pragma unroll
+                                for (int i = 0; i < 4; ++i) {
+                                    o[2 * i] = fix_nan(o[2 * i], prmt(w[i], 0u, 0x4140));
+                                    o[2 * i + 1] = fix_nan(o[2 * i + 1], prmt(w[i], 0u, 0x4342));
+                                }
+                            }
+                            __syncwarp();
+                        }
+                        need_buffer();
+                        tmem_st_32x32b_x8(abase + c * 8, o);
+                    }
+                }
+            }
+            if (dead) break;
+            if (lane == 0) mix_arrive(empty0 + 8u * s);  // the packed words (and scale rows) of this stage are in registers
+            tmem_st_wait();
+            ptx::tc_fence_before();
+            __syncwarp();
+            if (lane == 0) mix_arrive(afull0 + 8u * ab);
+            ab += 2u;
+            if (ab >= kMixABufs) { ab -= kMixABufs; apar ^= 1u; }
+            s += kNK ? 1u : 2u;
+            if (s >= stages) { s -= stages; par ^= 1u; }
+        }
+    } else {
+        // ======================= epilogue =======================
+        const int qd = warp & 3, et = (warp - kMixDqWarps) * 32 + lane;  // 0..127
+        const uint32_t tlane = (uint32_t)(qd * 32) << 16;
+        const int mycol = qd * 32 + mix_col_of_lane<kW, kNK>(lane);
+        const uint32_t rows = (uint32_t)a.rows;
+        uint32_t seg = 0;
+        int64_t u = u_begin;
+        auto store = [&](int64_t n, int tt, uint32_t c, const float (&f)[16]) {  // 16 rows of y, one column
+            if (n >= a.n) return;
+            const float b = a.bias != nullptr ? load_as_float(a.bias, n, a.bias_dtype) : 0.f;
+            const int r0 = tt * (int)rows + (int)c;
+            uint16_t* y = reinterpret_cast<uint16_t*>(a.y) + (int64_t)r0 * a.y_ld + n;
+#pragma unroll
+            for (int i = 0; i < 16; ++i) {
+                if (r0 + i >= a.m) break;
+                const float v = a.bias != nullptr ? __fadd_rn(f[i], b) : f[i];
+                y[(int64_t)i * a.y_ld] = kBf16 ? __bfloat16_as_ushort(__float2bfloat16_rn(v)) : __half_as_ushort(__float2half_rn(v));
+            }
+        };
+        while (u < u_end) {
+            const int64_t t = u / a.kb;
+            const int32_t kb = (int32_t)(u - t * a.kb);
+            const int64_t cnt = min((int64_t)(a.kb - kb), u_end - u);
+            const uint32_t dbuf = two_d ? (seg & 1u) : 0u, dpar = two_d ? ((seg >> 1) & 1u) : (seg & 1u);
+            const int64_t n0 = (t / a.t_tiles) * kMixTileN + mycol;
+            const int tt = (int)(t % a.t_tiles);
+            const bool whole = cnt == a.kb;
+            const bool got = __all_sync(0xffffffffu, ptx::mbar_wait_relaxed(&s_bars[2 * kMixMaxStages + 2 * kMixABufs + dbuf], dpar, abort_flag));
+            if (!got) mix_report(abort_flag, (4u << 8) | 1u);
+            asm volatile("bar.sync 1, 128;" ::: "memory");  // the four warps go on, or leave, together
+            if (*abort_flag != 0u) break;
+            ptx::tc_fence_after();
+            const int64_t first_t = u_begin / a.kb;
+            float4* mine = reinterpret_cast<float4*>(a.part) + (2 * (int64_t)blockIdx.x + (t == first_t ? 0 : 1)) * (2 * (rows / 4) * 128);
+#pragma unroll 1
+            for (uint32_t hc = 0; hc < 2 * rows; hc += 16) {
+                uint32_t v[16];
+                ptx::tmem_ld16(tmem + tlane + dbuf * 2u * rows + hc, v);
+                ptx::tmem_ld_wait();
+                float f[16];
+#pragma unroll
+                for (int i = 0; i < 16; ++i) f[i] = __uint_as_float(v[i]);
+                if (whole) {
+                    const uint32_t hh = hc >= rows ? 1u : 0u;
+                    store(n0 + 128 * hh, tt, hc - hh * rows, f);
+                } else {
+#pragma unroll
+                    for (int i = 0; i < 4; ++i) __stcg(mine + (hc / 4 + i) * 128 + et, make_float4(f[4 * i], f[4 * i + 1], f[4 * i + 2], f[4 * i + 3]));
+                }
+            }
+            ptx::tc_fence_before();
+            __syncwarp();
+            if (lane == 0) mix_arrive(dempty0 + 8u * dbuf);
+            if (!whole) {
+                // the CTAs whose pieces meet this tile
+                auto owner = [&](int64_t unit) {
+                    int64_t c = unit * a.grid / a.units;
+                    while (mix_begin(a, c + 1) <= unit) ++c;
+                    while (mix_begin(a, c) > unit) --c;
+                    return c;
+                };
+                const int64_t c0 = owner(t * a.kb), c1 = owner((t + 1) * a.kb - 1);
+                __threadfence();
+                asm volatile("bar.sync 1, 128;" ::: "memory");  // all of this CTA's partial sums are written and fenced
+                if (et == 0) {
+                    unsigned long long* cnt_p = a.count + t;
+                    unsigned long long cur = *reinterpret_cast<volatile unsigned long long*>(cnt_p), want = 0ull;
+                    bool done = false;
+                    for (int it = 0; it < 4096 && !done; ++it) {  // at most c1 - c0 other CTAs can get in between
+                        want = ((cur >> 8) == a.nonce) ? cur + 1ull : ((a.nonce << 8) | 1ull);
+                        const unsigned long long prev = atomicCAS(cnt_p, cur, want);
+                        done = prev == cur;
+                        cur = prev;
+                    }
+                    if (!done) mix_report(abort_flag, (4u << 8) | 2u);
+                    const bool last = done && (int64_t)(want & 0xFFull) == c1 - c0 + 1;
+                    if (last) *reinterpret_cast<volatile unsigned long long*>(cnt_p) = 0ull;  // a replay of this launch starts clean
+                    s_last = last ? 1u : 0u;
+                }
+                asm volatile("bar.sync 1, 128;" ::: "memory");
+                if (s_last != 0u) {
+                    __threadfence();
+                    const float4* part = reinterpret_cast<const float4*>(a.part);
+                    const int64_t slot = 2 * (rows / 4) * 128;
+#pragma unroll 1
+                    for (uint32_t hc = 0; hc < 2 * rows; hc += 16) {
+                        float f[16];
+#pragma unroll
+                        for (int i = 0; i < 16; ++i) f[i] = 0.f;
+#pragma unroll 2
+                        for (int64_t c = c0; c <= c1; ++c) {
+                            const int64_t sl = 2 * c + (mix_begin(a, c) / a.kb == t ? 0 : 1);
+                            const float4* p = part + sl * slot + (hc / 4) * 128 + et;
+                            float4 q[4];
+#pragma unroll
+                            for (int i = 0; i < 4; ++i) q[i] = __ldcg(p + i * 128);
+#pragma unroll
+                            for (int i = 0; i < 4; ++i) {
+                                f[4 * i] += q[i].x; f[4 * i + 1] += q[i].y; f[4 * i + 2] += q[i].z; f[4 * i + 3] += q[i].w;
+                            }
+                        }
+                        const uint32_t hh = hc >= rows ? 1u : 0u;
+                        store(n0 + 128 * hh, tt, hc - hh * rows, f);
+                    }
+                }
+            }
+            ++seg;
+            u += cnt;
+        }
+    }
+    // ---- teardown: everyone meets here, also after an aborted wait; then the allocating warp frees TMEM ----
+    if (*abort_flag != 0u) __nanosleep(200000);  // lets bulk copies that are still in flight land before the CTA leaves
+    ptx::tc_fence_before();
+    __syncthreads();
+    if (warp == kMixDqWarps + kMixEpWarps + 1) {
+        ptx::tc_fence_after();
+        ptx::tmem_dealloc(tmem, 512);
+    }
+}
+
+using MixEncodeFn = CUresult (*)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*, const cuuint64_t*, const cuuint32_t*,
+                                 const cuuint32_t*, CUtensorMapInterleave, CUtensorMapSwizzle, CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
+MixEncodeFn mix_encoder()
+{
+    static MixEncodeFn fn = [] {
+        void* p = nullptr;
+        cudaDriverEntryPointQueryResult q;
+        if (cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &p, cudaEnableDefault, &q) != cudaSuccess) p = nullptr;
+        return reinterpret_cast<MixEncodeFn>(p);
+    }();
+    return fn;
+}
+bool mix_map(CUtensorMap* map, const void* base, uint64_t inner_bytes, uint64_t rows, uint64_t pitch, uint32_t box_inner, uint32_t box_rows)
+{
+    MixEncodeFn enc = mix_encoder();
+    if (enc == nullptr) return false;
+    cuuint64_t dims[2] = {inner_bytes, rows};
+    cuuint64_t strides[1] = {pitch};
+    cuuint32_t box[2] = {box_inner, box_rows};
+    cuuint32_t estr[2] = {1, 1};
+    return enc(map, CU_TENSOR_MAP_DATA_TYPE_UINT8, 2, const_cast<void*>(base), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
+               box_inner == 64 ? CU_TENSOR_MAP_SWIZZLE_64B : CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+               CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+}
+
+struct MixPlan {
+    int t_tiles, rows, n_tiles, kb, grid;
+    int64_t units, tiles;
+};
+
+MixPlan mix_plan(const OpsnnWqbmmParams* p, int sms)
+{
+    MixPlan q;
+    q.t_tiles = (int)((p->m + kMixMaxRows - 1) / kMixMaxRows);
+    const int64_t per = (p->m + q.t_tiles - 1) / q.t_tiles;
+    q.rows = (int)((per + 15) / 16 * 16);
+    q.t_tiles = (int)((p->m + q.rows - 1) / q.rows);
+    q.n_tiles = (int)((p->n + kMixTileN - 1) / kMixTileN);
+    const int bk = p->trans_w ? 128 : 64;
+    q.kb = (int)((p->k + bk - 1) / bk);
+    q.tiles = (int64_t)q.n_tiles * q.t_tiles;
+    q.units = q.tiles * q.kb;
+    const int64_t least = 512 / bk;  // k rows a CTA should at least see: a shorter piece is mostly ramp and combination
+    int64_t grid = q.units / least;
+    if (grid > sms) grid = sms;
+    if (grid < 1) grid = 1;
+    if (const char* e = env("OPSNN_WQ_MIXED_GRID")) {
+        const int v = atoi(e);
+        if (v > 0 && v <= sms && v <= q.units) grid = v;
+    }
+    q.grid = (int)grid;
+    return q;
+}
+
+template <MixW kW, bool kNK, bool kBf16, bool kOff>
+int32_t mix_launch(const CUtensorMap& mw, const CUtensorMap& mx, const MixArgs& a, size_t smem, cudaStream_t stream)
+{
+    auto kern = wqbmm_mixed_kernel<kW, kNK, kBf16, kOff>;
+    static std::atomic<uint64_t> configured{0};
+    if (once_per_device(configured, [&] { return cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, kMixSmemMax); }) != cudaSuccess)
+        return (int32_t)cudaGetLastError();
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3((unsigned)a.grid, 1, 1);
+    cfg.blockDim = dim3(kMixThreads, 1, 1);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = stream;
+    cudaLaunchAttribute attr[1]{};
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    return (int32_t)cudaLaunchKernelEx(&cfg, kern, mw, mx, a);
+}
+
+template <MixW kW, bool kNK>
+int32_t mix_dispatch(bool bf16, bool off, const CUtensorMap& mw, const CUtensorMap& mx, const MixArgs& a, size_t smem, cudaStream_t stream)
+{
+    if constexpr (kW != MixW::kE4m3) {
+        if (off) return bf16 ? mix_launch<kW, kNK, true, true>(mw, mx, a, smem, stream) : mix_launch<kW, kNK, false, true>(mw, mx, a, smem, stream);
+    }
+    return bf16 ? mix_launch<kW, kNK, true, false>(mw, mx, a, smem, stream) : mix_launch<kW, kNK, false, false>(mw, mx, a, smem, stream);
+}
+
+}  // namespace
+
+// Layouts the kernel takes: int4 / int8 / e4m3 weights in either storage order with 16-byte aligned rows, one group or groups of whole
+// 64-row units, scales in x's dtype - for (k,n) storage contiguous along n (their rows are bulk-copied), any strides for (n,k).
+bool wqbmm_mixed_eligible(const OpsnnWqbmmParams* p)
+{
+    if (env("OPSNN_WQ_NO_MIXED")) return false;
+    if (p->nz_k0 != 0 || p->scale_dtype == ACL_FLOAT8_E8M0) return false;
+    if (p->w_dtype != ACL_INT4 && p->w_dtype != ACL_INT8 && p->w_dtype != ACL_FLOAT8_E4M3FN) return false;
+    if (p->w_dtype == ACL_FLOAT8_E4M3FN && p->offset != nullptr) return false;
+    if (p->x_dtype != ACL_BF16 && p->x_dtype != ACL_FLOAT16) return false;
+    if (p->m < 1 || p->n < 1 || p->k < 64 || p->m >= (1 << 24) || p->n >= ((int64_t)1 << 30) || p->k >= ((int64_t)1 << 29)) return false;
+    const int bits = p->w_dtype == ACL_INT4 ? 4 : 8;
+    auto al16 = [](const void* q) { return (reinterpret_cast<uintptr_t>(q) & 15) == 0; };
+    if (!al16(p->w) || !al16(p->x) || p->x_ld % 8 != 0 || (p->w_ld * bits / 8) % 16 != 0 || (p->w_ld * bits) % 8 != 0) return false;
+    if (p->group_size != 0 && p->group_size % 64 != 0) return false;
+    if (p->trans_w) {
+        if (bits == 4 && p->k % 2 != 0) return false;
+        if (p->scale_sn < 0 || p->scale_sg < 0) return false;
+    } else {
+        if (p->n % 8 != 0 || p->scale_sn != 1 || !al16(p->scale) || (p->offset != nullptr && !al16(p->offset))) return false;
+        if (p->group_size != 0 && p->scale_sg % 8 != 0) return false;
+    }
+    return true;
+}
+
+uint64_t wqbmm_mixed_workspace_size(const OpsnnWqbmmParams* p)
+{
+    const MixPlan q = mix_plan(p, current_sm_count());
+    const uint64_t counters = ((uint64_t)q.tiles * 8u + 255u) & ~(uint64_t)255u;
+    return 256u + counters + 2u * (uint64_t)q.grid * (uint64_t)q.rows * kMixTileN * 4u;
+}
+
+int32_t wqbmm_mixed_launch(const OpsnnWqbmmParams* p, cudaStream_t stream)
+{
+    const MixPlan q = mix_plan(p, current_sm_count());
+    if (p->workspace == nullptr || p->workspace_size < wqbmm_mixed_workspace_size(p)) return (int32_t)cudaErrorInvalidValue;
+    const bool nk = p->trans_w != 0, bf16 = p->x_dtype == ACL_BF16, off = p->offset != nullptr;
+    const int bits = p->w_dtype == ACL_INT4 ? 4 : 8;
+    MixArgs a{};
+    a.m = (int32_t)p->m;
+    a.n = p->n;
+    a.k = p->k;
+    a.n_tiles = q.n_tiles;
+    a.t_tiles = q.t_tiles;
+    a.rows = q.rows;
+    a.kb = q.kb;
+    a.units = q.units;
+    a.grid = q.grid;
+    const int bk = nk ? 128 : 64;
+    const int wbytes = kMixTileN * bk * bits / 8;
+    a.x_off = wbytes;
+    a.sc_off = wbytes + q.rows * 128 * (bk / 64);
+    a.stage_bytes = a.sc_off + (nk ? 0 : 1024);
+    a.stages = (kMixSmemMax - 2048) / a.stage_bytes;
+    if (a.stages > kMixMaxStages) a.stages = kMixMaxStages;
+    size_t smem = (size_t)a.stages * a.stage_bytes + 1024;
+    if (smem < 116 * 1024) smem = 116 * 1024;  // one CTA per SM: the kernel owns all of the SM's tensor memory
+    a.scale = p->scale;
+    a.offset = p->offset;
+    a.scale_sg = p->group_size > 0 ? p->scale_sg : 0;
+    a.scale_sn = p->scale_sn;
+    a.group = (int32_t)p->group_size;
+    a.bias = p->bias;
+    a.bias_dtype = p->bias_dtype;
+    a.y = p->y;
+    a.y_ld = p->y_ld;
+    uint8_t* ws = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(p->workspace) + 255) & ~(uintptr_t)255);
+    a.count = reinterpret_cast<unsigned long long*>(ws);
+    a.part = reinterpret_cast<float*>(ws + (((uint64_t)q.tiles * 8u + 255u) & ~(uint64_t)255u));
+    a.nonce = next_nonce() & 0x00FFFFFFFFFFFFFFull;
+    const uint32_t f = bf16 ? 1u : 0u;
+    a.idesc = make_idesc(1u, f, f, 0u, 0u, 128u, (uint32_t)q.rows);
+    CUtensorMap mw, mx;
+    const bool ok = nk ? mix_map(&mw, p->w, (uint64_t)p->k * bits / 8, (uint64_t)p->n, (uint64_t)p->w_ld * bits / 8, bits == 4 ? 64u : 128u, kMixTileN)
+                       : mix_map(&mw, p->w, (uint64_t)p->n * bits / 8, (uint64_t)p->k, (uint64_t)p->w_ld * bits / 8, 128u, 64u);
+    if (!ok || !mix_map(&mx, p->x, (uint64_t)p->k * 2, (uint64_t)p->m, (uint64_t)p->x_ld * 2, 128u, (uint32_t)q.rows)) return (int32_t)cudaErrorInvalidValue;
+    int32_t rc;
+    if (p->w_dtype == ACL_INT4) rc = nk ? mix_dispatch<MixW::kInt4, true>(bf16, off, mw, mx, a, smem, stream) : mix_dispatch<MixW::kInt4, false>(bf16, off, mw, mx, a, smem, stream);
+    else if (p->w_dtype == ACL_INT8) rc = nk ? mix_dispatch<MixW::kInt8, true>(bf16, off, mw, mx, a, smem, stream) : mix_dispatch<MixW::kInt8, false>(bf16, off, mw, mx, a, smem, stream);
+    else rc = nk ? mix_dispatch<MixW::kE4m3, true>(bf16, off, mw, mx, a, smem, stream) : mix_dispatch<MixW::kE4m3, false>(bf16, off, mw, mx, a, smem, stream);
+    note_launch(p->w_dtype == ACL_INT4 ? "wqbmm_decode" : "wqbmm_decode8");
+    return rc;
+}
+
+// Error word of this file's kernel on the current device (see opsnn_wqbmm_decode_status).
+uint32_t wqbmm_mixed_status(int reset)
+{
+    unsigned int v = 0;
+    cudaMemcpyFromSymbol(&v, g_mix_status, sizeof(v));
+    if (reset) {
+        unsigned int z = 0;
+        cudaMemcpyToSymbol(g_mix_status, &z, sizeof(z));
+    }
+    return v;
+}
+
+}  // namespace opsnn
