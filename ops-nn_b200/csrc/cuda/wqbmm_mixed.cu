@@ -39,21 +39,19 @@ constexpr int kMixMaxStages = 16;
 constexpr int kMixSmemMax = 225 * 1024;
 
 struct MixArgs {
-    int32_t m, n_tiles, t_tiles, rows;  // rows: rows of x per tile (N of the MMA)
-    int64_t n, k;
-    int32_t kb;          // k stages per tile
-    int32_t stages, stage_bytes, x_off, sc_off;
-    int32_t grid;
-    int64_t units;       // n_tiles * t_tiles * kb
+    int32_t m, t_tiles, rows;  // rows: rows of x per tile (N of the MMA)
+    uint32_t n, k, kb;         // kb: k stages per tile
+    uint32_t grid, units;      // units = tiles * kb, cut into `grid` contiguous pieces; units * grid < 2^32
+    uint32_t stages, stage_bytes, x_off, sc_off, sc_rows;  // sc_rows: scale rows a stage needs (2: groups that end inside a stage)
     const void* scale;
     const void* offset;
     int64_t scale_sg, scale_sn;
-    int32_t group;       // rows of k per group; 0: one group
+    uint32_t group;       // rows of k per group (one group: at least k)
     const void* bias;
     int32_t bias_dtype;
     void* y;
     int64_t y_ld;
-    float* part;                   // [2 grid][2][rows / 4][128] float4
+    float4* part;                  // [2 grid][2 rows / 4][128]
     unsigned long long* count;     // [tiles] (nonce << 8) | arrivals
     unsigned long long nonce;
     uint32_t idesc;
@@ -81,6 +79,17 @@ __device__ __forceinline__ void mix_arrive(uint32_t bar_addr)
 __device__ __forceinline__ bool mix_wait(uint32_t bar_addr, uint32_t parity, volatile uint32_t* abort_flag)
 {
     return __all_sync(0xffffffffu, ptx::mbar_wait_a(bar_addr, parity, abort_flag));
+}
+// Barrier of kThreads threads that tells all of them whether every one came with `ok`: they go on, or leave, together.
+template <int kBar, int kThreads>
+__device__ __forceinline__ bool mix_all_ok(bool ok)
+{
+    uint32_t r;
+    asm volatile("{\n\t.reg .pred p, q;\n\tsetp.ne.u32 q, %1, 0;\n\tbar.red.and.pred p, %2, %3, q;\n\tselp.u32 %0, 1, 0, p;\n\t}"
+                 : "=r"(r)
+                 : "r"(ok ? 1u : 0u), "n"(kBar), "n"(kThreads)
+                 : "memory");
+    return r != 0u;
 }
 __device__ __forceinline__ void mix_init(uint32_t bar_addr, uint32_t count)
 {
@@ -125,13 +134,13 @@ __device__ __forceinline__ void umma_f16_ta(uint32_t d_tmem, uint32_t a_tmem, ui
 
 enum class MixW { kInt4, kInt8, kE4m3 };
 
-template <MixW kW, bool kNK>
+// One stage: 128 rows of k x 256 columns. (With 64-row stages the producer's and the MMA issuer's fixed cost per stage showed.)
+template <MixW kW>
 struct MixCfg {
     static constexpr int kBits = kW == MixW::kInt4 ? 4 : 8;
-    static constexpr int kBK = kNK ? 128 : 64;  // k rows per stage: rows of 128 (or, int4 (n,k), 64) bytes for the copies
-    static constexpr int kUnits = kBK / 64;
+    static constexpr int kBK = 128;
     static constexpr int kWBytes = kMixTileN * kBK * kBits / 8;
-    static constexpr int kEmptyArrivals = (kNK ? kMixDqWarps : kMixDqWarps / 2) + 1;
+    static constexpr int kEmptyArrivals = kMixDqWarps + 1;
 };
 
 // A pair of weights, codes in the low bits of the two halves (other bits arbitrary), to the 16-bit type, exactly (int4: the caller has
@@ -188,30 +197,127 @@ __device__ __forceinline__ int mix_col_of_lane(int l)
 }
 
 // A CTA's contiguous piece of the (tile, stage) line.
-__device__ __forceinline__ int64_t mix_begin(const MixArgs& a, int64_t c) { return c * a.units / a.grid; }
+__device__ __forceinline__ uint32_t mix_begin(const MixArgs& a, uint32_t c) { return c * a.units / a.grid; }
+__device__ __forceinline__ uint32_t mix_owner(const MixArgs& a, uint32_t unit)
+{
+    uint32_t c = unit * a.grid / a.units;
+    while (mix_begin(a, c + 1) <= unit) ++c;
+    while (mix_begin(a, c) > unit) --c;
+    return c;
+}
+
+// One column of 16 rows of y.
+template <bool kBf16>
+__device__ __forceinline__ void mix_store(const MixArgs& a, uint32_t n, uint32_t r0, const float (&f)[16])
+{
+    if (n >= a.n) return;
+    const float b = a.bias != nullptr ? load_as_float(a.bias, n, a.bias_dtype) : 0.f;
+    uint16_t* y = reinterpret_cast<uint16_t*>(a.y) + (int64_t)r0 * a.y_ld + n;
+#pragma unroll
+    for (int i = 0; i < 16; ++i) {
+        if ((int)r0 + i >= a.m) break;
+        const float v = a.bias != nullptr ? __fadd_rn(f[i], b) : f[i];
+        y[(int64_t)i * a.y_ld] = kBf16 ? __bfloat16_as_ushort(__float2bfloat16_rn(v)) : __half_as_ushort(__float2half_rn(v));
+    }
+}
+
+// A finished piece of tile t (stages kb .. kb + cnt of it) out of the accumulator set at TMEM address `acc` (this warp's lanes): stored
+// if it is the whole tile, else parked in workspace, and combined by whoever arrives last. Run by kWarps warps (four per TMEM lane
+// quarter and column share): 4 of them beside the main loop, or 16 at the end of the CTA's work.
+template <bool kBf16, int kWarps>
+__device__ __forceinline__ void mix_finish(const MixArgs& a, uint32_t acc, uint32_t t, uint32_t cnt, int col, int qd, int lane, int share, bool leader,
+                                           volatile uint32_t* s_last, volatile uint32_t* abort_flag)
+{
+    constexpr int kBar = kWarps == 4 ? 1 : 2;
+    constexpr uint32_t kStep = 16u * (kWarps / 4);
+    const uint32_t rows = (uint32_t)a.rows, tn = t / (uint32_t)a.t_tiles, tt = t - tn * (uint32_t)a.t_tiles;
+    const uint32_t n0 = tn * kMixTileN + col;
+    const bool whole = cnt == a.kb;
+    const uint32_t slot = (rows / 2) * 128u, row = (uint32_t)(qd * 32 + lane);
+    float4* mine = a.part + (2u * blockIdx.x + (t == mix_begin(a, blockIdx.x) / a.kb ? 0u : 1u)) * slot + row;
+#pragma unroll 1
+    for (uint32_t hc = 16u * share; hc < 2u * rows; hc += kStep) {
+        uint32_t v[16];
+        ptx::tmem_ld16(acc + hc, v);
+        ptx::tmem_ld_wait();
+        float f[16];
+#pragma unroll
+        for (int i = 0; i < 16; ++i) f[i] = __uint_as_float(v[i]);
+        if (whole) {
+            const uint32_t h = hc >= rows ? 1u : 0u;
+            mix_store<kBf16>(a, n0 + 128u * h, tt * rows + hc - h * rows, f);
+        } else {
+#pragma unroll
+            for (int i = 0; i < 4; ++i) __stcg(mine + (hc / 4 + i) * 128u, make_float4(f[4 * i], f[4 * i + 1], f[4 * i + 2], f[4 * i + 3]));
+        }
+    }
+    if (whole) return;
+    const uint32_t c0 = mix_owner(a, t * a.kb), c1 = mix_owner(a, (t + 1u) * a.kb - 1u);  // the CTAs whose pieces meet this tile
+    __threadfence();
+    asm volatile("bar.sync %0, %1;" ::"n"(kBar), "n"(kWarps * 32) : "memory");  // all of this CTA's partial sums are written and fenced
+    if (leader) {
+        unsigned long long* cnt_p = a.count + t;
+        unsigned long long cur = *reinterpret_cast<volatile unsigned long long*>(cnt_p), want = 0ull;
+        bool done = false;
+        for (int it = 0; it < 4096 && !done; ++it) {  // at most c1 - c0 other CTAs can get in between
+            want = ((cur >> 8) == a.nonce) ? cur + 1ull : ((a.nonce << 8) | 1ull);
+            const unsigned long long prev = atomicCAS(cnt_p, cur, want);
+            done = prev == cur;
+            cur = prev;
+        }
+        if (!done) mix_report(abort_flag, (4u << 8) | 2u);
+        const bool last = done && (uint32_t)(want & 0xFFull) == c1 - c0 + 1u;
+        if (last) *reinterpret_cast<volatile unsigned long long*>(cnt_p) = 0ull;  // a replay of this launch starts clean
+        *s_last = last ? 1u : 0u;
+    }
+    asm volatile("bar.sync %0, %1;" ::"n"(kBar), "n"(kWarps * 32) : "memory");
+    if (*s_last == 0u) return;
+    __threadfence();
+#pragma unroll 1
+    for (uint32_t hc = 16u * share; hc < 2u * rows; hc += kStep) {
+        float f[16];
+#pragma unroll
+        for (int i = 0; i < 16; ++i) f[i] = 0.f;
+#pragma unroll 2
+        for (uint32_t c = c0; c <= c1; ++c) {
+            // only the first of a CTA's tiles can be shared with the CTAs before it: its other shared tile starts with it
+            const uint32_t sl = 2u * c + (c == c0 && mix_begin(a, c) / a.kb != t ? 1u : 0u);
+            const float4* p = a.part + sl * slot + (hc / 4) * 128u + row;
+            float4 q[4];
+#pragma unroll
+            for (int i = 0; i < 4; ++i) q[i] = __ldcg(p + i * 128);
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+                f[4 * i] += q[i].x; f[4 * i + 1] += q[i].y; f[4 * i + 2] += q[i].z; f[4 * i + 3] += q[i].w;
+            }
+        }
+        const uint32_t h = hc >= rows ? 1u : 0u;
+        mix_store<kBf16>(a, n0 + 128u * h, tt * rows + hc - h * rows, f);
+    }
+}
 
 template <MixW kW, bool kNK, bool kBf16, bool kOff>
 __global__ void __launch_bounds__(kMixThreads, 1)
-wqbmm_mixed_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUtensorMap map_x, const MixArgs a)
+wqbmm_mixed_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUtensorMap map_x, const __grid_constant__ MixArgs a)
 {
-    using C = MixCfg<kW, kNK>;
+    using C = MixCfg<kW>;
     const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0);
     const int lane = threadIdx.x & 31;
     extern __shared__ uint8_t dyn_raw[];
     const uint32_t smem0 = (ptx::smem_u32(dyn_raw) + 1023u) & ~1023u;
-    __shared__ __align__(8) uint64_t s_bars[2 * kMixMaxStages + 2 * kMixABufs + 4];
+    __shared__ __align__(8) uint64_t s_bars[2 * kMixMaxStages + 2 * kMixABufs + 5];
     __shared__ uint32_t s_tmem;
     __shared__ volatile uint32_t s_abort;
-    __shared__ uint32_t s_last;
+    __shared__ volatile uint32_t s_last[2];
     const uint32_t full0 = ptx::smem_u32(s_bars), empty0 = full0 + 8u * kMixMaxStages;
     const uint32_t afull0 = empty0 + 8u * kMixMaxStages, aempty0 = afull0 + 8u * kMixABufs;
-    const uint32_t dfull0 = aempty0 + 8u * kMixABufs, dempty0 = dfull0 + 16u;
+    const uint32_t dfull0 = aempty0 + 8u * kMixABufs, dempty0 = dfull0 + 16u, fin0 = dempty0 + 16u;
     volatile uint32_t* abort_flag = &s_abort;
 
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     if (threadIdx.x == 0) {
         s_abort = 0u;
-        for (int i = 0; i < a.stages; ++i) {
+        for (uint32_t i = 0; i < a.stages; ++i) {
             mix_init(full0 + 8u * i, 1u);
             mix_init(empty0 + 8u * i, (uint32_t)C::kEmptyArrivals);
         }
@@ -223,61 +329,71 @@ wqbmm_mixed_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
             mix_init(dfull0 + 8u * i, 1u);
             mix_init(dempty0 + 8u * i, kMixEpWarps);
         }
+        mix_init(fin0, 1u);  // the last piece's sums (its own barrier: the warps that wait for it have not followed the others' phases)
         ptx::fence_mbar_init();
         ptx::fence_proxy_async();
     }
     if (warp == kMixDqWarps + kMixEpWarps + 1) ptx::tmem_alloc(&s_tmem, 512);
+    if (warp == kMixDqWarps + kMixEpWarps && lane == 0) {
+        ptx::tma_prefetch_desc(&map_w);
+        ptx::tma_prefetch_desc(&map_x);
+    }
     ptx::tc_fence_before();
     __syncthreads();
     ptx::tc_fence_after();
     const uint32_t tmem = s_tmem;
     asm volatile("griddepcontrol.wait;" ::: "memory");  // nothing another kernel may have written is read before this
 
-    const int64_t u_begin = mix_begin(a, blockIdx.x), u_end = mix_begin(a, (int64_t)blockIdx.x + 1);
-    const uint32_t stages = (uint32_t)a.stages, stage_bytes = (uint32_t)a.stage_bytes;
+    const uint32_t u_begin = mix_begin(a, blockIdx.x), u_end = mix_begin(a, blockIdx.x + 1);
+    const uint32_t stages = a.stages, stage_bytes = a.stage_bytes;
     const uint32_t xunit = (uint32_t)a.rows * 128u;  // bytes of x per 64-row unit of k
     const bool two_d = a.rows <= 64;                 // two accumulator sets
+    const uint32_t d_set = 2u * (uint32_t)a.rows;
 
     if (warp == kMixDqWarps + kMixEpWarps) {
         // ======================= TMA producer =======================
-        if (lane == 0) {
-            ptx::tma_prefetch_desc(&map_w);
-            ptx::tma_prefetch_desc(&map_x);
-        }
-        __syncwarp();
+        // Its time per stage bounds the stream: no division but one by the group size, everything else counted along.
         uint32_t s = 0, par = 0;
-        int64_t t = u_begin / a.kb;
-        int32_t kb = (int32_t)(u_begin - t * a.kb);
-        for (int64_t u = u_begin; u < u_end; ++u) {
+        const uint32_t t0 = u_begin / a.kb;
+        uint32_t kb = u_begin - t0 * a.kb;
+        uint32_t n0 = t0 / (uint32_t)a.t_tiles, r0 = (t0 - n0 * (uint32_t)a.t_tiles) * (uint32_t)a.rows;
+        const uint32_t r_end = (uint32_t)(a.t_tiles * a.rows);
+        n0 *= kMixTileN;
+        const uint32_t sc_rows = kNK ? 0u : a.sc_rows * (kOff ? 2u : 1u);
+        for (uint32_t u = u_begin; u < u_end; ++u) {
             if (!mix_wait(empty0 + 8u * s, par ^ 1u, abort_flag)) {
                 mix_report(abort_flag, (1u << 8) | 1u);
                 break;
             }
             if (ptx::elect_one()) {
-                const int32_t tn = (int32_t)(t / a.t_tiles), tt = (int32_t)(t - (int64_t)tn * a.t_tiles);
-                const int32_t n0 = tn * kMixTileN, k0 = kb * C::kBK;
-                const uint32_t fb = full0 + 8u * s, dst = smem0 + s * stage_bytes;
-                uint32_t sc_bytes = 0;
-                if (!kNK) sc_bytes = (uint32_t)min((int64_t)(kMixTileN * 2), (a.n - n0) * 2);
-                ptx::mbar_expect_tx_a(fb, (uint32_t)C::kWBytes + xunit * C::kUnits + sc_bytes * (kOff ? 2u : 1u));
+                const uint32_t k0 = kb * C::kBK, fb = full0 + 8u * s, dst = smem0 + s * stage_bytes;
+                const uint32_t sc_bytes = min((uint32_t)kMixTileN, a.n - n0) * 2u;
+                ptx::mbar_expect_tx_a(fb, (uint32_t)C::kWBytes + 2u * xunit + sc_bytes * sc_rows);
                 if (kNK) {
-                    mix_tma_2d(dst, &map_w, fb, k0 * C::kBits / 8, n0);
+                    mix_tma_2d(dst, &map_w, fb, (int32_t)(k0 * C::kBits / 8), (int32_t)n0);
                 } else {
-                    mix_tma_2d(dst, &map_w, fb, n0 * C::kBits / 8, k0);
-                    if (C::kBits == 8) mix_tma_2d(dst + C::kWBytes / 2, &map_w, fb, n0 + 128, k0);
+                    mix_tma_2d(dst, &map_w, fb, (int32_t)(n0 * C::kBits / 8), (int32_t)k0);
+                    if (C::kBits == 8) mix_tma_2d(dst + C::kWBytes / 2, &map_w, fb, (int32_t)n0 + 128, (int32_t)k0);
                 }
-#pragma unroll
-                for (int i = 0; i < C::kUnits; ++i) mix_tma_2d(dst + a.x_off + i * xunit, &map_x, fb, (k0 + 64 * i) * 2, tt * a.rows);
+                mix_tma_2d(dst + a.x_off, &map_x, fb, (int32_t)k0 * 2, (int32_t)r0);
+                mix_tma_2d(dst + a.x_off + xunit, &map_x, fb, (int32_t)k0 * 2 + 128, (int32_t)r0);
                 if (!kNK) {
-                    const int64_t g = a.group > 0 ? min((int64_t)k0, a.k - 1) / a.group : 0;
-                    const int64_t at = g * a.scale_sg + n0;
-                    ptx::bulk_load_a(dst + a.sc_off, reinterpret_cast<const uint16_t*>(a.scale) + at, sc_bytes, fb);
-                    if (kOff) ptx::bulk_load_a(dst + a.sc_off + kMixTileN * 2, reinterpret_cast<const uint16_t*>(a.offset) + at, sc_bytes, fb);
+                    uint32_t sd = dst + a.sc_off;
+                    for (uint32_t i = 0; i < a.sc_rows; ++i) {
+                        const int64_t at = (int64_t)(min(k0 + 64u * i, a.k - 1u) / a.group) * a.scale_sg + n0;
+                        ptx::bulk_load_a(sd, reinterpret_cast<const uint16_t*>(a.scale) + at, sc_bytes, fb);
+                        if (kOff) ptx::bulk_load_a(sd + kMixTileN * 2, reinterpret_cast<const uint16_t*>(a.offset) + at, sc_bytes, fb);
+                        sd += kMixTileN * 4;
+                    }
                 }
             }
             __syncwarp();
             if (++s == stages) { s = 0; par ^= 1u; }
-            if (++kb == a.kb) { kb = 0; ++t; }
+            if (++kb == a.kb) {
+                kb = 0;
+                r0 += (uint32_t)a.rows;
+                if (r0 == r_end) { r0 = 0; n0 += kMixTileN; }
+            }
         }
     } else if (warp == kMixDqWarps + kMixEpWarps + 1) {
         // ======================= MMA issuer =======================
@@ -286,25 +402,24 @@ wqbmm_mixed_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
         const uint64_t b_hi = db & 0xFFFFFFFF00000000ull;
         uint32_t s = 0, par = 0, ab = 0, apar = 0, seg = 0;
         bool ok = true;
-        int64_t u = u_begin;
-        int32_t kb = (int32_t)(u_begin % a.kb);
+        uint32_t u = u_begin, kb = u_begin % a.kb;
         while (u < u_end && ok) {
-            const int32_t cnt = (int32_t)min((int64_t)(a.kb - kb), u_end - u);
+            const uint32_t cnt = min(a.kb - kb, u_end - u);
             const uint32_t dbuf = two_d ? (seg & 1u) : 0u, dpar = two_d ? ((seg >> 1) & 1u) : (seg & 1u);
             if (!mix_wait(dempty0 + 8u * dbuf, dpar ^ 1u, abort_flag)) {
                 mix_report(abort_flag, (2u << 8) | 1u);
                 break;
             }
-            const uint32_t d0 = tmem + dbuf * 2u * (uint32_t)a.rows;
+            const uint32_t d0 = tmem + dbuf * d_set;
             uint32_t acc = 0u;
-            for (int32_t i = 0; i < cnt && ok; ++i) {
+            for (uint32_t i = 0; i < cnt && ok; ++i) {
                 if (!mix_wait(full0 + 8u * s, par, abort_flag)) {
                     mix_report(abort_flag, (2u << 8) | 2u);
                     ok = false;
                     break;
                 }
 #pragma unroll
-                for (int un = 0; un < C::kUnits; ++un) {
+                for (int un = 0; un < 2; ++un) {
                     if (!mix_wait(afull0 + 8u * ab, apar, abort_flag)) {
                         mix_report(abort_flag, (2u << 8) | 3u);
                         ok = false;
@@ -322,7 +437,7 @@ wqbmm_mixed_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
                                             kk == 0 ? acc : 1u);
                         }
                         ptx::umma_commit_a(aempty0 + 8u * ab);
-                        if (un == C::kUnits - 1) ptx::umma_commit_a(empty0 + 8u * s);
+                        if (un == 1) ptx::umma_commit_a(empty0 + 8u * s);
                     }
                     __syncwarp();
                     acc = 1u;
@@ -331,53 +446,50 @@ wqbmm_mixed_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
                 if (++s == stages) { s = 0; par ^= 1u; }
             }
             if (!ok) break;
-            if (ptx::elect_one()) ptx::umma_commit_a(dfull0 + 8u * dbuf);
+            u += cnt;
+            if (ptx::elect_one()) ptx::umma_commit_a(u < u_end ? dfull0 + 8u * dbuf : fin0);
             __syncwarp();
             ++seg;
-            u += cnt;
             kb = 0;
         }
     } else if (warp < kMixDqWarps) {
         // ======================= dequantisation =======================
         const int qd = warp & 3, h = (warp >> 2) & 1;
-        const uint32_t grp = (uint32_t)warp >> 3;
+        const uint32_t un = (uint32_t)warp >> 3;  // the 64-row unit of every stage that this warp serves
         const int g = lane >> 2;
         const uint32_t tlane = (uint32_t)(qd * 32) << 16;
         const int wcol = h * 128 + qd * 32;  // the warp's first column in the tile
-        uint32_t s = 0, par = 0;
-        if (!kNK) {  // units alternate between the two groups of eight warps
-            s = grp;
-            if (s >= stages) { s -= stages; par ^= 1u; }
-        }
-        uint32_t ab = grp, apar = 0;
-        // (n,k) storage: the lane's own scale and offset, a stage's worth ahead
-        const int64_t u0 = u_begin + (kNK ? 0 : grp);
-        int64_t t = u0 / a.kb;
-        int32_t kb = (int32_t)(u0 - t * a.kb);
+        uint32_t s = 0, par = 0, ab = un, apar = 0;
+        uint32_t t = u_begin / a.kb, kb = u_begin - t * a.kb, seg = 0;
+        bool ok = true;
+        // (n,k) storage: the lane's own scale and offset, a stage ahead
         uint32_t sc_next = 0, of_next = 0;
-        auto fetch = [&](int64_t tile, int32_t stage) {
-            const int64_t n = min((tile / a.t_tiles) * kMixTileN + wcol + lane, a.n - 1);
-            const int64_t kk = min((int64_t)stage * C::kBK + 64 * grp, a.k - 1);
-            const int64_t at = (a.group > 0 ? kk / a.group : 0) * a.scale_sg + n * a.scale_sn;
+        auto fetch = [&](uint32_t tile, uint32_t stage) {
+            const uint32_t n = min((tile / (uint32_t)a.t_tiles) * kMixTileN + wcol + lane, a.n - 1u);
+            const int64_t at = (int64_t)(min(stage * C::kBK + 64u * un, a.k - 1u) / a.group) * a.scale_sg + (int64_t)n * a.scale_sn;
             sc_next = __ldg(reinterpret_cast<const uint16_t*>(a.scale) + at);
             if (kOff) of_next = __ldg(reinterpret_cast<const uint16_t*>(a.offset) + at);
         };
-        if (kNK && u0 < u_end) fetch(t, kb);
-        for (int64_t u = u0; u < u_end; u += kNK ? 1 : 2) {
+        if (kNK && u_begin < u_end) fetch(t, kb);
+        for (uint32_t u = u_begin; u < u_end; ++u) {
             uint32_t sc[4], of[4];
             if (kNK) {
                 sc[0] = sc_next | (sc_next << 16);
                 of[0] = of_next | (of_next << 16);
-                if (++kb == a.kb) { kb = 0; ++t; }
-                if (u + 1 < u_end) fetch(t, kb);
             }
+            if (++kb == a.kb) {
+                kb = 0;
+                if (u + 1 < u_end) { ++t; ++seg; }
+            }
+            if (kNK && u + 1 < u_end) fetch(t, kb);
             if (!mix_wait(full0 + 8u * s, par, abort_flag)) {
                 mix_report(abort_flag, (3u << 8) | 1u);
+                ok = false;
                 break;
             }
             const uint32_t base = smem0 + s * stage_bytes;
             if (!kNK) {  // int4: columns 4g .. 4g + 3; int8: 2g, 2g + 1 of each 16
-                const uint32_t at = base + a.sc_off + 2u * wcol;
+                const uint32_t at = base + a.sc_off + (a.sc_rows == 2u ? un * (kMixTileN * 4u) : 0u) + 2u * wcol;
                 uint32_t r0, r1, o0 = 0, o1 = 0;
                 const uint32_t p0 = kW == MixW::kInt4 ? at + 8u * g : at + 4u * g, p1 = kW == MixW::kInt4 ? p0 + 4u : p0 + 32u;
                 asm volatile("ld.shared.u32 %0, [%1];" : "=r"(r0) : "r"(p0) : "memory");
@@ -389,26 +501,25 @@ wqbmm_mixed_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
                 sc[0] = prmt(r0, r0, 0x1010); sc[1] = prmt(r0, r0, 0x3232); sc[2] = prmt(r1, r1, 0x1010); sc[3] = prmt(r1, r1, 0x3232);
                 of[0] = prmt(o0, o0, 0x1010); of[1] = prmt(o0, o0, 0x3232); of[2] = prmt(o1, o1, 0x1010); of[3] = prmt(o1, o1, 0x3232);
             }
-            bool waited = false, dead = false;
+            bool waited = false;
             const uint32_t abase = tmem + kMixACol + ab * 64u + h * 32u + tlane;
             auto need_buffer = [&]() {  // the MMAs that read this A buffer's previous contents are done
                 if (waited) return;
                 waited = true;
                 if (!mix_wait(aempty0 + 8u * ab, apar ^ 1u, abort_flag)) {
                     mix_report(abort_flag, (3u << 8) | 2u);
-                    dead = true;
+                    ok = false;
                 }
                 ptx::tc_fence_after();
             };
             if constexpr (!kNK) {
                 const int r = lane & 7, j = lane >> 3;
                 if constexpr (kW == MixW::kInt4) {
-                    // 64 rows of 128 bytes; matrix j of an ldmatrix = rows 8 j .. of a half of 32, the warp's 16 bytes of the row
-                    const uint32_t at = base + (uint32_t)(8 * j + r) * 128u + (uint32_t)(((h * 4 + qd) ^ r) << 4);
+                    // rows of 128 bytes; matrix j of an ldmatrix = rows 8 j .. of a half of 32, the warp's 16 bytes of the row
+                    const uint32_t at = base + un * (64u * 128u) + (uint32_t)(8 * j + r) * 128u + (uint32_t)(((h * 4 + qd) ^ r) << 4);
                     uint32_t w[2][4];
                     mix_ldsm4_trans(at, w[0]);
                     mix_ldsm4_trans(at + 32 * 128, w[1]);
-                    __syncwarp();
 #pragma unroll
                     for (int half = 0; half < 2; ++half) {
                         uint32_t o[2][8];
@@ -422,7 +533,7 @@ wqbmm_mixed_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
                         tmem_st_16x128b_x4(abase + half * 16 + (16u << 16), o[1]);
                     }
                 } else {
-                    const uint32_t box = base + h * (C::kWBytes / 2) + (uint32_t)(8 * j + r) * 128u;
+                    const uint32_t box = base + h * (C::kWBytes / 2) + un * (64u * 128u) + (uint32_t)(8 * j + r) * 128u;
 #pragma unroll
                     for (int half = 0; half < 2; ++half) {
 #pragma unroll
@@ -457,7 +568,7 @@ wqbmm_mixed_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
                     const uint32_t x = (uint32_t)(row >> 1) & 3u;  // 64-byte swizzle
 #pragma unroll
                     for (int c = 0; c < 2; ++c) {
-                        const uint4 v = mix_lds128(rb + (((2u * grp + c) ^ x) << 4));
+                        const uint4 v = mix_lds128(rb + (((2u * un + c) ^ x) << 4));
                         const uint32_t w[4] = {v.x, v.y, v.z, v.w};
 #pragma unroll
                         for (int hh = 0; hh < 2; ++hh) {
@@ -478,7 +589,7 @@ wqbmm_mixed_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
                     const uint32_t x = (uint32_t)row & 7u;  // 128-byte swizzle
 #pragma unroll
                     for (int c = 0; c < 4; ++c) {
-                        const uint4 v = mix_lds128(rb + (((4u * grp + c) ^ x) << 4));
+                        const uint4 v = mix_lds128(rb + (((4u * un + c) ^ x) << 4));
                         const uint32_t w[4] = {v.x, v.y, v.z, v.w};
                         uint32_t o[8];
 #pragma unroll
@@ -502,7 +613,8 @@ wqbmm_mixed_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
                     }
                 }
             }
-            if (dead) break;
+            if (!ok) break;
+            __syncwarp();
             if (lane == 0) mix_arrive(empty0 + 8u * s);  // the packed words (and scale rows) of this stage are in registers
             tmem_st_wait();
             ptx::tc_fence_before();
@@ -510,118 +622,40 @@ wqbmm_mixed_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
             if (lane == 0) mix_arrive(afull0 + 8u * ab);
             ab += 2u;
             if (ab >= kMixABufs) { ab -= kMixABufs; apar ^= 1u; }
-            s += kNK ? 1u : 2u;
-            if (s >= stages) { s -= stages; par ^= 1u; }
+            if (++s == stages) { s = 0; par ^= 1u; }
+        }
+        // the CTA's last piece: nothing is left to dequantise, all sixteen warps finish it
+        const uint32_t dbuf = two_d ? (seg & 1u) : 0u;
+        if (ok && !mix_wait(fin0, 0u, abort_flag)) {
+            mix_report(abort_flag, (3u << 8) | 3u);
+            ok = false;
+        }
+        if (mix_all_ok<2, kMixDqWarps * 32>(ok)) {
+            ptx::tc_fence_after();
+            mix_finish<kBf16, 16>(a, tmem + tlane + dbuf * d_set, t, min(u_end - t * a.kb, u_end - u_begin), qd * 32 + mix_col_of_lane<kW, kNK>(lane), qd,
+                                  lane, warp >> 2, threadIdx.x == 0, &s_last[1], abort_flag);
         }
     } else {
-        // ======================= epilogue =======================
-        const int qd = warp & 3, et = (warp - kMixDqWarps) * 32 + lane;  // 0..127
+        // ======================= epilogue of all but the last piece, beside the main loop =======================
+        const int qd = warp & 3;
         const uint32_t tlane = (uint32_t)(qd * 32) << 16;
-        const int mycol = qd * 32 + mix_col_of_lane<kW, kNK>(lane);
-        const uint32_t rows = (uint32_t)a.rows;
-        uint32_t seg = 0;
-        int64_t u = u_begin;
-        auto store = [&](int64_t n, int tt, uint32_t c, const float (&f)[16]) {  // 16 rows of y, one column
-            if (n >= a.n) return;
-            const float b = a.bias != nullptr ? load_as_float(a.bias, n, a.bias_dtype) : 0.f;
-            const int r0 = tt * (int)rows + (int)c;
-            uint16_t* y = reinterpret_cast<uint16_t*>(a.y) + (int64_t)r0 * a.y_ld + n;
-#pragma unroll
-            for (int i = 0; i < 16; ++i) {
-                if (r0 + i >= a.m) break;
-                const float v = a.bias != nullptr ? __fadd_rn(f[i], b) : f[i];
-                y[(int64_t)i * a.y_ld] = kBf16 ? __bfloat16_as_ushort(__float2bfloat16_rn(v)) : __half_as_ushort(__float2half_rn(v));
-            }
-        };
-        while (u < u_end) {
-            const int64_t t = u / a.kb;
-            const int32_t kb = (int32_t)(u - t * a.kb);
-            const int64_t cnt = min((int64_t)(a.kb - kb), u_end - u);
+        const int col = qd * 32 + mix_col_of_lane<kW, kNK>(lane);
+        uint32_t seg = 0, u = u_begin, t = u_begin / a.kb, kb = u_begin - t * a.kb;
+        while (u + (a.kb - kb) < u_end) {
+            const uint32_t cnt = a.kb - kb;
             const uint32_t dbuf = two_d ? (seg & 1u) : 0u, dpar = two_d ? ((seg >> 1) & 1u) : (seg & 1u);
-            const int64_t n0 = (t / a.t_tiles) * kMixTileN + mycol;
-            const int tt = (int)(t % a.t_tiles);
-            const bool whole = cnt == a.kb;
             const bool got = __all_sync(0xffffffffu, ptx::mbar_wait_relaxed(&s_bars[2 * kMixMaxStages + 2 * kMixABufs + dbuf], dpar, abort_flag));
             if (!got) mix_report(abort_flag, (4u << 8) | 1u);
-            asm volatile("bar.sync 1, 128;" ::: "memory");  // the four warps go on, or leave, together
-            if (*abort_flag != 0u) break;
+            if (!mix_all_ok<1, kMixEpWarps * 32>(got)) break;
             ptx::tc_fence_after();
-            const int64_t first_t = u_begin / a.kb;
-            float4* mine = reinterpret_cast<float4*>(a.part) + (2 * (int64_t)blockIdx.x + (t == first_t ? 0 : 1)) * (2 * (rows / 4) * 128);
-#pragma unroll 1
-            for (uint32_t hc = 0; hc < 2 * rows; hc += 16) {
-                uint32_t v[16];
-                ptx::tmem_ld16(tmem + tlane + dbuf * 2u * rows + hc, v);
-                ptx::tmem_ld_wait();
-                float f[16];
-#pragma unroll
-                for (int i = 0; i < 16; ++i) f[i] = __uint_as_float(v[i]);
-                if (whole) {
-                    const uint32_t hh = hc >= rows ? 1u : 0u;
-                    store(n0 + 128 * hh, tt, hc - hh * rows, f);
-                } else {
-#pragma unroll
-                    for (int i = 0; i < 4; ++i) __stcg(mine + (hc / 4 + i) * 128 + et, make_float4(f[4 * i], f[4 * i + 1], f[4 * i + 2], f[4 * i + 3]));
-                }
-            }
+            mix_finish<kBf16, 4>(a, tmem + tlane + dbuf * d_set, t, cnt, col, qd, lane, 0, warp == kMixDqWarps && lane == 0, &s_last[0], abort_flag);
             ptx::tc_fence_before();
             __syncwarp();
             if (lane == 0) mix_arrive(dempty0 + 8u * dbuf);
-            if (!whole) {
-                // the CTAs whose pieces meet this tile
-                auto owner = [&](int64_t unit) {
-                    int64_t c = unit * a.grid / a.units;
-                    while (mix_begin(a, c + 1) <= unit) ++c;
-                    while (mix_begin(a, c) > unit) --c;
-                    return c;
-                };
-                const int64_t c0 = owner(t * a.kb), c1 = owner((t + 1) * a.kb - 1);
-                __threadfence();
-                asm volatile("bar.sync 1, 128;" ::: "memory");  // all of this CTA's partial sums are written and fenced
-                if (et == 0) {
-                    unsigned long long* cnt_p = a.count + t;
-                    unsigned long long cur = *reinterpret_cast<volatile unsigned long long*>(cnt_p), want = 0ull;
-                    bool done = false;
-                    for (int it = 0; it < 4096 && !done; ++it) {  // at most c1 - c0 other CTAs can get in between
-                        want = ((cur >> 8) == a.nonce) ? cur + 1ull : ((a.nonce << 8) | 1ull);
-                        const unsigned long long prev = atomicCAS(cnt_p, cur, want);
-                        done = prev == cur;
-                        cur = prev;
-                    }
-                    if (!done) mix_report(abort_flag, (4u << 8) | 2u);
-                    const bool last = done && (int64_t)(want & 0xFFull) == c1 - c0 + 1;
-                    if (last) *reinterpret_cast<volatile unsigned long long*>(cnt_p) = 0ull;  // a replay of this launch starts clean
-                    s_last = last ? 1u : 0u;
-                }
-                asm volatile("bar.sync 1, 128;" ::: "memory");
-                if (s_last != 0u) {
-                    __threadfence();
-                    const float4* part = reinterpret_cast<const float4*>(a.part);
-                    const int64_t slot = 2 * (rows / 4) * 128;
-#pragma unroll 1
-                    for (uint32_t hc = 0; hc < 2 * rows; hc += 16) {
-                        float f[16];
-#pragma unroll
-                        for (int i = 0; i < 16; ++i) f[i] = 0.f;
-#pragma unroll 2
-                        for (int64_t c = c0; c <= c1; ++c) {
-                            const int64_t sl = 2 * c + (mix_begin(a, c) / a.kb == t ? 0 : 1);
-                            const float4* p = part + sl * slot + (hc / 4) * 128 + et;
-                            float4 q[4];
-#pragma unroll
-                            for (int i = 0; i < 4; ++i) q[i] = __ldcg(p + i * 128);
-#pragma unroll
-                            for (int i = 0; i < 4; ++i) {
-                                f[4 * i] += q[i].x; f[4 * i + 1] += q[i].y; f[4 * i + 2] += q[i].z; f[4 * i + 3] += q[i].w;
-                            }
-                        }
-                        const uint32_t hh = hc >= rows ? 1u : 0u;
-                        store(n0 + 128 * hh, tt, hc - hh * rows, f);
-                    }
-                }
-            }
             ++seg;
             u += cnt;
+            kb = 0;
+            ++t;
         }
     }
     // ---- teardown: everyone meets here, also after an aborted wait; then the allocating warp frees TMEM ----
@@ -646,7 +680,8 @@ MixEncodeFn mix_encoder()
     }();
     return fn;
 }
-bool mix_map(CUtensorMap* map, const void* base, uint64_t inner_bytes, uint64_t rows, uint64_t pitch, uint32_t box_inner, uint32_t box_rows)
+bool mix_map(CUtensorMap* map, const void* base, uint64_t inner_bytes, uint64_t rows, uint64_t pitch, uint32_t box_inner, uint32_t box_rows,
+             CUtensorMapL2promotion promotion = CU_TENSOR_MAP_L2_PROMOTION_L2_256B)
 {
     MixEncodeFn enc = mix_encoder();
     if (enc == nullptr) return false;
@@ -655,13 +690,13 @@ bool mix_map(CUtensorMap* map, const void* base, uint64_t inner_bytes, uint64_t 
     cuuint32_t box[2] = {box_inner, box_rows};
     cuuint32_t estr[2] = {1, 1};
     return enc(map, CU_TENSOR_MAP_DATA_TYPE_UINT8, 2, const_cast<void*>(base), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
-               box_inner == 64 ? CU_TENSOR_MAP_SWIZZLE_64B : CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+               box_inner == 64 ? CU_TENSOR_MAP_SWIZZLE_64B : CU_TENSOR_MAP_SWIZZLE_128B, promotion,
                CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
 struct MixPlan {
-    int t_tiles, rows, n_tiles, kb, grid;
-    int64_t units, tiles;
+    int t_tiles, rows;
+    int64_t n_tiles, kb, grid, units, tiles;
 };
 
 MixPlan mix_plan(const OpsnnWqbmmParams* p, int sms)
@@ -671,20 +706,15 @@ MixPlan mix_plan(const OpsnnWqbmmParams* p, int sms)
     const int64_t per = (p->m + q.t_tiles - 1) / q.t_tiles;
     q.rows = (int)((per + 15) / 16 * 16);
     q.t_tiles = (int)((p->m + q.rows - 1) / q.rows);
-    q.n_tiles = (int)((p->n + kMixTileN - 1) / kMixTileN);
-    const int bk = p->trans_w ? 128 : 64;
-    q.kb = (int)((p->k + bk - 1) / bk);
-    q.tiles = (int64_t)q.n_tiles * q.t_tiles;
+    q.n_tiles = (p->n + kMixTileN - 1) / kMixTileN;
+    q.kb = (p->k + 127) / 128;
+    q.tiles = q.n_tiles * q.t_tiles;
     q.units = q.tiles * q.kb;
-    const int64_t least = 512 / bk;  // k rows a CTA should at least see: a shorter piece is mostly ramp and combination
-    int64_t grid = q.units / least;
-    if (grid > sms) grid = sms;
-    if (grid < 1) grid = 1;
-    if (const char* e = env("OPSNN_WQ_MIXED_GRID")) {
-        const int v = atoi(e);
-        if (v > 0 && v <= sms && v <= q.units) grid = v;
-    }
-    q.grid = (int)grid;
+    int64_t least = 4;  // stages a CTA should at least see: a shorter piece is mostly ramp and combination
+    if (const char* e = env("OPSNN_WQ_MIXED_LEAST")) least = atoi(e) > 0 ? atoi(e) : least;
+    q.grid = q.units / least;
+    if (q.grid > sms) q.grid = sms;
+    if (q.grid < 1) q.grid = 1;
     return q;
 }
 
@@ -696,7 +726,7 @@ int32_t mix_launch(const CUtensorMap& mw, const CUtensorMap& mx, const MixArgs& 
     if (once_per_device(configured, [&] { return cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, kMixSmemMax); }) != cudaSuccess)
         return (int32_t)cudaGetLastError();
     cudaLaunchConfig_t cfg{};
-    cfg.gridDim = dim3((unsigned)a.grid, 1, 1);
+    cfg.gridDim = dim3(a.grid, 1, 1);
     cfg.blockDim = dim3(kMixThreads, 1, 1);
     cfg.dynamicSmemBytes = smem;
     cfg.stream = stream;
@@ -733,6 +763,7 @@ bool wqbmm_mixed_eligible(const OpsnnWqbmmParams* p)
     auto al16 = [](const void* q) { return (reinterpret_cast<uintptr_t>(q) & 15) == 0; };
     if (!al16(p->w) || !al16(p->x) || p->x_ld % 8 != 0 || (p->w_ld * bits / 8) % 16 != 0 || (p->w_ld * bits) % 8 != 0) return false;
     if (p->group_size != 0 && p->group_size % 64 != 0) return false;
+    if ((p->m + 15) / 16 * ((p->n + kMixTileN - 1) / kMixTileN) * ((p->k + 127) / 128) >= (1 << 24)) return false;  // 32-bit piece arithmetic
     if (p->trans_w) {
         if (bits == 4 && p->k % 2 != 0) return false;
         if (p->scale_sn < 0 || p->scale_sg < 0) return false;
@@ -758,41 +789,41 @@ int32_t wqbmm_mixed_launch(const OpsnnWqbmmParams* p, cudaStream_t stream)
     const int bits = p->w_dtype == ACL_INT4 ? 4 : 8;
     MixArgs a{};
     a.m = (int32_t)p->m;
-    a.n = p->n;
-    a.k = p->k;
-    a.n_tiles = q.n_tiles;
+    a.n = (uint32_t)p->n;
+    a.k = (uint32_t)p->k;
     a.t_tiles = q.t_tiles;
     a.rows = q.rows;
-    a.kb = q.kb;
-    a.units = q.units;
-    a.grid = q.grid;
-    const int bk = nk ? 128 : 64;
-    const int wbytes = kMixTileN * bk * bits / 8;
-    a.x_off = wbytes;
-    a.sc_off = wbytes + q.rows * 128 * (bk / 64);
-    a.stage_bytes = a.sc_off + (nk ? 0 : 1024);
+    a.kb = (uint32_t)q.kb;
+    a.units = (uint32_t)q.units;
+    a.grid = (uint32_t)q.grid;
+    a.group = p->group_size > 0 ? (uint32_t)p->group_size : 0x7FFFFFFFu;
+    a.sc_rows = p->group_size % 128 == 0 ? 1 : 2;
+    a.x_off = kMixTileN * 128 * bits / 8;
+    a.sc_off = a.x_off + q.rows * 256;
+    a.stage_bytes = a.sc_off + (nk ? 0 : 1024 * a.sc_rows);
     a.stages = (kMixSmemMax - 2048) / a.stage_bytes;
-    if (a.stages > kMixMaxStages) a.stages = kMixMaxStages;
+    if (a.stages > (uint32_t)kMixMaxStages) a.stages = kMixMaxStages;
     size_t smem = (size_t)a.stages * a.stage_bytes + 1024;
     if (smem < 116 * 1024) smem = 116 * 1024;  // one CTA per SM: the kernel owns all of the SM's tensor memory
     a.scale = p->scale;
     a.offset = p->offset;
     a.scale_sg = p->group_size > 0 ? p->scale_sg : 0;
     a.scale_sn = p->scale_sn;
-    a.group = (int32_t)p->group_size;
     a.bias = p->bias;
     a.bias_dtype = p->bias_dtype;
     a.y = p->y;
     a.y_ld = p->y_ld;
     uint8_t* ws = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(p->workspace) + 255) & ~(uintptr_t)255);
     a.count = reinterpret_cast<unsigned long long*>(ws);
-    a.part = reinterpret_cast<float*>(ws + (((uint64_t)q.tiles * 8u + 255u) & ~(uint64_t)255u));
+    a.part = reinterpret_cast<float4*>(ws + (((uint64_t)q.tiles * 8u + 255u) & ~(uint64_t)255u));
     a.nonce = next_nonce() & 0x00FFFFFFFFFFFFFFull;
     const uint32_t f = bf16 ? 1u : 0u;
     a.idesc = make_idesc(1u, f, f, 0u, 0u, 128u, (uint32_t)q.rows);
     CUtensorMap mw, mx;
     const bool ok = nk ? mix_map(&mw, p->w, (uint64_t)p->k * bits / 8, (uint64_t)p->n, (uint64_t)p->w_ld * bits / 8, bits == 4 ? 64u : 128u, kMixTileN)
-                       : mix_map(&mw, p->w, (uint64_t)p->n * bits / 8, (uint64_t)p->k, (uint64_t)p->w_ld * bits / 8, 128u, 64u);
+                       : mix_map(&mw, p->w, (uint64_t)p->n * bits / 8, (uint64_t)p->k, (uint64_t)p->w_ld * bits / 8, 128u, 128u,
+                                // a tile is 128 bytes of an int4 row: fetching 256 for it reads the neighbour's half twice (4.2 -> 5.5 TB/s)
+                                bits == 4 ? CU_TENSOR_MAP_L2_PROMOTION_L2_128B : CU_TENSOR_MAP_L2_PROMOTION_L2_256B);
     if (!ok || !mix_map(&mx, p->x, (uint64_t)p->k * 2, (uint64_t)p->m, (uint64_t)p->x_ld * 2, 128u, (uint32_t)q.rows)) return (int32_t)cudaErrorInvalidValue;
     int32_t rc;
     if (p->w_dtype == ACL_INT4) rc = nk ? mix_dispatch<MixW::kInt4, true>(bf16, off, mw, mx, a, smem, stream) : mix_dispatch<MixW::kInt4, false>(bf16, off, mw, mx, a, smem, stream);
