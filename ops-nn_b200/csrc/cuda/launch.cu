@@ -210,7 +210,9 @@ static int32_t decode_chunk_launches(const OpsnnWqbmmParams* p, cudaStream_t str
 // the packed weight dequantised into tensor memory, once for up to 128 rows of x) where that is the faster form.
 static bool mixed_instead(const OpsnnWqbmmParams* p, int32_t kernel_choice)
 {
-    if (p->m <= 16 || (kernel_choice != OPSNN_WQ_KERNEL_DECODE && kernel_choice != OPSNN_WQ_KERNEL_PREFILL)) return false;
+    int64_t min_m = 17;
+    if (const char* e = env("OPSNN_WQ_MIXED_MIN_M")) min_m = atoi(e);
+    if (p->m < min_m || (kernel_choice != OPSNN_WQ_KERNEL_DECODE && kernel_choice != OPSNN_WQ_KERNEL_PREFILL)) return false;
     if (kernel_choice == OPSNN_WQ_KERNEL_PREFILL && (p->prep_w != nullptr || p->k * p->n <= ((int64_t)1 << 22))) return false;
     int64_t max_m = 1024;
     if (const char* e = env("OPSNN_WQ_MIXED_MAX_M")) max_m = atoi(e);

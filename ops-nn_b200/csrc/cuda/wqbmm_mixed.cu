@@ -42,6 +42,7 @@ struct MixArgs {
     int32_t m, t_tiles, rows;  // rows: rows of x per tile (N of the MMA)
     uint32_t n, k, kb;         // kb: k stages per tile
     uint32_t grid, units;      // units = tiles * kb, cut into `grid` contiguous pieces; units * grid < 2^32
+    uint32_t split;            // > 0: grid = tiles * split, so that a tile is `split` whole pieces, launched as a cluster; 0: stream-k
     uint32_t stages, stage_bytes, x_off, sc_off, sc_rows;  // sc_rows: scale rows a stage needs (2: groups that end inside a stage)
     const void* scale;
     const void* offset;
@@ -140,7 +141,7 @@ struct MixCfg {
     static constexpr int kBits = kW == MixW::kInt4 ? 4 : 8;
     static constexpr int kBK = 128;
     static constexpr int kWBytes = kMixTileN * kBK * kBits / 8;
-    static constexpr int kEmptyArrivals = kMixDqWarps + 1;
+    static constexpr int kEmptyArrivals = kMixDqWarps / 2 + 1;
 };
 
 // A pair of weights, codes in the low bits of the two halves (other bits arbitrary), to the 16-bit type, exactly (int4: the caller has
@@ -293,6 +294,60 @@ __device__ __forceinline__ void mix_finish(const MixArgs& a, uint32_t acc, uint3
         }
         const uint32_t h = hc >= rows ? 1u : 0u;
         mix_store<kBf16>(a, n0 + 128u * h, tt * rows + hc - h * rows, f);
+    }
+}
+
+// A CTA's sums of its piece, from tensor memory into shared memory as [row of x][256 columns] fp32 (sixteen warps).
+__device__ __forceinline__ void mix_park(const MixArgs& a, uint32_t acc, uint32_t smem, int col, int share)
+{
+    const uint32_t rows = (uint32_t)a.rows;
+#pragma unroll 1
+    for (uint32_t hc = 16u * share; hc < 2u * rows; hc += 64u) {
+        uint32_t v[16];
+        ptx::tmem_ld16(acc + hc, v);
+        ptx::tmem_ld_wait();
+        const uint32_t h = hc >= rows ? 1u : 0u;
+        const uint32_t at = smem + (hc - h * rows) * (kMixTileN * 4u) + (128u * h + (uint32_t)col) * 4u;
+#pragma unroll
+        for (uint32_t i = 0; i < 16; ++i) asm volatile("st.shared.u32 [%0], %1;" ::"r"(at + i * (kMixTileN * 4u)), "r"(v[i]) : "memory");
+    }
+}
+
+// This CTA's slice of tile t: parked sums of the tile's `split` pieces added in piece order, + bias, stored (512 threads, 4 columns each).
+template <bool kBf16>
+__device__ __forceinline__ void mix_sum_and_store(const MixArgs& a, uint32_t smem, uint32_t t, uint32_t rank, uint32_t tid)
+{
+    const uint32_t rows = (uint32_t)a.rows, tn = t / (uint32_t)a.t_tiles, tt = t - tn * (uint32_t)a.t_tiles;
+    const uint32_t live = min(rows, (uint32_t)a.m - tt * rows), total = live * (kMixTileN / 4);
+    const uint32_t end = total * (rank + 1u) / a.split;
+    for (uint32_t i = total * rank / a.split + tid; i < end; i += kMixDqWarps * 32) {
+        const uint32_t row = i / (kMixTileN / 4), n = tn * kMixTileN + (i % (kMixTileN / 4)) * 4u;
+        if (n >= a.n) continue;
+        float4 f = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll 4
+        for (uint32_t j = 0; j < a.split; ++j) {
+            uint32_t at = smem + i * 16u;
+            float4 q;
+            if (a.split > 1u) asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(at) : "r"(smem + i * 16u), "r"(j));
+            asm volatile("ld.shared::cluster.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(q.x), "=f"(q.y), "=f"(q.z), "=f"(q.w) : "r"(at) : "memory");
+            f.x += q.x; f.y += q.y; f.z += q.z; f.w += q.w;
+        }
+        float v[4] = {f.x, f.y, f.z, f.w};
+        uint16_t o[4];
+        uint16_t* y = reinterpret_cast<uint16_t*>(a.y) + (int64_t)(tt * rows + row) * a.y_ld + n;
+        const uint32_t cols = min(4u, a.n - n);
+#pragma unroll
+        for (uint32_t c = 0; c < 4; ++c) {
+            if (a.bias != nullptr && c < cols) v[c] = __fadd_rn(v[c], load_as_float(a.bias, n + c, a.bias_dtype));
+            o[c] = kBf16 ? __bfloat16_as_ushort(__float2bfloat16_rn(v[c])) : __half_as_ushort(__float2half_rn(v[c]));
+        }
+        if (cols == 4u && (reinterpret_cast<uintptr_t>(y) & 7) == 0) {
+            *reinterpret_cast<uint2*>(y) = make_uint2((uint32_t)o[0] | ((uint32_t)o[1] << 16), (uint32_t)o[2] | ((uint32_t)o[3] << 16));
+        } else {
+#pragma unroll
+            for (uint32_t c = 0; c < 4; ++c)
+                if (c < cols) y[c] = o[c];
+        }
     }
 }
 
@@ -454,44 +509,54 @@ wqbmm_mixed_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
         }
     } else if (warp < kMixDqWarps) {
         // ======================= dequantisation =======================
+        // Eight warps take the even stages of the CTA's piece, eight the odd ones: one wait, one read of the scales and one release per
+        // 128 rows of k. A stage is two A buffers (64 rows each), so the four buffers alternate between the two groups.
         const int qd = warp & 3, h = (warp >> 2) & 1;
-        const uint32_t un = (uint32_t)warp >> 3;  // the 64-row unit of every stage that this warp serves
+        const uint32_t grp = (uint32_t)warp >> 3;
         const int g = lane >> 2;
         const uint32_t tlane = (uint32_t)(qd * 32) << 16;
         const int wcol = h * 128 + qd * 32;  // the warp's first column in the tile
-        uint32_t s = 0, par = 0, ab = un, apar = 0;
-        uint32_t t = u_begin / a.kb, kb = u_begin - t * a.kb, seg = 0;
+        uint32_t s = grp, par = 0, apar = 0;
+        if (s >= stages) { s -= stages; par ^= 1u; }
+        uint32_t t = (u_begin + grp) / a.kb, kb = u_begin + grp - t * a.kb;
         bool ok = true;
-        // (n,k) storage: the lane's own scale and offset, a stage ahead
-        uint32_t sc_next = 0, of_next = 0;
+        const bool two_rows = a.sc_rows == 2u;  // a stage's units have scale rows of their own
+        // (n,k) storage: the lane's own scales and offsets, a stage ahead
+        uint32_t sc_next[2] = {0, 0}, of_next[2] = {0, 0};
         auto fetch = [&](uint32_t tile, uint32_t stage) {
             const uint32_t n = min((tile / (uint32_t)a.t_tiles) * kMixTileN + wcol + lane, a.n - 1u);
-            const int64_t at = (int64_t)(min(stage * C::kBK + 64u * un, a.k - 1u) / a.group) * a.scale_sg + (int64_t)n * a.scale_sn;
-            sc_next = __ldg(reinterpret_cast<const uint16_t*>(a.scale) + at);
-            if (kOff) of_next = __ldg(reinterpret_cast<const uint16_t*>(a.offset) + at);
+#pragma unroll
+            for (int un = 0; un < 2; ++un) {
+                if (un == 1 && !two_rows) { sc_next[1] = sc_next[0]; of_next[1] = of_next[0]; break; }
+                const int64_t at = (int64_t)(min(stage * C::kBK + 64u * un, a.k - 1u) / a.group) * a.scale_sg + (int64_t)n * a.scale_sn;
+                sc_next[un] = __ldg(reinterpret_cast<const uint16_t*>(a.scale) + at);
+                if (kOff) of_next[un] = __ldg(reinterpret_cast<const uint16_t*>(a.offset) + at);
+            }
         };
-        if (kNK && u_begin < u_end) fetch(t, kb);
-        for (uint32_t u = u_begin; u < u_end; ++u) {
-            uint32_t sc[4], of[4];
+        if (kNK && u_begin + grp < u_end) fetch(t, kb);
+        for (uint32_t u = u_begin + grp; u < u_end; u += 2) {
+            uint32_t sc[4], of[4], sc_n[2], of_n[2];
             if (kNK) {
-                sc[0] = sc_next | (sc_next << 16);
-                of[0] = of_next | (of_next << 16);
+#pragma unroll
+                for (int un = 0; un < 2; ++un) {
+                    sc_n[un] = sc_next[un] | (sc_next[un] << 16);
+                    of_n[un] = of_next[un] | (of_next[un] << 16);
+                }
+                kb += 2;
+                while (kb >= a.kb) { kb -= a.kb; ++t; }
+                if (u + 2 < u_end) fetch(t, kb);
             }
-            if (++kb == a.kb) {
-                kb = 0;
-                if (u + 1 < u_end) { ++t; ++seg; }
-            }
-            if (kNK && u + 1 < u_end) fetch(t, kb);
             if (!mix_wait(full0 + 8u * s, par, abort_flag)) {
                 mix_report(abort_flag, (3u << 8) | 1u);
                 ok = false;
                 break;
             }
             const uint32_t base = smem0 + s * stage_bytes;
-            if (!kNK) {  // int4: columns 4g .. 4g + 3; int8: 2g, 2g + 1 of each 16
-                const uint32_t at = base + a.sc_off + (a.sc_rows == 2u ? un * (kMixTileN * 4u) : 0u) + 2u * wcol;
-                uint32_t r0, r1, o0 = 0, o1 = 0;
+            // int4: columns 4g .. 4g + 3; int8: 2g, 2g + 1 of each 16
+            auto load_scales = [&](uint32_t un) {
+                const uint32_t at = base + a.sc_off + un * (kMixTileN * 4u) + 2u * wcol;
                 const uint32_t p0 = kW == MixW::kInt4 ? at + 8u * g : at + 4u * g, p1 = kW == MixW::kInt4 ? p0 + 4u : p0 + 32u;
+                uint32_t r0, r1, o0 = 0, o1 = 0;
                 asm volatile("ld.shared.u32 %0, [%1];" : "=r"(r0) : "r"(p0) : "memory");
                 asm volatile("ld.shared.u32 %0, [%1];" : "=r"(r1) : "r"(p1) : "memory");
                 if (kOff) {
@@ -500,140 +565,170 @@ wqbmm_mixed_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
                 }
                 sc[0] = prmt(r0, r0, 0x1010); sc[1] = prmt(r0, r0, 0x3232); sc[2] = prmt(r1, r1, 0x1010); sc[3] = prmt(r1, r1, 0x3232);
                 of[0] = prmt(o0, o0, 0x1010); of[1] = prmt(o0, o0, 0x3232); of[2] = prmt(o1, o1, 0x1010); of[3] = prmt(o1, o1, 0x3232);
-            }
-            bool waited = false;
-            const uint32_t abase = tmem + kMixACol + ab * 64u + h * 32u + tlane;
-            auto need_buffer = [&]() {  // the MMAs that read this A buffer's previous contents are done
-                if (waited) return;
-                waited = true;
-                if (!mix_wait(aempty0 + 8u * ab, apar ^ 1u, abort_flag)) {
-                    mix_report(abort_flag, (3u << 8) | 2u);
-                    ok = false;
-                }
-                ptx::tc_fence_after();
             };
-            if constexpr (!kNK) {
-                const int r = lane & 7, j = lane >> 3;
-                if constexpr (kW == MixW::kInt4) {
-                    // rows of 128 bytes; matrix j of an ldmatrix = rows 8 j .. of a half of 32, the warp's 16 bytes of the row
-                    const uint32_t at = base + un * (64u * 128u) + (uint32_t)(8 * j + r) * 128u + (uint32_t)(((h * 4 + qd) ^ r) << 4);
-                    uint32_t w[2][4];
-                    mix_ldsm4_trans(at, w[0]);
-                    mix_ldsm4_trans(at + 32 * 128, w[1]);
+            if (!kNK) load_scales(0);
+            const int r = lane & 7, j = lane >> 3;
+            // (k,n) int4: rows of 128 bytes; matrix j of an ldmatrix = rows 8 j .. of a half of 32, the warp's 16 bytes of the row
+            uint32_t w4[4][4];
+            if constexpr (!kNK && kW == MixW::kInt4) {
+                const uint32_t at = base + (uint32_t)(8 * j + r) * 128u + (uint32_t)(((h * 4 + qd) ^ r) << 4);
 #pragma unroll
-                    for (int half = 0; half < 2; ++half) {
-                        uint32_t o[2][8];
+                for (int i = 0; i < 4; ++i) mix_ldsm4_trans(at + i * 32 * 128, w4[i]);
+                if (!two_rows) {  // the packed words and the scale rows of this stage are in registers
+                    __syncwarp();
+                    if (lane == 0) mix_arrive(empty0 + 8u * s);
+                }
+            }
 #pragma unroll
-                        for (int i = 0; i < 4; ++i)
-#pragma unroll
-                            for (int b = 0; b < 4; ++b)
-                                o[b >> 1][2 * i + (b & 1)] = mix_scale<kBf16, kOff>(mix_exact<kW, kBf16>(w[half][i] >> (4 * b)), sc[b], of[b]);
-                        need_buffer();
-                        tmem_st_16x128b_x4(abase + half * 16, o[0]);
-                        tmem_st_16x128b_x4(abase + half * 16 + (16u << 16), o[1]);
+            for (int un = 0; un < 2; ++un) {
+                const uint32_t ab = 2u * grp + un;
+                if (kNK) {
+                    sc[0] = sc_n[un];
+                    of[0] = of_n[un];
+                } else if (un == 1 && two_rows) {
+                    load_scales(1);
+                }
+                bool waited = false;
+                const uint32_t abase = tmem + kMixACol + ab * 64u + h * 32u + tlane;
+                auto need_buffer = [&]() {  // the MMAs that read this A buffer's previous contents are done
+                    if (waited) return;
+                    waited = true;
+                    if (!mix_wait(aempty0 + 8u * ab, apar ^ 1u, abort_flag)) {
+                        mix_report(abort_flag, (3u << 8) | 2u);
+                        ok = false;
                     }
-                } else {
-                    const uint32_t box = base + h * (C::kWBytes / 2) + un * (64u * 128u) + (uint32_t)(8 * j + r) * 128u;
+                    ptx::tc_fence_after();
+                };
+                if constexpr (!kNK) {
+                    if constexpr (kW == MixW::kInt4) {
 #pragma unroll
-                    for (int half = 0; half < 2; ++half) {
-#pragma unroll
-                        for (int cc = 0; cc < 2; ++cc) {
-                            uint32_t w[4], o[8];
-                            mix_ldsm4_trans(box + half * 32 * 128 + (uint32_t)(((2 * qd + cc) ^ r) << 4), w);
+                        for (int half = 0; half < 2; ++half) {
+                            uint32_t o[2][8];
 #pragma unroll
                             for (int i = 0; i < 4; ++i)
 #pragma unroll
-                                for (int b = 0; b < 2; ++b)
-                                    o[2 * i + b] = mix_scale<kBf16, kOff>(mix_exact<kW, kBf16>(w[i] >> (8 * b)), sc[2 * cc + b], of[2 * cc + b]);
+                                for (int b = 0; b < 4; ++b)
+                                    o[b >> 1][2 * i + (b & 1)] = mix_scale<kBf16, kOff>(mix_exact<kW, kBf16>(w4[2 * un + half][i] >> (4 * b)), sc[b], of[b]);
+                            need_buffer();
+                            tmem_st_16x128b_x4(abase + half * 16, o[0]);
+                            tmem_st_16x128b_x4(abase + half * 16 + (16u << 16), o[1]);
+                        }
+                    } else {
+                        const uint32_t box = base + h * (C::kWBytes / 2) + un * (64u * 128u) + (uint32_t)(8 * j + r) * 128u;
+#pragma unroll
+                        for (int half = 0; half < 2; ++half) {
+#pragma unroll
+                            for (int cc = 0; cc < 2; ++cc) {
+                                uint32_t w[4], o[8];
+                                mix_ldsm4_trans(box + half * 32 * 128 + (uint32_t)(((2 * qd + cc) ^ r) << 4), w);
+#pragma unroll
+                                for (int i = 0; i < 4; ++i)
+#pragma unroll
+                                    for (int b = 0; b < 2; ++b)
+                                        o[2 * i + b] = mix_scale<kBf16, kOff>(mix_exact<kW, kBf16>(w[i] >> (8 * b)), sc[2 * cc + b], of[2 * cc + b]);
+                                if (kW == MixW::kE4m3) {
+                                    const uint32_t any = has_nan8(w[0]) | has_nan8(w[1]) | has_nan8(w[2]) | has_nan8(w[3]);
+                                    if (any != 0u) {
+#pragma unroll
+                                        for (int i = 0; i < 4; ++i) {
+                                            o[2 * i] = fix_nan(o[2 * i], w[i]);
+                                            o[2 * i + 1] = fix_nan(o[2 * i + 1], w[i] >> 8);
+                                        }
+                                    }
+                                    __syncwarp();
+                                }
+                                need_buffer();
+                                tmem_st_16x128b_x4(abase + half * 16 + ((uint32_t)(16 * cc) << 16), o);
+                            }
+                        }
+                    }
+                } else {
+                    const int row = wcol + lane;
+                    if constexpr (kW == MixW::kInt4) {
+                        const uint32_t rb = base + (uint32_t)row * 64u;
+                        const uint32_t x = (uint32_t)(row >> 1) & 3u;  // 64-byte swizzle
+#pragma unroll
+                        for (int c = 0; c < 2; ++c) {
+                            const uint4 v = mix_lds128(rb + (((2u * un + c) ^ x) << 4));
+                            const uint32_t w[4] = {v.x, v.y, v.z, v.w};
+#pragma unroll
+                            for (int hh = 0; hh < 2; ++hh) {
+                                uint32_t o[8];
+#pragma unroll
+                                for (int i = 0; i < 2; ++i) {
+                                    const uint32_t lo = w[2 * hh + i], hi = lo >> 4;
+#pragma unroll
+                                    for (int b = 0; b < 4; ++b)  // nibbles 2 b and 2 b + 1: byte b of the word and of the word shifted by four
+                                        o[4 * i + b] = mix_scale<kBf16, kOff>(mix_exact<kW, kBf16>(prmt(lo, hi, (uint32_t)(b | ((4 + b) << 8)))), sc[0], of[0]);
+                                }
+                                need_buffer();
+                                tmem_st_32x32b_x8(abase + c * 16 + hh * 8, o);
+                            }
+                        }
+                    } else {
+                        const uint32_t rb = base + (uint32_t)row * 128u;
+                        const uint32_t x = (uint32_t)row & 7u;  // 128-byte swizzle
+#pragma unroll
+                        for (int c = 0; c < 4; ++c) {
+                            const uint4 v = mix_lds128(rb + (((4u * un + c) ^ x) << 4));
+                            const uint32_t w[4] = {v.x, v.y, v.z, v.w};
+                            uint32_t o[8];
+#pragma unroll
+                            for (int i = 0; i < 4; ++i) {
+                                o[2 * i] = mix_scale<kBf16, kOff>(mix_exact<kW, kBf16>(prmt(w[i], 0u, 0x4140)), sc[0], of[0]);
+                                o[2 * i + 1] = mix_scale<kBf16, kOff>(mix_exact<kW, kBf16>(prmt(w[i], 0u, 0x4342)), sc[0], of[0]);
+                            }
                             if (kW == MixW::kE4m3) {
                                 const uint32_t any = has_nan8(w[0]) | has_nan8(w[1]) | has_nan8(w[2]) | has_nan8(w[3]);
                                 if (any != 0u) {
 #pragma unroll
                                     for (int i = 0; i < 4; ++i) {
-                                        o[2 * i] = fix_nan(o[2 * i], w[i]);
-                                        o[2 * i + 1] = fix_nan(o[2 * i + 1], w[i] >> 8);
+                                        o[2 * i] = fix_nan(o[2 * i], prmt(w[i], 0u, 0x4140));
+                                        o[2 * i + 1] = fix_nan(o[2 * i + 1], prmt(w[i], 0u, 0x4342));
                                     }
                                 }
                                 __syncwarp();
                             }
                             need_buffer();
-                            tmem_st_16x128b_x4(abase + half * 16 + ((uint32_t)(16 * cc) << 16), o);
+                            tmem_st_32x32b_x8(abase + c * 8, o);
                         }
                     }
                 }
-            } else {
-                const int row = wcol + lane;
-                if constexpr (kW == MixW::kInt4) {
-                    const uint32_t rb = base + (uint32_t)row * 64u;
-                    const uint32_t x = (uint32_t)(row >> 1) & 3u;  // 64-byte swizzle
-#pragma unroll
-                    for (int c = 0; c < 2; ++c) {
-                        const uint4 v = mix_lds128(rb + (((2u * un + c) ^ x) << 4));
-                        const uint32_t w[4] = {v.x, v.y, v.z, v.w};
-#pragma unroll
-                        for (int hh = 0; hh < 2; ++hh) {
-                            uint32_t o[8];
-#pragma unroll
-                            for (int i = 0; i < 2; ++i) {
-                                const uint32_t lo = w[2 * hh + i], hi = lo >> 4;
-#pragma unroll
-                                for (int b = 0; b < 4; ++b)  // nibbles 2 b and 2 b + 1: byte b of the word and of the word shifted by four
-                                    o[4 * i + b] = mix_scale<kBf16, kOff>(mix_exact<kW, kBf16>(prmt(lo, hi, (uint32_t)(b | ((4 + b) << 8)))), sc[0], of[0]);
-                            }
-                            need_buffer();
-                            tmem_st_32x32b_x8(abase + c * 16 + hh * 8, o);
-                        }
-                    }
-                } else {
-                    const uint32_t rb = base + (uint32_t)row * 128u;
-                    const uint32_t x = (uint32_t)row & 7u;  // 128-byte swizzle
-#pragma unroll
-                    for (int c = 0; c < 4; ++c) {
-                        const uint4 v = mix_lds128(rb + (((4u * un + c) ^ x) << 4));
-                        const uint32_t w[4] = {v.x, v.y, v.z, v.w};
-                        uint32_t o[8];
-#pragma unroll
-                        for (int i = 0; i < 4; ++i) {
-                            o[2 * i] = mix_scale<kBf16, kOff>(mix_exact<kW, kBf16>(prmt(w[i], 0u, 0x4140)), sc[0], of[0]);
-                            o[2 * i + 1] = mix_scale<kBf16, kOff>(mix_exact<kW, kBf16>(prmt(w[i], 0u, 0x4342)), sc[0], of[0]);
-                        }
-                        if (kW == MixW::kE4m3) {
-                            const uint32_t any = has_nan8(w[0]) | has_nan8(w[1]) | has_nan8(w[2]) | has_nan8(w[3]);
-                            if (any != 0u) {
-#pragma unroll
-                                for (int i = 0; i < 4; ++i) {
-                                    o[2 * i] = fix_nan(o[2 * i], prmt(w[i], 0u, 0x4140));
-                                    o[2 * i + 1] = fix_nan(o[2 * i + 1], prmt(w[i], 0u, 0x4342));
-                                }
-                            }
-                            __syncwarp();
-                        }
-                        need_buffer();
-                        tmem_st_32x32b_x8(abase + c * 8, o);
-                    }
-                }
+                if (!ok) break;
+                tmem_st_wait();
+                ptx::tc_fence_before();
+                __syncwarp();
+                if (lane == 0) mix_arrive(afull0 + 8u * ab);
             }
             if (!ok) break;
-            __syncwarp();
-            if (lane == 0) mix_arrive(empty0 + 8u * s);  // the packed words (and scale rows) of this stage are in registers
-            tmem_st_wait();
-            ptx::tc_fence_before();
-            __syncwarp();
-            if (lane == 0) mix_arrive(afull0 + 8u * ab);
-            ab += 2u;
-            if (ab >= kMixABufs) { ab -= kMixABufs; apar ^= 1u; }
-            if (++s == stages) { s = 0; par ^= 1u; }
+            if (kNK || kW != MixW::kInt4 || two_rows) {
+                if (lane == 0) mix_arrive(empty0 + 8u * s);  // (every lane's reads lie before the __syncwarp above)
+            }
+            apar ^= 1u;
+            s += 2u;
+            if (s >= stages) { s -= stages; par ^= 1u; }
         }
-        // the CTA's last piece: nothing is left to dequantise, all sixteen warps finish it
-        const uint32_t dbuf = two_d ? (seg & 1u) : 0u;
+        // the CTA's last (often only) piece: nothing is left to dequantise, all sixteen warps finish it
+        const uint32_t t_first = u_begin / a.kb, t_last = (u_end - 1u) / a.kb;
+        const uint32_t dbuf = two_d ? ((t_last - t_first) & 1u) : 0u;
         if (ok && !mix_wait(fin0, 0u, abort_flag)) {
             mix_report(abort_flag, (3u << 8) | 3u);
             ok = false;
         }
         if (mix_all_ok<2, kMixDqWarps * 32>(ok)) {
             ptx::tc_fence_after();
-            mix_finish<kBf16, 16>(a, tmem + tlane + dbuf * d_set, t, min(u_end - t * a.kb, u_end - u_begin), qd * 32 + mix_col_of_lane<kW, kNK>(lane), qd,
-                                  lane, warp >> 2, threadIdx.x == 0, &s_last[1], abort_flag);
+            const uint32_t acc = tmem + tlane + dbuf * d_set;
+            const int col = qd * 32 + mix_col_of_lane<kW, kNK>(lane);
+            if (a.split != 0) {
+                mix_park(a, acc, smem0, col, warp >> 2);
+                if (a.split == 1) {
+                    asm volatile("bar.sync 2, 512;" ::: "memory");
+                    mix_sum_and_store<kBf16>(a, smem0, t_last, 0u, threadIdx.x);
+                }
+            } else {
+                mix_finish<kBf16, 16>(a, acc, t_last, min(u_end - t_last * a.kb, u_end - u_begin), col, qd, lane, warp >> 2, threadIdx.x == 0, &s_last[1],
+                                      abort_flag);
+            }
         }
     } else {
         // ======================= epilogue of all but the last piece, beside the main loop =======================
@@ -657,6 +752,22 @@ wqbmm_mixed_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
             kb = 0;
             ++t;
         }
+    }
+    if (a.split > 1u) {
+        // The tile's pieces ran as one thread-block cluster: every CTA sums a slice of the tile over the cluster's shared memory. A CTA that
+        // gave up a wait still joins both barriers; then nobody writes.
+        ptx::cluster_sync();
+        if (warp < kMixDqWarps) {
+            const uint32_t rank = ptx::cluster_ctarank();
+            uint32_t bad = 0u;
+            if ((uint32_t)lane < a.split) {
+                uint32_t remote;
+                asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(remote) : "r"(ptx::smem_u32(const_cast<uint32_t*>(&s_abort))), "r"((uint32_t)lane));
+                asm volatile("ld.shared::cluster.u32 %0, [%1];" : "=r"(bad) : "r"(remote) : "memory");
+            }
+            if (!__any_sync(0xffffffffu, bad != 0u)) mix_sum_and_store<kBf16>(a, smem0, blockIdx.x / a.split, rank, threadIdx.x);
+        }
+        ptx::cluster_sync();
     }
     // ---- teardown: everyone meets here, also after an aborted wait; then the allocating warp frees TMEM ----
     if (*abort_flag != 0u) __nanosleep(200000);  // lets bulk copies that are still in flight land before the CTA leaves
@@ -695,11 +806,16 @@ bool mix_map(CUtensorMap* map, const void* base, uint64_t inner_bytes, uint64_t 
 }
 
 struct MixPlan {
-    int t_tiles, rows;
+    int t_tiles, rows, split;
     int64_t n_tiles, kb, grid, units, tiles;
 };
 
-MixPlan mix_plan(const OpsnnWqbmmParams* p, int sms)
+// How the (tile, k stage) line is cut. Either every tile into `split` equal pieces, one CTA each, launched as a cluster and summed over
+// distributed shared memory; or stream-k, all SMs the same share, the tiles that straddle pieces summed through workspace. The first ends
+// sooner for the same number of stages per CTA, so stream-k has to save stages to win. `clusters(split)` is how many clusters of that
+// size the device keeps resident.
+template <typename F>
+MixPlan mix_plan(const OpsnnWqbmmParams* p, int sms, F&& clusters)
 {
     MixPlan q;
     q.t_tiles = (int)((p->m + kMixMaxRows - 1) / kMixMaxRows);
@@ -710,41 +826,65 @@ MixPlan mix_plan(const OpsnnWqbmmParams* p, int sms)
     q.kb = (p->k + 127) / 128;
     q.tiles = q.n_tiles * q.t_tiles;
     q.units = q.tiles * q.kb;
-    int64_t least = 4;  // stages a CTA should at least see: a shorter piece is mostly ramp and combination
-    if (const char* e = env("OPSNN_WQ_MIXED_LEAST")) least = atoi(e) > 0 ? atoi(e) : least;
-    q.grid = q.units / least;
+    q.split = 0;
+    q.grid = q.units / 4;  // stages a CTA should at least see: a shorter piece is mostly ramp and combination
     if (q.grid > sms) q.grid = sms;
     if (q.grid < 1) q.grid = 1;
+    int64_t stream_extra = 6 + q.rows / 4;
+    if (const char* e = env("OPSNN_WQ_MIXED_STREAM")) stream_extra = atoi(e);
+    int64_t best = (q.units + q.grid - 1) / q.grid + stream_extra;
+    int64_t most = sms / q.tiles;
+    if (most > 16) most = 16;
+    if (most > q.kb) most = q.kb;
+    for (int s = (int)most; s >= 1; --s) {
+        const int64_t cost = (q.kb + s - 1) / s + (s > 1 ? 3 : 0);
+        if (cost >= best || (s > 1 && (int64_t)clusters(s) < q.tiles)) continue;
+        best = cost;
+        q.split = s;
+        q.grid = q.tiles * s;
+    }
+    if (const char* e = env("OPSNN_WQ_MIXED_SPLIT")) {  // experiments
+        const int v = atoi(e);
+        if (v >= 1 && v <= most) { q.split = v; q.grid = q.tiles * v; }
+    }
     return q;
 }
 
-template <MixW kW, bool kNK, bool kBf16, bool kOff>
-int32_t mix_launch(const CUtensorMap& mw, const CUtensorMap& mx, const MixArgs& a, size_t smem, cudaStream_t stream)
-{
-    auto kern = wqbmm_mixed_kernel<kW, kNK, kBf16, kOff>;
-    static std::atomic<uint64_t> configured{0};
-    if (once_per_device(configured, [&] { return cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, kMixSmemMax); }) != cudaSuccess)
-        return (int32_t)cudaGetLastError();
-    cudaLaunchConfig_t cfg{};
-    cfg.gridDim = dim3(a.grid, 1, 1);
-    cfg.blockDim = dim3(kMixThreads, 1, 1);
-    cfg.dynamicSmemBytes = smem;
-    cfg.stream = stream;
-    cudaLaunchAttribute attr[1]{};
-    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attr[0].val.programmaticStreamSerializationAllowed = 1;
-    cfg.attrs = attr;
-    cfg.numAttrs = 1;
-    return (int32_t)cudaLaunchKernelEx(&cfg, kern, mw, mx, a);
-}
-
+using MixKernel = void (*)(const CUtensorMap, const CUtensorMap, const MixArgs);
 template <MixW kW, bool kNK>
-int32_t mix_dispatch(bool bf16, bool off, const CUtensorMap& mw, const CUtensorMap& mx, const MixArgs& a, size_t smem, cudaStream_t stream)
+MixKernel mix_kernel_of(bool bf16, bool off)
 {
     if constexpr (kW != MixW::kE4m3) {
-        if (off) return bf16 ? mix_launch<kW, kNK, true, true>(mw, mx, a, smem, stream) : mix_launch<kW, kNK, false, true>(mw, mx, a, smem, stream);
+        if (off) return bf16 ? &wqbmm_mixed_kernel<kW, kNK, true, true> : &wqbmm_mixed_kernel<kW, kNK, false, true>;
     }
-    return bf16 ? mix_launch<kW, kNK, true, false>(mw, mx, a, smem, stream) : mix_launch<kW, kNK, false, false>(mw, mx, a, smem, stream);
+    return bf16 ? &wqbmm_mixed_kernel<kW, kNK, true, false> : &wqbmm_mixed_kernel<kW, kNK, false, false>;
+}
+MixKernel mix_kernel(const OpsnnWqbmmParams* p, int* index)
+{
+    const bool bf16 = p->x_dtype == ACL_BF16, off = p->offset != nullptr, nk = p->trans_w != 0;
+    const int w = p->w_dtype == ACL_INT4 ? 0 : (p->w_dtype == ACL_INT8 ? 1 : 2);
+    *index = w * 8 + (nk ? 4 : 0) + (bf16 ? 2 : 0) + (off ? 1 : 0);
+    switch (w) {
+        case 0: return nk ? mix_kernel_of<MixW::kInt4, true>(bf16, off) : mix_kernel_of<MixW::kInt4, false>(bf16, off);
+        case 1: return nk ? mix_kernel_of<MixW::kInt8, true>(bf16, off) : mix_kernel_of<MixW::kInt8, false>(bf16, off);
+        default: return nk ? mix_kernel_of<MixW::kE4m3, true>(bf16, off) : mix_kernel_of<MixW::kE4m3, false>(bf16, off);
+    }
+}
+
+// The kernel of a call, ready to launch on the current device, and its plan.
+cudaError_t mix_prepare(const OpsnnWqbmmParams* p, MixKernel* kern, MixPlan* plan)
+{
+    static std::atomic<uint64_t> configured[24];
+    int index = 0;
+    const MixKernel k = mix_kernel(p, &index);
+    const cudaError_t rc = once_per_device(configured[index], [&] {
+        cudaFuncSetAttribute(k, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
+        return cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, kMixSmemMax);
+    });
+    if (rc != cudaSuccess) return rc;
+    *kern = k;
+    *plan = mix_plan(p, current_sm_count(), [&](int s) { return max_active_clusters(reinterpret_cast<const void*>(k), kMixThreads, kMixSmemMax, s, 0); });
+    return cudaSuccess;
 }
 
 }  // namespace
@@ -776,16 +916,26 @@ bool wqbmm_mixed_eligible(const OpsnnWqbmmParams* p)
 
 uint64_t wqbmm_mixed_workspace_size(const OpsnnWqbmmParams* p)
 {
-    const MixPlan q = mix_plan(p, current_sm_count());
+    // without a device (planning only) the stream-k form's need, which covers the other's
+    MixKernel kern;
+    MixPlan q;
+    int n = 0;
+    if (cudaGetDeviceCount(&n) != cudaSuccess || n == 0 || mix_prepare(p, &kern, &q) != cudaSuccess) {
+        cudaGetLastError();
+        q = mix_plan(p, 148, [](int) { return 0; });
+    }
+    if (q.split != 0) return 0;
     const uint64_t counters = ((uint64_t)q.tiles * 8u + 255u) & ~(uint64_t)255u;
     return 256u + counters + 2u * (uint64_t)q.grid * (uint64_t)q.rows * kMixTileN * 4u;
 }
 
 int32_t wqbmm_mixed_launch(const OpsnnWqbmmParams* p, cudaStream_t stream)
 {
-    const MixPlan q = mix_plan(p, current_sm_count());
-    if (p->workspace == nullptr || p->workspace_size < wqbmm_mixed_workspace_size(p)) return (int32_t)cudaErrorInvalidValue;
-    const bool nk = p->trans_w != 0, bf16 = p->x_dtype == ACL_BF16, off = p->offset != nullptr;
+    MixKernel kern;
+    MixPlan q;
+    if (const cudaError_t rc = mix_prepare(p, &kern, &q); rc != cudaSuccess) return (int32_t)rc;
+    if (q.split == 0 && (p->workspace == nullptr || p->workspace_size < wqbmm_mixed_workspace_size(p))) return (int32_t)cudaErrorInvalidValue;
+    const bool nk = p->trans_w != 0, bf16 = p->x_dtype == ACL_BF16;
     const int bits = p->w_dtype == ACL_INT4 ? 4 : 8;
     MixArgs a{};
     a.m = (int32_t)p->m;
@@ -796,6 +946,7 @@ int32_t wqbmm_mixed_launch(const OpsnnWqbmmParams* p, cudaStream_t stream)
     a.kb = (uint32_t)q.kb;
     a.units = (uint32_t)q.units;
     a.grid = (uint32_t)q.grid;
+    a.split = (uint32_t)q.split;
     a.group = p->group_size > 0 ? (uint32_t)p->group_size : 0x7FFFFFFFu;
     a.sc_rows = p->group_size % 128 == 0 ? 1 : 2;
     a.x_off = kMixTileN * 128 * bits / 8;
@@ -813,9 +964,11 @@ int32_t wqbmm_mixed_launch(const OpsnnWqbmmParams* p, cudaStream_t stream)
     a.bias_dtype = p->bias_dtype;
     a.y = p->y;
     a.y_ld = p->y_ld;
-    uint8_t* ws = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(p->workspace) + 255) & ~(uintptr_t)255);
-    a.count = reinterpret_cast<unsigned long long*>(ws);
-    a.part = reinterpret_cast<float4*>(ws + (((uint64_t)q.tiles * 8u + 255u) & ~(uint64_t)255u));
+    if (q.split == 0) {
+        uint8_t* ws = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(p->workspace) + 255) & ~(uintptr_t)255);
+        a.count = reinterpret_cast<unsigned long long*>(ws);
+        a.part = reinterpret_cast<float4*>(ws + (((uint64_t)q.tiles * 8u + 255u) & ~(uint64_t)255u));
+    }
     a.nonce = next_nonce() & 0x00FFFFFFFFFFFFFFull;
     const uint32_t f = bf16 ? 1u : 0u;
     a.idesc = make_idesc(1u, f, f, 0u, 0u, 128u, (uint32_t)q.rows);
@@ -825,10 +978,21 @@ int32_t wqbmm_mixed_launch(const OpsnnWqbmmParams* p, cudaStream_t stream)
                                 // a tile is 128 bytes of an int4 row: fetching 256 for it reads the neighbour's half twice (4.2 -> 5.5 TB/s)
                                 bits == 4 ? CU_TENSOR_MAP_L2_PROMOTION_L2_128B : CU_TENSOR_MAP_L2_PROMOTION_L2_256B);
     if (!ok || !mix_map(&mx, p->x, (uint64_t)p->k * 2, (uint64_t)p->m, (uint64_t)p->x_ld * 2, 128u, (uint32_t)q.rows)) return (int32_t)cudaErrorInvalidValue;
-    int32_t rc;
-    if (p->w_dtype == ACL_INT4) rc = nk ? mix_dispatch<MixW::kInt4, true>(bf16, off, mw, mx, a, smem, stream) : mix_dispatch<MixW::kInt4, false>(bf16, off, mw, mx, a, smem, stream);
-    else if (p->w_dtype == ACL_INT8) rc = nk ? mix_dispatch<MixW::kInt8, true>(bf16, off, mw, mx, a, smem, stream) : mix_dispatch<MixW::kInt8, false>(bf16, off, mw, mx, a, smem, stream);
-    else rc = nk ? mix_dispatch<MixW::kE4m3, true>(bf16, off, mw, mx, a, smem, stream) : mix_dispatch<MixW::kE4m3, false>(bf16, off, mw, mx, a, smem, stream);
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3(a.grid, 1, 1);
+    cfg.blockDim = dim3(kMixThreads, 1, 1);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = stream;
+    cudaLaunchAttribute attr[2]{};
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    attr[1].id = cudaLaunchAttributeClusterDimension;
+    attr[1].val.clusterDim.x = a.split;
+    attr[1].val.clusterDim.y = 1;
+    attr[1].val.clusterDim.z = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = a.split > 1u ? 2 : 1;
+    const int32_t rc = (int32_t)cudaLaunchKernelEx(&cfg, kern, mw, mx, a);
     note_launch(p->w_dtype == ACL_INT4 ? "wqbmm_decode" : "wqbmm_decode8");
     return rc;
 }
