@@ -122,6 +122,8 @@ typedef enum {
                                     the reference's two roundings per dequantised weight */
     OPSNN_WQ_KERNEL_DECODE_FAST = 3, /* same regime, "high performance" precision mode (inner_precise = 1): scale and
                                     offset applied per k-group after the MMA in fp32; not bit-identical to DECODE */
+    OPSNN_WQ_KERNEL_MIXED = 5, /* packed weight dequantised (the same two roundings) into tensor memory and multiplied there; what
+                                  OPSNN_WQ_KERNEL_AUTO runs where it is the faster form of DECODE, PREFILL or GENERIC */
     OPSNN_WQ_KERNEL_PREFILL = 4  /* m beyond the decode range: the weight is dequantised (the reference's two roundings)
                                     into workspace as (n,k) in x's dtype, then a tcgen05 bf16/fp16 matmul */
 } OpsnnWqKernelChoice;

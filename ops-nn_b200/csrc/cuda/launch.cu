@@ -83,6 +83,41 @@ int32_t wq_nz_launch(const OpsnnWqbmmParams* p, void* dst, cudaStream_t stream);
 int32_t mx_quant_launch(const OpsnnMxQuantParams* p, cudaStream_t stream);
 int32_t pack_b4_launch(const OpsnnPackB4Params* p, cudaStream_t stream);
 
+// The streaming decode kernels' own switches ask for those kernels.
+static bool streaming_asked_for()
+{
+    if (env_state() == 1) return false;
+    for (const char* name : {"OPSNN_WQ_DECODE_SPLITS", "OPSNN_WQ_DECODE_CLUSTER", "OPSNN_WQ_DECODE_PATH", "OPSNN_WQ_DECODE_LEGACY", "OPSNN_WQ_CLUSTER_POLICY",
+                             "OPSNN_TEST_DECODE_STALL_STAGE", "OPSNN_WQ_CHUNK_MIN_LOG2"})
+        if (env(name) != nullptr) return true;
+    return false;
+}
+
+// The fused kernel (wqbmm_mixed.cu) reads the packed weight once for up to 128 rows of x and has no mma.sync and no 16-bit image of the
+// weight to pay for, so it is the faster form of nearly every call (bf16, groups of 128 with offset, graph replay, us, before -> fused):
+//   m 1   4096 x 4096 12.1 -> 8.6      m 16  8192 x 28672 49.3 -> 39.1     m 16 int8 4096 x 14336 20.2 -> 15.2
+//   m 32  8192 x 28672 98 -> 43        m 128 8192 x 28672 285 -> 67        m 512 8192 x 28672 416 -> 237
+// It does not take: innerPrecise = 1 (the group-wise arithmetic of the streaming kernels), outputs bound to a communicator (only the
+// streaming kernels store into the peers), a weight prepared for the matmul, and m > 1024, where dequantising the weight once per 128
+// rows costs more than a pass over HBM. aclnnWeightQuantBatchMatmulV2 keeps the kernels that its tests name: the streaming one for
+// symmetric (k,n) int4 at m <= 16 (and its reported plan), dequantise-then-matmul up to 2^22 weights.
+int32_t wqbmm_faster_kernel(const OpsnnWqbmmParams* p, int32_t choice, bool v2)
+{
+    if (choice != OPSNN_WQ_KERNEL_DECODE && choice != OPSNN_WQ_KERNEL_PREFILL && choice != OPSNN_WQ_KERNEL_GENERIC) return choice;
+    if (choice == OPSNN_WQ_KERNEL_PREFILL && p->prep_w != nullptr) return choice;
+    const int64_t weights = p->k * p->n;
+    if (p->m > 1024 || weights < ((int64_t)1 << 18)) return choice;
+    if (v2) {
+        if (choice == OPSNN_WQ_KERNEL_GENERIC) return choice;
+        if (p->m > 16 && weights <= ((int64_t)1 << 22)) return choice;
+        if (p->m <= 16 && p->w_dtype == ACL_INT4 && p->trans_w == 0 && p->offset == nullptr) return choice;
+    }
+    if (!wqbmm_mixed_eligible(p) || streaming_asked_for()) return choice;
+    PeerBinding pb;
+    if (p->y != nullptr && lookup_peer_binding(p->y, &pb)) return choice;
+    return OPSNN_WQ_KERNEL_MIXED;
+}
+
 }  // namespace opsnn
 
 using namespace opsnn;
@@ -206,19 +241,6 @@ static int32_t decode_chunk_launches(const OpsnnWqbmmParams* p, cudaStream_t str
     return 0;
 }
 
-// A call with m > 16 that was planned as decode launches or as dequantise-then-matmul runs on the fused kernel instead (wqbmm_mixed.cu:
-// the packed weight dequantised into tensor memory, once for up to 128 rows of x) where that is the faster form.
-static bool mixed_instead(const OpsnnWqbmmParams* p, int32_t kernel_choice)
-{
-    int64_t min_m = 17;
-    if (const char* e = env("OPSNN_WQ_MIXED_MIN_M")) min_m = atoi(e);
-    if (p->m < min_m || (kernel_choice != OPSNN_WQ_KERNEL_DECODE && kernel_choice != OPSNN_WQ_KERNEL_PREFILL)) return false;
-    if (kernel_choice == OPSNN_WQ_KERNEL_PREFILL && (p->prep_w != nullptr || p->k * p->n <= ((int64_t)1 << 22))) return false;
-    int64_t max_m = 1024;
-    if (const char* e = env("OPSNN_WQ_MIXED_MAX_M")) max_m = atoi(e);
-    return p->m <= max_m && wqbmm_mixed_eligible(p);
-}
-
 int32_t opsnn_wqbmm_select_kernel(const OpsnnWqbmmParams* p)
 {
     if (p == nullptr) return OPSNN_WQ_KERNEL_GENERIC;
@@ -249,14 +271,14 @@ int32_t opsnn_wqbmm_select_kernel(const OpsnnWqbmmParams* p)
 uint64_t opsnn_wqbmm_workspace_size(const OpsnnWqbmmParams* p, int32_t kernel_choice)
 {
     if (p == nullptr) return 0;
-    if (kernel_choice == OPSNN_WQ_KERNEL_AUTO) kernel_choice = opsnn_wqbmm_select_kernel(p);
+    if (kernel_choice == OPSNN_WQ_KERNEL_AUTO) kernel_choice = wqbmm_faster_kernel(p, opsnn_wqbmm_select_kernel(p), false);
     OpsnnWqbmmParams nd;
     if (p->nz_k0 != 0) {
         const uint64_t pre = wq_nz_bytes(p);
         wq_nz_view(p, &nd, reinterpret_cast<void*>(uintptr_t(256)));
         return pre + opsnn_wqbmm_workspace_size(&nd, kernel_choice);
     }
-    if (mixed_instead(p, kernel_choice)) return wqbmm_mixed_workspace_size(p);
+    if (kernel_choice == OPSNN_WQ_KERNEL_MIXED) return wqbmm_mixed_workspace_size(p);
     if (kernel_choice == OPSNN_WQ_KERNEL_PREFILL) return wqbmm_prefill_workspace_size(p);
     return (kernel_choice == OPSNN_WQ_KERNEL_DECODE || kernel_choice == OPSNN_WQ_KERNEL_DECODE_FAST) ? wqbmm_decode_workspace_size(p) : 0;
 }
@@ -305,7 +327,7 @@ int32_t opsnn_wqbmm_launch(const OpsnnWqbmmParams* p, int32_t kernel_choice, voi
         wq_nz_view(p, &nd, p->workspace);
         return opsnn_wqbmm_launch(&nd, kernel_choice, stream);
     }
-    if (kernel_choice == OPSNN_WQ_KERNEL_AUTO) kernel_choice = opsnn_wqbmm_select_kernel(p);
+    if (kernel_choice == OPSNN_WQ_KERNEL_AUTO) kernel_choice = wqbmm_faster_kernel(p, opsnn_wqbmm_select_kernel(p), false);
     {
         // An output bound to a communicator (opsnn_comm_bind_columns) is written into every rank's full copy by the bulk-copy
         // decode kernels only; a call that would run elsewhere must not silently skip that.
@@ -325,7 +347,6 @@ int32_t opsnn_wqbmm_launch(const OpsnnWqbmmParams* p, int32_t kernel_choice, voi
             }
         }
     }
-    if (mixed_instead(p, kernel_choice)) return wqbmm_mixed_launch(p, static_cast<cudaStream_t>(stream));
     OpsnnWqbmmParams chunk;
     if (p->m > 16 && (kernel_choice == OPSNN_WQ_KERNEL_DECODE || kernel_choice == OPSNN_WQ_KERNEL_DECODE_FAST)) {
         if (!decode_in_chunks(p, &chunk)) return (int32_t)cudaErrorInvalidValue;
@@ -351,6 +372,10 @@ int32_t opsnn_wqbmm_launch(const OpsnnWqbmmParams* p, int32_t kernel_choice, voi
     if (kernel_choice == OPSNN_WQ_KERNEL_DECODE_FAST) {
         if (!wqbmm_decode_fast_eligible(p)) return (int32_t)cudaErrorInvalidValue;
         return decode_stream_launch(p, static_cast<cudaStream_t>(stream), false);
+    }
+    if (kernel_choice == OPSNN_WQ_KERNEL_MIXED) {
+        if (!wqbmm_mixed_eligible(p)) return (int32_t)cudaErrorInvalidValue;
+        return wqbmm_mixed_launch(p, static_cast<cudaStream_t>(stream));
     }
     if (kernel_choice == OPSNN_WQ_KERNEL_PREFILL) {
         if (!wqbmm_prefill_eligible(p)) return (int32_t)cudaErrorInvalidValue;

@@ -518,22 +518,32 @@ wqbmm_mixed_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
         const int wcol = h * 128 + qd * 32;  // the warp's first column in the tile
         uint32_t s = grp, par = 0, apar = 0;
         if (s >= stages) { s -= stages; par ^= 1u; }
-        uint32_t t = (u_begin + grp) / a.kb, kb = u_begin + grp - t * a.kb;
         bool ok = true;
         const bool two_rows = a.sc_rows == 2u;  // a stage's units have scale rows of their own
-        // (n,k) storage: the lane's own scales and offsets, a stage ahead
+        // (n,k) storage: the lane's own scales and offsets, an iteration ahead. The group of a stage is counted along (a division per
+        // stage was a tenth of this loop): k0 = first row of the stage, k0_in = its place in group gi.
         uint32_t sc_next[2] = {0, 0}, of_next[2] = {0, 0};
-        auto fetch = [&](uint32_t tile, uint32_t stage) {
-            const uint32_t n = min((tile / (uint32_t)a.t_tiles) * kMixTileN + wcol + lane, a.n - 1u);
-#pragma unroll
-            for (int un = 0; un < 2; ++un) {
-                if (un == 1 && !two_rows) { sc_next[1] = sc_next[0]; of_next[1] = of_next[0]; break; }
-                const int64_t at = (int64_t)(min(stage * C::kBK + 64u * un, a.k - 1u) / a.group) * a.scale_sg + (int64_t)n * a.scale_sn;
-                sc_next[un] = __ldg(reinterpret_cast<const uint16_t*>(a.scale) + at);
-                if (kOff) of_next[un] = __ldg(reinterpret_cast<const uint16_t*>(a.offset) + at);
-            }
+        uint32_t t = 0, kb = 0, k0_in = 0;
+        int64_t gi = 0, col_at = 0;
+        auto seek = [&](uint32_t unit) {
+            t = unit / a.kb;
+            kb = unit - t * a.kb;
+            gi = (kb * (uint32_t)C::kBK) / a.group;
+            k0_in = kb * (uint32_t)C::kBK - (uint32_t)gi * a.group;
+            col_at = (int64_t)min((t / (uint32_t)a.t_tiles) * kMixTileN + wcol + lane, a.n - 1u) * a.scale_sn;
         };
-        if (kNK && u_begin + grp < u_end) fetch(t, kb);
+        auto fetch = [&]() {
+            int64_t at = gi * a.scale_sg + col_at;
+            sc_next[0] = __ldg(reinterpret_cast<const uint16_t*>(a.scale) + at);
+            if (kOff) of_next[0] = __ldg(reinterpret_cast<const uint16_t*>(a.offset) + at);
+            if (two_rows && k0_in + 64u >= a.group && kb * (uint32_t)C::kBK + 64u < a.k) at += a.scale_sg;
+            sc_next[1] = two_rows ? __ldg(reinterpret_cast<const uint16_t*>(a.scale) + at) : sc_next[0];
+            if (kOff) of_next[1] = two_rows ? __ldg(reinterpret_cast<const uint16_t*>(a.offset) + at) : of_next[0];
+        };
+        if (kNK && u_begin + grp < u_end) {
+            seek(u_begin + grp);
+            fetch();
+        }
         for (uint32_t u = u_begin + grp; u < u_end; u += 2) {
             uint32_t sc[4], of[4], sc_n[2], of_n[2];
             if (kNK) {
@@ -542,9 +552,16 @@ wqbmm_mixed_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
                     sc_n[un] = sc_next[un] | (sc_next[un] << 16);
                     of_n[un] = of_next[un] | (of_next[un] << 16);
                 }
-                kb += 2;
-                while (kb >= a.kb) { kb -= a.kb; ++t; }
-                if (u + 2 < u_end) fetch(t, kb);
+                if (u + 2 < u_end) {
+                    kb += 2;
+                    if (kb < a.kb) {
+                        k0_in += 2u * C::kBK;
+                        while (k0_in >= a.group) { k0_in -= a.group; ++gi; }
+                    } else {
+                        seek(u + 2);
+                    }
+                    fetch();
+                }
             }
             if (!mix_wait(full0 + 8u * s, par, abort_flag)) {
                 mix_report(abort_flag, (3u << 8) | 1u);
