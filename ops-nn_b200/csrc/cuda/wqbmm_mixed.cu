@@ -43,7 +43,7 @@ struct MixArgs {
     uint32_t n, k, kb;         // kb: k stages per tile
     uint32_t grid, units;      // units = tiles * kb, cut into `grid` contiguous pieces; units * grid < 2^32
     uint32_t split;            // > 0: grid = tiles * split, so that a tile is `split` whole pieces, launched as a cluster; 0: stream-k
-    uint32_t stages, stage_bytes, x_off, sc_off, sc_rows;  // sc_rows: scale rows a stage needs (2: groups that end inside a stage)
+    uint32_t stages, stage_bytes, x_off, sc_off, sc_rows, sc_vec;  // sc_rows: scale rows a stage needs (2: groups that end inside a stage)
     const void* scale;
     const void* offset;
     int64_t scale_sg, scale_sn;
@@ -525,14 +525,34 @@ wqbmm_mixed_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
         uint32_t sc_next[2] = {0, 0}, of_next[2] = {0, 0};
         uint32_t t = 0, kb = 0, k0_in = 0;
         int64_t gi = 0, col_at = 0;
+        // rows of scales whose groups lie side by side: eight groups in one 16-byte load (a lane's 2-byte loads each drag a sector of their
+        // own through L2, as many bytes as the weight itself)
+        const bool vec = a.sc_vec != 0;
+        uint4 sc_v = make_uint4(0, 0, 0, 0), of_v = sc_v;
+        int64_t have = -1;
+        uint32_t sel = 0;
+        auto pick = [](const uint4& v, uint32_t i) {
+            const uint32_t w = (i & 4u) ? ((i & 2u) ? v.w : v.z) : ((i & 2u) ? v.y : v.x);
+            return prmt(w, w, (i & 1u) ? 0x3232u : 0x1010u);
+        };
         auto seek = [&](uint32_t unit) {
             t = unit / a.kb;
             kb = unit - t * a.kb;
             gi = (kb * (uint32_t)C::kBK) / a.group;
             k0_in = kb * (uint32_t)C::kBK - (uint32_t)gi * a.group;
             col_at = (int64_t)min((t / (uint32_t)a.t_tiles) * kMixTileN + wcol + lane, a.n - 1u) * a.scale_sn;
+            have = -1;
         };
         auto fetch = [&]() {
+            if (vec) {
+                sel = (uint32_t)gi & 7u;
+                if ((gi >> 3) != have) {
+                    have = gi >> 3;
+                    sc_v = __ldg(reinterpret_cast<const uint4*>(reinterpret_cast<const uint16_t*>(a.scale) + col_at + 8 * have));
+                    if (kOff) of_v = __ldg(reinterpret_cast<const uint4*>(reinterpret_cast<const uint16_t*>(a.offset) + col_at + 8 * have));
+                }
+                return;
+            }
             int64_t at = gi * a.scale_sg + col_at;
             sc_next[0] = __ldg(reinterpret_cast<const uint16_t*>(a.scale) + at);
             if (kOff) of_next[0] = __ldg(reinterpret_cast<const uint16_t*>(a.offset) + at);
@@ -547,10 +567,15 @@ wqbmm_mixed_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
         for (uint32_t u = u_begin + grp; u < u_end; u += 2) {
             uint32_t sc[4], of[4], sc_n[2], of_n[2];
             if (kNK) {
+                if (vec) {
+                    sc_n[0] = sc_n[1] = pick(sc_v, sel);
+                    of_n[0] = of_n[1] = kOff ? pick(of_v, sel) : 0u;
+                } else {
 #pragma unroll
-                for (int un = 0; un < 2; ++un) {
-                    sc_n[un] = sc_next[un] | (sc_next[un] << 16);
-                    of_n[un] = of_next[un] | (of_next[un] << 16);
+                    for (int un = 0; un < 2; ++un) {
+                        sc_n[un] = sc_next[un] | (sc_next[un] << 16);
+                        of_n[un] = of_next[un] | (of_next[un] << 16);
+                    }
                 }
                 if (u + 2 < u_end) {
                     kb += 2;
@@ -966,6 +991,11 @@ int32_t wqbmm_mixed_launch(const OpsnnWqbmmParams* p, cudaStream_t stream)
     a.split = (uint32_t)q.split;
     a.group = p->group_size > 0 ? (uint32_t)p->group_size : 0x7FFFFFFFu;
     a.sc_rows = p->group_size % 128 == 0 ? 1 : 2;
+    {
+        auto al16 = [](const void* v) { return (reinterpret_cast<uintptr_t>(v) & 15) == 0; };
+        a.sc_vec = nk && a.sc_rows == 1 && p->group_size > 0 && p->scale_sg == 1 && p->scale_sn % 8 == 0 && (p->k / p->group_size) % 8 == 0 &&
+                   p->k % p->group_size == 0 && al16(p->scale) && (p->offset == nullptr || al16(p->offset));
+    }
     a.x_off = kMixTileN * 128 * bits / 8;
     a.sc_off = a.x_off + q.rows * 256;
     a.stage_bytes = a.sc_off + (nk ? 0 : 1024 * a.sc_rows);

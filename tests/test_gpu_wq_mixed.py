@@ -1,0 +1,110 @@
+"""GPU: the fused weight-only kernel (packed weight dequantised into tensor memory) against the oracle, at the sizes where its tiles,
+stages, scale rows and ways of splitting the work begin and end. It reproduces the golden's two roundings per weight
+(wqbmmv2_kernel_golden.py:199-297), so only the fp32 summation order differs: <= 1 ulp of the output dtype."""
+import ml_dtypes
+import numpy as np
+import pytest
+
+from conftest import case_seed
+from oracle import wqbmm_oracle
+
+pytestmark = pytest.mark.gpu
+
+CASES = [
+    # weight, stored (n,k), x dtype, m, k, n, group, offset, bias
+    ("int4", False, "bfloat16", 1, 1024, 256, 128, True, False),      # one tile, cut into a cluster of pieces
+    ("int4", False, "bfloat16", 17, 4096, 2080, 128, True, True),     # last tile of 32 columns
+    ("int4", False, "float16", 128, 2112, 1056, 64, False, False),    # two scale rows per stage, k half a stage past the last
+    ("int4", True, "bfloat16", 129, 1184, 1000, 0, True, True),       # two row tiles (the second one row), ragged k, per-channel
+    ("int4", True, "float16", 77, 4096, 4608, 64, True, False),       # groups that end inside a stage
+    ("int4", True, "bfloat16", 16, 3072, 2304, 128, True, False),     # 24 groups a row: eight groups per load
+    ("int4", True, "bfloat16", 33, 2944, 2304, 128, False, False),    # 23 groups a row: one at a time
+    ("int4", False, "bfloat16", 40, 512, 40960, 256, True, False),    # more tiles than SMs: equal pieces across tiles
+    ("int8", False, "float16", 300, 1088, 25600, 0, True, True),      # the same, three row tiles, one accumulator set
+    ("int8", False, "bfloat16", 16, 4224, 1040, 64, True, False),
+    ("int8", True, "bfloat16", 65, 4224, 1032, 128, True, True),
+    ("e4m3", False, "bfloat16", 20, 2048, 784, 128, False, True),
+    ("e4m3", True, "float16", 100, 1600, 776, 0, False, False),
+]
+
+
+@pytest.mark.parametrize("case", CASES, ids=[str(c) for c in CASES])
+def test_mixed_kernel_equals_oracle(aclnn, case):
+    import torch
+
+    from gpu_util import desc, out_tensor, out_to_np
+
+    kind, nk, xdt, m, k, n, group, has_off, has_bias = case
+    rng = np.random.default_rng(case_seed(case))
+    np_dt = ml_dtypes.bfloat16 if xdt == "bfloat16" else np.float16
+    x = rng.standard_normal((m, k)).astype(np.float32).astype(np_dt)
+    sshape = (-(-k // group), n) if group else (n,)
+    scale = rng.uniform(0.005, 0.02, sshape).astype(np.float32).astype(np_dt)
+    offset = rng.uniform(-1, 1, sshape).astype(np.float32).astype(np_dt) if has_off else None
+    bias = rng.uniform(-1, 1, n).astype(np.float32).astype(np_dt) if has_bias else None
+    nan_cols = []
+    if kind == "int4":
+        w = rng.integers(-8, 8, (k, n)).astype(np.int8)
+        words = wqbmm_oracle.pack_int4_words(w.T.copy() if nk else w)
+        d_w = desc(aclnn, words, strides=(1, words.shape[1]), shape=(words.shape[1], words.shape[0])) if nk else desc(aclnn, words)
+    else:
+        if kind == "int8":
+            w = rng.integers(-128, 128, (k, n)).astype(np.int8)
+        else:  # every finite code, and both NaN codes in a few columns
+            codes = rng.integers(0, 256, (k, n)).astype(np.uint8)
+            codes[(codes & 0x7F) == 0x7F] ^= 0x01
+            nan_cols = [0, 17, 300, n - 1]
+            for i, c in enumerate(nan_cols):
+                codes[(i * 997 + 3) % k, c] = 0x7F if i % 2 == 0 else 0xFF
+            w = codes.view(ml_dtypes.float8_e4m3fn)
+        d_w = desc(aclnn, w.T.copy(), strides=(1, k), shape=(k, n)) if nk else desc(aclnn, w)
+
+    def sdesc(a):
+        if a is None:
+            return None
+        return desc(aclnn, a.T.copy(), strides=(1, a.shape[0]), shape=a.shape) if nk and a.ndim == 2 else desc(aclnn, a)
+
+    with np.errstate(invalid="ignore"):
+        want = wqbmm_oracle.weight_quant_batch_matmul(x, w, scale, offset, bias, group).astype(np.float64)
+    outs = []
+    for _ in range(2):  # twice: the second call finds the workspace as the first left it
+        out = out_tensor((m, n), xdt)
+        aclnn.weight_quant_batch_matmul(desc(aclnn, x), d_w, sdesc(scale), aclnn.Tensor((m, n), xdt, out), sdesc(offset), desc(aclnn, bias), group,
+                                        inner_precise=0)
+        torch.cuda.synchronize()
+        outs.append(out_to_np(out))
+    assert aclnn.last_kernel_name() == ("wqbmm_decode" if kind == "int4" else "wqbmm_decode8"), aclnn.last_kernel_name()
+    assert np.array_equal(outs[0].view(np.uint16), outs[1].view(np.uint16))
+    got = outs[0].astype(np.float64)
+    assert np.array_equal(np.isnan(got), np.isnan(want)) and sorted(set(np.nonzero(np.isnan(want[0]))[0])) == sorted(nan_cols)
+    ok = ~np.isnan(want)
+    rms = np.sqrt(np.mean(want[ok] ** 2))
+    ulp = 2.0 ** -7 if xdt == "bfloat16" else 2.0 ** -10
+    assert np.all(np.abs(got[ok] - want[ok]) <= ulp * np.maximum(np.abs(want[ok]), 0.05 * rms) * 1.01)
+
+
+def test_mixed_kernel_replays_from_a_graph(aclnn):
+    """Pieces combined through workspace: a replayed launch finds the arrival counts as the launch before it left them."""
+    import torch
+
+    from gpu_util import DEV
+
+    m, k, n, g = 48, 4096, 28672, 128
+    gen = torch.Generator(device=DEV).manual_seed(3)
+    x = torch.randn((m, k), generator=gen, device=DEV).to(torch.bfloat16)
+    w = torch.randint(-2 ** 31, 2 ** 31 - 1, (k, n // 8), generator=gen, device=DEV, dtype=torch.int32)
+    sc = (torch.rand((k // g, n), generator=gen, device=DEV) * 0.01 + 0.005).to(torch.bfloat16)
+    y = torch.empty((m, n), dtype=torch.bfloat16, device=DEV)
+    d = [aclnn.from_torch(t) for t in (x, w, sc, y)]
+    ws = torch.empty(max(1, aclnn.weight_quant_batch_matmul(*d, None, None, g, inner_precise=0)), dtype=torch.uint8, device=DEV)
+    torch.cuda.synchronize()
+    want = y.clone()
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        for _ in range(3):
+            aclnn.weight_quant_batch_matmul(*d, None, None, g, inner_precise=0, workspace=ws)
+    for _ in range(3):
+        y.fill_(-7777.0)
+        graph.replay()
+        torch.cuda.synchronize()
+        assert torch.equal(y, want)
