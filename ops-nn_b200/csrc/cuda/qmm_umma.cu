@@ -29,6 +29,7 @@
 #include <atomic>
 #include <cstdlib>
 
+#include "cluster_query.cuh"
 #include "common.cuh"
 #include "sm100_ptx.cuh"
 
@@ -801,6 +802,15 @@ int32_t launch_bn(int bn, const CUtensorMap& ma, const CUtensorMap& mb, UmmaArgs
 #include "qmm_umma_pair.cuh"
 #include "qmm_umma_pair_pb.cuh"
 #include "qmm_mx_umma_pair.cuh"
+#include "qmm_umma_split.cuh"
+
+// Whether a call runs on the split kernel (qmm_umma_split.cuh).
+static bool split_chosen(const OpsnnQmmParams* p)
+{
+    if (!split_takes(p)) return false;
+    if (const char* e = env("OPSNN_QMM_SPLIT")) return atoi(e) != 0;
+    return !pair_worthwhile(p) && !pair_pb_worthwhile(p);
+}
 
 bool qmm_umma_eligible(const OpsnnQmmParams* p)
 {
@@ -841,6 +851,12 @@ uint64_t qmm_umma_workspace_size(const OpsnnQmmParams* p)
 {
     if (p->mode == OPSNN_QMM_MX) return qmm_mx_umma_workspace_size(p);
     if (p->mode == OPSNN_QMM_PERGROUP_ASYM) return (uint64_t)p->m * (uint64_t)((p->k + 255) / 256) * 4u + 256u;  // row sums per k-group
+    if (split_chosen(p)) {
+        SplitKernel kern;
+        SplitPlan q;
+        if (split_prepare(p, &kern, &q) == cudaSuccess) return split_workspace(q);
+        cudaGetLastError();
+    }
     return p->mode == OPSNN_QMM_PERBLOCK ? 0 : ksplit_workspace(p);
 }
 
@@ -894,6 +910,10 @@ int32_t qmm_umma_launch(const OpsnnQmmParams* p, cudaStream_t stream)
 {
     if (const int32_t bad = umma_prelaunch_check()) return bad;
     if (p->mode == OPSNN_QMM_MX) return qmm_mx_umma_launch(p, stream);
+    if (split_chosen(p)) {
+        const int32_t rc = split_launch(p, stream);
+        if (rc >= 0) return rc;
+    }
     const bool pair = pair_worthwhile(p) && p->mode == OPSNN_QMM_DEQ && p->out_dtype != ACL_INT32 && p->out_dtype != ACL_INT8;
     // per-block on CTA pairs: 256 x 128 tiles
     const bool asym = p->mode == OPSNN_QMM_PERGROUP_ASYM;
