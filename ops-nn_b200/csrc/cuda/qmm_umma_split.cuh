@@ -32,7 +32,7 @@ struct SplitArgs {
 
 constexpr int kSplitThreads = 320;
 constexpr int kSplitMaxStages = 8;
-constexpr uint32_t kSplitSmem = 226 * 1024;
+constexpr uint32_t kSplitSmem = 225 * 1024;
 constexpr uint32_t kSplitRing = 8 * 2 * 128 * 4;  // per-block: 8 warps x 2 k-blocks x 128 rows of x
 
 __device__ __forceinline__ uint32_t split_begin(const SplitArgs& a, uint32_t c) { return (uint32_t)((uint64_t)c * a.units / a.grid); }
@@ -90,53 +90,80 @@ __device__ __forceinline__ SplitTile split_tile(const SplitArgs& a, uint32_t t)
 }
 
 // This CTA's slice of a tile whose pieces lie in the cluster's shared memory as [row of x][column] raw sums: 256 threads, 4 columns each.
-template <bool kPerBlock>
-__device__ __forceinline__ void split_sum_and_store(const SplitArgs& a, uint32_t smem, const SplitTile& t, uint32_t rank, uint32_t tid)
+// `sa`: the tile's x1 scales in shared memory; `c`: those of the thread's columns (split_cols4), both fetched during the main loop.
+struct SplitCols4 {
+    SplitCol c[4];
+};
+template <bool kPerBlock, uint32_t kHalves>
+__device__ __forceinline__ SplitCols4 split_cols4(const SplitArgs& a, const SplitTile& t, uint32_t tid)
 {
-    const uint32_t vecs = 32u * a.halves, total = t.live * vecs;  // 4-column pieces in a row; 256 is a multiple of vecs
-    const uint32_t begin = (total * rank / a.split) / vecs * vecs, end = rank + 1u == a.split ? total : (total * (rank + 1u) / a.split) / vecs * vecs;
+    SplitCols4 r;
+    const uint32_t n = t.n0 + (tid % (32u * kHalves)) * 4u;
+#pragma unroll
+    for (uint32_t i = 0; i < 4; ++i) r.c[i] = split_col<kPerBlock>(a, t.b, min((int64_t)n + i, a.n - 1));
+    return r;
+}
+template <bool kPerBlock, uint32_t kHalves>
+__device__ __forceinline__ void split_sum_and_store(const SplitArgs& a, uint32_t smem, const SplitTile& t, uint32_t rank, uint32_t tid, const float* s_sa,
+                                                    const SplitCols4& cols4)
+{
+    constexpr uint32_t vecs = 32u * kHalves;  // 4-column pieces in a row; 256 is a multiple of it
+    const uint32_t total = t.live * vecs;
+    const uint32_t split = a.split;
+    const uint32_t begin = (total * rank / split) / vecs * vecs, end = rank + 1u == split ? total : (total * (rank + 1u) / split) / vecs * vecs;
     const uint32_t n = t.n0 + (tid % vecs) * 4u;
     if (n >= a.n) return;
     const uint32_t cols = (uint32_t)min((int64_t)4, a.n - n);
-    SplitCol c[4];
-#pragma unroll
-    for (uint32_t i = 0; i < 4; ++i) c[i] = split_col<kPerBlock>(a, t.b, min((int64_t)n + i, a.n - 1));
-    const int ob = out_elem_bytes(a.out_dtype);
+    const int out_dtype = a.out_dtype, ob = out_elem_bytes(out_dtype);
     uint8_t* out = reinterpret_cast<uint8_t*>(a.out) + (t.b * a.out_bs + n) * ob;
-    for (uint32_t i = begin + tid; i < end; i += 256u) {
-        const uint32_t row = i / vecs;
-        const float sa = split_sa<kPerBlock>(a, t.r0 + row);
-        uint32_t v[4] = {0u, 0u, 0u, 0u};
-#pragma unroll 4
-        for (uint32_t j = 0; j < a.split; ++j) {
-            uint32_t at = smem + i * 16u;
-            uint32_t q[4];
-            if (a.split > 1u) asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(at) : "r"(smem + i * 16u), "r"(j));
-            asm volatile("ld.shared::cluster.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(q[0]), "=r"(q[1]), "=r"(q[2]), "=r"(q[3]) : "r"(at) : "memory");
+    const int64_t pitch = a.out_ld * ob;
+    const bool is_int = a.is_int && !kPerBlock;
+    constexpr int kBatch = 4;  // rows of x in flight: what bounds this loop is the latency of the reads from the other CTAs
+    for (uint32_t i0 = begin + tid; i0 < end; i0 += 256u * kBatch) {
+        uint32_t v[kBatch][4];
+        for (uint32_t j = 0; j < split; ++j) {
+            uint32_t q[kBatch][4];
 #pragma unroll
-            for (int e = 0; e < 4; ++e)
-                v[e] = a.is_int && !kPerBlock ? v[e] + q[e] : (j == 0 ? q[e] : __float_as_uint(__fadd_rn(__uint_as_float(v[e]), __uint_as_float(q[e]))));
-        }
-        float f[4];
-#pragma unroll
-        for (int e = 0; e < 4; ++e) f[e] = split_value<kPerBlock>(a, v[e], c[e], sa);
-        uint8_t* o = out + (int64_t)(t.r0 + row) * a.out_ld * ob;
-        if (cols == 4u && a.out_dtype != ACL_FLOAT && (reinterpret_cast<uintptr_t>(o) & 7) == 0) {
-            uint2 w;
-            if (a.out_dtype == ACL_BF16) {
-                const __nv_bfloat162 lo = __floats2bfloat162_rn(f[0], f[1]), hi = __floats2bfloat162_rn(f[2], f[3]);
-                w = make_uint2(*reinterpret_cast<const uint32_t*>(&lo), *reinterpret_cast<const uint32_t*>(&hi));
-            } else {
-                const __half2 lo = __floats2half2_rn(f[0], f[1]), hi = __floats2half2_rn(f[2], f[3]);
-                w = make_uint2(*reinterpret_cast<const uint32_t*>(&lo), *reinterpret_cast<const uint32_t*>(&hi));
+            for (int r = 0; r < kBatch; ++r) {
+                const uint32_t at = smem + min(i0 + 256u * r, total - 1u) * 16u;
+                uint32_t remote = at;
+                if (split > 1u) asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(remote) : "r"(at), "r"(j));
+                asm volatile("ld.shared::cluster.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(q[r][0]), "=r"(q[r][1]), "=r"(q[r][2]), "=r"(q[r][3]) : "r"(remote));
             }
-            *reinterpret_cast<uint2*>(o) = w;
-        } else if (cols == 4u && a.out_dtype == ACL_FLOAT && (reinterpret_cast<uintptr_t>(o) & 15) == 0) {
-            *reinterpret_cast<float4*>(o) = make_float4(f[0], f[1], f[2], f[3]);
-        } else {
 #pragma unroll
-            for (uint32_t e = 0; e < 4; ++e)
-                if (e < cols) store_out(o, e, f[e], a.out_dtype);
+            for (int r = 0; r < kBatch; ++r)
+#pragma unroll
+                for (int e = 0; e < 4; ++e)
+                    v[r][e] = j == 0 ? q[r][e]
+                                     : (is_int ? v[r][e] + q[r][e] : __float_as_uint(__fadd_rn(__uint_as_float(v[r][e]), __uint_as_float(q[r][e]))));
+        }
+#pragma unroll
+        for (int r = 0; r < kBatch; ++r) {
+            const uint32_t i = i0 + 256u * r;
+            if (i >= end) break;
+            const uint32_t row = i / vecs;
+            const float sa = kPerBlock ? 1.f : s_sa[row];
+            float f[4];
+#pragma unroll
+            for (int e = 0; e < 4; ++e) f[e] = split_value<kPerBlock>(a, v[r][e], cols4.c[e], sa);
+            uint8_t* o = out + (int64_t)(t.r0 + row) * pitch;
+            if (cols == 4u && out_dtype != ACL_FLOAT && (reinterpret_cast<uintptr_t>(o) & 7) == 0) {
+                uint2 w;
+                if (out_dtype == ACL_BF16) {
+                    const __nv_bfloat162 lo = __floats2bfloat162_rn(f[0], f[1]), hi = __floats2bfloat162_rn(f[2], f[3]);
+                    w = make_uint2(*reinterpret_cast<const uint32_t*>(&lo), *reinterpret_cast<const uint32_t*>(&hi));
+                } else {
+                    const __half2 lo = __floats2half2_rn(f[0], f[1]), hi = __floats2half2_rn(f[2], f[3]);
+                    w = make_uint2(*reinterpret_cast<const uint32_t*>(&lo), *reinterpret_cast<const uint32_t*>(&hi));
+                }
+                *reinterpret_cast<uint2*>(o) = w;
+            } else if (cols == 4u && out_dtype == ACL_FLOAT && (reinterpret_cast<uintptr_t>(o) & 15) == 0) {
+                *reinterpret_cast<float4*>(o) = make_float4(f[0], f[1], f[2], f[3]);
+            } else {
+#pragma unroll
+                for (uint32_t e = 0; e < 4; ++e)
+                    if (e < cols) store_out(o, e, f[e], out_dtype);
+            }
         }
     }
 }
@@ -224,7 +251,7 @@ __device__ __forceinline__ void split_finish(const SplitArgs& a, uint32_t t, uin
 }
 
 // kAcc: sums one epilogue thread keeps in registers (per-block mode), at least the rows of x that it serves.
-template <ptx::MmaKind kKind, bool kPerBlock, int kAcc>
+template <ptx::MmaKind kKind, bool kPerBlock, int kAcc, uint32_t kHalves>
 __global__ void __launch_bounds__(kSplitThreads, 1)
 qmm_umma_split_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUtensorMap map_x, const __grid_constant__ SplitArgs a)
 {
@@ -233,6 +260,7 @@ qmm_umma_split_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_co
     __shared__ __align__(8) uint64_t s_bars[2 * kSplitMaxStages + 8];
     __shared__ uint32_t s_tmem;
     __shared__ volatile uint32_t s_abort, s_last;
+    __shared__ float s_sa[256];  // x1 scales of the tile's rows (one piece per CTA)
     const uint32_t full0 = ptx::smem_u32(s_bars), empty0 = full0 + 8u * kSplitMaxStages, tfull0 = empty0 + 8u * kSplitMaxStages, tempty0 = tfull0 + 32u;
     volatile uint32_t* abort_flag = &s_abort;
     const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0);
@@ -264,11 +292,21 @@ qmm_umma_split_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_co
     asm volatile("griddepcontrol.wait;" ::: "memory");
 
     const uint32_t u_begin = split_begin(a, blockIdx.x), u_end = split_begin(a, blockIdx.x + 1);
-    const uint32_t set = a.halves * a.rows;  // TMEM columns of one accumulator buffer
+    SplitCols4 cols4;
+    if (warp < 8 && a.split != 0u) {
+        const SplitTile tile = split_tile(a, blockIdx.x / a.split);
+        cols4 = split_cols4<kPerBlock, kHalves>(a, tile, threadIdx.x);
+        if (threadIdx.x < a.rows) s_sa[threadIdx.x] = split_sa<kPerBlock>(a, tile.r0 + min(threadIdx.x, tile.live - 1u));
+    }
+    const uint32_t set = kHalves * a.rows;  // TMEM columns of one accumulator buffer
 
     if (warp == 8) {
         // ======================= TMA producer =======================
-        uint32_t s = 0, par = 0, t = u_begin / a.kb, kb = u_begin - t * a.kb;
+        // One warp with nothing to hide latency behind: everything the loop uses is in registers (with the launch parameters read where
+        // they are used, a k-block cost this warp and the next 0.6 us each, more than its copies and its MMAs).
+        const uint32_t stages = a.stages, stage_bytes = a.stage_bytes, x_off = a.x_off, kbs = a.kb, bytes = kHalves * kATile + a.rows * BK;
+        const bool w_mn = a.w_mn != 0, w_batched = a.w_batched != 0, x_batched = a.x_batched != 0;
+        uint32_t s = 0, par = 0, t = u_begin / kbs, kb = u_begin - t * kbs;
         SplitTile tile = split_tile(a, t);
         for (uint32_t u = u_begin; u < u_end; ++u) {
             if (!ptx::mbar_wait_a(empty0 + 8u * s, par ^ 1u, abort_flag)) {
@@ -276,18 +314,19 @@ qmm_umma_split_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_co
                 break;
             }
             if (ptx::elect_one()) {
-                const uint32_t fb = full0 + 8u * s, dst = smem0 + s * a.stage_bytes;
-                const int32_t k0 = (int32_t)(kb * BK), bw = a.w_batched ? (int32_t)tile.b : 0, bx = a.x_batched ? (int32_t)tile.b : 0;
-                ptx::mbar_expect_tx_a(fb, a.halves * kATile + a.rows * BK);
-                for (uint32_t h = 0; h < a.halves; ++h) {
+                const uint32_t fb = full0 + 8u * s, dst = smem0 + s * stage_bytes;
+                const int32_t k0 = (int32_t)(kb * BK), bw = w_batched ? (int32_t)tile.b : 0, bx = x_batched ? (int32_t)tile.b : 0;
+                ptx::mbar_expect_tx_a(fb, bytes);
+#pragma unroll
+                for (uint32_t h = 0; h < kHalves; ++h) {
                     const int32_t n0 = (int32_t)(tile.n0 + 128u * h);
-                    ptx::tma_load_3d_a(dst + h * kATile, &map_w, fb, a.w_mn ? n0 : k0, a.w_mn ? k0 : n0, bw);
+                    ptx::tma_load_3d_a(dst + h * kATile, &map_w, fb, w_mn ? n0 : k0, w_mn ? k0 : n0, bw);
                 }
-                ptx::tma_load_3d_a(dst + a.x_off, &map_x, fb, k0, (int32_t)tile.r0, bx);
+                ptx::tma_load_3d_a(dst + x_off, &map_x, fb, k0, (int32_t)tile.r0, bx);
             }
             __syncwarp();
-            if (++s == a.stages) { s = 0; par ^= 1u; }
-            if (++kb == a.kb) {
+            if (++s == stages) { s = 0; par ^= 1u; }
+            if (++kb == kbs) {
                 kb = 0;
                 if (u + 1 < u_end) tile = split_tile(a, ++t);
             }
@@ -298,7 +337,8 @@ qmm_umma_split_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_co
         const uint64_t dx = ptx::make_smem_desc(smem0 + a.x_off, 0, 1024, 2);
         const uint32_t w_lo = (uint32_t)dw, x_lo = (uint32_t)dx, w_k = a.w_mn ? 256u : 2u;
         const uint64_t w_hi = dw & 0xFFFFFFFF00000000ull, x_hi = dx & 0xFFFFFFFF00000000ull;
-        uint32_t s = 0, par = 0, buf = 0, bpar = 0, kb = u_begin % a.kb;
+        const uint32_t stages = a.stages, stage16 = a.stage_bytes >> 4, rows = a.rows, idesc = a.idesc, kbs = a.kb, dbufs = a.dbufs;
+        uint32_t s = 0, par = 0, off = 0, buf = 0, bpar = 0, kb = u_begin % kbs;
         uint32_t acc = 0u;
         bool fresh = true;
         for (uint32_t u = u_begin; u < u_end; ++u) {
@@ -314,32 +354,33 @@ qmm_umma_split_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_co
                 break;
             }
             ptx::tc_fence_after();
-            const bool last = kPerBlock || kb + 1 == a.kb || u + 1 == u_end;
+            const bool last = kPerBlock || kb + 1 == kbs || u + 1 == u_end;
             if (ptx::elect_one()) {
-                const uint32_t off = (s * a.stage_bytes) >> 4, d = tmem + buf * set;
+                const uint32_t d = tmem + buf * set, wl = w_lo + off, xl = x_lo + off;
 #pragma unroll
                 for (int k = 0; k < 4; ++k)
-                    for (uint32_t h = 0; h < a.halves; ++h)
-                        ptx::umma<kKind>(d + h * a.rows, w_hi | (uint64_t)(w_lo + off + h * (kATile >> 4) + k * w_k), x_hi | (uint64_t)(x_lo + off + 2u * k),
-                                         a.idesc, k == 0 ? acc : 1u);
+#pragma unroll
+                    for (uint32_t h = 0; h < kHalves; ++h)
+                        ptx::umma<kKind>(d + h * rows, w_hi | (uint64_t)(wl + h * (kATile >> 4) + k * w_k), x_hi | (uint64_t)(xl + 2u * k), idesc,
+                                         k == 0 ? acc : 1u);
                 ptx::umma_commit_a(empty0 + 8u * s);
                 if (last) ptx::umma_commit_a(tfull0 + 8u * buf);
             }
             __syncwarp();
-            acc = kPerBlock ? 0u : 1u;
+            acc = last ? 0u : 1u;
             if (last) {
-                acc = 0u;
                 fresh = true;
-                if (++buf == a.dbufs) { buf = 0; bpar ^= 1u; }
+                if (++buf == dbufs) { buf = 0; bpar ^= 1u; }
             }
-            if (++s == a.stages) { s = 0; par ^= 1u; }
-            if (++kb == a.kb) kb = 0;
+            off += stage16;
+            if (++s == stages) { s = 0; off = 0; par ^= 1u; }
+            if (++kb == kbs) kb = 0;
         }
     } else {
         // ======================= epilogue =======================
         const uint32_t quad = warp & 3, hf = (uint32_t)warp >> 2;
-        const uint32_t cnt_rows = a.halves == 2u ? a.rows : a.rows / 2u;  // rows of x this thread serves, of its one column
-        const uint32_t col = (a.halves == 2u ? hf * 128u : 0u) + quad * 32u + lane, row0 = a.halves == 2u ? 0u : hf * cnt_rows;
+        const uint32_t cnt_rows = kHalves == 2u ? a.rows : a.rows / 2u;  // rows of x this thread serves, of its one column
+        const uint32_t col = (kHalves == 2u ? hf * 128u : 0u) + quad * 32u + lane, row0 = kHalves == 2u ? 0u : hf * cnt_rows;
         const uint32_t tbase = tmem + ((quad * 32u) << 16) + hf * cnt_rows;
         const uint32_t ring = smem0 + a.stages * a.stage_bytes + (uint32_t)warp * (2u * 128u * 4u);
         uint32_t buf = 0, bpar = 0, u = u_begin, t = u_begin / a.kb, kb = u_begin - t * a.kb;
@@ -452,7 +493,7 @@ qmm_umma_split_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_co
                 }
                 if (a.split == 1u) {
                     asm volatile("bar.sync 1, 256;" ::: "memory");
-                    split_sum_and_store<kPerBlock>(a, smem0, split_tile(a, t), 0u, threadIdx.x);
+                    split_sum_and_store<kPerBlock, kHalves>(a, smem0, split_tile(a, t), 0u, threadIdx.x, s_sa, cols4);
                 }
             } else {
                 split_finish<kPerBlock>(a, t, cnt, cnt_rows, row0, col, threadIdx.x == 0, &s_last, abort_flag, get);
@@ -479,7 +520,7 @@ qmm_umma_split_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_co
                 asm volatile("ld.shared::cluster.u32 %0, [%1];" : "=r"(bad) : "r"(remote) : "memory");
             }
             if (!__any_sync(0xffffffffu, bad != 0u))
-                split_sum_and_store<kPerBlock>(a, smem0, split_tile(a, blockIdx.x / a.split), ptx::cluster_ctarank(), threadIdx.x);
+                split_sum_and_store<kPerBlock, kHalves>(a, smem0, split_tile(a, blockIdx.x / a.split), ptx::cluster_ctarank(), threadIdx.x, s_sa, cols4);
         }
         ptx::cluster_sync();
     }
@@ -553,22 +594,35 @@ SplitPlan split_candidate(const OpsnnQmmParams* p, uint32_t halves, int sms, F&&
     if (most > 16) most = 16;
     if (most > q.kb) most = q.kb;
     for (int s = (int)most; s >= 1; --s)
-        if (s == 1 || (int64_t)clusters(s) >= q.tiles) consider(q.tiles * s, (uint32_t)s, s > 1 ? 6.0 : 3.0);
+        if (s == 1 || (int64_t)clusters(q, s) >= q.tiles) consider(q.tiles * s, (uint32_t)s, s > 1 ? 6.0 : 3.0);
     q.cost = (int64_t)(best * 16.0);
     return q;
 }
 
-template <ptx::MmaKind kKind>
+template <ptx::MmaKind kKind, uint32_t kHalves>
 SplitKernel split_kernel_of(bool per_block, int acc)
 {
     if constexpr (kKind == ptx::MmaKind::kF8F6F4) {
         if (per_block) {
-            if (acc == 32) return &qmm_umma_split_kernel<kKind, true, 32>;
-            if (acc == 64) return &qmm_umma_split_kernel<kKind, true, 64>;
-            return &qmm_umma_split_kernel<kKind, true, 128>;
+            if (acc == 32) return &qmm_umma_split_kernel<kKind, true, 32, kHalves>;
+            if (acc == 64) return &qmm_umma_split_kernel<kKind, true, 64, kHalves>;
+            return &qmm_umma_split_kernel<kKind, true, 128, kHalves>;
         }
     }
-    return &qmm_umma_split_kernel<kKind, false, 16>;
+    return &qmm_umma_split_kernel<kKind, false, 16, kHalves>;
+}
+// The kernel of a plan, ready to launch on the current device; nullptr when it cannot be made ready.
+SplitKernel split_kernel(bool i8, bool per_block, const SplitPlan& q)
+{
+    const SplitKernel k = i8 ? (q.halves == 2 ? split_kernel_of<ptx::MmaKind::kI8, 2>(per_block, q.acc) : split_kernel_of<ptx::MmaKind::kI8, 1>(per_block, q.acc))
+                             : (q.halves == 2 ? split_kernel_of<ptx::MmaKind::kF8F6F4, 2>(per_block, q.acc) : split_kernel_of<ptx::MmaKind::kF8F6F4, 1>(per_block, q.acc));
+    static std::atomic<uint64_t> configured[16];
+    const int index = (q.halves == 2 ? 8 : 0) + (i8 ? 0 : (!per_block ? 1 : (q.acc == 32 ? 2 : (q.acc == 64 ? 3 : 4))));
+    const cudaError_t rc = once_per_device(configured[index], [&] {
+        cudaFuncSetAttribute(k, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
+        return cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, kSplitSmem);
+    });
+    return rc == cudaSuccess ? k : nullptr;
 }
 
 cudaError_t split_prepare(const OpsnnQmmParams* p, SplitKernel* kern, SplitPlan* plan)
@@ -576,34 +630,23 @@ cudaError_t split_prepare(const OpsnnQmmParams* p, SplitKernel* kern, SplitPlan*
     const bool i8 = p->a_dtype == ACL_INT8, pb = p->mode == OPSNN_QMM_PERBLOCK;
     int device = -1;
     const bool have_device = cudaGetDevice(&device) == cudaSuccess;
-    auto query = [&](int acc) {
-        return [=](int s) -> int {
-            if (!have_device) return 0;
-            const SplitKernel k = i8 ? split_kernel_of<ptx::MmaKind::kI8>(pb, acc) : split_kernel_of<ptx::MmaKind::kF8F6F4>(pb, acc);
-            static std::atomic<uint64_t> configured[8];
-            const int index = i8 ? 0 : (!pb ? 1 : (acc == 32 ? 2 : (acc == 64 ? 3 : 4)));
-            if (once_per_device(configured[index], [&] {
-                    cudaFuncSetAttribute(k, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
-                    return cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, kSplitSmem);
-                }) != cudaSuccess)
-                return 0;
-            return s == 0 ? 1 : max_active_clusters(reinterpret_cast<const void*>(k), kSplitThreads, kSplitSmem, s, 0);
-        };
-    };
     const int sms = have_device ? sm_count() : 148;
-    // the accumulator count (hence the kernel) of a candidate follows from its shape alone
-    auto served = [&](uint32_t halves) {
-        SplitPlan q = split_candidate(p, halves, sms, [](int) { return 0; });
-        return q.acc;
-    };
-    const int acc2 = served(2), acc1 = served(1);
-    SplitPlan two = split_candidate(p, 2, sms, query(acc2));
-    SplitPlan one = split_candidate(p, 1, sms, query(acc1));
-    *plan = two.cost <= one.cost ? two : one;
-    if (const char* e = env("OPSNN_QMM_SPLIT_HALVES")) *plan = atoi(e) == 2 ? two : one;  // experiments
-    *kern = i8 ? split_kernel_of<ptx::MmaKind::kI8>(pb, plan->acc) : split_kernel_of<ptx::MmaKind::kF8F6F4>(pb, plan->acc);
-    if (have_device && query(plan->acc)(0) == 0) return cudaGetLastError();
-    return cudaSuccess;
+    for (uint32_t halves = 2; halves >= 1; --halves) {
+        const SplitPlan q = split_candidate(p, halves, sms, [&](const SplitPlan& c, int s) -> int {
+            const SplitKernel k = have_device ? split_kernel(i8, pb, c) : nullptr;
+            return k == nullptr ? 0 : max_active_clusters(reinterpret_cast<const void*>(k), kSplitThreads, kSplitSmem, s, 0);
+        });
+        if (halves == 2 || q.cost < plan->cost) *plan = q;
+        if (const char* e = env("OPSNN_QMM_SPLIT_HALVES"))  // experiments
+            if (atoi(e) == (int)halves) {
+                *plan = q;
+                break;
+            }
+    }
+    *kern = nullptr;
+    if (!have_device) return cudaErrorNoDevice;
+    *kern = split_kernel(i8, pb, *plan);
+    return *kern != nullptr ? cudaSuccess : cudaGetLastError();
 }
 
 uint64_t split_workspace(const SplitPlan& q)

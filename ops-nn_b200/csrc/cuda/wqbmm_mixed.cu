@@ -409,12 +409,15 @@ wqbmm_mixed_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
         // ======================= TMA producer =======================
         // Its time per stage bounds the stream: no division but one by the group size, everything else counted along.
         uint32_t s = 0, par = 0;
-        const uint32_t t0 = u_begin / a.kb;
-        uint32_t kb = u_begin - t0 * a.kb;
-        uint32_t n0 = t0 / (uint32_t)a.t_tiles, r0 = (t0 - n0 * (uint32_t)a.t_tiles) * (uint32_t)a.rows;
+        const uint32_t kbs = a.kb, rows = (uint32_t)a.rows, n_all = a.n, x_off = a.x_off, sc_off = a.sc_off, nrows_sc = a.sc_rows, k_last = a.k - 1u, group = a.group;
+        const int64_t scale_sg = a.scale_sg;
+        const uint16_t *scale = reinterpret_cast<const uint16_t*>(a.scale), *offset = reinterpret_cast<const uint16_t*>(a.offset);
+        const uint32_t t0 = u_begin / kbs;
+        uint32_t kb = u_begin - t0 * kbs;
+        uint32_t n0 = t0 / (uint32_t)a.t_tiles, r0 = (t0 - n0 * (uint32_t)a.t_tiles) * rows;
         const uint32_t r_end = (uint32_t)(a.t_tiles * a.rows);
         n0 *= kMixTileN;
-        const uint32_t sc_rows = kNK ? 0u : a.sc_rows * (kOff ? 2u : 1u);
+        const uint32_t sc_rows = kNK ? 0u : nrows_sc * (kOff ? 2u : 1u);
         for (uint32_t u = u_begin; u < u_end; ++u) {
             if (!mix_wait(empty0 + 8u * s, par ^ 1u, abort_flag)) {
                 mix_report(abort_flag, (1u << 8) | 1u);
@@ -422,7 +425,7 @@ wqbmm_mixed_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
             }
             if (ptx::elect_one()) {
                 const uint32_t k0 = kb * C::kBK, fb = full0 + 8u * s, dst = smem0 + s * stage_bytes;
-                const uint32_t sc_bytes = min((uint32_t)kMixTileN, a.n - n0) * 2u;
+                const uint32_t sc_bytes = min((uint32_t)kMixTileN, n_all - n0) * 2u;
                 ptx::mbar_expect_tx_a(fb, (uint32_t)C::kWBytes + 2u * xunit + sc_bytes * sc_rows);
                 if (kNK) {
                     mix_tma_2d(dst, &map_w, fb, (int32_t)(k0 * C::kBits / 8), (int32_t)n0);
@@ -430,23 +433,23 @@ wqbmm_mixed_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
                     mix_tma_2d(dst, &map_w, fb, (int32_t)(n0 * C::kBits / 8), (int32_t)k0);
                     if (C::kBits == 8) mix_tma_2d(dst + C::kWBytes / 2, &map_w, fb, (int32_t)n0 + 128, (int32_t)k0);
                 }
-                mix_tma_2d(dst + a.x_off, &map_x, fb, (int32_t)k0 * 2, (int32_t)r0);
-                mix_tma_2d(dst + a.x_off + xunit, &map_x, fb, (int32_t)k0 * 2 + 128, (int32_t)r0);
+                mix_tma_2d(dst + x_off, &map_x, fb, (int32_t)k0 * 2, (int32_t)r0);
+                mix_tma_2d(dst + x_off + xunit, &map_x, fb, (int32_t)k0 * 2 + 128, (int32_t)r0);
                 if (!kNK) {
-                    uint32_t sd = dst + a.sc_off;
-                    for (uint32_t i = 0; i < a.sc_rows; ++i) {
-                        const int64_t at = (int64_t)(min(k0 + 64u * i, a.k - 1u) / a.group) * a.scale_sg + n0;
-                        ptx::bulk_load_a(sd, reinterpret_cast<const uint16_t*>(a.scale) + at, sc_bytes, fb);
-                        if (kOff) ptx::bulk_load_a(sd + kMixTileN * 2, reinterpret_cast<const uint16_t*>(a.offset) + at, sc_bytes, fb);
+                    uint32_t sd = dst + sc_off;
+                    for (uint32_t i = 0; i < nrows_sc; ++i) {
+                        const int64_t at = (int64_t)(min(k0 + 64u * i, k_last) / group) * scale_sg + n0;
+                        ptx::bulk_load_a(sd, scale + at, sc_bytes, fb);
+                        if (kOff) ptx::bulk_load_a(sd + kMixTileN * 2, offset + at, sc_bytes, fb);
                         sd += kMixTileN * 4;
                     }
                 }
             }
             __syncwarp();
             if (++s == stages) { s = 0; par ^= 1u; }
-            if (++kb == a.kb) {
+            if (++kb == kbs) {
                 kb = 0;
-                r0 += (uint32_t)a.rows;
+                r0 += rows;
                 if (r0 == r_end) { r0 = 0; n0 += kMixTileN; }
             }
         }
@@ -457,9 +460,10 @@ wqbmm_mixed_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
         const uint64_t b_hi = db & 0xFFFFFFFF00000000ull;
         uint32_t s = 0, par = 0, ab = 0, apar = 0, seg = 0;
         bool ok = true;
-        uint32_t u = u_begin, kb = u_begin % a.kb;
+        const uint32_t kbs = a.kb, rows = (uint32_t)a.rows, idesc = a.idesc;
+        uint32_t u = u_begin, kb = u_begin % kbs;
         while (u < u_end && ok) {
-            const uint32_t cnt = min(a.kb - kb, u_end - u);
+            const uint32_t cnt = min(kbs - kb, u_end - u);
             const uint32_t dbuf = two_d ? (seg & 1u) : 0u, dpar = two_d ? ((seg >> 1) & 1u) : (seg & 1u);
             if (!mix_wait(dempty0 + 8u * dbuf, dpar ^ 1u, abort_flag)) {
                 mix_report(abort_flag, (2u << 8) | 1u);
@@ -488,7 +492,7 @@ wqbmm_mixed_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
                         for (int kk = 0; kk < 4; ++kk) {
 #pragma unroll
                             for (int h = 0; h < 2; ++h)
-                                umma_f16_ta(d0 + h * (uint32_t)a.rows, a0 + h * 32 + kk * 8, b_hi | (uint64_t)(bl + 2u * kk), a.idesc,
+                                umma_f16_ta(d0 + h * rows, a0 + h * 32 + kk * 8, b_hi | (uint64_t)(bl + 2u * kk), idesc,
                                             kk == 0 ? acc : 1u);
                         }
                         ptx::umma_commit_a(aempty0 + 8u * ab);
