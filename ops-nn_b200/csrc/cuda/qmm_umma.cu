@@ -804,12 +804,48 @@ int32_t launch_bn(int bn, const CUtensorMap& ma, const CUtensorMap& mb, UmmaArgs
 #include "qmm_mx_umma_pair.cuh"
 #include "qmm_umma_split.cuh"
 
-// Whether a call runs on the split kernel (qmm_umma_split.cuh).
-static bool split_chosen(const OpsnnQmmParams* p)
+// Which of the three forms of the dequant and per-block kernels a call runs on.
+enum class Form { kSingle, kPair, kSplit };
+
+static Form choose_form(const OpsnnQmmParams* p)
 {
-    if (!split_takes(p)) return false;
-    if (const char* e = env("OPSNN_QMM_SPLIT")) return atoi(e) != 0;
-    return !pair_worthwhile(p) && !pair_pb_worthwhile(p);
+    const bool deq = p->mode == OPSNN_QMM_DEQ, pb = p->mode == OPSNN_QMM_PERBLOCK;
+    if (!deq && !pb) return Form::kSingle;
+    const bool pair_ok = pb || (p->out_dtype != ACL_INT32 && p->out_dtype != ACL_INT8);
+    if ((deq ? pair_worthwhile(p) : pair_pb_worthwhile(p)) && pair_ok) return Form::kPair;
+    const bool fixed = env("OPSNN_QMM_BN") || env("OPSNN_QMM_KSPLIT") || env("OPSNN_QMM_PAIR") || env("OPSNN_QMM_PB_EW") || env("OPSNN_QMM_PB_BN") ||
+                       env("OPSNN_TEST_UMMA_STALL_KBLOCK");
+    if (fixed) return Form::kSingle;
+    const char* split_env = env("OPSNN_QMM_SPLIT");
+    if (split_env != nullptr && atoi(split_env) != 0 && split_takes(p)) return Form::kSplit;
+    // Too few tiles for every pair of SMs: the cheapest by the times that were measured (us, k-blocks resident in L2), of
+    //   single  waves of 128 x BN tiles over the SMs; a k-block 0.155 / 0.21 / 0.27 / 0.36 at BN 32 / 64 / 128 / 256, per-block 0.43
+    //   pair    waves of 256 x 256 (per-block 256 x 128) tiles over the pairs; a k-block 0.36 (0.29), 2 (1.5) per tile
+    //   split   its own plan's cost
+    // (fp8, m717 k7168 n2304: 29.3 / 26.2 / 20.0; m1024 k7168 n4608: 38.1 / 29.9 / 34.7; m40 k8192 n3072: 16.3 / 25.1 / 10.9;
+    // per-block m100 k7168 n4096: 25.0 / 19.8 / 14.4, m512 k4096 n4096: 18.6 / 14.6 / 49)
+    const bool f16 = p->a_dtype == ACL_BF16 || p->a_dtype == ACL_FLOAT16;
+    const double kb = (double)((p->k * (f16 ? 2 : 1) + BK - 1) / BK);
+    auto waves = [](int64_t tiles, int64_t units) { return (double)((tiles + units - 1) / units); };
+    const int sms = sm_count(), bn = pick_bn(p);
+    const double per = pb ? 0.43 : (bn == 32 ? 0.155 : (bn == 64 ? 0.21 : (bn == 128 ? 0.27 : 0.36)));
+    double best = 5.0 + waves(p->batch * ((p->m + BM - 1) / BM) * ((p->n + bn - 1) / bn), sms) * kb * per;
+    Form form = Form::kSingle;
+    if (pair_ok && p->m > BM && p->n >= 256) {
+        const double cost = deq ? 4.0 + waves(p->batch * ((p->m + 255) / 256) * ((p->n + 255) / 256), sms / 2) * (kb * 0.36 + 2.0)
+                                : 5.0 + waves(p->batch * ((p->m + 255) / 256) * ((p->n + 127) / 128), sms / 2) * (kb * 0.29 + 1.5);
+        if (cost < best) {
+            best = cost;
+            form = Form::kPair;
+        }
+    }
+    if (split_takes(p) && (split_env == nullptr || atoi(split_env) != 0)) {
+        SplitKernel kern;
+        SplitPlan q;
+        if (split_prepare(p, &kern, &q) == cudaSuccess && q.cost < best) form = Form::kSplit;
+        else cudaGetLastError();
+    }
+    return form;
 }
 
 bool qmm_umma_eligible(const OpsnnQmmParams* p)
@@ -851,7 +887,7 @@ uint64_t qmm_umma_workspace_size(const OpsnnQmmParams* p)
 {
     if (p->mode == OPSNN_QMM_MX) return qmm_mx_umma_workspace_size(p);
     if (p->mode == OPSNN_QMM_PERGROUP_ASYM) return (uint64_t)p->m * (uint64_t)((p->k + 255) / 256) * 4u + 256u;  // row sums per k-group
-    if (split_chosen(p)) {
+    if (choose_form(p) == Form::kSplit) {
         SplitKernel kern;
         SplitPlan q;
         if (split_prepare(p, &kern, &q) == cudaSuccess) return split_workspace(q);
@@ -910,14 +946,15 @@ int32_t qmm_umma_launch(const OpsnnQmmParams* p, cudaStream_t stream)
 {
     if (const int32_t bad = umma_prelaunch_check()) return bad;
     if (p->mode == OPSNN_QMM_MX) return qmm_mx_umma_launch(p, stream);
-    if (split_chosen(p)) {
+    const Form form = choose_form(p);
+    if (form == Form::kSplit) {
         const int32_t rc = split_launch(p, stream);
         if (rc >= 0) return rc;
     }
-    const bool pair = pair_worthwhile(p) && p->mode == OPSNN_QMM_DEQ && p->out_dtype != ACL_INT32 && p->out_dtype != ACL_INT8;
+    const bool pair = form == Form::kPair && p->mode == OPSNN_QMM_DEQ;
     // per-block on CTA pairs: 256 x 128 tiles
     const bool asym = p->mode == OPSNN_QMM_PERGROUP_ASYM;
-    const bool pair_pb = asym || pair_pb_worthwhile(p);
+    const bool pair_pb = asym || (form == Form::kPair && p->mode == OPSNN_QMM_PERBLOCK);
     const uint8_t* b_ptr = static_cast<const uint8_t*>(p->b);
     int64_t b_ld = p->b_ld, b_bs = p->b_bs;
     int b_trans = p->trans_b;

@@ -292,11 +292,11 @@ qmm_umma_split_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_co
     asm volatile("griddepcontrol.wait;" ::: "memory");
 
     const uint32_t u_begin = split_begin(a, blockIdx.x), u_end = split_begin(a, blockIdx.x + 1);
-    SplitCols4 cols4;
+    SplitCols4 cols4;  // (per-block: only a bias, read at the end; 16 registers the sums need)
     if (warp < 8 && a.split != 0u) {
         const SplitTile tile = split_tile(a, blockIdx.x / a.split);
-        cols4 = split_cols4<kPerBlock, kHalves>(a, tile, threadIdx.x);
-        if (threadIdx.x < a.rows) s_sa[threadIdx.x] = split_sa<kPerBlock>(a, tile.r0 + min(threadIdx.x, tile.live - 1u));
+        if constexpr (!kPerBlock) cols4 = split_cols4<kPerBlock, kHalves>(a, tile, threadIdx.x);
+        if (!kPerBlock && threadIdx.x < a.rows) s_sa[threadIdx.x] = split_sa<kPerBlock>(a, tile.r0 + min(threadIdx.x, tile.live - 1u));
     }
     const uint32_t set = kHalves * a.rows;  // TMEM columns of one accumulator buffer
 
@@ -426,21 +426,31 @@ qmm_umma_split_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_co
                     }
                     ptx::tc_fence_after();
                     const uint32_t t0 = tbase + buf * set, rk = ring + (k & 1u) * 512u;
+                    // 16 sums at a time, the next 16 on their way while these are promoted
+                    uint32_t va[16], vb[16];
+                    auto promote16 = [&](const uint32_t (&v)[16], int i) {
 #pragma unroll
-                    for (int i = 0; i < kAcc; i += 16) {
+                        for (int e = 0; e < 16; e += 4) {
+                            float4 sc;
+                            asm volatile("ld.shared.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(sc.x), "=f"(sc.y), "=f"(sc.z), "=f"(sc.w) : "r"(rk + (i + e) * 4));
+                            acc[i + e] = fmaf(__uint_as_float(v[e]), sc.x, acc[i + e]);
+                            acc[i + e + 1] = fmaf(__uint_as_float(v[e + 1]), sc.y, acc[i + e + 1]);
+                            acc[i + e + 2] = fmaf(__uint_as_float(v[e + 2]), sc.z, acc[i + e + 2]);
+                            acc[i + e + 3] = fmaf(__uint_as_float(v[e + 3]), sc.w, acc[i + e + 3]);
+                        }
+                    };
+                    ptx::tmem_ld16(t0, va);
+#pragma unroll
+                    for (int i = 0; i < kAcc; i += 32) {
                         if ((uint32_t)i < cnt_rows) {
-                            uint32_t v[16];
-                            ptx::tmem_ld16(t0 + i, v);
                             ptx::tmem_ld_wait();
-#pragma unroll
-                            for (int e = 0; e < 16; e += 4) {
-                                float4 sc;
-                                asm volatile("ld.shared.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(sc.x), "=f"(sc.y), "=f"(sc.z), "=f"(sc.w) : "r"(rk + (i + e) * 4) : "memory");
-                                acc[i + e] = fmaf(__uint_as_float(v[e]), sc.x, acc[i + e]);
-                                acc[i + e + 1] = fmaf(__uint_as_float(v[e + 1]), sc.y, acc[i + e + 1]);
-                                acc[i + e + 2] = fmaf(__uint_as_float(v[e + 2]), sc.z, acc[i + e + 2]);
-                                acc[i + e + 3] = fmaf(__uint_as_float(v[e + 3]), sc.w, acc[i + e + 3]);
-                            }
+                            if ((uint32_t)(i + 16) < cnt_rows) ptx::tmem_ld16(t0 + i + 16, vb);
+                            promote16(va, i);
+                        }
+                        if ((uint32_t)(i + 16) < cnt_rows) {
+                            ptx::tmem_ld_wait();
+                            if (i + 32 < kAcc && (uint32_t)(i + 32) < cnt_rows) ptx::tmem_ld16(t0 + i + 32, va);
+                            promote16(vb, i + 16);
                         }
                     }
                     ptx::tc_fence_before();
@@ -493,6 +503,7 @@ qmm_umma_split_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_co
                 }
                 if (a.split == 1u) {
                     asm volatile("bar.sync 1, 256;" ::: "memory");
+                    if constexpr (kPerBlock) cols4 = split_cols4<kPerBlock, kHalves>(a, split_tile(a, t), threadIdx.x);
                     split_sum_and_store<kPerBlock, kHalves>(a, smem0, split_tile(a, t), 0u, threadIdx.x, s_sa, cols4);
                 }
             } else {
@@ -519,6 +530,7 @@ qmm_umma_split_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_co
                 asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(remote) : "r"(ptx::smem_u32(const_cast<uint32_t*>(&s_abort))), "r"((uint32_t)lane));
                 asm volatile("ld.shared::cluster.u32 %0, [%1];" : "=r"(bad) : "r"(remote) : "memory");
             }
+            if constexpr (kPerBlock) cols4 = split_cols4<kPerBlock, kHalves>(a, split_tile(a, blockIdx.x / a.split), threadIdx.x);
             if (!__any_sync(0xffffffffu, bad != 0u))
                 split_sum_and_store<kPerBlock, kHalves>(a, smem0, split_tile(a, blockIdx.x / a.split), ptx::cluster_ctarank(), threadIdx.x, s_sa, cols4);
         }
@@ -537,16 +549,17 @@ using SplitKernel = void (*)(const CUtensorMap, const CUtensorMap, const SplitAr
 
 struct SplitPlan {
     uint32_t rows = 0, halves = 0, t_tiles = 0, n_tiles = 0, kb = 0, split = 0, stages = 0, stage_bytes = 0;
-    int64_t tiles = 0, units = 0, grid = 0, cost = 0;
+    int64_t tiles = 0, units = 0, grid = 0;
+    double cost = 1e30;  // us
     int acc = 0;
 };
 
 // Whether the split kernel takes the call at all.
 bool split_takes(const OpsnnQmmParams* p)
 {
-    if (env("OPSNN_QMM_NO_SPLIT") || env("OPSNN_QMM_BN") || env("OPSNN_QMM_KSPLIT") || env("OPSNN_QMM_PAIR") || env("OPSNN_QMM_PB_EW") || env("OPSNN_QMM_PB_BN") ||
-        env("OPSNN_TEST_UMMA_STALL_KBLOCK"))
-        return false;
+    if (env("OPSNN_QMM_NO_SPLIT")) return false;
+    // beyond this the promotion (per-block) or the two-byte stores of shared tiles (dequant) cost more than idle SMs do
+    if (p->mode == OPSNN_QMM_PERBLOCK && p->m > 128) return false;
     const bool i8 = p->a_dtype == ACL_INT8, f8 = is_fp8(p->a_dtype);
     // int8 per-block sums are tested bit for bit against the reference's order of k-blocks: they are not split
     if (!(p->mode == OPSNN_QMM_DEQ && (i8 || f8)) && !(p->mode == OPSNN_QMM_PERBLOCK && f8)) return false;
@@ -556,14 +569,17 @@ bool split_takes(const OpsnnQmmParams* p)
     return p->batch * ((p->m + 15) / 16) * ((p->n + 127) / 128) * ((p->k + 127) / 128) < ((int64_t)1 << 31);
 }
 
-// One candidate tile shape, cut in the cheapest way; costs are in k-blocks of a 48 KB stage.
+// One candidate tile shape (halves; t_tiles row tiles more than needed), cut in the cheapest way. The costs (us) were fitted to fp8 and
+// int8 calls of 16 to 717 rows: launch and ramp, a k-block's fixed part, its tensor work (or promotion) and its share of a stream of
+// weights out of HBM, and the combination, which grows with the tile.
 template <typename F>
-SplitPlan split_candidate(const OpsnnQmmParams* p, uint32_t halves, int sms, F&& clusters)
+SplitPlan split_candidate(const OpsnnQmmParams* p, uint32_t halves, uint32_t more, int sms, F&& clusters)
 {
     SplitPlan q;
+    const bool pb = p->mode == OPSNN_QMM_PERBLOCK;
     const uint32_t most_rows = halves == 2 ? 128 : 256, unit = halves == 2 ? 16 : 32;
     q.halves = halves;
-    q.t_tiles = (uint32_t)((p->m + most_rows - 1) / most_rows);
+    q.t_tiles = (uint32_t)((p->m + most_rows - 1) / most_rows) + more;
     const uint32_t per = (uint32_t)((p->m + q.t_tiles - 1) / q.t_tiles);
     q.rows = (per + unit - 1) / unit * unit;
     q.t_tiles = (uint32_t)((p->m + q.rows - 1) / q.rows);
@@ -572,30 +588,29 @@ SplitPlan split_candidate(const OpsnnQmmParams* p, uint32_t halves, int sms, F&&
     q.tiles = p->batch * q.n_tiles * q.t_tiles;
     q.units = q.tiles * q.kb;
     const uint32_t served = halves == 2 ? q.rows : q.rows / 2;
-    q.acc = served <= 32 ? 32 : (served <= 64 ? 64 : 128);
+    if (pb && served > 64) return q;
+    q.acc = served <= 32 ? 32 : 64;
     q.stage_bytes = halves * kATile + q.rows * BK;
-    const uint32_t ring = p->mode == OPSNN_QMM_PERBLOCK ? kSplitRing : 0u;
-    q.stages = (kSplitSmem - 2048 - ring) / q.stage_bytes;
+    q.stages = (kSplitSmem - 2048 - (pb ? kSplitRing : 0u)) / q.stage_bytes;
     if (q.stages > (uint32_t)kSplitMaxStages) q.stages = kSplitMaxStages;
-    // time of a k-block relative to a full 48 KB stage: operand feed, or the promotion of the accumulators
-    const double feed = q.stage_bytes / 49152.0, promote = p->mode == OPSNN_QMM_PERBLOCK ? 0.1 + 1.4 * served / 128.0 : 0.0;
-    const double w = feed > promote ? feed : promote;
-    double best = 1e30;
+    const double area = (double)q.rows * halves;
     auto consider = [&](int64_t grid, uint32_t split, double extra) {
-        const double cost = (double)((q.units + grid - 1) / grid) * w + extra;
-        if (cost < best) {
-            best = cost;
+        double w = 0.12 + (pb ? 0.0075 * served : 0.00135 * area);
+        const double hbm = (double)grid * halves * kATile / q.t_tiles / 5.8e6;  // all CTAs' weights of one k-block
+        if (hbm > w) w = hbm;
+        const double cost = 5.5 + (double)((q.units + grid - 1) / grid) * w + extra;
+        if (cost < q.cost) {
+            q.cost = cost;
             q.grid = grid;
             q.split = split;
         }
     };
-    consider(q.units < sms ? q.units : sms, 0, 12.0 + q.rows * halves / 24.0);
+    consider(q.units < sms ? q.units : sms, 0, 4.0 + area * 0.1);
     int64_t most = sms / q.tiles;
     if (most > 16) most = 16;
     if (most > q.kb) most = q.kb;
     for (int s = (int)most; s >= 1; --s)
-        if (s == 1 || (int64_t)clusters(q, s) >= q.tiles) consider(q.tiles * s, (uint32_t)s, s > 1 ? 6.0 : 3.0);
-    q.cost = (int64_t)(best * 16.0);
+        if (s == 1 || (int64_t)clusters(q, s) >= q.tiles) consider(q.tiles * s, (uint32_t)s, s > 1 ? 1.2 + 0.011 * area : 0.03 * area);
     return q;
 }
 
@@ -605,8 +620,7 @@ SplitKernel split_kernel_of(bool per_block, int acc)
     if constexpr (kKind == ptx::MmaKind::kF8F6F4) {
         if (per_block) {
             if (acc == 32) return &qmm_umma_split_kernel<kKind, true, 32, kHalves>;
-            if (acc == 64) return &qmm_umma_split_kernel<kKind, true, 64, kHalves>;
-            return &qmm_umma_split_kernel<kKind, true, 128, kHalves>;
+            return &qmm_umma_split_kernel<kKind, true, 64, kHalves>;
         }
     }
     return &qmm_umma_split_kernel<kKind, false, 16, kHalves>;
@@ -617,7 +631,7 @@ SplitKernel split_kernel(bool i8, bool per_block, const SplitPlan& q)
     const SplitKernel k = i8 ? (q.halves == 2 ? split_kernel_of<ptx::MmaKind::kI8, 2>(per_block, q.acc) : split_kernel_of<ptx::MmaKind::kI8, 1>(per_block, q.acc))
                              : (q.halves == 2 ? split_kernel_of<ptx::MmaKind::kF8F6F4, 2>(per_block, q.acc) : split_kernel_of<ptx::MmaKind::kF8F6F4, 1>(per_block, q.acc));
     static std::atomic<uint64_t> configured[16];
-    const int index = (q.halves == 2 ? 8 : 0) + (i8 ? 0 : (!per_block ? 1 : (q.acc == 32 ? 2 : (q.acc == 64 ? 3 : 4))));
+    const int index = (q.halves == 2 ? 8 : 0) + (i8 ? 0 : (!per_block ? 1 : (q.acc == 32 ? 2 : 3)));
     const cudaError_t rc = once_per_device(configured[index], [&] {
         cudaFuncSetAttribute(k, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
         return cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, kSplitSmem);
@@ -631,18 +645,18 @@ cudaError_t split_prepare(const OpsnnQmmParams* p, SplitKernel* kern, SplitPlan*
     int device = -1;
     const bool have_device = cudaGetDevice(&device) == cudaSuccess;
     const int sms = have_device ? sm_count() : 148;
-    for (uint32_t halves = 2; halves >= 1; --halves) {
-        const SplitPlan q = split_candidate(p, halves, sms, [&](const SplitPlan& c, int s) -> int {
+    *plan = SplitPlan{};
+    for (uint32_t c = 0; c < 8; ++c) {
+        const uint32_t halves = 2u - (c & 1u);
+        const SplitPlan q = split_candidate(p, halves, c >> 1, sms, [&](const SplitPlan& c, int s) -> int {
             const SplitKernel k = have_device ? split_kernel(i8, pb, c) : nullptr;
             return k == nullptr ? 0 : max_active_clusters(reinterpret_cast<const void*>(k), kSplitThreads, kSplitSmem, s, 0);
         });
-        if (halves == 2 || q.cost < plan->cost) *plan = q;
         if (const char* e = env("OPSNN_QMM_SPLIT_HALVES"))  // experiments
-            if (atoi(e) == (int)halves) {
-                *plan = q;
-                break;
-            }
+            if (atoi(e) != (int)halves) continue;
+        if (q.cost < plan->cost) *plan = q;
     }
+    if (plan->grid == 0) return cudaErrorNotSupported;
     *kern = nullptr;
     if (!have_device) return cudaErrorNoDevice;
     *kern = split_kernel(i8, pb, *plan);
@@ -661,7 +675,10 @@ int32_t split_launch(const OpsnnQmmParams* p, cudaStream_t stream)
 {
     SplitKernel kern;
     SplitPlan q;
-    if (const cudaError_t rc = split_prepare(p, &kern, &q); rc != cudaSuccess) return (int32_t)rc;
+    if (split_prepare(p, &kern, &q) != cudaSuccess) {
+        cudaGetLastError();
+        return -1;
+    }
     if (q.split == 0 && (p->workspace == nullptr || p->workspace_size < split_workspace(q))) return -1;
     const bool pb = p->mode == OPSNN_QMM_PERBLOCK;
     SplitArgs a{};
