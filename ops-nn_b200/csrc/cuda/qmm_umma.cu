@@ -818,6 +818,8 @@ static Form choose_form(const OpsnnQmmParams* p)
     if (fixed) return Form::kSingle;
     const char* split_env = env("OPSNN_QMM_SPLIT");
     if (split_env != nullptr && atoi(split_env) != 0 && split_takes(p)) return Form::kSplit;
+    // A decoding step: 128-row tiles would be mostly padding (m16 k4096 n4096 14.3 -> 7.3 us, m8 k7168 n18432 53 -> 27).
+    if (p->m <= 64 && split_takes(p) && (split_env == nullptr || atoi(split_env) != 0)) return Form::kSplit;
     // Too few tiles for every pair of SMs: the cheapest by the times that were measured (us, k-blocks resident in L2), of
     //   single  waves of 128 x BN tiles over the SMs; a k-block 0.155 / 0.21 / 0.27 / 0.36 at BN 32 / 64 / 128 / 256, per-block 0.43
     //   pair    waves of 256 x 256 (per-block 256 x 128) tiles over the pairs; a k-block 0.36 (0.29), 2 (1.5) per tile

@@ -605,12 +605,12 @@ SplitPlan split_candidate(const OpsnnQmmParams* p, uint32_t halves, uint32_t mor
             q.split = split;
         }
     };
-    consider(q.units < sms ? q.units : sms, 0, 4.0 + area * 0.1);
+    consider(q.units < sms ? q.units : sms, 0, 1.0 + area * 0.05);
     int64_t most = sms / q.tiles;
     if (most > 16) most = 16;
     if (most > q.kb) most = q.kb;
     for (int s = (int)most; s >= 1; --s)
-        if (s == 1 || (int64_t)clusters(q, s) >= q.tiles) consider(q.tiles * s, (uint32_t)s, s > 1 ? 1.2 + 0.011 * area : 0.03 * area);
+        if (s == 1 || (int64_t)clusters(q, s) >= q.tiles) consider(q.tiles * s, (uint32_t)s, s > 1 ? std::max(0.4, 0.6 * s + 0.012 * area - 1.8) : 0.02 * area);
     return q;
 }
 

@@ -1,0 +1,71 @@
+"""GPU: the split kernel of the dequant and per-block modes (weight columns as the MMA's M, k cut into pieces) against the oracle, at the
+sizes where its tiles, pieces and ways of combining them begin and end. int8 sums are exact, so those outputs are bit-exact; fp8 differs by
+fp32 summation order."""
+import ml_dtypes
+import numpy as np
+import pytest
+
+from conftest import case_seed
+from oracle import qbmm_oracle
+
+pytestmark = pytest.mark.gpu
+
+E4M3, E5M2 = ml_dtypes.float8_e4m3fn, ml_dtypes.float8_e5m2
+
+CASES = [
+    # mode, batch, m, k, n, x2 stored (n,k), bias, out
+    ("int8", (), 1, 4096, 256, True, "i32", "bfloat16"),       # one or two tiles, a piece per CTA of a cluster
+    ("int8", (), 17, 2064, 2064, False, "f32", "bfloat16"),    # ragged k and n, x2 along n
+    ("int8", (), 64, 512, 22000, True, None, "float16"),       # more tiles than SMs: equal pieces across tiles
+    ("int8", (), 130, 4112, 272, True, "i32", "bfloat16"),     # two row tiles, few columns
+    ("int8", (2,), 33, 1040, 656, True, None, "bfloat16"),     # batched
+    ("fp8", (), 16, 6144, 1040, False, "f32", "float16"),
+    ("fp8", (), 250, 2048, 528, True, None, "float32"),
+    ("e5m2", (), 40, 1072, 20000, True, "f32", "bfloat16"),
+    ("block", (), 1, 7168, 400, True, None, "bfloat16"),
+    ("block", (), 48, 1152, 20096, False, None, "float16"),    # per-block pieces across tiles
+    ("block", (), 100, 3072, 640, True, None, "float32"),
+    ("block", (3,), 20, 1088, 320, True, None, "bfloat16"),    # last k-block half full
+]
+
+
+@pytest.mark.parametrize("case", CASES, ids=[str(c) for c in CASES])
+def test_split_kernel_equals_oracle(aclnn, monkeypatch, case):
+    import torch
+
+    from gpu_util import check_close, desc, out_tensor, out_to_np
+
+    mode, batch, m, k, n, nk, bias_kind, out_name = case
+    monkeypatch.setenv("OPSNN_QMM_SPLIT", "1")
+    rng = np.random.default_rng(case_seed(case))
+    if mode == "int8":
+        x1 = rng.integers(-127, 128, batch + (m, k), dtype=np.int8)
+        x2 = rng.integers(-127, 128, batch + ((n, k) if nk else (k, n)), dtype=np.int8)
+    else:
+        dt = E5M2 if mode == "e5m2" else E4M3
+        x1 = rng.standard_normal(batch + (m, k)).astype(np.float32).astype(E4M3)
+        x2 = rng.standard_normal(batch + ((n, k) if nk else (k, n))).astype(np.float32).astype(dt)
+    group = 0
+    if mode == "block":
+        kb, ng = -(-k // 128), -(-n // 128)
+        s1 = rng.uniform(0.5, 2, batch + (m, kb)).astype(np.float32)
+        s2 = rng.uniform(0.5, 2, batch + ((ng, kb) if nk else (kb, ng))).astype(np.float32)
+        group = (1 << 32) | (128 << 16) | 128
+    else:
+        s1 = rng.uniform(1e-3, 1e-2, m).astype(np.float32) if not batch else None
+        s2 = rng.uniform(1e-3, 1e-2, n).astype(np.float32)
+    bias = {None: None, "i32": rng.integers(-1000, 1001, n).astype(np.int32), "f32": rng.uniform(-1, 1, n).astype(np.float32)}[bias_kind]
+    want = qbmm_oracle.quant_matmul_v5(x1, x2, s1, s2, bias, False, nk, group, out_name)
+    outs = []
+    for _ in range(2):  # twice: the second call finds the workspace as the first left it
+        out = out_tensor(batch + (m, n), out_name)
+        aclnn.quant_matmul_v5(desc(aclnn, x1), desc(aclnn, x2), desc(aclnn, s1), desc(aclnn, s2), aclnn.Tensor(out.shape, out_name, out), desc(aclnn, bias),
+                              False, nk, group)
+        torch.cuda.synchronize()
+        outs.append(out_to_np(out))
+    assert aclnn.last_kernel_name() == ("qmm_umma_perblock" if mode == "block" else "qmm_umma_deq"), aclnn.last_kernel_name()
+    assert np.array_equal(outs[0].view(np.uint8), outs[1].view(np.uint8))
+    if mode == "int8":
+        assert np.array_equal(outs[0].view(np.uint8), np.asarray(want).view(np.uint8))
+    else:
+        check_close(outs[0], want, qbmm_oracle.quant_matmul_v5(x1, x2, s1, s2, bias, False, nk, group, "float32"), out_name)
