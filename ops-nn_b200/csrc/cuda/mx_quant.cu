@@ -140,62 +140,104 @@ __global__ void __launch_bounds__(256) mx_quant_kernel(const OpsnnMxQuantParams 
     }
 }
 
-// Streaming form: k % 32 == 0, x and y 16-byte aligned. One lane = 8 consecutive elements; lanes 4j..4j+3 = one block.
+// Largest magnitude of two packed pairs, per half; a NaN loses against a number, as fmaxf has it.
 template <bool kBf16>
+__device__ __forceinline__ uint32_t max_pair(uint32_t a, uint32_t b)
+{
+    uint32_t d;
+    if (kBf16) asm("max.bf16x2 %0, %1, %2;" : "=r"(d) : "r"(a), "r"(b));
+    else asm("max.f16x2 %0, %1, %2;" : "=r"(d) : "r"(a), "r"(b));
+    return d;
+}
+// Two values to the destination type, round to nearest even, saturating (NaN: e4m3 / e5m2 NaN, e2m1 +6); `lo` into the low half.
+__device__ __forceinline__ uint32_t cvt_e2m1x2(float lo, float hi)
+{
+    uint32_t r;
+    asm("{\n\t.reg .b8 t;\n\tcvt.rn.satfinite.e2m1x2.f32 t, %2, %1;\n\tcvt.u32.u8 %0, t;\n\t}" : "=r"(r) : "f"(lo), "f"(hi));
+    return r;
+}
+template <bool kE4m3>
+__device__ __forceinline__ uint32_t cvt_fp8x2(float lo, float hi)
+{
+    return __nv_cvt_float2_to_fp8x2(make_float2(lo, hi), __NV_SATFINITE, kE4m3 ? __NV_E4M3 : __NV_E5M2);
+}
+
+// Streaming form: k % 32 == 0, x and y 16-byte aligned. One lane = 8 consecutive elements; lanes 4j..4j+3 = one block.
+// HBM bound, so: kUnroll loads of 16 bytes in flight per thread (4 where that still leaves every SM several CTAs), the block maximum on
+// packed pairs, the hardware's paired conversions (element by element, e2m1 by comparisons, this was issue bound at 1.3 TB/s, e4m3 at
+// 3.5), no division where the blocks of a row are an even number.
+template <bool kBf16, int kUnroll>
 __global__ void __launch_bounds__(256) mx_quant_stream_kernel(const OpsnnMxQuantParams p, int64_t blocks_per_row, int64_t scale_row)
 {
     const int64_t pieces = p.rows * blocks_per_row * 4;  // 8-element pieces
     const int emax = p.y_dtype == ACL_FLOAT4_E2M1 ? 2 : (p.y_dtype == ACL_FLOAT8_E4M3FN ? 8 : 15);
     const uint4* src = reinterpret_cast<const uint4*>(p.x);
-    for (int64_t i0 = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) & ~(int64_t)31; i0 < pieces; i0 += (int64_t)gridDim.x * blockDim.x) {
-        const int64_t i = i0 + (threadIdx.x & 31);
-        const bool live = i < pieces;  // pieces is a multiple of 4, so a block's four lanes are live together
-        uint4 raw = make_uint4(0u, 0u, 0u, 0u);
-        if (live) raw = __ldcs(src + i);
-        const uint32_t w[4] = {raw.x, raw.y, raw.z, raw.w};
+    const int64_t i0 = (int64_t)blockIdx.x * (256 * kUnroll) + threadIdx.x;
+    uint4 raw[kUnroll];
+#pragma unroll
+    for (int u = 0; u < kUnroll; ++u) {
+        const int64_t i = i0 + u * 256;
+        raw[u] = i < pieces ? __ldcs(src + i) : make_uint4(0u, 0u, 0u, 0u);  // pieces is a multiple of 4: a block's four lanes are live together
+    }
+#pragma unroll
+    for (int u = 0; u < kUnroll; ++u) {
+        const int64_t i = i0 + u * 256;
+        const uint32_t w[4] = {raw[u].x, raw[u].y, raw[u].z, raw[u].w};
+        constexpr uint32_t kMag = 0x7FFF7FFFu;
+        uint32_t m = max_pair<kBf16>(max_pair<kBf16>(w[0] & kMag, w[1] & kMag), max_pair<kBf16>(w[2] & kMag, w[3] & kMag));
+        m = max_pair<kBf16>(m, __shfl_xor_sync(0xffffffffu, m, 1));
+        m = max_pair<kBf16>(m, __shfl_xor_sync(0xffffffffu, m, 2));
+        m = max_pair<kBf16>(m, m >> 16);
+        const float amax = kBf16 ? __uint_as_float(m << 16) : __half2float(__ushort_as_half((unsigned short)(m & 0xFFFFu)));
+        const int e = mx_block_exp(amax, p, emax);
+        if (i >= pieces) continue;
+        const int64_t blk_lin = i >> 2;
+        if ((i & 3) == 0) {
+            const uint8_t byte = e > 127 ? 255 : (uint8_t)(e + 127);
+            uint8_t* sc = reinterpret_cast<uint8_t*>(p.scale);
+            if (scale_row == blocks_per_row) {
+                sc[blk_lin] = byte;
+            } else {  // one padding entry per row makes the count even
+                const int64_t row = blk_lin < (int64_t)0x7FFFFFFF ? (int64_t)((uint32_t)blk_lin / (uint32_t)blocks_per_row) : blk_lin / blocks_per_row;
+                const int64_t blk = blk_lin - row * blocks_per_row;
+                sc[blk_lin + row] = byte;
+                if (blk == blocks_per_row - 1) sc[blk_lin + row + 1] = 0;
+            }
+        }
+        // 2^-e; 2^-127 is subnormal: that scale is applied as two exact factors
+        const float s0 = e > 127 ? __uint_as_float(0x7FC00000u) : (e == 127 ? __uint_as_float(1u << 23) : __uint_as_float((uint32_t)(127 - e) << 23));
         float v[8];
 #pragma unroll
         for (int j = 0; j < 4; ++j) {
             if (kBf16) {
-                v[2 * j] = __uint_as_float(w[j] << 16);
-                v[2 * j + 1] = __uint_as_float(w[j] & 0xFFFF0000u);
+                v[2 * j] = __uint_as_float(w[j] << 16) * s0;
+                v[2 * j + 1] = __uint_as_float(w[j] & 0xFFFF0000u) * s0;
             } else {
                 const float2 f2 = __half22float2(*reinterpret_cast<const __half2*>(&w[j]));
-                v[2 * j] = f2.x;
-                v[2 * j + 1] = f2.y;
+                v[2 * j] = f2.x * s0;
+                v[2 * j + 1] = f2.y * s0;
             }
         }
-        float amax = 0.f;
+        if (e == 127) {
 #pragma unroll
-        for (int j = 0; j < 8; ++j) amax = fmaxf(amax, fabsf(v[j]));
-        amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, 1));
-        amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, 2));
-        const int e = mx_block_exp(amax, p, emax);
-        if (!live) continue;
-        const int64_t blk_lin = i >> 2;
-        if ((i & 3) == 0) {
-            const int64_t row = blk_lin / blocks_per_row, blk = blk_lin % blocks_per_row;
-            uint8_t* sc = reinterpret_cast<uint8_t*>(p.scale) + row * scale_row + blk;
-            *sc = e > 127 ? 255 : (uint8_t)(e + 127);
-            if (blk == blocks_per_row - 1 && scale_row != blocks_per_row) sc[1] = 0;  // padding entry that makes the count even
+            for (int j = 0; j < 8; ++j) v[j] *= 0.5f;
         }
-        const float inv = e > 127 ? __uint_as_float(0x7FC00000u) : __uint_as_float((uint32_t)(127 - e) << 23 | 0u);  // 2^-e, e in [-127, 127]
-        const float inv2 = (e == 127) ? 0.5f : 1.f;  // 2^-127 is subnormal: split the scale in two exact factors
-        const float s0 = (e == 127) ? __uint_as_float(1u << 23) : inv;  // 2^-126 when e == 127
         if (p.y_dtype == ACL_FLOAT4_E2M1) {
             uint32_t out = 0;
+            if (p.round_mode == 0) {
 #pragma unroll
-            for (int j = 0; j < 8; ++j) out |= (uint32_t)quant_fp4_e2m1_mode(v[j] * s0 * inv2, p.round_mode) << (4 * j);
-            reinterpret_cast<uint32_t*>(p.y)[i] = out;
-        } else {
-            const __nv_fp8_interpretation_t kind = p.y_dtype == ACL_FLOAT8_E4M3FN ? __NV_E4M3 : __NV_E5M2;
-            uint32_t lo = 0, hi = 0;
+                for (int j = 0; j < 4; ++j) out |= cvt_e2m1x2(v[2 * j], v[2 * j + 1]) << (8 * j);
+            } else {
 #pragma unroll
-            for (int j = 0; j < 4; ++j) {
-                lo |= (uint32_t)__nv_cvt_float_to_fp8(v[j] * s0 * inv2, __NV_SATFINITE, kind) << (8 * j);
-                hi |= (uint32_t)__nv_cvt_float_to_fp8(v[4 + j] * s0 * inv2, __NV_SATFINITE, kind) << (8 * j);
+                for (int j = 0; j < 8; ++j) out |= (uint32_t)quant_fp4_e2m1_mode(v[j], p.round_mode) << (4 * j);
             }
-            reinterpret_cast<uint2*>(p.y)[i] = make_uint2(lo, hi);
+            reinterpret_cast<uint32_t*>(p.y)[i] = out;
+        } else if (p.y_dtype == ACL_FLOAT8_E4M3FN) {
+            reinterpret_cast<uint2*>(p.y)[i] = make_uint2(cvt_fp8x2<true>(v[0], v[1]) | (cvt_fp8x2<true>(v[2], v[3]) << 16),
+                                                          cvt_fp8x2<true>(v[4], v[5]) | (cvt_fp8x2<true>(v[6], v[7]) << 16));
+        } else {
+            reinterpret_cast<uint2*>(p.y)[i] = make_uint2(cvt_fp8x2<false>(v[0], v[1]) | (cvt_fp8x2<false>(v[2], v[3]) << 16),
+                                                          cvt_fp8x2<false>(v[4], v[5]) | (cvt_fp8x2<false>(v[6], v[7]) << 16));
         }
     }
 }
@@ -291,10 +333,14 @@ int32_t mx_quant_launch(const OpsnnMxQuantParams* p, cudaStream_t stream)
                            env("OPSNN_MXQ_GENERIC") == nullptr;
     if (stream_ok) {
         const int64_t pieces = p->rows * blocks_per_row * 4;
-        int64_t g2 = (pieces + 255) / 256;
-        if (g2 > 148 * 16) g2 = 148 * 16;
-        if (p->x_dtype == ACL_BF16) mx_quant_stream_kernel<true><<<(unsigned)g2, 256, 0, stream>>>(*p, blocks_per_row, scale_row);
-        else mx_quant_stream_kernel<false><<<(unsigned)g2, 256, 0, stream>>>(*p, blocks_per_row, scale_row);
+        const bool many = pieces >= (int64_t)148 * 8 * 256 * 4;
+        const int64_t per = 256 * (many ? 4 : 1), g2 = (pieces + per - 1) / per;
+        if (g2 > 0x7FFFFFFF) return (int32_t)cudaErrorInvalidConfiguration;
+        const bool bf = p->x_dtype == ACL_BF16;
+        if (bf && many) mx_quant_stream_kernel<true, 4><<<(unsigned)g2, 256, 0, stream>>>(*p, blocks_per_row, scale_row);
+        else if (bf) mx_quant_stream_kernel<true, 1><<<(unsigned)g2, 256, 0, stream>>>(*p, blocks_per_row, scale_row);
+        else if (many) mx_quant_stream_kernel<false, 4><<<(unsigned)g2, 256, 0, stream>>>(*p, blocks_per_row, scale_row);
+        else mx_quant_stream_kernel<false, 1><<<(unsigned)g2, 256, 0, stream>>>(*p, blocks_per_row, scale_row);
         note_launch("mx_quant_stream");
         return (int32_t)cudaGetLastError();
     }
