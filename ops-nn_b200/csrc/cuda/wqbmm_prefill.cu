@@ -12,8 +12,10 @@
 // HBM cost of the pre-pass: n*k/2 (int4) read + 2*n*k written, then 2*n*k read once by the matmul (x stays in L2):
 // worthwhile once the matmul's 2*m*n*k flops dominate; below m = 17 the fused streaming decode kernels are used.
 #include <cstdlib>
+#include <type_traits>
 
 #include "common.cuh"
+#include "wq_convert.cuh"
 #include "wqbmm_decode_common.cuh"
 
 namespace opsnn {
@@ -97,141 +99,146 @@ __device__ __forceinline__ float2 unpack2(uint32_t v)
     return __half22float2(*reinterpret_cast<const __half2*>(&v));
 }
 
-// The common layout: int4 stored (k,n) as 32-bit words of 8 columns, n % 8 == 0, word-aligned rows, scale/offset
-// contiguous along n and constant over a 64-row tile (per-channel, or groups of a multiple of 64 rows).
-// Thread = one word column (8 n) x two adjacent k rows: the two rows of a column leave as one packed pair, so the tile
-// is written with 32-bit stores; 16-byte pieces of a tile row are XOR-swizzled by the word column (conflict-free both ways).
-template <bool kBf16>
-__global__ void __launch_bounds__(NT) wq_dequant_nk_words_kernel(const OpsnnWqbmmParams p, uint16_t* __restrict__ dst, int64_t kp,
-                                                                 float* __restrict__ one)
+// Weight stored (k,n): a tile of 64 k rows x 32 words (256 int4 or 128 8-bit columns), so that a row of it is 128 bytes in the weight and
+// a column 128 bytes in the image. A thread owns one word column over 8 k rows; a pair conversion gives two columns of one row, two
+// rows' results are re-paired into (k, k + 1) words with byte permutes and kept at word (k pair ^ word column), which is free of bank
+// conflicts both ways and leaves a 16-byte piece together (in another order). Bound by HBM: 0.5 (1) bytes in, 2 out per weight; with
+// 32-byte pieces of rows and 4-byte stores it was 252 us for 8192 x 28672 int4, 588 MB.
+// Needs word-aligned rows, n a multiple of a word's columns, scales in x's dtype, groups of a multiple of 8 rows.
+template <MixW kW, bool kBf16, bool kOff>
+__global__ void __launch_bounds__(NT) wq_dequant_kn_kernel(const OpsnnWqbmmParams p, uint16_t* __restrict__ dst, int64_t kp, float* __restrict__ one,
+                                                           uint32_t tiles_n)
 {
-    __shared__ __align__(16) uint32_t tile[TN][TK / 2];  // [n][k pair], 128 bytes per row
-    const int tid = threadIdx.x;
-    const int64_t tiles_n = (p.n + TN - 1) / TN;
-    const int64_t k0 = ((int64_t)blockIdx.x / tiles_n) * TK, n0 = ((int64_t)blockIdx.x % tiles_n) * TN;
+    constexpr int kCols = kW == MixW::kInt4 ? 8 : 4, kPairs = kCols / 2, kTileN = 32 * kCols;
+    __shared__ __align__(16) uint32_t tile[kTileN * 32];
+    const int tid = threadIdx.x, wj = tid & 31, kr = tid >> 5;
+    const uint32_t tk = blockIdx.x / tiles_n;
+    const int64_t k0 = (int64_t)tk * 64, n0 = (int64_t)(blockIdx.x - tk * tiles_n) * kTileN;
     if (blockIdx.x == 0 && tid == 0) *one = 1.0f;
-    const int wj = tid & 7, kr = tid >> 3;  // word column 0..7, row pair 0..31
-    const int64_t gn = n0 + wj * 8, gk = k0 + 2 * kr;
-    const bool col_live = gn < p.n;
-    uint32_t w0 = 0u, w1 = 0u;
-    if (col_live && gk < p.k) w0 = __ldcs(reinterpret_cast<const uint32_t*>(p.w) + (gk * p.w_ld + gn) / 8);
-    if (col_live && gk + 1 < p.k) w1 = __ldcs(reinterpret_cast<const uint32_t*>(p.w) + ((gk + 1) * p.w_ld + gn) / 8);
-    float sc[8], of[8];
-    {
-        const int64_t g = p.group_size > 0 ? min(k0, p.k - 1) / p.group_size : 0;
-        const int64_t sidx = g * p.scale_sg + (col_live ? gn : 0) * p.scale_sn;
-#pragma unroll
-        for (int j = 0; j < 8; ++j) {
-            sc[j] = load_x<kBf16>(p.scale, sidx + j * p.scale_sn);
-            of[j] = p.offset != nullptr ? load_x<kBf16>(p.offset, sidx + j * p.scale_sn) : 0.f;
-        }
-    }
-    const bool has_off = p.offset != nullptr;
-#pragma unroll
-    for (int j = 0; j < 8; ++j) {
-        float a = (float)(((int32_t)(w0 << (28 - 4 * j))) >> 28);  // sign-extended nibble j of each row
-        float b = (float)(((int32_t)(w1 << (28 - 4 * j))) >> 28);
-        if (has_off) {
-            const float2 r = unpack2<kBf16>(pack2<kBf16>(__fadd_rn(a, of[j]), __fadd_rn(b, of[j])));  // first rounding
-            a = r.x;
-            b = r.y;
-        }
-        uint32_t v = pack2<kBf16>(__fmul_rn(a, sc[j]), __fmul_rn(b, sc[j]));  // second rounding
-        if (gk >= p.k) v = 0u;
-        else if (gk + 1 >= p.k) v &= 0xFFFFu;
-        tile[wj * 8 + j][(((kr >> 2) ^ wj) << 2) | (kr & 3)] = v;
-    }
-    __syncthreads();
-#pragma unroll
-    for (int e = tid; e < TN * 8; e += NT) {
-        const int nn = e >> 3, c = e & 7;  // row, 16-byte piece (8 k)
-        const int64_t on = n0 + nn, ok = k0 + c * 8;
-        if (on < p.n && ok < kp)
-            *reinterpret_cast<uint4*>(dst + on * kp + ok) = *reinterpret_cast<const uint4*>(&tile[nn][(c ^ (nn >> 3)) << 2]);
-    }
-}
-
-// The streaming form of the same layout: a thread owns one word column (8 n) over 8 consecutive k rows and does the
-// arithmetic on packed pairs exactly as the decode kernels do (nibble -> 136 + w by one lop3, then sub / add / mul .rn on
-// bf16x2 or f16x2: the reference's two roundings). A lop3 pairs columns j and j + 4 of one row; two rows' results are
-// re-paired into (k, k + 1) words of one column with byte permutes and stored into a 64 x 256 tile whose word index is
-// XOR-swizzled by the word column (bank = column + index, 129-word rows: conflict-free writes and reads).
-// Needs group_size % 8 == 0 (a thread's 8 rows share their scales).
-constexpr int PK = 256, PN = 64, PP = PK / 2 + 1;
-
-template <bool kBf16>
-__global__ void __launch_bounds__(NT) wq_dequant_nk_pairs_kernel(const OpsnnWqbmmParams p, uint16_t* __restrict__ dst, int64_t kp,
-                                                                 float* __restrict__ one, int vec_scale)
-{
-    using N = Num<kBf16>;
-    extern __shared__ uint32_t ptile[];  // [PN][PP]
-    const int tid = threadIdx.x;
-    const int64_t tiles_n = (p.n + PN - 1) / PN;
-    const int64_t k0 = ((int64_t)blockIdx.x / tiles_n) * PK, n0 = ((int64_t)blockIdx.x % tiles_n) * PN;
-    if (blockIdx.x == 0 && tid == 0) *one = 1.0f;
-    const int wj = tid & 7, kr = tid >> 3;
-    const int64_t gn = n0 + wj * 8, gk = k0 + 8 * kr;
+    const int64_t gn = n0 + wj * kCols, gk = k0 + 8 * kr;
     const bool col_live = gn < p.n;
     uint32_t w[8];
+    const uint8_t* src = static_cast<const uint8_t*>(p.w) + (gk * p.w_ld + gn) * (32 / kCols) / 8;
+    const int64_t pitch = p.w_ld * (32 / kCols) / 8;
 #pragma unroll
-    for (int i = 0; i < 8; ++i)
-        w[i] = (col_live && gk + i < p.k) ? __ldcs(reinterpret_cast<const uint32_t*>(p.w) + ((gk + i) * p.w_ld + gn) / 8) : 0u;
-    // scale / offset of columns (j, j + 4), j = 0..3, as packed pairs
-    uint32_t sp[4], op[4];
-    const bool has_off = p.offset != nullptr;
+    for (int i = 0; i < 8; ++i) w[i] = (col_live && gk + i < p.k) ? __ldcs(reinterpret_cast<const uint32_t*>(src + i * pitch)) : 0u;
+    uint32_t sp[kPairs], op[kPairs];  // scale / offset of columns (j, j + kCols / 2)
     {
         const int64_t g = p.group_size > 0 ? min(gk, p.k - 1) / p.group_size : 0;
-        const int64_t sidx = g * p.scale_sg + (col_live ? gn : 0) * p.scale_sn;
-        if (vec_scale) {
-            const uint4 sv = __ldg(reinterpret_cast<const uint4*>(reinterpret_cast<const uint16_t*>(p.scale) + sidx));
-            sp[0] = __byte_perm(sv.x, sv.z, 0x5410); sp[1] = __byte_perm(sv.x, sv.z, 0x7632);
-            sp[2] = __byte_perm(sv.y, sv.w, 0x5410); sp[3] = __byte_perm(sv.y, sv.w, 0x7632);
-            if (has_off) {
-                const uint4 ov = __ldg(reinterpret_cast<const uint4*>(reinterpret_cast<const uint16_t*>(p.offset) + sidx));
-                op[0] = __byte_perm(ov.x, ov.z, 0x5410); op[1] = __byte_perm(ov.x, ov.z, 0x7632);
-                op[2] = __byte_perm(ov.y, ov.w, 0x5410); op[3] = __byte_perm(ov.y, ov.w, 0x7632);
-            }
-        } else {
-            const uint16_t* sc = reinterpret_cast<const uint16_t*>(p.scale);
-            const uint16_t* of = reinterpret_cast<const uint16_t*>(p.offset);
+        const int64_t at = g * p.scale_sg + (col_live ? gn : 0) * p.scale_sn;
+        const uint16_t *sc = reinterpret_cast<const uint16_t*>(p.scale) + at, *of = reinterpret_cast<const uint16_t*>(p.offset) + at;
 #pragma unroll
-            for (int j = 0; j < 4; ++j) {
-                sp[j] = (uint32_t)__ldg(sc + sidx + j * p.scale_sn) | ((uint32_t)__ldg(sc + sidx + (j + 4) * p.scale_sn) << 16);
-                if (has_off) op[j] = (uint32_t)__ldg(of + sidx + j * p.scale_sn) | ((uint32_t)__ldg(of + sidx + (j + 4) * p.scale_sn) << 16);
-            }
+        for (int j = 0; j < kPairs; ++j) {
+            sp[j] = (uint32_t)__ldg(sc + j * p.scale_sn) | ((uint32_t)__ldg(sc + (j + kPairs) * p.scale_sn) << 16);
+            op[j] = kOff ? (uint32_t)__ldg(of + j * p.scale_sn) | ((uint32_t)__ldg(of + (j + kPairs) * p.scale_sn) << 16) : 0u;
         }
     }
-    const int swz = (wj & 3) | ((wj >> 2) << 4);
 #pragma unroll
     for (int rp = 0; rp < 4; ++rp) {
-        const int col = (4 * kr + rp) ^ swz;
+        const int at = (4 * kr + rp) ^ wj;
 #pragma unroll
-        for (int j = 0; j < 4; ++j) {
-            uint32_t t0, t1;
-            asm("lop3.b32 %0, %1, %2, %3, 0x6a;" : "=r"(t0) : "r"(w[2 * rp] >> (4 * j)), "n"(0x000F000F), "r"(N::kMagic));
-            asm("lop3.b32 %0, %1, %2, %3, 0x6a;" : "=r"(t1) : "r"(w[2 * rp + 1] >> (4 * j)), "n"(0x000F000F), "r"(N::kMagic));
-            t0 = N::sub(t0, N::kBias);
-            t1 = N::sub(t1, N::kBias);
-            if (has_off) {
-                t0 = N::add(t0, op[j]);
-                t1 = N::add(t1, op[j]);
+        for (int j = 0; j < kPairs; ++j) {
+            // the codes of columns j and j + kCols / 2 in the low bits of the halves
+            const uint32_t c0 = w[2 * rp] >> ((kW == MixW::kInt4 ? 4 : 8) * j), c1 = w[2 * rp + 1] >> ((kW == MixW::kInt4 ? 4 : 8) * j);
+            uint32_t t0 = mix_scale<kBf16, kOff>(mix_exact<kW, kBf16>(c0), sp[j], op[j]);
+            uint32_t t1 = mix_scale<kBf16, kOff>(mix_exact<kW, kBf16>(c1), sp[j], op[j]);
+            if (kW == MixW::kE4m3) {
+                t0 = fix_nan(t0, c0);
+                t1 = fix_nan(t1, c1);
             }
-            t0 = N::mul(t0, sp[j]);
-            t1 = N::mul(t1, sp[j]);
-            ptile[(wj * 8 + j) * PP + col] = __byte_perm(t0, t1, 0x5410);      // column j: rows (2rp, 2rp + 1)
-            ptile[(wj * 8 + j + 4) * PP + col] = __byte_perm(t0, t1, 0x7632);  // column j + 4
+            if (gk + 2 * rp >= p.k) t0 = 0u;  // rows past k are zeros in the image (an offset would make them something else)
+            if (gk + 2 * rp + 1 >= p.k) t1 = 0u;
+            tile[(wj * kCols + j) * 32 + at] = prmt(t0, t1, 0x5410);
+            tile[(wj * kCols + j + kPairs) * 32 + at] = prmt(t0, t1, 0x7632);
         }
     }
     __syncthreads();
-    uint32_t* out = reinterpret_cast<uint32_t*>(dst);
-    for (int e = tid; e < PN * (PK / 2); e += NT) {
-        const int nn = e >> 7, c = e & 127;
-        const int64_t on = n0 + nn, ok = k0 + 2 * c;
-        if (on < p.n && ok < kp) out[(on * kp + ok) >> 1] = ptile[nn * PP + (c ^ (((nn >> 3) & 3) | (((nn >> 5) & 1) << 4)))];
+#pragma unroll
+    for (int e = tid; e < kTileN * 8; e += NT) {
+        const int nn = e >> 3, c = e & 7, x = nn / kCols;  // column, 16-byte piece (8 k), its word column
+        const int64_t on = n0 + nn, ok = k0 + c * 8;
+        uint4 v = *reinterpret_cast<const uint4*>(&tile[nn * 32 + ((c ^ (x >> 2)) << 2)]);
+        if (x & 1) v = make_uint4(v.y, v.x, v.w, v.z);
+        if (x & 2) v = make_uint4(v.z, v.w, v.x, v.y);
+        if (on < p.n && ok < kp) *reinterpret_cast<uint4*>(dst + on * kp + ok) = v;
     }
 }
 
-// 8-bit weights (int8 / fp8) stored (k,n): a thread owns one 32-bit word (4 columns) over 4 consecutive k rows, the two row
+// Weight stored (n,k): the destination has the same orientation. A thread turns 32-bit words of a column into 16 (int4) or 8 bytes of
+// pairs, four words in flight, words of a warp side by side; a block is one column's stretch, so scales cost no division per word.
+// (n, k) = (18432, 7168) int4: 91 us one element at a time, 330 MB.
+template <MixW kW, bool kBf16, bool kOff>
+__global__ void __launch_bounds__(NT) wq_dequant_nk_kernel_fast(const OpsnnWqbmmParams p, uint16_t* __restrict__ dst, int64_t kp, float* __restrict__ one,
+                                                                uint32_t chunks)
+{
+    constexpr int kPer = kW == MixW::kInt4 ? 8 : 4;  // weights in a word
+    const uint32_t row = blockIdx.x / chunks, chunk = blockIdx.x - row * chunks;
+    if (blockIdx.x == 0 && threadIdx.x == 0) *one = 1.0f;
+    const uint32_t words = (uint32_t)(p.k / kPer), w0 = chunk * (4 * NT) + threadIdx.x, group = p.group_size > 0 ? (uint32_t)p.group_size : 0x7FFFFFFFu;
+    const uint32_t* src = reinterpret_cast<const uint32_t*>(static_cast<const uint8_t*>(p.w) + (int64_t)row * p.w_ld * (32 / kPer) / 8);
+    uint32_t w[4], sc[4], of[4];
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+        const uint32_t at = w0 + i * NT;
+        if (at >= words) continue;
+        w[i] = __ldcs(src + at);
+        const int64_t s = (int64_t)(at * kPer / group) * p.scale_sg + (int64_t)row * p.scale_sn;
+        sc[i] = __ldg(reinterpret_cast<const uint16_t*>(p.scale) + s);
+        of[i] = kOff ? __ldg(reinterpret_cast<const uint16_t*>(p.offset) + s) : 0u;
+    }
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+        const uint32_t at = w0 + i * NT;
+        if (at >= words) continue;
+        const uint32_t s2 = sc[i] | (sc[i] << 16), o2 = of[i] | (of[i] << 16);
+        uint32_t o[kPer / 2];
+#pragma unroll
+        for (int j = 0; j < kPer / 2; ++j) {
+            // weights 2 j and 2 j + 1: nibbles of byte j (it and the word shifted by four), or bytes 2 j and 2 j + 1
+            const uint32_t c = kW == MixW::kInt4 ? prmt(w[i], w[i] >> 4, (uint32_t)(j | ((4 + j) << 8))) : prmt(w[i], 0u, j == 0 ? 0x4140u : 0x4342u);
+            o[j] = mix_scale<kBf16, kOff>(mix_exact<kW, kBf16>(c), s2, o2);
+            if (kW == MixW::kE4m3) o[j] = fix_nan(o[j], c);
+        }
+        uint16_t* d = dst + (int64_t)row * kp + (int64_t)at * kPer;
+        if constexpr (kPer == 8) *reinterpret_cast<uint4*>(d) = make_uint4(o[0], o[1], o[2], o[3]);
+        else *reinterpret_cast<uint2*>(d) = make_uint2(o[0], o[1]);
+    }
+}
+
+template <MixW kW>
+void dequant_fast(const OpsnnWqbmmParams* p, uint16_t* dst, int64_t kp, float* one, cudaStream_t stream)
+{
+    constexpr int kPer = kW == MixW::kInt4 ? 8 : 4;
+    const bool bf = p->x_dtype == ACL_BF16, off = p->offset != nullptr;
+    auto go = [&](auto bf_c, auto off_c) {
+        constexpr bool kB = decltype(bf_c)::value, kO = decltype(off_c)::value && kW != MixW::kE4m3;
+        if (p->trans_w) {
+            const uint32_t chunks = (uint32_t)((p->k / kPer + 4 * NT - 1) / (4 * NT));
+            wq_dequant_nk_kernel_fast<kW, kB, kO><<<(unsigned)(p->n * chunks), NT, 0, stream>>>(*p, dst, kp, one, chunks);
+        } else {
+            const uint32_t tiles_n = (uint32_t)((p->n + 32 * kPer - 1) / (32 * kPer));
+            wq_dequant_kn_kernel<kW, kB, kO><<<(unsigned)(tiles_n * ((p->k + 63) / 64)), NT, 0, stream>>>(*p, dst, kp, one, tiles_n);
+        }
+    };
+    if (bf && off) go(std::true_type{}, std::true_type{});
+    else if (bf) go(std::true_type{}, std::false_type{});
+    else if (off) go(std::false_type{}, std::true_type{});
+    else go(std::false_type{}, std::false_type{});
+}
+
+// Layouts of the two kernels above.
+bool dequant_fast_takes(const OpsnnWqbmmParams* p)
+{
+    if (env("OPSNN_WQ_PREFILL_SIMPLE") || p->scale_dtype == ACL_FLOAT8_E8M0 || (reinterpret_cast<uintptr_t>(p->w) & 3) != 0) return false;
+    if (p->w_dtype != ACL_INT4 && p->w_dtype != ACL_INT8 && p->w_dtype != ACL_FLOAT8_E4M3FN) return false;
+    if (p->w_dtype == ACL_FLOAT8_E4M3FN && p->offset != nullptr) return false;
+    const int per = p->w_dtype == ACL_INT4 ? 8 : 4;
+    if (p->w_ld % per != 0 || p->k >= ((int64_t)1 << 30)) return false;
+    if (p->trans_w) return p->k % per == 0 && p->group_size % per == 0 && p->n * ((p->k / per + 4 * NT - 1) / (4 * NT)) <= 0x7FFFFFFF;
+    return p->n % per == 0 && p->group_size % 8 == 0 && ((p->n + 32 * per - 1) / (32 * per)) * ((p->k + 63) / 64) <= 0x7FFFFFFF;
+}
+
+// fp8 weights stored (k,n) that the kernels above do not take (e5m2, or with an offset): a thread owns one 32-bit word (4 columns) over 4 consecutive k rows, the two row
 // pairs of a column leave as packed words; 64 x 64 tile with 33-word rows. Needs n % 4 == 0, word-aligned rows,
 // group_size % 4 == 0 and scales in x's dtype.
 template <bool kBf16>
@@ -261,14 +268,13 @@ __global__ void __launch_bounds__(NT) wq_dequant_nk_bytes_kernel(const OpsnnWqbm
             of[j] = has_off ? load_x<kBf16>(p.offset, sidx + j * p.scale_sn) : 0.f;
         }
     }
-    const bool is_int = p.w_dtype == ACL_INT8;
 #pragma unroll
     for (int j = 0; j < 4; ++j) {
         float v[4];
 #pragma unroll
         for (int i = 0; i < 4; ++i) {
             const uint32_t byte = (w[i] >> (8 * j)) & 0xFFu;
-            v[i] = is_int ? (float)(int8_t)byte : fp8_to_float((uint8_t)byte, p.w_dtype);
+            v[i] = fp8_to_float((uint8_t)byte, p.w_dtype);
         }
 #pragma unroll
         for (int h = 0; h < 2; ++h) {
@@ -290,7 +296,7 @@ __global__ void __launch_bounds__(NT) wq_dequant_nk_bytes_kernel(const OpsnnWqbm
     }
 }
 
-// Weight stored (n,k) (the transposed-view case, e.g. a torch Linear weight): the destination has the same orientation, so a
+// fp4 / fp8 weight stored (n,k) that the kernel above does not take: the destination has the same orientation, so a
 // thread dequantises one 32-bit word - kPer consecutive k of one column (8 for 4-bit, 4 for 8-bit weights) - and stores it as
 // one 16- / 8-byte piece. One scale / offset per word (groups are multiples of kPer, or per-channel).
 template <bool kBf16, int kPer>
@@ -312,17 +318,12 @@ __global__ void __launch_bounds__(NT) wq_dequant_nk_rows_kernel(const OpsnnWqbmm
             float a, b;
             if (kPer == 8) {
                 const uint32_t n0 = (word >> (8 * h)) & 0xFu, n1 = (word >> (8 * h + 4)) & 0xFu;
-                if (p.w_dtype == ACL_INT4) {
-                    a = (float)((int)(n0 ^ 8u) - 8);
-                    b = (float)((int)(n1 ^ 8u) - 8);
-                } else {
-                    a = fp4_e2m1_to_float((uint8_t)n0);
-                    b = fp4_e2m1_to_float((uint8_t)n1);
-                }
+                a = fp4_e2m1_to_float((uint8_t)n0);
+                b = fp4_e2m1_to_float((uint8_t)n1);
             } else {
                 const uint32_t b0 = (word >> (16 * h)) & 0xFFu, b1 = (word >> (16 * h + 8)) & 0xFFu;
-                a = p.w_dtype == ACL_INT8 ? (float)(int8_t)b0 : fp8_to_float((uint8_t)b0, p.w_dtype);
-                b = p.w_dtype == ACL_INT8 ? (float)(int8_t)b1 : fp8_to_float((uint8_t)b1, p.w_dtype);
+                a = fp8_to_float((uint8_t)b0, p.w_dtype);
+                b = fp8_to_float((uint8_t)b1, p.w_dtype);
             }
             if (has_off) {
                 const float2 r = unpack2<kBf16>(pack2<kBf16>(__fadd_rn(a, of), __fadd_rn(b, of)));
@@ -390,20 +391,17 @@ int32_t wqbmm_prefill_prepass(const OpsnnWqbmmParams* p, uint8_t* ws, cudaStream
     float* one = reinterpret_cast<float*>(ws + (((uint64_t)p->n * kp * 2u + 15u) & ~(uint64_t)15u));
     const int64_t tiles = ((p->n + TN - 1) / TN) * ((p->k + TK - 1) / TK);
     if (tiles > 0x7FFFFFFF) return (int32_t)cudaErrorInvalidConfiguration;
-    const bool tile_const_scale = p->group_size == 0 || p->group_size % TK == 0;
-    const bool fast = p->w_dtype == ACL_INT4 && !p->trans_w && p->w_ld % 8 == 0 && p->n % 8 == 0 &&
-                      (reinterpret_cast<uintptr_t>(p->w) & 3) == 0 && tile_const_scale && p->scale_dtype != ACL_FLOAT8_E8M0;
     const bool bf = p->x_dtype == ACL_BF16;
-    const bool pairs = p->w_dtype == ACL_INT4 && !p->trans_w && p->w_ld % 8 == 0 && p->n % 8 == 0 &&
-                       (reinterpret_cast<uintptr_t>(p->w) & 3) == 0 && (p->group_size == 0 || p->group_size % 8 == 0) &&
-                       p->scale_dtype != ACL_FLOAT8_E8M0 &&
-                       env("OPSNN_WQ_PREFILL_SIMPLE") == nullptr;
-    const bool four = p->w_dtype == ACL_INT4 || p->w_dtype == ACL_FLOAT4_E2M1;
+    const bool four = p->w_dtype == ACL_FLOAT4_E2M1, fp8 = p->w_dtype == ACL_FLOAT8_E4M3FN || p->w_dtype == ACL_FLOAT8_E5M2;
     const int per = four ? 8 : 4;
-    const bool rows_path = p->trans_w && p->k % per == 0 && p->w_ld % per == 0 && (p->group_size == 0 || p->group_size % per == 0) &&
+    const bool rows_path = (four || fp8) && p->trans_w && p->k % per == 0 && p->w_ld % per == 0 && (p->group_size == 0 || p->group_size % per == 0) &&
                            p->scale_dtype != ACL_FLOAT8_E8M0 && (reinterpret_cast<uintptr_t>(p->w) & 3) == 0 &&
                            env("OPSNN_WQ_PREFILL_SIMPLE") == nullptr;
-    if (rows_path) {
+    if (dequant_fast_takes(p)) {
+        if (p->w_dtype == ACL_INT4) dequant_fast<MixW::kInt4>(p, wdeq, kp, one, stream);
+        else if (p->w_dtype == ACL_INT8) dequant_fast<MixW::kInt8>(p, wdeq, kp, one, stream);
+        else dequant_fast<MixW::kE4m3>(p, wdeq, kp, one, stream);
+    } else if (rows_path) {
         const int64_t work = p->n * (p->k / per);
         int64_t grid = (work + NT - 1) / NT;
         if (grid > 148 * 32) grid = 148 * 32;
@@ -412,28 +410,13 @@ int32_t wqbmm_prefill_prepass(const OpsnnWqbmmParams* p, uint8_t* ws, cudaStream
         else if (bf) wq_dequant_nk_rows_kernel<true, 4><<<(unsigned)grid, NT, 0, stream>>>(*p, wdeq, kp, one);
         else if (four) wq_dequant_nk_rows_kernel<false, 8><<<(unsigned)grid, NT, 0, stream>>>(*p, wdeq, kp, one);
         else wq_dequant_nk_rows_kernel<false, 4><<<(unsigned)grid, NT, 0, stream>>>(*p, wdeq, kp, one);
-    } else if (pairs) {
-        const int64_t ptiles = ((p->n + PN - 1) / PN) * ((p->k + PK - 1) / PK);
-        if (ptiles > 0x7FFFFFFF) return (int32_t)cudaErrorInvalidConfiguration;
-        const int vec = p->scale_sn == 1 && p->scale_sg % 8 == 0 && (reinterpret_cast<uintptr_t>(p->scale) & 15) == 0 &&
-                        (p->offset == nullptr || (reinterpret_cast<uintptr_t>(p->offset) & 15) == 0);
-        const size_t sm = (size_t)PN * PP * 4;
-        static std::atomic<uint64_t> configured{0};
-        once_per_device(configured, [&] {
-            cudaFuncSetAttribute(wq_dequant_nk_pairs_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
-            return cudaFuncSetAttribute(wq_dequant_nk_pairs_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
-        });
-        if (bf) wq_dequant_nk_pairs_kernel<true><<<(unsigned)ptiles, NT, sm, stream>>>(*p, wdeq, kp, one, vec);
-        else wq_dequant_nk_pairs_kernel<false><<<(unsigned)ptiles, NT, sm, stream>>>(*p, wdeq, kp, one, vec);
-    } else if ((p->w_dtype == ACL_INT8 || p->w_dtype == ACL_FLOAT8_E4M3FN || p->w_dtype == ACL_FLOAT8_E5M2) && !p->trans_w &&
+    } else if (fp8 && !p->trans_w &&
                p->n % 4 == 0 && p->w_ld % 4 == 0 && (reinterpret_cast<uintptr_t>(p->w) & 3) == 0 &&
                (p->group_size == 0 || p->group_size % 4 == 0) && p->scale_dtype != ACL_FLOAT8_E8M0 &&
                env("OPSNN_WQ_PREFILL_SIMPLE") == nullptr) {
         if (bf) wq_dequant_nk_bytes_kernel<true><<<(unsigned)tiles, NT, 0, stream>>>(*p, wdeq, kp, one);
         else wq_dequant_nk_bytes_kernel<false><<<(unsigned)tiles, NT, 0, stream>>>(*p, wdeq, kp, one);
-    } else if (bf && fast) wq_dequant_nk_words_kernel<true><<<(unsigned)tiles, NT, 0, stream>>>(*p, wdeq, kp, one);
-    else if (bf) wq_dequant_nk_kernel<true><<<(unsigned)tiles, NT, 0, stream>>>(*p, wdeq, kp, one);
-    else if (fast) wq_dequant_nk_words_kernel<false><<<(unsigned)tiles, NT, 0, stream>>>(*p, wdeq, kp, one);
+    } else if (bf) wq_dequant_nk_kernel<true><<<(unsigned)tiles, NT, 0, stream>>>(*p, wdeq, kp, one);
     else wq_dequant_nk_kernel<false><<<(unsigned)tiles, NT, 0, stream>>>(*p, wdeq, kp, one);
     note_launch("wq_dequant_nk");
     return (int32_t)cudaGetLastError();

@@ -28,8 +28,30 @@ CASES = [
 ]
 
 
+# Small weights, which the fused kernel leaves to the dequantisation pre-pass (16-bit image of the weight, then the dense matmul)
+IMAGE_CASES = [
+    ("int4", False, "bfloat16", 20, 1000, 256, 0, True, False),       # k tile of 40 rows, one tile of 256 columns
+    ("int4", False, "float16", 33, 992, 264, 32, True, True),         # last tile of one word, groups within a tile
+    ("int4", True, "bfloat16", 40, 992, 264, 32, True, False),
+    ("int4", True, "float16", 18, 8200, 24, 0, False, True),          # two stretches a row, the second of one word
+    ("int8", False, "bfloat16", 50, 328, 132, 0, True, False),        # last tile of one word
+    ("int8", True, "float16", 17, 4104, 36, 0, True, True),
+    ("e4m3", False, "bfloat16", 40, 448, 388, 64, False, False),
+    ("e4m3", True, "bfloat16", 24, 480, 304, 32, False, True),
+]
+
+
+@pytest.mark.parametrize("case", IMAGE_CASES, ids=[str(c) for c in IMAGE_CASES])
+def test_dequantised_image_equals_oracle(aclnn, case):
+    _against_oracle(aclnn, case, ("qmm_umma_deq", "qmm_umma_pair_deq", "qmm_umma_split_deq"))
+
+
 @pytest.mark.parametrize("case", CASES, ids=[str(c) for c in CASES])
 def test_mixed_kernel_equals_oracle(aclnn, case):
+    _against_oracle(aclnn, case, ("wqbmm_decode" if case[0] == "int4" else "wqbmm_decode8",))
+
+
+def _against_oracle(aclnn, case, kernels):
     import torch
 
     from gpu_util import desc, out_tensor, out_to_np
@@ -73,7 +95,7 @@ def test_mixed_kernel_equals_oracle(aclnn, case):
                                         inner_precise=0)
         torch.cuda.synchronize()
         outs.append(out_to_np(out))
-    assert aclnn.last_kernel_name() == ("wqbmm_decode" if kind == "int4" else "wqbmm_decode8"), aclnn.last_kernel_name()
+    assert aclnn.last_kernel_name() in kernels, aclnn.last_kernel_name()
     assert np.array_equal(outs[0].view(np.uint16), outs[1].view(np.uint16))
     got = outs[0].astype(np.float64)
     assert np.array_equal(np.isnan(got), np.isnan(want)) and sorted(set(np.nonzero(np.isnan(want[0]))[0])) == sorted(nan_cols)
