@@ -110,6 +110,24 @@ __device__ __forceinline__ void report(volatile uint32_t* abort_flag, unsigned i
     }
 }
 
+// 32 floats as 16 packed pairs of the 16-bit output type.
+__device__ __forceinline__ void pack16(int32_t dtype, const float (&f)[32], uint32_t (&pk)[16])
+{
+    if (dtype == ACL_BF16) {
+#pragma unroll
+        for (int i = 0; i < 16; ++i) {
+            __nv_bfloat162 h = __floats2bfloat162_rn(f[2 * i], f[2 * i + 1]);
+            pk[i] = *reinterpret_cast<uint32_t*>(&h);
+        }
+    } else {
+#pragma unroll
+        for (int i = 0; i < 16; ++i) {
+            __half2 h = __floats2half2_rn(f[2 * i], f[2 * i + 1]);
+            pk[i] = *reinterpret_cast<uint32_t*>(&h);
+        }
+    }
+}
+
 // Converts 32 accumulator columns of one output row and stores them. `col` is the first column (global), valid = number
 // of columns inside n. Register arrays are only ever indexed with compile-time constants (a run-time index would move
 // them to local memory).
@@ -147,19 +165,7 @@ __device__ __forceinline__ void store_row32(const UmmaArgs& a, uint8_t* out, int
         return;
     }
     uint32_t pk[16];
-    if (a.out_dtype == ACL_BF16) {
-#pragma unroll
-        for (int i = 0; i < 16; ++i) {
-            __nv_bfloat162 h = __floats2bfloat162_rn(f[2 * i], f[2 * i + 1]);
-            pk[i] = *reinterpret_cast<uint32_t*>(&h);
-        }
-    } else {
-#pragma unroll
-        for (int i = 0; i < 16; ++i) {
-            __half2 h = __floats2half2_rn(f[2 * i], f[2 * i + 1]);
-            pk[i] = *reinterpret_cast<uint32_t*>(&h);
-        }
-    }
+    pack16(a.out_dtype, f, pk);
     uint16_t* o = reinterpret_cast<uint16_t*>(out) + row * a.out_ld + col;
     if (valid == 32 && (reinterpret_cast<uintptr_t>(o) & 15) == 0) {
 #pragma unroll
@@ -1068,10 +1074,3 @@ extern "C" __attribute__((visibility("default"))) uint32_t opsnn_qmm_umma_status
     }
     return v;
 }
-
-#ifdef OPSNN_PB_DIAG
-extern "C" __attribute__((visibility("default"))) int32_t opsnn_pb_diag(unsigned long long* host_out, int32_t ctas)
-{
-    return (int32_t)cudaMemcpyFromSymbol(host_out, opsnn::g_pb_diag, (size_t)ctas * 5 * sizeof(unsigned long long));
-}
-#endif

@@ -18,21 +18,26 @@
 // All waits bounded, teardown through a cluster barrier, as in qmm_umma_pair.cuh.
 namespace {
 
+// Two neighbouring columns; fp8's fused multiply-adds go as one packed instruction (each half rounded on its own).
+template <ptx::MmaKind kKind>
+__device__ __forceinline__ void promote2(uint32_t v0, uint32_t v1, float sc, float& a0, float& a1)
+{
+#ifdef X2
+    if constexpr (kKind != ptx::MmaKind::kI8) {
+        asm("{\n\t.reg .b64 a, v, s;\n\tmov.b64 a, {%0, %1};\n\tmov.b64 v, {%2, %3};\n\tmov.b64 s, {%4, %4};\n\tfma.rn.f32x2 a, v, s, a;\n\tmov.b64 {%0, %1}, a;\n\t}"
+            : "+f"(a0), "+f"(a1)
+            : "r"(v0), "r"(v1), "f"(sc));
+        return;
+    }
+#endif
+    a0 = promote<kKind>(v0, sc, a0);
+    a1 = promote<kKind>(v1, sc, a1);
+}
+
 // 256-column tiles: 128 sums per epilogue thread need more registers than an even split of the register file over the CTA's
 // warps gives (168 with ten warps), so the block is three whole warpgroups - epilogue warps 0..7, then {producer, MMA issuer, two
 // idle warps} - and setmaxnreg moves registers from the third group (40 each) to the first two (232 each): per scheduler
 // 2 x 232 + 40 = 504 of the 512 registers per lane.
-#ifdef OPSNN_PB_DIAG
-// Diagnostic builds only: clocks the MMA issuer spent waiting for a free accumulator buffer / for operands, and its total; clocks
-// epilogue warp 0 spent waiting for a full buffer, and its total. [CTA][5]
-__device__ unsigned long long g_pb_diag[1024 * 5];
-#define OPSNN_PB_T(var) const long long var = clock64()
-#define OPSNN_PB_ADD(acc, t0) acc += clock64() - (t0)
-#else
-#define OPSNN_PB_T(var) do { } while (0)
-#define OPSNN_PB_ADD(acc, t0) do { } while (0)
-#endif
-
 // (Code that runs under setmaxnreg cannot call an out-of-line function: the bounded spin is inlined for those instances.)
 template <bool kInline>
 __device__ __forceinline__ bool pb_wait(uint32_t bar_addr, uint32_t parity, volatile uint32_t* abort_flag)
@@ -48,8 +53,10 @@ __device__ __forceinline__ bool pb_wait(uint32_t bar_addr, uint32_t parity, vola
     return false;
 }
 
-template <int EW, int BN>
-constexpr int pair_pb_threads() { return (EW + (BN == 256 ? 4 : 2)) * 32; }
+template <int EW, bool kAsym>
+constexpr int pair_pb_threads() { return (EW + (kAsym ? 2 : 4)) * 32; }
+
+constexpr int kPbScaleRun = 4;  // k-blocks of scales per buffer of the ring
 
 // kAsym: INT4 x INT4 asymmetric per-group (quant_batch_matmul_v4_pertoken_pergroup.h; golden qbmmv4_kernel_golden.py:328-395), both
 // operands widened to INT8 beforehand. An accumulation group is two k-blocks (256 of k); per group and element
@@ -58,12 +65,17 @@ constexpr int pair_pb_threads() { return (EW + (BN == 256 ? 4 : 2)) * 32; }
 // group ahead (three buffers, one named barrier per group whose reduced predicate also carries the abort flag, so that the
 // epilogue warps can only leave together).
 template <ptx::MmaKind kKind, int EW, int BN, bool kAsym = false>
-__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(pair_pb_threads<EW, BN>(), 1)
+__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(pair_pb_threads<EW, kAsym>(), 1)
 qmm_umma_pair_pb_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b, const UmmaArgs a)
 {
     static_assert(BN == 128 || (BN == 256 && EW == 8), "256-column tiles keep 128 sums per thread: eight epilogue warps");
     static_assert(!kAsym || (BN == 128 && EW == 4 && kKind == ptx::MmaKind::kI8), "the asymmetric per-group epilogue: int8, 128 columns, four warps");
     __shared__ float s_cols[kAsym ? 3 * 2 * BN : 1];  // kAsym: [buffer][offset | scale][column]
+    // otherwise: scales of a run of k-blocks, two buffers ([k-block][row], then [k-block][128-column block]), and 2 KB per epilogue warp
+    // through which its rows leave as 64-byte pieces
+    __shared__ __align__(16) float s_scale[kAsym ? 1 : 2][kAsym ? 1 : kPbScaleRun * 130];
+    __shared__ __align__(16) uint8_t s_out[kAsym ? 16 : EW * 2048];
+    __shared__ uint64_t s_bars[4];  // scale buffers: [2] full, [2] empty
     constexpr int NBUF = 512 / BN;              // accumulator buffers in the 512 TMEM columns
     constexpr int kCols = BN * 4 / EW;          // accumulator columns per epilogue thread
     constexpr uint32_t kBHalf = (BN / 2) * BK;  // this CTA's half of the B tile
@@ -94,6 +106,10 @@ qmm_umma_pair_pb_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_
             ptx::mbar_init(&tfull[b], 1);
             ptx::mbar_init(&tempty[b], 2 * EW);
         }
+        for (int b = 0; b < 2; ++b) {
+            ptx::mbar_init(&s_bars[b], 2);       // two loading warps
+            ptx::mbar_init(&s_bars[2 + b], EW);  // the epilogue warps
+        }
         *abort_flag = 0u;
         ptx::fence_mbar_init();
     }
@@ -110,6 +126,7 @@ qmm_umma_pair_pb_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_
     const uint32_t smem0 = ptx::smem_u32(smem), full0 = ptx::smem_u32(full), empty0 = ptx::smem_u32(empty);
     const uint32_t tfull0 = ptx::smem_u32(tfull), tempty0 = ptx::smem_u32(tempty);
     const uint32_t stages = (uint32_t)a.stages;
+    const uint32_t sfull0 = ptx::smem_u32(s_bars), sempty0 = sfull0 + 16u;
     const int kblocks = a.kblocks;
 
     if (warp == EW) {
@@ -170,26 +187,20 @@ qmm_umma_pair_pb_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_
             const uint64_t a_hi = da0 & 0xFFFFFFFF00000000ull, b_hi = db0 & 0xFFFFFFFF00000000ull;
             const uint32_t a_k1 = a.a_mn_major ? 256u : 2u, b_k1 = a.b_mn_major ? (BN == 128 ? 128u : 256u) : 2u;
             const uint32_t idesc = a.idesc;
-            long long d_tempty = 0, d_full = 0;
-            OPSNN_PB_T(d_start);
             for (uint32_t tile = pair; tile < ntiles && ok; tile += npairs) {
                 for (int kb = 0; kb < kblocks; ++kb) {
                     // kAsym: k-blocks 2g and 2g + 1 accumulate into one buffer; otherwise every k-block is its own group
                     const bool first = !kAsym || (kb & 1) == 0, last = !kAsym || (kb & 1) == 1 || kb == kblocks - 1;
-                    OPSNN_PB_T(d_t0);
                     if (first && !pb_wait<BN == 256>(tempty0 + 8u * buf, bpar ^ 1u, abort_flag)) {
                         report(abort_flag, (2u << 8) | 1u);
                         ok = false;
                         break;
                     }
-                    OPSNN_PB_ADD(d_tempty, d_t0);
-                    OPSNN_PB_T(d_t1);
                     if (!pb_wait<BN == 256>(full0 + 8u * s, par, abort_flag)) {
                         report(abort_flag, (2u << 8) | 2u);
                         ok = false;
                         break;
                     }
-                    OPSNN_PB_ADD(d_full, d_t1);
                     ptx::tc_fence_after();
                     if (ptx::elect_one()) {
                         const uint32_t stage_off = (s * kStage) >> 4;
@@ -213,15 +224,6 @@ qmm_umma_pair_pb_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_
                     }
                 }
             }
-#ifdef OPSNN_PB_DIAG
-            if (lane == 0) {
-                g_pb_diag[blockIdx.x * 5 + 0] = (unsigned long long)d_tempty;
-                g_pb_diag[blockIdx.x * 5 + 1] = (unsigned long long)d_full;
-                g_pb_diag[blockIdx.x * 5 + 2] = (unsigned long long)(clock64() - d_start);
-            }
-#endif
-            (void)d_tempty;
-            (void)d_full;
         }
     } else if (warp < EW) {
         // ======================= epilogue warps (both CTAs): own 128 rows, kCols columns each =======================
@@ -229,10 +231,8 @@ qmm_umma_pair_pb_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_
         const int quad = warp & 3, part = warp >> 2;
         const uint32_t lane_addr = ((uint32_t)(quad * 32) << 16) + (uint32_t)(part * kCols);
         const uint32_t lead_tempty0 = tempty0 & ptx::kPeerBitMask;
-        uint32_t buf = 0, bpar = 0;
+        uint32_t buf = 0, bpar = 0, sbuf = 0, spar = 0;
         bool ok = true;
-        long long d_tfull = 0;
-        OPSNN_PB_T(d_estart);
         for (uint32_t tile = pair; tile < ntiles && ok; tile += npairs) {
             const uint32_t b = tile / tiles_per_batch, r = tile % tiles_per_batch;
             uint32_t tm, tn;
@@ -329,87 +329,100 @@ qmm_umma_pair_pb_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_
                     for (int i = 0; i < kCols; ++i) acc[i] = __fmul_rn(acc[i], sa);
                 }
             } else {
-                const float* s1 = reinterpret_cast<const float*>(a.scale_a) + b * a.sa_bs;
-                const float* s2 = reinterpret_cast<const float*>(a.scale_b) + b * a.sb_bs;
-                const int64_t mg = (row_ok ? row : 0) / a.group_m;
-                const int64_t n_mg = (a.m + a.group_m - 1) / a.group_m, n_ng = (a.n + 127) / 128;
-                const int64_t ng = min(colbase / 128, n_ng - 1);
-                auto load_s1 = [&](int kb) {
-                    kb = min(kb, a.kblocks - 1);
-                    return a.trans_a ? __ldg(s1 + kb * n_mg + mg) : __ldg(s1 + mg * a.kblocks + kb);
-                };
-                auto load_s2 = [&](int kb) {
-                    kb = min(kb, a.kblocks - 1);
-                    return a.trans_b ? __ldg(s2 + ng * a.kblocks + kb) : __ldg(s2 + kb * n_ng + ng);
-                };
-                float s1_next[4], s2_next[4];  // raw scales of the next four k-blocks; multiplied when their turn comes
-    #pragma unroll
-                for (int j = 0; j < 4; ++j) {
-                    s1_next[j] = load_s1(j);
-                    s2_next[j] = load_s2(j);
-                }
-                for (int kb0 = 0; kb0 < a.kblocks && ok; kb0 += 4) {
-                    float sc_cur[4];
-    #pragma unroll
-                    for (int j = 0; j < 4; ++j) sc_cur[j] = __fmul_rn(s1_next[j], s2_next[j]);
-    #pragma unroll
-                    for (int j = 0; j < 4; ++j) {
-                        s1_next[j] = load_s1(kb0 + 4 + j);
-                        s2_next[j] = load_s2(kb0 + 4 + j);
+                const uint32_t nb = (uint32_t)(part * kCols) >> 7;  // 128-column block of the tile
+                for (int kb = 0; kb < kblocks; ++kb) {
+                    const int j = kb % kPbScaleRun;
+                    if (j == 0 && !__all_sync(0xffffffffu, pb_wait<BN == 256>(sfull0 + 8u * sbuf, spar, abort_flag))) {
+                        report(abort_flag, (3u << 8) | 3u);
+                        ok = false;
+                        break;
                     }
-    #pragma unroll
-                    for (int j = 0; j < 4; ++j) {
-                        if (kb0 + j >= a.kblocks) break;
-                        const float sc = sc_cur[j];
-                        OPSNN_PB_T(d_t2);
-                        if (!pb_wait<BN == 256>(tfull0 + 8u * buf, bpar, abort_flag)) {
-                            report(abort_flag, (3u << 8) | 2u);
-                            ok = false;
-                            break;
+                    const float sc = __fmul_rn(s_scale[sbuf][j * 128 + quad * 32 + lane], s_scale[sbuf][kPbScaleRun * 128 + 2 * j + nb]);
+                    if (!__all_sync(0xffffffffu, pb_wait<BN == 256>(tfull0 + 8u * buf, bpar, abort_flag))) {
+                        report(abort_flag, (3u << 8) | 2u);
+                        ok = false;
+                        break;
+                    }
+                    ptx::tc_fence_after();
+#ifndef PBW
+#define PBW 16
+#endif
+                    constexpr int W = PBW;  // staging registers per TMEM load (two sets in flight)
+                    const uint32_t t0 = tmem_base + lane_addr + buf * BN;
+                    uint32_t va[W], vb[W];
+                    ptx::tmem_ld_n(t0, va);
+#pragma unroll
+                    for (int c = 0; c < kCols; c += 2 * W) {
+                        ptx::tmem_ld_wait();
+                        ptx::tmem_ld_n(t0 + c + W, vb);
+#pragma unroll
+                        for (int i = 0; i < W; i += 2) promote2<kKind>(va[i], va[i + 1], sc, acc[c + i], acc[c + i + 1]);
+                        ptx::tmem_ld_wait();
+                        if (c + 2 * W < kCols) {
+                            ptx::tmem_ld_n(t0 + c + 2 * W, va);
+                        } else {
+                            ptx::tc_fence_before();
+                            __syncwarp();
+                            if (lane == 0) ptx::mbar_arrive_cluster(lead_tempty0 + 8u * buf);
                         }
-                        OPSNN_PB_ADD(d_tfull, d_t2);
-                        ptx::tc_fence_after();
-    #if defined(OPSNN_PB_EXPERIMENT) && OPSNN_PB_EXPERIMENT == 1
-                        // diagnostic build: the buffer is released unread (main loop alone)
-                        ptx::tc_fence_before();
+#pragma unroll
+                        for (int i = 0; i < W; i += 2) promote2<kKind>(vb[i], vb[i + 1], sc, acc[c + W + i], acc[c + W + i + 1]);
+                    }
+                    if (++buf == NBUF) {
+                        buf = 0;
+                        bpar ^= 1u;
+                    }
+                    if (j == kPbScaleRun - 1 || kb == kblocks - 1) {
                         __syncwarp();
-                        if (lane == 0) ptx::mbar_arrive_cluster(lead_tempty0 + 8u * buf);
-                        if (++buf == NBUF) {
-                            buf = 0;
-                            bpar ^= 1u;
+                        if (lane == 0) ptx::mbar_arrive(&s_bars[2 + sbuf]);
+                        sbuf ^= 1u;
+                        if (sbuf == 0u) spar ^= 1u;
+                    }
+                }
+            }
+            if constexpr (!kAsym) {
+                // Whole tiles with 16-byte rows: a thread's row goes through shared memory and leaves with its neighbours as 64-byte
+                // pieces (pieces of a row XOR-swizzled by the row pair: no bank conflicts either way).
+                const int es = out_elem_bytes(a.out_dtype);
+                if (ok && colbase + kCols <= a.n && ((reinterpret_cast<uintptr_t>(out) | (uintptr_t)(a.out_ld * es)) & 15) == 0) {
+                    uint8_t* st = s_out + warp * 2048;
+                    const uint8_t* bias = a.bias == nullptr ? nullptr : reinterpret_cast<const uint8_t*>(a.bias) +
+                                              b * a.bias_bs * ((a.bias_dtype == ACL_FLOAT || a.bias_dtype == ACL_INT32) ? 4 : 2);
+                    auto piece = [&](int p) { return st + lane * 64 + ((p ^ ((lane >> 1) & 3)) << 4); };
+                    uint8_t* orow = out + (m0 + quad * 32 + (lane >> 2)) * a.out_ld * es + colbase * es + (lane & 3) * 16;
+                    const int64_t rows_left = a.m - (m0 + quad * 32 + (lane >> 2));
+                    auto flush = [&](int c) {  // the warp's 32 rows x 64 bytes, from column c
+                        __syncwarp();
+#pragma unroll
+                        for (int i = 0; i < 4; ++i) {
+                            const int r = (lane >> 2) + 8 * i;
+                            const uint4 v = *reinterpret_cast<const uint4*>(st + r * 64 + (((lane & 3) ^ ((r >> 1) & 3)) << 4));
+                            if (8 * i < rows_left) *reinterpret_cast<uint4*>(orow + (int64_t)(8 * i) * a.out_ld * es + c * es) = v;
                         }
-                        acc[0] += sc;
-                        continue;
-    #endif
-    #ifndef OPSNN_PB256_W
-    #define OPSNN_PB256_W 16
-    #endif
-                        constexpr int W = BN == 256 ? OPSNN_PB256_W : 16;  // staging registers per TMEM load (two sets in flight)
-                        const uint32_t t0 = tmem_base + lane_addr + buf * BN;
-                        uint32_t va[W], vb[W];
-                        ptx::tmem_ld_n(t0, va);
-    #pragma unroll
-                        for (int c = 0; c < kCols; c += 2 * W) {
-                            ptx::tmem_ld_wait();
-                            ptx::tmem_ld_n(t0 + c + W, vb);
-    #pragma unroll
-                            for (int i = 0; i < W; ++i) acc[c + i] = promote<kKind>(va[i], sc, acc[c + i]);
-                            ptx::tmem_ld_wait();
-                            if (c + 2 * W < kCols) {
-                                ptx::tmem_ld_n(t0 + c + 2 * W, va);
-                            } else {
-                                ptx::tc_fence_before();
-                                __syncwarp();
-                                if (lane == 0) ptx::mbar_arrive_cluster(lead_tempty0 + 8u * buf);
+                        __syncwarp();
+                    };
+#pragma unroll
+                    for (int c = 0; c < kCols; c += 32) {
+                        float f[32];
+#pragma unroll
+                        for (int i = 0; i < 32; ++i) f[i] = bias == nullptr ? acc[c + i] : __fadd_rn(acc[c + i], load_as_float(bias, colbase + c + i, a.bias_dtype));
+                        if (a.out_dtype == ACL_FLOAT) {
+#pragma unroll
+                            for (int h = 0; h < 32; h += 16) {
+#pragma unroll
+                                for (int i = 0; i < 4; ++i)
+                                    *reinterpret_cast<float4*>(piece(i)) = make_float4(f[h + 4 * i], f[h + 4 * i + 1], f[h + 4 * i + 2], f[h + 4 * i + 3]);
+                                flush(c + h);
                             }
-    #pragma unroll
-                            for (int i = 0; i < W; ++i) acc[c + W + i] = promote<kKind>(vb[i], sc, acc[c + W + i]);
-                        }
-                        if (++buf == NBUF) {
-                            buf = 0;
-                            bpar ^= 1u;
+                        } else {
+                            uint32_t pk[16];
+                            pack16(a.out_dtype, f, pk);
+#pragma unroll
+                            for (int i = 0; i < 4; ++i) *reinterpret_cast<uint4*>(piece(i)) = make_uint4(pk[4 * i], pk[4 * i + 1], pk[4 * i + 2], pk[4 * i + 3]);
+                            flush(c);
                         }
                     }
+                    continue;
                 }
             }
             if (ok && row_ok) {
@@ -433,20 +446,61 @@ qmm_umma_pair_pb_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_
                 }
             }
         }
-#ifdef OPSNN_PB_DIAG
-        if (warp == 0 && lane == 0) {
-            g_pb_diag[blockIdx.x * 5 + 3] = (unsigned long long)d_tfull;
-            g_pb_diag[blockIdx.x * 5 + 4] = (unsigned long long)(clock64() - d_estart);
+    } else if constexpr (!kAsym) {
+        // ======================= scale loaders (two warps): s1 of this CTA's 128 rows, s2 of the tile's column blocks =======================
+        if (BN == 256) asm volatile("setmaxnreg.dec.sync.aligned.u32 40;");
+        const int t = (int)threadIdx.x - (EW + 2) * 32;  // 0 .. 63: rows t and t + 64
+        const uint32_t n_mg = (uint32_t)((a.m + a.group_m - 1) / a.group_m), n_ng = (uint32_t)((a.n + 127) / 128);
+        const uint32_t rs = a.trans_a ? 1u : (uint32_t)kblocks, ks = a.trans_a ? n_mg : 1u;  // strides of s1 per row group and per k-block
+        const bool vec = !a.trans_a && kblocks % 4 == 0 && (reinterpret_cast<uintptr_t>(a.scale_a) & 15) == 0 && (a.sa_bs & 3) == 0;
+        uint32_t sbuf = 0, spar = 0;
+        bool ok = true;
+        for (uint32_t tile = pair; tile < ntiles && ok; tile += npairs) {
+            const uint32_t b = tile / tiles_per_batch, r = tile % tiles_per_batch;
+            uint32_t tm, tn;
+            tile_of<8>(r, (uint32_t)a.tiles_m, (uint32_t)a.tiles_n, tm, tn);
+            const uint32_t row = tm * 256u + rank * 128u + (uint32_t)t, last = (uint32_t)a.m - 1u;
+            const float* s1 = reinterpret_cast<const float*>(a.scale_a) + b * a.sa_bs;
+            const float* r0 = s1 + (int64_t)(min(row, last) / (uint32_t)a.group_m) * rs;
+            const float* r1 = s1 + (int64_t)(min(row + 64u, last) / (uint32_t)a.group_m) * rs;
+            // the first threads: s2 of k-block t / 2 of the run, column block t % 2
+            const uint32_t ng = min(tn * (BN / 128) + (uint32_t)(t & 1), n_ng - 1u);
+            const float* s2 = reinterpret_cast<const float*>(a.scale_b) + b * a.sb_bs + (a.trans_b ? (int64_t)ng * kblocks : (int64_t)ng);
+            const uint32_t s2k = a.trans_b ? 1u : n_ng;
+            for (int kb = 0; kb < kblocks; kb += kPbScaleRun) {
+                float v0[kPbScaleRun], v1[kPbScaleRun], w = 0.f;
+                if (vec) {
+                    const float4 x = __ldg(reinterpret_cast<const float4*>(r0 + kb)), y = __ldg(reinterpret_cast<const float4*>(r1 + kb));
+                    v0[0] = x.x; v0[1] = x.y; v0[2] = x.z; v0[3] = x.w;
+                    v1[0] = y.x; v1[1] = y.y; v1[2] = y.z; v1[3] = y.w;
+                } else {
+#pragma unroll
+                    for (int h = 0; h < kPbScaleRun; ++h) {
+                        const int64_t at = (int64_t)min(kb + h, kblocks - 1) * ks;
+                        v0[h] = __ldg(r0 + at);
+                        v1[h] = __ldg(r1 + at);
+                    }
+                }
+                if (t < 2 * kPbScaleRun) w = __ldg(s2 + (int64_t)min(kb + (t >> 1), kblocks - 1) * s2k);
+                if (!__all_sync(0xffffffffu, pb_wait<BN == 256>(sempty0 + 8u * sbuf, spar ^ 1u, abort_flag))) {
+                    report(abort_flag, (4u << 8) | 1u);
+                    ok = false;
+                    break;
+                }
+                float* d = s_scale[sbuf];
+#pragma unroll
+                for (int h = 0; h < kPbScaleRun; ++h) {
+                    d[h * 128 + t] = v0[h];
+                    d[h * 128 + 64 + t] = v1[h];
+                }
+                if (t < 2 * kPbScaleRun) d[kPbScaleRun * 128 + t] = w;
+                __syncwarp();
+                if (lane == 0) ptx::mbar_arrive(&s_bars[sbuf]);
+                sbuf ^= 1u;
+                if (sbuf == 0u) spar ^= 1u;
+            }
         }
-#endif
-        (void)d_tfull;
     }
-    else if (BN == 256) {
-        asm volatile("setmaxnreg.dec.sync.aligned.u32 40;");  // the two idle warps of the third warpgroup
-    }
-#ifdef OPSNN_PB_DIAG
-    // (epilogue warp 0's counters are written from inside its branch)
-#endif
     // ---- teardown ----
     if (*abort_flag != 0u) __nanosleep(200000);
     ptx::tc_fence_before();
@@ -462,7 +516,7 @@ template <ptx::MmaKind KIND, int EW, int BN = 128, bool ASYM = false>
 int32_t launch_pair_pb(const CUtensorMap& ma, const CUtensorMap& mb, UmmaArgs& a, cudaStream_t stream)
 {
     constexpr int kStage = kATile + (BN / 2) * BK;
-    constexpr int kDynMax = 227 * 1024 - (ASYM ? 4096 : 0);  // the asymmetric epilogue keeps 3 KB of static shared memory for its column buffers
+    constexpr int kDynMax = 227 * 1024 - (ASYM ? 4096 : 5 * 1024 + EW * 2048);  // less the static buffers
     int stages = (kDynMax - 2048) / kStage;
     if (stages > 8) stages = 8;
     if (stages > a.kblocks + 1) stages = a.kblocks + 1 > 2 ? a.kblocks + 1 : 2;
@@ -474,7 +528,7 @@ int32_t launch_pair_pb(const CUtensorMap& ma, const CUtensorMap& mb, UmmaArgs& a
         return (int32_t)cudaGetLastError();
     int64_t pairs = sm_count() / 2;
     if (a.num_tiles < pairs) pairs = a.num_tiles;
-    kern<<<(unsigned)(2 * pairs), pair_pb_threads<EW, BN>(), smem, stream>>>(ma, mb, a);
+    kern<<<(unsigned)(2 * pairs), pair_pb_threads<EW, ASYM>(), smem, stream>>>(ma, mb, a);
     note_launch(ASYM ? "qmm_umma_pair_pergroup_asym" : "qmm_umma_pair_perblock");
     return (int32_t)cudaGetLastError();
 }
