@@ -1046,7 +1046,7 @@ int32_t qmm_umma_launch(const OpsnnQmmParams* p, cudaStream_t stream)
             return a.is_int ? launch_pair_pb<ptx::MmaKind::kI8, 8, 256>(ma, mb, a, stream)
                             : launch_pair_pb<ptx::MmaKind::kF8F6F4, 8, 256>(ma, mb, a, stream);
         if (a.is_int) return launch_pair_pb<ptx::MmaKind::kI8, 8>(ma, mb, a, stream);
-        return launch_pair_pb<ptx::MmaKind::kF8F6F4, 4>(ma, mb, a, stream);
+        return launch_pair_pb<ptx::MmaKind::kF8F6F4, 8>(ma, mb, a, stream);
     }
     if (pair && f16) return launch_pair<ptx::MmaKind::kF16>(ma, mb, a, stream);
     if (pair) return a.is_int ? launch_pair<ptx::MmaKind::kI8>(ma, mb, a, stream) : launch_pair<ptx::MmaKind::kF8F6F4>(ma, mb, a, stream);

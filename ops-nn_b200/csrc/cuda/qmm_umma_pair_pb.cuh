@@ -15,6 +15,13 @@
 //   MMA warp (even CTA)   : wait tempty[buf] (all epilogue warps of the pair), wait full[s], 4 pair MMAs (first overwrites),
 //                           commit -> empty[s] and tfull[buf] of both CTAs
 //   epilogue (both CTAs)  : wait own tfull[buf]; TMEM -> registers; acc += part * (s1 * s2); arrive on the even CTA's tempty[buf]
+//   scale loaders         : two warps keep s1 of the CTA's rows and s2 of the tile's column blocks two runs of k-blocks ahead in shared
+//                           memory
+// Bound by the epilogue warps: TMEM reads and multiply-adds of 128 x 256 sums per k-block beside the running MMA, ~1000 clocks for 512 of
+// tensor work, and at 4096 x 7168 x 18432 by the power limit as well. With the scales read from global memory by every epilogue
+// thread (32 sectors a load) and rows stored 16 bytes a thread, those two took 180 and 120 of 1117 clocks per k-block. Measured, fp8:
+// 1024 x 4096 x 7168 51.5 -> 45 us, 4096 x 7168 x 18432 652 -> 637 (power-limited). Two N = 128 MMAs a k-block with four half
+// buffers are slower (57 us, 750 us).
 // All waits bounded, teardown through a cluster barrier, as in qmm_umma_pair.cuh.
 namespace {
 
@@ -22,14 +29,12 @@ namespace {
 template <ptx::MmaKind kKind>
 __device__ __forceinline__ void promote2(uint32_t v0, uint32_t v1, float sc, float& a0, float& a1)
 {
-#ifdef X2
     if constexpr (kKind != ptx::MmaKind::kI8) {
         asm("{\n\t.reg .b64 a, v, s;\n\tmov.b64 a, {%0, %1};\n\tmov.b64 v, {%2, %3};\n\tmov.b64 s, {%4, %4};\n\tfma.rn.f32x2 a, v, s, a;\n\tmov.b64 {%0, %1}, a;\n\t}"
             : "+f"(a0), "+f"(a1)
             : "r"(v0), "r"(v1), "f"(sc));
         return;
     }
-#endif
     a0 = promote<kKind>(v0, sc, a0);
     a1 = promote<kKind>(v1, sc, a1);
 }
@@ -330,53 +335,55 @@ qmm_umma_pair_pb_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_
                 }
             } else {
                 const uint32_t nb = (uint32_t)(part * kCols) >> 7;  // 128-column block of the tile
-                for (int kb = 0; kb < kblocks; ++kb) {
-                    const int j = kb % kPbScaleRun;
-                    if (j == 0 && !__all_sync(0xffffffffu, pb_wait<BN == 256>(sfull0 + 8u * sbuf, spar, abort_flag))) {
+                for (int kb0 = 0; kb0 < kblocks && ok; kb0 += kPbScaleRun) {
+                    if (!__all_sync(0xffffffffu, pb_wait<BN == 256>(sfull0 + 8u * sbuf, spar, abort_flag))) {
                         report(abort_flag, (3u << 8) | 3u);
                         ok = false;
                         break;
                     }
-                    const float sc = __fmul_rn(s_scale[sbuf][j * 128 + quad * 32 + lane], s_scale[sbuf][kPbScaleRun * 128 + 2 * j + nb]);
-                    if (!__all_sync(0xffffffffu, pb_wait<BN == 256>(tfull0 + 8u * buf, bpar, abort_flag))) {
-                        report(abort_flag, (3u << 8) | 2u);
-                        ok = false;
-                        break;
-                    }
-                    ptx::tc_fence_after();
-#ifndef PBW
-#define PBW 16
-#endif
-                    constexpr int W = PBW;  // staging registers per TMEM load (two sets in flight)
-                    const uint32_t t0 = tmem_base + lane_addr + buf * BN;
-                    uint32_t va[W], vb[W];
-                    ptx::tmem_ld_n(t0, va);
+                    float run[kPbScaleRun];  // the run's scales; the buffer goes back at once
 #pragma unroll
-                    for (int c = 0; c < kCols; c += 2 * W) {
-                        ptx::tmem_ld_wait();
-                        ptx::tmem_ld_n(t0 + c + W, vb);
+                    for (int j = 0; j < kPbScaleRun; ++j)
+                        run[j] = __fmul_rn(s_scale[sbuf][j * 128 + quad * 32 + lane], s_scale[sbuf][kPbScaleRun * 128 + 2 * j + nb]);
+                    __syncwarp();
+                    if (lane == 0) ptx::mbar_arrive(&s_bars[2 + sbuf]);
+                    sbuf ^= 1u;
+                    if (sbuf == 0u) spar ^= 1u;
 #pragma unroll
-                        for (int i = 0; i < W; i += 2) promote2<kKind>(va[i], va[i + 1], sc, acc[c + i], acc[c + i + 1]);
-                        ptx::tmem_ld_wait();
-                        if (c + 2 * W < kCols) {
-                            ptx::tmem_ld_n(t0 + c + 2 * W, va);
-                        } else {
-                            ptx::tc_fence_before();
-                            __syncwarp();
-                            if (lane == 0) ptx::mbar_arrive_cluster(lead_tempty0 + 8u * buf);
+                    for (int j = 0; j < kPbScaleRun; ++j) {
+                        if (kb0 + j >= kblocks) break;
+                        const float sc = run[j];
+                        if (!__all_sync(0xffffffffu, pb_wait<BN == 256>(tfull0 + 8u * buf, bpar, abort_flag))) {
+                            report(abort_flag, (3u << 8) | 2u);
+                            ok = false;
+                            break;
                         }
+                        ptx::tc_fence_after();
+                        constexpr int W = 16;  // staging registers per TMEM load (two sets in flight)
+                        const uint32_t t0 = tmem_base + lane_addr + buf * BN;
+                        uint32_t va[W], vb[W];
+                        ptx::tmem_ld_n(t0, va);
 #pragma unroll
-                        for (int i = 0; i < W; i += 2) promote2<kKind>(vb[i], vb[i + 1], sc, acc[c + W + i], acc[c + W + i + 1]);
-                    }
-                    if (++buf == NBUF) {
-                        buf = 0;
-                        bpar ^= 1u;
-                    }
-                    if (j == kPbScaleRun - 1 || kb == kblocks - 1) {
-                        __syncwarp();
-                        if (lane == 0) ptx::mbar_arrive(&s_bars[2 + sbuf]);
-                        sbuf ^= 1u;
-                        if (sbuf == 0u) spar ^= 1u;
+                        for (int c = 0; c < kCols; c += 2 * W) {
+                            ptx::tmem_ld_wait();
+                            ptx::tmem_ld_n(t0 + c + W, vb);
+#pragma unroll
+                            for (int i = 0; i < W; i += 2) promote2<kKind>(va[i], va[i + 1], sc, acc[c + i], acc[c + i + 1]);
+                            ptx::tmem_ld_wait();
+                            if (c + 2 * W < kCols) {
+                                ptx::tmem_ld_n(t0 + c + 2 * W, va);
+                            } else {
+                                ptx::tc_fence_before();
+                                __syncwarp();
+                                if (lane == 0) ptx::mbar_arrive_cluster(lead_tempty0 + 8u * buf);
+                            }
+#pragma unroll
+                            for (int i = 0; i < W; i += 2) promote2<kKind>(vb[i], vb[i + 1], sc, acc[c + W + i], acc[c + W + i + 1]);
+                        }
+                        if (++buf == NBUF) {
+                            buf = 0;
+                            bpar ^= 1u;
+                        }
                     }
                 }
             }
@@ -405,7 +412,11 @@ qmm_umma_pair_pb_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_
                     for (int c = 0; c < kCols; c += 32) {
                         float f[32];
 #pragma unroll
-                        for (int i = 0; i < 32; ++i) f[i] = bias == nullptr ? acc[c + i] : __fadd_rn(acc[c + i], load_as_float(bias, colbase + c + i, a.bias_dtype));
+                        for (int i = 0; i < 32; ++i) f[i] = acc[c + i];
+                        if (bias != nullptr) {
+#pragma unroll
+                            for (int i = 0; i < 32; ++i) f[i] = __fadd_rn(f[i], load_as_float(bias, colbase + c + i, a.bias_dtype));
+                        }
                         if (a.out_dtype == ACL_FLOAT) {
 #pragma unroll
                             for (int h = 0; h < 32; h += 16) {
