@@ -17,12 +17,12 @@
 //   epilogue (both CTAs)  : wait own tfull[buf]; TMEM -> registers; acc += part * (s1 * s2); arrive on the even CTA's tempty[buf]
 //   scale loaders         : two warps keep s1 of the CTA's rows and s2 of the tile's column blocks two runs of k-blocks ahead in shared
 //                           memory
-// Bound by the epilogue warps: TMEM reads and multiply-adds of 128 x 256 sums per k-block beside the running MMA, ~1000 clocks for 512 of
-// tensor work, and at 4096 x 7168 x 18432 by the power limit as well. With the scales read from global memory by every epilogue
-// thread (32 sectors a load) and rows stored 16 bytes a thread, those two took 180 and 120 of 1117 clocks per k-block. Measured, fp8:
-// 1024 x 4096 x 7168 51.5 -> 45 us, 4096 x 7168 x 18432 652 -> 637 (power-limited). Two N = 128 MMAs a k-block with four half
-// buffers are slower (57 us, 750 us).
-// All waits bounded, teardown through a cluster barrier, as in qmm_umma_pair.cuh.
+// Bound by the epilogue warps' chain per k-block (barrier, TMEM reads beside the running MMA, multiply-adds of 128 x 256 sums: ~900
+// clocks for 512 of tensor work) and, at 4096 x 7168 x 18432, by the power limit as well. Every epilogue thread used to read its scales
+// from global memory (32 sectors a load) and to store its row 16 bytes at a time: 180 and 120 of 1117 clocks. A run's scales are in
+// registers before its first k-block: read per k-block, they cost 8 % of the chain. fp8, bf16 out: 4096 x 7168 x 18432 655 -> 600 us,
+// 1024 x 4096 x 7168 51.5 -> 42.5, 512 x 7168 x 4608 27.3 -> 19.5, 2000 x 2048 x 2048 18.4 -> 16.
+// Tried: two N = 128 MMAs a k-block on four half buffers (57 us at 1024 x 4096 x 7168), 32 columns a TMEM load (spills, 54 us).
 namespace {
 
 // Two neighbouring columns; fp8's fused multiply-adds go as one packed instruction (each half rounded on its own).
@@ -353,7 +353,7 @@ qmm_umma_pair_pb_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_
                     for (int j = 0; j < kPbScaleRun; ++j) {
                         if (kb0 + j >= kblocks) break;
                         const float sc = run[j];
-                        if (!__all_sync(0xffffffffu, pb_wait<BN == 256>(tfull0 + 8u * buf, bpar, abort_flag))) {
+                        if (!pb_wait<BN == 256>(tfull0 + 8u * buf, bpar, abort_flag)) {
                             report(abort_flag, (3u << 8) | 2u);
                             ok = false;
                             break;
