@@ -15,6 +15,29 @@
 
 namespace opsnn {
 
+// Programmatic dependent launch. A kernel launched by launch_dependent may be placed and set up while the kernel before it on the stream
+// finishes; it calls pdl_wait before it touches global memory, and pdl_trigger lets the next one come. A kernel that allocates tensor
+// memory triggers only once it holds it: its successor, which may land on the same SM, could otherwise take what it still waits for.
+__device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+
+template <typename... Params, typename... Args>
+inline void launch_dependent(void (*kernel)(Params...), dim3 grid, unsigned threads, size_t smem, cudaStream_t stream, Args&&... args)
+{
+    cudaLaunchAttribute attr;
+    attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr.val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = grid;
+    cfg.blockDim = dim3(threads);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = stream;
+    cfg.attrs = &attr;
+    cfg.numAttrs = 1;
+    cudaLaunchKernelEx(&cfg, kernel, static_cast<Args&&>(args)...);  // an error stays for cudaGetLastError
+}
+
+
 // Host: count a launch and remember which kernel family ran (read back through opsnn_launch_count /
 // opsnn_last_kernel_name).
 void note_launch(const char* name, uint64_t n = 1);

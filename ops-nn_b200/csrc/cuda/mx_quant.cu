@@ -169,6 +169,8 @@ __device__ __forceinline__ uint32_t cvt_fp8x2(float lo, float hi)
 template <bool kBf16, int kUnroll>
 __global__ void __launch_bounds__(256) mx_quant_stream_kernel(const OpsnnMxQuantParams p, int64_t blocks_per_row, int64_t scale_row)
 {
+    pdl_trigger();
+    pdl_wait();
     const int64_t pieces = p.rows * blocks_per_row * 4;  // 8-element pieces
     const int emax = p.y_dtype == ACL_FLOAT4_E2M1 ? 2 : (p.y_dtype == ACL_FLOAT8_E4M3FN ? 8 : 15);
     const uint4* src = reinterpret_cast<const uint4*>(p.x);
@@ -337,10 +339,10 @@ int32_t mx_quant_launch(const OpsnnMxQuantParams* p, cudaStream_t stream)
         const int64_t per = 256 * (many ? 4 : 1), g2 = (pieces + per - 1) / per;
         if (g2 > 0x7FFFFFFF) return (int32_t)cudaErrorInvalidConfiguration;
         const bool bf = p->x_dtype == ACL_BF16;
-        if (bf && many) mx_quant_stream_kernel<true, 4><<<(unsigned)g2, 256, 0, stream>>>(*p, blocks_per_row, scale_row);
-        else if (bf) mx_quant_stream_kernel<true, 1><<<(unsigned)g2, 256, 0, stream>>>(*p, blocks_per_row, scale_row);
-        else if (many) mx_quant_stream_kernel<false, 4><<<(unsigned)g2, 256, 0, stream>>>(*p, blocks_per_row, scale_row);
-        else mx_quant_stream_kernel<false, 1><<<(unsigned)g2, 256, 0, stream>>>(*p, blocks_per_row, scale_row);
+        if (bf && many) launch_dependent(mx_quant_stream_kernel<true, 4>, dim3((unsigned)g2), 256, 0, stream, *p, blocks_per_row, scale_row);
+        else if (bf) launch_dependent(mx_quant_stream_kernel<true, 1>, dim3((unsigned)g2), 256, 0, stream, *p, blocks_per_row, scale_row);
+        else if (many) launch_dependent(mx_quant_stream_kernel<false, 4>, dim3((unsigned)g2), 256, 0, stream, *p, blocks_per_row, scale_row);
+        else launch_dependent(mx_quant_stream_kernel<false, 1>, dim3((unsigned)g2), 256, 0, stream, *p, blocks_per_row, scale_row);
         note_launch("mx_quant_stream");
         return (int32_t)cudaGetLastError();
     }

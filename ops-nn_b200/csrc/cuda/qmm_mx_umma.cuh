@@ -66,8 +66,10 @@ __global__ void mx_sf_relayout_kernel(const uint8_t* __restrict__ src, uint8_t* 
 constexpr int kSfChunk = 256;
 __global__ void __launch_bounds__(256) mx_sf_relayout_tiled_kernel(const uint8_t* __restrict__ src, uint8_t* __restrict__ dst, int64_t rows,
                                                                    int64_t kblocks, int64_t kq, int transposed_layout, int64_t tiles,
-                                                                   int64_t stages, int atoms, int64_t src_bs, int tile_rows, int row_atoms)
+                                                                   int64_t stages, int atoms, int64_t src_bs, int tile_rows, int row_atoms, int chunk)
 {
+    pdl_trigger();
+    pdl_wait();
     __shared__ __align__(16) uint8_t sm[128][kSfChunk + 4];
     int64_t r = blockIdx.x;
     const int ra = (int)(r % row_atoms); r /= row_atoms;
@@ -79,8 +81,8 @@ __global__ void __launch_bounds__(256) mx_sf_relayout_tiled_kernel(const uint8_t
     const int64_t kb_total = stages * atoms * 4;                            // k-blocks the atoms cover (>= kblocks)
     const int tid = threadIdx.x;
     // blockIdx.y: a chunk of k-blocks (a long k against few row tiles was one CTA's serial loop: 31 us for 10 x 391 x 15104 fp4)
-    for (int64_t kc0 = (int64_t)blockIdx.y * kSfChunk; kc0 < kb_total; kc0 += (int64_t)gridDim.y * kSfChunk) {
-        const int kc = (int)min((int64_t)kSfChunk, kb_total - kc0);         // multiple of 4
+    for (int64_t kc0 = (int64_t)blockIdx.y * chunk; kc0 < kb_total; kc0 += (int64_t)gridDim.y * chunk) {
+        const int kc = (int)min((int64_t)chunk, kb_total - kc0);         // multiple of 4
         __syncthreads();
         const bool vec16 = !transposed_layout && ((2 * kq) & 15) == 0 && (reinterpret_cast<uintptr_t>(s) & 15) == 0 && (kc & 15) == 0 &&
                            kc0 + kc <= kblocks;
@@ -370,6 +372,8 @@ qmm_mx_umma_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_const
     __syncthreads();
     ptx::tc_fence_after();
     const uint32_t tmem_base = *tmem_ptr;
+    pdl_trigger();
+    pdl_wait();
 
     const uint32_t tiles_per_batch = (uint32_t)a.tiles_m * (uint32_t)a.tiles_n;
     const uint32_t ntiles = (uint32_t)a.num_tiles;
@@ -633,7 +637,7 @@ int32_t mx_launch_one(const CUtensorMap& ma, const CUtensorMap& mb, UmmaArgs& a,
             configured, [&] { return cudaFuncSetAttribute(qmm_mx_umma_kernel<BN, kF4>, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024); });
         if (rc != cudaSuccess) return (int32_t)rc;
     }
-    qmm_mx_umma_kernel<BN, kF4><<<(unsigned)grid, 192, smem, stream>>>(ma, mb, a);
+    launch_dependent(qmm_mx_umma_kernel<BN, kF4>, dim3((unsigned)grid), 192, smem, stream, ma, mb, a);
     note_launch(kF4 ? "qmm_umma_mxfp4" : "qmm_umma_mxfp8");
     return (int32_t)cudaGetLastError();
 }
@@ -669,11 +673,17 @@ uint64_t qmm_mx_umma_workspace_size(const OpsnnQmmParams* p0)
     return q.nb_a * q.sfa_bytes_per_batch + q.nb_b * q.sfb_bytes_per_batch + q.tr_a_bytes + q.tr_b_bytes + 3 * 256;
 }
 
-// Chunks of k-blocks that the tiled relayout is spread over.
-unsigned sf_chunks(const MxPlan& q)
+// Launch of the tiled relayout: `columns` row atoms, k-blocks in chunks of 256, or smaller ones while they leave SMs without a block (one
+// block with a few hundred bytes a row took 5 us, all of it latency).
+static void sf_relayout(int64_t columns, const MxPlan& q, cudaStream_t stream, const void* src, uint8_t* dst, int64_t rows, int k_major, int64_t tiles,
+                        int64_t src_bs, int tile_rows, int row_atoms)
 {
-    const int64_t chunks = (q.kstages * q.atoms * 4 + kSfChunk - 1) / kSfChunk;
-    return (unsigned)std::min<int64_t>(std::max<int64_t>(chunks, 1), 65535);
+    const int64_t total = q.kstages * q.atoms * 4;
+    int chunk = kSfChunk;
+    while (chunk > 16 && columns * ((total + chunk - 1) / chunk) < sm_count()) chunk /= 2;
+    const unsigned gy = (unsigned)std::min<int64_t>((total + chunk - 1) / chunk, 65535);
+    launch_dependent(mx_sf_relayout_tiled_kernel, dim3((unsigned)columns, gy), 256, 0, stream, static_cast<const uint8_t*>(src), dst, rows,
+                     (int64_t)q.kblocks32, (int64_t)q.kq, k_major, tiles, (int64_t)q.kstages, (int)q.atoms, src_bs, tile_rows, row_atoms, chunk);
 }
 
 // x2Scale of p (all batches) into scale-atom order at dst, for the tile width of plan q.
@@ -681,8 +691,7 @@ static void mx_relayout_sfb(const OpsnnQmmParams* p, const MxPlan& q, int scale_
 {
     const int64_t gb = (int64_t)q.nb_b * q.tiles_n * q.row_atoms;
     if (env("OPSNN_MX_SF_SIMPLE") == nullptr && gb < 0x7FFFFFFF) {
-        mx_sf_relayout_tiled_kernel<<<dim3((unsigned)gb, sf_chunks(q)), 256, 0, stream>>>(reinterpret_cast<const uint8_t*>(p->scale_b), dst, p->n, q.kblocks32, q.kq,
-                                                                      scale_b_k_major, q.tiles_n, q.kstages, q.atoms, p->sb_bs, q.bn, q.row_atoms);
+        sf_relayout(gb, q, stream, p->scale_b, dst, p->n, scale_b_k_major, q.tiles_n, p->sb_bs, q.bn, q.row_atoms);
     } else {
         const int64_t wb = (int64_t)q.nb_b * q.tiles_n * q.kstages * q.atoms * q.row_atoms * 128;
         mx_sf_relayout_kernel<<<(unsigned)std::min<int64_t>((wb + 255) / 256, 148 * 16), 256, 0, stream>>>(
@@ -760,8 +769,7 @@ int32_t qmm_mx_umma_launch(const OpsnnQmmParams* p0, cudaStream_t stream)
         (void)wb;
         (void)gb;
         if (env("OPSNN_MX_SF_SIMPLE") == nullptr && ga < 0x7FFFFFFF) {
-            mx_sf_relayout_tiled_kernel<<<dim3((unsigned)ga, sf_chunks(q)), 256, 0, stream>>>(reinterpret_cast<const uint8_t*>(p->scale_a), sfa, p->m, q.kblocks32,
-                                                                          q.kq, p->trans_a ? 1 : 0, q.tiles_m, q.kstages, q.atoms, p->sa_bs, BM, 1);
+            sf_relayout(ga, q, stream, p->scale_a, sfa, p->m, p->trans_a ? 1 : 0, q.tiles_m, p->sa_bs, BM, 1);
         } else {
             mx_sf_relayout_kernel<<<blocks(wa), threads, 0, stream>>>(reinterpret_cast<const uint8_t*>(p->scale_a), sfa, p->m, q.kblocks32, q.kq,
                                                                       p->trans_a ? 1 : 0, q.tiles_m, q.kstages, q.atoms, (int64_t)q.nb_a, p->sa_bs,

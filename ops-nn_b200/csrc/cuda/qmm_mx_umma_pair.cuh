@@ -57,6 +57,8 @@ qmm_mx_umma_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_
     ptx::cluster_sync();
     ptx::tc_fence_after();
     const uint32_t tmem_base = *tmem_ptr;
+    pdl_trigger();
+    pdl_wait();
 
     const uint32_t tiles_per_batch = (uint32_t)a.tiles_m * (uint32_t)a.tiles_n;
     const uint32_t ntiles = (uint32_t)a.num_tiles;
@@ -285,7 +287,7 @@ int32_t mx_launch_pair(const CUtensorMap& ma, const CUtensorMap& mb, UmmaArgs& a
     }
     int64_t pairs = sm_count() / 2;
     if (a.num_tiles < pairs) pairs = a.num_tiles;
-    qmm_mx_umma_pair_kernel<kF4><<<(unsigned)(2 * pairs), 192, smem, stream>>>(ma, mb, msa, msb, a);
+    launch_dependent(qmm_mx_umma_pair_kernel<kF4>, dim3((unsigned)(2 * pairs)), 192, smem, stream, ma, mb, msa, msb, a);
     note_launch(kF4 ? "qmm_umma_pair_mxfp4" : "qmm_umma_pair_mxfp8");
     return (int32_t)cudaGetLastError();
 }

@@ -351,6 +351,8 @@ qmm_umma_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant
     __syncthreads();
     ptx::tc_fence_after();
     const uint32_t tmem_base = *tmem_ptr;
+    pdl_trigger();
+    pdl_wait();
 
     const uint32_t tiles_per_batch = (uint32_t)a.tiles_m * (uint32_t)a.tiles_n;
     const uint32_t ntiles = (uint32_t)a.num_tiles;
@@ -770,7 +772,7 @@ int32_t launch_one(const CUtensorMap& ma, const CUtensorMap& mb, UmmaArgs& a, cu
         return (int32_t)cudaGetLastError();
     const int64_t work = a.num_tiles * (PB ? 1 : a.ksplit);
     int64_t grid = work < sm_count() ? work : sm_count();
-    kern<<<(unsigned)grid, (EW + 2) * 32, smem, stream>>>(ma, mb, a);
+    launch_dependent(kern, dim3((unsigned)grid), (EW + 2) * 32, smem, stream, ma, mb, a);
     note_launch(PB ? "qmm_umma_perblock" : (a.ksplit > 1 ? "qmm_umma_deq_splitk" : "qmm_umma_deq"));
     return (int32_t)cudaGetLastError();
 }

@@ -60,6 +60,8 @@ qmm_umma_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_con
     ptx::cluster_sync();  // both CTAs' barriers are initialised before anybody signals across the pair
     ptx::tc_fence_after();
     const uint32_t tmem_base = *tmem_ptr;
+    pdl_trigger();
+    pdl_wait();
 
     const uint32_t tiles_per_batch = (uint32_t)a.tiles_m * (uint32_t)a.tiles_n;
     const uint32_t ntiles = (uint32_t)a.num_tiles;
@@ -223,7 +225,7 @@ int32_t launch_pair(const CUtensorMap& ma, const CUtensorMap& mb, UmmaArgs& a, c
         return (int32_t)cudaGetLastError();
     int64_t pairs = sm_count() / 2;
     if (a.num_tiles < pairs) pairs = a.num_tiles;
-    kern<<<(unsigned)(2 * pairs), 192, smem, stream>>>(ma, mb, a);
+    launch_dependent(kern, dim3((unsigned)(2 * pairs)), 192, smem, stream, ma, mb, a);
     note_launch("qmm_umma_pair_deq");
     return (int32_t)cudaGetLastError();
 }

@@ -124,6 +124,8 @@ qmm_umma_pair_pb_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_
     ptx::cluster_sync();
     ptx::tc_fence_after();
     const uint32_t tmem_base = *tmem_ptr;
+    pdl_trigger();
+    pdl_wait();
 
     const uint32_t tiles_per_batch = (uint32_t)a.tiles_m * (uint32_t)a.tiles_n;
     const uint32_t ntiles = (uint32_t)a.num_tiles;
@@ -539,7 +541,7 @@ int32_t launch_pair_pb(const CUtensorMap& ma, const CUtensorMap& mb, UmmaArgs& a
         return (int32_t)cudaGetLastError();
     int64_t pairs = sm_count() / 2;
     if (a.num_tiles < pairs) pairs = a.num_tiles;
-    kern<<<(unsigned)(2 * pairs), pair_pb_threads<EW, ASYM>(), smem, stream>>>(ma, mb, a);
+    launch_dependent(kern, dim3((unsigned)(2 * pairs)), pair_pb_threads<EW, ASYM>(), smem, stream, ma, mb, a);
     note_launch(ASYM ? "qmm_umma_pair_pergroup_asym" : "qmm_umma_pair_perblock");
     return (int32_t)cudaGetLastError();
 }

@@ -267,7 +267,6 @@ qmm_umma_split_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_co
     const int lane = threadIdx.x & 31;
 
     // programmatic dependent launch: placed and set up under the tail of the kernel before it, reads nothing until that has finished
-    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     if (threadIdx.x == 0) {
         s_abort = 0u;
         for (uint32_t i = 0; i < a.stages; ++i) {
@@ -289,7 +288,8 @@ qmm_umma_split_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_co
     __syncthreads();
     ptx::tc_fence_after();
     const uint32_t tmem = s_tmem;
-    asm volatile("griddepcontrol.wait;" ::: "memory");
+    pdl_trigger();
+    pdl_wait();
 
     const uint32_t u_begin = split_begin(a, blockIdx.x), u_end = split_begin(a, blockIdx.x + 1);
     SplitCols4 cols4;  // (per-block: only a bias, read at the end; 16 registers the sums need)

@@ -323,7 +323,6 @@ wqbmm_mixed_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
     const uint32_t dfull0 = aempty0 + 8u * kMixABufs, dempty0 = dfull0 + 16u, fin0 = dempty0 + 16u;
     volatile uint32_t* abort_flag = &s_abort;
 
-    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     if (threadIdx.x == 0) {
         s_abort = 0u;
         for (uint32_t i = 0; i < a.stages; ++i) {
@@ -351,7 +350,8 @@ wqbmm_mixed_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
     __syncthreads();
     ptx::tc_fence_after();
     const uint32_t tmem = s_tmem;
-    asm volatile("griddepcontrol.wait;" ::: "memory");  // nothing another kernel may have written is read before this
+    pdl_trigger();
+    pdl_wait();  // nothing another kernel may have written is read before this
 
     const uint32_t u_begin = mix_begin(a, blockIdx.x), u_end = mix_begin(a, blockIdx.x + 1);
     const uint32_t stages = a.stages, stage_bytes = a.stage_bytes;

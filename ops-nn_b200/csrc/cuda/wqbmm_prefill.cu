@@ -109,6 +109,8 @@ template <MixW kW, bool kBf16, bool kOff>
 __global__ void __launch_bounds__(NT) wq_dequant_kn_kernel(const OpsnnWqbmmParams p, uint16_t* __restrict__ dst, int64_t kp, float* __restrict__ one,
                                                            uint32_t tiles_n)
 {
+    pdl_trigger();
+    pdl_wait();
     constexpr int kCols = kW == MixW::kInt4 ? 8 : 4, kPairs = kCols / 2, kTileN = 32 * kCols;
     __shared__ __align__(16) uint32_t tile[kTileN * 32];
     const int tid = threadIdx.x, wj = tid & 31, kr = tid >> 5;
@@ -171,6 +173,8 @@ template <MixW kW, bool kBf16, bool kOff>
 __global__ void __launch_bounds__(NT) wq_dequant_nk_kernel_fast(const OpsnnWqbmmParams p, uint16_t* __restrict__ dst, int64_t kp, float* __restrict__ one,
                                                                 uint32_t chunks)
 {
+    pdl_trigger();
+    pdl_wait();
     constexpr int kPer = kW == MixW::kInt4 ? 8 : 4;  // weights in a word
     const uint32_t row = blockIdx.x / chunks, chunk = blockIdx.x - row * chunks;
     if (blockIdx.x == 0 && threadIdx.x == 0) *one = 1.0f;
@@ -214,10 +218,10 @@ void dequant_fast(const OpsnnWqbmmParams* p, uint16_t* dst, int64_t kp, float* o
         constexpr bool kB = decltype(bf_c)::value, kO = decltype(off_c)::value && kW != MixW::kE4m3;
         if (p->trans_w) {
             const uint32_t chunks = (uint32_t)((p->k / kPer + 4 * NT - 1) / (4 * NT));
-            wq_dequant_nk_kernel_fast<kW, kB, kO><<<(unsigned)(p->n * chunks), NT, 0, stream>>>(*p, dst, kp, one, chunks);
+            launch_dependent(wq_dequant_nk_kernel_fast<kW, kB, kO>, dim3((unsigned)(p->n * chunks)), NT, 0, stream, *p, dst, kp, one, chunks);
         } else {
             const uint32_t tiles_n = (uint32_t)((p->n + 32 * kPer - 1) / (32 * kPer));
-            wq_dequant_kn_kernel<kW, kB, kO><<<(unsigned)(tiles_n * ((p->k + 63) / 64)), NT, 0, stream>>>(*p, dst, kp, one, tiles_n);
+            launch_dependent(wq_dequant_kn_kernel<kW, kB, kO>, dim3((unsigned)(tiles_n * ((p->k + 63) / 64))), NT, 0, stream, *p, dst, kp, one, tiles_n);
         }
     };
     if (bf && off) go(std::true_type{}, std::true_type{});
