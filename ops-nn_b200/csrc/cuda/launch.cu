@@ -98,15 +98,16 @@ static bool streaming_asked_for()
 //   m 1   4096 x 4096 12.1 -> 8.6      m 16  8192 x 28672 49.3 -> 39.1     m 16 int8 4096 x 14336 20.2 -> 15.2
 //   m 32  8192 x 28672 98 -> 43        m 128 8192 x 28672 285 -> 67        m 512 8192 x 28672 416 -> 237
 // It does not take: innerPrecise = 1 (the group-wise arithmetic of the streaming kernels), outputs bound to a communicator (only the
-// streaming kernels store into the peers), a weight prepared for the matmul, and m > 1024, where dequantising the weight once per 128
-// rows costs more than a pass over HBM. aclnnWeightQuantBatchMatmulV2 keeps the kernels that its tests name: the streaming one for
+// streaming kernels store into the peers), a weight prepared for the matmul, and m > 1152, where dequantising the weight once per 128
+// rows costs more than a pass over HBM (against pre-pass and matmul, us: m 1100 8192 x 28672 int4 514 / 578, 4096^2 40 / 53; m 1280 610 / 597,
+// 52 / 54, int8 4096 x 14336 169 / 160). aclnnWeightQuantBatchMatmulV2 keeps the kernels that its tests name: the streaming one for
 // symmetric (k,n) int4 at m <= 16 (and its reported plan), dequantise-then-matmul up to 2^22 weights.
 int32_t wqbmm_faster_kernel(const OpsnnWqbmmParams* p, int32_t choice, bool v2)
 {
     if (choice != OPSNN_WQ_KERNEL_DECODE && choice != OPSNN_WQ_KERNEL_PREFILL && choice != OPSNN_WQ_KERNEL_GENERIC) return choice;
     if (choice == OPSNN_WQ_KERNEL_PREFILL && p->prep_w != nullptr) return choice;
     const int64_t weights = p->k * p->n;
-    if (p->m > 1024 || weights < ((int64_t)1 << 18)) return choice;
+    if (p->m > 1152 || weights < ((int64_t)1 << 18)) return choice;
     if (v2) {
         if (choice == OPSNN_WQ_KERNEL_GENERIC) return choice;
         if (p->m > 16 && weights <= ((int64_t)1 << 22)) return choice;
