@@ -1,8 +1,7 @@
 // Per-block (1x128 / 128x128 fp32 scales) fp8 and int8 matmul on CTA pairs (tcgen05 cta_group::2). Included by qmm_umma.cu.
 //
 // Why. The single-CTA per-block kernel uses 128 x 128 tiles (the promotion epilogue keeps 128 fp32 sums per thread), which
-// pull 32 KB of operands from L2 per 128-deep k-block; with the epilogue switched off the main loop still needs ~700 cycles
-// per k-block against 256 of tensor work: it is bound by the L2 -> SM operand feed. A CTA pair shares a 256 x 128 tile: each
+// pull 32 KB of operands from L2 per 128-deep k-block of 256 clocks of tensor work. A CTA pair shares a 256 x 128 tile: each
 // CTA loads its own 128 rows of A and 64 of the 128 rows of B (24 KB per k-block), keeps a 128 x 128 accumulator in its own
 // TMEM and runs the same promotion on it.
 //
@@ -41,7 +40,7 @@ __device__ __forceinline__ void promote2(uint32_t v0, uint32_t v1, float sc, flo
 
 // 256-column tiles: 128 sums per epilogue thread need more registers than an even split of the register file over the CTA's
 // warps gives (168 with ten warps), so the block is three whole warpgroups - epilogue warps 0..7, then {producer, MMA issuer, two
-// idle warps} - and setmaxnreg moves registers from the third group (40 each) to the first two (232 each): per scheduler
+// scale loaders} - and setmaxnreg moves registers from the third group (40 each) to the first two (232 each): per scheduler
 // 2 x 232 + 40 = 504 of the 512 registers per lane.
 // (Code that runs under setmaxnreg cannot call an out-of-line function: the bounded spin is inlined for those instances.)
 template <bool kInline>
@@ -577,7 +576,7 @@ bool pair_pb_worthwhile(const OpsnnQmmParams* p)
 }
 
 // Tile width of the per-block pair kernel: 256 columns (32 KB of operands per CTA and k-block for twice the tensor work of the
-// 128-column tile's 24 KB: the L2 -> SM feed is what bounds the main loop) once there are enough such tiles for every pair.
+// 128-column tile's 24 KB, and one hand-over of an accumulator instead of two) once there are enough such tiles for every pair.
 // OPSNN_QMM_PB_BN=128|256 fixes it.
 int pair_pb_bn(const OpsnnQmmParams* p)
 {

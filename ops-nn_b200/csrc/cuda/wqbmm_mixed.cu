@@ -1,4 +1,4 @@
-// Weight-only quant matmul for 16 < m: the packed weight is dequantised straight into tensor memory and multiplied there
+// Weight-only quant matmul: the packed weight is dequantised straight into tensor memory and multiplied there
 // (tcgen05 kind::f16 with A in TMEM), one pass over the weight for up to 128 rows of x. No 16-bit image of the weight in HBM.
 //
 // Reference: weight_quant_batch_matmul_v2/op_kernel/arch35/weight_quant_batch_matmul_v2_reg_base_common.h:164-286 (vector cores
