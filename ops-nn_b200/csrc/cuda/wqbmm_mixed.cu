@@ -19,6 +19,7 @@
 // A operand buffers: four units of 64 k x 256 columns (64 TMEM columns each) at columns 256-511; accumulators at 0-255 (two sets while
 // N <= 64).
 // Every wait is bounded; a wait that gives up raises the CTA's abort flag, records a code and the CTA tears down (TMEM freed).
+#include <algorithm>
 #include <cstdio>
 
 #include "common.cuh"
@@ -39,10 +40,20 @@ constexpr uint32_t kMixACol = 256;  // first TMEM column of the A buffers
 constexpr int kMixMaxStages = 16;
 constexpr int kMixSmemMax = 225 * 1024;
 
+// How a CTA sums its piece over k. The tensor core cuts each addition to an accumulator off instead of rounding it, so the error grows with
+// the length of the chain of MMAs on one accumulator. Up to 48 rows of x the streaming kernels, which cut k over more CTAs, chain a quarter
+// as many MMAs as a piece here has; the sums are to be as exact as theirs (outputs that are not the rounded exact sum, fp16,
+// 16 x 8192 x 28672: 2.1 % as one chain, 0.8 % there, 0.65 % here).
+//   kChain    one accumulator: the chain is no longer than that of the matmul on a dequantised weight
+//   kCopies   4 or 8 accumulators take turns, MMA by MMA (they fit for 16 rows, or 32 where one set is enough)
+//   kChunks   the accumulator is added to a sum in tensor memory, with rounding, every few stages, by the epilogue warps
+enum class MixSum { kChain, kCopies, kChunks };
+
 struct MixArgs {
     int32_t m, t_tiles, rows;  // rows: rows of x per tile (N of the MMA)
     uint32_t n, k, kb;         // kb: k stages per tile
     uint32_t grid, units;      // units = tiles * kb, cut into `grid` contiguous pieces; units * grid < 2^32
+    uint32_t copies, chunk;    // MixSum: accumulators, k stages to a chunk
     uint32_t split;            // > 0: grid = tiles * split, so that a tile is `split` whole pieces, launched as a cluster; 0: stream-k
     uint32_t stages, stage_bytes, x_off, sc_off, sc_rows, sc_vec;  // sc_rows: scale rows a stage needs (2: groups that end inside a stage)
     const void* scale;
@@ -124,6 +135,17 @@ __device__ __forceinline__ void tmem_st_32x32b_x8(uint32_t taddr, const uint32_t
                  "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7])
                  : "memory");
 }
+// 32 TMEM lanes x 32 columns of 32-bit sums
+__device__ __forceinline__ void tmem_st_32x32b_x32(uint32_t taddr, const uint32_t (&r)[32])
+{
+    asm volatile(
+        "tcgen05.st.sync.aligned.32x32b.x32.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, %16, "
+        "%17, %18, %19, %20, %21, %22, %23, %24, %25, %26, %27, %28, %29, %30, %31, %32};" ::"r"(taddr),
+        "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7]), "r"(r[8]), "r"(r[9]), "r"(r[10]), "r"(r[11]),
+        "r"(r[12]), "r"(r[13]), "r"(r[14]), "r"(r[15]), "r"(r[16]), "r"(r[17]), "r"(r[18]), "r"(r[19]), "r"(r[20]), "r"(r[21]), "r"(r[22]),
+        "r"(r[23]), "r"(r[24]), "r"(r[25]), "r"(r[26]), "r"(r[27]), "r"(r[28]), "r"(r[29]), "r"(r[30]), "r"(r[31])
+        : "memory");
+}
 __device__ __forceinline__ void tmem_st_wait() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
 // kind::f16, A (128 x 16) in tensor memory, B in shared memory
 __device__ __forceinline__ void umma_f16_ta(uint32_t d_tmem, uint32_t a_tmem, uint64_t bdesc, uint32_t idesc, uint32_t accumulate)
@@ -176,11 +198,58 @@ __device__ __forceinline__ void mix_store(const MixArgs& a, uint32_t n, uint32_t
     }
 }
 
-// A finished piece of tile t (stages kb .. kb + cnt of it) out of the accumulator set at TMEM address `acc` (this warp's lanes): stored
+// 16 columns of a piece's sums. kMany: of `n` accumulators (1 or an even number), `step` columns apart.
+template <bool kMany>
+__device__ __forceinline__ void mix_sums16(uint32_t acc, uint32_t n, uint32_t step, float (&f)[16])
+{
+    uint32_t v[16];
+    ptx::tmem_ld16(acc, v);
+    if constexpr (!kMany) {
+        ptx::tmem_ld_wait();
+#pragma unroll
+        for (int i = 0; i < 16; ++i) f[i] = __uint_as_float(v[i]);
+    } else {
+        uint32_t q[16];
+        if (n > 1u) ptx::tmem_ld16(acc + step, q);
+        ptx::tmem_ld_wait();
+#pragma unroll
+        for (int i = 0; i < 16; ++i) f[i] = n > 1u ? __fadd_rn(__uint_as_float(v[i]), __uint_as_float(q[i])) : __uint_as_float(v[i]);
+#pragma unroll 1
+        for (uint32_t j = 2; j < n; j += 2) {
+            ptx::tmem_ld16(acc + j * step, v);
+            ptx::tmem_ld16(acc + (j + 1u) * step, q);
+            ptx::tmem_ld_wait();
+#pragma unroll
+            for (int i = 0; i < 16; ++i) f[i] = __fadd_rn(f[i], __fadd_rn(__uint_as_float(v[i]), __uint_as_float(q[i])));
+        }
+    }
+}
+
+// sum = acc (the first chunk) or sum + acc, `cols` columns (a multiple of 32) of this warp's lanes.
+__device__ __forceinline__ void mix_promote(uint32_t acc, uint32_t sum, uint32_t cols, bool first)
+{
+#pragma unroll 1
+    for (uint32_t c = 0; c < cols; c += 32) {
+        uint32_t v[32], q[32];
+        ptx::tmem_ld32(acc + c, v);
+        if (!first) {
+            ptx::tmem_ld32(sum + c, q);
+            ptx::tmem_ld_wait();
+#pragma unroll
+            for (int i = 0; i < 32; ++i) v[i] = __float_as_uint(__fadd_rn(__uint_as_float(q[i]), __uint_as_float(v[i])));
+        } else {
+            ptx::tmem_ld_wait();
+        }
+        tmem_st_32x32b_x32(sum + c, v);
+    }
+    tmem_st_wait();
+}
+
+// A finished piece of tile t (stages kb .. kb + cnt of it) out of the accumulators at TMEM address `acc` (this warp's lanes): stored
 // if it is the whole tile, else parked in workspace, and combined by whoever arrives last. Run by kWarps warps (four per TMEM lane
 // quarter and column share): 4 of them beside the main loop, or 16 at the end of the CTA's work.
-template <bool kBf16, int kWarps>
-__device__ __forceinline__ void mix_finish(const MixArgs& a, uint32_t acc, uint32_t t, uint32_t cnt, int col, int qd, int lane, int share, bool leader,
+template <bool kBf16, int kWarps, bool kMany>
+__device__ __forceinline__ void mix_finish(const MixArgs& a, uint32_t acc, uint32_t n_acc, uint32_t step, uint32_t t, uint32_t cnt, int col, int qd, int lane, int share, bool leader,
                                            volatile uint32_t* s_last, volatile uint32_t* abort_flag)
 {
     constexpr int kBar = kWarps == 4 ? 1 : 2;
@@ -192,12 +261,8 @@ __device__ __forceinline__ void mix_finish(const MixArgs& a, uint32_t acc, uint3
     float4* mine = a.part + (2u * blockIdx.x + (t == mix_begin(a, blockIdx.x) / a.kb ? 0u : 1u)) * slot + row;
 #pragma unroll 1
     for (uint32_t hc = 16u * share; hc < 2u * rows; hc += kStep) {
-        uint32_t v[16];
-        ptx::tmem_ld16(acc + hc, v);
-        ptx::tmem_ld_wait();
         float f[16];
-#pragma unroll
-        for (int i = 0; i < 16; ++i) f[i] = __uint_as_float(v[i]);
+        mix_sums16<kMany>(acc + hc, n_acc, step, f);
         if (whole) {
             const uint32_t h = hc >= rows ? 1u : 0u;
             mix_store<kBf16>(a, n0 + 128u * h, tt * rows + hc - h * rows, f);
@@ -252,18 +317,18 @@ __device__ __forceinline__ void mix_finish(const MixArgs& a, uint32_t acc, uint3
 }
 
 // A CTA's sums of its piece, from tensor memory into shared memory as [row of x][256 columns] fp32 (sixteen warps).
-__device__ __forceinline__ void mix_park(const MixArgs& a, uint32_t acc, uint32_t smem, int col, int share)
+template <bool kMany>
+__device__ __forceinline__ void mix_park(const MixArgs& a, uint32_t acc, uint32_t n_acc, uint32_t step, uint32_t smem, int col, int share)
 {
     const uint32_t rows = (uint32_t)a.rows;
 #pragma unroll 1
     for (uint32_t hc = 16u * share; hc < 2u * rows; hc += 64u) {
-        uint32_t v[16];
-        ptx::tmem_ld16(acc + hc, v);
-        ptx::tmem_ld_wait();
+        float f[16];
+        mix_sums16<kMany>(acc + hc, n_acc, step, f);
         const uint32_t h = hc >= rows ? 1u : 0u;
         const uint32_t at = smem + (hc - h * rows) * (kMixTileN * 4u) + (128u * h + (uint32_t)col) * 4u;
 #pragma unroll
-        for (uint32_t i = 0; i < 16; ++i) asm volatile("st.shared.u32 [%0], %1;" ::"r"(at + i * (kMixTileN * 4u)), "r"(v[i]) : "memory");
+        for (uint32_t i = 0; i < 16; ++i) asm volatile("st.shared.f32 [%0], %1;" ::"r"(at + i * (kMixTileN * 4u)), "f"(f[i]) : "memory");
     }
 }
 
@@ -305,7 +370,7 @@ __device__ __forceinline__ void mix_sum_and_store(const MixArgs& a, uint32_t sme
     }
 }
 
-template <MixW kW, bool kNK, bool kBf16, bool kOff>
+template <MixW kW, bool kNK, bool kBf16, bool kOff, MixSum kSum>
 __global__ void __launch_bounds__(kMixThreads, 1)
 wqbmm_mixed_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUtensorMap map_x, const __grid_constant__ MixArgs a)
 {
@@ -314,13 +379,13 @@ wqbmm_mixed_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
     const int lane = threadIdx.x & 31;
     extern __shared__ uint8_t dyn_raw[];
     const uint32_t smem0 = (ptx::smem_u32(dyn_raw) + 1023u) & ~1023u;
-    __shared__ __align__(8) uint64_t s_bars[2 * kMixMaxStages + 2 * kMixABufs + 5];
+    __shared__ __align__(8) uint64_t s_bars[2 * kMixMaxStages + 2 * kMixABufs + 6];
     __shared__ uint32_t s_tmem;
     __shared__ volatile uint32_t s_abort;
     __shared__ volatile uint32_t s_last[2];
     const uint32_t full0 = ptx::smem_u32(s_bars), empty0 = full0 + 8u * kMixMaxStages;
     const uint32_t afull0 = empty0 + 8u * kMixMaxStages, aempty0 = afull0 + 8u * kMixABufs;
-    const uint32_t dfull0 = aempty0 + 8u * kMixABufs, dempty0 = dfull0 + 16u, fin0 = dempty0 + 16u;
+    const uint32_t dfull0 = aempty0 + 8u * kMixABufs, dempty0 = dfull0 + 16u, fin0 = dempty0 + 16u, fsum0 = fin0 + 8u;
     volatile uint32_t* abort_flag = &s_abort;
 
     if (threadIdx.x == 0) {
@@ -337,7 +402,10 @@ wqbmm_mixed_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
             mix_init(dfull0 + 8u * i, 1u);
             mix_init(dempty0 + 8u * i, kMixEpWarps);
         }
-        mix_init(fin0, 1u);  // the last piece's sums (its own barrier: the warps that wait for it have not followed the others' phases)
+        // the last piece's sums, and those of its chunks before the last (barriers of their own: the warps that wait for them have not
+        // followed the others' phases)
+        mix_init(fin0, 1u);
+        mix_init(fsum0, kMixEpWarps);
         ptx::fence_mbar_init();
         ptx::fence_proxy_async();
     }
@@ -356,8 +424,10 @@ wqbmm_mixed_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
     const uint32_t u_begin = mix_begin(a, blockIdx.x), u_end = mix_begin(a, blockIdx.x + 1);
     const uint32_t stages = a.stages, stage_bytes = a.stage_bytes;
     const uint32_t xunit = (uint32_t)a.rows * 128u;  // bytes of x per 64-row unit of k
-    const bool two_d = a.rows <= 64;                 // two accumulator sets
-    const uint32_t d_set = 2u * (uint32_t)a.rows;
+    // accumulators: two sets where there is room, beside them the sums of the chunks that are done
+    const uint32_t d_one = 2u * (uint32_t)a.rows, d_set = kSum == MixSum::kCopies ? a.copies * d_one : d_one;
+    const bool two_d = kSum == MixSum::kChain ? a.rows <= 64 : (kSum == MixSum::kCopies ? a.split == 0u : a.rows <= 32);
+    const uint32_t d_sum = two_d ? 2u * d_set : d_set;
 
     if (warp == kMixDqWarps + kMixEpWarps) {
         // ======================= TMA producer =======================
@@ -412,13 +482,13 @@ wqbmm_mixed_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
         const uint64_t db = ptx::make_smem_desc(smem0 + a.x_off, 0, 1024, 2);
         const uint32_t b_lo = (uint32_t)db;
         const uint64_t b_hi = db & 0xFFFFFFFF00000000ull;
-        uint32_t s = 0, par = 0, ab = 0, apar = 0, seg = 0;
+        uint32_t s = 0, par = 0, ab = 0, apar = 0, dbuf = 0, dpar = 0;
         bool ok = true;
-        const uint32_t kbs = a.kb, rows = (uint32_t)a.rows, idesc = a.idesc;
+        const uint32_t kbs = a.kb, rows = (uint32_t)a.rows, idesc = a.idesc, chunk = kSum == MixSum::kChunks ? a.chunk : kbs;
+        const uint32_t copies = a.copies, turn1 = d_one, turn2 = 2u * d_one, turn3 = 3u * d_one;
         uint32_t u = u_begin, kb = u_begin % kbs;
         while (u < u_end && ok) {
-            const uint32_t cnt = min(kbs - kb, u_end - u);
-            const uint32_t dbuf = two_d ? (seg & 1u) : 0u, dpar = two_d ? ((seg >> 1) & 1u) : (seg & 1u);
+            const uint32_t cnt = min(min(kbs - kb, u_end - u), chunk);
             if (!mix_wait(dempty0 + 8u * dbuf, dpar ^ 1u, abort_flag)) {
                 mix_report(abort_flag, (2u << 8) | 1u);
                 break;
@@ -444,16 +514,18 @@ wqbmm_mixed_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
                         const uint32_t a0 = tmem + kMixACol + ab * 64u;
 #pragma unroll
                         for (int kk = 0; kk < 4; ++kk) {
+                            uint32_t d = d0;
+                            if (kSum == MixSum::kCopies) d += (kk == 0 ? 0u : (kk == 1 ? turn1 : (kk == 2 ? turn2 : turn3))) + (un == 1 && copies == 8u ? 4u * d_one : 0u);
 #pragma unroll
                             for (int h = 0; h < 2; ++h)
-                                umma_f16_ta(d0 + h * rows, a0 + h * 32 + kk * 8, b_hi | (uint64_t)(bl + 2u * kk), idesc,
-                                            kk == 0 ? acc : 1u);
+                                umma_f16_ta(d + h * rows, a0 + h * 32 + kk * 8, b_hi | (uint64_t)(bl + 2u * kk), idesc,
+                                            kk == 0 || kSum == MixSum::kCopies ? acc : 1u);
                         }
                         ptx::umma_commit_a(aempty0 + 8u * ab);
                         if (un == 1) ptx::umma_commit_a(empty0 + 8u * s);
                     }
                     __syncwarp();
-                    acc = 1u;
+                    if (kSum != MixSum::kCopies || un == 1 || copies != 8u) acc = 1u;
                     if (++ab == kMixABufs) { ab = 0; apar ^= 1u; }
                 }
                 if (++s == stages) { s = 0; par ^= 1u; }
@@ -462,8 +534,10 @@ wqbmm_mixed_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
             u += cnt;
             if (ptx::elect_one()) ptx::umma_commit_a(u < u_end ? dfull0 + 8u * dbuf : fin0);
             __syncwarp();
-            ++seg;
-            kb = 0;
+            kb += cnt;
+            if (kb == kbs) kb = 0;
+            if (two_d) dbuf ^= 1u;
+            if (dbuf == 0u) dpar ^= 1u;
         }
     } else if (warp < kMixDqWarps) {
         // ======================= dequantisation =======================
@@ -710,47 +784,89 @@ wqbmm_mixed_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
         }
         // the CTA's last (often only) piece: nothing is left to dequantise, all sixteen warps finish it
         const uint32_t t_first = u_begin / a.kb, t_last = (u_end - 1u) / a.kb;
-        const uint32_t dbuf = two_d ? ((t_last - t_first) & 1u) : 0u;
-        if (ok && !mix_wait(fin0, 0u, abort_flag)) {
+        const uint32_t last_cnt = min(u_end - t_last * a.kb, u_end - u_begin);
+        uint32_t before = t_last - t_first;  // accumulator sets used before the last one
+        bool has_sum = false;
+        if constexpr (kSum == MixSum::kChunks) {
+            auto chunks = [&](uint32_t c) { return (c + a.chunk - 1u) / a.chunk; };
+            const uint32_t n = chunks(last_cnt);
+            has_sum = n > 1u;
+            before = n - 1u + (t_first == t_last ? 0u : chunks((t_first + 1u) * a.kb - u_begin) + (t_last - t_first - 1u) * chunks(a.kb));
+        }
+        const uint32_t dbuf = two_d ? (before & 1u) : 0u;
+        if (ok && (!mix_wait(fin0, 0u, abort_flag) || (has_sum && !mix_wait(fsum0, 0u, abort_flag)))) {
             mix_report(abort_flag, (3u << 8) | 3u);
             ok = false;
         }
         if (mix_all_ok<2, kMixDqWarps * 32>(ok)) {
             ptx::tc_fence_after();
+            constexpr bool kMany = kSum != MixSum::kChain;
             const uint32_t acc = tmem + tlane + dbuf * d_set;
+            // (with chunks: the last one and the sum of those before it)
+            const uint32_t n_acc = kSum == MixSum::kCopies ? a.copies : (has_sum ? 2u : 1u), step = kSum == MixSum::kCopies ? d_one : tmem + tlane + d_sum - acc;
             const int col = qd * 32 + mix_col_of_lane<kW, kNK>(lane);
             if (a.split != 0) {
-                mix_park(a, acc, smem0, col, warp >> 2);
+                mix_park<kMany>(a, acc, n_acc, step, smem0, col, warp >> 2);
                 if (a.split == 1) {
                     asm volatile("bar.sync 2, 512;" ::: "memory");
                     mix_sum_and_store<kBf16>(a, smem0, t_last, 0u, threadIdx.x);
                 }
             } else {
-                mix_finish<kBf16, 16>(a, acc, t_last, min(u_end - t_last * a.kb, u_end - u_begin), col, qd, lane, warp >> 2, threadIdx.x == 0, &s_last[1],
-                                      abort_flag);
+                mix_finish<kBf16, 16, kMany>(a, acc, n_acc, step, t_last, last_cnt, col, qd, lane, warp >> 2, threadIdx.x == 0, &s_last[1], abort_flag);
             }
         }
     } else {
-        // ======================= epilogue of all but the last piece, beside the main loop =======================
+        // ======================= epilogue of all but the last piece, beside the main loop; chunks are added up =======================
         const int qd = warp & 3;
         const uint32_t tlane = (uint32_t)(qd * 32) << 16;
         const int col = qd * 32 + mix_col_of_lane<kW, kNK>(lane);
-        uint32_t seg = 0, u = u_begin, t = u_begin / a.kb, kb = u_begin - t * a.kb;
-        while (u + (a.kb - kb) < u_end) {
-            const uint32_t cnt = a.kb - kb;
-            const uint32_t dbuf = two_d ? (seg & 1u) : 0u, dpar = two_d ? ((seg >> 1) & 1u) : (seg & 1u);
-            const bool got = __all_sync(0xffffffffu, ptx::mbar_wait_relaxed(&s_bars[2 * kMixMaxStages + 2 * kMixABufs + dbuf], dpar, abort_flag));
+        const bool leader = warp == kMixDqWarps && lane == 0;
+        uint32_t dbuf = 0, dpar = 0, u = u_begin, t = u_begin / a.kb, kb = u_begin - t * a.kb;
+        auto next_set = [&](bool relaxed) {  // waits for an accumulator set; the four warps go on, or leave, together
+            const bool got = relaxed ? __all_sync(0xffffffffu, ptx::mbar_wait_relaxed(&s_bars[2 * kMixMaxStages + 2 * kMixABufs + dbuf], dpar, abort_flag))
+                                     : mix_wait(dfull0 + 8u * dbuf, dpar, abort_flag);
             if (!got) mix_report(abort_flag, (4u << 8) | 1u);
-            if (!mix_all_ok<1, kMixEpWarps * 32>(got)) break;
+            const bool ok = mix_all_ok<1, kMixEpWarps * 32>(got);
             ptx::tc_fence_after();
-            mix_finish<kBf16, 4>(a, tmem + tlane + dbuf * d_set, t, cnt, col, qd, lane, 0, warp == kMixDqWarps && lane == 0, &s_last[0], abort_flag);
+            return ok;
+        };
+        auto give_back = [&]() {
             ptx::tc_fence_before();
             __syncwarp();
             if (lane == 0) mix_arrive(dempty0 + 8u * dbuf);
-            ++seg;
-            u += cnt;
-            kb = 0;
-            ++t;
+            if (two_d) dbuf ^= 1u;
+            if (dbuf == 0u) dpar ^= 1u;
+        };
+        if constexpr (kSum != MixSum::kChunks) {
+            while (u + (a.kb - kb) < u_end) {
+                const uint32_t cnt = a.kb - kb;
+                if (!next_set(true)) break;
+                mix_finish<kBf16, 4, kSum == MixSum::kCopies>(a, tmem + tlane + dbuf * d_set, a.copies, d_one, t, cnt, col, qd, lane, 0, leader, &s_last[0], abort_flag);
+                give_back();
+                u += cnt;
+                kb = 0;
+                ++t;
+            }
+        } else {
+            const uint32_t sum = tmem + tlane + d_sum;
+            bool ok = true;
+            while (u < u_end && ok) {
+                const uint32_t cnt = min(a.kb - kb, u_end - u);
+                const bool mine = u + cnt < u_end;  // the last chunk of the last piece is the dequantising warps'
+                for (uint32_t c = 0; (mine ? c : c + a.chunk) < cnt; c += a.chunk) {
+                    ok = next_set(two_d);  // (with one set the MMA issuer waits for this)
+                    if (!ok) break;
+                    mix_promote(tmem + tlane + dbuf * d_set, sum, d_one, c == 0u);
+                    give_back();
+                }
+                if (mine && ok) mix_finish<kBf16, 4, false>(a, sum, 1u, 0u, t, cnt, col, qd, lane, 0, leader, &s_last[0], abort_flag);
+                u += cnt;
+                kb = 0;
+                ++t;
+            }
+            ptx::tc_fence_before();
+            __syncwarp();
+            if (ok && lane == 0) mix_arrive(fsum0);
         }
     }
     if (a.split > 1u) {
@@ -806,7 +922,8 @@ bool mix_map(CUtensorMap* map, const void* base, uint64_t inner_bytes, uint64_t 
 }
 
 struct MixPlan {
-    int t_tiles, rows, split;
+    int t_tiles, rows, split, copies, chunk;
+    MixSum sum;
     int64_t n_tiles, kb, grid, units, tiles;
 };
 
@@ -847,44 +964,63 @@ MixPlan mix_plan(const OpsnnWqbmmParams* p, int sms, F&& clusters)
         const int v = atoi(e);
         if (v >= 1 && v <= most) { q.split = v; q.grid = q.tiles * v; }
     }
+    // The longest chain of MMAs (8 a stage) that leaves the sums as exact as the streaming kernels' (MixSum): a quarter of an SM's share of
+    // the work, or what is left of k when they have cut it sixteen ways. They took more than 16 rows of x from 2^24 weights on, more than 32
+    // from 3 x 2^24 (16 rows a launch).
+    const int64_t chain = std::max<int64_t>(2 * q.units / sms, (q.kb * 9 + 19) / 20), piece = (q.units + q.grid - 1) / q.grid;
+    q.sum = MixSum::kChain;
+    q.copies = 1;
+    q.chunk = (int)std::min<int64_t>(std::max<int64_t>(1, chain / 8), q.kb);
+    if (q.rows == 16 || (q.rows == 32 && q.split != 0 && 2 * piece <= chain)) {
+        q.sum = MixSum::kCopies;
+        q.copies = q.split != 0 && 2 * piece > chain ? 8 : 4;
+    } else if ((q.rows == 32 && p->k * p->n >= ((int64_t)1 << 24)) || (q.rows == 48 && p->k * p->n >= ((int64_t)3 << 24))) {
+        q.sum = MixSum::kChunks;
+    }
     return q;
 }
 
 using MixKernel = void (*)(const CUtensorMap, const CUtensorMap, const MixArgs);
-template <MixW kW, bool kNK>
+template <MixW kW, bool kNK, MixSum kSum>
 MixKernel mix_kernel_of(bool bf16, bool off)
 {
     if constexpr (kW != MixW::kE4m3) {
-        if (off) return bf16 ? &wqbmm_mixed_kernel<kW, kNK, true, true> : &wqbmm_mixed_kernel<kW, kNK, false, true>;
+        if (off) return bf16 ? &wqbmm_mixed_kernel<kW, kNK, true, true, kSum> : &wqbmm_mixed_kernel<kW, kNK, false, true, kSum>;
     }
-    return bf16 ? &wqbmm_mixed_kernel<kW, kNK, true, false> : &wqbmm_mixed_kernel<kW, kNK, false, false>;
+    return bf16 ? &wqbmm_mixed_kernel<kW, kNK, true, false, kSum> : &wqbmm_mixed_kernel<kW, kNK, false, false, kSum>;
 }
-MixKernel mix_kernel(const OpsnnWqbmmParams* p, int* index)
+template <MixSum kSum>
+MixKernel mix_kernel_of(int w, bool nk, bool bf16, bool off)
 {
+    switch (w) {
+        case 0: return nk ? mix_kernel_of<MixW::kInt4, true, kSum>(bf16, off) : mix_kernel_of<MixW::kInt4, false, kSum>(bf16, off);
+        case 1: return nk ? mix_kernel_of<MixW::kInt8, true, kSum>(bf16, off) : mix_kernel_of<MixW::kInt8, false, kSum>(bf16, off);
+        default: return nk ? mix_kernel_of<MixW::kE4m3, true, kSum>(bf16, off) : mix_kernel_of<MixW::kE4m3, false, kSum>(bf16, off);
+    }
+}
+// The kernel of a form, ready to launch on the current device.
+cudaError_t mix_kernel(const OpsnnWqbmmParams* p, MixSum sum, MixKernel* kern)
+{
+    static std::atomic<uint64_t> configured[3 * 24];
     const bool bf16 = p->x_dtype == ACL_BF16, off = p->offset != nullptr, nk = p->trans_w != 0;
     const int w = p->w_dtype == ACL_INT4 ? 0 : (p->w_dtype == ACL_INT8 ? 1 : 2);
-    *index = w * 8 + (nk ? 4 : 0) + (bf16 ? 2 : 0) + (off ? 1 : 0);
-    switch (w) {
-        case 0: return nk ? mix_kernel_of<MixW::kInt4, true>(bf16, off) : mix_kernel_of<MixW::kInt4, false>(bf16, off);
-        case 1: return nk ? mix_kernel_of<MixW::kInt8, true>(bf16, off) : mix_kernel_of<MixW::kInt8, false>(bf16, off);
-        default: return nk ? mix_kernel_of<MixW::kE4m3, true>(bf16, off) : mix_kernel_of<MixW::kE4m3, false>(bf16, off);
-    }
-}
-
-// The kernel of a call, ready to launch on the current device, and its plan.
-cudaError_t mix_prepare(const OpsnnWqbmmParams* p, MixKernel* kern, MixPlan* plan)
-{
-    static std::atomic<uint64_t> configured[24];
-    int index = 0;
-    const MixKernel k = mix_kernel(p, &index);
-    const cudaError_t rc = once_per_device(configured[index], [&] {
+    const MixKernel k = sum == MixSum::kChain    ? mix_kernel_of<MixSum::kChain>(w, nk, bf16, off)
+                        : sum == MixSum::kCopies ? mix_kernel_of<MixSum::kCopies>(w, nk, bf16, off)
+                                                 : mix_kernel_of<MixSum::kChunks>(w, nk, bf16, off);
+    *kern = k;
+    return once_per_device(configured[(int)sum * 24 + w * 8 + (nk ? 4 : 0) + (bf16 ? 2 : 0) + (off ? 1 : 0)], [&] {
         cudaFuncSetAttribute(k, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
         return cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, kMixSmemMax);
     });
-    if (rc != cudaSuccess) return rc;
-    *kern = k;
-    *plan = mix_plan(p, current_sm_count(), [&](int s) { return max_active_clusters(reinterpret_cast<const void*>(k), kMixThreads, kMixSmemMax, s, 0); });
-    return cudaSuccess;
+}
+
+// A call's plan and its kernel. (Every form takes an SM for itself, so clusters of one are placed as those of the others.)
+cudaError_t mix_prepare(const OpsnnWqbmmParams* p, MixKernel* kern, MixPlan* plan)
+{
+    MixKernel any;
+    if (const cudaError_t rc = mix_kernel(p, MixSum::kCopies, &any); rc != cudaSuccess) return rc;
+    *plan = mix_plan(p, current_sm_count(), [&](int s) { return max_active_clusters(reinterpret_cast<const void*>(any), kMixThreads, kMixSmemMax, s, 0); });
+    return mix_kernel(p, plan->sum, kern);
 }
 
 }  // namespace
@@ -947,6 +1083,8 @@ int32_t wqbmm_mixed_launch(const OpsnnWqbmmParams* p, cudaStream_t stream)
     a.units = (uint32_t)q.units;
     a.grid = (uint32_t)q.grid;
     a.split = (uint32_t)q.split;
+    a.copies = (uint32_t)q.copies;
+    a.chunk = (uint32_t)q.chunk;
     a.group = p->group_size > 0 ? (uint32_t)p->group_size : 0x7FFFFFFFu;
     a.sc_rows = p->group_size % 128 == 0 ? 1 : 2;
     {
