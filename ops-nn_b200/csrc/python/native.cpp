@@ -51,6 +51,17 @@ PyObject* guarded(F&& f)
     return nullptr;
 }
 
+// Python's lock given up while the library plans and launches and torch's allocator works: a launch waits where the stream's queue is full,
+// an allocation in cudaMalloc, a first call for the module to load, and other threads of the program go on meanwhile. Comes back on every
+// way out, so that errors are raised with the lock held.
+struct Unlocked {
+    PyThreadState* state = PyEval_SaveThread();
+    ~Unlocked() { PyEval_RestoreThread(state); }
+    Unlocked() = default;
+    Unlocked(const Unlocked&) = delete;
+    Unlocked& operator=(const Unlocked&) = delete;
+};
+
 [[noreturn]] void fail_call(const char* api, aclnnStatus status)
 {
     PyObject* err = PyObject_CallFunction(g_call_error, "si", api, (int)status);
@@ -116,9 +127,9 @@ int code_of(PyObject* dtype)  // a name of aclnn.DTYPE_BY_NAME or an aclDataType
     return (int)as_int(dtype);
 }
 
-int code_of(const at::Tensor& t)
+int code_of(at::ScalarType type)
 {
-    switch (t.scalar_type()) {
+    switch (type) {
         case at::kFloat: return ACL_FLOAT;
         case at::kHalf: return ACL_FLOAT16;
         case at::kBFloat16: return ACL_BF16;
@@ -131,9 +142,10 @@ int code_of(const at::Tensor& t)
         case at::ScalarType::Float8_e5m2: return ACL_FLOAT8_E5M2;
         default: break;
     }
-    PyErr_Format(PyExc_KeyError, "torch.%s has no aclDataType", c10::toString(t.scalar_type()));
+    PyErr_Format(PyExc_KeyError, "torch.%s has no aclDataType", c10::toString(type));
     throw PyFail{};
 }
+int code_of(const at::Tensor& t) { return code_of(t.scalar_type()); }
 
 const at::Tensor* tensor_of(PyObject* o, const char* what)  // nullptr for None
 {
@@ -187,14 +199,13 @@ void need_cuda(c10::Device device)
     throw PyFail{};
 }
 
-// A workspace block of torch's allocator on the current stream.
+// A workspace block of torch's allocator on the current stream of `device`, a CUDA device (need_cuda).
 struct Workspace {
     c10::DataPtr block;
     void* ptr = nullptr;
     Workspace(uint64_t bytes, c10::Device device)
     {
         if (bytes == 0) return;
-        need_cuda(device);
         const c10::cuda::OptionalCUDAGuard guard(device);
         block = c10::cuda::CUDACachingAllocator::get()->allocate(bytes);
         ptr = block.get();
@@ -218,11 +229,9 @@ struct Plan {
 
 void* stream() { return c10::cuda::getCurrentCUDAStream().stream(); }
 
-PyObject* empty_output(c10::IntArrayRef sizes, at::ScalarType type, c10::Device device, at::Tensor* out)
+PyObject* wrap(const at::Tensor& out)
 {
-    need_cuda(device);
-    *out = at::Tensor(at::detail::empty_cuda(sizes, type, device, std::nullopt));
-    PyObject* o = THPVariable_Wrap(*out);
+    PyObject* o = THPVariable_Wrap(out);
     if (o == nullptr) throw PyFail{};
     return o;
 }
@@ -231,12 +240,6 @@ PyObject* empty_output(c10::IntArrayRef sizes, at::ScalarType type, c10::Device 
 struct Ref {
     PyObject* o;
     ~Ref() { Py_XDECREF(o); }
-    PyObject* release()
-    {
-        PyObject* r = o;
-        o = nullptr;
-        return r;
-    }
 };
 
 bool arity(Py_ssize_t got, Py_ssize_t want, const char* name)
@@ -272,17 +275,29 @@ PyObject* npu_quant_matmul(PyObject*, PyObject* const* a, Py_ssize_t na)
         shape.assign(batched.sizes().data(), batched.sizes().data() + (batched.dim() - 2));
         shape.push_back(x1.dim(-2));
         shape.push_back(x2.dim(-1));
+        const at::ScalarType type = reinterpret_cast<THPDtype*>(a[6])->scalar_type;
+        const c10::Device device = t1->device();
+        need_cuda(device);
+        const int out_code = code_of(type);
+        const int64_t group = as_int(a[7]);
         at::Tensor out;
-        Ref ret{empty_output(c10::IntArrayRef(shape.begin(), shape.size()), reinterpret_cast<THPDtype*>(a[6])->scalar_type, t1->device(), &out)};
-        fill(&y, out, code_of(out));
-        uint64_t ws = 0;
-        Plan plan;
-        check_call("aclnnQuantMatmulV5GetWorkspaceSize",
-                   aclnnQuantMatmulV5GetWorkspaceSize(&x1, &x2, ptp, scp, nullptr, nullptr, ofp, nullptr, bip, false, false, as_int(a[7]), &y, &ws,
-                                                      &plan.ex));
-        Workspace w(ws, t1->device());
-        check_call("aclnnQuantMatmulV5", aclnnQuantMatmulV5(w.ptr, ws, plan.take(), stream()));
-        return ret.release();
+        const char* api = "aclnnQuantMatmulV5GetWorkspaceSize";
+        aclnnStatus status;
+        {
+            const Unlocked unlocked;
+            out = at::Tensor(at::detail::empty_cuda(c10::IntArrayRef(shape.begin(), shape.size()), type, device, std::nullopt));
+            fill(&y, out, out_code);
+            uint64_t ws = 0;
+            Plan plan;
+            status = aclnnQuantMatmulV5GetWorkspaceSize(&x1, &x2, ptp, scp, nullptr, nullptr, ofp, nullptr, bip, false, false, group, &y, &ws, &plan.ex);
+            if (status == ACLNN_SUCCESS) {
+                const Workspace w(ws, device);
+                api = "aclnnQuantMatmulV5";
+                status = aclnnQuantMatmulV5(w.ptr, ws, plan.take(), stream());
+            }
+        }
+        check_call(api, status);
+        return wrap(out);
     });
 }
 
@@ -303,17 +318,27 @@ PyObject* npu_weight_quant_batchmatmul(PyObject*, PyObject* const* a, Py_ssize_t
         const aclTensor* ofp = describe(a[3], Py_None, "antiquant_offset", &of);
         const aclTensor* bip = describe(a[4], Py_None, "bias", &bi);
         const int64_t shape[2] = {tx->size(0), tw->size(-1) * (tw->scalar_type() == at::kInt && tw->stride(-1) == 1 ? 8 : 1)};
+        const c10::Device device = tx->device();
+        need_cuda(device);
+        const int out_code = code_of(*tx), group = (int)as_int(a[5]), inner_precise = (int)as_int(a[6]);
         at::Tensor out;
-        Ref ret{empty_output(c10::IntArrayRef(shape, 2), tx->scalar_type(), tx->device(), &out)};
-        fill(&y, out, code_of(out));
-        uint64_t ws = 0;
-        Plan plan;
-        check_call("aclnnWeightQuantBatchMatmulV3GetWorkspaceSize",
-                   aclnnWeightQuantBatchMatmulV3GetWorkspaceSize(&x, &w, scp, ofp, nullptr, nullptr, bip, (int)as_int(a[5]), (int)as_int(a[6]), &y, &ws,
-                                                                 &plan.ex));
-        Workspace space(ws, tx->device());
-        check_call("aclnnWeightQuantBatchMatmulV3", aclnnWeightQuantBatchMatmulV3(space.ptr, ws, plan.take(), stream()));
-        return ret.release();
+        const char* api = "aclnnWeightQuantBatchMatmulV3GetWorkspaceSize";
+        aclnnStatus status;
+        {
+            const Unlocked unlocked;
+            out = at::Tensor(at::detail::empty_cuda(c10::IntArrayRef(shape, 2), tx->scalar_type(), device, std::nullopt));
+            fill(&y, out, out_code);
+            uint64_t ws = 0;
+            Plan plan;
+            status = aclnnWeightQuantBatchMatmulV3GetWorkspaceSize(&x, &w, scp, ofp, nullptr, nullptr, bip, group, inner_precise, &y, &ws, &plan.ex);
+            if (status == ACLNN_SUCCESS) {
+                const Workspace space(ws, device);
+                api = "aclnnWeightQuantBatchMatmulV3";
+                status = aclnnWeightQuantBatchMatmulV3(space.ptr, ws, plan.take(), stream());
+            }
+        }
+        check_call(api, status);
+        return wrap(out);
     });
 }
 
@@ -456,50 +481,59 @@ PyObject* from_torch(PyObject*, PyObject* args, PyObject* kw)
     });
 }
 
-// The workspace of a two-phase call on descriptors: the caller's tensor where it is large enough, else a block of the allocator on the
-// device of the output's storage.
-struct CallWorkspace {
-    void* ptr = nullptr;
-    uint64_t bytes = 0;
-    std::optional<Workspace> own;
-    CallWorkspace(uint64_t need, PyObject* given, const TensorObject* out)
+// Both phases of a call on descriptors: its workspace is the caller's tensor where that is large enough, else a block of the allocator on
+// the device of the output's storage. Returns the workspace size that the plan asked for.
+template <typename Phase1, typename Phase2>
+PyObject* run_on_descriptors(const char* api1, const char* api2, PyObject* given, const TensorObject* out, Phase1&& phase1, Phase2&& phase2)
+{
+    const at::Tensor* t = tensor_of(given, "workspace");
+    void* const given_ptr = t != nullptr ? t->data_ptr() : nullptr;
+    const uint64_t given_bytes = t != nullptr ? (uint64_t)t->numel() : 0;
+    const bool backed = out != nullptr && out->keep != nullptr && THPVariable_Check(out->keep);
+    const c10::Device device = backed ? THPVariable_Unpack(out->keep).device() : c10::Device(c10::kCPU);
+    uint64_t ws = 0;
+    const char* api = api1;
+    aclnnStatus status;
+    bool no_workspace = false;
     {
-        bytes = need;
-        if (given != Py_None) {
-            const at::Tensor& t = *tensor_of(given, "workspace");
-            if ((uint64_t)t.numel() >= need) {
-                ptr = t.data_ptr();
-                bytes = (uint64_t)t.numel();
-                return;
+        const Unlocked unlocked;
+        Plan plan;
+        status = phase1(&ws, &plan.ex);
+        if (status == ACLNN_SUCCESS) {
+            const bool own = t == nullptr || given_bytes < ws;
+            no_workspace = own && ws != 0 && !device.is_cuda();
+            if (!no_workspace) {
+                const Workspace w(own ? ws : 0, device);
+                api = api2;
+                status = phase2(own ? w.ptr : given_ptr, own ? ws : given_bytes, plan.take(), stream());
             }
         }
-        if (need == 0) return;
-        if (out == nullptr || !THPVariable_Check(out->keep)) {
-            PyErr_SetString(PyExc_AttributeError, "a workspace is needed and the output descriptor is not backed by a torch tensor");
-            throw PyFail{};
-        }
-        own.emplace(need, THPVariable_Unpack(out->keep).device());
-        ptr = own->ptr;
     }
-};
+    if (no_workspace) {
+        if (backed) need_cuda(device);
+        PyErr_SetString(PyExc_AttributeError, "a workspace is needed and the output descriptor is not backed by a torch tensor");
+        throw PyFail{};
+    }
+    check_call(api, status);
+    return PyLong_FromUnsignedLongLong(ws);
+}
 
 // quant_matmul_v5(x1, x2, x1_scale, x2_scale, out, bias, transpose_x1, transpose_x2, group_size, x2_offset, workspace, y_scale, weight_nz)
 PyObject* quant_matmul_v5(PyObject*, PyObject* const* a, Py_ssize_t na)
 {
     if (!arity(na, 13, "quant_matmul_v5")) return nullptr;
     return guarded([&]() -> PyObject* {
-        const bool nz = PyObject_IsTrue(a[12]) != 0;
+        const bool nz = PyObject_IsTrue(a[12]) != 0, tr1 = PyObject_IsTrue(a[6]) != 0, tr2 = PyObject_IsTrue(a[7]) != 0;
+        const aclTensor *x1 = handle_of(a[0], "x1"), *x2 = handle_of(a[1], "x2"), *s1 = handle_of(a[2], "x1_scale"), *s2 = handle_of(a[3], "x2_scale");
+        const aclTensor *ys = handle_of(a[11], "y_scale"), *of = handle_of(a[9], "x2_offset"), *bi = handle_of(a[5], "bias");
+        aclTensor* const out = handle_of(a[4], "out");
+        const int64_t group = as_int(a[8]);
         const auto phase1 = nz ? aclnnQuantMatmulWeightNzGetWorkspaceSize : aclnnQuantMatmulV5GetWorkspaceSize;
-        uint64_t ws = 0;
-        Plan plan;
-        check_call(nz ? "aclnnQuantMatmulWeightNzGetWorkspaceSize" : "aclnnQuantMatmulV5GetWorkspaceSize",
-                   phase1(handle_of(a[0], "x1"), handle_of(a[1], "x2"), handle_of(a[2], "x1_scale"), handle_of(a[3], "x2_scale"),
-                          handle_of(a[11], "y_scale"), nullptr, handle_of(a[9], "x2_offset"), nullptr, handle_of(a[5], "bias"),
-                          PyObject_IsTrue(a[6]) != 0, PyObject_IsTrue(a[7]) != 0, as_int(a[8]), handle_of(a[4], "out"), &ws, &plan.ex));
-        CallWorkspace w(ws, a[10], desc_of(a[4], "out"));
-        if (nz) check_call("aclnnQuantMatmulWeightNz", aclnnQuantMatmulWeightNz(w.ptr, w.bytes, plan.take(), stream()));
-        else check_call("aclnnQuantMatmulV5", aclnnQuantMatmulV5(w.ptr, w.bytes, plan.take(), stream()));
-        return PyLong_FromUnsignedLongLong(ws);
+        const auto phase2 = nz ? aclnnQuantMatmulWeightNz : aclnnQuantMatmulV5;
+        return run_on_descriptors(
+            nz ? "aclnnQuantMatmulWeightNzGetWorkspaceSize" : "aclnnQuantMatmulV5GetWorkspaceSize", nz ? "aclnnQuantMatmulWeightNz" : "aclnnQuantMatmulV5",
+            a[10], desc_of(a[4], "out"),
+            [&](uint64_t* ws, aclOpExecutor** ex) { return phase1(x1, x2, s1, s2, ys, nullptr, of, nullptr, bi, tr1, tr2, group, out, ws, ex); }, phase2);
     });
 }
 
@@ -508,28 +542,31 @@ PyObject* weight_quant_batch_matmul(PyObject*, PyObject* const* a, Py_ssize_t na
 {
     if (!arity(na, 9, "weight_quant_batch_matmul")) return nullptr;
     return guarded([&]() -> PyObject* {
-        aclTensor *x = handle_of(a[0], "x"), *w = handle_of(a[1], "weight"), *sc = handle_of(a[2], "antiquant_scale"), *y = handle_of(a[3], "y");
-        aclTensor *of = handle_of(a[4], "antiquant_offset"), *bi = handle_of(a[5], "bias");
+        const aclTensor *x = handle_of(a[0], "x"), *w = handle_of(a[1], "weight"), *sc = handle_of(a[2], "antiquant_scale"), *y = handle_of(a[3], "y");
+        const aclTensor *of = handle_of(a[4], "antiquant_offset"), *bi = handle_of(a[5], "bias");
+        const TensorObject* out = desc_of(a[3], "y");
         const int group = (int)as_int(a[6]);
-        uint64_t ws = 0;
-        Plan plan;
-        if (a[7] == Py_None) {
-            check_call("aclnnWeightQuantBatchMatmulV2GetWorkspaceSize",
-                       aclnnWeightQuantBatchMatmulV2GetWorkspaceSize(x, w, sc, of, nullptr, nullptr, bi, group, y, &ws, &plan.ex));
-            CallWorkspace space(ws, a[8], desc_of(a[3], "y"));
-            check_call("aclnnWeightQuantBatchMatmulV2", aclnnWeightQuantBatchMatmulV2(space.ptr, space.bytes, plan.take(), stream()));
-        } else if (PyUnicode_Check(a[7]) && PyUnicode_CompareWithASCIIString(a[7], "nz") == 0) {
-            check_call("aclnnWeightQuantBatchMatmulNzGetWorkspaceSize",
-                       aclnnWeightQuantBatchMatmulNzGetWorkspaceSize(x, w, sc, of, nullptr, nullptr, bi, group, y, &ws, &plan.ex));
-            CallWorkspace space(ws, a[8], desc_of(a[3], "y"));
-            check_call("aclnnWeightQuantBatchMatmulNz", aclnnWeightQuantBatchMatmulNz(space.ptr, space.bytes, plan.take(), stream()));
-        } else {
-            check_call("aclnnWeightQuantBatchMatmulV3GetWorkspaceSize",
-                       aclnnWeightQuantBatchMatmulV3GetWorkspaceSize(x, w, sc, of, nullptr, nullptr, bi, group, (int)as_int(a[7]), y, &ws, &plan.ex));
-            CallWorkspace space(ws, a[8], desc_of(a[3], "y"));
-            check_call("aclnnWeightQuantBatchMatmulV3", aclnnWeightQuantBatchMatmulV3(space.ptr, space.bytes, plan.take(), stream()));
-        }
-        return PyLong_FromUnsignedLongLong(ws);
+        if (a[7] == Py_None)
+            return run_on_descriptors(
+                "aclnnWeightQuantBatchMatmulV2GetWorkspaceSize", "aclnnWeightQuantBatchMatmulV2", a[8], out,
+                [&](uint64_t* ws, aclOpExecutor** ex) {
+                    return aclnnWeightQuantBatchMatmulV2GetWorkspaceSize(x, w, sc, of, nullptr, nullptr, bi, group, y, ws, ex);
+                },
+                aclnnWeightQuantBatchMatmulV2);
+        if (PyUnicode_Check(a[7]) && PyUnicode_CompareWithASCIIString(a[7], "nz") == 0)
+            return run_on_descriptors(
+                "aclnnWeightQuantBatchMatmulNzGetWorkspaceSize", "aclnnWeightQuantBatchMatmulNz", a[8], out,
+                [&](uint64_t* ws, aclOpExecutor** ex) {
+                    return aclnnWeightQuantBatchMatmulNzGetWorkspaceSize(x, w, sc, of, nullptr, nullptr, bi, group, y, ws, ex);
+                },
+                aclnnWeightQuantBatchMatmulNz);
+        const int inner_precise = (int)as_int(a[7]);
+        return run_on_descriptors(
+            "aclnnWeightQuantBatchMatmulV3GetWorkspaceSize", "aclnnWeightQuantBatchMatmulV3", a[8], out,
+            [&](uint64_t* ws, aclOpExecutor** ex) {
+                return aclnnWeightQuantBatchMatmulV3GetWorkspaceSize(x, w, sc, of, nullptr, nullptr, bi, group, inner_precise, y, ws, ex);
+            },
+            aclnnWeightQuantBatchMatmulV3);
     });
 }
 
@@ -543,12 +580,22 @@ PyObject* dynamic_mx_quant(PyObject*, PyObject* const* a, Py_ssize_t na)
             mode = PyBytes_AsString(a[5]);
             if (mode == nullptr) throw PyFail{};
         }
-        uint64_t ws = 0;
-        Plan plan;
-        check_call("aclnnDynamicMxQuantGetWorkspaceSize",
-                   aclnnDynamicMxQuantGetWorkspaceSize(handle_of(a[0], "x"), as_int(a[4]), mode, code_of(a[3]), as_int(a[6]), as_int(a[7]),
-                                                       handle_of(a[1], "y_out"), handle_of(a[2], "mxscale_out"), &ws, &plan.ex));
-        check_call("aclnnDynamicMxQuant", aclnnDynamicMxQuant(nullptr, 0, plan.take(), stream()));
+        const aclTensor *x = handle_of(a[0], "x"), *y = handle_of(a[1], "y_out"), *sc = handle_of(a[2], "mxscale_out");
+        const int64_t axis = as_int(a[4]), block = as_int(a[6]), alg = as_int(a[7]);
+        const int dst = code_of(a[3]);
+        const char* api = "aclnnDynamicMxQuantGetWorkspaceSize";
+        aclnnStatus status;
+        {
+            const Unlocked unlocked;
+            uint64_t ws = 0;
+            Plan plan;
+            status = aclnnDynamicMxQuantGetWorkspaceSize(x, axis, mode, dst, block, alg, y, sc, &ws, &plan.ex);
+            if (status == ACLNN_SUCCESS) {
+                api = "aclnnDynamicMxQuant";
+                status = aclnnDynamicMxQuant(nullptr, 0, plan.take(), stream());
+            }
+        }
+        check_call(api, status);
         Py_RETURN_NONE;
     });
 }
