@@ -168,7 +168,7 @@ void fill(aclTensor* d, const at::Tensor& t, int code)
     d->strides.assign(strides.data(), strides.data() + strides.size());
     d->storage_shape = d->shape;
     d->dtype = (aclDataType)code;
-    d->data = const_cast<void*>(t.const_data_ptr());
+    d->data = t.data_ptr();
 }
 
 // The descriptor of an optional argument: `dtype` (None, a name or a code) names the element type of storage that torch cannot type
@@ -399,7 +399,7 @@ PyObject* tensor_new(PyTypeObject*, PyObject* args, PyObject* kw)
             ptr = PyLong_AsVoidPtr(data);
             if (ptr == nullptr && PyErr_Occurred()) throw PyFail{};
         } else if (THPVariable_Check(data)) {
-            ptr = const_cast<void*>(THPVariable_Unpack(data).const_data_ptr());
+            ptr = THPVariable_Unpack(data).data_ptr();
         } else if (data != Py_None) {
             Ref r{PyObject_CallMethod(data, "data_ptr", nullptr)};
             if (r.o == nullptr) throw PyFail{};
