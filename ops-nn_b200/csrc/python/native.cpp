@@ -114,6 +114,17 @@ opsnn::Dims as_dims(PyObject* o)
     return d;
 }
 
+opsnn::Dims as_strides(PyObject* o, const opsnn::Dims& shape)  // what is missing is 0
+{
+    opsnn::Dims d = as_dims(o);
+    if (d.size() > shape.size()) {
+        PyErr_SetString(PyExc_IndexError, "more strides than dims");
+        throw PyFail{};
+    }
+    d.resize(shape.size());
+    return d;
+}
+
 int code_of(PyObject* dtype)  // a name of aclnn.DTYPE_BY_NAME or an aclDataType value
 {
     if (PyUnicode_Check(dtype)) {
@@ -349,11 +360,13 @@ struct TensorObject {
     PyObject* shape;   // tuple
     PyObject* keep;    // what backs the view: a torch tensor, an address, or None
     PyObject* handle;  // the aclTensor's address, or None once it has been destroyed
+    PyObject* dict;    // as a class written in Python has them: attributes, weak references, subclasses, cycles collected
+    PyObject* weak;
     int dtype;
 };
 PyTypeObject* g_tensor_type = nullptr;
 
-PyObject* new_tensor(const opsnn::Dims& shape, int code, void* data, PyObject* keep, const opsnn::Dims* strides, int64_t offset, int format,
+PyObject* new_tensor(PyTypeObject* type, const opsnn::Dims& shape, int code, void* data, PyObject* keep, const opsnn::Dims* strides, int64_t offset, int format,
                      const opsnn::Dims& storage)
 {
     aclTensor* d = aclCreateTensor(shape.begin(), shape.size(), (aclDataType)code, strides ? strides->begin() : nullptr, offset, (aclFormat)format,
@@ -362,7 +375,7 @@ PyObject* new_tensor(const opsnn::Dims& shape, int code, void* data, PyObject* k
         PyErr_SetString(PyExc_ValueError, "aclCreateTensor rejected the arguments");
         throw PyFail{};
     }
-    TensorObject* t = reinterpret_cast<TensorObject*>(g_tensor_type->tp_alloc(g_tensor_type, 0));
+    TensorObject* t = reinterpret_cast<TensorObject*>(type->tp_alloc(type, 0));
     if (t == nullptr) {
         aclDestroyTensor(d);
         throw PyFail{};
@@ -376,7 +389,7 @@ PyObject* new_tensor(const opsnn::Dims& shape, int code, void* data, PyObject* k
     return reinterpret_cast<PyObject*>(t);
 }
 
-PyObject* tensor_new(PyTypeObject*, PyObject* args, PyObject* kw)
+PyObject* tensor_new(PyTypeObject* type, PyObject* args, PyObject* kw)
 {
     static const char* names[] = {"shape", "dtype", "data", "strides", "offset", "fmt", "storage_shape", nullptr};
     PyObject *shape = nullptr, *dtype = nullptr, *data = nullptr, *strides = Py_None, *storage = Py_None;
@@ -387,11 +400,7 @@ PyObject* tensor_new(PyTypeObject*, PyObject* args, PyObject* kw)
     return guarded([&]() -> PyObject* {
         const opsnn::Dims dims = as_dims(shape);
         opsnn::Dims st;
-        if (strides != Py_None) st = as_dims(strides);
-        if (strides != Py_None && st.size() != dims.size()) {
-            PyErr_SetString(PyExc_ValueError, "strides must have one entry per dim");
-            throw PyFail{};
-        }
+        if (strides != Py_None) st = as_strides(strides, dims);
         Ref zero{PyLong_FromLong(0)};
         if (data == nullptr) data = zero.o;
         void* ptr = nullptr;
@@ -406,20 +415,38 @@ PyObject* tensor_new(PyTypeObject*, PyObject* args, PyObject* kw)
             ptr = PyLong_AsVoidPtr(r.o);
             if (ptr == nullptr && PyErr_Occurred()) throw PyFail{};
         }
-        return new_tensor(dims, code_of(dtype), ptr, data, strides == Py_None ? nullptr : &st, offset, format,
+        return new_tensor(type, dims, code_of(dtype), ptr, data, strides == Py_None ? nullptr : &st, offset, format,
                           storage == Py_None ? dims : as_dims(storage));
     });
 }
 
-void tensor_dealloc(PyObject* o)
+int tensor_traverse(PyObject* o, visitproc visit, void* arg)
 {
     TensorObject* t = reinterpret_cast<TensorObject*>(o);
+    Py_VISIT(Py_TYPE(o));
+    Py_VISIT(t->shape);
+    Py_VISIT(t->keep);
+    Py_VISIT(t->dict);
+    return 0;
+}
+int tensor_clear(PyObject* o)
+{
+    TensorObject* t = reinterpret_cast<TensorObject*>(o);
+    Py_CLEAR(t->keep);
+    Py_CLEAR(t->dict);
+    return 0;
+}
+void tensor_dealloc(PyObject* o)
+{
+    PyObject_GC_UnTrack(o);
+    TensorObject* t = reinterpret_cast<TensorObject*>(o);
+    if (t->weak != nullptr) PyObject_ClearWeakRefs(o);
     if (t->handle != nullptr && PyLong_Check(t->handle)) {
         if (void* p = PyLong_AsVoidPtr(t->handle)) aclDestroyTensor(static_cast<aclTensor*>(p));
     }
     Py_XDECREF(t->handle);
     Py_XDECREF(t->shape);
-    Py_XDECREF(t->keep);
+    tensor_clear(o);
     PyTypeObject* type = Py_TYPE(o);
     type->tp_free(o);
     Py_DECREF(type);
@@ -430,21 +457,27 @@ PyMemberDef tensor_members[] = {
     {"dtype", T_INT, offsetof(TensorObject, dtype), 0, "aclDataType"},
     {"handle", T_OBJECT, offsetof(TensorObject, handle), 0, "address of the aclTensor, None when destroyed"},
     {"_keep", T_OBJECT, offsetof(TensorObject, keep), 0, "what backs the view"},
+    {"__dictoffset__", T_PYSSIZET, offsetof(TensorObject, dict), READONLY, nullptr},
+    {"__weaklistoffset__", T_PYSSIZET, offsetof(TensorObject, weak), READONLY, nullptr},
     {nullptr, 0, 0, 0, nullptr},
 };
+PyGetSetDef tensor_getset[] = {{"__dict__", PyObject_GenericGetDict, PyObject_GenericSetDict, nullptr, nullptr}, {nullptr, nullptr, nullptr, nullptr, nullptr}};
 PyType_Slot tensor_slots[] = {
     {Py_tp_new, reinterpret_cast<void*>(tensor_new)},
     {Py_tp_dealloc, reinterpret_cast<void*>(tensor_dealloc)},
+    {Py_tp_traverse, reinterpret_cast<void*>(tensor_traverse)},
+    {Py_tp_clear, reinterpret_cast<void*>(tensor_clear)},
+    {Py_tp_getset, tensor_getset},
     {Py_tp_members, tensor_members},
     {Py_tp_doc, const_cast<char*>("An aclTensor descriptor. `data` is a device address (int) or a torch tensor whose storage backs the view.")},
     {0, nullptr},
 };
-PyType_Spec tensor_spec = {"ops_nn_b200.Tensor", sizeof(TensorObject), 0, Py_TPFLAGS_DEFAULT, tensor_slots};
+PyType_Spec tensor_spec = {"ops_nn_b200.aclnn.Tensor", sizeof(TensorObject), 0, Py_TPFLAGS_DEFAULT | Py_TPFLAGS_BASETYPE | Py_TPFLAGS_HAVE_GC, tensor_slots};
 
 const TensorObject* desc_of(PyObject* o, const char* what)  // nullptr for None
 {
     if (o == Py_None) return nullptr;
-    if (Py_TYPE(o) != g_tensor_type) {
+    if (!PyObject_TypeCheck(o, g_tensor_type)) {
         PyErr_Format(PyExc_TypeError, "%s must be an aclnn.Tensor, got %s", what, Py_TYPE(o)->tp_name);
         throw PyFail{};
     }
@@ -469,15 +502,11 @@ PyObject* from_torch(PyObject*, PyObject* args, PyObject* kw)
         const at::Tensor& v = *tensor_of(t, "t");
         aclTensor d;
         fill(&d, v, dtype == Py_None ? code_of(v) : code_of(dtype));
-        if (shape == Py_None) return new_tensor(d.shape, d.dtype, d.data, t, &d.strides, 0, ACL_FORMAT_ND, d.shape);
+        if (shape == Py_None) return new_tensor(g_tensor_type, d.shape, d.dtype, d.data, t, &d.strides, 0, ACL_FORMAT_ND, d.shape);
         const opsnn::Dims dims = as_dims(shape);
         opsnn::Dims st;
-        if (strides != Py_None) st = as_dims(strides);
-        if (strides != Py_None && st.size() != dims.size()) {
-            PyErr_SetString(PyExc_ValueError, "strides must have one entry per dim");
-            throw PyFail{};
-        }
-        return new_tensor(dims, d.dtype, d.data, t, strides == Py_None ? nullptr : &st, 0, ACL_FORMAT_ND, dims);
+        if (strides != Py_None) st = as_strides(strides, dims);
+        return new_tensor(g_tensor_type, dims, d.dtype, d.data, t, strides == Py_None ? nullptr : &st, 0, ACL_FORMAT_ND, dims);
     });
 }
 
