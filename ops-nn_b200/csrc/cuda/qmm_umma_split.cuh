@@ -727,7 +727,7 @@ int32_t split_launch(const OpsnnQmmParams* p, cudaStream_t stream)
     cfg.attrs = attr;
     cfg.numAttrs = a.split > 1u ? 2 : 1;
     const int32_t rc = (int32_t)cudaLaunchKernelEx(&cfg, kern, mw, mx, a);
-    note_launch(pb ? "qmm_umma_perblock" : "qmm_umma_deq");
+    note_launch(pb ? "qmm_umma_split_perblock" : "qmm_umma_split_deq");
     return rc;
 }
 

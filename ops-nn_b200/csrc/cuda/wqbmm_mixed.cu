@@ -1136,7 +1136,7 @@ int32_t wqbmm_mixed_launch(const OpsnnWqbmmParams* p, cudaStream_t stream)
     cfg.attrs = attr;
     cfg.numAttrs = a.split > 1u ? 2 : 1;
     const int32_t rc = (int32_t)cudaLaunchKernelEx(&cfg, kern, mw, mx, a);
-    note_launch(p->w_dtype == ACL_INT4 ? "wqbmm_decode" : "wqbmm_decode8");
+    note_launch("wqbmm_mixed");
     return rc;
 }
 

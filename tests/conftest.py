@@ -44,6 +44,13 @@ def aclnn(pkg):
     return pkg.aclnn
 
 
+@pytest.fixture
+def streaming(monkeypatch):
+    """For tests of the streaming decode kernels and of dequantise-then-matmul: keeps their calls off the fused weight-only kernel, which
+    they run on otherwise."""
+    monkeypatch.setenv("OPSNN_WQ_NO_MIXED", "1")
+
+
 @pytest.fixture(autouse=True)
 def _device_status_words(request):
     """After every GPU test: no kernel of the library may have given up a bounded wait. A give-up leaves the output

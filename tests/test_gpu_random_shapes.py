@@ -106,17 +106,22 @@ def test_weight_only_random_shapes(aclnn, seed):
         assert np.all(np.abs(got - wv) <= 2 * ulp * np.maximum(np.abs(wv), 0.05 * rms) * 1.01), tag
 
 
+@pytest.mark.parametrize("fused", [False, True], ids=["streaming", "fused"])
 @pytest.mark.parametrize("seed", [11, 12, 13])
-def test_streaming_decode_kernels_random_shapes(aclnn, seed):
+def test_streaming_decode_kernels_random_shapes(aclnn, monkeypatch, seed, fused):
     """Weights large enough (k n >= 2^20) for the streaming decode kernels at m <= 16, every kind they take - INT4 in int32 words,
     INT8, FLOAT8_E4M3FN, each stored (k,n) or (n,k) with the scales stored the same way - ragged strips, k that is not a multiple of
     a stage, per-channel and per-group scales, offsets, bias: within 1 ulp of the output dtype of the oracle (fp32 summation order
-    is the only difference), and most draws must really have run on a streaming kernel."""
+    is the only difference), and most draws must really have run on a streaming kernel. The same draws on the fused kernel, which such calls
+    run on by default."""
     import torch
 
     from gpu_util import desc, out_tensor, out_to_np
 
     rng = np.random.default_rng(seed)
+    if not fused:
+        monkeypatch.setenv("OPSNN_WQ_NO_MIXED", "1")
+    names = ("wqbmm_mixed",) if fused else ("wqbmm_decode", "wqbmm_decode8")
     streamed = 0
     draws = 12
     for _ in range(draws):
@@ -160,7 +165,7 @@ def test_streaming_decode_kernels_random_shapes(aclnn, seed):
         out = out_tensor((m, n), name)
         aclnn.weight_quant_batch_matmul(desc(aclnn, x), d_w, sdesc(scale), aclnn.Tensor((m, n), name, out), sdesc(offset), desc(aclnn, bias), g)
         torch.cuda.synchronize()
-        streamed += aclnn.last_kernel_name() in ("wqbmm_decode", "wqbmm_decode8")
+        streamed += aclnn.last_kernel_name() in names
         assert aclnn.lib().opsnn_wqbmm_decode_status(1) == 0, tag
         got, wv = out_to_np(out).astype(np.float64), want.astype(np.float64)
         assert not np.any(got == -7777.0), tag

@@ -50,7 +50,7 @@ INT8_CASES = [
     (300, 400, 384, False, False, 64, True, "i32", "bfloat16"),      # n-major B in the 64-byte swizzle
     (130, 528, 208, False, False, 32, True, "f32", "float16"),       # n-major B in the 32-byte swizzle, n tail
     (272, 528, 400, True, False, 32, False, None, "bfloat16"),       # both operands stored along m / n
-    (128, 4096, 1024, False, False, None, True, "i32", "bfloat16"),  # few tiles: the host picks a narrow tile by itself
+    (128, 4096, 1024, False, False, None, True, "i32", "bfloat16"),  # few tiles: the host cuts k by itself
     (2200, 256, 304, False, False, 128, True, "i32", "bfloat16"),    # 18 tile rows: a band of 16 and a ragged band of 2
 ]
 
@@ -66,7 +66,8 @@ def test_int8_dequant_bit_exact(aclnn, case):
     bias = {None: None, "i32": rng.integers(-1000, 1001, n).astype(np.int32), "f32": rng.uniform(-1, 1, n).astype(np.float32),
             "bf16": rng.uniform(-1, 1, n).astype(np.float32).astype(ml_dtypes.bfloat16)}[bias_kind]
     want = qbmm_oracle.quant_matmul_v5(x1, x2, s1, s2, bias, t1, t2, 0, out_name)
-    got = _run(aclnn, x1, x2, s1, s2, bias, t1, t2, 0, out_name, "qmm_umma_deq", bn)
+    kernel = "qmm_umma_split_deq" if (m, n) in ((1, 16), (128, 1024)) else "qmm_umma_deq"  # few tiles, no tile width asked for
+    got = _run(aclnn, x1, x2, s1, s2, bias, t1, t2, 0, out_name, kernel, bn)
     assert np.array_equal(np.asarray(got).view(np.uint8), np.asarray(want).view(np.uint8)), \
         "%d of %d elements differ" % ((np.asarray(got).astype(np.float64) != np.asarray(want).astype(np.float64)).sum(), got.size)
 

@@ -63,7 +63,7 @@ def test_split_kernel_equals_oracle(aclnn, monkeypatch, case):
                               False, nk, group)
         torch.cuda.synchronize()
         outs.append(out_to_np(out))
-    assert aclnn.last_kernel_name() == ("qmm_umma_perblock" if mode == "block" else "qmm_umma_deq"), aclnn.last_kernel_name()
+    assert aclnn.last_kernel_name() == ("qmm_umma_split_perblock" if mode == "block" else "qmm_umma_split_deq"), aclnn.last_kernel_name()
     assert np.array_equal(outs[0].view(np.uint8), outs[1].view(np.uint8))
     if mode == "int8":
         assert np.array_equal(outs[0].view(np.uint8), np.asarray(want).view(np.uint8))

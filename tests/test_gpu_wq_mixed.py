@@ -43,12 +43,12 @@ IMAGE_CASES = [
 
 @pytest.mark.parametrize("case", IMAGE_CASES, ids=[str(c) for c in IMAGE_CASES])
 def test_dequantised_image_equals_oracle(aclnn, case):
-    _against_oracle(aclnn, case, ("qmm_umma_deq", "qmm_umma_pair_deq", "qmm_umma_split_deq"))
+    _against_oracle(aclnn, case, ("qmm_umma_deq", "qmm_umma_pair_deq"))
 
 
 @pytest.mark.parametrize("case", CASES, ids=[str(c) for c in CASES])
 def test_mixed_kernel_equals_oracle(aclnn, case):
-    _against_oracle(aclnn, case, ("wqbmm_decode" if case[0] == "int4" else "wqbmm_decode8",))
+    _against_oracle(aclnn, case, ("wqbmm_mixed",))
 
 
 def _against_oracle(aclnn, case, kernels):

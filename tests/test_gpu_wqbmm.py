@@ -34,6 +34,7 @@ def test_fixture(aclnn, name, kernel):
     check_close(got, a["out"], _ref64(a, meta), np_name(a["out"]), floor_rms=0.05)
 
 
+@pytest.mark.usefixtures("streaming")
 def test_decode_kernel_is_selected_and_matches_golden_tightly(aclnn):
     """The small-m int4 fixtures must run on the streaming decode kernel, and since it reproduces the reference's two
     roundings per weight its output may differ from the golden only by fp32 summation order: <= 1 ulp of the output
@@ -53,7 +54,8 @@ def test_decode_kernel_is_selected_and_matches_golden_tightly(aclnn):
         assert np.mean(g != w) < 0.05, name
 
 
-def test_decode_c2_shape_properties(aclnn):
+@pytest.mark.parametrize("kernel", ["wqbmm_mixed", "wqbmm_decode"])
+def test_decode_c2_shape_properties(aclnn, monkeypatch, kernel):
     """Full benchmark shape (m16 k8192 n28672 g128): checked through size-independent properties and a sampled oracle.
       * linearity in x: f(2x) == 2 f(x) bit for bit (powers of two commute with every rounding here);
       * zero rows of x give exactly-zero rows of y; rows are independent (row i of a 16-row call == the 1-row call);
@@ -62,6 +64,8 @@ def test_decode_c2_shape_properties(aclnn):
 
     from gpu_util import DEV, out_to_np
 
+    if kernel == "wqbmm_decode":
+        monkeypatch.setenv("OPSNN_WQ_NO_MIXED", "1")
     m, k, n, g = 16, 8192, 28672, 128
     gen = torch.Generator(device=DEV).manual_seed(1002)
     x = torch.randn((m, k), generator=gen, device=DEV, dtype=torch.float32).to(torch.bfloat16)
@@ -78,7 +82,7 @@ def test_decode_c2_shape_properties(aclnn):
         aclnn.weight_quant_batch_matmul(aclnn.from_torch(xx), aclnn.from_torch(words), aclnn.from_torch(scale),
                                         aclnn.from_torch(y), aclnn.from_torch(offset), None, g)
         torch.cuda.synchronize()
-        assert aclnn.last_kernel_name() == "wqbmm_decode"
+        assert aclnn.last_kernel_name() == kernel
         return y
 
     y1 = run(x)
@@ -137,6 +141,7 @@ PREFILL_CASES = [
 
 
 @pytest.mark.parametrize("case", PREFILL_CASES, ids=[str(c) for c in PREFILL_CASES])
+@pytest.mark.usefixtures("streaming")
 def test_prefill_dequant_then_tensor_core_matmul(aclnn, case):
     """m beyond the decode range: the weight is dequantised with the reference's two roundings into workspace and multiplied
     by the tcgen05 bf16/fp16 kernel, so the output differs from the golden only by fp32 summation order."""
@@ -168,6 +173,7 @@ def test_prefill_dequant_then_tensor_core_matmul(aclnn, case):
 
 
 @pytest.mark.parametrize("m,inner_precise,n", [(40, 0, 16384), (33, 1, 16384), (32, 0, 4096)])
+@pytest.mark.usefixtures("streaming")
 def test_decode_kernel_in_chunks_of_16_rows(aclnn, m, inner_precise, n):
     """16 < m <= 48 against a large weight: one launch of the streaming decode kernel per 16 rows of x (two launches from 2^24
     weights on, three from 3 x 2^24)."""
@@ -309,6 +315,7 @@ def test_cluster_combine_equals_workspace_combine(aclnn, monkeypatch, case):
     assert np.all(np.abs(got - want) <= tol * np.maximum(np.abs(want), 0.05 * rms) * 1.01)
 
 
+@pytest.mark.usefixtures("streaming")
 def test_narrow_output_is_planned_as_clusters(aclnn):
     """A 1/8 column shard of the benchmark's decode shape (what one of eight GPUs gets): the k-ranges of a strip run as one
     thread-block cluster of as many CTAs as the device keeps resident for all seven strips at once. The full width (56 strips
@@ -350,6 +357,7 @@ W4_NK_CASES = [
 
 
 @pytest.mark.parametrize("case", W4_NK_CASES, ids=[str(c) for c in W4_NK_CASES])
+@pytest.mark.usefixtures("streaming")
 def test_w4a16_weight_stored_nk_streaming_kernel(aclnn, case):
     """INT4 weights stored (n,k) - the transposed view of the API, k contiguous, scales stored (n, groups) - at m <= 16 run on the
     (n,k) form of the bulk-copy decode kernel with the golden's two roundings per weight (wqbmmv2_kernel_golden.py:242-297): only the
@@ -426,6 +434,7 @@ def _dev16(aclnn, a):
 
 
 @pytest.mark.parametrize("case", F8_CASES, ids=[str(c) for c in F8_CASES])
+@pytest.mark.usefixtures("streaming")
 def test_a16f8_small_m_streaming_kernel(aclnn, case):
     """FLOAT8_E4M3FN weights at m <= 16 run on the 8-bit streaming kernel. Every byte code occurs (subnormals, both zeros, +-448);
     the dequantised weight rn(w * scale) is the golden's (wqbmmv2_kernel_golden.py:199-297), so only the fp32 summation order
@@ -474,8 +483,9 @@ def test_a16f8_small_m_streaming_kernel(aclnn, case):
 
 @pytest.mark.parametrize("trans", [False, True], ids=["(k,n)", "(n,k)"])
 @pytest.mark.parametrize("xdt", ["bfloat16", "float16"])
-def test_a16f8_dequantisation_is_bit_exact(aclnn, xdt, trans):
-    """With one-hot rows of x the product is the dequantised weight row itself (every other term is a zero), so the streaming kernel's
+@pytest.mark.parametrize("kernel", ["wqbmm_mixed", "wqbmm_decode8"])
+def test_a16f8_dequantisation_is_bit_exact(aclnn, monkeypatch, xdt, trans, kernel):
+    """With one-hot rows of x the product is the dequantised weight row itself (every other term is a zero), so the kernel's
     e4m3 -> 16-bit conversion and its single rounding of w * scale are compared bit for bit with the oracle, for every finite byte
     code in every selected row (subnormals and both zeros included) and for scales that push products into the 16-bit type's
     subnormal range."""
@@ -484,6 +494,8 @@ def test_a16f8_dequantisation_is_bit_exact(aclnn, xdt, trans):
 
     from gpu_util import DEV, out_to_np
 
+    if kernel == "wqbmm_decode8":
+        monkeypatch.setenv("OPSNN_WQ_NO_MIXED", "1")
     m, k, n, group = 16, 2048, 1024, 128
     rng = np.random.default_rng(41 if xdt == "bfloat16" else 43)
     np_dt = ml_dtypes.bfloat16 if xdt == "bfloat16" else np.float16
@@ -502,7 +514,7 @@ def test_a16f8_dequantisation_is_bit_exact(aclnn, xdt, trans):
     aclnn.weight_quant_batch_matmul(_dev16(aclnn, x), _f8_tensor(aclnn, codes, trans), _dev16_t(aclnn, sc) if trans else _dev16(aclnn, sc),
                                     aclnn.from_torch(y), None, None, group)
     torch.cuda.synchronize()
-    assert aclnn.last_kernel_name() == "wqbmm_decode8", aclnn.last_kernel_name()
+    assert aclnn.last_kernel_name() == kernel, aclnn.last_kernel_name()
     want = wqbmm_oracle.weight_quant_batch_matmul(x, w, sc, None, None, group)
     got = out_to_np(y)
     assert np.array_equal(got.astype(np.float32), want.astype(np.float32))
@@ -518,6 +530,7 @@ CHUNK8_CASES = [
 
 
 @pytest.mark.parametrize("case", CHUNK8_CASES, ids=[str(c) for c in CHUNK8_CASES])
+@pytest.mark.usefixtures("streaming")
 def test_8bit_and_nk_decode_kernels_in_chunks_of_16_rows(aclnn, case):
     """16 < m <= 48 against a large weight: the 8-bit streaming kernels and the (n,k) int4 kernel run once per 16 rows of x, like the
     (k,n) int4 kernel; same <= 1 ulp criterion as a single launch."""
@@ -576,6 +589,7 @@ W8_CASES = [
 
 
 @pytest.mark.parametrize("case", W8_CASES, ids=[str(c) for c in W8_CASES])
+@pytest.mark.usefixtures("streaming")
 def test_w8a16_small_m_streaming_kernel(aclnn, case):
     """INT8 weights at m <= 16 run on their own streaming kernel (the reference's n-first regime,
     weight_quant_batch_matmul_v2/op_kernel/arch35/n_first/*); it reproduces the golden's two roundings per weight, so only the
