@@ -100,19 +100,12 @@ static bool streaming_asked_for()
 // It does not take: innerPrecise = 1 (the group-wise arithmetic of the streaming kernels), outputs bound to a communicator (only the
 // streaming kernels store into the peers), a weight prepared for the matmul, and m > 1152, where dequantising the weight once per 128
 // rows costs more than a pass over HBM (against pre-pass and matmul, us: m 1100 8192 x 28672 int4 514 / 578, 4096^2 40 / 53; m 1280 610 / 597,
-// 52 / 54, int8 4096 x 14336 169 / 160). aclnnWeightQuantBatchMatmulV2 keeps the kernels that its tests name: the streaming one for
-// symmetric (k,n) int4 at m <= 16 (and its reported plan), dequantise-then-matmul up to 2^22 weights.
-int32_t wqbmm_faster_kernel(const OpsnnWqbmmParams* p, int32_t choice, bool v2)
+// 52 / 54, int8 4096 x 14336 169 / 160).
+int32_t wqbmm_faster_kernel(const OpsnnWqbmmParams* p, int32_t choice)
 {
     if (choice != OPSNN_WQ_KERNEL_DECODE && choice != OPSNN_WQ_KERNEL_PREFILL && choice != OPSNN_WQ_KERNEL_GENERIC) return choice;
     if (choice == OPSNN_WQ_KERNEL_PREFILL && p->prep_w != nullptr) return choice;
-    const int64_t weights = p->k * p->n;
-    if (p->m > 1152 || weights < ((int64_t)1 << 18)) return choice;
-    if (v2) {
-        if (choice == OPSNN_WQ_KERNEL_GENERIC) return choice;
-        if (p->m > 16 && weights <= ((int64_t)1 << 22)) return choice;
-        if (p->m <= 16 && p->w_dtype == ACL_INT4 && p->trans_w == 0 && p->offset == nullptr) return choice;
-    }
+    if (p->m > 1152 || p->k * p->n < ((int64_t)1 << 18)) return choice;
     if (!wqbmm_mixed_eligible(p) || streaming_asked_for()) return choice;
     PeerBinding pb;
     if (p->y != nullptr && lookup_peer_binding(p->y, &pb)) return choice;
@@ -272,7 +265,7 @@ int32_t opsnn_wqbmm_select_kernel(const OpsnnWqbmmParams* p)
 uint64_t opsnn_wqbmm_workspace_size(const OpsnnWqbmmParams* p, int32_t kernel_choice)
 {
     if (p == nullptr) return 0;
-    if (kernel_choice == OPSNN_WQ_KERNEL_AUTO) kernel_choice = wqbmm_faster_kernel(p, opsnn_wqbmm_select_kernel(p), false);
+    if (kernel_choice == OPSNN_WQ_KERNEL_AUTO) kernel_choice = wqbmm_faster_kernel(p, opsnn_wqbmm_select_kernel(p));
     OpsnnWqbmmParams nd;
     if (p->nz_k0 != 0) {
         const uint64_t pre = wq_nz_bytes(p);
@@ -328,7 +321,7 @@ int32_t opsnn_wqbmm_launch(const OpsnnWqbmmParams* p, int32_t kernel_choice, voi
         wq_nz_view(p, &nd, p->workspace);
         return opsnn_wqbmm_launch(&nd, kernel_choice, stream);
     }
-    if (kernel_choice == OPSNN_WQ_KERNEL_AUTO) kernel_choice = wqbmm_faster_kernel(p, opsnn_wqbmm_select_kernel(p), false);
+    if (kernel_choice == OPSNN_WQ_KERNEL_AUTO) kernel_choice = wqbmm_faster_kernel(p, opsnn_wqbmm_select_kernel(p));
     {
         // An output bound to a communicator (opsnn_comm_bind_columns) is written into every rank's full copy by the bulk-copy
         // decode kernels only; a call that would run elsewhere must not silently skip that.

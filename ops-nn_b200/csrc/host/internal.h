@@ -113,7 +113,6 @@ struct aclOpExecutor {
     uint64_t workspace_size = 0;
     OpsnnQmmParams qmm{};
     OpsnnWqbmmParams wq{};
-    bool wq_v2 = false;  // planned by aclnnWeightQuantBatchMatmulV2
     OpsnnMxQuantParams mxq{};
     OpsnnPackB4Params pack{};
     // aclnnQuantMatmulWeightNz: x2 arrives FRACTAL_NZ and is rewritten row-major into the head of the workspace before the matmul
@@ -130,7 +129,7 @@ namespace opsnn {
 
 // The kernel a weight-only call runs on, given what opsnn_wqbmm_select_kernel answered for it: OPSNN_WQ_KERNEL_MIXED where that is the
 // faster form, else `choice`.
-int32_t wqbmm_faster_kernel(const OpsnnWqbmmParams* p, int32_t choice, bool v2);
+int32_t wqbmm_faster_kernel(const OpsnnWqbmmParams* p, int32_t choice);
 
 // Records the text returned by aclGetRecentErrMsg() for the calling thread and, when OPSNN_LOG_LEVEL >= 1,
 // prints it to stderr.

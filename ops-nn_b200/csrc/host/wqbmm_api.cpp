@@ -54,8 +54,6 @@ void attach_prepared_w(OpsnnWqbmmParams* p)
         return ACLNN_ERR_PARAM_INVALID; \
     } while (0)
 
-constexpr int kInnerPreciseV2 = -1;  // aclnnWeightQuantBatchMatmulV2 has no innerPrecise: high precision, and its own kernel rules
-
 aclnnStatus wq_common(const char* api, const aclTensor* x, const aclTensor* weight, const aclTensor* antiquantScale,
                       const aclTensor* antiquantOffset, const aclTensor* quantScale, const aclTensor* quantOffset,
                       const aclTensor* bias, int antiquantGroupSize, int innerPrecise, const aclTensor* y,
@@ -224,8 +222,7 @@ aclnnStatus wq_common(const char* api, const aclTensor* x, const aclTensor* weig
 
     // innerPrecise = 1 asks for the high-performance mode; it only changes anything where the reference says it does
     // (A16W4 per-group, small m: docs/aclnnWeightQuantBatchMatmulV3.md:389), i.e. where the fast decode kernel applies
-    p.inner_precise = innerPrecise < 0 ? 0 : innerPrecise;
-    exec->wq_v2 = innerPrecise < 0;
+    p.inner_precise = innerPrecise;
     p.nz_k0 = nz_k0;
     p.nz_n0 = nz_n0;
     if (nz_k0 != 0 && trans_w) no_kernel("a FRACTAL_NZ weight must be the plain (k,n) view");
@@ -241,7 +238,7 @@ aclnnStatus wq_common(const char* api, const aclTensor* x, const aclTensor* weig
             probe.w = probe.x = probe.scale = dummy;
             if (probe.offset == nullptr && antiquantOffset) probe.offset = dummy;
         }
-        int choice = exec->kernel_choice == OPSNN_WQ_KERNEL_AUTO ? wqbmm_faster_kernel(&probe, opsnn_wqbmm_select_kernel(&probe), exec->wq_v2) : exec->kernel_choice;
+        int choice = exec->kernel_choice == OPSNN_WQ_KERNEL_AUTO ? wqbmm_faster_kernel(&probe, opsnn_wqbmm_select_kernel(&probe)) : exec->kernel_choice;
         exec->workspace_size = opsnn_wqbmm_workspace_size(&probe, choice);
     }
     *workspaceSize = exec->workspace_size;
@@ -283,7 +280,7 @@ aclnnStatus wq_run(const char* api, void* workspace, uint64_t workspaceSize, acl
     p.workspace_size = workspaceSize;
     int choice = exec->kernel_choice;
     if (choice == OPSNN_WQ_KERNEL_AUTO) {
-        choice = wqbmm_faster_kernel(&p, opsnn_wqbmm_select_kernel(&p), exec->wq_v2);
+        choice = wqbmm_faster_kernel(&p, opsnn_wqbmm_select_kernel(&p));
         // the plan sized the workspace for the decode kernel only if the shapes allowed it
         if (choice != OPSNN_WQ_KERNEL_GENERIC && workspaceSize < opsnn_wqbmm_workspace_size(&p, choice))
             choice = OPSNN_WQ_KERNEL_GENERIC;
@@ -311,7 +308,7 @@ aclnnStatus aclnnWeightQuantBatchMatmulV2GetWorkspaceSize(const aclTensor* x, co
 {
     OPSNN_DFX_RANGE("aclnnWeightQuantBatchMatmulV2GetWorkspaceSize");
     return wq_common("aclnnWeightQuantBatchMatmulV2GetWorkspaceSize", x, weight, antiquantScale, antiquantOffsetOptional,
-                     quantScaleOptional, quantOffsetOptional, biasOptional, antiquantGroupSize, kInnerPreciseV2, y, workspaceSize, executor);
+                     quantScaleOptional, quantOffsetOptional, biasOptional, antiquantGroupSize, 0, y, workspaceSize, executor);
 }
 
 aclnnStatus aclnnWeightQuantBatchMatmulV2(void* workspace, uint64_t workspaceSize, aclOpExecutor* executor,

@@ -87,6 +87,7 @@ WQ_CASES = [
 ]
 
 
+@pytest.mark.usefixtures("streaming")
 @pytest.mark.parametrize("case", WQ_CASES, ids=[str(c) for c in WQ_CASES])
 def test_prepared_prefill_weight_equals_unprepared(aclnn, case):
     """aclnnWeightQuantBatchMatmulV2 beyond the decode range dequantises the whole weight per call; with the weight registered

@@ -184,3 +184,28 @@ def test_sums_are_as_exact_as_the_streaming_kernels(aclnn, monkeypatch, case):
         lost += int((y[:, cols] != want).sum())
         lost_stream += int((y_stream[:, cols] != want).sum())
     assert lost <= lost_stream + 4 * (2 * lost_stream) ** 0.5, (lost, lost_stream, m * n)
+
+
+@pytest.mark.parametrize("case", [("int4", False, 16, 1024, 1024, False), ("int4", False, 40, 1024, 2048, True), ("int8", True, 1, 512, 1024, False)])
+def test_both_entry_points_run_the_same_kernel(aclnn, case):
+    """aclnnWeightQuantBatchMatmulV2 and V3 (high precision) are one operator: same kernel, same bits."""
+    import torch
+
+    from gpu_util import DEV
+
+    kind, nk, m, k, n, has_off = case
+    gen = torch.Generator(device=DEV).manual_seed(case_seed(case))
+    x = torch.randn((m, k), generator=gen, device=DEV).to(torch.bfloat16)
+    if kind == "int4":
+        w = torch.randint(-2 ** 31, 2 ** 31, (k, n // 8), generator=gen, device=DEV, dtype=torch.int32)
+    else:
+        w = torch.randint(-127, 128, (n, k), generator=gen, device=DEV, dtype=torch.int8).t()
+    sc = (torch.rand(n, generator=gen, device=DEV) * 0.01 + 0.005).to(torch.bfloat16)
+    of = torch.rand(n, generator=gen, device=DEV).to(torch.bfloat16) if has_off else None
+    outs = []
+    for inner_precise in (None, 0):
+        y = torch.empty((m, n), dtype=torch.bfloat16, device=DEV)
+        aclnn.weight_quant_batch_matmul(*(aclnn.from_torch(t) for t in (x, w, sc, y, of)), None, 0, inner_precise=inner_precise)
+        outs.append(y)
+        assert aclnn.last_kernel_name() == "wqbmm_mixed"
+    assert torch.equal(outs[0], outs[1])
