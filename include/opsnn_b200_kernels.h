@@ -167,6 +167,7 @@ OPSNN_API uint64_t opsnn_wqbmm_workspace_size(const OpsnnWqbmmParams* p, int32_t
  * and p->m are not read. Afterwards set p->prep_w = storage in calls on the same weight, scale, offset and x dtype. */
 OPSNN_API uint64_t opsnn_wqbmm_prepare_size(const OpsnnWqbmmParams* p);
 OPSNN_API int32_t opsnn_wqbmm_prepare_launch(const OpsnnWqbmmParams* p, void* storage, uint64_t storage_size, void* stream);
+/* The kernel that OPSNN_WQ_KERNEL_AUTO stands for. */
 OPSNN_API int32_t opsnn_wqbmm_select_kernel(const OpsnnWqbmmParams* p);
 OPSNN_API int32_t opsnn_wqbmm_launch(const OpsnnWqbmmParams* p, int32_t kernel_choice, void* stream);
 
@@ -177,9 +178,11 @@ OPSNN_API int32_t opsnn_wqbmm_launch(const OpsnnWqbmmParams* p, int32_t kernel_c
  *
  *   - The cross-CTA scratch is a 9,964,032-byte array inside the library's device image; p->workspace and
  *     p->workspace_size are ignored. Neither this function nor anything it calls allocates host-visible device memory.
- *   - Limits: the parameters must satisfy the decode kernel's range (opsnn_wqbmm_select_kernel(p) ==
- *     OPSNN_WQ_KERNEL_DECODE with inner_precise = 0; inner_precise is ignored here) and n <= 155,648 columns (304 CTAs x 512). Anything else returns cudaErrorInvalidValue
- *     and leaves the reason in aclGetRecentErrMsg().
+ *   - Limits: the decode kernel's range, which is an INT4 weight stored (k,n), m <= 16, k % 16 == 0, n, w_ld and x_ld % 8 == 0, groups of a
+ *     multiple of 16 (or none), scales contiguous along n (or one), 16-byte aligned x, scale and offset rows; inner_precise is ignored
+ *     here. And n <= 155,648 columns (304 CTAs x 512). Anything else returns cudaErrorInvalidValue and leaves the reason in
+ *     aclGetRecentErrMsg(). (opsnn_wqbmm_select_kernel answers OPSNN_WQ_KERNEL_MIXED for most of this range: what a call with
+ *     OPSNN_WQ_KERNEL_AUTO runs on.)
  *   - The first call on each device (with that device current) resolves the array's address; this may load the
  *     library's device code. Make that first call during start-up, before any stream capture begins.
  *   - The array is shared by every call on the device and keeps its last contents. Nothing in it has to start at

@@ -98,10 +98,10 @@ static bool streaming_asked_for()
 //   m 1   4096 x 4096 12.1 -> 8.6      m 16  8192 x 28672 49.3 -> 39.1     m 16 int8 4096 x 14336 20.2 -> 15.2
 //   m 32  8192 x 28672 98 -> 43        m 128 8192 x 28672 285 -> 67        m 512 8192 x 28672 416 -> 237
 // It does not take: innerPrecise = 1 (the group-wise arithmetic of the streaming kernels), outputs bound to a communicator (only the
-// streaming kernels store into the peers), a weight prepared for the matmul, and m > 1152, where dequantising the weight once per 128
-// rows costs more than a pass over HBM (against pre-pass and matmul, us: m 1100 8192 x 28672 int4 514 / 578, 4096^2 40 / 53; m 1280 610 / 597,
-// 52 / 54, int8 4096 x 14336 169 / 160).
-int32_t wqbmm_faster_kernel(const OpsnnWqbmmParams* p, int32_t choice)
+// streaming kernels store into the peers), a weight prepared for the matmul, a FRACTAL_NZ weight, and m > 1152, where dequantising the weight
+// once per 128 rows costs more than a pass over HBM (against pre-pass and matmul, us: m 1100 8192 x 28672 int4 514 / 578, 4096^2 40 / 53;
+// m 1280 610 / 597, 52 / 54, int8 4096 x 14336 169 / 160).
+static int32_t faster_kernel(const OpsnnWqbmmParams* p, int32_t choice)
 {
     if (choice != OPSNN_WQ_KERNEL_DECODE && choice != OPSNN_WQ_KERNEL_PREFILL && choice != OPSNN_WQ_KERNEL_GENERIC) return choice;
     if (choice == OPSNN_WQ_KERNEL_PREFILL && p->prep_w != nullptr) return choice;
@@ -235,14 +235,9 @@ static int32_t decode_chunk_launches(const OpsnnWqbmmParams* p, cudaStream_t str
     return 0;
 }
 
-int32_t opsnn_wqbmm_select_kernel(const OpsnnWqbmmParams* p)
+// The kernel of a call if there were no fused one.
+static int32_t unfused_kernel(const OpsnnWqbmmParams* p)
 {
-    if (p == nullptr) return OPSNN_WQ_KERNEL_GENERIC;
-    OpsnnWqbmmParams nd;
-    if (p->nz_k0 != 0) {  // FRACTAL_NZ weight: selection is that of the row-major copy (stand-in address with allocation alignment)
-        wq_nz_view(p, &nd, reinterpret_cast<void*>(uintptr_t(256)));
-        p = &nd;
-    }
     if (p->inner_precise == 1 && wqbmm_decode_fast_eligible(p)) return OPSNN_WQ_KERNEL_DECODE_FAST;
     if (wqbmm_decode_eligible(p)) return OPSNN_WQ_KERNEL_DECODE;
     // 8-bit weights (int8, e4m3) at small m: their own streaming kernel once the weight is large enough to be worth a k-split grid
@@ -262,10 +257,21 @@ int32_t opsnn_wqbmm_select_kernel(const OpsnnWqbmmParams* p)
     return OPSNN_WQ_KERNEL_GENERIC;
 }
 
+int32_t opsnn_wqbmm_select_kernel(const OpsnnWqbmmParams* p)
+{
+    if (p == nullptr) return OPSNN_WQ_KERNEL_GENERIC;
+    OpsnnWqbmmParams nd;
+    if (p->nz_k0 != 0) {  // FRACTAL_NZ weight: selection is that of the row-major copy (stand-in address with allocation alignment)
+        wq_nz_view(p, &nd, reinterpret_cast<void*>(uintptr_t(256)));
+        return unfused_kernel(&nd);
+    }
+    return faster_kernel(p, unfused_kernel(p));
+}
+
 uint64_t opsnn_wqbmm_workspace_size(const OpsnnWqbmmParams* p, int32_t kernel_choice)
 {
     if (p == nullptr) return 0;
-    if (kernel_choice == OPSNN_WQ_KERNEL_AUTO) kernel_choice = wqbmm_faster_kernel(p, opsnn_wqbmm_select_kernel(p));
+    if (kernel_choice == OPSNN_WQ_KERNEL_AUTO) kernel_choice = opsnn_wqbmm_select_kernel(p);
     OpsnnWqbmmParams nd;
     if (p->nz_k0 != 0) {
         const uint64_t pre = wq_nz_bytes(p);
@@ -313,6 +319,7 @@ int32_t opsnn_wqbmm_launch(const OpsnnWqbmmParams* p, int32_t kernel_choice, voi
 {
     if (p == nullptr) return (int32_t)cudaErrorInvalidValue;
     if (p->m <= 0 || p->n <= 0) return 0;
+    if (kernel_choice == OPSNN_WQ_KERNEL_AUTO) kernel_choice = opsnn_wqbmm_select_kernel(p);  // (as the workspace was sized: before the rewriting)
     OpsnnWqbmmParams nd;
     if (p->nz_k0 != 0) {
         if (p->workspace == nullptr || p->workspace_size < wq_nz_bytes(p)) return (int32_t)cudaErrorInvalidValue;
@@ -321,7 +328,6 @@ int32_t opsnn_wqbmm_launch(const OpsnnWqbmmParams* p, int32_t kernel_choice, voi
         wq_nz_view(p, &nd, p->workspace);
         return opsnn_wqbmm_launch(&nd, kernel_choice, stream);
     }
-    if (kernel_choice == OPSNN_WQ_KERNEL_AUTO) kernel_choice = wqbmm_faster_kernel(p, opsnn_wqbmm_select_kernel(p));
     {
         // An output bound to a communicator (opsnn_comm_bind_columns) is written into every rank's full copy by the bulk-copy
         // decode kernels only; a call that would run elsewhere must not silently skip that.

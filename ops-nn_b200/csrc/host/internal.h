@@ -127,10 +127,6 @@ struct aclOpExecutor {
 
 namespace opsnn {
 
-// The kernel a weight-only call runs on, given what opsnn_wqbmm_select_kernel answered for it: OPSNN_WQ_KERNEL_MIXED where that is the
-// faster form, else `choice`.
-int32_t wqbmm_faster_kernel(const OpsnnWqbmmParams* p, int32_t choice);
-
 // Records the text returned by aclGetRecentErrMsg() for the calling thread and, when OPSNN_LOG_LEVEL >= 1,
 // prints it to stderr.
 void set_err(const char* fmt, ...) __attribute__((format(printf, 1, 2)));

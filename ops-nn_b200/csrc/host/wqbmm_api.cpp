@@ -238,7 +238,7 @@ aclnnStatus wq_common(const char* api, const aclTensor* x, const aclTensor* weig
             probe.w = probe.x = probe.scale = dummy;
             if (probe.offset == nullptr && antiquantOffset) probe.offset = dummy;
         }
-        int choice = exec->kernel_choice == OPSNN_WQ_KERNEL_AUTO ? wqbmm_faster_kernel(&probe, opsnn_wqbmm_select_kernel(&probe)) : exec->kernel_choice;
+        int choice = exec->kernel_choice == OPSNN_WQ_KERNEL_AUTO ? opsnn_wqbmm_select_kernel(&probe) : exec->kernel_choice;
         exec->workspace_size = opsnn_wqbmm_workspace_size(&probe, choice);
     }
     *workspaceSize = exec->workspace_size;
@@ -280,7 +280,7 @@ aclnnStatus wq_run(const char* api, void* workspace, uint64_t workspaceSize, acl
     p.workspace_size = workspaceSize;
     int choice = exec->kernel_choice;
     if (choice == OPSNN_WQ_KERNEL_AUTO) {
-        choice = wqbmm_faster_kernel(&p, opsnn_wqbmm_select_kernel(&p));
+        choice = opsnn_wqbmm_select_kernel(&p);
         // the plan sized the workspace for the decode kernel only if the shapes allowed it
         if (choice != OPSNN_WQ_KERNEL_GENERIC && workspaceSize < opsnn_wqbmm_workspace_size(&p, choice))
             choice = OPSNN_WQ_KERNEL_GENERIC;

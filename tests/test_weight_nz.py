@@ -121,3 +121,39 @@ def test_quant_matmul_weight_nz_gives_the_nd_result(aclnn, case):
         outs.append(out_to_np(out).view(np.uint16))
     assert np.array_equal(outs[0], want.view(np.uint16))
     assert np.array_equal(outs[1], outs[0])
+
+
+@pytest.mark.gpu
+def test_weight_only_launch_chooses_the_kernel_that_its_workspace_was_sized_for(aclnn):
+    """The kernel-level interface with the automatic choice on a FRACTAL_NZ weight with more column tiles than SMs: sizing and launch once
+    answered for different layouts, and the launch refused the workspace that had been asked for."""
+    import ctypes
+
+    import torch
+
+    from gpu_util import DEV
+
+    m, k, n, g = 128, 320, 38144, 64
+    gen = torch.Generator(device=DEV).manual_seed(3)
+    w = torch.randint(-8, 8, (k, n), generator=gen, device=DEV, dtype=torch.int32)
+    nz = wqbmm_oracle.nd_to_nz(w.cpu().numpy().astype(np.int8), 16, 64)
+    nib = nz.astype(np.uint8) & 0xF
+    store = torch.from_numpy((nib[..., 0::2] | (nib[..., 1::2] << 4)).copy()).to(DEV)
+    x = torch.randn((m, k), generator=gen, device=DEV).to(torch.bfloat16)
+    sc = (torch.rand((k // g, n), generator=gen, device=DEV) * 0.01 + 0.005).to(torch.bfloat16)
+    y = torch.empty((m, n), dtype=torch.bfloat16, device=DEV)
+    p = aclnn.WqbmmParams()
+    p.x_dtype, p.w_dtype, p.bias_dtype, p.trans_w = aclnn.ACL_BF16, aclnn.ACL_INT4, -1, 0
+    p.m, p.n, p.k, p.nz_k0, p.nz_n0 = m, n, k, 16, 64
+    p.x, p.x_ld, p.w, p.w_ld, p.scale, p.offset, p.bias = x.data_ptr(), k, store.data_ptr(), n, sc.data_ptr(), None, None
+    p.group_size, p.scale_sg, p.scale_sn = g, n, 1
+    p.y, p.y_ld = y.data_ptr(), n
+    L = aclnn.lib()
+    ws = torch.empty(L.opsnn_wqbmm_workspace_size(ctypes.byref(p), 0), dtype=torch.uint8, device=DEV)
+    p.workspace, p.workspace_size = ws.data_ptr(), ws.numel()
+    assert L.opsnn_wqbmm_launch(ctypes.byref(p), 0, None) == 0, aclnn.last_error()
+    torch.cuda.synchronize()
+    wd = (w.float() * sc.float().repeat_interleave(g, 0)).to(torch.bfloat16)
+    want = x.double() @ wd.double()
+    rms = want.square().mean().sqrt()
+    assert bool(((y.double() - want).abs() <= 2.0 ** -7 * torch.maximum(want.abs(), 0.05 * rms) * 1.01).all())

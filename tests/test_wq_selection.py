@@ -4,7 +4,13 @@ import ctypes
 
 import pytest
 
-GENERIC, DECODE, DECODE_FAST, PREFILL = 1, 2, 3, 4
+GENERIC, DECODE, DECODE_FAST, PREFILL, MIXED = 1, 2, 3, 4, 5
+
+
+@pytest.fixture(autouse=True)
+def _without_the_fused_kernel(monkeypatch):
+    """The rules below are those among the kernels that the fused one leaves; its own tests take the switch back."""
+    monkeypatch.setenv("OPSNN_WQ_NO_MIXED", "1")
 
 
 def _probe(aclnn, m, k, n, g=128, w_dtype=None, trans=False, inner_precise=0, scale_dtype=None, offset=True):
@@ -70,3 +76,24 @@ def test_eight_bit_weights_take_the_streaming_kernel_from_2_20_weights_on(aclnn)
 def test_e8m0_scales_never_reach_the_decode_kernels(aclnn):
     assert _sel(aclnn, 16, 4096, 4096, g=32, scale_dtype=aclnn.ACL_FLOAT8_E8M0) not in (DECODE, DECODE_FAST)
     assert _sel(aclnn, 16, 4096, 4096, g=0, w_dtype=aclnn.ACL_INT8, scale_dtype=aclnn.ACL_FLOAT8_E8M0) not in (DECODE, DECODE_FAST)
+
+
+def test_the_fused_kernel_is_the_answer_where_it_is_what_runs(aclnn, monkeypatch):
+    """The answer is what a call with the automatic choice runs on, and its workspace is sized for that."""
+    monkeypatch.delenv("OPSNN_WQ_NO_MIXED")
+    for m in (1, 16, 17, 48, 300, 1152):
+        for wd, off in ((aclnn.ACL_INT4, True), (aclnn.ACL_INT4, False), (aclnn.ACL_INT8, True), (aclnn.ACL_FLOAT8_E4M3FN, False)):
+            for trans in (False, True):
+                assert _sel(aclnn, m, 4096, 4096, w_dtype=wd, trans=trans, offset=off) == MIXED
+    assert _sel(aclnn, 1153, 4096, 4096) == PREFILL
+    assert _sel(aclnn, 16, 512, 256) != MIXED                             # 2^17 weights
+    assert _sel(aclnn, 16, 4096, 4096, g=32) == DECODE                    # groups of half a 64-row unit
+    assert _sel(aclnn, 16, 4096, 4096, inner_precise=1) == DECODE_FAST
+    p = _probe(aclnn, 16, 4096, 4096)
+    p.nz_k0, p.nz_n0 = 16, 64                                             # FRACTAL_NZ
+    assert aclnn.lib().opsnn_wqbmm_select_kernel(ctypes.byref(p)) == DECODE
+    size = aclnn.lib().opsnn_wqbmm_workspace_size
+    for nz in (0, 16):
+        q = _probe(aclnn, 128, 320, 38144, g=64)
+        q.nz_k0, q.nz_n0 = nz, 4 * nz
+        assert size(ctypes.byref(q), 0) == size(ctypes.byref(q), aclnn.lib().opsnn_wqbmm_select_kernel(ctypes.byref(q)))
