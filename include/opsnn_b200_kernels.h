@@ -156,8 +156,9 @@ typedef struct OpsnnWqbmmParams {
     int32_t nz_k0, nz_n0;
     int32_t scale_dtype;    /* 0 or x_dtype: scale in x's dtype; ACL_FLOAT8_E8M0: mx antiquant (group_size 32, no offset) */
     /* Optional: the weight as the prefill path would dequantise it (opsnn_wqbmm_prepare_launch wrote it, once, into caller
-       memory). With it set, calls on the prefill path (m > 16) skip the dequantisation pre-pass and need no workspace; results
-       are identical. Ignored by the decode kernels, which stream the packed weight. */
+       memory). With it set, calls on the prefill path skip the dequantisation pre-pass and need no workspace; results are
+       identical. Ignored by the decode and the fused kernels, which read the packed weight; OPSNN_WQ_KERNEL_AUTO takes the image instead
+       of the fused kernel from m = 129 on, and below 2^24 weights. */
     const void* prep_w;
 } OpsnnWqbmmParams;
 

@@ -40,9 +40,11 @@ ACLNN_API aclnnStatus opsnnQuantMatmulReleaseX2(const aclTensor* x2);
  * The same for aclnnWeightQuantBatchMatmulV2 / V3 beyond the decode range (m > 16). There a call first dequantises the whole
  * weight into 16-bit workspace (k x n x 2 bytes: 470 MB for the benchmark's decode weight) and then runs the tensor-core
  * matmul; the first step does not depend on the activations. opsnnWeightQuantPrepare runs it once into caller memory and
- * registers the image under the weight's device address; later calls with the same weight, antiquantScale, antiquantOffset,
- * antiquantGroupSize and x dtype and m > 16 skip the pre-pass and ask for no workspace (bit-identical results). Calls with
- * m <= 16 keep streaming the packed weight. The price is memory: the image is four (int4) or two (int8 / fp8) times the packed
+ * registers the image under the weight's device address. Later calls with the same weight, antiquantScale, antiquantOffset,
+ * antiquantGroupSize and x dtype skip the pre-pass and ask for no workspace if they have more than 128 rows of x (more than 16 for a
+ * weight of fewer than 2^24 elements). Results are bit-identical where the unprepared call runs the pre-pass; up to m = 1152 it mostly
+ * runs the fused kernel instead: the same dequantised weights, fp32 sums in another order. Calls with fewer rows read the packed weight
+ * as they do without the image, which is faster. The price is memory: the image is four (int4) or two (int8 / fp8) times the packed
  * weight, which is why this is the caller's choice. Weights with no prefill path report size 0 and register nothing.
  *
  *   xDtype   ACL_BF16 or ACL_FLOAT16: the dtype of the activations of the calls to come (the reference rounds the dequantised

@@ -98,13 +98,16 @@ static bool streaming_asked_for()
 //   m 1   4096 x 4096 12.1 -> 8.6      m 16  8192 x 28672 49.3 -> 39.1     m 16 int8 4096 x 14336 20.2 -> 15.2
 //   m 32  8192 x 28672 98 -> 43        m 128 8192 x 28672 285 -> 67        m 512 8192 x 28672 416 -> 237
 // It does not take: innerPrecise = 1 (the group-wise arithmetic of the streaming kernels), outputs bound to a communicator (only the
-// streaming kernels store into the peers), a weight prepared for the matmul, a FRACTAL_NZ weight, and m > 1152, where dequantising the weight
+// streaming kernels store into the peers), a FRACTAL_NZ weight, and m > 1152, where dequantising the weight
 // once per 128 rows costs more than a pass over HBM (against pre-pass and matmul, us: m 1100 8192 x 28672 int4 514 / 578, 4096^2 40 / 53;
 // m 1280 610 / 597, 52 / 54, int8 4096 x 14336 169 / 160).
+// A weight prepared for the matmul has no pre-pass to save: up to 128 rows the packed weight is still the smaller stream from 2^24 weights
+// on (us, fused / prepared image: m 32 8192 x 28672 int4 42 / 83, 4096 x 14336 17 / 31; m 128 57 / 88, 21 / 32, int8 70 / 92, 4096^2 14.7 / 16.2;
+// m 256 123 / 110, 31.1 / 30.6; m 1024 463 / 340; 1024 x 4096 at m 64 10 / 6.8).
 static int32_t faster_kernel(const OpsnnWqbmmParams* p, int32_t choice)
 {
     if (choice != OPSNN_WQ_KERNEL_DECODE && choice != OPSNN_WQ_KERNEL_PREFILL && choice != OPSNN_WQ_KERNEL_GENERIC) return choice;
-    if (choice == OPSNN_WQ_KERNEL_PREFILL && p->prep_w != nullptr) return choice;
+    if (choice == OPSNN_WQ_KERNEL_PREFILL && p->prep_w != nullptr && (p->m > 128 || p->k * p->n < ((int64_t)1 << 24))) return choice;
     if (p->m > 1152 || p->k * p->n < ((int64_t)1 << 18)) return choice;
     if (!wqbmm_mixed_eligible(p) || streaming_asked_for()) return choice;
     PeerBinding pb;

@@ -145,3 +145,35 @@ def test_prepared_prefill_weight_equals_unprepared(aclnn, case):
     rms = np.sqrt(np.mean(want ** 2))
     tol = 2.0 ** -7 if xdt == "bfloat16" else 2.0 ** -9
     assert np.all(np.abs(got - want) <= tol * np.maximum(np.abs(want), 0.05 * rms) * 1.01)
+
+
+def test_prepared_weight_beside_the_fused_kernel(aclnn):
+    """Up to 128 rows a prepared weight of 2^24 elements runs as an unprepared one does, bit for bit; with more rows it runs on its image,
+    whose sums are in another order."""
+    import torch
+
+    from gpu_util import DEV
+
+    k, n, g = 4096, 4096, 128
+    gen = torch.Generator(device=DEV).manual_seed(17)
+    w = torch.randint(-2 ** 31, 2 ** 31, (k, n // 8), generator=gen, device=DEV, dtype=torch.int32)
+    sc = (torch.rand((k // g, n), generator=gen, device=DEV) * 0.01 + 0.005).to(torch.bfloat16)
+    xs = {m: torch.randn((m, k), generator=gen, device=DEV).to(torch.bfloat16) for m in (128, 300)}
+    d_w, d_s = aclnn.from_torch(w), aclnn.from_torch(sc)
+
+    def run(m):
+        y = torch.empty((m, n), dtype=torch.bfloat16, device=DEV)
+        aclnn.weight_quant_batch_matmul(aclnn.from_torch(xs[m]), d_w, d_s, aclnn.from_torch(y), None, None, g, inner_precise=0)
+        return y, aclnn.last_kernel_name()
+
+    plain = {m: run(m) for m in xs}
+    storage = aclnn.prepare_weight(d_w, d_s, None, g, "bfloat16")
+    assert storage is not None
+    try:
+        prepared = {m: run(m) for m in xs}
+    finally:
+        aclnn.release_weight(d_w)
+    assert plain[128][1] == prepared[128][1] == plain[300][1] == "wqbmm_mixed" and torch.equal(plain[128][0], prepared[128][0])
+    assert prepared[300][1].startswith("qmm_umma")
+    a, b = plain[300][0].double(), prepared[300][0].double()
+    assert bool(((a - b).abs() <= 2.0 ** -7 * torch.maximum(a.abs(), 0.05 * a.square().mean().sqrt()) * 1.01).all())

@@ -97,3 +97,15 @@ def test_the_fused_kernel_is_the_answer_where_it_is_what_runs(aclnn, monkeypatch
         q = _probe(aclnn, 128, 320, 38144, g=64)
         q.nz_k0, q.nz_n0 = nz, 4 * nz
         assert size(ctypes.byref(q), 0) == size(ctypes.byref(q), aclnn.lib().opsnn_wqbmm_select_kernel(ctypes.byref(q)))
+
+
+def test_a_prepared_weight_is_used_where_it_is_the_faster_way(aclnn, monkeypatch):
+    monkeypatch.delenv("OPSNN_WQ_NO_MIXED")
+
+    def sel(m, k, n):
+        p = _probe(aclnn, m, k, n)
+        p.prep_w = 24576
+        return aclnn.lib().opsnn_wqbmm_select_kernel(ctypes.byref(p))
+
+    assert [sel(m, 4096, 4096) for m in (16, 17, 128, 129, 1152)] == [MIXED, MIXED, MIXED, PREFILL, PREFILL]
+    assert [sel(m, 4096, 2048) for m in (16, 17, 128)] == [MIXED, PREFILL, PREFILL]
