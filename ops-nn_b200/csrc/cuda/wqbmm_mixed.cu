@@ -173,6 +173,28 @@ __device__ __forceinline__ int mix_col_of_lane(int l)
     return kW == MixW::kInt4 ? 4 * (l & 7) + (l >> 3) : 16 * (l >> 4) + 2 * (l & 7) + ((l >> 3) & 1);
 }
 
+// The rows past `live` of a unit of A (64 rows of k, two to a column) cleared, this warp's 32 lanes of it at `abase`. A stage's rows past k
+// are zero in x and in the packed weight, but their dequantised weight is (0 + offset) * scale, and zero times an infinity is NaN.
+__device__ __forceinline__ void mix_clear_past(uint32_t abase, uint32_t live)
+{
+    tmem_st_wait();
+#pragma unroll 1
+    for (uint32_t c = live / 32u * 16u; c < 32u; c += 16u) {
+        uint32_t v[16], lo[8], hi[8];
+        ptx::tmem_ld16(abase + c, v);
+        ptx::tmem_ld_wait();
+#pragma unroll
+        for (uint32_t i = 0; i < 16; ++i) {
+            const uint32_t row = 2u * (c + i);
+            const uint32_t kept = row + 1u < live ? v[i] : (row < live ? v[i] & 0xFFFFu : 0u);
+            if (i < 8) lo[i] = kept;
+            else hi[i - 8] = kept;
+        }
+        tmem_st_32x32b_x8(abase + c, lo);
+        tmem_st_32x32b_x8(abase + c + 8u, hi);
+    }
+}
+
 // A CTA's contiguous piece of the (tile, stage) line.
 __device__ __forceinline__ uint32_t mix_begin(const MixArgs& a, uint32_t c) { return c * a.units / a.grid; }
 __device__ __forceinline__ uint32_t mix_owner(const MixArgs& a, uint32_t unit)
@@ -370,7 +392,9 @@ __device__ __forceinline__ void mix_sum_and_store(const MixArgs& a, uint32_t sme
     }
 }
 
-template <MixW kW, bool kNK, bool kBf16, bool kOff, MixSum kSum>
+// kRagged: k is not a whole number of stages. (As a question asked in every stage it cost the calls with whole ones up to 3 %: 4 x 4096 x 14336
+// int8 18.1 -> 18.7 us.)
+template <MixW kW, bool kNK, bool kBf16, bool kOff, MixSum kSum, bool kRagged>
 __global__ void __launch_bounds__(kMixThreads, 1)
 wqbmm_mixed_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUtensorMap map_x, const __grid_constant__ MixArgs a)
 {
@@ -552,6 +576,8 @@ wqbmm_mixed_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
         if (s >= stages) { s -= stages; par ^= 1u; }
         bool ok = true;
         const bool two_rows = a.sc_rows == 2u;  // a stage's units have scale rows of their own
+        const uint32_t k_in_last = a.k - (a.kb - 1u) * (uint32_t)C::kBK;  // rows of k in a tile's last stage
+        uint32_t ragged = (u_begin / a.kb + 1u) * a.kb - 1u;  // the next last stage
         // (n,k) storage: the lane's own scales and offsets, an iteration ahead. The group of a stage is counted along (a division per
         // stage was a tenth of this loop): k0 = first row of the stage, k0_in = its place in group gi.
         uint32_t sc_next[2] = {0, 0}, of_next[2] = {0, 0};
@@ -598,6 +624,9 @@ wqbmm_mixed_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
         }
         for (uint32_t u = u_begin + grp; u < u_end; u += 2) {
             uint32_t sc[4], of[4], sc_n[2], of_n[2];
+            if constexpr (kRagged) {
+                while (ragged < u) ragged += a.kb;
+            }
             if (kNK) {
                 if (vec) {
                     sc_n[0] = sc_n[1] = pick(sc_v, sel);
@@ -769,6 +798,9 @@ wqbmm_mixed_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
                     }
                 }
                 if (!ok) break;
+                if constexpr (kRagged) {
+                    if (u == ragged && k_in_last < 64u * (un + 1)) mix_clear_past(abase, k_in_last > 64u * un ? k_in_last - 64u * un : 0u);
+                }
                 tmem_st_wait();
                 ptx::tc_fence_before();
                 __syncwarp();
@@ -981,34 +1013,41 @@ MixPlan mix_plan(const OpsnnWqbmmParams* p, int sms, F&& clusters)
 }
 
 using MixKernel = void (*)(const CUtensorMap, const CUtensorMap, const MixArgs);
-template <MixW kW, bool kNK, MixSum kSum>
+template <MixW kW, bool kNK, MixSum kSum, bool kRagged>
 MixKernel mix_kernel_of(bool bf16, bool off)
 {
     if constexpr (kW != MixW::kE4m3) {
-        if (off) return bf16 ? &wqbmm_mixed_kernel<kW, kNK, true, true, kSum> : &wqbmm_mixed_kernel<kW, kNK, false, true, kSum>;
+        if (off) return bf16 ? &wqbmm_mixed_kernel<kW, kNK, true, true, kSum, kRagged> : &wqbmm_mixed_kernel<kW, kNK, false, true, kSum, kRagged>;
     }
-    return bf16 ? &wqbmm_mixed_kernel<kW, kNK, true, false, kSum> : &wqbmm_mixed_kernel<kW, kNK, false, false, kSum>;
+    return bf16 ? &wqbmm_mixed_kernel<kW, kNK, true, false, kSum, kRagged> : &wqbmm_mixed_kernel<kW, kNK, false, false, kSum, kRagged>;
 }
-template <MixSum kSum>
+template <MixSum kSum, bool kRagged>
 MixKernel mix_kernel_of(int w, bool nk, bool bf16, bool off)
 {
     switch (w) {
-        case 0: return nk ? mix_kernel_of<MixW::kInt4, true, kSum>(bf16, off) : mix_kernel_of<MixW::kInt4, false, kSum>(bf16, off);
-        case 1: return nk ? mix_kernel_of<MixW::kInt8, true, kSum>(bf16, off) : mix_kernel_of<MixW::kInt8, false, kSum>(bf16, off);
-        default: return nk ? mix_kernel_of<MixW::kE4m3, true, kSum>(bf16, off) : mix_kernel_of<MixW::kE4m3, false, kSum>(bf16, off);
+        case 0: return nk ? mix_kernel_of<MixW::kInt4, true, kSum, kRagged>(bf16, off) : mix_kernel_of<MixW::kInt4, false, kSum, kRagged>(bf16, off);
+        case 1: return nk ? mix_kernel_of<MixW::kInt8, true, kSum, kRagged>(bf16, off) : mix_kernel_of<MixW::kInt8, false, kSum, kRagged>(bf16, off);
+        default: return nk ? mix_kernel_of<MixW::kE4m3, true, kSum, kRagged>(bf16, off) : mix_kernel_of<MixW::kE4m3, false, kSum, kRagged>(bf16, off);
+    }
+}
+template <bool kRagged>
+MixKernel mix_kernel_of(MixSum sum, int w, bool nk, bool bf16, bool off)
+{
+    switch (sum) {
+        case MixSum::kChain: return mix_kernel_of<MixSum::kChain, kRagged>(w, nk, bf16, off);
+        case MixSum::kCopies: return mix_kernel_of<MixSum::kCopies, kRagged>(w, nk, bf16, off);
+        default: return mix_kernel_of<MixSum::kChunks, kRagged>(w, nk, bf16, off);
     }
 }
 // The kernel of a form, ready to launch on the current device.
 cudaError_t mix_kernel(const OpsnnWqbmmParams* p, MixSum sum, MixKernel* kern)
 {
-    static std::atomic<uint64_t> configured[3 * 24];
-    const bool bf16 = p->x_dtype == ACL_BF16, off = p->offset != nullptr, nk = p->trans_w != 0;
+    static std::atomic<uint64_t> configured[2 * 3 * 24];
+    const bool bf16 = p->x_dtype == ACL_BF16, off = p->offset != nullptr, nk = p->trans_w != 0, ragged = p->k % 128 != 0;
     const int w = p->w_dtype == ACL_INT4 ? 0 : (p->w_dtype == ACL_INT8 ? 1 : 2);
-    const MixKernel k = sum == MixSum::kChain    ? mix_kernel_of<MixSum::kChain>(w, nk, bf16, off)
-                        : sum == MixSum::kCopies ? mix_kernel_of<MixSum::kCopies>(w, nk, bf16, off)
-                                                 : mix_kernel_of<MixSum::kChunks>(w, nk, bf16, off);
+    const MixKernel k = ragged ? mix_kernel_of<true>(sum, w, nk, bf16, off) : mix_kernel_of<false>(sum, w, nk, bf16, off);
     *kern = k;
-    return once_per_device(configured[(int)sum * 24 + w * 8 + (nk ? 4 : 0) + (bf16 ? 2 : 0) + (off ? 1 : 0)], [&] {
+    return once_per_device(configured[(ragged ? 72 : 0) + (int)sum * 24 + w * 8 + (nk ? 4 : 0) + (bf16 ? 2 : 0) + (off ? 1 : 0)], [&] {
         cudaFuncSetAttribute(k, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
         return cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, kMixSmemMax);
     });

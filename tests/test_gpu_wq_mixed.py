@@ -209,3 +209,41 @@ def test_both_entry_points_run_the_same_kernel(aclnn, case):
         outs.append(y)
         assert aclnn.last_kernel_name() == "wqbmm_mixed"
     assert torch.equal(outs[0], outs[1])
+
+
+# k ends half a stage, half a unit, one k step, half a k step and half a pair past the last whole one ((n,k): in rows of whole 16 bytes)
+@pytest.mark.parametrize("kind,nk,k", [(kind, nk, k) for kind in ("int4", "int8", "e4m3") for nk in (False, True) for k in (1088, 1120, 1136, 1128, 1131)
+                                       if not nk or k % (32 if kind == "int4" else 16) == 0])
+def test_rows_past_k_add_nothing_to_an_infinite_column(aclnn, kind, nk, k):
+    """A stage's rows past k read as zero in x and in the packed weight; times an infinite scale they must not turn the column's sum into
+    NaN. (5 rows: accumulators that take turns; 100: one chain.)"""
+    import torch
+
+    from gpu_util import desc, out_tensor, out_to_np
+
+    n = 1056
+    rng = np.random.default_rng(case_seed((kind, nk, k)))
+    if kind == "e4m3":
+        w = rng.uniform(0.5, 2, (k, n)).astype(np.float32).astype(ml_dtypes.float8_e4m3fn)
+    else:
+        w = rng.integers(1, 8, (k, n)).astype(np.int8)
+    scale = rng.uniform(0.005, 0.02, n).astype(np.float32).astype(np.float16)
+    inf_cols = [0, 5, 130, 255, n - 1]
+    scale[inf_cols] = np.inf
+    stored = w.T.copy() if nk else w
+    words = wqbmm_oracle.pack_int4_words(stored) if kind == "int4" else stored
+    d_w = desc(aclnn, words, strides=(1, words.shape[1]), shape=(words.shape[1], words.shape[0])) if nk else desc(aclnn, words)
+    pitch = -(-k // 8) * 8  # rows of x of whole 16 bytes
+    for m in (5, 100):
+        xp = np.zeros((m, pitch), np.float16)
+        xp[:, :k] = rng.uniform(0.5, 1, (m, k)).astype(np.float16)
+        want = wqbmm_oracle.weight_quant_batch_matmul(xp[:, :k].copy(), w, scale, None, None, 0).astype(np.float64)
+        y = out_tensor((m, n), "float16")
+        aclnn.weight_quant_batch_matmul(desc(aclnn, xp, strides=(pitch, 1), shape=(m, k)), d_w, desc(aclnn, scale), aclnn.Tensor((m, n), "float16", y),
+                                        None, None, 0, inner_precise=0)
+        torch.cuda.synchronize()
+        assert aclnn.last_kernel_name() == "wqbmm_mixed", aclnn.last_kernel_name()
+        got = out_to_np(y).astype(np.float64)
+        assert np.array_equal(np.isinf(got), np.isinf(want)) and np.isinf(want[:, inf_cols]).all() and not np.isnan(got).any()
+        ok = np.isfinite(want)
+        assert np.all(np.abs(got[ok] - want[ok]) <= 2.0 ** -10 * np.abs(want[ok]) * 1.01)
