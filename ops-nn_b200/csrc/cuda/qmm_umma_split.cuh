@@ -28,6 +28,7 @@ struct SplitArgs {
     uint32_t* part;                // [2 grid][rows][128 halves] raw 32-bit sums
     unsigned long long* count;     // [tiles] (nonce << 8) | arrivals
     unsigned long long nonce;
+    uint32_t test_stop;  // tests of the give-up path only: k-blocks that a CTA's producer copies before it stops; otherwise all
 };
 
 constexpr int kSplitThreads = 320;
@@ -308,7 +309,8 @@ qmm_umma_split_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_co
         const bool w_mn = a.w_mn != 0, w_batched = a.w_batched != 0, x_batched = a.x_batched != 0;
         uint32_t s = 0, par = 0, t = u_begin / kbs, kb = u_begin - t * kbs;
         SplitTile tile = split_tile(a, t);
-        for (uint32_t u = u_begin; u < u_end; ++u) {
+        const uint32_t u_stop = u_begin + min(u_end - u_begin, a.test_stop);
+        for (uint32_t u = u_begin; u < u_stop; ++u) {
             if (!ptx::mbar_wait_a(empty0 + 8u * s, par ^ 1u, abort_flag)) {
                 report(abort_flag, (1u << 8) | 1u);
                 break;
@@ -706,6 +708,13 @@ int32_t split_launch(const OpsnnQmmParams* p, cudaStream_t stream)
         a.part = reinterpret_cast<uint32_t*>(ws + (((uint64_t)q.tiles * 8u + 255u) & ~(uint64_t)255u));
     }
     a.nonce = next_ks_nonce();
+    a.test_stop = 0xFFFFFFFFu;
+    if (const char* e = env("OPSNN_TEST_SPLIT_STALL_KBLOCK")) {  // tests of the give-up path only
+        a.test_stop = (uint32_t)atoi(e);
+        const char* pl = env("OPSNN_TEST_UMMA_POLL_LIMIT");
+        const uint32_t limit = pl != nullptr ? (uint32_t)atoi(pl) : 20000u;
+        cudaMemcpyToSymbolAsync(ptx::g_spin_limit, &limit, sizeof(limit), 0, cudaMemcpyHostToDevice, stream);
+    }
     CUtensorMap mw, mx;
     const uint64_t nbw = a.w_batched ? (uint64_t)p->batch : 1, nbx = a.x_batched ? (uint64_t)p->batch : 1;
     bool ok = a.w_mn ? make_map(&mw, p->b, (uint64_t)p->n, (uint64_t)p->k, nbw, (uint64_t)p->b_ld, (uint64_t)p->b_bs, 128)

@@ -16,16 +16,20 @@ CASES = [
     # mode, batch, m, k, n, x2 stored (n,k), bias, out
     ("int8", (), 1, 4096, 256, True, "i32", "bfloat16"),       # one or two tiles, a piece per CTA of a cluster
     ("int8", (), 17, 2064, 2064, False, "f32", "bfloat16"),    # ragged k and n, x2 along n
-    ("int8", (), 64, 512, 22000, True, None, "float16"),       # more tiles than SMs: equal pieces across tiles
+    ("int8", (), 64, 512, 22000, True, None, "float16"),       # few k-blocks: a tile a CTA
     ("int8", (), 130, 4112, 272, True, "i32", "bfloat16"),     # two row tiles, few columns
     ("int8", (2,), 33, 1040, 656, True, None, "bfloat16"),     # batched
     ("fp8", (), 16, 6144, 1040, False, "f32", "float16"),
     ("fp8", (), 250, 2048, 528, True, None, "float32"),
     ("e5m2", (), 40, 1072, 20000, True, "f32", "bfloat16"),
     ("block", (), 1, 7168, 400, True, None, "bfloat16"),
-    ("block", (), 48, 1152, 20096, False, None, "float16"),    # per-block pieces across tiles
+    ("block", (), 48, 1152, 20096, False, None, "float16"),    # per-block, a tile a CTA
     ("block", (), 100, 3072, 640, True, None, "float32"),
     ("block", (3,), 20, 1088, 320, True, None, "bfloat16"),    # last k-block half full
+    # more tiles of either shape than SMs: pieces across tiles, summed through workspace
+    ("int8", (), 64, 384, 40960, True, "i32", "float16"),
+    ("fp8", (), 20, 1040, 38416, True, "f32", "bfloat16"),
+    ("block", (), 33, 640, 38416, True, None, "bfloat16"),
 ]
 
 
@@ -69,3 +73,48 @@ def test_split_kernel_equals_oracle(aclnn, monkeypatch, case):
         assert np.array_equal(outs[0].view(np.uint8), np.asarray(want).view(np.uint8))
     else:
         check_close(outs[0], want, qbmm_oracle.quant_matmul_v5(x1, x2, s1, s2, bias, False, nk, group, "float32"), out_name)
+
+
+@pytest.mark.parametrize("mode,m,k,n", [("int8", 128, 4096, 4096),   # a cluster of pieces
+                                        ("int8", 64, 1024, 40960),   # more tiles than SMs: pieces across tiles
+                                        ("block", 24, 7168, 400),     # per-block, pieces across tiles
+                                        ("block", 24, 2048, 9216)])   # a cluster
+def test_wait_that_runs_out_ends_the_call(aclnn, monkeypatch, mode, m, k, n):
+    """The producer stops after its first k-block: every wait behind it runs out, all CTAs of a cluster still meet, nothing is written, later
+    calls are refused until the condition is cleared, and then find tensor memory and workspace as they should."""
+    import torch
+
+    from gpu_util import DEV
+
+    monkeypatch.setenv("OPSNN_QMM_SPLIT", "1")
+    gen = torch.Generator(device=DEV).manual_seed(6)
+    if mode == "int8":
+        x, w = (torch.randint(-127, 128, s, generator=gen, device=DEV, dtype=torch.int8) for s in ((m, k), (n, k)))
+        s1, s2 = (torch.rand(c, generator=gen, device=DEV) * 1e-2 for c in (m, n))
+        group = 0
+    else:
+        x, w = (torch.randn(s, generator=gen, device=DEV).to(torch.float8_e4m3fn) for s in ((m, k), (n, k)))
+        s1, s2 = (torch.rand((-(-c // g), k // 128), generator=gen, device=DEV) for c, g in ((m, 1), (n, 128)))
+        group = (1 << 32) | (128 << 16) | 128
+
+    def run():
+        y = torch.full((m, n), -7777.0, dtype=torch.bfloat16, device=DEV)
+        aclnn.quant_matmul_v5(*(aclnn.from_torch(t) for t in (x, w, s1, s2, y)), None, False, True, group)
+        torch.cuda.synchronize()
+        assert aclnn.last_kernel_name() == ("qmm_umma_split_perblock" if mode == "block" else "qmm_umma_split_deq")
+        return y
+
+    want = run()
+    status = aclnn.lib().opsnn_qmm_umma_status
+    assert status(1) == 0
+    monkeypatch.setenv("OPSNN_TEST_SPLIT_STALL_KBLOCK", "1")
+    monkeypatch.setenv("OPSNN_TEST_UMMA_POLL_LIMIT", "3000")
+    bad = run()
+    monkeypatch.delenv("OPSNN_TEST_SPLIT_STALL_KBLOCK")
+    monkeypatch.delenv("OPSNN_TEST_UMMA_POLL_LIMIT")
+    with pytest.raises(aclnn.AclnnError):
+        run()
+    code = status(1)  # read and cleared, which also restores the poll limit
+    assert (code >> 8) in (2, 3), hex(code)
+    assert bool((bad == -7777.0).all())
+    assert torch.equal(run(), want) and status(1) == 0
