@@ -68,6 +68,7 @@ struct MixArgs {
     unsigned long long* count;     // [tiles] (nonce << 8) | arrivals
     unsigned long long nonce;
     uint32_t idesc;
+    uint32_t test_stop;  // tests of the give-up path only: stages that a CTA's producer copies before it stops; otherwise all
 };
 
 __device__ unsigned int g_mix_status = 0;
@@ -465,8 +466,8 @@ wqbmm_mixed_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
         uint32_t n0 = t0 / (uint32_t)a.t_tiles, r0 = (t0 - n0 * (uint32_t)a.t_tiles) * rows;
         const uint32_t r_end = (uint32_t)(a.t_tiles * a.rows);
         n0 *= kMixTileN;
-        const uint32_t sc_rows = kNK ? 0u : nrows_sc * (kOff ? 2u : 1u);
-        for (uint32_t u = u_begin; u < u_end; ++u) {
+        const uint32_t sc_rows = kNK ? 0u : nrows_sc * (kOff ? 2u : 1u), u_stop = u_begin + min(u_end - u_begin, a.test_stop);
+        for (uint32_t u = u_begin; u < u_stop; ++u) {
             if (!mix_wait(empty0 + 8u * s, par ^ 1u, abort_flag)) {
                 mix_report(abort_flag, (1u << 8) | 1u);
                 break;
@@ -1154,6 +1155,13 @@ int32_t wqbmm_mixed_launch(const OpsnnWqbmmParams* p, cudaStream_t stream)
     a.nonce = next_nonce() & 0x00FFFFFFFFFFFFFFull;
     const uint32_t f = bf16 ? 1u : 0u;
     a.idesc = make_idesc(1u, f, f, 0u, 0u, 128u, (uint32_t)q.rows);
+    a.test_stop = 0xFFFFFFFFu;
+    if (const char* e = env("OPSNN_TEST_MIXED_STALL_STAGE")) {  // tests of the give-up path only
+        a.test_stop = (uint32_t)atoi(e);
+        const char* pl = env("OPSNN_TEST_UMMA_POLL_LIMIT");
+        const uint32_t limit = pl != nullptr ? (uint32_t)atoi(pl) : 20000u;
+        cudaMemcpyToSymbolAsync(ptx::g_spin_limit, &limit, sizeof(limit), 0, cudaMemcpyHostToDevice, stream);
+    }
     CUtensorMap mw, mx;
     const bool ok = nk ? mix_map(&mw, p->w, (uint64_t)p->k * bits / 8, (uint64_t)p->n, (uint64_t)p->w_ld * bits / 8, bits == 4 ? 64u : 128u, kMixTileN)
                        : mix_map(&mw, p->w, (uint64_t)p->n * bits / 8, (uint64_t)p->k, (uint64_t)p->w_ld * bits / 8, 128u, 128u,
@@ -1187,6 +1195,8 @@ uint32_t wqbmm_mixed_status(int reset)
     if (reset) {
         unsigned int z = 0;
         cudaMemcpyToSymbol(g_mix_status, &z, sizeof(z));
+        const uint32_t limit = ptx::kSpinLimit;  // a test may have shortened the waits
+        cudaMemcpyToSymbol(ptx::g_spin_limit, &limit, sizeof(limit));
     }
     return v;
 }

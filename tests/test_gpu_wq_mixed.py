@@ -247,3 +247,40 @@ def test_rows_past_k_add_nothing_to_an_infinite_column(aclnn, kind, nk, k):
         assert np.array_equal(np.isinf(got), np.isinf(want)) and np.isinf(want[:, inf_cols]).all() and not np.isnan(got).any()
         ok = np.isfinite(want)
         assert np.all(np.abs(got[ok] - want[ok]) <= 2.0 ** -10 * np.abs(want[ok]) * 1.01)
+
+
+@pytest.mark.parametrize("m,k,n", [(1, 4096, 4096),     # a cluster of pieces, accumulators that take turns
+                                   (16, 2048, 40960),   # more tiles than SMs: pieces across tiles
+                                   (40, 2048, 40960),   # the same, summed in chunks
+                                   (100, 4096, 4096)])  # a cluster, one chain
+def test_wait_that_runs_out_ends_the_call(aclnn, monkeypatch, m, k, n):
+    """The producer stops after its first stage: every wait behind it runs out, all CTAs of a cluster still meet, nothing is written, the
+    condition is recorded, and the next call finds tensor memory and workspace as it should."""
+    import torch
+
+    from gpu_util import DEV
+
+    gen = torch.Generator(device=DEV).manual_seed(5)
+    x = torch.randn((m, k), generator=gen, device=DEV).to(torch.bfloat16)
+    w = torch.randint(-2 ** 31, 2 ** 31, (k, n // 8), generator=gen, device=DEV, dtype=torch.int32)
+    sc = (torch.rand((k // 128, n), generator=gen, device=DEV) * 0.01 + 0.005).to(torch.bfloat16)
+
+    def run():
+        y = torch.full((m, n), -7777.0, dtype=torch.bfloat16, device=DEV)
+        aclnn.weight_quant_batch_matmul(*(aclnn.from_torch(t) for t in (x, w, sc, y)), None, None, 128, inner_precise=0)
+        torch.cuda.synchronize()
+        assert aclnn.last_kernel_name() == "wqbmm_mixed"
+        return y
+
+    want = run()
+    status = aclnn.lib().opsnn_wqbmm_decode_status
+    assert status(1) == 0
+    monkeypatch.setenv("OPSNN_TEST_MIXED_STALL_STAGE", "1")
+    monkeypatch.setenv("OPSNN_TEST_UMMA_POLL_LIMIT", "3000")
+    bad = run()
+    monkeypatch.delenv("OPSNN_TEST_MIXED_STALL_STAGE")
+    monkeypatch.delenv("OPSNN_TEST_UMMA_POLL_LIMIT")
+    code = status(1)  # read and cleared, which also restores the poll limit
+    assert (code >> 8) in (2, 3, 4), hex(code)  # the MMA issuer, a dequantising or an epilogue warp
+    assert bool((bad == -7777.0).all())
+    assert torch.equal(run(), want) and status(1) == 0
