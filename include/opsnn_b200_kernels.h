@@ -239,12 +239,13 @@ OPSNN_API const char* opsnn_last_kernel_name(void);
  * inside them completed; otherwise the code of the first wait that gave up (the kernel then returned early and its
  * output is undefined). Synchronises the device. reset != 0 clears the word after reading it.
  * The same condition also reaches the caller without polling: the word is mirrored into pinned host memory, and every later
- * tensor-core launch of the process (opsnn_qmm_launch, and through it aclnnQuantMatmulV3/V4/V5 and the prefill path of
- * aclnnWeightQuantBatchMatmul*) first looks at the mirror and, while it is non-zero, refuses with cudaErrorLaunchFailure
+ * tensor-core launch of the process (opsnn_qmm_launch, and through it aclnnQuantMatmulV3/V4/V5 and aclnnWeightQuantBatchMatmul*
+ * with more than 16 rows, whether on a dequantised weight or on OPSNN_WQ_KERNEL_MIXED) first looks at the mirror and, while it is non-zero, refuses with cudaErrorLaunchFailure
  * (ACLNN_ERR_RUNTIME_ERROR at the aclnn level, reason in aclGetRecentErrMsg) until this function is called with reset != 0. */
 OPSNN_API uint32_t opsnn_qmm_umma_status(int32_t reset);
-/* The same for the streaming W4A16 decode kernel that feeds shared memory with bulk tensor copies: 0, or 1 (a stage of
- * operands never arrived) / 2 (a stage buffer was never released). Synchronises the device. */
+/* The same for the streaming decode kernels that feed shared memory with bulk tensor copies: 0, or 1 (a stage of operands never arrived) /
+ * 2 (a stage buffer was never released); and for OPSNN_WQ_KERNEL_MIXED: the role << 8 | reason of the first wait that gave up.
+ * Synchronises the device. */
 OPSNN_API uint32_t opsnn_wqbmm_decode_status(int32_t reset);
 /* How the calling thread's last streaming decode launch (W4A16 / W8A16, bulk-copy kernels) cut the problem: strips of 512
  * columns, k-ranges per strip, and whether the k-ranges of a strip ran as one thread-block cluster (summed over distributed

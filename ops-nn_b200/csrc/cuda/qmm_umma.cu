@@ -910,6 +910,7 @@ namespace {
 
 std::atomic<unsigned int*> g_status_host_word{nullptr};
 std::atomic<uint64_t> g_status_armed{0};
+std::atomic<unsigned int*> g_status_device_word[64];  // the word's address on each device
 
 // Once per process: one pinned, device-visible word. Once per device: its address into g_umma_status_host.
 cudaError_t arm_status_mirror()
@@ -927,7 +928,12 @@ cudaError_t arm_status_mirror()
         unsigned int* dptr = nullptr;
         cudaError_t rc = cudaHostGetDevicePointer(reinterpret_cast<void**>(&dptr), w, 0);
         if (rc != cudaSuccess) return rc;
-        return cudaMemcpyToSymbol(g_umma_status_host, &dptr, sizeof(dptr));
+        rc = cudaMemcpyToSymbol(g_umma_status_host, &dptr, sizeof(dptr));
+        if (rc != cudaSuccess) return rc;
+        int dev = 0;
+        cudaGetDevice(&dev);
+        g_status_device_word[dev & 63].store(dptr, std::memory_order_release);
+        return cudaSuccess;
     });
 }
 
@@ -950,6 +956,22 @@ int32_t umma_prelaunch_check()
             "opsnn_qmm_umma_status(1) clears the condition",
             code >> 8, code & 0xFFu);
     return (int32_t)cudaErrorLaunchFailure;
+}
+
+// The same for a kernel with an error word of its own: also the mirror's address on the current device, nullptr where there is none yet and
+// `stream` is being captured (which allows neither the allocation nor the copy).
+int32_t umma_prelaunch_check(cudaStream_t stream, unsigned int** mirror)
+{
+    *mirror = nullptr;
+    int dev = 0;
+    cudaGetDevice(&dev);
+    if (g_status_device_word[dev & 63].load(std::memory_order_acquire) == nullptr) {
+        cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
+        if (cudaStreamIsCapturing(stream, &capture) != cudaSuccess || capture != cudaStreamCaptureStatusNone) return 0;
+    }
+    const int32_t bad = umma_prelaunch_check();
+    *mirror = g_status_device_word[dev & 63].load(std::memory_order_acquire);
+    return bad;
 }
 
 int32_t qmm_umma_launch(const OpsnnQmmParams* p, cudaStream_t stream)
@@ -1067,12 +1089,14 @@ extern "C" __attribute__((visibility("default"))) uint32_t opsnn_qmm_umma_status
 {
     unsigned int v = 0;
     cudaMemcpyFromSymbol(&v, opsnn::g_umma_status, sizeof(v));
+    volatile unsigned int* const mirror = opsnn::g_status_host_word.load(std::memory_order_acquire);
+    if (v == 0u && mirror != nullptr) v = *mirror;  // the fused weight-only kernel's
     if (reset) {
         unsigned int z = 0;
         cudaMemcpyToSymbol(opsnn::g_umma_status, &z, sizeof(z));
         const uint32_t limit = opsnn::ptx::kSpinLimit;  // a test may have shortened the waits: back to the normal limit
         cudaMemcpyToSymbol(opsnn::ptx::g_spin_limit, &limit, sizeof(limit));
-        if (unsigned int* w = opsnn::g_status_host_word.load(std::memory_order_acquire)) *reinterpret_cast<volatile unsigned int*>(w) = 0u;
+        if (mirror != nullptr) *mirror = 0u;
     }
     return v;
 }

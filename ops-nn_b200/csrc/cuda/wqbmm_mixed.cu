@@ -8,13 +8,15 @@
 // Orientation: D^T = W'^T x^T. The MMA's 128 rows are weight columns, its N is the rows of x (16 ... 128 of them, a multiple of 16), so
 // the tensor core's work shrinks with m while the dequantisation - what bounds this kernel - is done once whatever m is.
 //   CTA tile: 256 weight columns (two M = 128 accumulators) x N rows of x; persistent, one CTA per SM (all 512 TMEM columns).
-//   Work is cut stream-k: the (tile, k stage) pairs in one line, every CTA an equal contiguous piece. A tile that several CTAs share is
-//   combined through workspace in CTA order by whichever of them arrives last (deterministic; nobody waits for anybody).
+//   The (tile, k stage of 128 rows) pairs lie in one line, and every CTA has a contiguous piece of it (mix_plan):
+//     a tile into `split` equal pieces, launched as a cluster: every CTA sums a slice of the tile out of the cluster's shared memory; or
+//     stream-k, all CTAs the same share: a tile that several CTAs share is combined through workspace by whichever arrives last.
+//   Pieces are added in the order of k either way (deterministic; in the second nobody waits for anybody).
 //   warps 0-15   dequantise. Warp w serves TMEM lanes 32 (w % 4) .. (a hardware rule), accumulator half (w / 4) % 2, and every other
-//                64-row unit of k (w / 8). packed words -> registers (ldmatrix.trans for (k,n) storage: a register then holds nibbles /
+//                stage (w / 8). packed words -> registers (ldmatrix.trans for (k,n) storage: a register then holds nibbles /
 //                bytes of k rows 2q, 2q + 1, already the pair that a TMEM cell of A wants; a row per lane for (n,k) storage) ->
 //                the decode kernels' pair arithmetic -> tcgen05.st.
-//   warps 16-19  epilogue, overlapped with the next tile's main loop.
+//   warps 16-19  epilogue of all but the CTA's last tile, overlapped with the next tile's main loop; the last is finished by warps 0-15.
 //   warp 20      TMA producer (packed weight, x, scale / offset rows), warp 21 MMA issuer.
 // A operand buffers: four units of 64 k x 256 columns (64 TMEM columns each) at columns 256-511; accumulators at 0-255 (two sets while
 // N <= 64).
@@ -28,6 +30,8 @@
 #include "wqbmm_decode_common.cuh"
 
 namespace opsnn {
+
+int32_t umma_prelaunch_check(cudaStream_t stream, unsigned int** mirror);
 
 namespace {
 
@@ -68,15 +72,20 @@ struct MixArgs {
     unsigned long long* count;     // [tiles] (nonce << 8) | arrivals
     unsigned long long nonce;
     uint32_t idesc;
+    volatile unsigned int* status_host;  // pinned mirror of the error word that later launches look at; nullptr: none
     uint32_t test_stop;  // tests of the give-up path only: stages that a CTA's producer copies before it stops; otherwise all
 };
 
 __device__ unsigned int g_mix_status = 0;
 
-__device__ __forceinline__ void mix_report(volatile uint32_t* abort_flag, unsigned int code)
+__device__ __forceinline__ void mix_report(const MixArgs& a, volatile uint32_t* abort_flag, unsigned int code)
 {
     *abort_flag = 1u;
     atomicCAS(&g_mix_status, 0u, code);
+    if (a.status_host != nullptr) {
+        *a.status_host = code;
+        __threadfence_system();
+    }
 }
 
 __device__ __forceinline__ void mix_tma_2d(uint32_t smem_dst, const CUtensorMap* map, uint32_t bar_addr, int32_t c0, int32_t c1)
@@ -308,7 +317,7 @@ __device__ __forceinline__ void mix_finish(const MixArgs& a, uint32_t acc, uint3
             done = prev == cur;
             cur = prev;
         }
-        if (!done) mix_report(abort_flag, (4u << 8) | 2u);
+        if (!done) mix_report(a, abort_flag, (4u << 8) | 2u);
         const bool last = done && (uint32_t)(want & 0xFFull) == c1 - c0 + 1u;
         if (last) *reinterpret_cast<volatile unsigned long long*>(cnt_p) = 0ull;  // a replay of this launch starts clean
         *s_last = last ? 1u : 0u;
@@ -469,7 +478,7 @@ wqbmm_mixed_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
         const uint32_t sc_rows = kNK ? 0u : nrows_sc * (kOff ? 2u : 1u), u_stop = u_begin + min(u_end - u_begin, a.test_stop);
         for (uint32_t u = u_begin; u < u_stop; ++u) {
             if (!mix_wait(empty0 + 8u * s, par ^ 1u, abort_flag)) {
-                mix_report(abort_flag, (1u << 8) | 1u);
+                mix_report(a, abort_flag, (1u << 8) | 1u);
                 break;
             }
             if (ptx::elect_one()) {
@@ -515,21 +524,21 @@ wqbmm_mixed_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
         while (u < u_end && ok) {
             const uint32_t cnt = min(min(kbs - kb, u_end - u), chunk);
             if (!mix_wait(dempty0 + 8u * dbuf, dpar ^ 1u, abort_flag)) {
-                mix_report(abort_flag, (2u << 8) | 1u);
+                mix_report(a, abort_flag, (2u << 8) | 1u);
                 break;
             }
             const uint32_t d0 = tmem + dbuf * d_set;
             uint32_t acc = 0u;
             for (uint32_t i = 0; i < cnt && ok; ++i) {
                 if (!mix_wait(full0 + 8u * s, par, abort_flag)) {
-                    mix_report(abort_flag, (2u << 8) | 2u);
+                    mix_report(a, abort_flag, (2u << 8) | 2u);
                     ok = false;
                     break;
                 }
 #pragma unroll
                 for (int un = 0; un < 2; ++un) {
                     if (!mix_wait(afull0 + 8u * ab, apar, abort_flag)) {
-                        mix_report(abort_flag, (2u << 8) | 3u);
+                        mix_report(a, abort_flag, (2u << 8) | 3u);
                         ok = false;
                         break;
                     }
@@ -651,7 +660,7 @@ wqbmm_mixed_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
                 }
             }
             if (!mix_wait(full0 + 8u * s, par, abort_flag)) {
-                mix_report(abort_flag, (3u << 8) | 1u);
+                mix_report(a, abort_flag, (3u << 8) | 1u);
                 ok = false;
                 break;
             }
@@ -698,7 +707,7 @@ wqbmm_mixed_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
                     if (waited) return;
                     waited = true;
                     if (!mix_wait(aempty0 + 8u * ab, apar ^ 1u, abort_flag)) {
-                        mix_report(abort_flag, (3u << 8) | 2u);
+                        mix_report(a, abort_flag, (3u << 8) | 2u);
                         ok = false;
                     }
                     ptx::tc_fence_after();
@@ -828,7 +837,7 @@ wqbmm_mixed_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
         }
         const uint32_t dbuf = two_d ? (before & 1u) : 0u;
         if (ok && (!mix_wait(fin0, 0u, abort_flag) || (has_sum && !mix_wait(fsum0, 0u, abort_flag)))) {
-            mix_report(abort_flag, (3u << 8) | 3u);
+            mix_report(a, abort_flag, (3u << 8) | 3u);
             ok = false;
         }
         if (mix_all_ok<2, kMixDqWarps * 32>(ok)) {
@@ -858,7 +867,7 @@ wqbmm_mixed_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
         auto next_set = [&](bool relaxed) {  // waits for an accumulator set; the four warps go on, or leave, together
             const bool got = relaxed ? __all_sync(0xffffffffu, ptx::mbar_wait_relaxed(&s_bars[2 * kMixMaxStages + 2 * kMixABufs + dbuf], dpar, abort_flag))
                                      : mix_wait(dfull0 + 8u * dbuf, dpar, abort_flag);
-            if (!got) mix_report(abort_flag, (4u << 8) | 1u);
+            if (!got) mix_report(a, abort_flag, (4u << 8) | 1u);
             const bool ok = mix_all_ok<1, kMixEpWarps * 32>(got);
             ptx::tc_fence_after();
             return ok;
@@ -1155,6 +1164,12 @@ int32_t wqbmm_mixed_launch(const OpsnnWqbmmParams* p, cudaStream_t stream)
     a.nonce = next_nonce() & 0x00FFFFFFFFFFFFFFull;
     const uint32_t f = bf16 ? 1u : 0u;
     a.idesc = make_idesc(1u, f, f, 0u, 0u, 128u, (uint32_t)q.rows);
+    // More than 16 rows: as a dequantised weight's matmul would, a call after one that gave up a wait is refused.
+    if (p->m > 16) {
+        unsigned int* mirror;
+        if (const int32_t bad = umma_prelaunch_check(stream, &mirror)) return bad;
+        a.status_host = mirror;
+    }
     a.test_stop = 0xFFFFFFFFu;
     if (const char* e = env("OPSNN_TEST_MIXED_STALL_STAGE")) {  // tests of the give-up path only
         a.test_stop = (uint32_t)atoi(e);

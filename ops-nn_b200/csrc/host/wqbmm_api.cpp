@@ -287,7 +287,8 @@ aclnnStatus wq_run(const char* api, void* workspace, uint64_t workspaceSize, acl
     }
     int32_t rc = opsnn_wqbmm_launch(&p, choice, stream);
     if (rc != 0) {
-        set_err("%s: kernel launch failed with CUDA error %d", api, rc);
+        const std::string why = aclGetRecentErrMsg() ? aclGetRecentErrMsg() : "";
+        set_err("%s: kernel launch failed with CUDA error %d%s%s", api, rc, why.empty() ? "" : ": ", why.c_str());
         return ACLNN_ERR_RUNTIME_ERROR;
     }
     return ACLNN_SUCCESS;

@@ -280,6 +280,11 @@ def test_wait_that_runs_out_ends_the_call(aclnn, monkeypatch, m, k, n):
     bad = run()
     monkeypatch.delenv("OPSNN_TEST_MIXED_STALL_STAGE")
     monkeypatch.delenv("OPSNN_TEST_UMMA_POLL_LIMIT")
+    if m > 16:  # as with a dequantised weight's matmul, whose calls these were: refused before anything is enqueued, until cleared
+        with pytest.raises(aclnn.AclnnError) as err:
+            run()
+        assert err.value.status == aclnn.ACLNN_ERR_RUNTIME_ERROR and "bounded wait" in str(err.value)
+        assert aclnn.lib().opsnn_qmm_umma_status(1) != 0
     code = status(1)  # read and cleared, which also restores the poll limit
     assert (code >> 8) in (2, 3, 4), hex(code)  # the MMA issuer, a dequantising or an epilogue warp
     assert bool((bad == -7777.0).all())
