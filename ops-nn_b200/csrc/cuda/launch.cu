@@ -95,8 +95,8 @@ static bool streaming_asked_for()
 
 // The fused kernel (wqbmm_mixed.cu) reads the packed weight once for up to 128 rows of x and has no mma.sync and no 16-bit image of the
 // weight to pay for, so it is the faster form of nearly every call (bf16, groups of 128 with offset, graph replay, us, before -> fused):
-//   m 1   4096 x 4096 12.1 -> 8.6      m 16  8192 x 28672 49.3 -> 39.1     m 16 int8 4096 x 14336 20.2 -> 15.2
-//   m 32  8192 x 28672 98 -> 43        m 128 8192 x 28672 285 -> 67        m 512 8192 x 28672 416 -> 237
+//   m 1   4096 x 4096 12.1 -> 9.05     m 16  8192 x 28672 49.3 -> 39.7     m 16 int8 4096 x 14336 20.2 -> 17.2
+//   m 32  8192 x 28672 98 -> 40        m 128 8192 x 28672 285 -> 59        m 512 8192 x 28672 416 -> 233
 // It does not take: innerPrecise = 1 (the group-wise arithmetic of the streaming kernels), outputs bound to a communicator (only the
 // streaming kernels store into the peers), a FRACTAL_NZ weight, and m > 1152, where dequantising the weight
 // once per 128 rows costs more than a pass over HBM (against pre-pass and matmul, us: m 1100 8192 x 28672 int4 514 / 578, 4096^2 40 / 53;

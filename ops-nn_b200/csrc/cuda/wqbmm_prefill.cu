@@ -10,7 +10,8 @@
 // summation order.
 //
 // HBM cost of the pre-pass: n*k/2 (int4) read + 2*n*k written, then 2*n*k read once by the matmul (x stays in L2):
-// worthwhile once the matmul's 2*m*n*k flops dominate; below m = 17 the fused streaming decode kernels are used.
+// worthwhile once the matmul's 2*m*n*k flops dominate; up to m = 1152 the fused kernel (wqbmm_mixed.cu) and the streaming decode
+// kernels take what they can.
 #include <cstdlib>
 #include <type_traits>
 
