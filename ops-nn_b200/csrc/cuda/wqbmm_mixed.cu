@@ -78,15 +78,17 @@ struct MixArgs {
 
 __device__ unsigned int g_mix_status = 0;
 
-__device__ __forceinline__ void mix_report(const MixArgs& a, volatile uint32_t* abort_flag, unsigned int code)
+// (Out of line: a dozen calls of it are in the kernel, none of them on the way that it takes.)
+static __device__ __noinline__ void mix_report_at(volatile unsigned int* status_host, volatile uint32_t* abort_flag, unsigned int code)
 {
     *abort_flag = 1u;
     atomicCAS(&g_mix_status, 0u, code);
-    if (a.status_host != nullptr) {
-        *a.status_host = code;
+    if (status_host != nullptr) {
+        *status_host = code;
         __threadfence_system();
     }
 }
+__device__ __forceinline__ void mix_report(const MixArgs& a, volatile uint32_t* abort_flag, unsigned int code) { mix_report_at(a.status_host, abort_flag, code); }
 
 __device__ __forceinline__ void mix_tma_2d(uint32_t smem_dst, const CUtensorMap* map, uint32_t bar_addr, int32_t c0, int32_t c1)
 {
