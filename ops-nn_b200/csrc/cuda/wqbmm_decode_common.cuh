@@ -90,6 +90,12 @@ struct Num<true> {
         asm("mul.rn.bf16x2 %0, %1, %2;" : "=r"(d) : "r"(a), "r"(b));
         return d;
     }
+    __device__ __forceinline__ static uint32_t fma(uint32_t a, uint32_t b, uint32_t c)
+    {
+        uint32_t d;
+        asm("fma.rn.bf16x2 %0, %1, %2, %3;" : "=r"(d) : "r"(a), "r"(b), "r"(c));
+        return d;
+    }
     // same instruction, not volatile: the compiler may interleave it with the logic ops of the next k-step
     __device__ __forceinline__ static void mma_free(float (&d)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1)
     {
@@ -125,6 +131,12 @@ struct Num<false> {
     {
         uint32_t d;
         asm("mul.rn.f16x2 %0, %1, %2;" : "=r"(d) : "r"(a), "r"(b));
+        return d;
+    }
+    __device__ __forceinline__ static uint32_t fma(uint32_t a, uint32_t b, uint32_t c)
+    {
+        uint32_t d;
+        asm("fma.rn.f16x2 %0, %1, %2, %3;" : "=r"(d) : "r"(a), "r"(b), "r"(c));
         return d;
     }
     __device__ __forceinline__ static void mma_free(float (&d)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1)

@@ -17,12 +17,19 @@
 //                bytes of k rows 2q, 2q + 1, already the pair that a TMEM cell of A wants; a row per lane for (n,k) storage) ->
 //                the decode kernels' pair arithmetic -> tcgen05.st.
 //   warps 16-19  epilogue of all but the CTA's last tile, overlapped with the next tile's main loop; the last is finished by warps 0-15.
-//   warp 20      TMA producer (packed weight, x, scale / offset rows), warp 21 MMA issuer.
-// A operand buffers: four units of 64 k x 256 columns (64 TMEM columns each) at columns 256-511; accumulators at 0-255 (two sets while
-// N <= 64).
+//   warp 20      TMA producer (packed weight, x, scale / offset rows), warps 21 and 22 MMA issuers, one for each accumulator half.
+// A operand buffers: four of 128 k x 128 columns (64 TMEM columns each) at columns 256-511, one for either half of two stages in turn;
+// accumulators at 0-255 (two sets while N <= 64).
+// What bounds it: instructions issued by the dequantising warps. A stage is 64 pairs a lane (int4 3 - 4.75 instructions each, the integer ones
+// and the 16-bit ones two clocks a warp) and as much again of waits, scales, arrivals and other roles' polling; every wait, even for a
+// barrier long completed, is 80 clocks. So buffers change hands by the stage and not by 64 rows of k, a warp arrives under a predicate
+// instead of a branch, and scales that allow it save the magic number (MixFast). Before / after, us: 16 x 8192 x 28672 int4 with offset
+// 39.7 / 37.3, 77 x 7168 x 18432 int4 (n,k) fp16 28.1 / 24.7, 4 x 4096 x 14336 int8 (n,k) fp16 18.3 / 16.3, 1 x 4096 x 4096 9.3 / 8.8. Without the
+// arithmetic the second is 20, without the MMAs 24; stores to tensor memory run at 0.5 - 1 KB a clock and cost nothing.
 // Every wait is bounded; a wait that gives up raises the CTA's abort flag, records a code and the CTA tears down (TMEM freed).
 #include <algorithm>
 #include <cstdio>
+#include <type_traits>
 
 #include "common.cuh"
 #include "sm100_ptx.cuh"
@@ -37,7 +44,8 @@ namespace {
 
 constexpr int kMixTileN = 256;
 constexpr int kMixDqWarps = 16, kMixEpWarps = 4;
-constexpr int kMixThreads = (kMixDqWarps + kMixEpWarps + 2) * 32;
+constexpr int kMixMmaWarps = 2;
+constexpr int kMixThreads = (kMixDqWarps + kMixEpWarps + 1 + kMixMmaWarps) * 32;
 constexpr int kMixMaxRows = 128;   // rows of x per pass over the weight
 constexpr int kMixABufs = 4;
 constexpr uint32_t kMixACol = 256;  // first TMEM column of the A buffers
@@ -100,10 +108,46 @@ __device__ __forceinline__ void mix_arrive(uint32_t bar_addr)
 {
     asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(bar_addr) : "memory");
 }
+// Has the phase completed? Does not wait.
+__device__ __forceinline__ bool mix_test(uint32_t bar_addr, uint32_t parity)
+{
+    uint32_t ok;
+    asm volatile("{\n\t.reg .pred p;\n\tmbarrier.test_wait.parity.shared::cta.b64 p, [%1], %2;\n\tselp.u32 %0, 1, 0, p;\n\t}"
+                 : "=r"(ok)
+                 : "r"(bar_addr), "r"(parity)
+                 : "memory");
+    return ok != 0;
+}
+// A wait that is expected to be long and whose end is not urgent: the four epilogue warps sleep between polls, else their polling is a fifth of
+// all instructions issued.
+static __device__ __noinline__ bool mix_wait_asleep(uint32_t bar_addr, uint32_t parity, volatile uint32_t* abort_flag)
+{
+    const uint32_t limit = ptx::g_spin_limit / 64u + 1u;
+    for (uint32_t i = 0; i < limit; ++i) {
+        if (ptx::mbar_try_wait_a(bar_addr, parity)) return true;
+        if (*abort_flag != 0u) return false;
+        __nanosleep(1000);
+    }
+    *abort_flag = 1u;
+    return false;
+}
 // Bounded wait with one answer for the warp: what follows it is .sync.aligned.
 __device__ __forceinline__ bool mix_wait(uint32_t bar_addr, uint32_t parity, volatile uint32_t* abort_flag)
 {
-    return __all_sync(0xffffffffu, ptx::mbar_wait_a(bar_addr, parity, abort_flag));
+    uint32_t done;
+    asm volatile(
+        "{\n\t.reg .pred p, q;\n\tmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\tvote.sync.all.pred q, p, 0xffffffff;\n\t"
+        "selp.u32 %0, 1, 0, q;\n\t}"
+        : "=r"(done)
+        : "r"(bar_addr), "r"(parity)
+        : "memory");
+    return done != 0u || __all_sync(0xffffffffu, ptx::mbar_wait_slow_a(bar_addr, parity, abort_flag));
+}
+// A warp's arrival: one for all its lanes' earlier accesses (predicated: no branch).
+__device__ __forceinline__ void mix_arrive_warp(uint32_t bar_addr, int lane)
+{
+    __syncwarp();
+    asm volatile("{\n\t.reg .pred p;\n\tsetp.eq.s32 p, %1, 0;\n\t@p mbarrier.arrive.shared::cta.b64 _, [%0];\n\t}" ::"r"(bar_addr), "r"(lane) : "memory");
 }
 // Barrier of kThreads threads that tells all of them whether every one came with `ok`: they go on, or leave, together.
 template <int kBar, int kThreads>
@@ -168,13 +212,105 @@ __device__ __forceinline__ void umma_f16_ta(uint32_t d_tmem, uint32_t a_tmem, ui
         : "memory");
 }
 
+// The same weights in fewer instructions, where a lane's scales allow it. Integer and 16-bit-pair instructions both take two clocks a warp, and
+// a pair of int4 weights was 1.75 - 2.25 of the first and two of the second.
+// A code (less its sign flip: w + z, z = 8 or 128) left in the low bits of a 16-bit half is a subnormal there: it reads as (w + z) * 2^-E, E by the
+// bit it starts at, without a magic number to take off again. So fma(code, s * 2^E, -z * s) = rn(w * s): product and subtrahend are exact,
+// one rounding, one instruction. Needs s * 2^E finite: |s| < 2^-5 (bf16; fp16 int4), 2^-8 (fp16 int8). (e4m3: its magnitude bits read as
+// w * 2^-120 / 2^-8 already, and the product with s * 2^120 / 2^8 is the one rounding; |s| < 2^8.)
+// A warp one of whose lanes has other scales in a stage (infinities and NaN among them) takes the general arithmetic for that stage.
+// With an offset (two roundings) the same idea saves no 16-bit instruction, and what the scaled offsets cost is more than the two shifts it
+// saves (16 x 8192 x 28672 bf16: 38.6 -> 40.0 us): general arithmetic.
+template <MixW kW, bool kNK, bool kBf16, bool kOff>
+struct MixFast {
+    using N = Num<kBf16>;
+    static constexpr bool kHas = !kOff;
+    static constexpr uint32_t pow2(int e)
+    {
+        const uint32_t v = kBf16 ? (uint32_t)(127 + e) << 7 : (uint32_t)(15 + e) << 10;
+        return v | (v << 16);
+    }
+    static constexpr int kTop = kBf16 ? 127 : 15;  // the largest power of two
+    // E of the code of word position b ((k,n) int4: the word's columns alternate between two)
+    static constexpr int exponent(int b)
+    {
+        if (kW == MixW::kE4m3) return kBf16 ? 120 : 8;
+        if (kW == MixW::kInt8) return kBf16 ? 133 : 24;
+        if (kNK) return kBf16 ? 133 : 21;
+        return kBf16 ? ((b & 1) ? 129 : 133) : ((b & 1) ? 17 : 21);
+    }
+    static constexpr uint32_t kZero = kW == MixW::kInt4 ? (kBf16 ? 0xC100C100u : 0xC800C800u) : (kBf16 ? 0xC300C300u : 0xD800D800u);  // -z
+    __device__ __forceinline__ static uint32_t lop(uint32_t a, uint32_t mask, uint32_t flip)
+    {
+        uint32_t v;
+        asm("lop3.b32 %0, %1, %2, %3, 0x6A;" : "=r"(v) : "r"(a), "r"(mask), "r"(flip));
+        return v;
+    }
+    // Scales of two columns (or one, twice) whose word positions are b0 (low half) and b1: multiplier and addend of `pair` below. Returns whether
+    // they allow it.
+    __device__ __forceinline__ static bool prepare(uint32_t sc, int b0, int b1, uint32_t& mul, uint32_t& add)
+    {
+        if (kW == MixW::kE4m3) {
+            mul = N::mul(sc, pow2(exponent(0)));
+        } else {
+            const uint32_t rest = (pow2(exponent(b0) > kTop ? exponent(b0) - kTop : 0) & 0xFFFFu) | (pow2(exponent(b1) > kTop ? exponent(b1) - kTop : 0) & 0xFFFF0000u);
+            mul = N::mul(N::mul(sc, pow2(kTop)), rest);
+        }
+        add = N::mul(sc, kZero);
+        // an infinity or NaN carries into bit 15 or 31
+        return (((mul & 0x7FFF7FFFu) + (kBf16 ? 0x00800080u : 0x04000400u)) & 0x80008000u) == 0u;
+    }
+    __device__ __forceinline__ static uint32_t pair(uint32_t code, uint32_t mul, uint32_t add) { return kW == MixW::kE4m3 ? N::mul(code, mul) : N::fma(code, mul, add); }
+    // (k,n) int4: the pair of column b of a word (its nibble b and nibble 4 + b)
+    __device__ __forceinline__ static void codes4(uint32_t w, uint32_t (&c)[4])
+    {
+        const uint32_t lo = kBf16 ? w : w << 3, hi = kBf16 ? w >> 8 : w >> 5;
+        constexpr uint32_t m0 = kBf16 ? 0x000F000Fu : 0x00780078u, f0 = kBf16 ? 0x00080008u : 0x00400040u;
+        constexpr uint32_t m1 = kBf16 ? 0x00F000F0u : 0x07800780u, f1 = kBf16 ? 0x00800080u : 0x04000400u;
+        c[0] = lop(lo, m0, f0);
+        c[1] = lop(lo, m1, f1);
+        c[2] = lop(hi, m0, f0);
+        c[3] = lop(hi, m1, f1);
+    }
+    // (n,k) int4: the pairs of nibbles 2 b and 2 b + 1. A byte's zero top bit, replicated, is the half's upper byte.
+    __device__ __forceinline__ static void codes4_nk(uint32_t w, uint32_t (&c)[4])
+    {
+        const uint32_t a = kBf16 ? lop(w, 0x0F0F0F0Fu, 0x08080808u) : lop(w << 3, 0x78787878u, 0x40404040u);
+        const uint32_t d = kBf16 ? lop(w >> 4, 0x0F0F0F0Fu, 0x08080808u) : lop(w >> 1, 0x78787878u, 0x40404040u);
+        c[0] = prmt(a, d, 0xC480u);
+        c[1] = prmt(a, d, 0xD591u);
+        c[2] = prmt(a, d, 0xE6A2u);
+        c[3] = prmt(a, d, 0xF7B3u);
+    }
+    // (k,n), 8 bits: the pair of column b; (n,k), 8 bits: the pair of bytes 2 b, 2 b + 1
+    __device__ __forceinline__ static void codes8(uint32_t w, uint32_t (&c)[2])
+    {
+        if constexpr (kW == MixW::kE4m3) {
+            c[0] = e4m3_bits(kNK ? prmt(w, 0u, 0x4140u) : w);
+            c[1] = e4m3_bits(kNK ? prmt(w, 0u, 0x4342u) : w >> 8);
+        } else if constexpr (kNK) {
+            const uint32_t x = w ^ 0x80808080u;
+            c[0] = prmt(x, 0u, 0x4140u);
+            c[1] = prmt(x, 0u, 0x4342u);
+        } else {
+            c[0] = lop(w, 0x00FF00FFu, 0x00800080u);
+            c[1] = lop(w >> 8, 0x00FF00FFu, 0x00800080u);
+        }
+    }
+    __device__ __forceinline__ static uint32_t e4m3_bits(uint32_t p)
+    {
+        uint32_t v = (p << (kBf16 ? 4 : 7)) & (kBf16 ? 0x07F007F0u : 0x3F803F80u);
+        asm("lop3.b32 %0, %1, %2, %3, 0xEA;" : "=r"(v) : "r"(p << 8), "n"(0x80008000), "r"(v));
+        return v;
+    }
+};
+
 // One stage: 128 rows of k x 256 columns. (With 64-row stages the producer's and the MMA issuer's fixed cost per stage showed.)
 template <MixW kW>
 struct MixCfg {
     static constexpr int kBits = kW == MixW::kInt4 ? 4 : 8;
     static constexpr int kBK = 128;
     static constexpr int kWBytes = kMixTileN * kBK * kBits / 8;
-    static constexpr int kEmptyArrivals = kMixDqWarps / 2 + 1;
 };
 
 // TMEM lane (within a warp's 32) -> weight column (within the warp's 32)
@@ -411,6 +547,7 @@ __global__ void __launch_bounds__(kMixThreads, 1)
 wqbmm_mixed_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUtensorMap map_x, const __grid_constant__ MixArgs a)
 {
     using C = MixCfg<kW>;
+    using F = MixFast<kW, kNK, kBf16, kOff>;
     const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0);
     const int lane = threadIdx.x & 31;
     extern __shared__ uint8_t dyn_raw[];
@@ -428,19 +565,19 @@ wqbmm_mixed_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
         s_abort = 0u;
         for (uint32_t i = 0; i < a.stages; ++i) {
             mix_init(full0 + 8u * i, 1u);
-            mix_init(empty0 + 8u * i, (uint32_t)C::kEmptyArrivals);
+            mix_init(empty0 + 8u * i, kMixDqWarps / 2 + kMixMmaWarps);
         }
         for (int i = 0; i < kMixABufs; ++i) {
-            mix_init(afull0 + 8u * i, kMixDqWarps / 2);
+            mix_init(afull0 + 8u * i, 4u);
             mix_init(aempty0 + 8u * i, 1u);
         }
         for (int i = 0; i < 2; ++i) {
-            mix_init(dfull0 + 8u * i, 1u);
+            mix_init(dfull0 + 8u * i, kMixMmaWarps);
             mix_init(dempty0 + 8u * i, kMixEpWarps);
         }
         // the last piece's sums, and those of its chunks before the last (barriers of their own: the warps that wait for them have not
         // followed the others' phases)
-        mix_init(fin0, 1u);
+        mix_init(fin0, kMixMmaWarps);
         mix_init(fsum0, kMixEpWarps);
         ptx::fence_mbar_init();
         ptx::fence_proxy_async();
@@ -513,13 +650,18 @@ wqbmm_mixed_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
                 if (r0 == r_end) { r0 = 0; n0 += kMixTileN; }
             }
         }
-    } else if (warp == kMixDqWarps + kMixEpWarps + 1) {
-        // ======================= MMA issuer =======================
+    } else if (warp > kMixDqWarps + kMixEpWarps) {
+        // ======================= MMA issuers =======================
+        // Two warps, one for each accumulator half (and so on schedulers of their own): a buffer's MMAs are few and short (N = 16: 20 clocks
+        // each), so what else it costs shows: a wait for a barrier that has long completed is 80 clocks of latency. So the next buffer's
+        // barrier is looked at before this one's MMAs are issued, and the stage's own barrier not at all: the dequantising warps have
+        // waited for it before they arrived on `afull`.
         const uint64_t db = ptx::make_smem_desc(smem0 + a.x_off, 0, 1024, 2);
         const uint32_t b_lo = (uint32_t)db;
         const uint64_t b_hi = db & 0xFFFFFFFF00000000ull;
-        uint32_t s = 0, par = 0, ab = 0, apar = 0, dbuf = 0, dpar = 0;
-        bool ok = true;
+        const uint32_t h = (uint32_t)(warp - (kMixDqWarps + kMixEpWarps + 1));
+        uint32_t s = 0, ab = h, apar = 0, dbuf = 0, dpar = 0;
+        bool ok = true, ready = false;
         const uint32_t kbs = a.kb, rows = (uint32_t)a.rows, idesc = a.idesc, chunk = kSum == MixSum::kChunks ? a.chunk : kbs;
         const uint32_t copies = a.copies, turn1 = d_one, turn2 = 2u * d_one, turn3 = 3u * d_one;
         uint32_t u = u_begin, kb = u_begin % kbs;
@@ -529,42 +671,37 @@ wqbmm_mixed_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
                 mix_report(a, abort_flag, (2u << 8) | 1u);
                 break;
             }
-            const uint32_t d0 = tmem + dbuf * d_set;
+            const uint32_t d0 = tmem + dbuf * d_set + h * rows;
             uint32_t acc = 0u;
-            for (uint32_t i = 0; i < cnt && ok; ++i) {
-                if (!mix_wait(full0 + 8u * s, par, abort_flag)) {
-                    mix_report(a, abort_flag, (2u << 8) | 2u);
+            for (uint32_t i = 0; i < cnt; ++i) {
+                if (!__all_sync(0xffffffffu, ready) && !mix_wait(afull0 + 8u * ab, apar, abort_flag)) {
+                    mix_report(a, abort_flag, (2u << 8) | 3u);
                     ok = false;
                     break;
                 }
+                const uint32_t a0 = tmem + kMixACol + ab * 64u, freed = aempty0 + 8u * ab;
+                ab ^= 2u;
+                if (ab == h) apar ^= 1u;
+                ready = mix_test(afull0 + 8u * ab, apar);
+                ptx::tc_fence_after();
+                if (ptx::elect_one()) {
+                    const uint32_t bl = b_lo + ((s * stage_bytes) >> 4);
 #pragma unroll
-                for (int un = 0; un < 2; ++un) {
-                    if (!mix_wait(afull0 + 8u * ab, apar, abort_flag)) {
-                        mix_report(a, abort_flag, (2u << 8) | 3u);
-                        ok = false;
-                        break;
-                    }
-                    ptx::tc_fence_after();
-                    if (ptx::elect_one()) {
-                        const uint32_t bl = b_lo + ((s * stage_bytes + un * xunit) >> 4);
-                        const uint32_t a0 = tmem + kMixACol + ab * 64u;
-#pragma unroll
-                        for (int kk = 0; kk < 4; ++kk) {
-                            uint32_t d = d0;
-                            if (kSum == MixSum::kCopies) d += (kk == 0 ? 0u : (kk == 1 ? turn1 : (kk == 2 ? turn2 : turn3))) + (un == 1 && copies == 8u ? 4u * d_one : 0u);
-#pragma unroll
-                            for (int h = 0; h < 2; ++h)
-                                umma_f16_ta(d + h * rows, a0 + h * 32 + kk * 8, b_hi | (uint64_t)(bl + 2u * kk), idesc,
-                                            kk == 0 || kSum == MixSum::kCopies ? acc : 1u);
+                    for (int kk = 0; kk < 8; ++kk) {
+                        uint32_t d = d0, go_on = kk == 0 ? acc : 1u;
+                        if (kSum == MixSum::kCopies) {
+                            d += (kk & 3) == 0 ? 0u : ((kk & 3) == 1 ? turn1 : ((kk & 3) == 2 ? turn2 : turn3));
+                            if (kk >= 4) d += copies == 8u ? 4u * d_one : 0u;
+                            go_on = kk < 4 || copies == 8u ? acc : 1u;
                         }
-                        ptx::umma_commit_a(aempty0 + 8u * ab);
-                        if (un == 1) ptx::umma_commit_a(empty0 + 8u * s);
+                        umma_f16_ta(d, a0 + kk * 8, b_hi | (uint64_t)(bl + (kk >= 4 ? xunit >> 4 : 0u) + 2u * (kk & 3)), idesc, go_on);
                     }
-                    __syncwarp();
-                    if (kSum != MixSum::kCopies || un == 1 || copies != 8u) acc = 1u;
-                    if (++ab == kMixABufs) { ab = 0; apar ^= 1u; }
+                    ptx::umma_commit_a(freed);
+                    ptx::umma_commit_a(empty0 + 8u * s);
                 }
-                if (++s == stages) { s = 0; par ^= 1u; }
+                __syncwarp();
+                acc = 1u;
+                if (++s == stages) s = 0;
             }
             if (!ok) break;
             u += cnt;
@@ -578,12 +715,13 @@ wqbmm_mixed_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
     } else if (warp < kMixDqWarps) {
         // ======================= dequantisation =======================
         // Eight warps take the even stages of the CTA's piece, eight the odd ones: one wait, one read of the scales and one release per
-        // 128 rows of k. A stage is two A buffers (64 rows each), so the four buffers alternate between the two groups.
+        // 128 rows of k. A warp fills its lanes of one A buffer a stage (its half), so the four buffers alternate between the two groups.
         const int qd = warp & 3, h = (warp >> 2) & 1;
         const uint32_t grp = (uint32_t)warp >> 3;
         const int g = lane >> 2;
         const uint32_t tlane = (uint32_t)(qd * 32) << 16;
         const int wcol = h * 128 + qd * 32;  // the warp's first column in the tile
+        const uint32_t ab = 2u * grp + h;  // the warp's A buffer, shared with the three other lane quarters
         uint32_t s = grp, par = 0, apar = 0;
         if (s >= stages) { s -= stages; par ^= 1u; }
         bool ok = true;
@@ -593,13 +731,14 @@ wqbmm_mixed_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
         // (n,k) storage: the lane's own scales and offsets, an iteration ahead. The group of a stage is counted along (a division per
         // stage was a tenth of this loop): k0 = first row of the stage, k0_in = its place in group gi.
         uint32_t sc_next[2] = {0, 0}, of_next[2] = {0, 0};
-        uint32_t t = 0, kb = 0, k0_in = 0;
-        int64_t gi = 0, col_at = 0;
+        uint32_t t = 0, kb = 0, k0_in = 0, gi = 0;
+        const uint32_t step_g = 2u * C::kBK / a.group, step_in = 2u * C::kBK - step_g * a.group;
+        int64_t col_at = 0;
         // rows of scales whose groups lie side by side: eight groups in one 16-byte load (a lane's 2-byte loads each drag a sector of their
         // own through L2, as many bytes as the weight itself)
         const bool vec = a.sc_vec != 0;
         uint4 sc_v = make_uint4(0, 0, 0, 0), of_v = sc_v;
-        int64_t have = -1;
+        uint32_t have = 0xFFFFFFFFu;
         uint32_t sel = 0;
         auto pick = [](const uint4& v, uint32_t i) {
             const uint32_t w = (i & 4u) ? ((i & 2u) ? v.w : v.z) : ((i & 2u) ? v.y : v.x);
@@ -609,21 +748,21 @@ wqbmm_mixed_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
             t = unit / a.kb;
             kb = unit - t * a.kb;
             gi = (kb * (uint32_t)C::kBK) / a.group;
-            k0_in = kb * (uint32_t)C::kBK - (uint32_t)gi * a.group;
+            k0_in = kb * (uint32_t)C::kBK - gi * a.group;
             col_at = (int64_t)min((t / (uint32_t)a.t_tiles) * kMixTileN + wcol + lane, a.n - 1u) * a.scale_sn;
-            have = -1;
+            have = 0xFFFFFFFFu;
         };
         auto fetch = [&]() {
             if (vec) {
-                sel = (uint32_t)gi & 7u;
+                sel = gi & 7u;
                 if ((gi >> 3) != have) {
                     have = gi >> 3;
-                    sc_v = __ldg(reinterpret_cast<const uint4*>(reinterpret_cast<const uint16_t*>(a.scale) + col_at + 8 * have));
-                    if (kOff) of_v = __ldg(reinterpret_cast<const uint4*>(reinterpret_cast<const uint16_t*>(a.offset) + col_at + 8 * have));
+                    sc_v = __ldg(reinterpret_cast<const uint4*>(reinterpret_cast<const uint16_t*>(a.scale) + col_at + 8u * have));
+                    if (kOff) of_v = __ldg(reinterpret_cast<const uint4*>(reinterpret_cast<const uint16_t*>(a.offset) + col_at + 8u * have));
                 }
                 return;
             }
-            int64_t at = gi * a.scale_sg + col_at;
+            int64_t at = (int64_t)gi * a.scale_sg + col_at;
             sc_next[0] = __ldg(reinterpret_cast<const uint16_t*>(a.scale) + at);
             if (kOff) of_next[0] = __ldg(reinterpret_cast<const uint16_t*>(a.offset) + at);
             if (two_rows && k0_in + 64u >= a.group && kb * (uint32_t)C::kBK + 64u < a.k) at += a.scale_sg;
@@ -635,7 +774,7 @@ wqbmm_mixed_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
             fetch();
         }
         for (uint32_t u = u_begin + grp; u < u_end; u += 2) {
-            uint32_t sc[4], of[4], sc_n[2], of_n[2];
+            uint32_t sc_n[2], of_n[2];
             if constexpr (kRagged) {
                 while (ragged < u) ragged += a.kb;
             }
@@ -653,8 +792,9 @@ wqbmm_mixed_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
                 if (u + 2 < u_end) {
                     kb += 2;
                     if (kb < a.kb) {
-                        k0_in += 2u * C::kBK;
-                        while (k0_in >= a.group) { k0_in -= a.group; ++gi; }
+                        k0_in += step_in;
+                        gi += step_g;
+                        if (k0_in >= a.group) { k0_in -= a.group; ++gi; }
                     } else {
                         seek(u + 2);
                     }
@@ -667,21 +807,43 @@ wqbmm_mixed_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
                 break;
             }
             const uint32_t base = smem0 + s * stage_bytes;
-            // int4: columns 4g .. 4g + 3; int8: 2g, 2g + 1 of each 16
+            // scales and offsets (or what MixFast makes of them) of the lane's columns: int4 4g .. 4g + 3, 8 bits 2g, 2g + 1 of each 16, or its one
+            uint32_t sc[4], of[4];
+            bool fast = false;
             auto load_scales = [&](uint32_t un) {
-                const uint32_t at = base + a.sc_off + un * (kMixTileN * 4u) + 2u * wcol;
-                const uint32_t p0 = kW == MixW::kInt4 ? at + 8u * g : at + 4u * g, p1 = kW == MixW::kInt4 ? p0 + 4u : p0 + 32u;
+                const uint32_t at = base + a.sc_off + un * (kMixTileN * 4u) + 2u * wcol + (kW == MixW::kInt4 ? 8u * g : 4u * g);
                 uint32_t r0, r1, o0 = 0, o1 = 0;
-                asm volatile("ld.shared.u32 %0, [%1];" : "=r"(r0) : "r"(p0) : "memory");
-                asm volatile("ld.shared.u32 %0, [%1];" : "=r"(r1) : "r"(p1) : "memory");
-                if (kOff) {
-                    asm volatile("ld.shared.u32 %0, [%1];" : "=r"(o0) : "r"(p0 + kMixTileN * 2) : "memory");
-                    asm volatile("ld.shared.u32 %0, [%1];" : "=r"(o1) : "r"(p1 + kMixTileN * 2) : "memory");
+                if (kW == MixW::kInt4) {
+                    asm volatile("ld.shared.v2.u32 {%0, %1}, [%2];" : "=r"(r0), "=r"(r1) : "r"(at) : "memory");
+                    if (kOff) asm volatile("ld.shared.v2.u32 {%0, %1}, [%2];" : "=r"(o0), "=r"(o1) : "r"(at + kMixTileN * 2) : "memory");
+                } else {
+                    asm volatile("ld.shared.u32 %0, [%1];" : "=r"(r0) : "r"(at) : "memory");
+                    asm volatile("ld.shared.u32 %0, [%1];" : "=r"(r1) : "r"(at + 32u) : "memory");
+                    if (kOff) {
+                        asm volatile("ld.shared.u32 %0, [%1];" : "=r"(o0) : "r"(at + kMixTileN * 2) : "memory");
+                        asm volatile("ld.shared.u32 %0, [%1];" : "=r"(o1) : "r"(at + kMixTileN * 2 + 32u) : "memory");
+                    }
+                }
+                if constexpr (F::kHas) {
+                    uint32_t m0, m1, a0, a1;
+                    const bool f0 = F::prepare(r0, 0, 1, m0, a0), f1 = F::prepare(r1, 0, 1, m1, a1);
+                    fast = __all_sync(0xffffffffu, f0 && f1);
+                    if (fast) { r0 = m0; r1 = m1; o0 = a0; o1 = a1; }
                 }
                 sc[0] = prmt(r0, r0, 0x1010); sc[1] = prmt(r0, r0, 0x3232); sc[2] = prmt(r1, r1, 0x1010); sc[3] = prmt(r1, r1, 0x3232);
                 of[0] = prmt(o0, o0, 0x1010); of[1] = prmt(o0, o0, 0x3232); of[2] = prmt(o1, o1, 0x1010); of[3] = prmt(o1, o1, 0x3232);
             };
-            if (!kNK) load_scales(0);
+            auto own_scales = [&](uint32_t un) {
+                sc[0] = sc_n[un];
+                of[0] = of_n[un];
+                if constexpr (F::kHas) {
+                    uint32_t m0, a0;
+                    fast = __all_sync(0xffffffffu, F::prepare(sc[0], 0, 0, m0, a0));
+                    if (fast) { sc[0] = m0; of[0] = a0; }
+                }
+            };
+            if (kNK) own_scales(0);
+            else load_scales(0);
             const int r = lane & 7, j = lane >> 3;
             // (k,n) int4: rows of 128 bytes; matrix j of an ldmatrix = rows 8 j .. of a half of 32, the warp's 16 bytes of the row
             uint32_t w4[4][4];
@@ -689,30 +851,32 @@ wqbmm_mixed_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
                 const uint32_t at = base + (uint32_t)(8 * j + r) * 128u + (uint32_t)(((h * 4 + qd) ^ r) << 4);
 #pragma unroll
                 for (int i = 0; i < 4; ++i) mix_ldsm4_trans(at + i * 32 * 128, w4[i]);
-                if (!two_rows) {  // the packed words and the scale rows of this stage are in registers
-                    __syncwarp();
-                    if (lane == 0) mix_arrive(empty0 + 8u * s);
-                }
+                if (!two_rows) mix_arrive_warp(empty0 + 8u * s, lane);  // the packed words and the scale rows of this stage are in registers
             }
-#pragma unroll
-            for (int un = 0; un < 2; ++un) {
-                const uint32_t ab = 2u * grp + un;
-                if (kNK) {
-                    sc[0] = sc_n[un];
-                    of[0] = of_n[un];
-                } else if (un == 1 && two_rows) {
-                    load_scales(1);
+            const uint32_t abase0 = tmem + kMixACol + ab * 64u + tlane;
+            auto need_buffer = [&]() {  // the MMAs that read this A buffer's previous contents are done
+                if (!mix_wait(aempty0 + 8u * ab, apar ^ 1u, abort_flag)) {
+                    mix_report(a, abort_flag, (3u << 8) | 2u);
+                    ok = false;
                 }
-                bool waited = false;
-                const uint32_t abase = tmem + kMixACol + ab * 64u + h * 32u + tlane;
-                auto need_buffer = [&]() {  // the MMAs that read this A buffer's previous contents are done
-                    if (waited) return;
-                    waited = true;
-                    if (!mix_wait(aempty0 + 8u * ab, apar ^ 1u, abort_flag)) {
-                        mix_report(a, abort_flag, (3u << 8) | 2u);
-                        ok = false;
+                ptx::tc_fence_after();
+            };
+            auto unit = [&](auto fast_c, auto un_c) {  // 64 rows of packed words -> half of the A buffer
+                constexpr bool kFast = decltype(fast_c)::value;
+                constexpr int un = decltype(un_c)::value;
+                const uint32_t abase = abase0 + un * 32u;
+                // one word of four columns, or of one column's four bytes / eight nibbles
+                auto word8 = [&](uint32_t w, int at, uint32_t& o0, uint32_t& o1) {
+                    if constexpr (kFast) {
+                        uint32_t c[2];
+                        F::codes8(w, c);
+                        o0 = F::pair(c[0], sc[at], of[at]);
+                        o1 = kNK ? F::pair(c[1], sc[0], of[0]) : F::pair(c[1], sc[at + 1], of[at + 1]);
+                    } else {
+                        o0 = mix_scale<kBf16, kOff>(mix_exact<kW, kBf16>(kNK ? prmt(w, 0u, 0x4140) : w), sc[at], of[at]);
+                        o1 = kNK ? mix_scale<kBf16, kOff>(mix_exact<kW, kBf16>(prmt(w, 0u, 0x4342)), sc[0], of[0])
+                                 : mix_scale<kBf16, kOff>(mix_exact<kW, kBf16>(w >> 8), sc[at + 1], of[at + 1]);
                     }
-                    ptx::tc_fence_after();
                 };
                 if constexpr (!kNK) {
                     if constexpr (kW == MixW::kInt4) {
@@ -720,11 +884,17 @@ wqbmm_mixed_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
                         for (int half = 0; half < 2; ++half) {
                             uint32_t o[2][8];
 #pragma unroll
-                            for (int i = 0; i < 4; ++i)
+                            for (int i = 0; i < 4; ++i) {
+                                const uint32_t w = w4[2 * un + half][i];
+                                uint32_t c[4];
+                                if constexpr (kFast) F::codes4(w, c);
 #pragma unroll
-                                for (int b = 0; b < 4; ++b)
-                                    o[b >> 1][2 * i + (b & 1)] = mix_scale<kBf16, kOff>(mix_exact<kW, kBf16>(w4[2 * un + half][i] >> (4 * b)), sc[b], of[b]);
-                            need_buffer();
+                                for (int b = 0; b < 4; ++b) {
+                                    if constexpr (kFast) o[b >> 1][2 * i + (b & 1)] = F::pair(c[b], sc[b], of[b]);
+                                    else o[b >> 1][2 * i + (b & 1)] = mix_scale<kBf16, kOff>(mix_exact<kW, kBf16>(w >> (4 * b)), sc[b], of[b]);
+                                }
+                            }
+                            if (un == 0 && half == 0) need_buffer();
                             tmem_st_16x128b_x4(abase + half * 16, o[0]);
                             tmem_st_16x128b_x4(abase + half * 16 + (16u << 16), o[1]);
                         }
@@ -737,10 +907,7 @@ wqbmm_mixed_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
                                 uint32_t w[4], o[8];
                                 mix_ldsm4_trans(box + half * 32 * 128 + (uint32_t)(((2 * qd + cc) ^ r) << 4), w);
 #pragma unroll
-                                for (int i = 0; i < 4; ++i)
-#pragma unroll
-                                    for (int b = 0; b < 2; ++b)
-                                        o[2 * i + b] = mix_scale<kBf16, kOff>(mix_exact<kW, kBf16>(w[i] >> (8 * b)), sc[2 * cc + b], of[2 * cc + b]);
+                                for (int i = 0; i < 4; ++i) word8(w[i], 2 * cc, o[2 * i], o[2 * i + 1]);
                                 if (kW == MixW::kE4m3) {
                                     const uint32_t any = has_nan8(w[0]) | has_nan8(w[1]) | has_nan8(w[2]) | has_nan8(w[3]);
                                     if (any != 0u) {
@@ -752,7 +919,7 @@ wqbmm_mixed_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
                                     }
                                     __syncwarp();
                                 }
-                                need_buffer();
+                                if (un == 0 && half == 0 && cc == 0) need_buffer();
                                 tmem_st_16x128b_x4(abase + half * 16 + ((uint32_t)(16 * cc) << 16), o);
                             }
                         }
@@ -772,11 +939,15 @@ wqbmm_mixed_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
 #pragma unroll
                                 for (int i = 0; i < 2; ++i) {
                                     const uint32_t lo = w[2 * hh + i], hi = lo >> 4;
+                                    uint32_t code[4];
+                                    if constexpr (kFast) F::codes4_nk(lo, code);
 #pragma unroll
-                                    for (int b = 0; b < 4; ++b)  // nibbles 2 b and 2 b + 1: byte b of the word and of the word shifted by four
-                                        o[4 * i + b] = mix_scale<kBf16, kOff>(mix_exact<kW, kBf16>(prmt(lo, hi, (uint32_t)(b | ((4 + b) << 8)))), sc[0], of[0]);
+                                    for (int b = 0; b < 4; ++b) {  // nibbles 2 b and 2 b + 1: byte b of the word and of the word shifted by four
+                                        if constexpr (kFast) o[4 * i + b] = F::pair(code[b], sc[0], of[0]);
+                                        else o[4 * i + b] = mix_scale<kBf16, kOff>(mix_exact<kW, kBf16>(prmt(lo, hi, (uint32_t)(b | ((4 + b) << 8)))), sc[0], of[0]);
+                                    }
                                 }
-                                need_buffer();
+                                if (un == 0 && c == 0 && hh == 0) need_buffer();
                                 tmem_st_32x32b_x8(abase + c * 16 + hh * 8, o);
                             }
                         }
@@ -789,10 +960,7 @@ wqbmm_mixed_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
                             const uint32_t w[4] = {v.x, v.y, v.z, v.w};
                             uint32_t o[8];
 #pragma unroll
-                            for (int i = 0; i < 4; ++i) {
-                                o[2 * i] = mix_scale<kBf16, kOff>(mix_exact<kW, kBf16>(prmt(w[i], 0u, 0x4140)), sc[0], of[0]);
-                                o[2 * i + 1] = mix_scale<kBf16, kOff>(mix_exact<kW, kBf16>(prmt(w[i], 0u, 0x4342)), sc[0], of[0]);
-                            }
+                            for (int i = 0; i < 4; ++i) word8(w[i], 0, o[2 * i], o[2 * i + 1]);
                             if (kW == MixW::kE4m3) {
                                 const uint32_t any = has_nan8(w[0]) | has_nan8(w[1]) | has_nan8(w[2]) | has_nan8(w[3]);
                                 if (any != 0u) {
@@ -804,24 +972,43 @@ wqbmm_mixed_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
                                 }
                                 __syncwarp();
                             }
-                            need_buffer();
+                            if (un == 0 && c == 0) need_buffer();
                             tmem_st_32x32b_x8(abase + c * 8, o);
                         }
                     }
                 }
-                if (!ok) break;
-                if constexpr (kRagged) {
-                    if (u == ragged && k_in_last < 64u * (un + 1)) mix_clear_past(abase, k_in_last > 64u * un ? k_in_last - 64u * un : 0u);
+            };
+            using U0 = std::integral_constant<int, 0>;
+            using U1 = std::integral_constant<int, 1>;
+            using Fast = std::bool_constant<F::kHas>;
+            if (!two_rows) {  // (one branch for the stage)
+                if (fast) {
+                    unit(Fast{}, U0{});
+                    unit(Fast{}, U1{});
+                } else {
+                    unit(std::false_type{}, U0{});
+                    unit(std::false_type{}, U1{});
                 }
-                tmem_st_wait();
-                ptx::tc_fence_before();
-                __syncwarp();
-                if (lane == 0) mix_arrive(afull0 + 8u * ab);
+            } else {  // groups that end inside a stage: scales for each unit
+                if (fast) unit(Fast{}, U0{});
+                else unit(std::false_type{}, U0{});
+                if (kNK) own_scales(1);
+                else load_scales(1);
+                if (fast) unit(Fast{}, U1{});
+                else unit(std::false_type{}, U1{});
             }
             if (!ok) break;
-            if (kNK || kW != MixW::kInt4 || two_rows) {
-                if (lane == 0) mix_arrive(empty0 + 8u * s);  // (every lane's reads lie before the __syncwarp above)
+            if constexpr (kRagged) {
+                if (u == ragged) {
+                    if (k_in_last < 64u) mix_clear_past(abase0, k_in_last);
+                    mix_clear_past(abase0 + 32u, k_in_last > 64u ? k_in_last - 64u : 0u);
+                }
             }
+            tmem_st_wait();
+            ptx::tc_fence_before();
+            mix_arrive_warp(afull0 + 8u * ab, lane);
+            // (the packed words of the other layouts are read on the way)
+            if (kNK || kW != MixW::kInt4 || two_rows) mix_arrive_warp(empty0 + 8u * s, lane);
             apar ^= 1u;
             s += 2u;
             if (s >= stages) { s -= stages; par ^= 1u; }
@@ -866,9 +1053,8 @@ wqbmm_mixed_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
         const int col = qd * 32 + mix_col_of_lane<kW, kNK>(lane);
         const bool leader = warp == kMixDqWarps && lane == 0;
         uint32_t dbuf = 0, dpar = 0, u = u_begin, t = u_begin / a.kb, kb = u_begin - t * a.kb;
-        auto next_set = [&](bool relaxed) {  // waits for an accumulator set; the four warps go on, or leave, together
-            const bool got = relaxed ? __all_sync(0xffffffffu, ptx::mbar_wait_relaxed(&s_bars[2 * kMixMaxStages + 2 * kMixABufs + dbuf], dpar, abort_flag))
-                                     : mix_wait(dfull0 + 8u * dbuf, dpar, abort_flag);
+        auto next_set = [&](bool urgent) {  // waits for an accumulator set; the four warps go on, or leave, together
+            const bool got = urgent ? mix_wait(dfull0 + 8u * dbuf, dpar, abort_flag) : __all_sync(0xffffffffu, mix_wait_asleep(dfull0 + 8u * dbuf, dpar, abort_flag));
             if (!got) mix_report(a, abort_flag, (4u << 8) | 1u);
             const bool ok = mix_all_ok<1, kMixEpWarps * 32>(got);
             ptx::tc_fence_after();
@@ -884,7 +1070,7 @@ wqbmm_mixed_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
         if constexpr (kSum != MixSum::kChunks) {
             while (u + (a.kb - kb) < u_end) {
                 const uint32_t cnt = a.kb - kb;
-                if (!next_set(true)) break;
+                if (!next_set(!two_d)) break;  // (with one set the MMA issuers wait for this)
                 mix_finish<kBf16, 4, kSum == MixSum::kCopies>(a, tmem + tlane + dbuf * d_set, a.copies, d_one, t, cnt, col, qd, lane, 0, leader, &s_last[0], abort_flag);
                 give_back();
                 u += cnt;
@@ -898,7 +1084,7 @@ wqbmm_mixed_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
                 const uint32_t cnt = min(a.kb - kb, u_end - u);
                 const bool mine = u + cnt < u_end;  // the last chunk of the last piece is the dequantising warps'
                 for (uint32_t c = 0; (mine ? c : c + a.chunk) < cnt; c += a.chunk) {
-                    ok = next_set(two_d);  // (with one set the MMA issuer waits for this)
+                    ok = next_set(!two_d);
                     if (!ok) break;
                     mix_promote(tmem + tlane + dbuf * d_set, sum, d_one, c == 0u);
                     give_back();

@@ -105,6 +105,56 @@ def _against_oracle(aclnn, case, kernels):
     assert np.all(np.abs(got[ok] - want[ok]) <= ulp * np.maximum(np.abs(want[ok]), 0.05 * rms) * 1.01)
 
 
+@pytest.mark.parametrize("xdt", ["bfloat16", "float16"])
+@pytest.mark.parametrize("kind,nk", [(kind, nk) for kind in ("int4", "int8", "e4m3") for nk in (False, True)])
+def test_scales_at_the_limit_of_the_short_arithmetic(aclnn, kind, nk, xdt):
+    """Without offset a warp whose 32 columns all have small enough scales takes fewer instructions a weight (below 2^-5, 2^-8 for int8 in
+    fp16, 2^8 for e4m3); the scales here lie just below the limit, at it and far above it, per group and warp, zeros and signs among them."""
+    import torch
+
+    from gpu_util import desc, out_tensor, out_to_np
+
+    np_dt = ml_dtypes.bfloat16 if xdt == "bfloat16" else np.float16
+    limit = 2.0 ** 8 if kind == "e4m3" else (2.0 ** -8 if kind == "int8" and xdt == "float16" else 2.0 ** -5)
+    m, k, n, g = 3, 1024, 288, 128
+    rng = np.random.default_rng(case_seed((kind, nk, xdt)))
+    below = limit * (1 - 2.0 ** (-8 if xdt == "bfloat16" else -11))
+    scale = limit * rng.uniform(0.1, 0.9, (k // g, n))
+    scale[:, 0:32:3] = below
+    scale[:, 1:32:3] = -below
+    scale[1, 2:32:3] = 0
+    scale[0, 50] = limit          # one column of a warp, one group
+    scale[2, 64:96] = 4 * limit   # a whole warp
+    scale[:, 100] = -2 * limit
+    scale[3, 128:160] *= 2.0 ** -6
+    scale = scale.astype(np.float32).astype(np_dt)
+    x = (rng.uniform(-1, 1, (m, k)) / 64).astype(np.float32).astype(np_dt)
+    if kind == "int4":
+        w = rng.integers(-8, 8, (k, n)).astype(np.int8)
+        stored = wqbmm_oracle.pack_int4_words(w.T.copy() if nk else w)
+    elif kind == "int8":
+        w = rng.integers(-128, 128, (k, n)).astype(np.int8)
+        stored = w.T.copy() if nk else w
+    else:
+        codes = rng.integers(0, 256, (k, n)).astype(np.uint8)
+        codes[(codes & 0x7F) == 0x7F] ^= 0x01
+        codes[(codes & 0x78) >= 0x58] &= 0xBF  # below 16: finite products in fp16
+        w = codes.view(ml_dtypes.float8_e4m3fn)
+        stored = w.T.copy() if nk else w
+    d_w = desc(aclnn, stored, strides=(1, stored.shape[1]), shape=(stored.shape[1], stored.shape[0])) if nk else desc(aclnn, stored)
+    d_s = desc(aclnn, scale.T.copy(), strides=(1, scale.shape[0]), shape=scale.shape) if nk else desc(aclnn, scale)
+    want = wqbmm_oracle.weight_quant_batch_matmul(x, w, scale, None, None, g).astype(np.float64)
+    assert np.isfinite(want).all()
+    out = out_tensor((m, n), xdt)
+    aclnn.weight_quant_batch_matmul(desc(aclnn, x), d_w, d_s, aclnn.Tensor((m, n), xdt, out), None, None, g, inner_precise=0)
+    torch.cuda.synchronize()
+    assert aclnn.last_kernel_name() == "wqbmm_mixed", aclnn.last_kernel_name()
+    got = out_to_np(out).astype(np.float64)
+    ulp = 2.0 ** -7 if xdt == "bfloat16" else 2.0 ** -10
+    rms = np.sqrt(np.mean(want ** 2, axis=0, keepdims=True))  # a column's own: its scales set its size
+    assert np.all(np.abs(got - want) <= ulp * np.maximum(np.abs(want), 0.05 * rms) * 1.01)
+
+
 def test_mixed_kernel_replays_from_a_graph(aclnn):
     """Pieces combined through workspace: a replayed launch finds the arrival counts as the launch before it left them."""
     import torch
