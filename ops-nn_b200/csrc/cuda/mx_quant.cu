@@ -8,10 +8,11 @@
 //   e    clamped to [-127, 127]; stored as e8m0 byte e + 127
 //   q    = saturate( round_to_nearest_even( x / 2^e ) ) in the destination format
 //   the scale row is padded to an even count with byte 0 (2^-127) and shaped (.., ceil(k/64), 2)
-// Purely HBM bound. Rows whose length is a multiple of 32 (16-byte aligned) take the streaming kernel: four lanes share a
-// 32-block, each moving 16 bytes in and 8 (4) bytes out, the block maximum combined with two shuffles; anything ragged
+// Purely HBM bound. Rows whose length is a multiple of 32 (16-byte aligned) take the streaming kernel: two lanes share a
+// 32-block, each moving 32 bytes in and 16 (8) bytes out, the block maximum combined with one shuffle; anything ragged
 // takes the one-thread-per-block kernel.
 #include <cstdlib>
+#include <type_traits>
 
 #include "common.cuh"
 
@@ -140,13 +141,13 @@ __global__ void __launch_bounds__(256) mx_quant_kernel(const OpsnnMxQuantParams 
     }
 }
 
-// Largest magnitude of two packed pairs, per half; a NaN loses against a number, as fmaxf has it.
+// Largest magnitude of two packed pairs, per half (its sign means nothing); a NaN loses against a number, as fmaxf has it.
 template <bool kBf16>
 __device__ __forceinline__ uint32_t max_pair(uint32_t a, uint32_t b)
 {
     uint32_t d;
-    if (kBf16) asm("max.bf16x2 %0, %1, %2;" : "=r"(d) : "r"(a), "r"(b));
-    else asm("max.f16x2 %0, %1, %2;" : "=r"(d) : "r"(a), "r"(b));
+    if (kBf16) asm("max.xorsign.abs.bf16x2 %0, %1, %2;" : "=r"(d) : "r"(a), "r"(b));
+    else asm("max.xorsign.abs.f16x2 %0, %1, %2;" : "=r"(d) : "r"(a), "r"(b));
     return d;
 }
 // Two values to the destination type, round to nearest even, saturating (NaN: e4m3 / e5m2 NaN, e2m1 +6); `lo` into the low half.
@@ -162,55 +163,74 @@ __device__ __forceinline__ uint32_t cvt_fp8x2(float lo, float hi)
     return __nv_cvt_float2_to_fp8x2(make_float2(lo, hi), __NV_SATFINITE, kE4m3 ? __NV_E4M3 : __NV_E5M2);
 }
 
-// Streaming form: k % 32 == 0, x and y 16-byte aligned. One lane = 8 consecutive elements; lanes 4j..4j+3 = one block.
-// HBM bound, so: kUnroll loads of 16 bytes in flight per thread (4 where that still leaves every SM several CTAs), the block maximum on
-// packed pairs, the hardware's paired conversions (element by element, e2m1 by comparisons, this was issue bound at 1.3 TB/s, e4m3 at
-// 3.5), no division where the blocks of a row are an even number.
-template <bool kBf16, int kUnroll>
-__global__ void __launch_bounds__(256) mx_quant_stream_kernel(const OpsnnMxQuantParams p, int64_t blocks_per_row, int64_t scale_row)
+// 32 bytes: one load where the address allows it (kWide), else two.
+template <bool kWide>
+__device__ __forceinline__ void load_32(const uint8_t* p, uint32_t (&w)[8])
+{
+    if (kWide) {
+        asm volatile("ld.global.L1::no_allocate.v8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+                     : "=r"(w[0]), "=r"(w[1]), "=r"(w[2]), "=r"(w[3]), "=r"(w[4]), "=r"(w[5]), "=r"(w[6]), "=r"(w[7])
+                     : "l"(p));
+    } else {
+        const uint4 a = __ldcs(reinterpret_cast<const uint4*>(p)), b = __ldcs(reinterpret_cast<const uint4*>(p) + 1);
+        w[0] = a.x; w[1] = a.y; w[2] = a.z; w[3] = a.w; w[4] = b.x; w[5] = b.y; w[6] = b.z; w[7] = b.w;
+    }
+}
+
+// Streaming form: k % 32 == 0, x 16-byte and y 8-byte aligned. One lane = 16 consecutive elements, two lanes = one block.
+// HBM bound if the instructions allow it: integer ones take two clocks a warp, so the type and the golden's usual modes (kPlain: OCP scale,
+// round to nearest even) are template arguments, magnitudes are compared in pairs and without masking, and a lane moves 32 bytes
+// (eight elements a lane and run-time types took about as many instructions for half of the elements). us before / after: 32768 x 7168 to e4m3
+// 128 / 101 (7.0 TB/s), 65536 x 4096 to e2m1 139 / 102 (6.6 TB/s), 30001 x 4128 (129 blocks a row) to e4m3 79.6 / 54.9.
+// kUnroll pieces are in flight per thread (2 where that still leaves every SM several CTAs).
+template <bool kBf16, int32_t kDst, bool kPlain, bool kWide, int kUnroll>
+__global__ void __launch_bounds__(256) mx_quant_stream_kernel(const OpsnnMxQuantParams p, uint32_t blocks_per_row, uint32_t odd, uint32_t div_m, uint32_t div_s)
 {
     pdl_trigger();
     pdl_wait();
-    const int64_t pieces = p.rows * blocks_per_row * 4;  // 8-element pieces
-    const int emax = p.y_dtype == ACL_FLOAT4_E2M1 ? 2 : (p.y_dtype == ACL_FLOAT8_E4M3FN ? 8 : 15);
-    const uint4* src = reinterpret_cast<const uint4*>(p.x);
+    const int64_t pieces = p.rows * (int64_t)blocks_per_row * 2;  // 16-element pieces
+    constexpr int emax = kDst == ACL_FLOAT4_E2M1 ? 2 : (kDst == ACL_FLOAT8_E4M3FN ? 8 : 15);
+    const uint8_t* src = reinterpret_cast<const uint8_t*>(p.x);
     const int64_t i0 = (int64_t)blockIdx.x * (256 * kUnroll) + threadIdx.x;
-    uint4 raw[kUnroll];
+    uint32_t raw[kUnroll][8];
 #pragma unroll
     for (int u = 0; u < kUnroll; ++u) {
         const int64_t i = i0 + u * 256;
-        raw[u] = i < pieces ? __ldcs(src + i) : make_uint4(0u, 0u, 0u, 0u);  // pieces is a multiple of 4: a block's four lanes are live together
+        if (i < pieces) {  // pieces is even: a block's two lanes are live together
+            load_32<kWide>(src + i * 32, raw[u]);
+        } else {
+#pragma unroll
+            for (int c = 0; c < 8; ++c) raw[u][c] = 0u;
+        }
     }
 #pragma unroll
     for (int u = 0; u < kUnroll; ++u) {
         const int64_t i = i0 + u * 256;
-        const uint32_t w[4] = {raw[u].x, raw[u].y, raw[u].z, raw[u].w};
-        constexpr uint32_t kMag = 0x7FFF7FFFu;
-        uint32_t m = max_pair<kBf16>(max_pair<kBf16>(w[0] & kMag, w[1] & kMag), max_pair<kBf16>(w[2] & kMag, w[3] & kMag));
+        const uint32_t (&w)[8] = raw[u];
+        uint32_t m = max_pair<kBf16>(max_pair<kBf16>(max_pair<kBf16>(w[0], w[1]), max_pair<kBf16>(w[2], w[3])),
+                                     max_pair<kBf16>(max_pair<kBf16>(w[4], w[5]), max_pair<kBf16>(w[6], w[7])));
         m = max_pair<kBf16>(m, __shfl_xor_sync(0xffffffffu, m, 1));
-        m = max_pair<kBf16>(m, __shfl_xor_sync(0xffffffffu, m, 2));
-        m = max_pair<kBf16>(m, m >> 16);
-        const float amax = kBf16 ? __uint_as_float(m << 16) : __half2float(__ushort_as_half((unsigned short)(m & 0xFFFFu)));
-        const int e = mx_block_exp(amax, p, emax);
+        m = max_pair<kBf16>(m, m >> 16) & 0x7FFFu;
+        const float amax = kBf16 ? __uint_as_float(m << 16) : __half2float(__ushort_as_half((unsigned short)m));
+        const int e = kPlain ? mx_shared_exp(amax, emax) : mx_block_exp(amax, p, emax);
         if (i >= pieces) continue;
-        const int64_t blk_lin = i >> 2;
-        if ((i & 3) == 0) {
+        if ((i & 1) == 0) {
             const uint8_t byte = e > 127 ? 255 : (uint8_t)(e + 127);
-            uint8_t* sc = reinterpret_cast<uint8_t*>(p.scale);
-            if (scale_row == blocks_per_row) {
-                sc[blk_lin] = byte;
-            } else {  // one padding entry per row makes the count even
-                const int64_t row = blk_lin < (int64_t)0x7FFFFFFF ? (int64_t)((uint32_t)blk_lin / (uint32_t)blocks_per_row) : blk_lin / blocks_per_row;
-                const int64_t blk = blk_lin - row * blocks_per_row;
-                sc[blk_lin + row] = byte;
-                if (blk == blocks_per_row - 1) sc[blk_lin + row + 1] = 0;
+            const int64_t blk = i >> 1;
+            uint8_t* sc = reinterpret_cast<uint8_t*>(p.scale) + blk;
+            if (odd == 0u) {
+                *sc = byte;
+            } else {  // one padding entry per row makes the count even; below 2^31 blocks the row is a multiplication and a shift away
+                const int64_t row = blk < (int64_t)0x7FFFFFFF ? (int64_t)(((uint64_t)(uint32_t)blk * div_m) >> div_s) : blk / (int64_t)blocks_per_row;
+                sc[row] = byte;
+                if (blk - row * (int64_t)blocks_per_row == (int64_t)blocks_per_row - 1) sc[row + 1] = 0;
             }
         }
         // 2^-e; 2^-127 is subnormal: that scale is applied as two exact factors
         const float s0 = e > 127 ? __uint_as_float(0x7FC00000u) : (e == 127 ? __uint_as_float(1u << 23) : __uint_as_float((uint32_t)(127 - e) << 23));
-        float v[8];
+        float v[16];
 #pragma unroll
-        for (int j = 0; j < 4; ++j) {
+        for (int j = 0; j < 8; ++j) {
             if (kBf16) {
                 v[2 * j] = __uint_as_float(w[j] << 16) * s0;
                 v[2 * j + 1] = __uint_as_float(w[j] & 0xFFFF0000u) * s0;
@@ -222,26 +242,47 @@ __global__ void __launch_bounds__(256) mx_quant_stream_kernel(const OpsnnMxQuant
         }
         if (e == 127) {
 #pragma unroll
-            for (int j = 0; j < 8; ++j) v[j] *= 0.5f;
+            for (int j = 0; j < 16; ++j) v[j] *= 0.5f;
         }
-        if (p.y_dtype == ACL_FLOAT4_E2M1) {
-            uint32_t out = 0;
-            if (p.round_mode == 0) {
+        if (kDst == ACL_FLOAT4_E2M1) {
+            uint32_t out[2] = {0, 0};
+            if (kPlain) {
 #pragma unroll
-                for (int j = 0; j < 4; ++j) out |= cvt_e2m1x2(v[2 * j], v[2 * j + 1]) << (8 * j);
+                for (int j = 0; j < 8; ++j) out[j >> 2] |= cvt_e2m1x2(v[2 * j], v[2 * j + 1]) << (8 * (j & 3));
             } else {
 #pragma unroll
-                for (int j = 0; j < 8; ++j) out |= (uint32_t)quant_fp4_e2m1_mode(v[j], p.round_mode) << (4 * j);
+                for (int j = 0; j < 16; ++j) out[j >> 3] |= (uint32_t)quant_fp4_e2m1_mode(v[j], p.round_mode) << (4 * (j & 7));
             }
-            reinterpret_cast<uint32_t*>(p.y)[i] = out;
-        } else if (p.y_dtype == ACL_FLOAT8_E4M3FN) {
-            reinterpret_cast<uint2*>(p.y)[i] = make_uint2(cvt_fp8x2<true>(v[0], v[1]) | (cvt_fp8x2<true>(v[2], v[3]) << 16),
-                                                          cvt_fp8x2<true>(v[4], v[5]) | (cvt_fp8x2<true>(v[6], v[7]) << 16));
+            reinterpret_cast<uint2*>(p.y)[i] = make_uint2(out[0], out[1]);
         } else {
-            reinterpret_cast<uint2*>(p.y)[i] = make_uint2(cvt_fp8x2<false>(v[0], v[1]) | (cvt_fp8x2<false>(v[2], v[3]) << 16),
-                                                          cvt_fp8x2<false>(v[4], v[5]) | (cvt_fp8x2<false>(v[6], v[7]) << 16));
+            constexpr bool kE4m3 = kDst == ACL_FLOAT8_E4M3FN;
+            uint32_t out[4];
+#pragma unroll
+            for (int j = 0; j < 4; ++j) out[j] = cvt_fp8x2<kE4m3>(v[4 * j], v[4 * j + 1]) | (cvt_fp8x2<kE4m3>(v[4 * j + 2], v[4 * j + 3]) << 16);
+            if (kWide) {
+                reinterpret_cast<uint4*>(p.y)[i] = make_uint4(out[0], out[1], out[2], out[3]);
+            } else {
+                reinterpret_cast<uint2*>(p.y)[2 * i] = make_uint2(out[0], out[1]);
+                reinterpret_cast<uint2*>(p.y)[2 * i + 1] = make_uint2(out[2], out[3]);
+            }
         }
     }
+}
+
+template <bool kBf16, int32_t kDst, bool kPlain>
+void launch_stream(const OpsnnMxQuantParams* p, uint32_t blocks_per_row, bool wide, bool many, unsigned grid, cudaStream_t stream)
+{
+    // blk / d for 31-bit blk: (blk * m) >> s with s = 31 + ceil(log2 d), m = floor(2^s / d) + 1 (below 2^32 for every d > 1)
+    uint32_t bits = 0;
+    while ((1ull << bits) < blocks_per_row) ++bits;
+    const uint32_t odd = blocks_per_row & 1u, s = 31u + bits;
+    const uint32_t m = blocks_per_row > 1u ? (uint32_t)((1ull << s) / blocks_per_row + 1u) : 0u;
+    const uint32_t div_m = blocks_per_row > 1u ? m : 1u, div_s = blocks_per_row > 1u ? s : 0u;
+    auto go = [&](auto kern) { launch_dependent(kern, dim3(grid), 256, 0, stream, *p, blocks_per_row, odd, div_m, div_s); };
+    if (wide && many) go(mx_quant_stream_kernel<kBf16, kDst, kPlain, true, 2>);
+    else if (wide) go(mx_quant_stream_kernel<kBf16, kDst, kPlain, true, 1>);
+    else if (many) go(mx_quant_stream_kernel<kBf16, kDst, kPlain, false, 2>);
+    else go(mx_quant_stream_kernel<kBf16, kDst, kPlain, false, 1>);
 }
 
 // Blocks along a non-last axis: x is (rows, k, inner); a thread owns one column i (two adjacent columns for fp4, which packs
@@ -331,18 +372,24 @@ int32_t mx_quant_launch(const OpsnnMxQuantParams* p, cudaStream_t stream)
     const int64_t scale_row = ((blocks_per_row + 1) / 2) * 2;
     const int64_t total = p->rows * scale_row;
     if (total == 0) return 0;
-    const bool stream_ok = p->k % 32 == 0 && (reinterpret_cast<uintptr_t>(p->x) & 15) == 0 && (reinterpret_cast<uintptr_t>(p->y) & 7) == 0 &&
+    const bool stream_ok = p->k % 32 == 0 && blocks_per_row <= 0x7FFFFFFF && (reinterpret_cast<uintptr_t>(p->x) & 15) == 0 && (reinterpret_cast<uintptr_t>(p->y) & 7) == 0 &&
                            env("OPSNN_MXQ_GENERIC") == nullptr;
     if (stream_ok) {
-        const int64_t pieces = p->rows * blocks_per_row * 4;
-        const bool many = pieces >= (int64_t)148 * 8 * 256 * 4;
-        const int64_t per = 256 * (many ? 4 : 1), g2 = (pieces + per - 1) / per;
+        const int64_t pieces = p->rows * blocks_per_row * 2;
+        const bool many = pieces >= (int64_t)148 * 8 * 256 * 2;
+        const int64_t per = 256 * (many ? 2 : 1), g2 = (pieces + per - 1) / per;
         if (g2 > 0x7FFFFFFF) return (int32_t)cudaErrorInvalidConfiguration;
-        const bool bf = p->x_dtype == ACL_BF16;
-        if (bf && many) launch_dependent(mx_quant_stream_kernel<true, 4>, dim3((unsigned)g2), 256, 0, stream, *p, blocks_per_row, scale_row);
-        else if (bf) launch_dependent(mx_quant_stream_kernel<true, 1>, dim3((unsigned)g2), 256, 0, stream, *p, blocks_per_row, scale_row);
-        else if (many) launch_dependent(mx_quant_stream_kernel<false, 4>, dim3((unsigned)g2), 256, 0, stream, *p, blocks_per_row, scale_row);
-        else launch_dependent(mx_quant_stream_kernel<false, 1>, dim3((unsigned)g2), 256, 0, stream, *p, blocks_per_row, scale_row);
+        const bool wide = (reinterpret_cast<uintptr_t>(p->x) & 31) == 0 && (reinterpret_cast<uintptr_t>(p->y) & 15) == 0;
+        const bool f4 = p->y_dtype == ACL_FLOAT4_E2M1, plain = f4 ? p->round_mode == 0 : p->scale_alg != 1;
+        const uint32_t bpr = (uint32_t)blocks_per_row;
+        auto go = [&](auto bf, auto plain_c) {
+            constexpr bool kBf = decltype(bf)::value, kPlain = decltype(plain_c)::value;
+            if (f4) launch_stream<kBf, ACL_FLOAT4_E2M1, kPlain>(p, bpr, wide, many, (unsigned)g2, stream);
+            else if (p->y_dtype == ACL_FLOAT8_E4M3FN) launch_stream<kBf, ACL_FLOAT8_E4M3FN, kPlain>(p, bpr, wide, many, (unsigned)g2, stream);
+            else launch_stream<kBf, ACL_FLOAT8_E5M2, kPlain>(p, bpr, wide, many, (unsigned)g2, stream);
+        };
+        if (p->x_dtype == ACL_BF16) plain ? go(std::true_type{}, std::true_type{}) : go(std::true_type{}, std::false_type{});
+        else plain ? go(std::false_type{}, std::true_type{}) : go(std::false_type{}, std::false_type{});
         note_launch("mx_quant_stream");
         return (int32_t)cudaGetLastError();
     }

@@ -173,6 +173,39 @@ def test_dynamic_mx_quant_streaming_kernel_matches_oracle(aclnn, dst, xdt):
     assert np.array_equal(y.cpu().numpy(), wy_bytes)
 
 
+@pytest.mark.parametrize("shift", [0, 8])  # x 32- / 16-byte, y 16- / 8-byte aligned
+@pytest.mark.parametrize("dst", ["float8_e4m3fn", "float8_e5m2", "float4_e2m1"])
+@pytest.mark.parametrize("rows,k", [(1, 32), (7, 32), (5, 96), (33, 992), (3001, 3232), (2048, 5120)])
+def test_dynamic_mx_quant_streaming_forms_equal_the_general_kernel(aclnn, monkeypatch, rows, k, dst, shift):
+    """Odd and even numbers of blocks a row, one and two pieces a thread, both widths of loads: the bytes of the kernel that takes one block
+    a thread, infinities, NaN, zeros and subnormals among the values."""
+    import torch
+
+    from gpu_util import DEV
+
+    gen = torch.Generator(device=DEV).manual_seed(rows * 7 + k)
+    buf = torch.randn(rows * k + 64, generator=gen, device=DEV).to(torch.bfloat16)
+    at = torch.randint(0, rows * k, (max(8, rows * k // 500),), generator=gen, device=DEV)
+    special = torch.tensor([float("inf"), float("nan"), -float("inf"), 1e30, -1e-39, 0.0, -0.0, 3e38], device=DEV).to(torch.bfloat16)
+    buf[at + shift] = special[at % 8]
+    buf[shift : shift + 32] = 0.0
+    x = buf[shift : shift + rows * k].view(rows, k)
+    nbytes, srow = rows * k // (2 if dst == "float4_e2m1" else 1), -(-k // 64) * 2
+    outs = []
+    for generic in (False, True):
+        if generic:
+            monkeypatch.setenv("OPSNN_MXQ_GENERIC", "1")
+        ybuf = torch.full((nbytes + 64,), 0xAA, dtype=torch.uint8, device=DEV)
+        s = torch.full((rows, srow // 2, 2), 0xAA, dtype=torch.uint8, device=DEV)
+        y = ybuf[shift : shift + nbytes].view(rows, -1)
+        aclnn.dynamic_mx_quant(aclnn.from_torch(x), aclnn.from_torch(y, dst, (rows, k)), aclnn.from_torch(s, "float8_e8m0"), dst)
+        torch.cuda.synchronize()
+        assert aclnn.last_kernel_name() == ("mx_quant" if generic else "mx_quant_stream")
+        assert bool((ybuf[:shift] == 0xAA).all()) and bool((ybuf[shift + nbytes :] == 0xAA).all())
+        outs.append((y.clone(), s))
+    assert torch.equal(outs[0][0], outs[1][0]) and torch.equal(outs[0][1], outs[1][1])
+
+
 MX4_LAYOUT_CASES = [
     # batch, m, k, n, x1 stored (k,m), x2 stored (n,k)
     ((), 128, 256, 160, False, False),     # x2 given as (k,n): rewritten k-contiguous by the pre-pass
