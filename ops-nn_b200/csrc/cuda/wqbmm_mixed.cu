@@ -552,11 +552,13 @@ wqbmm_mixed_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
     const int lane = threadIdx.x & 31;
     extern __shared__ uint8_t dyn_raw[];
     const uint32_t smem0 = (ptx::smem_u32(dyn_raw) + 1023u) & ~1023u;
-    __shared__ __align__(8) uint64_t s_bars[2 * kMixMaxStages + 2 * kMixABufs + 6];
+    // `full` has two barriers a slot, used in turn: so one belongs to one group of dequantising warps, which sees every one of its phases (with an
+    // odd number of slots a group meets a slot in every second phase only, and a parity does not tell a phase from the one two before it)
+    __shared__ __align__(8) uint64_t s_bars[3 * kMixMaxStages + 2 * kMixABufs + 6];
     __shared__ uint32_t s_tmem;
     __shared__ volatile uint32_t s_abort;
     __shared__ volatile uint32_t s_last[2];
-    const uint32_t full0 = ptx::smem_u32(s_bars), empty0 = full0 + 8u * kMixMaxStages;
+    const uint32_t full0 = ptx::smem_u32(s_bars), empty0 = full0 + 16u * kMixMaxStages;
     const uint32_t afull0 = empty0 + 8u * kMixMaxStages, aempty0 = afull0 + 8u * kMixABufs;
     const uint32_t dfull0 = aempty0 + 8u * kMixABufs, dempty0 = dfull0 + 16u, fin0 = dempty0 + 16u, fsum0 = fin0 + 8u;
     volatile uint32_t* abort_flag = &s_abort;
@@ -565,6 +567,7 @@ wqbmm_mixed_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
         s_abort = 0u;
         for (uint32_t i = 0; i < a.stages; ++i) {
             mix_init(full0 + 8u * i, 1u);
+            mix_init(full0 + 8u * (a.stages + i), 1u);
             mix_init(empty0 + 8u * i, kMixDqWarps / 2 + kMixMmaWarps);
         }
         for (int i = 0; i < kMixABufs; ++i) {
@@ -605,7 +608,7 @@ wqbmm_mixed_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
     if (warp == kMixDqWarps + kMixEpWarps) {
         // ======================= TMA producer =======================
         // Its time per stage bounds the stream: no division but one by the group size, everything else counted along.
-        uint32_t s = 0, par = 0;
+        uint32_t s = 0, par = 0, second = 0;  // second: the slot's other barrier
         const uint32_t kbs = a.kb, rows = (uint32_t)a.rows, n_all = a.n, x_off = a.x_off, sc_off = a.sc_off, nrows_sc = a.sc_rows, k_last = a.k - 1u, group = a.group;
         const int64_t scale_sg = a.scale_sg;
         const uint16_t *scale = reinterpret_cast<const uint16_t*>(a.scale), *offset = reinterpret_cast<const uint16_t*>(a.offset);
@@ -621,7 +624,7 @@ wqbmm_mixed_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
                 break;
             }
             if (ptx::elect_one()) {
-                const uint32_t k0 = kb * C::kBK, fb = full0 + 8u * s, dst = smem0 + s * stage_bytes;
+                const uint32_t k0 = kb * C::kBK, fb = full0 + 8u * (s + second), dst = smem0 + s * stage_bytes;
                 const uint32_t sc_bytes = min((uint32_t)kMixTileN, n_all - n0) * 2u;
                 ptx::mbar_expect_tx_a(fb, (uint32_t)C::kWBytes + 2u * xunit + sc_bytes * sc_rows);
                 if (kNK) {
@@ -643,7 +646,7 @@ wqbmm_mixed_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
                 }
             }
             __syncwarp();
-            if (++s == stages) { s = 0; par ^= 1u; }
+            if (++s == stages) { s = 0; par ^= 1u; second ^= stages; }
             if (++kb == kbs) {
                 kb = 0;
                 r0 += rows;
@@ -722,8 +725,7 @@ wqbmm_mixed_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
         const uint32_t tlane = (uint32_t)(qd * 32) << 16;
         const int wcol = h * 128 + qd * 32;  // the warp's first column in the tile
         const uint32_t ab = 2u * grp + h;  // the warp's A buffer, shared with the three other lane quarters
-        uint32_t s = grp, par = 0, apar = 0;
-        if (s >= stages) { s -= stages; par ^= 1u; }
+        uint32_t s = grp, fs = grp, par = 0, apar = 0;  // slot and its barrier (two or more slots)
         bool ok = true;
         const bool two_rows = a.sc_rows == 2u;  // a stage's units have scale rows of their own
         const uint32_t k_in_last = a.k - (a.kb - 1u) * (uint32_t)C::kBK;  // rows of k in a tile's last stage
@@ -801,7 +803,7 @@ wqbmm_mixed_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
                     fetch();
                 }
             }
-            if (!mix_wait(full0 + 8u * s, par, abort_flag)) {
+            if (!mix_wait(full0 + 8u * fs, par, abort_flag)) {
                 mix_report(a, abort_flag, (3u << 8) | 1u);
                 ok = false;
                 break;
@@ -1010,8 +1012,9 @@ wqbmm_mixed_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
             // (the packed words of the other layouts are read on the way)
             if (kNK || kW != MixW::kInt4 || two_rows) mix_arrive_warp(empty0 + 8u * s, lane);
             apar ^= 1u;
-            s += 2u;
-            if (s >= stages) { s -= stages; par ^= 1u; }
+            fs += 2u;
+            if (fs >= 2u * stages) { fs -= 2u * stages; par ^= 1u; }
+            s = fs >= stages ? fs - stages : fs;
         }
         // the CTA's last (often only) piece: nothing is left to dequantise, all sixteen warps finish it
         const uint32_t t_first = u_begin / a.kb, t_last = (u_end - 1u) / a.kb;

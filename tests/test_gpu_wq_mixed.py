@@ -182,6 +182,45 @@ def test_mixed_kernel_replays_from_a_graph(aclnn):
         assert torch.equal(y, want)
 
 
+@pytest.mark.parametrize("kind,nk,m,k,n", [("int8", False, 1100, 4096, 14336), ("int8", True, 1152, 4096, 14336),  # three stages fit, 128 rows
+                                           ("int8", False, 300, 4096, 14336),   # three, 112 rows
+                                           ("int4", False, 96, 8192, 14336),    # five would fit
+                                           ("int4", True, 48, 8192, 14336)])    # seven would fit
+def test_two_groups_of_warps_share_a_ring_of_any_length(aclnn, kind, nk, m, k, n):
+    """Two groups of dequantising warps take the stages in turn. Where the ring has an odd number of slots a group meets a slot in every
+    second phase only and must not take the phase before the missing one for it: every repeat gives the same bits, and the right ones."""
+    import torch
+
+    from gpu_util import DEV
+
+    for seed in range(2):
+        gen = torch.Generator(device=DEV).manual_seed(case_seed((kind, nk, m, k, n, seed)))
+        x = torch.randn((m, k), generator=gen, device=DEV).to(torch.bfloat16)
+        q = torch.randint(-8 if kind == "int4" else -127, 8 if kind == "int4" else 128, (n, k) if nk else (k, n), generator=gen, device=DEV, dtype=torch.int32)
+        if kind == "int4":
+            w = torch.zeros((q.shape[0], q.shape[1] // 8), dtype=torch.int32, device=DEV)
+            for j in range(8):
+                w |= (q[:, j::8] & 0xF) << (4 * j)
+        else:
+            w = q.to(torch.int8)
+        scale = (torch.rand((n, k // 128) if nk else (k // 128, n), generator=gen, device=DEV) * 0.001 + 0.0005).to(torch.bfloat16)
+        if nk:
+            w, q, scale = w.t(), q.t(), scale.t()
+        outs = []
+        for _ in range(6):
+            y = torch.empty((m, n), dtype=torch.bfloat16, device=DEV)
+            aclnn.weight_quant_batch_matmul(*(aclnn.from_torch(t) for t in (x, w, scale, y)), None, None, 128, inner_precise=0)
+            assert aclnn.last_kernel_name() == "wqbmm_mixed"
+            outs.append(y)
+        wd = (q.float() * scale.float().repeat_interleave(128, 0)).to(torch.bfloat16)
+        want = (x.float() @ wd.float()).double()
+        assert all(torch.equal(y, outs[0]) for y in outs[1:])
+        err = (outs[0].double() - want).abs()
+        # one unit in the last place (2^-7), as above: half of one is the rounding of y; the chain of k / 16 = 256 additions that the tensor core
+        # cuts off at 2^-23 of a sum of up to 3 std loses up to 256 * 3 std * 2^-23 = 1e-4 std, a quarter of 2^-7 * 0.05 std
+        assert bool((err <= 2.0 ** -7 * 1.01 * torch.maximum(want.abs(), 0.05 * want.std())).all())
+
+
 SUM_CASES = [
     # weight, stored (n,k), m, k, n: what the streaming kernels took before, in one launch or one per 16 rows
     ("int4", False, 16, 8192, 8192),      # clusters of pieces, accumulators that take turns
