@@ -95,12 +95,12 @@ static bool streaming_asked_for()
 
 // The fused kernel (wqbmm_mixed.cu) reads the packed weight once for up to 128 rows of x and has no mma.sync and no 16-bit image of the
 // weight to pay for, so it is the faster form of nearly every call (bf16, groups of 128 with offset, graph replay, us, before -> fused):
-//   m 1   4096 x 4096 12.1 -> 9.05     m 16  8192 x 28672 49.3 -> 39.7     m 16 int8 4096 x 14336 20.2 -> 17.2
+//   m 1   4096 x 4096 12.1 -> 8.8      m 16  8192 x 28672 49.3 -> 37.4     m 16 int8 4096 x 14336 20.2 -> 17.2
 //   m 32  8192 x 28672 98 -> 40        m 128 8192 x 28672 285 -> 59        m 512 8192 x 28672 416 -> 233
 // It does not take: innerPrecise = 1 (the group-wise arithmetic of the streaming kernels), outputs bound to a communicator (only the
 // streaming kernels store into the peers), a FRACTAL_NZ weight, and m > 1152, where dequantising the weight
 // once per 128 rows costs more than a pass over HBM (against pre-pass and matmul, us: m 1100 8192 x 28672 int4 514 / 578, 4096^2 40 / 53;
-// m 1280 610 / 597, 52 / 54, int8 4096 x 14336 169 / 160).
+// m 1280 610 / 597, 52 / 54, int8 4096 x 14336 159 / 160; m 2048 963 / 902, 4096^2 70 / 67).
 // A weight prepared for the matmul has no pre-pass to save: up to 128 rows the packed weight is still the smaller stream from 2^24 weights
 // on (us, fused / prepared image: m 32 8192 x 28672 int4 42 / 83, 4096 x 14336 17 / 31; m 128 57 / 88, 21 / 32, int8 70 / 92, 4096^2 14.7 / 16.2;
 // m 256 123 / 110, 31.1 / 30.6; m 1024 463 / 340; 1024 x 4096 at m 64 10 / 6.8).
