@@ -9,7 +9,7 @@
 // the tensor core's work shrinks with m while the dequantisation - what bounds this kernel - is done once whatever m is.
 //   CTA tile: 256 weight columns (two M = 128 accumulators) x N rows of x; persistent, one CTA per SM (all 512 TMEM columns).
 //   The (tile, k stage of 128 rows) pairs lie in one line, and every CTA has a contiguous piece of it (mix_plan):
-//     a tile into `split` equal pieces, launched as a cluster: every CTA sums a slice of the tile out of the cluster's shared memory; or
+//     a tile into `split` equal pieces, launched as a cluster: every CTA sums the rows of the tile that the cluster's CTAs send it (mix_push); or
 //     stream-k, all CTAs the same share: a tile that several CTAs share is combined through workspace by whichever arrives last.
 //   Pieces are added in the order of k either way (deterministic; in the second nobody waits for anybody).
 //   warps 0-15   dequantise. Warp w serves TMEM lanes 32 (w % 4) .. (a hardware rule), accumulator half (w / 4) % 2, and every other
@@ -435,6 +435,9 @@ __device__ __forceinline__ void mix_finish(const MixArgs& a, uint32_t acc, uint3
     const uint32_t n0 = tn * kMixTileN + col;
     const bool whole = cnt == a.kb;
     const uint32_t slot = (rows / 2) * 128u, row = (uint32_t)(qd * 32 + lane);
+    unsigned long long* const cnt_p = a.count + t;
+    unsigned long long cur = 0ull;
+    if (leader && !whole) cur = *reinterpret_cast<volatile unsigned long long*>(cnt_p);  // (a guess, here while the sums are parked)
     float4* mine = a.part + (2u * blockIdx.x + (t == mix_begin(a, blockIdx.x) / a.kb ? 0u : 1u)) * slot + row;
 #pragma unroll 1
     for (uint32_t hc = 16u * share; hc < 2u * rows; hc += kStep) {
@@ -450,11 +453,10 @@ __device__ __forceinline__ void mix_finish(const MixArgs& a, uint32_t acc, uint3
     }
     if (whole) return;
     const uint32_t c0 = mix_owner(a, t * a.kb), c1 = mix_owner(a, (t + 1u) * a.kb - 1u);  // the CTAs whose pieces meet this tile
-    __threadfence();
-    asm volatile("bar.sync %0, %1;" ::"n"(kBar), "n"(kWarps * 32) : "memory");  // all of this CTA's partial sums are written and fenced
+    asm volatile("bar.sync %0, %1;" ::"n"(kBar), "n"(kWarps * 32) : "memory");  // all of this CTA's partial sums are written
     if (leader) {
-        unsigned long long* cnt_p = a.count + t;
-        unsigned long long cur = *reinterpret_cast<volatile unsigned long long*>(cnt_p), want = 0ull;
+        __threadfence();  // for all of them: the barrier puts them before it
+        unsigned long long want = 0ull;
         bool done = false;
         for (int it = 0; it < 4096 && !done; ++it) {  // at most c1 - c0 other CTAs can get in between
             want = ((cur >> 8) == a.nonce) ? cur + 1ull : ((a.nonce << 8) | 1ull);
@@ -465,11 +467,11 @@ __device__ __forceinline__ void mix_finish(const MixArgs& a, uint32_t acc, uint3
         if (!done) mix_report(a, abort_flag, (4u << 8) | 2u);
         const bool last = done && (uint32_t)(want & 0xFFull) == c1 - c0 + 1u;
         if (last) *reinterpret_cast<volatile unsigned long long*>(cnt_p) = 0ull;  // a replay of this launch starts clean
+        __threadfence();
         *s_last = last ? 1u : 0u;
     }
     asm volatile("bar.sync %0, %1;" ::"n"(kBar), "n"(kWarps * 32) : "memory");
     if (*s_last == 0u) return;
-    __threadfence();
 #pragma unroll 1
     for (uint32_t hc = 16u * share; hc < 2u * rows; hc += kStep) {
         float f[16];
@@ -493,56 +495,65 @@ __device__ __forceinline__ void mix_finish(const MixArgs& a, uint32_t acc, uint3
     }
 }
 
-// A CTA's sums of its piece, from tensor memory into shared memory as [row of x][256 columns] fp32 (sixteen warps).
+// A tile that is `split` whole pieces. Its live rows of x, four at a time, are dealt to the CTAs, mix_share fours each in order of rank; every CTA
+// stores its sums of them in their owner's shared memory, [piece][four of the share][256 columns][4 rows] fp32 in the place of the stages (at
+// most 180 KB, 12 KB less than the stages of any form), and the owner adds the pieces up. Bound by latency: two cluster barriers, a
+// remote store, and code that runs once. Pulled instead, out of the others' memory between two barriers, with their abort flags and the bias
+// read on the way: 4 x 4096 x 14336 int8 (n,k) fp16 16.37 -> 15.52 us, 4 x 11776 x 8192 int4 with offset 20.18 -> 19.09, 1 x 4096 x 4096 8.43 ->
+// 8.27 (graph replay, weights from HBM). Sent row by row, a thread's rows lying apart: 16.01, 19.97, 8.01, and 77 x 7168 x 18432 2 % more.
+__device__ __forceinline__ uint32_t mix_share(uint32_t live, uint32_t split) { return ((live + 3u) / 4u + split - 1u) / split; }
+constexpr uint32_t kMixFourBytes = kMixTileN * 16u;
+
+// This CTA's sums (sixteen warps) to their owners.
 template <bool kMany>
-__device__ __forceinline__ void mix_park(const MixArgs& a, uint32_t acc, uint32_t n_acc, uint32_t step, uint32_t smem, int col, int share)
+__device__ __forceinline__ void mix_push(const MixArgs& a, uint32_t acc, uint32_t n_acc, uint32_t step, uint32_t smem, uint32_t live, uint32_t rank, int col, int share)
 {
-    const uint32_t rows = (uint32_t)a.rows;
+    const uint32_t rows = (uint32_t)a.rows, per = mix_share(live, a.split);
 #pragma unroll 1
     for (uint32_t hc = 16u * share; hc < 2u * rows; hc += 64u) {
+        const uint32_t h = hc >= rows ? 1u : 0u, r0 = hc - h * rows;
+        if (r0 >= live) continue;
         float f[16];
         mix_sums16<kMany>(acc + hc, n_acc, step, f);
-        const uint32_t h = hc >= rows ? 1u : 0u;
-        const uint32_t at = smem + (hc - h * rows) * (kMixTileN * 4u) + (128u * h + (uint32_t)col) * 4u;
+        uint32_t owner = r0 / 4u / per, four = r0 / 4u - owner * per;
+        const uint32_t mine = smem + rank * per * kMixFourBytes + (128u * h + (uint32_t)col) * 16u;
 #pragma unroll
-        for (uint32_t i = 0; i < 16; ++i) asm volatile("st.shared.f32 [%0], %1;" ::"r"(at + i * (kMixTileN * 4u)), "f"(f[i]) : "memory");
+        for (uint32_t i = 0; i < 16; i += 4) {
+            if (r0 + i >= live) break;
+            uint32_t to;
+            asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(to) : "r"(mine), "r"(owner));
+            asm volatile("st.shared::cluster.v4.f32 [%0], {%1, %2, %3, %4};" ::"r"(to + four * kMixFourBytes), "f"(f[i]), "f"(f[i + 1]), "f"(f[i + 2]), "f"(f[i + 3])
+                         : "memory");
+            if (++four == per) { four = 0; ++owner; }
+        }
     }
 }
 
-// This CTA's slice of tile t: parked sums of the tile's `split` pieces added in piece order, + bias, stored (512 threads, 4 columns each).
+// This CTA's share of tile t: the pieces added in their order, + bias, stored (512 threads, one column of four rows each).
 template <bool kBf16>
-__device__ __forceinline__ void mix_sum_and_store(const MixArgs& a, uint32_t smem, uint32_t t, uint32_t rank, uint32_t tid)
+__device__ __forceinline__ void mix_sum_and_store(const MixArgs& a, uint32_t smem, uint32_t t, uint32_t live, uint32_t rank, uint32_t tid, float bias)
 {
-    const uint32_t rows = (uint32_t)a.rows, tn = t / (uint32_t)a.t_tiles, tt = t - tn * (uint32_t)a.t_tiles;
-    const uint32_t live = min(rows, (uint32_t)a.m - tt * rows), total = live * (kMixTileN / 4);
-    const uint32_t end = total * (rank + 1u) / a.split;
-    for (uint32_t i = total * rank / a.split + tid; i < end; i += kMixDqWarps * 32) {
-        const uint32_t row = i / (kMixTileN / 4), n = tn * kMixTileN + (i % (kMixTileN / 4)) * 4u;
-        if (n >= a.n) continue;
-        float4 f = make_float4(0.f, 0.f, 0.f, 0.f);
-#pragma unroll 4
-        for (uint32_t j = 0; j < a.split; ++j) {
-            uint32_t at = smem + i * 16u;
-            float4 q;
-            if (a.split > 1u) asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(at) : "r"(smem + i * 16u), "r"(j));
-            asm volatile("ld.shared::cluster.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(q.x), "=f"(q.y), "=f"(q.z), "=f"(q.w) : "r"(at) : "memory");
-            f.x += q.x; f.y += q.y; f.z += q.z; f.w += q.w;
+    const uint32_t tn = t / (uint32_t)a.t_tiles, tt = t - tn * (uint32_t)a.t_tiles;
+    const uint32_t per = mix_share(live, a.split), n = tn * kMixTileN + tid % kMixTileN;
+    if (n >= a.n) return;
+    const bool biased = a.bias != nullptr;
+    uint16_t* out = reinterpret_cast<uint16_t*>(a.y) + (int64_t)(tt * (uint32_t)a.rows) * a.y_ld + n;
+#pragma unroll 1
+    for (uint32_t four = tid / kMixTileN; four < per; four += kMixDqWarps * 32 / kMixTileN) {
+        const uint32_t row = (rank * per + four) * 4u;
+        float v[4] = {0.f, 0.f, 0.f, 0.f};
+        uint32_t at = smem + four * kMixFourBytes + tid % kMixTileN * 16u;
+#pragma unroll 2
+        for (uint32_t j = 0; j < a.split; ++j, at += per * kMixFourBytes) {
+            const uint4 q = mix_lds128(at);
+            v[0] += __uint_as_float(q.x); v[1] += __uint_as_float(q.y); v[2] += __uint_as_float(q.z); v[3] += __uint_as_float(q.w);
         }
-        float v[4] = {f.x, f.y, f.z, f.w};
-        uint16_t o[4];
-        uint16_t* y = reinterpret_cast<uint16_t*>(a.y) + (int64_t)(tt * rows + row) * a.y_ld + n;
-        const uint32_t cols = min(4u, a.n - n);
+        uint16_t* y = out + (int64_t)row * a.y_ld;
 #pragma unroll
-        for (uint32_t c = 0; c < 4; ++c) {
-            if (a.bias != nullptr && c < cols) v[c] = __fadd_rn(v[c], load_as_float(a.bias, n + c, a.bias_dtype));
-            o[c] = kBf16 ? __bfloat16_as_ushort(__float2bfloat16_rn(v[c])) : __half_as_ushort(__float2half_rn(v[c]));
-        }
-        if (cols == 4u && (reinterpret_cast<uintptr_t>(y) & 7) == 0) {
-            *reinterpret_cast<uint2*>(y) = make_uint2((uint32_t)o[0] | ((uint32_t)o[1] << 16), (uint32_t)o[2] | ((uint32_t)o[3] << 16));
-        } else {
-#pragma unroll
-            for (uint32_t c = 0; c < 4; ++c)
-                if (c < cols) y[c] = o[c];
+        for (uint32_t r = 0; r < 4; ++r) {
+            if (row + r >= live) break;
+            const float f = biased ? __fadd_rn(v[r], bias) : v[r];
+            y[(int64_t)r * a.y_ld] = kBf16 ? __bfloat16_as_ushort(__float2bfloat16_rn(f)) : __half_as_ushort(__float2half_rn(f));
         }
     }
 }
@@ -565,6 +576,7 @@ wqbmm_mixed_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
     __shared__ uint32_t s_tmem;
     __shared__ volatile uint32_t s_abort;
     __shared__ volatile uint32_t s_last[2];
+    __shared__ volatile uint32_t s_bad;  // a CTA of the cluster gave up a wait
     const uint32_t full0 = ptx::smem_u32(s_bars), empty0 = full0 + 16u * kMixMaxStages;
     const uint32_t afull0 = empty0 + 8u * kMixMaxStages, aempty0 = afull0 + 8u * kMixABufs;
     const uint32_t dfull0 = aempty0 + 8u * kMixABufs, dempty0 = dfull0 + 16u, fin0 = dempty0 + 16u, fsum0 = fin0 + 8u;
@@ -572,6 +584,7 @@ wqbmm_mixed_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
 
     if (threadIdx.x == 0) {
         s_abort = 0u;
+        s_bad = 0u;
         for (uint32_t i = 0; i < a.stages; ++i) {
             mix_init(full0 + 8u * i, 1u);
             mix_init(full0 + 8u * (a.stages + i), 1u);
@@ -606,6 +619,8 @@ wqbmm_mixed_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
 
     const uint32_t u_begin = mix_begin(a, blockIdx.x), u_end = mix_begin(a, blockIdx.x + 1);
     const uint32_t stages = a.stages, stage_bytes = a.stage_bytes;
+    const uint32_t live = min((uint32_t)a.rows, (uint32_t)a.m - (u_begin / a.kb) % (uint32_t)a.t_tiles * (uint32_t)a.rows);  // rows of x in the first tile
+    float bias = 0.f;  // of the column that this thread serves in mix_sum_and_store
     const uint32_t xunit = (uint32_t)a.rows * 128u;  // bytes of x per 64-row unit of k
     // accumulators: two sets where there is room, beside them the sums of the chunks that are done
     const uint32_t d_one = 2u * (uint32_t)a.rows, d_set = kSum == MixSum::kCopies ? a.copies * d_one : d_one;
@@ -1041,19 +1056,27 @@ wqbmm_mixed_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
             mix_report(a, abort_flag, (3u << 8) | 3u);
             ok = false;
         }
-        if (mix_all_ok<2, kMixDqWarps * 32>(ok)) {
+        constexpr bool kMany = kSum != MixSum::kChain;
+        const uint32_t acc = tmem + tlane + dbuf * d_set;
+        // (with chunks: the last one and the sum of those before it)
+        const uint32_t n_acc = kSum == MixSum::kCopies ? a.copies : (has_sum ? 2u : 1u), step = kSum == MixSum::kCopies ? d_one : tmem + tlane + d_sum - acc;
+        const int col = qd * 32 + mix_col_of_lane<kW, kNK>(lane);
+        if (a.split > 1u) {
+            // Its pieces ran as one thread-block cluster: where every CTA of it is done with its stages, the sums go to their owners. What a CTA that
+            // gave up a wait sends is not used.
             ptx::tc_fence_after();
-            constexpr bool kMany = kSum != MixSum::kChain;
-            const uint32_t acc = tmem + tlane + dbuf * d_set;
-            // (with chunks: the last one and the sum of those before it)
-            const uint32_t n_acc = kSum == MixSum::kCopies ? a.copies : (has_sum ? 2u : 1u), step = kSum == MixSum::kCopies ? d_one : tmem + tlane + d_sum - acc;
-            const int col = qd * 32 + mix_col_of_lane<kW, kNK>(lane);
-            if (a.split != 0) {
-                mix_park<kMany>(a, acc, n_acc, step, smem0, col, warp >> 2);
-                if (a.split == 1) {
-                    asm volatile("bar.sync 2, 512;" ::: "memory");
-                    mix_sum_and_store<kBf16>(a, smem0, t_last, 0u, threadIdx.x);
-                }
+            __syncwarp();
+            ptx::cluster_arrive();
+            if (a.bias != nullptr) bias = load_as_float(a.bias, min(t_last / (uint32_t)a.t_tiles * kMixTileN + threadIdx.x % kMixTileN, a.n - 1u), a.bias_dtype);
+            ptx::cluster_wait();
+            mix_push<kMany>(a, acc, n_acc, step, smem0, live, ptx::cluster_ctarank(), col, warp >> 2);
+        } else if (mix_all_ok<2, kMixDqWarps * 32>(ok)) {
+            ptx::tc_fence_after();
+            if (a.split != 0u) {
+                if (a.bias != nullptr) bias = load_as_float(a.bias, min(t_last / (uint32_t)a.t_tiles * kMixTileN + threadIdx.x % kMixTileN, a.n - 1u), a.bias_dtype);
+                mix_push<kMany>(a, acc, n_acc, step, smem0, live, 0u, col, warp >> 2);
+                asm volatile("bar.sync 2, 512;" ::: "memory");
+                mix_sum_and_store<kBf16>(a, smem0, t_last, live, 0u, threadIdx.x, bias);
             } else {
                 mix_finish<kBf16, 16, kMany>(a, acc, n_acc, step, t_last, last_cnt, col, qd, lane, warp >> 2, threadIdx.x == 0, &s_last[1], abort_flag);
             }
@@ -1112,20 +1135,22 @@ wqbmm_mixed_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
         }
     }
     if (a.split > 1u) {
-        // The tile's pieces ran as one thread-block cluster: every CTA sums a slice of the tile over the cluster's shared memory. A CTA that
-        // gave up a wait still joins both barriers; then nobody writes.
-        ptx::cluster_sync();
-        if (warp < kMixDqWarps) {
-            const uint32_t rank = ptx::cluster_ctarank();
-            uint32_t bad = 0u;
-            if ((uint32_t)lane < a.split) {
-                uint32_t remote;
-                asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(remote) : "r"(ptx::smem_u32(const_cast<uint32_t*>(&s_abort))), "r"((uint32_t)lane));
-                asm volatile("ld.shared::cluster.u32 %0, [%1];" : "=r"(bad) : "r"(remote) : "memory");
-            }
-            if (!__any_sync(0xffffffffu, bad != 0u)) mix_sum_and_store<kBf16>(a, smem0, blockIdx.x / a.split, rank, threadIdx.x);
+        if (warp >= kMixDqWarps) {
+            __syncwarp();
+            ptx::cluster_arrive();
+            ptx::cluster_wait();
         }
-        ptx::cluster_sync();
+        // every warp's waits lie behind it, so the abort flag is final
+        if (threadIdx.x < a.split && *abort_flag != 0u) {
+            uint32_t remote;
+            asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(remote) : "r"(ptx::smem_u32(const_cast<uint32_t*>(&s_bad))), "r"(threadIdx.x));
+            asm volatile("st.shared::cluster.u32 [%0], %1;" ::"r"(remote), "r"(1u) : "memory");
+        }
+        __syncwarp();
+        ptx::cluster_arrive();
+        ptx::cluster_wait();
+        // (nobody reaches into another CTA's shared memory from here on: they leave when they are done)
+        if (warp < kMixDqWarps && s_bad == 0u) mix_sum_and_store<kBf16>(a, smem0, blockIdx.x / a.split, live, ptx::cluster_ctarank(), threadIdx.x, bias);
     }
     // ---- teardown: everyone meets here, also after an aborted wait; then the allocating warp frees TMEM ----
     if (*abort_flag != 0u) __nanosleep(200000);  // lets bulk copies that are still in flight land before the CTA leaves
