@@ -815,7 +815,7 @@ int32_t launch_bn(int bn, const CUtensorMap& ma, const CUtensorMap& mb, UmmaArgs
 // Which of the three forms of the dequant and per-block kernels a call runs on.
 enum class Form { kSingle, kPair, kSplit };
 
-static Form choose_form(const OpsnnQmmParams* p)
+static Form choose_form(const OpsnnQmmParams* p, SplitChoice& split)
 {
     const bool deq = p->mode == OPSNN_QMM_DEQ, pb = p->mode == OPSNN_QMM_PERBLOCK;
     if (!deq && !pb) return Form::kSingle;
@@ -850,10 +850,7 @@ static Form choose_form(const OpsnnQmmParams* p)
         }
     }
     if (split_takes(p) && (split_env == nullptr || atoi(split_env) != 0)) {
-        SplitKernel kern;
-        SplitPlan q;
-        if (split_prepare(p, &kern, &q) == cudaSuccess && q.cost < best) form = Form::kSplit;
-        else cudaGetLastError();
+        if (split.get(p) && split.plan.cost < best) form = Form::kSplit;
     }
     return form;
 }
@@ -897,12 +894,8 @@ uint64_t qmm_umma_workspace_size(const OpsnnQmmParams* p)
 {
     if (p->mode == OPSNN_QMM_MX) return qmm_mx_umma_workspace_size(p);
     if (p->mode == OPSNN_QMM_PERGROUP_ASYM) return (uint64_t)p->m * (uint64_t)((p->k + 255) / 256) * 4u + 256u;  // row sums per k-group
-    if (choose_form(p) == Form::kSplit) {
-        SplitKernel kern;
-        SplitPlan q;
-        if (split_prepare(p, &kern, &q) == cudaSuccess) return split_workspace(q);
-        cudaGetLastError();
-    }
+    SplitChoice split;
+    if (choose_form(p, split) == Form::kSplit && split.get(p)) return split_workspace(split.plan);
     return p->mode == OPSNN_QMM_PERBLOCK ? 0 : ksplit_workspace(p);
 }
 
@@ -978,9 +971,10 @@ int32_t qmm_umma_launch(const OpsnnQmmParams* p, cudaStream_t stream)
 {
     if (const int32_t bad = umma_prelaunch_check()) return bad;
     if (p->mode == OPSNN_QMM_MX) return qmm_mx_umma_launch(p, stream);
-    const Form form = choose_form(p);
+    SplitChoice split;
+    const Form form = choose_form(p, split);
     if (form == Form::kSplit) {
-        const int32_t rc = split_launch(p, stream);
+        const int32_t rc = split_launch(p, split, stream);
         if (rc >= 0) return rc;
     }
     const bool pair = form == Form::kPair && p->mode == OPSNN_QMM_DEQ;

@@ -573,9 +573,10 @@ bool split_takes(const OpsnnQmmParams* p)
 
 // One candidate tile shape (halves; t_tiles row tiles more than needed), cut in the cheapest way. The costs (us) were fitted to fp8 and
 // int8 calls of 16 to 717 rows: launch and ramp, a k-block's fixed part, its tensor work (or promotion) and its share of a stream of
-// weights out of HBM, and the combination, which grows with the tile.
+// weights out of HBM, and the combination, which grows with the tile. `most_cost`: a way that costs as much is of no use, so that the device is not
+// asked about its clusters (asked about all of them, eight candidates of up to sixteen, it took most of a call's 11 - 17 us on the host).
 template <typename F>
-SplitPlan split_candidate(const OpsnnQmmParams* p, uint32_t halves, uint32_t more, int sms, F&& clusters)
+SplitPlan split_candidate(const OpsnnQmmParams* p, uint32_t halves, uint32_t more, int sms, double most_cost, F&& clusters)
 {
     SplitPlan q;
     const bool pb = p->mode == OPSNN_QMM_PERBLOCK;
@@ -596,23 +597,22 @@ SplitPlan split_candidate(const OpsnnQmmParams* p, uint32_t halves, uint32_t mor
     q.stages = (kSplitSmem - 2048 - (pb ? kSplitRing : 0u)) / q.stage_bytes;
     if (q.stages > (uint32_t)kSplitMaxStages) q.stages = kSplitMaxStages;
     const double area = (double)q.rows * halves;
+    q.cost = most_cost;
     auto consider = [&](int64_t grid, uint32_t split, double extra) {
         double w = 0.12 + (pb ? 0.0075 * served : 0.00135 * area);
         const double hbm = (double)grid * halves * kATile / q.t_tiles / 5.8e6;  // all CTAs' weights of one k-block
         if (hbm > w) w = hbm;
         const double cost = 5.5 + (double)((q.units + grid - 1) / grid) * w + extra;
-        if (cost < q.cost) {
-            q.cost = cost;
-            q.grid = grid;
-            q.split = split;
-        }
+        if (cost >= q.cost || (split > 1u && (int64_t)clusters(q, (int)split) < q.tiles)) return;
+        q.cost = cost;
+        q.grid = grid;
+        q.split = split;
     };
     consider(q.units < sms ? q.units : sms, 0, 1.0 + area * 0.05);
     int64_t most = sms / q.tiles;
     if (most > 16) most = 16;
     if (most > q.kb) most = q.kb;
-    for (int s = (int)most; s >= 1; --s)
-        if (s == 1 || (int64_t)clusters(q, s) >= q.tiles) consider(q.tiles * s, (uint32_t)s, s > 1 ? std::max(0.4, 0.6 * s + 0.012 * area - 1.8) : 0.02 * area);
+    for (int s = (int)most; s >= 1; --s) consider(q.tiles * s, (uint32_t)s, s > 1 ? std::max(0.4, 0.6 * s + 0.012 * area - 1.8) : 0.02 * area);
     return q;
 }
 
@@ -647,16 +647,16 @@ cudaError_t split_prepare(const OpsnnQmmParams* p, SplitKernel* kern, SplitPlan*
     int device = -1;
     const bool have_device = cudaGetDevice(&device) == cudaSuccess;
     const int sms = have_device ? sm_count() : 148;
+    const char* only = env("OPSNN_QMM_SPLIT_HALVES");  // experiments
     *plan = SplitPlan{};
     for (uint32_t c = 0; c < 8; ++c) {
         const uint32_t halves = 2u - (c & 1u);
-        const SplitPlan q = split_candidate(p, halves, c >> 1, sms, [&](const SplitPlan& c, int s) -> int {
+        if (only != nullptr && atoi(only) != (int)halves) continue;
+        const SplitPlan q = split_candidate(p, halves, c >> 1, sms, plan->cost, [&](const SplitPlan& c, int s) -> int {
             const SplitKernel k = have_device ? split_kernel(i8, pb, c) : nullptr;
             return k == nullptr ? 0 : max_active_clusters(reinterpret_cast<const void*>(k), kSplitThreads, kSplitSmem, s, 0);
         });
-        if (const char* e = env("OPSNN_QMM_SPLIT_HALVES"))  // experiments
-            if (atoi(e) != (int)halves) continue;
-        if (q.cost < plan->cost) *plan = q;
+        if (q.grid != 0 && q.cost < plan->cost) *plan = q;
     }
     if (plan->grid == 0) return cudaErrorNotSupported;
     *kern = nullptr;
@@ -672,15 +672,27 @@ uint64_t split_workspace(const SplitPlan& q)
     return 256u + counters + 2u * (uint64_t)q.grid * q.rows * 128u * q.halves * 4u;
 }
 
-// 0: launched (or a CUDA error); -1: not this kernel's call.
-int32_t split_launch(const OpsnnQmmParams* p, cudaStream_t stream)
-{
-    SplitKernel kern;
-    SplitPlan q;
-    if (split_prepare(p, &kern, &q) != cudaSuccess) {
-        cudaGetLastError();
-        return -1;
+// A call's kernel and plan, made once by whoever asks first.
+struct SplitChoice {
+    SplitKernel kern = nullptr;
+    SplitPlan plan;
+    int known = 0;  // 1: they are there, -1: there are none
+    bool get(const OpsnnQmmParams* p)
+    {
+        if (known == 0) {
+            known = split_prepare(p, &kern, &plan) == cudaSuccess ? 1 : -1;
+            if (known < 0) cudaGetLastError();
+        }
+        return known > 0;
     }
+};
+
+// 0: launched (or a CUDA error); -1: not this kernel's call.
+int32_t split_launch(const OpsnnQmmParams* p, SplitChoice& choice, cudaStream_t stream)
+{
+    if (!choice.get(p)) return -1;
+    const SplitKernel kern = choice.kern;
+    const SplitPlan& q = choice.plan;
     if (q.split == 0 && (p->workspace == nullptr || p->workspace_size < split_workspace(q))) return -1;
     const bool pb = p->mode == OPSNN_QMM_PERBLOCK;
     SplitArgs a{};
