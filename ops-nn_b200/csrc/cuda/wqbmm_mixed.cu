@@ -495,64 +495,63 @@ __device__ __forceinline__ void mix_finish(const MixArgs& a, uint32_t acc, uint3
     }
 }
 
-// A tile that is `split` whole pieces. Its live rows of x, four at a time, are dealt to the CTAs, mix_share fours each in order of rank; every CTA
-// stores its sums of them in their owner's shared memory, [piece][four of the share][256 columns][4 rows] fp32 in the place of the stages (at
-// most 180 KB, 12 KB less than the stages of any form), and the owner adds the pieces up. Bound by latency: two cluster barriers, a
-// remote store, and code that runs once. Pulled instead, out of the others' memory between two barriers, with their abort flags and the bias
-// read on the way: 4 x 4096 x 14336 int8 (n,k) fp16 16.37 -> 15.52 us, 4 x 11776 x 8192 int4 with offset 20.18 -> 19.09, 1 x 4096 x 4096 8.43 ->
-// 8.27 (graph replay, weights from HBM). Sent row by row, a thread's rows lying apart: 16.01, 19.97, 8.01, and 77 x 7168 x 18432 2 % more.
-__device__ __forceinline__ uint32_t mix_share(uint32_t live, uint32_t split) { return ((live + 3u) / 4u + split - 1u) / split; }
-constexpr uint32_t kMixFourBytes = kMixTileN * 16u;
+// A tile that is `split` whole pieces is dealt to the CTAs in parts of four live rows x 64 columns, mix_share parts each in order of rank; every CTA
+// stores its sums of them in their owner's shared memory, [piece][part of the share][64 columns][4 rows] fp32 in the place of the stages (at
+// most 143 KB, less than the stages of any form), and the owner adds the pieces up. Bound by latency: two cluster barriers, a remote store, and
+// code that runs once and so is fetched while everybody waits for it: fewer instructions here are microseconds. us, graph replay, weights from
+// HBM, before (sums, abort flags and bias fetched out of the others' memory and HBM between two barriers) / dealt as four rows of all columns, a
+// piece alone stored through shared memory too / now: 1 x 4096 x 4096 8.45 / 8.28 / 7.99, 4 x 4096 x 14336 int8 (n,k) fp16 16.3 / 15.5 / 15.2,
+// 4 x 11776 x 8192 with bias 20.2 / 19.1 / 19.2, 6 x 3072 x 1728 int8 7.63 / 7.68 / 6.83, 21 x 1792 x 25440 (n,k) 16.2 / 15.3 / 14.7, 173 x 1280 x 17184
+// (n,k) 14.1 / 14.1 / 11.9. (Sent row by row 77 x 7168 x 18432 lost 2 %.)
+__device__ __forceinline__ uint32_t mix_parts(uint32_t live) { return (live + 3u) / 4u * (kMixTileN / 64); }
+__device__ __forceinline__ uint32_t mix_share(uint32_t live, uint32_t split) { return (mix_parts(live) + split - 1u) / split; }
+constexpr uint32_t kMixPartBytes = 64u * 16u;
 
 // This CTA's sums (sixteen warps) to their owners.
 template <bool kMany>
 __device__ __forceinline__ void mix_push(const MixArgs& a, uint32_t acc, uint32_t n_acc, uint32_t step, uint32_t smem, uint32_t live, uint32_t rank, int col, int share)
 {
-    const uint32_t rows = (uint32_t)a.rows, per = mix_share(live, a.split);
+    const uint32_t rows = (uint32_t)a.rows, per = mix_share(live, a.split), inverse = 65535u / per + 1u;  // part * per < 2^16: the quotient is exact
+    const uint32_t mine = smem + rank * per * kMixPartBytes + ((uint32_t)col & 63u) * 16u;
 #pragma unroll 1
     for (uint32_t hc = 16u * share; hc < 2u * rows; hc += 64u) {
         const uint32_t h = hc >= rows ? 1u : 0u, r0 = hc - h * rows;
         if (r0 >= live) continue;
         float f[16];
         mix_sums16<kMany>(acc + hc, n_acc, step, f);
-        uint32_t owner = r0 / 4u / per, four = r0 / 4u - owner * per;
-        const uint32_t mine = smem + rank * per * kMixFourBytes + (128u * h + (uint32_t)col) * 16u;
 #pragma unroll
         for (uint32_t i = 0; i < 16; i += 4) {
             if (r0 + i >= live) break;
+            const uint32_t part = r0 + i + 2u * h + ((uint32_t)col >> 6), owner = part * inverse >> 16;
             uint32_t to;
-            asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(to) : "r"(mine), "r"(owner));
-            asm volatile("st.shared::cluster.v4.f32 [%0], {%1, %2, %3, %4};" ::"r"(to + four * kMixFourBytes), "f"(f[i]), "f"(f[i + 1]), "f"(f[i + 2]), "f"(f[i + 3])
-                         : "memory");
-            if (++four == per) { four = 0; ++owner; }
+            asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(to) : "r"(mine + (part - owner * per) * kMixPartBytes), "r"(owner));
+            asm volatile("st.shared::cluster.v4.f32 [%0], {%1, %2, %3, %4};" ::"r"(to), "f"(f[i]), "f"(f[i + 1]), "f"(f[i + 2]), "f"(f[i + 3]) : "memory");
         }
     }
 }
 
-// This CTA's share of tile t: the pieces added in their order, + bias, stored (512 threads, one column of four rows each).
+// This CTA's share of tile t: the pieces added in their order, + bias (s_bias: the tile's columns), stored (512 threads, one column of four rows each).
 template <bool kBf16>
-__device__ __forceinline__ void mix_sum_and_store(const MixArgs& a, uint32_t smem, uint32_t t, uint32_t live, uint32_t rank, uint32_t tid, float bias)
+__device__ __forceinline__ void mix_sum_and_store(const MixArgs& a, uint32_t smem, uint32_t t, uint32_t live, uint32_t rank, uint32_t tid, const float* s_bias)
 {
-    const uint32_t tn = t / (uint32_t)a.t_tiles, tt = t - tn * (uint32_t)a.t_tiles;
-    const uint32_t per = mix_share(live, a.split), n = tn * kMixTileN + tid % kMixTileN;
-    if (n >= a.n) return;
-    const bool biased = a.bias != nullptr;
-    uint16_t* out = reinterpret_cast<uint16_t*>(a.y) + (int64_t)(tt * (uint32_t)a.rows) * a.y_ld + n;
+    const uint32_t tn = t / (uint32_t)a.t_tiles, tt = t - tn * (uint32_t)a.t_tiles, per = mix_share(live, a.split), parts = mix_parts(live);
+    uint16_t* out = reinterpret_cast<uint16_t*>(a.y) + (int64_t)(tt * (uint32_t)a.rows) * a.y_ld;
 #pragma unroll 1
-    for (uint32_t four = tid / kMixTileN; four < per; four += kMixDqWarps * 32 / kMixTileN) {
-        const uint32_t row = (rank * per + four) * 4u;
+    for (uint32_t slot = tid / 64u; slot < per; slot += kMixDqWarps * 32 / 64) {
+        const uint32_t part = rank * per + slot, row = part & ~3u, n = tn * kMixTileN + (part & 3u) * 64u + tid % 64u;
+        if (part >= parts || n >= a.n) continue;
         float v[4] = {0.f, 0.f, 0.f, 0.f};
-        uint32_t at = smem + four * kMixFourBytes + tid % kMixTileN * 16u;
+        uint32_t at = smem + slot * kMixPartBytes + tid % 64u * 16u;
 #pragma unroll 2
-        for (uint32_t j = 0; j < a.split; ++j, at += per * kMixFourBytes) {
+        for (uint32_t j = 0; j < a.split; ++j, at += per * kMixPartBytes) {
             const uint4 q = mix_lds128(at);
             v[0] += __uint_as_float(q.x); v[1] += __uint_as_float(q.y); v[2] += __uint_as_float(q.z); v[3] += __uint_as_float(q.w);
         }
-        uint16_t* y = out + (int64_t)row * a.y_ld;
+        uint16_t* y = out + (int64_t)row * a.y_ld + n;
 #pragma unroll
         for (uint32_t r = 0; r < 4; ++r) {
             if (row + r >= live) break;
-            const float f = biased ? __fadd_rn(v[r], bias) : v[r];
+            const float f = a.bias != nullptr ? __fadd_rn(v[r], s_bias[(part & 3u) * 64u + tid % 64u]) : v[r];
             y[(int64_t)r * a.y_ld] = kBf16 ? __bfloat16_as_ushort(__float2bfloat16_rn(f)) : __half_as_ushort(__float2half_rn(f));
         }
     }
@@ -576,7 +575,8 @@ wqbmm_mixed_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
     __shared__ uint32_t s_tmem;
     __shared__ volatile uint32_t s_abort;
     __shared__ volatile uint32_t s_last[2];
-    __shared__ volatile uint32_t s_bad;  // a CTA of the cluster gave up a wait
+    __shared__ volatile uint32_t s_bad;   // a CTA of the cluster gave up a wait
+    __shared__ float s_bias[kMixTileN];  // of the tile's columns, where its pieces are a cluster
     const uint32_t full0 = ptx::smem_u32(s_bars), empty0 = full0 + 16u * kMixMaxStages;
     const uint32_t afull0 = empty0 + 8u * kMixMaxStages, aempty0 = afull0 + 8u * kMixABufs;
     const uint32_t dfull0 = aempty0 + 8u * kMixABufs, dempty0 = dfull0 + 16u, fin0 = dempty0 + 16u, fsum0 = fin0 + 8u;
@@ -620,7 +620,6 @@ wqbmm_mixed_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
     const uint32_t u_begin = mix_begin(a, blockIdx.x), u_end = mix_begin(a, blockIdx.x + 1);
     const uint32_t stages = a.stages, stage_bytes = a.stage_bytes;
     const uint32_t live = min((uint32_t)a.rows, (uint32_t)a.m - (u_begin / a.kb) % (uint32_t)a.t_tiles * (uint32_t)a.rows);  // rows of x in the first tile
-    float bias = 0.f;  // of the column that this thread serves in mix_sum_and_store
     const uint32_t xunit = (uint32_t)a.rows * 128u;  // bytes of x per 64-row unit of k
     // accumulators: two sets where there is room, beside them the sums of the chunks that are done
     const uint32_t d_one = 2u * (uint32_t)a.rows, d_set = kSum == MixSum::kCopies ? a.copies * d_one : d_one;
@@ -1067,19 +1066,11 @@ wqbmm_mixed_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
             ptx::tc_fence_after();
             __syncwarp();
             ptx::cluster_arrive();
-            if (a.bias != nullptr) bias = load_as_float(a.bias, min(t_last / (uint32_t)a.t_tiles * kMixTileN + threadIdx.x % kMixTileN, a.n - 1u), a.bias_dtype);
             ptx::cluster_wait();
             mix_push<kMany>(a, acc, n_acc, step, smem0, live, ptx::cluster_ctarank(), col, warp >> 2);
         } else if (mix_all_ok<2, kMixDqWarps * 32>(ok)) {
             ptx::tc_fence_after();
-            if (a.split != 0u) {
-                if (a.bias != nullptr) bias = load_as_float(a.bias, min(t_last / (uint32_t)a.t_tiles * kMixTileN + threadIdx.x % kMixTileN, a.n - 1u), a.bias_dtype);
-                mix_push<kMany>(a, acc, n_acc, step, smem0, live, 0u, col, warp >> 2);
-                asm volatile("bar.sync 2, 512;" ::: "memory");
-                mix_sum_and_store<kBf16>(a, smem0, t_last, live, 0u, threadIdx.x, bias);
-            } else {
-                mix_finish<kBf16, 16, kMany>(a, acc, n_acc, step, t_last, last_cnt, col, qd, lane, warp >> 2, threadIdx.x == 0, &s_last[1], abort_flag);
-            }
+            mix_finish<kBf16, 16, kMany>(a, acc, n_acc, step, t_last, last_cnt, col, qd, lane, warp >> 2, threadIdx.x == 0, &s_last[1], abort_flag);
         }
     } else {
         // ======================= epilogue of all but the last piece, beside the main loop; chunks are added up =======================
@@ -1088,6 +1079,10 @@ wqbmm_mixed_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
         const int col = qd * 32 + mix_col_of_lane<kW, kNK>(lane);
         const bool leader = warp == kMixDqWarps && lane == 0;
         uint32_t dbuf = 0, dpar = 0, u = u_begin, t = u_begin / a.kb, kb = u_begin - t * a.kb;
+        if (a.split > 1u && a.bias != nullptr) {  // these warps have the time; read at the end it cost up to 0.6 us, by the dequantising warps 0.1 - 0.2
+            for (uint32_t c = threadIdx.x - kMixDqWarps * 32; c < (uint32_t)kMixTileN; c += kMixEpWarps * 32)
+                s_bias[c] = load_as_float(a.bias, min(t / (uint32_t)a.t_tiles * kMixTileN + c, a.n - 1u), a.bias_dtype);
+        }
         auto next_set = [&](bool urgent) {  // waits for an accumulator set; the four warps go on, or leave, together
             const bool got = urgent ? mix_wait(dfull0 + 8u * dbuf, dpar, abort_flag) : __all_sync(0xffffffffu, mix_wait_asleep(dfull0 + 8u * dbuf, dpar, abort_flag));
             if (!got) mix_report(a, abort_flag, (4u << 8) | 1u);
@@ -1150,7 +1145,7 @@ wqbmm_mixed_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
         ptx::cluster_arrive();
         ptx::cluster_wait();
         // (nobody reaches into another CTA's shared memory from here on: they leave when they are done)
-        if (warp < kMixDqWarps && s_bad == 0u) mix_sum_and_store<kBf16>(a, smem0, blockIdx.x / a.split, live, ptx::cluster_ctarank(), threadIdx.x, bias);
+        if (warp < kMixDqWarps && s_bad == 0u) mix_sum_and_store<kBf16>(a, smem0, blockIdx.x / a.split, live, ptx::cluster_ctarank(), threadIdx.x, s_bias);
     }
     // ---- teardown: everyone meets here, also after an aborted wait; then the allocating warp frees TMEM ----
     if (*abort_flag != 0u) __nanosleep(200000);  // lets bulk copies that are still in flight land before the CTA leaves
