@@ -28,6 +28,7 @@ struct SplitArgs {
     uint32_t* part;                // [2 grid][rows][128 halves] raw 32-bit sums
     unsigned long long* count;     // [tiles] (nonce << 8) | arrivals
     unsigned long long nonce;
+    uint32_t push;       // a cluster's sums are sent to their owners (split_push16), not fetched
     uint32_t test_stop;  // tests of the give-up path only: k-blocks that a CTA's producer copies before it stops; otherwise all
 };
 
@@ -169,6 +170,60 @@ __device__ __forceinline__ void split_sum_and_store(const SplitArgs& a, uint32_t
     }
 }
 
+// The same tile where few rows are left to a CTA (split_launch: `push`). Its live rows of x, four at a time, are dealt to the CTAs, split_share fours
+// each in order of rank; every CTA stores its sums of them in their owner's shared memory, [piece][four of the share][columns][4 rows] in the
+// place of the stages (at least 12 KB less than the stages of any form), and the owner adds the pieces up. Nobody reads another CTA's memory,
+// so there is no second trip for the sums and nobody waits to leave.
+__host__ __device__ __forceinline__ uint32_t split_share(uint32_t live, uint32_t split) { return ((live + 3u) / 4u + split - 1u) / split; }
+
+// 16 rows of this thread's column, from row `row` of the tile on (a multiple of 16), to their owners.
+template <uint32_t kHalves>
+__device__ __forceinline__ void split_push16(uint32_t smem, uint32_t live, uint32_t split, uint32_t rank, uint32_t row, uint32_t col, const uint32_t (&v)[16])
+{
+    constexpr uint32_t kFour = 128u * kHalves * 16u;  // bytes of four rows
+    const uint32_t per = split_share(live, split), mine = smem + rank * per * kFour + col * 16u;
+    uint32_t owner = row / 4u / per, four = row / 4u - owner * per;
+#pragma unroll
+    for (uint32_t i = 0; i < 16; i += 4) {
+        if (row + i >= live) break;
+        uint32_t to;
+        asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(to) : "r"(mine), "r"(owner));
+        asm volatile("st.shared::cluster.v4.u32 [%0], {%1, %2, %3, %4};" ::"r"(to + four * kFour), "r"(v[i]), "r"(v[i + 1]), "r"(v[i + 2]), "r"(v[i + 3]) : "memory");
+        if (++four == per) { four = 0; ++owner; }
+    }
+}
+
+// This CTA's share of a tile: the pieces added in their order and stored (256 threads, one column of four rows each; `c`: the column's scale and
+// bias, `s_sa`: the tile's x1 scales, both fetched during the main loop).
+template <uint32_t kHalves>
+__device__ __forceinline__ void split_sum_fours(const SplitArgs& a, uint32_t smem, const SplitTile& t, uint32_t rank, uint32_t tid, const float* s_sa, const SplitCol& c)
+{
+    constexpr uint32_t kWidth = 128u * kHalves, kFour = kWidth * 16u;
+    const uint32_t split = a.split, per = split_share(t.live, split), n = t.n0 + tid % kWidth;
+    if (n >= a.n) return;
+    const bool is_int = a.is_int != 0;
+    const int64_t base = t.b * a.out_bs + n;
+#pragma unroll 1
+    for (uint32_t four = tid / kWidth; four < per; four += 256u / kWidth) {
+        const uint32_t row = (rank * per + four) * 4u;
+        uint32_t at = smem + four * kFour + tid % kWidth * 16u;
+        uint32_t v[4];
+#pragma unroll 2
+        for (uint32_t j = 0; j < split; ++j, at += per * kFour) {
+            uint32_t q[4];
+            asm volatile("ld.shared.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(q[0]), "=r"(q[1]), "=r"(q[2]), "=r"(q[3]) : "r"(at) : "memory");
+#pragma unroll
+            for (int e = 0; e < 4; ++e)
+                v[e] = j == 0 ? q[e] : (is_int ? v[e] + q[e] : __float_as_uint(__fadd_rn(__uint_as_float(v[e]), __uint_as_float(q[e]))));
+        }
+#pragma unroll
+        for (uint32_t e = 0; e < 4; ++e) {
+            if (row + e >= t.live) break;
+            store_out(a.out, base + (int64_t)(t.r0 + row + e) * a.out_ld, split_value<false>(a, v[e], c, s_sa[row + e]), a.out_dtype);
+        }
+    }
+}
+
 // One thread's column of 16 rows of x, straight to the output (stream-k form).
 template <bool kPerBlock>
 __device__ __forceinline__ void split_store16(const SplitArgs& a, const SplitTile& t, int64_t n, const SplitCol& c, uint32_t row, const uint32_t (&v)[16])
@@ -260,7 +315,7 @@ qmm_umma_split_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_co
     const uint32_t smem0 = (ptx::smem_u32(smem_raw) + 1023u) & ~1023u;
     __shared__ __align__(8) uint64_t s_bars[2 * kSplitMaxStages + 8];
     __shared__ uint32_t s_tmem;
-    __shared__ volatile uint32_t s_abort, s_last;
+    __shared__ volatile uint32_t s_abort, s_last, s_bad;  // s_bad: a CTA of the cluster gave up a wait
     __shared__ float s_sa[256];  // x1 scales of the tile's rows (one piece per CTA)
     const uint32_t full0 = ptx::smem_u32(s_bars), empty0 = full0 + 8u * kSplitMaxStages, tfull0 = empty0 + 8u * kSplitMaxStages, tempty0 = tfull0 + 32u;
     volatile uint32_t* abort_flag = &s_abort;
@@ -270,6 +325,7 @@ qmm_umma_split_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_co
     // programmatic dependent launch: placed and set up under the tail of the kernel before it, reads nothing until that has finished
     if (threadIdx.x == 0) {
         s_abort = 0u;
+        s_bad = 0u;
         for (uint32_t i = 0; i < a.stages; ++i) {
             ptx::mbar_init(&s_bars[i], 1);
             ptx::mbar_init(&s_bars[kSplitMaxStages + i], 1);
@@ -294,9 +350,15 @@ qmm_umma_split_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_co
 
     const uint32_t u_begin = split_begin(a, blockIdx.x), u_end = split_begin(a, blockIdx.x + 1);
     SplitCols4 cols4;  // (per-block: only a bias, read at the end; 16 registers the sums need)
+    const bool push = !kPerBlock && a.push != 0u;
+    SplitCol own{1.f, 0.f, 0};  // push: of the column that this thread serves in the end
+    bool met = false;           // push: this warp has met the cluster's others at the end of the stages
     if (warp < 8 && a.split != 0u) {
         const SplitTile tile = split_tile(a, blockIdx.x / a.split);
-        if constexpr (!kPerBlock) cols4 = split_cols4<kPerBlock, kHalves>(a, tile, threadIdx.x);
+        if constexpr (!kPerBlock) {
+            if (push) own = split_col<false>(a, tile.b, min((int64_t)tile.n0 + threadIdx.x % (128u * kHalves), a.n - 1));
+            else cols4 = split_cols4<kPerBlock, kHalves>(a, tile, threadIdx.x);
+        }
         if (!kPerBlock && threadIdx.x < a.rows) s_sa[threadIdx.x] = split_sa<kPerBlock>(a, tile.r0 + min(threadIdx.x, tile.live - 1u));
     }
     const uint32_t set = kHalves * a.rows;  // TMEM columns of one accumulator buffer
@@ -461,7 +523,7 @@ qmm_umma_split_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_co
                     if (++buf == a.dbufs) { buf = 0; bpar ^= 1u; }
                 }
             } else {
-                if (!__all_sync(0xffffffffu, ptx::mbar_wait_relaxed(&s_bars[2 * kSplitMaxStages + buf], bpar, abort_flag))) {
+                if (!__all_sync(0xffffffffu, ptx::mbar_wait_a(tfull0 + 8u * buf, bpar, abort_flag))) {
                     report(abort_flag, (3u << 8) | 1u);
                     ok = false;
                 }
@@ -491,7 +553,20 @@ qmm_umma_split_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_co
                     ptx::tmem_ld_wait();
                 }
             };
-            if (a.split != 0u) {
+            if (push) {
+                // where every CTA of the cluster is done with its stages, the sums go to their owners
+                const uint32_t live = split_tile(a, t).live;
+                __syncwarp();
+                ptx::cluster_arrive();
+                ptx::cluster_wait();
+                met = true;
+#pragma unroll 1
+                for (uint32_t i = 0; i < cnt_rows && row0 + i < live; i += 16) {
+                    uint32_t v[16];
+                    get(i, v);
+                    split_push16<kHalves>(smem0, live, a.split, ptx::cluster_ctarank(), row0 + i, col, v);
+                }
+            } else if (a.split != 0u) {
                 // the tile's only piece here: into shared memory (no copy is in flight any more), as [row of x][column]
                 const uint32_t width = 128u * a.halves;
 #pragma unroll
@@ -521,7 +596,23 @@ qmm_umma_split_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_co
             ++t;
         }
     }
-    if (a.split > 1u) {
+    if (push) {
+        // A CTA that gave up a wait joins both barriers too; what it sends is not used, and then nobody writes.
+        if (!met) {
+            __syncwarp();
+            ptx::cluster_arrive();
+            ptx::cluster_wait();
+        }
+        if (threadIdx.x < a.split && *abort_flag != 0u) {  // (final: every warp's waits lie behind it)
+            uint32_t remote;
+            asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(remote) : "r"(ptx::smem_u32(const_cast<uint32_t*>(&s_bad))), "r"(threadIdx.x));
+            asm volatile("st.shared::cluster.u32 [%0], %1;" ::"r"(remote), "r"(1u) : "memory");
+        }
+        __syncwarp();
+        ptx::cluster_arrive();
+        ptx::cluster_wait();
+        if (warp < 8 && s_bad == 0u) split_sum_fours<kHalves>(a, smem0, split_tile(a, blockIdx.x / a.split), ptx::cluster_ctarank(), threadIdx.x, s_sa, own);
+    } else if (a.split > 1u) {
         // the pieces of the tile meet; a CTA that gave up a wait still joins both barriers, and then nobody writes
         __syncwarp();
         ptx::cluster_sync();
@@ -719,6 +810,11 @@ int32_t split_launch(const OpsnnQmmParams* p, SplitChoice& choice, cudaStream_t 
         a.count = reinterpret_cast<unsigned long long*>(ws);
         a.part = reinterpret_cast<uint32_t*>(ws + (((uint64_t)q.tiles * 8u + 255u) & ~(uint64_t)255u));
     }
+    // Sent or fetched: a column of four rows at a time is summed with less code and fewer waits, but by 256 threads whose stores are two bytes wide.
+    // us, graph replay, fetched / sent, by the fours that a thread sums: one, 16 x 1472 x 4880 int8 5.85 / 5.21, 32 x 4096 x 3072 fp8 7.70 / 6.79;
+    // two, 64 x 4096 x 3072 8.23 / 8.05, 64 x 2048 x 4096 int8 6.56 / 6.28; four, 128 x 4096 x 4096 int8 8.98 / 9.27; twelve, 717 x 7168 x 2304 fp8
+    // 16.8 / 19.7. Per-block, whose sums are in registers, it is 3 - 6 % slower at 14 and 100 rows.
+    a.push = !pb && q.split > 1u && split_share(std::min(q.rows, a.m), q.split) * q.halves <= 4u ? 1u : 0u;
     a.nonce = next_ks_nonce();
     a.test_stop = 0xFFFFFFFFu;
     if (const char* e = env("OPSNN_TEST_SPLIT_STALL_KBLOCK")) {  // tests of the give-up path only

@@ -26,6 +26,15 @@ CASES = [
     ("block", (), 48, 1152, 20096, False, None, "float16"),    # per-block, a tile a CTA
     ("block", (), 100, 3072, 640, True, None, "float32"),
     ("block", (3,), 20, 1088, 320, True, None, "bfloat16"),    # last k-block half full
+    # a cluster's sums sent to their owners: rows that fours and owners do not divide, fewer fours than owners, one and two fours a thread, and the
+    # first sizes past them, where they are fetched
+    ("fp8", (), 5, 1472, 1296, False, "f32", "float32"),
+    ("int8", (), 30, 4096, 3088, True, "f32", "bfloat16"),
+    # (bf16: these outputs are 1e-3 and less, and half a unit of fp16's subnormals, 3e-8, is 2 % of check_close's floor of 1.5e-6)
+    ("fp8", (), 61, 2048, 4112, False, None, "bfloat16"),
+    ("fp8", (), 64, 4096, 3072, True, "f32", "bfloat16"),
+    ("int8", (), 83, 4096, 3072, True, "i32", "bfloat16"),
+    ("int8", (2,), 21, 3072, 400, False, None, "bfloat16"),
     # more tiles of either shape than SMs: pieces across tiles, summed through workspace
     ("int8", (), 64, 384, 40960, True, "i32", "float16"),
     ("fp8", (), 20, 1040, 38416, True, "f32", "bfloat16"),
