@@ -327,10 +327,46 @@ __global__ void __launch_bounds__(256) byte_transpose_kernel(const uint8_t* __re
     }
 }
 
-template <int BN, bool kF4>
+// kSplit: too few tiles for the SMs and a long k (a decoding step). A tile's k stages are cut into a.ksplit pieces, one CTA each, launched as a cluster;
+// its live rows are dealt to the CTAs, mx_share rows each in order of rank, every CTA stores its sums of them in their owner's shared memory
+// ([piece][row of the share][kMxPitch floats], in the place of the stages) and the owner adds the pieces up in the order of k. One CTA a tile is
+// bound by the chain of its stages, 0.2 - 0.3 us each whatever the rows are. us, graph replay, weights from HBM, before /
+// after: 12 x 9216 x 1408 fp8 20.0 / 9.4, 64 x 7168 x 2304 fp8 17.2 / 10.0, 3 x 3 x 13184 x 2112 fp8 33.3 / 27.1, 1 x 4096 x 4096 fp4 8.1 / 7.5.
+constexpr uint32_t kMxPitch = 132;  // four more than the columns: neighbouring rows start in other banks
+__host__ __device__ __forceinline__ uint32_t mx_share(uint32_t live, uint32_t split) { return (live + split - 1u) / split; }
+
+// Four neighbouring columns of an output row.
+__device__ __forceinline__ void mx_store4(const UmmaArgs& a, uint8_t* out, int64_t row, int64_t col, const float (&f)[4], int valid)
+{
+    if (a.out_dtype == ACL_FLOAT) {
+        float* o = reinterpret_cast<float*>(out) + row * a.out_ld + col;
+        if (valid >= 4 && (reinterpret_cast<uintptr_t>(o) & 15) == 0) {
+            *reinterpret_cast<float4*>(o) = make_float4(f[0], f[1], f[2], f[3]);
+        } else {
+#pragma unroll
+            for (int i = 0; i < 4; ++i)
+                if (i < valid) o[i] = f[i];
+        }
+        return;
+    }
+    uint16_t* o = reinterpret_cast<uint16_t*>(out) + row * a.out_ld + col;
+    uint16_t h[4];
+#pragma unroll
+    for (int i = 0; i < 4; ++i) h[i] = a.out_dtype == ACL_BF16 ? __bfloat16_as_ushort(__float2bfloat16_rn(f[i])) : __half_as_ushort(__float2half_rn(f[i]));
+    if (valid >= 4 && (reinterpret_cast<uintptr_t>(o) & 7) == 0) {
+        *reinterpret_cast<uint2*>(o) = make_uint2((uint32_t)h[0] | ((uint32_t)h[1] << 16), (uint32_t)h[2] | ((uint32_t)h[3] << 16));
+    } else {
+#pragma unroll
+        for (int i = 0; i < 4; ++i)
+            if (i < valid) o[i] = h[i];
+    }
+}
+
+template <int BN, bool kF4, bool kSplit = false>
 __global__ void __launch_bounds__(192, 1)
 qmm_mx_umma_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b, const UmmaArgs a)
 {
+    static_assert(!kSplit || BN == 128, "pieces: 128-column tiles");
     constexpr int EW = 4;
     constexpr int kAtoms = kF4 ? 2 : 1;  // k atoms per stage: a stage is 128 bytes of k = 4 (fp8) / 8 (fp4) k-blocks of 32
     constexpr int RA = MxTile<BN>::kRowAtoms;
@@ -351,6 +387,7 @@ qmm_mx_umma_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_const
     uint64_t* tempty = tfull + 2;
     uint32_t* tmem_ptr = reinterpret_cast<uint32_t*>(tempty + 2);
     volatile uint32_t* abort_flag = tmem_ptr + 1;
+    volatile uint32_t* bad = tmem_ptr + 2;  // kSplit: a CTA of the cluster gave up a wait
     float* s_bias = reinterpret_cast<float*>(tmem_ptr + 4);  // [256]
 
     const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0);
@@ -365,6 +402,7 @@ qmm_mx_umma_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_const
             ptx::mbar_init(&tempty[b], EW);  // one arrival per epilogue warp
         }
         *abort_flag = 0u;
+        *bad = 0u;
         ptx::fence_mbar_init();
     }
     if (warp == EW + 1) ptx::tmem_alloc(tmem_ptr, kTmemCols);
@@ -380,7 +418,12 @@ qmm_mx_umma_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_const
     const uint32_t smem0 = ptx::smem_u32(smem), full0 = ptx::smem_u32(full), empty0 = ptx::smem_u32(empty);
     const uint32_t stages = (uint32_t)a.stages;
     const int kstages = a.kblocks;  // 128-byte k stages per tile
+    // kSplit: one tile a cluster, stages [k_first, k_last) of it here; otherwise every gridDim.x-th tile, whole
+    const uint32_t rank = kSplit ? ptx::cluster_ctarank() : 0u, ksplit = kSplit ? (uint32_t)a.ksplit : 1u;
+    const uint32_t tile0 = kSplit ? blockIdx.x / ksplit : blockIdx.x, tile_step = kSplit ? ntiles : gridDim.x;
+    const int k_first = kSplit ? (int)((uint32_t)kstages * rank / ksplit) : 0, k_last = kSplit ? (int)((uint32_t)kstages * (rank + 1u) / ksplit) : kstages;
 
+    bool met = false;  // kSplit: this warp has met the cluster's others at the end of the stages
     if (warp == EW) {
         // ======================= producer: two TMA loads and two scale-atom bulk copies per stage =======================
         if (lane == 0) {
@@ -391,18 +434,18 @@ qmm_mx_umma_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_const
         uint32_t s = 0, par = 0;
         bool ok = true;
         const bool b_mn = a.b_mn_major != 0, a_mn = a.a_mn_major != 0;
-        for (uint32_t tile = blockIdx.x; tile < ntiles && ok; tile += gridDim.x) {
+        for (uint32_t tile = tile0; tile < ntiles && ok; tile += tile_step) {
             const uint32_t b = tile / tiles_per_batch, r = tile % tiles_per_batch;
             uint32_t tm, tn;
             tile_of<16>(r, (uint32_t)a.tiles_m, (uint32_t)a.tiles_n, tm, tn);
             const int32_t m0 = (int32_t)tm * BM, n0 = (int32_t)tn * BN;
             const int32_t ba = a.a_batched ? (int32_t)b : 0, bb = a.b_batched ? (int32_t)b : 0;
-            const uint8_t* sfa = a.sfa + (int64_t)ba * a.sfa_bs + ((int64_t)tm * kstages) * kSfaBytes;
-            const uint8_t* sfb = a.sfb + (int64_t)bb * a.sfb_bs + ((int64_t)tn * kstages) * kSfbBytes;
+            const uint8_t* sfa = a.sfa + (int64_t)ba * a.sfa_bs + ((int64_t)tm * kstages + k_first) * kSfaBytes;
+            const uint8_t* sfb = a.sfb + (int64_t)bb * a.sfb_bs + ((int64_t)tn * kstages + k_first) * kSfbBytes;
             // bytes one stage's copies deliver: k-major B is one box of BN rows, n-major B whole 128-column boxes
             const uint32_t tx = (uint32_t)kATile + (b_mn ? kBTile : (uint32_t)(BN * BK)) + kSfaBytes + kSfbBytes;
-            int32_t kk = 0;
-            for (int kb = 0; kb < kstages; ++kb) {
+            int32_t kk = k_first * BK;
+            for (int kb = k_first; kb < k_last; ++kb) {
                 if (!ptx::mbar_wait_a(empty0 + 8u * s, par ^ 1u, abort_flag)) {
                     report(abort_flag, (1u << 8) | 1u);
                     ok = false;
@@ -440,14 +483,14 @@ qmm_mx_umma_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_const
         const uint64_t a_hi = da0 & 0xFFFFFFFF00000000ull, b_hi = db0 & 0xFFFFFFFF00000000ull, sf_hi = dsf0 & 0xFFFFFFFF00000000ull;
         const uint32_t a_k1 = a.a_mn_major ? 256u : 2u, b_k1 = a.b_mn_major ? 256u : 2u;
         const uint32_t idesc = a.idesc;
-        for (uint32_t tile = blockIdx.x; tile < ntiles && ok; tile += gridDim.x) {
+        for (uint32_t tile = tile0; tile < ntiles && ok; tile += tile_step) {
             uint32_t acc = 0u;
             if (!ptx::mbar_wait_a(tempty0 + 8u * (grp & 1u), ((grp >> 1) & 1u) ^ 1u, abort_flag)) {
                 report(abort_flag, (2u << 8) | 1u);
                 ok = false;
                 break;
             }
-            for (int kb = 0; kb < kstages; ++kb) {
+            for (int kb = k_first; kb < k_last; ++kb) {
                 if (!ptx::mbar_wait_a(full0 + 8u * s, par, abort_flag)) {
                     report(abort_flag, (2u << 8) | 2u);
                     ok = false;
@@ -495,7 +538,8 @@ qmm_mx_umma_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_const
         const uint32_t lane_addr = (uint32_t)(quad * 32) << 16;
         uint32_t grp = 0;
         bool ok = true;
-        for (uint32_t tile = blockIdx.x; tile < ntiles && ok; tile += gridDim.x) {
+        (void)met;
+        for (uint32_t tile = tile0; tile < ntiles && ok; tile += tile_step) {
             const uint32_t b = tile / tiles_per_batch, r = tile % tiles_per_batch;
             uint32_t tm, tn;
             tile_of<16>(r, (uint32_t)a.tiles_m, (uint32_t)a.tiles_n, tm, tn);
@@ -517,6 +561,32 @@ qmm_mx_umma_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_const
                 break;
             }
             ptx::tc_fence_after();
+            if constexpr (kSplit) {
+                __syncwarp();
+                ptx::cluster_arrive();
+                ptx::cluster_wait();
+                met = true;
+                const uint32_t live = (uint32_t)min((int64_t)BM, a.m - m0), per = mx_share(live, ksplit), mine = (uint32_t)(quad * 32 + lane);
+                if ((uint32_t)(quad * 32) < live) {
+                    const uint32_t owner = min(mine / per, ksplit - 1u);
+                    uint32_t to;
+                    asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(to) : "r"(smem0 + (rank * per + mine - owner * per) * (kMxPitch * 4u)), "r"(owner));
+#pragma unroll 1
+                    for (int c = 0; c < BN; c += 32) {
+                        uint32_t v[32];
+                        ptx::tmem_ld32(tmem_base + lane_addr + buf * kAcc1 + c, v);
+                        ptx::tmem_ld_wait();
+                        if (mine < live) {
+#pragma unroll
+                            for (int i = 0; i < 32; i += 4)
+                                asm volatile("st.shared::cluster.v4.u32 [%0], {%1, %2, %3, %4};" ::"r"(to + (uint32_t)(c + i) * 4u), "r"(v[i]), "r"(v[i + 1]), "r"(v[i + 2]),
+                                             "r"(v[i + 3])
+                                             : "memory");
+                        }
+                    }
+                }
+                break;
+            }
 #pragma unroll 1
             for (int c = 0; c < BN; c += 32) {
                 uint32_t v[32];
@@ -541,6 +611,45 @@ qmm_mx_umma_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_const
             __syncwarp();
                 if (lane == 0) ptx::mbar_arrive(&tempty[buf]);
             ++grp;
+        }
+    }
+    if constexpr (kSplit) {
+        // A CTA that gave up a wait joins both barriers too; what it sends is not used, and then nobody writes.
+        if (!met) {
+            __syncwarp();
+            ptx::cluster_arrive();
+            ptx::cluster_wait();
+        }
+        if (threadIdx.x < ksplit && *abort_flag != 0u) {  // (final: every warp's waits lie behind it)
+            uint32_t remote;
+            asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(remote) : "r"(ptx::smem_u32(const_cast<uint32_t*>(bad))), "r"(threadIdx.x));
+            asm volatile("st.shared::cluster.u32 [%0], %1;" ::"r"(remote), "r"(1u) : "memory");
+        }
+        __syncwarp();
+        ptx::cluster_arrive();
+        ptx::cluster_wait();
+        if (warp < EW && *bad == 0u) {
+            const uint32_t b = tile0 / tiles_per_batch, r = tile0 % tiles_per_batch;
+            uint32_t tm, tn;
+            tile_of<16>(r, (uint32_t)a.tiles_m, (uint32_t)a.tiles_n, tm, tn);
+            const int64_t m0 = (int64_t)tm * BM, col = (int64_t)tn * BN + lane * 4;
+            const uint32_t live = (uint32_t)min((int64_t)BM, a.m - m0), per = mx_share(live, ksplit), end = min(live, (rank + 1u) * per);
+            uint8_t* out = reinterpret_cast<uint8_t*>(a.out) + b * a.out_bs * (a.out_dtype == ACL_FLOAT ? 4 : 2);
+            const int valid = (int)max((int64_t)0, min((int64_t)4, a.n - col));
+            const float4 bias = *reinterpret_cast<const float4*>(s_bias + lane * 4);
+#pragma unroll 1
+            for (uint32_t row = rank * per + (uint32_t)warp; row < end; row += EW) {
+                float f[4] = {0.f, 0.f, 0.f, 0.f};
+                uint32_t at = smem0 + (row - rank * per) * (kMxPitch * 4u) + (uint32_t)lane * 16u;
+#pragma unroll 2
+                for (uint32_t j = 0; j < ksplit; ++j, at += per * (kMxPitch * 4u)) {
+                    float4 q;
+                    asm volatile("ld.shared.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(q.x), "=f"(q.y), "=f"(q.z), "=f"(q.w) : "r"(at) : "memory");
+                    f[0] += q.x; f[1] += q.y; f[2] += q.z; f[3] += q.w;
+                }
+                f[0] = __fadd_rn(f[0], bias.x); f[1] = __fadd_rn(f[1], bias.y); f[2] = __fadd_rn(f[2], bias.z); f[3] = __fadd_rn(f[3], bias.w);
+                if (valid > 0) mx_store4(a, out, m0 + row, col, f, valid);
+            }
         }
     }
     if (*abort_flag != 0u) __nanosleep(200000);  // lets copies that are still in flight land before the CTA leaves
@@ -640,6 +749,70 @@ int32_t mx_launch_one(const CUtensorMap& ma, const CUtensorMap& mb, UmmaArgs& a,
     launch_dependent(qmm_mx_umma_kernel<BN, kF4>, dim3((unsigned)grid), 192, smem, stream, ma, mb, a);
     note_launch(kF4 ? "qmm_umma_mxfp4" : "qmm_umma_mxfp8");
     return (int32_t)cudaGetLastError();
+}
+
+// How many pieces a tile's k is cut into (kSplit), 1: none. In us: a stage of the chain 0.18, the two cluster barriers 0.9, a piece to add 0.15, a row to
+// send 0.018 (fitted; graph replay, by pieces, 12 x 9216 x 1408 fp8: one 20.0, two 13.4, four 9.9, eight 9.4, twelve 9.7; 128 x 4096 x 4096 one 12.5, two
+// 13.0, four 11.8; 2 x 300 x 2048 x 1024, which stays whole, one 9.4, three 11.4).
+template <bool kF4>
+int mx_pick_split(const UmmaArgs& a, size_t smem)
+{
+    const char* e = env("OPSNN_MX_SPLIT");  // experiments
+    const int sms = sm_count();
+    int most = (int)std::min<int64_t>(std::min<int64_t>(16, a.kblocks / 2), sms / std::max<int64_t>(a.num_tiles, 1));
+    if (e != nullptr) most = std::min(most, atoi(e));
+    if (most < 2) return 1;
+    static std::atomic<uint64_t> configured{0};
+    const auto kern = qmm_mx_umma_kernel<128, kF4, true>;
+    const cudaError_t rc = once_per_device(configured, [&] {
+        cudaFuncSetAttribute(kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
+        return cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024);
+    });
+    if (rc != cudaSuccess) {
+        cudaGetLastError();
+        return 1;
+    }
+    int best = 1;
+    double cost = 0.18 * a.kblocks;
+    for (int s = most; s >= 2; --s) {
+        const double c = 0.18 * ((a.kblocks + s - 1) / s) + 0.9 + 0.15 * s + 0.018 * (double)std::min<int64_t>(a.m, BM);
+        if (c < cost && max_active_clusters(reinterpret_cast<const void*>(kern), 192, (int)smem, s, 0) >= a.num_tiles) {
+            cost = c;
+            best = s;
+        }
+    }
+    return best;
+}
+
+// The 128-column kernel with a tile's k in pieces; -1: not this call.
+template <bool kF4>
+int32_t mx_launch_split(const CUtensorMap& ma, const CUtensorMap& mb, UmmaArgs& a, cudaStream_t stream)
+{
+    constexpr uint32_t stage = (uint32_t)kATile + MxTile<128>::kBSmem + (kF4 ? 2 : 1) * 512 * 2;
+    constexpr int kStages = (227 * 1024 - 2048) / (int)stage;  // six; the shares of a tile, at most (128 + 15) rows of 528 bytes, need three
+    static_assert(3 * stage >= (128 + 15) * kMxPitch * 4, "the shares lie in the place of the stages");
+    const size_t smem = (size_t)kStages * stage + 1024 + 256 + 256 * 4;
+    const int split = mx_pick_split<kF4>(a, smem);
+    if (split < 2) return -1;
+    a.stages = kStages;
+    a.ksplit = split;
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3((unsigned)(a.num_tiles * split), 1, 1);
+    cfg.blockDim = dim3(192, 1, 1);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = stream;
+    cudaLaunchAttribute attr[2]{};
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    attr[1].id = cudaLaunchAttributeClusterDimension;
+    attr[1].val.clusterDim.x = (unsigned)split;
+    attr[1].val.clusterDim.y = 1;
+    attr[1].val.clusterDim.z = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 2;
+    const int32_t rc = (int32_t)cudaLaunchKernelEx(&cfg, qmm_mx_umma_kernel<128, kF4, true>, ma, mb, a);
+    note_launch(kF4 ? "qmm_umma_mxfp4_split" : "qmm_umma_mxfp8_split");
+    return rc;
 }
 
 }  // namespace
@@ -839,5 +1012,9 @@ int32_t qmm_mx_umma_launch(const OpsnnQmmParams* p0, cudaStream_t stream)
 
     if (q.pair) return q.f4 ? mx_launch_pair<true>(ma, mb, a, stream) : mx_launch_pair<false>(ma, mb, a, stream);
     if (q.bn == 224) return q.f4 ? mx_launch_one<224, true>(ma, mb, a, stream) : mx_launch_one<224, false>(ma, mb, a, stream);
+    if (env("OPSNN_QMM_MX_BN") == nullptr) {
+        const int32_t rc = q.f4 ? mx_launch_split<true>(ma, mb, a, stream) : mx_launch_split<false>(ma, mb, a, stream);
+        if (rc >= 0) return rc;
+    }
     return q.f4 ? mx_launch_one<128, true>(ma, mb, a, stream) : mx_launch_one<128, false>(ma, mb, a, stream);
 }

@@ -139,6 +139,31 @@ def test_mx_fixtures_run_on_the_tensor_core_kernels(aclnn):
         _check(got, a["out"], meta["out_dtype"])
 
 
+@pytest.mark.parametrize("case", [
+    # dtype, batch, m, k, n, x2 stored (n,k), bias, out
+    (E4M3, (), 1, 4128, 1000, True, True, "bfloat16"),       # one live row, k a quarter of a stage past the last, n no whole tile
+    (E4M3, (), 13, 9216, 1408, False, False, "float16"),     # rows that the owners do not divide, x2 along n
+    (E4M3, (3,), 3, 6144, 264, True, True, "bfloat16"),      # batched, more owners than rows
+    (E4M3, (), 100, 7168, 384, True, False, "float32"),
+    (E4M3, (), 128, 8192, 130, True, True, "float16"),       # a whole tile of rows, the last tile two columns
+    (E4M3, (), 130, 8192, 512, False, True, "bfloat16"),     # two row tiles, two rows in the second
+    (E2M1, (), 5, 8192, 640, True, True, "bfloat16"),
+    (E2M1, (2,), 70, 16448, 200, True, False, "float32"),    # k a quarter of a stage past the last
+], ids=str)
+def test_mx_pieces_of_k_equal_oracle(aclnn, case):
+    """Few tiles and a long k: the pieces of a tile's k on the CTAs of a cluster, summed by the owners of its rows. Twice, for the same bits."""
+    dt, batch, m, k, n, nk, has_bias, out_name = case
+    rng = np.random.default_rng(case_seed(case))
+    x1, x2 = _q(rng, batch + (m, k), dt), _q(rng, batch + ((n, k) if nk else (k, n)), dt)
+    kq = -(-k // 64)
+    s1, s2 = _e8m0(rng, batch + (m, kq, 2)), _e8m0(rng, batch + ((n, kq, 2) if nk else (kq, n, 2)))
+    bias = rng.uniform(-2, 2, n).astype(np.float32) if has_bias else None
+    name = "qmm_umma_mxfp4_split" if dt == E2M1 else "qmm_umma_mxfp8_split"
+    got = [_run(aclnn, x1, x2, s1, s2, bias, False, nk, out_name, name) for _ in range(2)]
+    assert np.array_equal(got[0].view(np.uint8), got[1].view(np.uint8))
+    _check(got[0], _oracle(x1, x2, s1, s2, bias, False, nk, out_name), out_name)
+
+
 @pytest.mark.parametrize("dst", ["float8_e4m3fn", "float8_e5m2", "float4_e2m1"])
 @pytest.mark.parametrize("xdt", ["bfloat16", "float16"])
 def test_dynamic_mx_quant_streaming_kernel_matches_oracle(aclnn, dst, xdt):
