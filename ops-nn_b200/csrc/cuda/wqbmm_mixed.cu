@@ -519,12 +519,13 @@ __device__ __forceinline__ void mix_push(const MixArgs& a, uint32_t acc, uint32_
         if (r0 >= live) continue;
         float f[16];
         mix_sums16<kMany>(acc + hc, n_acc, step, f);
+        uint32_t part = r0 + 2u * h + ((uint32_t)col >> 6), owner = part * inverse >> 16, slot = part - owner * per;
 #pragma unroll
         for (uint32_t i = 0; i < 16; i += 4) {
             if (r0 + i >= live) break;
-            const uint32_t part = r0 + i + 2u * h + ((uint32_t)col >> 6), owner = part * inverse >> 16;
             uint32_t to;
-            asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(to) : "r"(mine + (part - owner * per) * kMixPartBytes), "r"(owner));
+            asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(to) : "r"(mine + slot * kMixPartBytes), "r"(owner));
+            for (slot += 4u; slot >= per; slot -= per) ++owner;  // the next four rows
             asm volatile("st.shared::cluster.v4.f32 [%0], {%1, %2, %3, %4};" ::"r"(to), "f"(f[i]), "f"(f[i + 1]), "f"(f[i + 2]), "f"(f[i + 3]) : "memory");
         }
     }
@@ -619,7 +620,7 @@ wqbmm_mixed_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
 
     const uint32_t u_begin = mix_begin(a, blockIdx.x), u_end = mix_begin(a, blockIdx.x + 1);
     const uint32_t stages = a.stages, stage_bytes = a.stage_bytes;
-    const uint32_t live = min((uint32_t)a.rows, (uint32_t)a.m - (u_begin / a.kb) % (uint32_t)a.t_tiles * (uint32_t)a.rows);  // rows of x in the first tile
+    auto rows_live = [&] { return min((uint32_t)a.rows, (uint32_t)a.m - (blockIdx.x / a.split) % (uint32_t)a.t_tiles * (uint32_t)a.rows); };  // rows of x in the (only) tile
     const uint32_t xunit = (uint32_t)a.rows * 128u;  // bytes of x per 64-row unit of k
     // accumulators: two sets where there is room, beside them the sums of the chunks that are done
     const uint32_t d_one = 2u * (uint32_t)a.rows, d_set = kSum == MixSum::kCopies ? a.copies * d_one : d_one;
@@ -1067,7 +1068,7 @@ wqbmm_mixed_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
             __syncwarp();
             ptx::cluster_arrive();
             ptx::cluster_wait();
-            mix_push<kMany>(a, acc, n_acc, step, smem0, live, ptx::cluster_ctarank(), col, warp >> 2);
+            mix_push<kMany>(a, acc, n_acc, step, smem0, rows_live(), ptx::cluster_ctarank(), col, warp >> 2);
         } else if (mix_all_ok<2, kMixDqWarps * 32>(ok)) {
             ptx::tc_fence_after();
             mix_finish<kBf16, 16, kMany>(a, acc, n_acc, step, t_last, last_cnt, col, qd, lane, warp >> 2, threadIdx.x == 0, &s_last[1], abort_flag);
@@ -1145,7 +1146,7 @@ wqbmm_mixed_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
         ptx::cluster_arrive();
         ptx::cluster_wait();
         // (nobody reaches into another CTA's shared memory from here on: they leave when they are done)
-        if (warp < kMixDqWarps && s_bad == 0u) mix_sum_and_store<kBf16>(a, smem0, blockIdx.x / a.split, live, ptx::cluster_ctarank(), threadIdx.x, s_bias);
+        if (warp < kMixDqWarps && s_bad == 0u) mix_sum_and_store<kBf16>(a, smem0, blockIdx.x / a.split, rows_live(), ptx::cluster_ctarank(), threadIdx.x, s_bias);
     }
     // ---- teardown: everyone meets here, also after an aborted wait; then the allocating warp frees TMEM ----
     if (*abort_flag != 0u) __nanosleep(200000);  // lets bulk copies that are still in flight land before the CTA leaves
