@@ -985,7 +985,7 @@ int32_t qmm_umma_launch(const OpsnnQmmParams* p, cudaStream_t stream)
     int64_t b_ld = p->b_ld, b_bs = p->b_bs;
     int b_trans = p->trans_b;
     const int pb_bn = asym ? 128 : (pair_pb ? pair_pb_bn(p) : 0);
-    const int bn = pair ? 256 : (pair_pb ? pb_bn : pick_bn(p));
+    const int bn = pair ? pair_tile(p) : (pair_pb ? pb_bn : pick_bn(p));
     const int bm = (pair || pair_pb) ? 256 : BM;
     UmmaArgs a{};
     a.mode = p->mode;
@@ -1041,7 +1041,7 @@ int32_t qmm_umma_launch(const OpsnnQmmParams* p, cudaStream_t stream)
     else if (a.b_mn_major) ok = ok && make_map(&mb, b_ptr, (uint64_t)p->n, (uint64_t)p->k, nb_b, (uint64_t)b_ld, (uint64_t)b_bs, 128,
                                                bn < 128 ? (uint32_t)bn : 128u);
     else ok = ok && make_map(&mb, b_ptr, (uint64_t)p->k * es, (uint64_t)p->n, nb_b, (uint64_t)b_ld * es, (uint64_t)b_bs * es,
-                             pair ? 128u : (pair_pb ? (uint32_t)(pb_bn / 2) : (uint32_t)bn));
+                             pair || pair_pb ? (uint32_t)(bn / 2) : (uint32_t)bn);
     if (!ok) return (int32_t)cudaErrorInvalidValue;
     if (asym) {
         if (p->workspace == nullptr || p->workspace_size < qmm_umma_workspace_size(p)) return (int32_t)cudaErrorInvalidValue;
@@ -1066,8 +1066,8 @@ int32_t qmm_umma_launch(const OpsnnQmmParams* p, cudaStream_t stream)
         if (a.is_int) return launch_pair_pb<ptx::MmaKind::kI8, 8>(ma, mb, a, stream);
         return launch_pair_pb<ptx::MmaKind::kF8F6F4, 8>(ma, mb, a, stream);
     }
-    if (pair && f16) return launch_pair<ptx::MmaKind::kF16>(ma, mb, a, stream);
-    if (pair) return a.is_int ? launch_pair<ptx::MmaKind::kI8>(ma, mb, a, stream) : launch_pair<ptx::MmaKind::kF8F6F4>(ma, mb, a, stream);
+    if (pair && f16) return launch_pair<ptx::MmaKind::kF16>(bn, ma, mb, a, stream);
+    if (pair) return a.is_int ? launch_pair<ptx::MmaKind::kI8>(bn, ma, mb, a, stream) : launch_pair<ptx::MmaKind::kF8F6F4>(bn, ma, mb, a, stream);
     if (f16) return launch_bn<false, ptx::MmaKind::kF16>(bn, ma, mb, a, stream);
 
     if (p->mode == OPSNN_QMM_PERBLOCK)

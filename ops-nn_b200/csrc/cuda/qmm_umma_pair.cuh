@@ -16,14 +16,15 @@
 // the two CTAs meet at a cluster barrier before the first remote signal and before TMEM is freed.
 namespace {
 
-template <ptx::MmaKind kKind>
+// BN: 256, or 224 / 192 where that leaves less of the last wave idle (pair_tile).
+template <ptx::MmaKind kKind, int BN>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(192, 1)
 qmm_umma_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b, const UmmaArgs a)
 {
-    constexpr int BN = 256, EW = 4;         // pair tile 256 x 256; each CTA: 128 rows of A, 128 columns of B, 128 x 256 accumulator
-    constexpr uint32_t kBHalf = 128 * BK;   // this CTA's half of the B tile
+    constexpr int EW = 4;                       // pair tile 256 x BN; each CTA: 128 rows of A, BN / 2 columns of B, 128 x BN accumulator
+    constexpr uint32_t kBHalf = (BN / 2) * BK;  // this CTA's half of the B tile
     constexpr uint32_t kStage = kATile + kBHalf;
-    constexpr uint32_t kTmemCols = 512;     // two accumulator buffers of 256 columns
+    constexpr uint32_t kTmemCols = 512, kBuf = 256;  // two accumulator buffers
 
     extern __shared__ uint8_t smem_raw[];
     uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
@@ -87,7 +88,7 @@ qmm_umma_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_con
             uint32_t tm, tn;
             tile_of<8>(r, (uint32_t)a.tiles_m, (uint32_t)a.tiles_n, tm, tn);
             const int32_t m0 = (int32_t)tm * 256 + (int32_t)rank * 128;
-            const int32_t n0 = (int32_t)tn * BN + (int32_t)rank * 128;
+            const int32_t n0 = (int32_t)tn * BN + (int32_t)rank * (BN / 2);
             const int32_t ba = a.a_batched ? (int32_t)b : 0, bb = a.b_batched ? (int32_t)b : 0;
             int32_t kk = 0;
             for (int kb = 0; kb < kblocks; ++kb) {
@@ -138,7 +139,7 @@ qmm_umma_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_con
                     ptx::tc_fence_after();
                     if (ptx::elect_one()) {
                         const uint32_t stage_off = (s * kStage) >> 4;
-                        const uint32_t d = tmem_base + (grp & 1u) * BN;
+                        const uint32_t d = tmem_base + (grp & 1u) * kBuf;
                         const uint32_t al = a_lo + stage_off, bl = b_lo + stage_off;
 #pragma unroll
                         for (int k = 0; k < 4; ++k)
@@ -192,7 +193,7 @@ qmm_umma_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_con
                 break;
             }
             ptx::tc_fence_after();
-            deq_store_cols<BN>(a, tmem_base + lane_addr + buf * BN, out, row, row_ok, n0, s_scale, s_bias, sav, has_sa, has_fbias, has_ibias);
+            deq_store_cols<BN>(a, tmem_base + lane_addr + buf * kBuf, out, row, row_ok, n0, s_scale, s_bias, sav, has_sa, has_fbias, has_ibias);
             ptx::tc_fence_before();
             __syncwarp();
             if (lane == 0) ptx::mbar_arrive_cluster(lead_tempty0 + 8u * buf);
@@ -210,16 +211,39 @@ qmm_umma_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_con
     }
 }
 
-template <ptx::MmaKind KIND>
+// Columns of the pair kernel's tiles. All pairs run tiles of one size in waves, and a last wave that is nearly empty takes as long as a full one: 1024 rows
+// x 7168 columns are 1.5 waves of 256 columns and 1.7 of 224. A k-block is 2 BN clocks of tensor work and some 24 more; narrower tiles load A more often
+// per column, which costs 4 and 9 % under the power limit. us, 256 / 224 / 192 columns, back to back: 1024 x 4096 x 7168 int8 30.5 / 28.4 / 30.7,
+// 1300 x 8192 x 7168 16-bit after its pre-pass 190 / 182 / 194, 2048 x 8192 x 28672 876 / 869 / 888, 4096 x 4096 x 4096 fp8 61.2 / 62.8 / 62.3,
+// 2048 x 7168 x 4608 fp8 58.1 / 63.8 / 61.1. x2 stored along n keeps 256 columns, whole 128-byte rows a CTA. OPSNN_QMM_PAIR_BN fixes it.
+int pair_tile(const OpsnnQmmParams* p)
+{
+    if (!p->trans_b) return 256;
+    if (const char* e = env("OPSNN_QMM_PAIR_BN")) return atoi(e) == 224 ? 224 : (atoi(e) == 192 ? 192 : 256);
+    const int64_t rows = p->batch * ((p->m + 255) / 256), pairs = std::max(sm_count() / 2, 1);
+    int best = 256;
+    double cost = 1e30;
+    for (int bn = 256; bn >= 192; bn -= 32) {
+        const int64_t waves = (rows * ((p->n + bn - 1) / bn) + pairs - 1) / pairs;
+        const double c = (double)waves * (2 * bn + 24) * (bn == 256 ? 1.0 : (bn == 224 ? 1.04 : 1.09));
+        if (c < cost) {
+            cost = c;
+            best = bn;
+        }
+    }
+    return best;
+}
+
+template <ptx::MmaKind KIND, int BN>
 int32_t launch_pair(const CUtensorMap& ma, const CUtensorMap& mb, UmmaArgs& a, cudaStream_t stream)
 {
-    constexpr int kStage = kATile + 128 * BK;
+    constexpr int kStage = kATile + (BN / 2) * BK;
     int stages = (227 * 1024 - 2048) / kStage;
     if (stages > 6) stages = 6;
     if (stages > a.kblocks + 1) stages = a.kblocks + 1 > 2 ? a.kblocks + 1 : 2;
     a.stages = stages;
     const size_t smem = (size_t)stages * kStage + 1024 + 256 + 2 * 256 * 4;
-    auto kern = qmm_umma_pair_kernel<KIND>;
+    auto kern = qmm_umma_pair_kernel<KIND, BN>;
     static std::atomic<uint64_t> configured{0};
     if (once_per_device(configured, [&] { return cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024); }) != cudaSuccess)
         return (int32_t)cudaGetLastError();
@@ -228,6 +252,14 @@ int32_t launch_pair(const CUtensorMap& ma, const CUtensorMap& mb, UmmaArgs& a, c
     launch_dependent(kern, dim3((unsigned)(2 * pairs)), 192, smem, stream, ma, mb, a);
     note_launch("qmm_umma_pair_deq");
     return (int32_t)cudaGetLastError();
+}
+
+template <ptx::MmaKind KIND>
+int32_t launch_pair(int bn, const CUtensorMap& ma, const CUtensorMap& mb, UmmaArgs& a, cudaStream_t stream)
+{
+    if (bn == 224) return launch_pair<KIND, 224>(ma, mb, a, stream);
+    if (bn == 192) return launch_pair<KIND, 192>(ma, mb, a, stream);
+    return launch_pair<KIND, 256>(ma, mb, a, stream);
 }
 
 // Pairs pay off when there is a 256 x 256 tile for about every pair of SMs; small problems keep the single-CTA kernel.

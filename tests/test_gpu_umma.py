@@ -190,6 +190,31 @@ def test_int8_dequant_cta_pairs_bit_exact(aclnn, case, monkeypatch):
     assert np.array_equal(np.asarray(got).view(np.uint8), np.asarray(want).view(np.uint8))
 
 
+@pytest.mark.parametrize("tile_n", ["224", "192"])
+@pytest.mark.parametrize("m,k,n,t1,dtype", [(256, 256, 224, False, "int8"), (300, 400, 192, False, "int8"), (640, 528, 452, True, "int8"), (257, 2048, 16, False, "int8"),
+                                            (2500, 256, 700, False, "int8"), (1024, 640, 7168, False, "int8"), (390, 400, 640, False, "fp8")])
+def test_narrower_pair_tiles(aclnn, monkeypatch, m, k, n, t1, dtype, tile_n):
+    """224 and 192 columns a pair tile: a CTA's half of B is 112 or 96 rows. n of one tile, a few columns past one, fewer than a half, many waves."""
+    from gpu_util import check_close
+
+    monkeypatch.setenv("OPSNN_QMM_PAIR", "1")
+    monkeypatch.setenv("OPSNN_QMM_PAIR_BN", tile_n)
+    rng = np.random.default_rng(case_seed((m, k, n, t1, dtype)))
+    s1, s2 = rng.uniform(1e-3, 1e-2, m).astype(np.float32), rng.uniform(1e-3, 1e-2, n).astype(np.float32)
+    if dtype == "int8":
+        x1 = rng.integers(-127, 128, (k, m) if t1 else (m, k), dtype=np.int8)
+        x2 = rng.integers(-127, 128, (n, k), dtype=np.int8)
+        bias = rng.integers(-1000, 1001, n).astype(np.int32)
+    else:
+        x1, x2, bias = _fp8(rng, (m, k), E4M3), _fp8(rng, (n, k), E4M3), None
+    want = qbmm_oracle.quant_matmul_v5(x1, x2, s1, s2, bias, t1, True, 0, "bfloat16")
+    got = _run(aclnn, x1, x2, s1, s2, bias, t1, True, 0, "bfloat16", "qmm_umma_pair_deq")
+    if dtype == "int8":
+        assert np.array_equal(np.asarray(got).view(np.uint8), np.asarray(want).view(np.uint8))
+    else:
+        check_close(got, want, qbmm_oracle.quant_matmul_v5(x1, x2, s1, s2, None, t1, True, 0, "float32"), "bfloat16")
+
+
 def test_cta_pairs_batched_fp8_and_auto_selection(aclnn, monkeypatch):
     from gpu_util import check_close
 
