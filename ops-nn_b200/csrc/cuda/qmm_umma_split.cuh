@@ -523,7 +523,7 @@ qmm_umma_split_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_co
                     if (++buf == a.dbufs) { buf = 0; bpar ^= 1u; }
                 }
             } else {
-                if (!__all_sync(0xffffffffu, ptx::mbar_wait_a(tfull0 + 8u * buf, bpar, abort_flag))) {
+                if (!__all_sync(0xffffffffu, ptx::mbar_wait_relaxed(&s_bars[2 * kSplitMaxStages + buf], bpar, abort_flag))) {
                     report(abort_flag, (3u << 8) | 1u);
                     ok = false;
                 }
