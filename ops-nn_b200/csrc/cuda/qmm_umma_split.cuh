@@ -312,6 +312,11 @@ __global__ void __launch_bounds__(kSplitThreads, 1)
 qmm_umma_split_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUtensorMap map_x, const __grid_constant__ SplitArgs a)
 {
     extern __shared__ uint8_t smem_raw[];
+    // The dequant instances have the out-of-line part of their waits for themselves. Shared by all kernels of the file it is compiled to a convention that all
+    // of them can live with, and these, whose chain of waits is most of a call, lost 5 - 10 %. us, graph replay, shared / own: 128 x 4096 x 4096 int8
+    // 9.81 / 9.03, 717 x 7168 x 2304 fp8 18.6 / 18.0, 14 x 8640 x 6048 fp8 17.5 / 15.7, 300 x 4096 x 2048 int8 11.1 / 10.2, 32 x 4096 x 3072 fp8 7.38 / 6.80.
+    // (Per-block 15 x 11136 x 8768 22.5 / 22.7; the fused weight-only, pair and block-scaled kernels do not change.)
+    constexpr int kMe = kPerBlock ? 0 : 1 + (int)kKind * 2 + (int)kHalves;
     const uint32_t smem0 = (ptx::smem_u32(smem_raw) + 1023u) & ~1023u;
     __shared__ __align__(8) uint64_t s_bars[2 * kSplitMaxStages + 8];
     __shared__ uint32_t s_tmem;
@@ -373,7 +378,7 @@ qmm_umma_split_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_co
         SplitTile tile = split_tile(a, t);
         const uint32_t u_stop = u_begin + min(u_end - u_begin, a.test_stop);
         for (uint32_t u = u_begin; u < u_stop; ++u) {
-            if (!ptx::mbar_wait_a(empty0 + 8u * s, par ^ 1u, abort_flag)) {
+            if (!ptx::mbar_wait_a<kMe>(empty0 + 8u * s, par ^ 1u, abort_flag)) {
                 report(abort_flag, (1u << 8) | 1u);
                 break;
             }
@@ -407,13 +412,13 @@ qmm_umma_split_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_co
         bool fresh = true;
         for (uint32_t u = u_begin; u < u_end; ++u) {
             if (kPerBlock || fresh) {
-                if (!ptx::mbar_wait_a(tempty0 + 8u * buf, bpar ^ 1u, abort_flag)) {
+                if (!ptx::mbar_wait_a<kMe>(tempty0 + 8u * buf, bpar ^ 1u, abort_flag)) {
                     report(abort_flag, (2u << 8) | 1u);
                     break;
                 }
                 fresh = false;
             }
-            if (!ptx::mbar_wait_a(full0 + 8u * s, par, abort_flag)) {
+            if (!ptx::mbar_wait_a<kMe>(full0 + 8u * s, par, abort_flag)) {
                 report(abort_flag, (2u << 8) | 2u);
                 break;
             }
@@ -483,7 +488,7 @@ qmm_umma_split_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_co
                 for (uint32_t k = kb; k < kb + cnt; ++k) {
                     publish(k + 1);
                     fetch(k + 2);
-                    if (!__all_sync(0xffffffffu, ptx::mbar_wait_a(tfull0 + 8u * buf, bpar, abort_flag))) {
+                    if (!__all_sync(0xffffffffu, ptx::mbar_wait_a<kMe>(tfull0 + 8u * buf, bpar, abort_flag))) {
                         report(abort_flag, (3u << 8) | 2u);
                         ok = false;
                         break;

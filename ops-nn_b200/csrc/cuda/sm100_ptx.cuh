@@ -82,6 +82,8 @@ __device__ __forceinline__ bool mbar_try_wait_a(uint32_t bar_addr, uint32_t pari
                  : "memory");
     return ok != 0;
 }
+// (kUser: a copy of the out-of-line part for the kernels that name it.)
+template <int kUser = 0>
 static __device__ __noinline__ bool mbar_wait_slow_a(uint32_t bar_addr, uint32_t parity, volatile uint32_t* abort_flag)
 {
     const uint32_t limit = g_spin_limit;
@@ -93,10 +95,11 @@ static __device__ __noinline__ bool mbar_wait_slow_a(uint32_t bar_addr, uint32_t
     return false;
 }
 // Bounded wait whose common case (the phase has completed, or completes within one try_wait) is two instructions.
+template <int kUser = 0>
 __device__ __forceinline__ bool mbar_wait_a(uint32_t bar_addr, uint32_t parity, volatile uint32_t* abort_flag)
 {
     if (mbar_try_wait_a(bar_addr, parity)) return true;
-    return mbar_wait_slow_a(bar_addr, parity, abort_flag);
+    return mbar_wait_slow_a<kUser>(bar_addr, parity, abort_flag);
 }
 __device__ __forceinline__ void mbar_expect_tx_a(uint32_t bar_addr, uint32_t bytes)
 {

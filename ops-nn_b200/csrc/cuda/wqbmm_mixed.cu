@@ -146,7 +146,7 @@ __device__ __forceinline__ bool mix_wait(uint32_t bar_addr, uint32_t parity, vol
         : "=r"(done)
         : "r"(bar_addr), "r"(parity)
         : "memory");
-    return done != 0u || __all_sync(0xffffffffu, ptx::mbar_wait_slow_a(bar_addr, parity, abort_flag));
+    return done != 0u || __all_sync(0xffffffffu, ptx::mbar_wait_slow_a<>(bar_addr, parity, abort_flag));
 }
 // A warp's arrival: one for all its lanes' earlier accesses (predicated: no branch).
 __device__ __forceinline__ void mix_arrive_warp(uint32_t bar_addr, int lane)
