@@ -21,6 +21,9 @@
 // from global memory (32 sectors a load) and to store its row 16 bytes at a time: 180 and 120 of 1117 clocks. A run's scales are in
 // registers before its first k-block: read per k-block, they cost 8 % of the chain. fp8, bf16 out: 4096 x 7168 x 18432 655 -> 600 us,
 // 1024 x 4096 x 7168 51.5 -> 42.5, 512 x 7168 x 4608 27.3 -> 19.5, 2000 x 2048 x 2048 18.4 -> 16.
+// Neither the MMAs nor the TMEM port are the bound: 901 clocks a k-block, 962 (instrumented) without any MMA, 577 - 640 for a skeleton of the same TMEM
+// loads and multiply-adds. Tried besides: products of the scales from the loaders, one k-block an iteration, waits without divergence (878 clocks;
+// 593 / 595 us under the power limit); 32-byte stores from registers (883).
 // Tried: two N = 128 MMAs a k-block on four half buffers (57 us at 1024 x 4096 x 7168), 32 columns a TMEM load (spills, 54 us).
 namespace {
 
