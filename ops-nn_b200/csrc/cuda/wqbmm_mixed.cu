@@ -510,19 +510,21 @@ __device__ __forceinline__ uint32_t mix_parts(uint32_t live) { return (live + 3u
 __device__ __forceinline__ uint32_t mix_share(uint32_t live, uint32_t split) { return (mix_parts(live) + split - 1u) / split; }
 constexpr uint32_t kMixPartBytes = 64u * 16u;
 
-// This CTA's sums (sixteen warps) to their owners.
+// This CTA's sums (sixteen warps) to their owners. Within a part they lie in the order of the TMEM lanes (`lane`, of 128) and not of the columns, which in
+// (k,n) storage are permuted: in their order eight neighbouring lanes met in two of a shared memory's eight 16-byte banks (int4; in four, 8 bits):
+// us, graph replay, fetched / sent in the columns' order / in the lanes': 128 x 2048 x 12544 int4 15.7 / 16.3 / 15.6, 244 x 2560 x 8544 16.9 / 17.4 / 16.7.
 template <bool kMany>
-__device__ __forceinline__ void mix_push(const MixArgs& a, uint32_t acc, uint32_t n_acc, uint32_t step, uint32_t smem, uint32_t live, uint32_t rank, int col, int share)
+__device__ __forceinline__ void mix_push(const MixArgs& a, uint32_t acc, uint32_t n_acc, uint32_t step, uint32_t smem, uint32_t live, uint32_t rank, uint32_t lane, uint32_t share)
 {
     const uint32_t rows = (uint32_t)a.rows, per = mix_share(live, a.split), inverse = 65535u / per + 1u;  // part * per < 2^16: the quotient is exact
-    const uint32_t mine = smem + rank * per * kMixPartBytes + ((uint32_t)col & 63u) * 16u;
+    const uint32_t mine = smem + rank * per * kMixPartBytes + (lane & 63u) * 16u;
 #pragma unroll 1
     for (uint32_t hc = 16u * share; hc < 2u * rows; hc += 64u) {
         const uint32_t h = hc >= rows ? 1u : 0u, r0 = hc - h * rows;
         if (r0 >= live) continue;
         float f[16];
         mix_sums16<kMany>(acc + hc, n_acc, step, f);
-        uint32_t part = r0 + 2u * h + ((uint32_t)col >> 6), owner = part * inverse >> 16, slot = part - owner * per;
+        uint32_t part = r0 + 2u * h + (lane >> 6), owner = part * inverse >> 16, slot = part - owner * per;
 #pragma unroll
         for (uint32_t i = 0; i < 16; i += 4) {
             if (r0 + i >= live) break;
@@ -535,14 +537,15 @@ __device__ __forceinline__ void mix_push(const MixArgs& a, uint32_t acc, uint32_
 }
 
 // This CTA's share of tile t: the pieces added in their order, + bias (s_bias: the tile's columns), stored (512 threads, one column of four rows each).
-template <bool kBf16>
+template <MixW kW, bool kNK, bool kBf16>
 __device__ __forceinline__ void mix_sum_and_store(const MixArgs& a, uint32_t smem, uint32_t t, uint32_t live, uint32_t rank, uint32_t tid, const float* s_bias)
 {
     const uint32_t tn = t / (uint32_t)a.t_tiles, tt = t - tn * (uint32_t)a.t_tiles, per = mix_share(live, a.split), parts = mix_parts(live);
+    const uint32_t col = (tid & 32u) + (uint32_t)mix_col_of_lane<kW, kNK>((int)(tid & 31u));  // of its part
     uint16_t* out = reinterpret_cast<uint16_t*>(a.y) + (int64_t)(tt * (uint32_t)a.rows) * a.y_ld;
 #pragma unroll 1
     for (uint32_t slot = tid / 64u; slot < per; slot += kMixDqWarps * 32 / 64) {
-        const uint32_t part = rank * per + slot, row = part & ~3u, n = tn * kMixTileN + (part & 3u) * 64u + tid % 64u;
+        const uint32_t part = rank * per + slot, row = part & ~3u, n = tn * kMixTileN + (part & 3u) * 64u + col;
         if (part >= parts || n >= a.n) continue;
         float v[4] = {0.f, 0.f, 0.f, 0.f};
         uint32_t at = smem + slot * kMixPartBytes + tid % 64u * 16u;
@@ -555,7 +558,7 @@ __device__ __forceinline__ void mix_sum_and_store(const MixArgs& a, uint32_t sme
 #pragma unroll
         for (uint32_t r = 0; r < 4; ++r) {
             if (row + r >= live) break;
-            const float f = a.bias != nullptr ? __fadd_rn(v[r], s_bias[(part & 3u) * 64u + tid % 64u]) : v[r];
+            const float f = a.bias != nullptr ? __fadd_rn(v[r], s_bias[(part & 3u) * 64u + col]) : v[r];
             y[(int64_t)r * a.y_ld] = kBf16 ? __bfloat16_as_ushort(__float2bfloat16_rn(f)) : __half_as_ushort(__float2half_rn(f));
         }
     }
@@ -1071,7 +1074,7 @@ wqbmm_mixed_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
             __syncwarp();
             ptx::cluster_arrive();
             ptx::cluster_wait();
-            mix_push<kMany>(a, acc, n_acc, step, smem0, rows_live(), ptx::cluster_ctarank(), col, warp >> 2);
+            mix_push<kMany>(a, acc, n_acc, step, smem0, rows_live(), ptx::cluster_ctarank(), (uint32_t)(qd * 32 + lane), (uint32_t)warp >> 2);
         } else if (mix_all_ok<2, kMixDqWarps * 32>(ok)) {
             ptx::tc_fence_after();
             mix_finish<kBf16, 16, kMany>(a, acc, n_acc, step, t_last, last_cnt, col, qd, lane, warp >> 2, threadIdx.x == 0, &s_last[1], abort_flag);
@@ -1149,7 +1152,7 @@ wqbmm_mixed_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
         ptx::cluster_arrive();
         ptx::cluster_wait();
         // (nobody reaches into another CTA's shared memory from here on: they leave when they are done)
-        if (warp < kMixDqWarps && s_bad == 0u) mix_sum_and_store<kBf16>(a, smem0, blockIdx.x / a.split, rows_live(), ptx::cluster_ctarank(), threadIdx.x, s_bias);
+        if (warp < kMixDqWarps && s_bad == 0u) mix_sum_and_store<kW, kNK, kBf16>(a, smem0, blockIdx.x / a.split, rows_live(), ptx::cluster_ctarank(), threadIdx.x, s_bias);
     }
     // ---- teardown: everyone meets here, also after an aborted wait; then the allocating warp frees TMEM ----
     if (*abort_flag != 0u) __nanosleep(200000);  // lets bulk copies that are still in flight land before the CTA leaves

@@ -156,3 +156,26 @@ def check_close(got, want, ref32, out_name, exact=False, floor_rms=1e-3):
     tol = 1e-2 if out_name == "bfloat16" else 5e-3
     assert frac >= 0.999 and rel.max() <= tol, "isclose fraction %.5f (need 0.999), max rel err vs fp32 product %.3g (tol %g)" % (
         frac, rel.max() if rel.size else 0.0, tol)
+
+
+def least_times(calls, replays=20, per_graph=20):
+    """{name: call} -> {name: ms}: each call captured `per_graph` times into a graph of its own (after one run), the graphs replayed in turn, the
+    least of `replays`."""
+    graphs = {}
+    for name, call in calls.items():
+        call()
+        torch.cuda.synchronize()
+        graphs[name] = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(graphs[name]):
+            for _ in range(per_graph):
+                call()
+    times = {name: [] for name in calls}
+    for _ in range(replays):
+        for name, graph in graphs.items():
+            t0, t1 = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
+            t0.record()
+            graph.replay()
+            t1.record()
+            torch.cuda.synchronize()
+            times[name].append(t0.elapsed_time(t1))
+    return {name: min(t) for name, t in times.items()}
