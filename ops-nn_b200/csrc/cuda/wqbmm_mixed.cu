@@ -513,13 +513,18 @@ constexpr uint32_t kMixPartBytes = 64u * 16u;
 // This CTA's sums (sixteen warps) to their owners. Within a part they lie in the order of the TMEM lanes (`lane`, of 128) and not of the columns, which in
 // (k,n) storage are permuted: in their order eight neighbouring lanes met in two of a shared memory's eight 16-byte banks (int4; in four, 8 bits):
 // us, graph replay, fetched / sent in the columns' order / in the lanes': 128 x 2048 x 12544 int4 15.7 / 16.3 / 15.6, 244 x 2560 x 8544 16.9 / 17.4 / 16.7.
+// Each CTA begins a quarter of its sums further on than the one before it: all beginning with the first rows, they were all sending to the same
+// few owners. fetched / from the first / further on and with four pieces on their way to an owner's registers instead of two: 128 rows, eight pieces,
+// 2048 x 4608 int4 12.8 / 13.0 / 12.2, seven, 339 x 1408 x 1696 11.9 / 12.2 / 11.4, five, 2048 x 7424 12.7 / 13.4 / 12.8 (112 rows 12.1 / 12.7 / 12.2), fourteen,
+// 2048 x 2560 13.0 / 12.2 / 11.5.
 template <bool kMany>
 __device__ __forceinline__ void mix_push(const MixArgs& a, uint32_t acc, uint32_t n_acc, uint32_t step, uint32_t smem, uint32_t live, uint32_t rank, uint32_t lane, uint32_t share)
 {
     const uint32_t rows = (uint32_t)a.rows, per = mix_share(live, a.split), inverse = 65535u / per + 1u;  // part * per < 2^16: the quotient is exact
     const uint32_t mine = smem + rank * per * kMixPartBytes + (lane & 63u) * 16u;
 #pragma unroll 1
-    for (uint32_t hc = 16u * share; hc < 2u * rows; hc += 64u) {
+    for (uint32_t left = (2u * rows + 48u - 16u * share) / 64u, hc = 16u * share + 64u * (rank & 3u); left != 0u; --left, hc += 64u) {
+        if (hc >= 2u * rows) hc = 16u * share;  // (round to the first)
         const uint32_t h = hc >= rows ? 1u : 0u, r0 = hc - h * rows;
         if (r0 >= live) continue;
         float f[16];
@@ -549,7 +554,7 @@ __device__ __forceinline__ void mix_sum_and_store(const MixArgs& a, uint32_t sme
         if (part >= parts || n >= a.n) continue;
         float v[4] = {0.f, 0.f, 0.f, 0.f};
         uint32_t at = smem + slot * kMixPartBytes + tid % 64u * 16u;
-#pragma unroll 2
+#pragma unroll 4
         for (uint32_t j = 0; j < a.split; ++j, at += per * kMixPartBytes) {
             const uint4 q = mix_lds128(at);
             v[0] += __uint_as_float(q.x); v[1] += __uint_as_float(q.y); v[2] += __uint_as_float(q.z); v[3] += __uint_as_float(q.w);
