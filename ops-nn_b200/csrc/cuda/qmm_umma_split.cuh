@@ -306,17 +306,21 @@ __device__ __forceinline__ void split_finish(const SplitArgs& a, uint32_t t, uin
     }
 }
 
-// kAcc: sums one epilogue thread keeps in registers (per-block mode), at least the rows of x that it serves.
-template <ptx::MmaKind kKind, bool kPerBlock, int kAcc, uint32_t kHalves>
+// kAcc: sums one epilogue thread keeps in registers (per-block mode), at least the rows of x that it serves. kOrder: how x2 is stored.
+constexpr int kOrderAny = 0, kOrderKN = 1, kOrderNK = 2;
+template <ptx::MmaKind kKind, bool kPerBlock, int kAcc, uint32_t kHalves, int kOrder>
 __global__ void __launch_bounds__(kSplitThreads, 1)
 qmm_umma_split_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUtensorMap map_x, const __grid_constant__ SplitArgs a)
 {
     extern __shared__ uint8_t smem_raw[];
-    // The dequant instances have the out-of-line part of their waits for themselves. Shared by all kernels of the file it is compiled to a convention that all
-    // of them can live with, and these, whose chain of waits is most of a call, lost 5 - 10 %. us, graph replay, shared / own: 128 x 4096 x 4096 int8
-    // 9.81 / 9.03, 717 x 7168 x 2304 fp8 18.6 / 18.0, 14 x 8640 x 6048 fp8 17.5 / 15.7, 300 x 4096 x 2048 int8 11.1 / 10.2, 32 x 4096 x 3072 fp8 7.38 / 6.80.
-    // (Per-block 15 x 11136 x 8768 22.5 / 22.7; the fused weight-only, pair and block-scaled kernels do not change.)
-    constexpr int kMe = kPerBlock ? 0 : 1 + (int)kKind * 2 + (int)kHalves;
+    // The out-of-line part of the waits, shared by all kernels of the file, is compiled to a convention that all of them can live with. Where the chain of
+    // waits is most of a call it is worth a copy for the instance alone: us, graph replay, weights from HBM, shared / own, 128 x 4096 x 4096 int8 10.6 / 9.9,
+    // 717 x 7168 x 2304 fp8 18.7 / 17.2, 14 x 8640 x 6048 fp8 17.9 / 16.0, 300 x 4096 x 2048 int8 11.6 / 10.8; per-block on weights stored (n,k)
+    // 5 x 8320 x 14080 27.6 / 24.9, 14 x 4480 x 15872 17.3 / 16.2, 24 x 7168 x 18432 25.4 / 25.3. Per-block on (k,n) it is not: 16 x 10368 x 3584 15.3 / 14.8, but
+    // 5 x 8320 x 14080 28.3 / 28.8, 14 x 4480 x 15872 18.9 / 19.1, 100 x 7168 x 4096 15.9 / 16.2. That is why the order is a template argument there.
+    // (The fused weight-only, pair and block-scaled kernels do not change.)
+    constexpr int kMe = !kPerBlock ? 1 + (int)kKind * 2 + (int)kHalves : (kOrder == kOrderNK ? 20 + kAcc + (int)kHalves : 0);
+    const bool w_mn = kOrder == kOrderAny ? a.w_mn != 0u : kOrder == kOrderKN;
     const uint32_t smem0 = (ptx::smem_u32(smem_raw) + 1023u) & ~1023u;
     __shared__ __align__(8) uint64_t s_bars[2 * kSplitMaxStages + 8];
     __shared__ uint32_t s_tmem;
@@ -373,7 +377,7 @@ qmm_umma_split_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_co
         // One warp with nothing to hide latency behind: everything the loop uses is in registers (with the launch parameters read where
         // they are used, a k-block cost this warp and the next 0.6 us each, more than its copies and its MMAs).
         const uint32_t stages = a.stages, stage_bytes = a.stage_bytes, x_off = a.x_off, kbs = a.kb, bytes = kHalves * kATile + a.rows * BK;
-        const bool w_mn = a.w_mn != 0, w_batched = a.w_batched != 0, x_batched = a.x_batched != 0;
+        const bool w_batched = a.w_batched != 0, x_batched = a.x_batched != 0;
         uint32_t s = 0, par = 0, t = u_begin / kbs, kb = u_begin - t * kbs;
         SplitTile tile = split_tile(a, t);
         const uint32_t u_stop = u_begin + min(u_end - u_begin, a.test_stop);
@@ -402,9 +406,9 @@ qmm_umma_split_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_co
         }
     } else if (warp == 9) {
         // ======================= MMA issuer =======================
-        const uint64_t dw = a.w_mn ? ptx::make_smem_desc(smem0, 128 * BK, 1024, 2) : ptx::make_smem_desc(smem0, 0, 1024, 2);
+        const uint64_t dw = w_mn ? ptx::make_smem_desc(smem0, 128 * BK, 1024, 2) : ptx::make_smem_desc(smem0, 0, 1024, 2);
         const uint64_t dx = ptx::make_smem_desc(smem0 + a.x_off, 0, 1024, 2);
-        const uint32_t w_lo = (uint32_t)dw, x_lo = (uint32_t)dx, w_k = a.w_mn ? 256u : 2u;
+        const uint32_t w_lo = (uint32_t)dw, x_lo = (uint32_t)dx, w_k = w_mn ? 256u : 2u;
         const uint64_t w_hi = dw & 0xFFFFFFFF00000000ull, x_hi = dx & 0xFFFFFFFF00000000ull;
         const uint32_t stages = a.stages, stage16 = a.stage_bytes >> 4, rows = a.rows, idesc = a.idesc, kbs = a.kb, dbufs = a.dbufs;
         uint32_t s = 0, par = 0, off = 0, buf = 0, bpar = 0, kb = u_begin % kbs;
@@ -713,23 +717,23 @@ SplitPlan split_candidate(const OpsnnQmmParams* p, uint32_t halves, uint32_t mor
 }
 
 template <ptx::MmaKind kKind, uint32_t kHalves>
-SplitKernel split_kernel_of(bool per_block, int acc)
+SplitKernel split_kernel_of(bool per_block, int acc, bool w_mn)
 {
     if constexpr (kKind == ptx::MmaKind::kF8F6F4) {
         if (per_block) {
-            if (acc == 32) return &qmm_umma_split_kernel<kKind, true, 32, kHalves>;
-            return &qmm_umma_split_kernel<kKind, true, 64, kHalves>;
+            if (acc == 32) return w_mn ? &qmm_umma_split_kernel<kKind, true, 32, kHalves, kOrderKN> : &qmm_umma_split_kernel<kKind, true, 32, kHalves, kOrderNK>;
+            return w_mn ? &qmm_umma_split_kernel<kKind, true, 64, kHalves, kOrderKN> : &qmm_umma_split_kernel<kKind, true, 64, kHalves, kOrderNK>;
         }
     }
-    return &qmm_umma_split_kernel<kKind, false, 16, kHalves>;
+    return &qmm_umma_split_kernel<kKind, false, 16, kHalves, kOrderAny>;
 }
 // The kernel of a plan, ready to launch on the current device; nullptr when it cannot be made ready.
-SplitKernel split_kernel(bool i8, bool per_block, const SplitPlan& q)
+SplitKernel split_kernel(bool i8, bool per_block, bool w_mn, const SplitPlan& q)
 {
-    const SplitKernel k = i8 ? (q.halves == 2 ? split_kernel_of<ptx::MmaKind::kI8, 2>(per_block, q.acc) : split_kernel_of<ptx::MmaKind::kI8, 1>(per_block, q.acc))
-                             : (q.halves == 2 ? split_kernel_of<ptx::MmaKind::kF8F6F4, 2>(per_block, q.acc) : split_kernel_of<ptx::MmaKind::kF8F6F4, 1>(per_block, q.acc));
+    const SplitKernel k = i8 ? (q.halves == 2 ? split_kernel_of<ptx::MmaKind::kI8, 2>(per_block, q.acc, w_mn) : split_kernel_of<ptx::MmaKind::kI8, 1>(per_block, q.acc, w_mn))
+                             : (q.halves == 2 ? split_kernel_of<ptx::MmaKind::kF8F6F4, 2>(per_block, q.acc, w_mn) : split_kernel_of<ptx::MmaKind::kF8F6F4, 1>(per_block, q.acc, w_mn));
     static std::atomic<uint64_t> configured[16];
-    const int index = (q.halves == 2 ? 8 : 0) + (i8 ? 0 : (!per_block ? 1 : (q.acc == 32 ? 2 : 3)));
+    const int index = (q.halves == 2 ? 8 : 0) + (i8 ? 0 : (!per_block ? 1 : (q.acc == 32 ? 2 : 4) + (w_mn ? 1 : 0)));
     const cudaError_t rc = once_per_device(configured[index], [&] {
         cudaFuncSetAttribute(k, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
         return cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, kSplitSmem);
@@ -749,7 +753,7 @@ cudaError_t split_prepare(const OpsnnQmmParams* p, SplitKernel* kern, SplitPlan*
         const uint32_t halves = 2u - (c & 1u);
         if (only != nullptr && atoi(only) != (int)halves) continue;
         const SplitPlan q = split_candidate(p, halves, c >> 1, sms, plan->cost, [&](const SplitPlan& c, int s) -> int {
-            const SplitKernel k = have_device ? split_kernel(i8, pb, c) : nullptr;
+            const SplitKernel k = have_device ? split_kernel(i8, pb, p->trans_b == 0, c) : nullptr;
             return k == nullptr ? 0 : max_active_clusters(reinterpret_cast<const void*>(k), kSplitThreads, kSplitSmem, s, 0);
         });
         if (q.grid != 0 && q.cost < plan->cost) *plan = q;
@@ -757,7 +761,7 @@ cudaError_t split_prepare(const OpsnnQmmParams* p, SplitKernel* kern, SplitPlan*
     if (plan->grid == 0) return cudaErrorNotSupported;
     *kern = nullptr;
     if (!have_device) return cudaErrorNoDevice;
-    *kern = split_kernel(i8, pb, *plan);
+    *kern = split_kernel(i8, pb, p->trans_b == 0, *plan);
     return *kern != nullptr ? cudaSuccess : cudaGetLastError();
 }
 

@@ -44,12 +44,26 @@ CASES = [
 
 @pytest.mark.parametrize("case", CASES, ids=[str(c) for c in CASES])
 def test_split_kernel_equals_oracle(aclnn, monkeypatch, case):
+    monkeypatch.setenv("OPSNN_QMM_SPLIT", "1")
+    _against_oracle(aclnn, case)
+
+
+@pytest.mark.parametrize("halves", ["1", "2"])
+@pytest.mark.parametrize("nk", [False, True])
+@pytest.mark.parametrize("m,k,n", [(9, 4224, 1168), (50, 2176, 1296), (127, 1216, 400)])
+def test_per_block_instances(aclnn, monkeypatch, m, k, n, nk, halves):
+    """The instances of the per-block form: x2 in either order, 256 and 128 columns a tile, 32 and 64 sums a thread."""
+    monkeypatch.setenv("OPSNN_QMM_SPLIT", "1")
+    monkeypatch.setenv("OPSNN_QMM_SPLIT_HALVES", halves)
+    _against_oracle(aclnn, ("block", (), m, k, n, nk, None, "bfloat16"))
+
+
+def _against_oracle(aclnn, case):
     import torch
 
     from gpu_util import check_close, desc, out_tensor, out_to_np
 
     mode, batch, m, k, n, nk, bias_kind, out_name = case
-    monkeypatch.setenv("OPSNN_QMM_SPLIT", "1")
     rng = np.random.default_rng(case_seed(case))
     if mode == "int8":
         x1 = rng.integers(-127, 128, batch + (m, k), dtype=np.int8)
@@ -127,3 +141,33 @@ def test_wait_that_runs_out_ends_the_call(aclnn, monkeypatch, mode, m, k, n):
     assert (code >> 8) in (2, 3), hex(code)
     assert bool((bad == -7777.0).all())
     assert torch.equal(run(), want) and status(1) == 0
+
+
+def test_per_block_on_weights_stored_along_k(aclnn):
+    """Few rows and a long k: the waits of the instances for x2 stored (n,k) gain by an out-of-line part of their own (with the one that all kernels
+    of the file share such a call took as long as on (k,n), with its own 0.92 times). Up to five attempts, for a GPU whose clock moves."""
+    import torch
+
+    from gpu_util import DEV, least_times
+
+    m, k, n = 9, 8448, 6144
+    gen = torch.Generator(device=DEV).manual_seed(12)
+    x = torch.randn((m, k), generator=gen, device=DEV).to(torch.float8_e4m3fn)
+    s1 = torch.rand((m, k // 128), generator=gen, device=DEV)
+    calls = {}
+    for nk in (True, False):
+        w = torch.randn((n, k) if nk else (k, n), generator=gen, device=DEV).to(torch.float8_e4m3fn)
+        s2 = torch.rand((n // 128, k // 128) if nk else (k // 128, n // 128), generator=gen, device=DEV)
+        y = torch.empty((m, n), dtype=torch.bfloat16, device=DEV)
+        d = [aclnn.from_torch(t) for t in (x, w, s1, s2, y)]
+        group = (1 << 32) | (128 << 16) | 128
+        ws = torch.empty(max(1, aclnn.quant_matmul_v5(*d, None, False, nk, group)), dtype=torch.uint8, device=DEV)
+        assert aclnn.last_kernel_name() == "qmm_umma_split_perblock"
+        calls[nk] = lambda d=d, nk=nk, ws=ws, keep=(w, s2, y): aclnn.quant_matmul_v5(*d, None, False, nk, group, workspace=ws)
+    ratios = []
+    for _ in range(5):
+        t = least_times(calls)
+        ratios.append(t[True] / t[False])
+        if ratios[-1] <= 0.96:
+            return
+    assert False, ratios
