@@ -28,7 +28,6 @@ struct SplitArgs {
     uint32_t* part;                // [2 grid][rows][128 halves] raw 32-bit sums
     unsigned long long* count;     // [tiles] (nonce << 8) | arrivals
     unsigned long long nonce;
-    uint32_t push;       // a cluster's sums are sent to their owners (split_push16), not fetched
     uint32_t test_stop;  // tests of the give-up path only: k-blocks that a CTA's producer copies before it stops; otherwise all
 };
 
@@ -306,9 +305,14 @@ __device__ __forceinline__ void split_finish(const SplitArgs& a, uint32_t t, uin
     }
 }
 
-// kAcc: sums one epilogue thread keeps in registers (per-block mode), at least the rows of x that it serves. kOrder: how x2 is stored.
+// kAcc: sums one epilogue thread keeps in registers (per-block mode), at least the rows of x that it serves. kOrder: how x2 is stored (kMe). kForm: how the
+// line is cut and its pieces come together. An instance each: the forms' ends in one kernel cost all of them registers and instruction fetches. us, weights
+// from HBM, one instance / each its own: streams 64 x 384 x 40960 int8 24.2 / 23.6, 60 x 512 x 36864 10.7 / 9.5, 48 x 7168 x 30720 fp8 39.6 / 38.6; fetched
+// 128 x 4096 x 4096 int8 9.9 / 9.7, 717 x 7168 x 2304 fp8 17.5 / 17.1, 300 x 4096 x 2048 int8 10.8 / 10.5; sent 16 x 1472 x 4880 int8 6.2 / 6.1; per-block
+// 128 x 4096 x 4096 12.5 / 12.1, (n,k) 100 x 7168 x 4096 14.6 / 13.9.
 constexpr int kOrderAny = 0, kOrderKN = 1, kOrderNK = 2;
-template <ptx::MmaKind kKind, bool kPerBlock, int kAcc, uint32_t kHalves, int kOrder>
+constexpr int kFormStream = 1, kFormFetch = 2, kFormPush = 3;  // kFormFetch: also one piece a tile
+template <ptx::MmaKind kKind, bool kPerBlock, int kAcc, uint32_t kHalves, int kOrder, int kForm>
 __global__ void __launch_bounds__(kSplitThreads, 1)
 qmm_umma_split_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUtensorMap map_x, const __grid_constant__ SplitArgs a)
 {
@@ -319,7 +323,7 @@ qmm_umma_split_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_co
     // 5 x 8320 x 14080 27.6 / 24.9, 14 x 4480 x 15872 17.3 / 16.2, 24 x 7168 x 18432 25.4 / 25.3. Per-block on (k,n) it is not: 16 x 10368 x 3584 15.3 / 14.8, but
     // 5 x 8320 x 14080 28.3 / 28.8, 14 x 4480 x 15872 18.9 / 19.1, 100 x 7168 x 4096 15.9 / 16.2. That is why the order is a template argument there.
     // (The fused weight-only, pair and block-scaled kernels do not change.)
-    constexpr int kMe = !kPerBlock ? 1 + (int)kKind * 2 + (int)kHalves : (kOrder == kOrderNK ? 20 + kAcc + (int)kHalves : 0);
+    constexpr int kMe = !kPerBlock ? 100 * kForm + (int)kKind * 2 + (int)kHalves : (kOrder == kOrderNK ? 1000 * kForm + kAcc + (int)kHalves : 0);
     const bool w_mn = kOrder == kOrderAny ? a.w_mn != 0u : kOrder == kOrderKN;
     const uint32_t smem0 = (ptx::smem_u32(smem_raw) + 1023u) & ~1023u;
     __shared__ __align__(8) uint64_t s_bars[2 * kSplitMaxStages + 8];
@@ -359,10 +363,11 @@ qmm_umma_split_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_co
 
     const uint32_t u_begin = split_begin(a, blockIdx.x), u_end = split_begin(a, blockIdx.x + 1);
     SplitCols4 cols4;  // (per-block: only a bias, read at the end; 16 registers the sums need)
-    const bool push = !kPerBlock && a.push != 0u;
+    constexpr bool push = kForm == kFormPush;  // a cluster's sums are sent to their owners (split_push16), not fetched
+    constexpr bool stream = kForm == kFormStream;
     SplitCol own{1.f, 0.f, 0};  // push: of the column that this thread serves in the end
     bool met = false;           // push: this warp has met the cluster's others at the end of the stages
-    if (warp < 8 && a.split != 0u) {
+    if (warp < 8 && !stream) {
         const SplitTile tile = split_tile(a, blockIdx.x / a.split);
         if constexpr (!kPerBlock) {
             if (push) own = split_col<false>(a, tile.b, min((int64_t)tile.n0 + threadIdx.x % (128u * kHalves), a.n - 1));
@@ -562,7 +567,9 @@ qmm_umma_split_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_co
                     ptx::tmem_ld_wait();
                 }
             };
-            if (push) {
+            if (stream) {
+                split_finish<kPerBlock>(a, t, cnt, cnt_rows, row0, col, threadIdx.x == 0, &s_last, abort_flag, get);
+            } else if (push) {
                 // where every CTA of the cluster is done with its stages, the sums go to their owners
                 const uint32_t live = split_tile(a, t).live;
                 __syncwarp();
@@ -575,10 +582,11 @@ qmm_umma_split_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_co
                     get(i, v);
                     split_push16<kHalves>(smem0, live, a.split, ptx::cluster_ctarank(), row0 + i, col, v);
                 }
-            } else if (a.split != 0u) {
+            } else {
                 // the tile's only piece here: into shared memory (no copy is in flight any more), as [row of x][column]
-                const uint32_t width = 128u * a.halves;
-#pragma unroll
+                constexpr uint32_t width = 128u * kHalves;
+                constexpr int kUnroll = kPerBlock ? 8 : 1;  // (per-block: its sums are registers)
+#pragma unroll kUnroll
                 for (uint32_t i = 0; i < 128; i += 16) {
                     if (i >= cnt_rows) break;
                     uint32_t v[16];
@@ -592,8 +600,6 @@ qmm_umma_split_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_co
                     if constexpr (kPerBlock) cols4 = split_cols4<kPerBlock, kHalves>(a, split_tile(a, t), threadIdx.x);
                     split_sum_and_store<kPerBlock, kHalves>(a, smem0, split_tile(a, t), 0u, threadIdx.x, s_sa, cols4);
                 }
-            } else {
-                split_finish<kPerBlock>(a, t, cnt, cnt_rows, row0, col, threadIdx.x == 0, &s_last, abort_flag, get);
             }
             if (!kPerBlock) {
                 ptx::tc_fence_before();
@@ -621,7 +627,7 @@ qmm_umma_split_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_co
         ptx::cluster_arrive();
         ptx::cluster_wait();
         if (warp < 8 && s_bad == 0u) split_sum_fours<kHalves>(a, smem0, split_tile(a, blockIdx.x / a.split), ptx::cluster_ctarank(), threadIdx.x, s_sa, own);
-    } else if (a.split > 1u) {
+    } else if (!stream && a.split > 1u) {
         // the pieces of the tile meet; a CTA that gave up a wait still joins both barriers, and then nobody writes
         __syncwarp();
         ptx::cluster_sync();
@@ -716,29 +722,50 @@ SplitPlan split_candidate(const OpsnnQmmParams* p, uint32_t halves, uint32_t mor
     return q;
 }
 
+template <uint32_t kHalves, int kOrder, int kForm>
+SplitKernel split_per_block(int acc)
+{
+    if (acc == 32) return &qmm_umma_split_kernel<ptx::MmaKind::kF8F6F4, true, 32, kHalves, kOrder, kForm>;
+    return &qmm_umma_split_kernel<ptx::MmaKind::kF8F6F4, true, 64, kHalves, kOrder, kForm>;
+}
 template <ptx::MmaKind kKind, uint32_t kHalves>
-SplitKernel split_kernel_of(bool per_block, int acc, bool w_mn)
+SplitKernel split_kernel_of(bool per_block, int acc, bool w_mn, int form)
 {
     if constexpr (kKind == ptx::MmaKind::kF8F6F4) {
         if (per_block) {
-            if (acc == 32) return w_mn ? &qmm_umma_split_kernel<kKind, true, 32, kHalves, kOrderKN> : &qmm_umma_split_kernel<kKind, true, 32, kHalves, kOrderNK>;
-            return w_mn ? &qmm_umma_split_kernel<kKind, true, 64, kHalves, kOrderKN> : &qmm_umma_split_kernel<kKind, true, 64, kHalves, kOrderNK>;
+            if (form == kFormStream) return w_mn ? split_per_block<kHalves, kOrderKN, kFormStream>(acc) : split_per_block<kHalves, kOrderNK, kFormStream>(acc);
+            return w_mn ? split_per_block<kHalves, kOrderKN, kFormFetch>(acc) : split_per_block<kHalves, kOrderNK, kFormFetch>(acc);
         }
     }
-    return &qmm_umma_split_kernel<kKind, false, 16, kHalves, kOrderAny>;
+    if (form == kFormPush) return &qmm_umma_split_kernel<kKind, false, 16, kHalves, kOrderAny, kFormPush>;
+    if (form == kFormStream) return &qmm_umma_split_kernel<kKind, false, 16, kHalves, kOrderAny, kFormStream>;
+    return &qmm_umma_split_kernel<kKind, false, 16, kHalves, kOrderAny, kFormFetch>;
 }
 // The kernel of a plan, ready to launch on the current device; nullptr when it cannot be made ready.
-SplitKernel split_kernel(bool i8, bool per_block, bool w_mn, const SplitPlan& q)
+SplitKernel split_kernel(bool i8, bool per_block, bool w_mn, const SplitPlan& q, int form)
 {
-    const SplitKernel k = i8 ? (q.halves == 2 ? split_kernel_of<ptx::MmaKind::kI8, 2>(per_block, q.acc, w_mn) : split_kernel_of<ptx::MmaKind::kI8, 1>(per_block, q.acc, w_mn))
-                             : (q.halves == 2 ? split_kernel_of<ptx::MmaKind::kF8F6F4, 2>(per_block, q.acc, w_mn) : split_kernel_of<ptx::MmaKind::kF8F6F4, 1>(per_block, q.acc, w_mn));
-    static std::atomic<uint64_t> configured[16];
-    const int index = (q.halves == 2 ? 8 : 0) + (i8 ? 0 : (!per_block ? 1 : (q.acc == 32 ? 2 : 4) + (w_mn ? 1 : 0)));
+    const SplitKernel k = i8 ? (q.halves == 2 ? split_kernel_of<ptx::MmaKind::kI8, 2>(per_block, q.acc, w_mn, form) : split_kernel_of<ptx::MmaKind::kI8, 1>(per_block, q.acc, w_mn, form))
+                             : (q.halves == 2 ? split_kernel_of<ptx::MmaKind::kF8F6F4, 2>(per_block, q.acc, w_mn, form) : split_kernel_of<ptx::MmaKind::kF8F6F4, 1>(per_block, q.acc, w_mn, form));
+    static std::atomic<uint64_t> configured[2 * 14];
+    const int index = (q.halves == 2 ? 14 : 0) + (!per_block ? (i8 ? 0 : 3) + form - 1 : 6 + (q.acc == 32 ? 0 : 4) + (w_mn ? 2 : 0) + form - 1);
     const cudaError_t rc = once_per_device(configured[index], [&] {
         cudaFuncSetAttribute(k, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
         return cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, kSplitSmem);
     });
     return rc == cudaSuccess ? k : nullptr;
+}
+
+// Sent or fetched: a column of four rows at a time is summed with less code and fewer waits, but by 256 threads whose stores are two bytes wide; up to four
+// fours a thread it is the faster. us, graph replay, weights from HBM, fetched / sent, where it is sent: 16 x 1472 x 4880 int8 6.65 / 6.07, 24 x 7168 x 384 7.82 /
+// 6.89, 32 x 4096 x 3072 fp8 8.53 / 8.06, 64 x 4096 x 3072 8.91 / 8.87, 83 x 4096 x 3072 int8 8.96 / 8.78, 200 x 4096 x 1024 8.96 / 7.79 (14 x 8640 x 6048 fp8 15.70 /
+// 15.86); where it is fetched: 96 x 4096 x 4096 int8 9.78 / 10.25, 128 rows 9.92 / 10.35, 300 x 4096 x 2048 10.46 / 11.18, 717 x 7168 x 2304 fp8 16.9 / 18.9.
+// Per-block, whose sums are in registers, it is 3 - 6 % slower at 14 and 100 rows.
+int split_form(const OpsnnQmmParams* p, const SplitPlan& q)
+{
+    if (q.split == 0) return kFormStream;
+    if (p->mode == OPSNN_QMM_PERBLOCK) return kFormFetch;
+    if (const char* e = env("OPSNN_QMM_SPLIT_PUSH")) return q.split > 1u && atoi(e) != 0 ? kFormPush : kFormFetch;  // tests and experiments (any share fits)
+    return q.split > 1u && split_share(std::min(q.rows, (uint32_t)p->m), q.split) * q.halves <= 4u ? kFormPush : kFormFetch;
 }
 
 cudaError_t split_prepare(const OpsnnQmmParams* p, SplitKernel* kern, SplitPlan* plan)
@@ -753,7 +780,7 @@ cudaError_t split_prepare(const OpsnnQmmParams* p, SplitKernel* kern, SplitPlan*
         const uint32_t halves = 2u - (c & 1u);
         if (only != nullptr && atoi(only) != (int)halves) continue;
         const SplitPlan q = split_candidate(p, halves, c >> 1, sms, plan->cost, [&](const SplitPlan& c, int s) -> int {
-            const SplitKernel k = have_device ? split_kernel(i8, pb, p->trans_b == 0, c) : nullptr;
+            const SplitKernel k = have_device ? split_kernel(i8, pb, p->trans_b == 0, c, kFormFetch) : nullptr;  // (clusters of all forms are placed alike)
             return k == nullptr ? 0 : max_active_clusters(reinterpret_cast<const void*>(k), kSplitThreads, kSplitSmem, s, 0);
         });
         if (q.grid != 0 && q.cost < plan->cost) *plan = q;
@@ -761,7 +788,7 @@ cudaError_t split_prepare(const OpsnnQmmParams* p, SplitKernel* kern, SplitPlan*
     if (plan->grid == 0) return cudaErrorNotSupported;
     *kern = nullptr;
     if (!have_device) return cudaErrorNoDevice;
-    *kern = split_kernel(i8, pb, p->trans_b == 0, *plan);
+    *kern = split_kernel(i8, pb, p->trans_b == 0, *plan, split_form(p, *plan));
     return *kern != nullptr ? cudaSuccess : cudaGetLastError();
 }
 
@@ -819,11 +846,6 @@ int32_t split_launch(const OpsnnQmmParams* p, SplitChoice& choice, cudaStream_t 
         a.count = reinterpret_cast<unsigned long long*>(ws);
         a.part = reinterpret_cast<uint32_t*>(ws + (((uint64_t)q.tiles * 8u + 255u) & ~(uint64_t)255u));
     }
-    // Sent or fetched: a column of four rows at a time is summed with less code and fewer waits, but by 256 threads whose stores are two bytes wide.
-    // us, graph replay, fetched / sent, by the fours that a thread sums: one, 16 x 1472 x 4880 int8 5.85 / 5.21, 32 x 4096 x 3072 fp8 7.70 / 6.79;
-    // two, 64 x 4096 x 3072 8.23 / 8.05, 64 x 2048 x 4096 int8 6.56 / 6.28; four, 128 x 4096 x 4096 int8 8.98 / 9.27; twelve, 717 x 7168 x 2304 fp8
-    // 16.8 / 19.7. Per-block, whose sums are in registers, it is 3 - 6 % slower at 14 and 100 rows.
-    a.push = !pb && q.split > 1u && split_share(std::min(q.rows, a.m), q.split) * q.halves <= 4u ? 1u : 0u;
     a.nonce = next_ks_nonce();
     a.test_stop = 0xFFFFFFFFu;
     if (const char* e = env("OPSNN_TEST_SPLIT_STALL_KBLOCK")) {  // tests of the give-up path only

@@ -26,8 +26,7 @@ CASES = [
     ("block", (), 48, 1152, 20096, False, None, "float16"),    # per-block, a tile a CTA
     ("block", (), 100, 3072, 640, True, None, "float32"),
     ("block", (3,), 20, 1088, 320, True, None, "bfloat16"),    # last k-block half full
-    # a cluster's sums sent to their owners: rows that fours and owners do not divide, fewer fours than owners, one and two fours a thread, and the
-    # first sizes past them, where they are fetched
+    # a cluster's sums sent to their owners: rows that fours and owners do not divide, fewer fours than owners, one to four fours a thread
     ("fp8", (), 5, 1472, 1296, False, "f32", "float32"),
     ("int8", (), 30, 4096, 3088, True, "f32", "bfloat16"),
     # (bf16: these outputs are 1e-3 and less, and half a unit of fp16's subnormals, 3e-8, is 2 % of check_close's floor of 1.5e-6)
@@ -56,6 +55,28 @@ def test_per_block_instances(aclnn, monkeypatch, m, k, n, nk, halves):
     monkeypatch.setenv("OPSNN_QMM_SPLIT", "1")
     monkeypatch.setenv("OPSNN_QMM_SPLIT_HALVES", halves)
     _against_oracle(aclnn, ("block", (), m, k, n, nk, None, "bfloat16"))
+
+
+@pytest.mark.parametrize("case", [
+    # mode, batch, m, k, n, x2 stored (n,k), bias, out
+    ("fp8", (), 5, 1472, 1296, False, "f32", "float32"),
+    ("int8", (), 30, 4096, 3088, True, "f32", "bfloat16"),
+    ("int8", (), 83, 4096, 3072, True, "i32", "bfloat16"),
+    ("int8", (2,), 21, 3072, 400, False, None, "bfloat16"),
+    ("int8", (), 128, 4096, 4096, True, None, "bfloat16"),
+    ("fp8", (), 250, 2048, 528, True, None, "float32"),
+    ("int8", (), 130, 4112, 272, True, "i32", "bfloat16"),
+], ids=str)
+@pytest.mark.parametrize("halves", ["1", "2"])
+def test_sums_of_a_cluster_sent_or_fetched(aclnn, monkeypatch, case, halves):
+    """Either way of bringing the pieces of a tile together, at shares that the host would and would not send: the same additions, the same bits."""
+    monkeypatch.setenv("OPSNN_QMM_SPLIT", "1")
+    monkeypatch.setenv("OPSNN_QMM_SPLIT_HALVES", halves)
+    outs = []
+    for push in ("0", "1"):
+        monkeypatch.setenv("OPSNN_QMM_SPLIT_PUSH", push)
+        outs.append(_against_oracle(aclnn, case))
+    assert np.array_equal(outs[0].view(np.uint8), outs[1].view(np.uint8))
 
 
 def _against_oracle(aclnn, case):
@@ -96,13 +117,16 @@ def _against_oracle(aclnn, case):
         assert np.array_equal(outs[0].view(np.uint8), np.asarray(want).view(np.uint8))
     else:
         check_close(outs[0], want, qbmm_oracle.quant_matmul_v5(x1, x2, s1, s2, bias, False, nk, group, "float32"), out_name)
+    return outs[0]
 
 
-@pytest.mark.parametrize("mode,m,k,n", [("int8", 128, 4096, 4096),   # a cluster of pieces
-                                        ("int8", 64, 1024, 40960),   # more tiles than SMs: pieces across tiles
-                                        ("block", 24, 7168, 400),     # per-block, pieces across tiles
-                                        ("block", 24, 2048, 9216)])   # a cluster
-def test_wait_that_runs_out_ends_the_call(aclnn, monkeypatch, mode, m, k, n):
+@pytest.mark.parametrize("mode,m,k,n,push", [("int8", 128, 4096, 4096, None),   # a cluster of pieces, their sums fetched
+                                             ("int8", 64, 1024, 40960, None),   # more tiles than SMs: pieces across tiles
+                                             ("block", 24, 7168, 400, None),     # per-block, pieces across tiles
+                                             ("block", 24, 2048, 9216, None),    # a cluster
+                                             ("int8", 64, 4096, 3072, "1"),      # a cluster's sums sent: two and sixteen pieces a tile
+                                             ("int8", 21, 4096, 512, "1")])
+def test_wait_that_runs_out_ends_the_call(aclnn, monkeypatch, mode, m, k, n, push):
     """The producer stops after its first k-block: every wait behind it runs out, all CTAs of a cluster still meet, nothing is written, later
     calls are refused until the condition is cleared, and then find tensor memory and workspace as they should."""
     import torch
@@ -110,6 +134,8 @@ def test_wait_that_runs_out_ends_the_call(aclnn, monkeypatch, mode, m, k, n):
     from gpu_util import DEV
 
     monkeypatch.setenv("OPSNN_QMM_SPLIT", "1")
+    if push is not None:
+        monkeypatch.setenv("OPSNN_QMM_SPLIT_PUSH", push)
     gen = torch.Generator(device=DEV).manual_seed(6)
     if mode == "int8":
         x, w = (torch.randint(-127, 128, s, generator=gen, device=DEV, dtype=torch.int8) for s in ((m, k), (n, k)))
