@@ -704,21 +704,44 @@ SplitPlan split_candidate(const OpsnnQmmParams* p, uint32_t halves, uint32_t mor
     if (q.stages > (uint32_t)kSplitMaxStages) q.stages = kSplitMaxStages;
     const double area = (double)q.rows * halves;
     q.cost = most_cost;
-    auto consider = [&](int64_t grid, uint32_t split, double extra) {
+    auto cost_of = [&](int64_t grid, double extra) {
         double w = 0.12 + (pb ? 0.0075 * served : 0.00135 * area);
         const double hbm = (double)grid * halves * kATile / q.t_tiles / 5.8e6;  // all CTAs' weights of one k-block
         if (hbm > w) w = hbm;
-        const double cost = 5.5 + (double)((q.units + grid - 1) / grid) * w + extra;
-        if (cost >= q.cost || (split > 1u && (int64_t)clusters(q, (int)split) < q.tiles)) return;
+        return 5.5 + (double)((q.units + grid - 1) / grid) * w + extra;
+    };
+    auto take = [&](int64_t grid, uint32_t split, double cost) {
         q.cost = cost;
         q.grid = grid;
         q.split = split;
     };
-    consider(q.units < sms ? q.units : sms, 0, 1.0 + area * 0.05);
+    const int64_t all = q.units < sms ? q.units : sms;
+    // Whoever arrives last adds a tile's pieces up alone, 0.6 us each: few tiles with a long k are many pieces (us, before / since that was counted:
+    // 8 x 7168 x 512 int8 56.0 / 8.4, 16 x 16384 x 256 fp8 131.6 / 11.4, per-block 24 x 7168 x 384 43.4 / 8.1, 1 x 8192 x 1024 35.5 / 9.0).
+    const double stream = cost_of(all, 1.0 + area * 0.05 + 0.6 * std::max(0.0, (double)q.kb * all / q.units - 4.0));
+    if (stream < q.cost) take(all, 0, stream);
     int64_t most = sms / q.tiles;
     if (most > 16) most = 16;
     if (most > q.kb) most = q.kb;
-    for (int s = (int)most; s >= 1; --s) consider(q.tiles * s, (uint32_t)s, s > 1 ? std::max(0.4, 0.6 * s + 0.012 * area - 1.8) : 0.02 * area);
+    // of the cheapest first, so that one answer is enough nearly always
+    for (uint32_t refused = 0;;) {
+        int best = 0;
+        double cost = q.cost;
+        for (int s = (int)most; s >= 1; --s) {
+            if ((refused >> s) & 1u) continue;
+            const double c = cost_of(q.tiles * s, s > 1 ? std::max(0.4, 0.6 * s + 0.012 * area - 1.8) : 0.02 * area);
+            if (c < cost) {
+                cost = c;
+                best = s;
+            }
+        }
+        if (best == 0) break;
+        if (best == 1 || (int64_t)clusters(q, best) >= q.tiles) {
+            take(q.tiles * best, (uint32_t)best, cost);
+            break;
+        }
+        refused |= 1u << best;
+    }
     return q;
 }
 

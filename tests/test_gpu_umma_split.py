@@ -197,3 +197,32 @@ def test_per_block_on_weights_stored_along_k(aclnn):
         if ratios[-1] <= 0.96:
             return
     assert False, ratios
+
+
+def test_fewer_columns_do_not_take_longer(aclnn):
+    """A stream's pieces of a tile are added up by whoever arrives last: two tiles of 128 k-blocks, cut that way, took nine times as long as eight times
+    the columns; cut into clusters they take less. Up to five attempts, for a GPU whose clock moves between the two."""
+    import torch
+
+    from gpu_util import DEV, least_times
+
+    m, k = 16, 16384
+    gen = torch.Generator(device=DEV).manual_seed(13)
+    x = torch.randn((m, k), generator=gen, device=DEV).to(torch.float8_e4m3fn)
+    s1 = torch.rand(m, generator=gen, device=DEV)
+    calls = {}
+    for n in (256, 2048):
+        w = torch.randn((n, k), generator=gen, device=DEV).to(torch.float8_e4m3fn)
+        s2 = torch.rand(n, generator=gen, device=DEV)
+        y = torch.empty((m, n), dtype=torch.bfloat16, device=DEV)
+        d = [aclnn.from_torch(t) for t in (x, w, s1, s2, y)]
+        ws = torch.empty(max(1, aclnn.quant_matmul_v5(*d, None, False, True)), dtype=torch.uint8, device=DEV)
+        assert aclnn.last_kernel_name() == "qmm_umma_split_deq"
+        calls[n] = lambda d=d, ws=ws, keep=(w, s2, y): aclnn.quant_matmul_v5(*d, None, False, True, workspace=ws)
+    ratios = []
+    for _ in range(5):
+        t = least_times(calls)
+        ratios.append(t[256] / t[2048])
+        if ratios[-1] <= 1.0:
+            return
+    assert False, ratios
