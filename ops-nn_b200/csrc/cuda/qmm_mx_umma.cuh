@@ -423,7 +423,7 @@ qmm_mx_umma_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_const
     const uint32_t tile0 = kSplit ? blockIdx.x / ksplit : blockIdx.x, tile_step = kSplit ? ntiles : gridDim.x;
     const int k_first = kSplit ? (int)((uint32_t)kstages * rank / ksplit) : 0, k_last = kSplit ? (int)((uint32_t)kstages * (rank + 1u) / ksplit) : kstages;
 
-    bool met = false;  // kSplit: this warp has met the cluster's others at the end of the stages
+    [[maybe_unused]] bool met = false;  // kSplit: this warp has met the cluster's others at the end of the stages
     if (warp == EW) {
         // ======================= producer: two TMA loads and two scale-atom bulk copies per stage =======================
         if (lane == 0) {
@@ -434,6 +434,7 @@ qmm_mx_umma_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_const
         uint32_t s = 0, par = 0;
         bool ok = true;
         const bool b_mn = a.b_mn_major != 0, a_mn = a.a_mn_major != 0;
+        const int k_stop = kSplit && a.test_stall_kblock > 0 ? min(k_last, k_first + a.test_stall_kblock) : k_last;  // (tests of the give-up path)
         for (uint32_t tile = tile0; tile < ntiles && ok; tile += tile_step) {
             const uint32_t b = tile / tiles_per_batch, r = tile % tiles_per_batch;
             uint32_t tm, tn;
@@ -445,7 +446,7 @@ qmm_mx_umma_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_const
             // bytes one stage's copies deliver: k-major B is one box of BN rows, n-major B whole 128-column boxes
             const uint32_t tx = (uint32_t)kATile + (b_mn ? kBTile : (uint32_t)(BN * BK)) + kSfaBytes + kSfbBytes;
             int32_t kk = k_first * BK;
-            for (int kb = k_first; kb < k_last; ++kb) {
+            for (int kb = k_first; kb < k_stop; ++kb) {
                 if (!ptx::mbar_wait_a(empty0 + 8u * s, par ^ 1u, abort_flag)) {
                     report(abort_flag, (1u << 8) | 1u);
                     ok = false;
@@ -538,7 +539,6 @@ qmm_mx_umma_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_const
         const uint32_t lane_addr = (uint32_t)(quad * 32) << 16;
         uint32_t grp = 0;
         bool ok = true;
-        (void)met;
         for (uint32_t tile = tile0; tile < ntiles && ok; tile += tile_step) {
             const uint32_t b = tile / tiles_per_batch, r = tile % tiles_per_batch;
             uint32_t tm, tn;
@@ -796,6 +796,12 @@ int32_t mx_launch_split(const CUtensorMap& ma, const CUtensorMap& mb, UmmaArgs& 
     if (split < 2) return -1;
     a.stages = kStages;
     a.ksplit = split;
+    if (const char* e = env("OPSNN_TEST_MX_STALL_STAGE")) {  // tests of the give-up path only: stages that a CTA's producer copies before it stops
+        a.test_stall_kblock = atoi(e);
+        const char* pl = env("OPSNN_TEST_UMMA_POLL_LIMIT");
+        const uint32_t limit = pl != nullptr ? (uint32_t)atoi(pl) : 20000u;
+        cudaMemcpyToSymbolAsync(ptx::g_spin_limit, &limit, sizeof(limit), 0, cudaMemcpyHostToDevice, stream);
+    }
     cudaLaunchConfig_t cfg{};
     cfg.gridDim = dim3((unsigned)(a.num_tiles * split), 1, 1);
     cfg.blockDim = dim3(192, 1, 1);

@@ -19,6 +19,9 @@ CASES = [
     (E4M3, (), 256, 512, 896, True),       # already (n,k): only the scale atoms are prepared
     (E2M1, (), 512, 1024, 1344, False),    # MXFP4 stored (k,n): the transposition the tensor core needs, once
     (E2M1, (2,), 256, 512, 448, True),
+    (E4M3, (), 20, 6144, 640, False),      # few tiles, a long k: the pieces of a tile on the CTAs of a cluster
+    (E4M3, (2,), 9, 6208, 392, True),
+    (E2M1, (), 20, 8192, 640, False),
 ]
 
 

@@ -164,6 +164,54 @@ def test_mx_pieces_of_k_equal_oracle(aclnn, case):
     _check(got[0], _oracle(x1, x2, s1, s2, bias, False, nk, out_name), out_name)
 
 
+@pytest.mark.parametrize("t1,nk,da,db", [(True, True, E4M3, E4M3), (True, False, E4M3, E5M2), (False, False, E5M2, E4M3), (False, True, E5M2, E5M2)])
+def test_mx_pieces_of_k_in_other_orders_and_types(aclnn, t1, nk, da, db):
+    """x1 stored (k,m), e5m2 on either side, k a quarter of a stage past the last."""
+    m, k, n = 48, 6176, 400
+    rng = np.random.default_rng(case_seed((t1, nk, str(da), str(db))))
+    kq = -(-k // 64)
+    x1, x2 = _q(rng, (k, m) if t1 else (m, k), da), _q(rng, (n, k) if nk else (k, n), db)
+    s1, s2 = _e8m0(rng, (kq, m, 2) if t1 else (m, kq, 2)), _e8m0(rng, (n, kq, 2) if nk else (kq, n, 2))
+    got = _run(aclnn, x1, x2, s1, s2, None, t1, nk, "bfloat16", "qmm_umma_mxfp8_split")
+    _check(got, _oracle(x1, x2, s1, s2, None, t1, nk, "bfloat16"), "bfloat16")
+
+
+@pytest.mark.parametrize("f4", [False, True])
+def test_wait_that_runs_out_ends_the_call(aclnn, monkeypatch, f4):
+    """The producers of a tile's pieces stop after their first stage: every wait behind it runs out, all CTAs of a cluster still meet, nothing is
+    written, later calls are refused until the condition is cleared, and then find tensor memory as they should."""
+    import torch
+
+    from gpu_util import desc, out_tensor
+
+    m, k, n = 12, 8192, 1408
+    rng = np.random.default_rng(21)
+    dt, name = (E2M1, "qmm_umma_mxfp4_split") if f4 else (E4M3, "qmm_umma_mxfp8_split")
+    d = [desc(aclnn, a) for a in (_q(rng, (m, k), dt), _q(rng, (n, k), dt), _e8m0(rng, (m, k // 64, 2)), _e8m0(rng, (n, k // 64, 2)))]
+
+    def run():
+        y = out_tensor((m, n), "bfloat16")
+        aclnn.quant_matmul_v5(*d, aclnn.from_torch(y), None, False, True, GROUP_MX)
+        torch.cuda.synchronize()
+        assert aclnn.last_kernel_name() == name
+        return y
+
+    want = run()
+    status = aclnn.lib().opsnn_qmm_umma_status
+    assert status(1) == 0
+    monkeypatch.setenv("OPSNN_TEST_MX_STALL_STAGE", "1")
+    monkeypatch.setenv("OPSNN_TEST_UMMA_POLL_LIMIT", "3000")
+    bad = run()
+    monkeypatch.delenv("OPSNN_TEST_MX_STALL_STAGE")
+    monkeypatch.delenv("OPSNN_TEST_UMMA_POLL_LIMIT")
+    with pytest.raises(aclnn.AclnnError):
+        run()
+    code = status(1)  # read and cleared, which also restores the poll limit
+    assert (code >> 8) in (2, 3), hex(code)
+    assert bool((bad == -7777.0).all())
+    assert torch.equal(run(), want) and status(1) == 0
+
+
 @pytest.mark.parametrize("dst", ["float8_e4m3fn", "float8_e5m2", "float4_e2m1"])
 @pytest.mark.parametrize("xdt", ["bfloat16", "float16"])
 def test_dynamic_mx_quant_streaming_kernel_matches_oracle(aclnn, dst, xdt):
