@@ -172,12 +172,16 @@ PAIR_CASES = [
 ]
 
 
+@pytest.mark.parametrize("tile_n", [None, "256"])
 @pytest.mark.parametrize("case", PAIR_CASES, ids=[str(c) for c in PAIR_CASES])
-def test_int8_dequant_cta_pairs_bit_exact(aclnn, case, monkeypatch):
-    """The cta_group::2 kernel (two CTAs of a cluster share a 256 x 256 tile), forced for shapes the host tile selection
-    would give to the single-CTA kernel, against the oracle: bit for bit."""
+def test_int8_dequant_cta_pairs_bit_exact(aclnn, case, monkeypatch, tile_n):
+    """The cta_group::2 kernel (two CTAs of a cluster share a tile of 256 rows), forced for shapes the host tile selection would give to the
+    single-CTA kernel, against the oracle: bit for bit. tile_n: columns of a tile; None leaves them to the host, which takes 256 for x2 stored
+    (k,n) and here fewer for (n,k)."""
     m, k, n, t1, t2, pertoken, bias_kind, out_name = case
     monkeypatch.setenv("OPSNN_QMM_PAIR", "1")
+    if tile_n is not None:
+        monkeypatch.setenv("OPSNN_QMM_PAIR_BN", tile_n)
     rng = np.random.default_rng(case_seed(case))
     x1 = rng.integers(-127, 128, (k, m) if t1 else (m, k), dtype=np.int8)
     x2 = rng.integers(-127, 128, (n, k) if t2 else (k, n), dtype=np.int8)
@@ -190,11 +194,12 @@ def test_int8_dequant_cta_pairs_bit_exact(aclnn, case, monkeypatch):
     assert np.array_equal(np.asarray(got).view(np.uint8), np.asarray(want).view(np.uint8))
 
 
-@pytest.mark.parametrize("tile_n", ["224", "192"])
+@pytest.mark.parametrize("tile_n", ["256", "224", "192"])
 @pytest.mark.parametrize("m,k,n,t1,dtype", [(256, 256, 224, False, "int8"), (300, 400, 192, False, "int8"), (640, 528, 452, True, "int8"), (257, 2048, 16, False, "int8"),
                                             (2500, 256, 700, False, "int8"), (1024, 640, 7168, False, "int8"), (390, 400, 640, False, "fp8")])
 def test_narrower_pair_tiles(aclnn, monkeypatch, m, k, n, t1, dtype, tile_n):
-    """224 and 192 columns a pair tile: a CTA's half of B is 112 or 96 rows. n of one tile, a few columns past one, fewer than a half, many waves."""
+    """256, 224 and 192 columns a pair tile: a CTA's half of B is 128, 112 or 96 rows. n of one tile, a few columns past one, fewer than a half,
+    many waves."""
     from gpu_util import check_close
 
     monkeypatch.setenv("OPSNN_QMM_PAIR", "1")
@@ -213,6 +218,22 @@ def test_narrower_pair_tiles(aclnn, monkeypatch, m, k, n, t1, dtype, tile_n):
         assert np.array_equal(np.asarray(got).view(np.uint8), np.asarray(want).view(np.uint8))
     else:
         check_close(got, want, qbmm_oracle.quant_matmul_v5(x1, x2, s1, s2, None, t1, True, 0, "float32"), "bfloat16")
+
+
+@pytest.mark.parametrize("tile_n", ["256", "224", "192"])
+@pytest.mark.parametrize("broadcast", [False, True])
+def test_pair_tile_widths_batched(aclnn, monkeypatch, tile_n, broadcast):
+    """A batch's tiles, the last of each ragged in both directions, with an x2 of its own or one for all."""
+    monkeypatch.setenv("OPSNN_QMM_PAIR", "1")
+    monkeypatch.setenv("OPSNN_QMM_PAIR_BN", tile_n)
+    rng = np.random.default_rng(case_seed((tile_n, broadcast)))
+    x1 = rng.integers(-127, 128, (3, 300, 400), dtype=np.int8)
+    x2 = rng.integers(-127, 128, (() if broadcast else (3,)) + (600, 400), dtype=np.int8)
+    s2 = rng.uniform(1e-3, 1e-2, 600).astype(np.float32)
+    bias = rng.integers(-1000, 1001, 600).astype(np.int32)
+    want = qbmm_oracle.quant_matmul_v5(x1, x2, None, s2, bias, False, True, 0, "bfloat16")
+    got = _run(aclnn, x1, x2, None, s2, bias, False, True, 0, "bfloat16", "qmm_umma_pair_deq")
+    assert np.array_equal(got.view(np.uint16), want.view(np.uint16))
 
 
 def test_cta_pairs_batched_fp8_and_auto_selection(aclnn, monkeypatch):

@@ -145,6 +145,25 @@ PREFILL_CASES = [
 def test_prefill_dequant_then_tensor_core_matmul(aclnn, case):
     """m beyond the decode range: the weight is dequantised with the reference's two roundings into workspace and multiplied
     by the tcgen05 bf16/fp16 kernel, so the output differs from the golden only by fp32 summation order."""
+    _prefill_against_oracle(aclnn, case, ("qmm_umma_deq", "qmm_umma_pair_deq"))
+
+
+@pytest.mark.parametrize("tile_n", ["256", "224", "192"])
+@pytest.mark.parametrize("case", [
+    (300, 1000, 712, 0, True, False, False, True, "x", "float16"),      # a k that ends inside a block, tails in m and n
+    (700, 1024, 456, 128, True, False, True, True, None, "bfloat16"),   # n past two tiles of 224, past one of 256
+    (270, 520, 1000, 0, False, True, False, True, "x", "bfloat16"),     # int8 weight stored (n,k)
+    (257, 768, 200, 64, True, True, False, False, "f32", "bfloat16"),   # one row in the second CTA's half, fewer columns than a tile
+], ids=str)
+@pytest.mark.usefixtures("streaming")
+def test_prefill_on_pair_tiles_of_every_width(aclnn, monkeypatch, case, tile_n):
+    """The matmul on the dequantised weight, 16-bit operands, on CTA pairs (forced for sizes that the host gives to single CTAs)."""
+    monkeypatch.setenv("OPSNN_QMM_PAIR", "1")
+    monkeypatch.setenv("OPSNN_QMM_PAIR_BN", tile_n)
+    _prefill_against_oracle(aclnn, case, ("qmm_umma_pair_deq",))
+
+
+def _prefill_against_oracle(aclnn, case, kernels):
     import ml_dtypes
 
     from gpu_util import np_name, run_wq_fixture
@@ -163,7 +182,7 @@ def test_prefill_dequant_then_tensor_core_matmul(aclnn, case):
              offset=None if offset is None else (offset.T.copy() if (tw and offset.ndim == 2) else offset), bias=bias, out=want)
     meta = dict(transpose_weight=tw, w_is_int4=int4, packed_int32=words, group_size=group)
     got = run_wq_fixture(aclnn, a, meta, kernel=0)
-    assert aclnn.last_kernel_name() in ("qmm_umma_deq", "qmm_umma_pair_deq"), aclnn.last_kernel_name()
+    assert aclnn.last_kernel_name() in kernels, aclnn.last_kernel_name()
     assert aclnn.lib().opsnn_qmm_umma_status(1) == 0
     g, wv = got.astype(np.float64), want.astype(np.float64)
     ulp = 2.0 ** -7 if np_name(want) == "bfloat16" else 2.0 ** -10
