@@ -539,7 +539,8 @@ qmm_mx_umma_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_const
         const uint32_t lane_addr = (uint32_t)(quad * 32) << 16;
         uint32_t grp = 0;
         bool ok = true;
-        for (uint32_t tile = tile0; tile < ntiles && ok; tile += tile_step) {
+        uint32_t tile = tile0;
+        for (; tile < ntiles && ok; tile += tile_step) {
             const uint32_t b = tile / tiles_per_batch, r = tile % tiles_per_batch;
             uint32_t tm, tn;
             tile_of<16>(r, (uint32_t)a.tiles_m, (uint32_t)a.tiles_n, tm, tn);
@@ -612,6 +613,7 @@ qmm_mx_umma_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_const
                 if (lane == 0) ptx::mbar_arrive(&tempty[buf]);
             ++grp;
         }
+        if (!kSplit && !ok) epilogue_leaves(tile, ntiles, tile_step, 2u);
     }
     if constexpr (kSplit) {
         // A CTA that gave up a wait joins both barriers too; what it sends is not used, and then nobody writes.

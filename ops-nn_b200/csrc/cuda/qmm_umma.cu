@@ -110,6 +110,16 @@ __device__ __forceinline__ void report(volatile uint32_t* abort_flag, unsigned i
     }
 }
 
+// The barriers of the four epilogue warps (`per_tile` of them, two behind it in this tile) in the tiles that a warp leaves out which has seen that a wait of
+// this CTA was given up: one that has not, because the flag was set a moment later, still comes to them, and they have no limit. (Out of the loop:
+// a reduction of the flag over the four warps in it cost a call up to 0.1 us, staying in it to the last tile up to 5 % where k is short.)
+__device__ __forceinline__ void epilogue_leaves(uint32_t tile, uint32_t ntiles, uint32_t step, uint32_t per_tile)
+{
+    uint32_t bars = per_tile - 2u;
+    for (tile += step; tile < ntiles; tile += step) bars += per_tile;
+    for (; bars != 0u; --bars) asm volatile("bar.sync 1, 128;" ::: "memory");
+}
+
 // 32 floats as 16 packed pairs of the 16-bit output type.
 __device__ __forceinline__ void pack16(int32_t dtype, const float (&f)[32], uint32_t (&pk)[16])
 {
@@ -485,7 +495,8 @@ qmm_umma_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant
         const uint32_t lane_addr = (uint32_t)(quad * 32) << 16;
         uint32_t grp = 0;
         bool ok = true;
-        for (uint32_t work = blockIdx.x; work < nwork && ok; work += gridDim.x) {
+        uint32_t work = blockIdx.x;
+        for (; work < nwork && ok; work += gridDim.x) {
             const uint32_t tile = work / ks, split = work - tile * ks;
             const uint32_t b = tile / tiles_per_batch, r = tile % tiles_per_batch;
             uint32_t tm, tn;
@@ -509,7 +520,6 @@ qmm_umma_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant
                 asm volatile("bar.sync 1, 128;" ::: "memory");  // the previous tile's readers are done
                 deq_stage_cols<BN>(a, bias, has_ibias, has_fbias, n0, s_scale, s_bias);
                 if (!ptx::mbar_wait_relaxed(&tfull[buf], gpar, abort_flag)) report(abort_flag, (3u << 8) | 1u);
-                // the four epilogue warps leave together: a named barrier is only safe if nobody has left the loop
                 asm volatile("bar.sync 1, 128;" ::: "memory");
                 if (*abort_flag != 0u) {
                     ok = false;
@@ -653,6 +663,7 @@ qmm_umma_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant
                 }
             }
         }
+        if (!kPerBlock && !ok) epilogue_leaves(work, nwork, gridDim.x, ks > 1u ? 4u : 2u);
     }
     // ---- teardown: everyone meets here, also after an aborted wait; then the allocating warp frees TMEM ----
     if (*abort_flag != 0u) __nanosleep(200000);  // lets bulk copies that are still in flight land before the CTA leaves

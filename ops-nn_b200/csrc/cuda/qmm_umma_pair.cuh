@@ -168,7 +168,8 @@ qmm_umma_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_con
         const uint32_t lead_tempty0 = tempty0 & ptx::kPeerBitMask;
         uint32_t grp = 0;
         bool ok = true;
-        for (uint32_t tile = pair; tile < ntiles && ok; tile += npairs) {
+        uint32_t tile = pair;
+        for (; tile < ntiles && ok; tile += npairs) {
             const uint32_t b = tile / tiles_per_batch, r = tile % tiles_per_batch;
             uint32_t tm, tn;
             tile_of<8>(r, (uint32_t)a.tiles_m, (uint32_t)a.tiles_n, tm, tn);
@@ -199,6 +200,7 @@ qmm_umma_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_con
             if (lane == 0) ptx::mbar_arrive_cluster(lead_tempty0 + 8u * buf);
             ++grp;
         }
+        if (!ok) epilogue_leaves(tile, ntiles, npairs, 2u);
     }
     // ---- teardown: both CTAs meet (the even CTA's MMAs read the odd CTA's shared memory until the very end), then free TMEM ----
     if (*abort_flag != 0u) __nanosleep(200000);

@@ -435,3 +435,41 @@ def test_tensor_core_wait_that_runs_out_reaches_the_caller(aclnn, monkeypatch):
     assert L.opsnn_qmm_umma_status(1) == 0
     want = qbmm_oracle.quant_matmul_v5(x1, x2, s1, s2, None, out_dtype="bfloat16")
     assert np.array_equal(out_to_np(out).view(np.uint16), want.view(np.uint16))
+
+
+@pytest.mark.parametrize("ksplit", [None, "2"])
+def test_wait_that_runs_out_in_the_first_of_several_tiles(aclnn, monkeypatch, ksplit):
+    """More tiles than CTAs (with a ksplit: than half of them): the epilogue warps leave in the first, whoever has seen the give-up, and come together at the end."""
+    import torch
+
+    from gpu_util import DEV
+
+    m, k, n = 1024, 2048, 24576
+    gen = torch.Generator(device=DEV).manual_seed(14)
+    x, w = (torch.randint(-127, 128, s, generator=gen, device=DEV, dtype=torch.int8) for s in ((m, k), (n, k)))
+    s1, s2 = (torch.rand(c, generator=gen, device=DEV) * 1e-2 for c in (m, n))
+    monkeypatch.setenv("OPSNN_QMM_PAIR", "0")
+    if ksplit is not None:
+        monkeypatch.setenv("OPSNN_QMM_KSPLIT", ksplit)
+
+    def run():
+        y = torch.full((m, n), -7777.0, dtype=torch.bfloat16, device=DEV)
+        aclnn.quant_matmul_v5(*(aclnn.from_torch(t) for t in (x, w, s1, s2, y)), None, False, True)
+        torch.cuda.synchronize()
+        assert aclnn.last_kernel_name() == ("qmm_umma_deq" if ksplit is None else "qmm_umma_deq_splitk")
+        return y
+
+    want = run()
+    status = aclnn.lib().opsnn_qmm_umma_status
+    assert status(1) == 0
+    monkeypatch.setenv("OPSNN_TEST_UMMA_STALL_KBLOCK", "4")
+    monkeypatch.setenv("OPSNN_TEST_UMMA_POLL_LIMIT", "3000")
+    bad = run()
+    monkeypatch.delenv("OPSNN_TEST_UMMA_STALL_KBLOCK")
+    monkeypatch.delenv("OPSNN_TEST_UMMA_POLL_LIMIT")
+    with pytest.raises(aclnn.AclnnError):
+        run()
+    code = status(1)
+    assert (code >> 8) in (1, 2, 3), hex(code)
+    assert bool((bad == -7777.0).all())
+    assert torch.equal(run(), want) and status(1) == 0
