@@ -841,7 +841,7 @@ static Form choose_form(const OpsnnQmmParams* p, SplitChoice& split)
     if (p->m <= 64 && split_takes(p) && (split_env == nullptr || atoi(split_env) != 0)) return Form::kSplit;
     // Too few tiles for every pair of SMs: the cheapest by the times that were measured (us, k-blocks resident in L2), of
     //   single  waves of 128 x BN tiles over the SMs; a k-block 0.155 / 0.21 / 0.27 / 0.36 at BN 32 / 64 / 128 / 256, per-block 0.43
-    //   pair    waves of 256 x 256 (per-block 256 x 128) tiles over the pairs; a k-block 0.36 (0.29), 2 (1.5) per tile
+    //   pair    waves of 256 x pair_tile (per-block 256 x 128) tiles over the pairs; a k-block 0.25 / 0.32 / 0.36 at 192 / 224 / 256 columns (0.29), 2 (1.5) per tile
     //   split   its own plan's cost
     // (fp8, m717 k7168 n2304: 29.3 / 26.2 / 20.0; m1024 k7168 n4608: 38.1 / 29.9 / 34.7; m40 k8192 n3072: 16.3 / 25.1 / 10.9;
     // per-block m100 k7168 n4096: 25.0 / 19.8 / 14.4, m512 k4096 n4096: 18.6 / 14.6 / 49)
@@ -853,7 +853,8 @@ static Form choose_form(const OpsnnQmmParams* p, SplitChoice& split)
     double best = 5.0 + waves(p->batch * ((p->m + BM - 1) / BM) * ((p->n + bn - 1) / bn), sms) * kb * per;
     Form form = Form::kSingle;
     if (pair_ok && p->m > BM && p->n >= 256) {
-        const double cost = deq ? 4.0 + waves(p->batch * ((p->m + 255) / 256) * ((p->n + 255) / 256), sms / 2) * (kb * 0.36 + 2.0)
+        const int pbn = deq ? pair_tile(p) : 0;
+        const double cost = deq ? 4.0 + waves(p->batch * ((p->m + 255) / 256) * ((p->n + pbn - 1) / pbn), sms / 2) * (kb * (pbn == 192 ? 0.25 : (pbn == 224 ? 0.32 : 0.36)) + 2.0)
                                 : 5.0 + waves(p->batch * ((p->m + 255) / 256) * ((p->n + 127) / 128), sms / 2) * (kb * 0.29 + 1.5);
         if (cost < best) {
             best = cost;

@@ -473,3 +473,25 @@ def test_wait_that_runs_out_in_the_first_of_several_tiles(aclnn, monkeypatch, ks
     assert (code >> 8) in (1, 2, 3), hex(code)
     assert bool((bad == -7777.0).all())
     assert torch.equal(run(), want) and status(1) == 0
+
+
+@pytest.mark.parametrize("m,k,n,kernel", [(150, 12288, 10240, "qmm_umma_pair_deq"),   # one wave of 192 columns, 32 us; as a stream of pieces 76
+                                          (1054, 2368, 2016, "qmm_umma_pair_deq"),    # 11 us; in pieces 14
+                                          (300, 4096, 2048, "qmm_umma_split_deq")])   # 10.5 us; on pairs 13
+def test_pairs_are_priced_with_the_tile_they_get(aclnn, m, k, n, kernel):
+    """Fewer tiles than pairs of SMs: which form a call runs on is decided by its cost, for pairs that of the narrower tiles that they would run."""
+    import torch
+
+    from gpu_util import DEV
+
+    gen = torch.Generator(device=DEV).manual_seed(15)
+    x, w = (torch.randint(-127, 128, s, generator=gen, device=DEV, dtype=torch.int8) for s in ((m, k), (n, k)))
+    s1, s2 = (torch.rand(c, generator=gen, device=DEV) * 1e-2 for c in (m, n))
+    y = torch.empty((m, n), dtype=torch.bfloat16, device=DEV)
+    aclnn.quant_matmul_v5(*(aclnn.from_torch(t) for t in (x, w, s1, s2, y)), None, False, True)
+    torch.cuda.synchronize()
+    assert aclnn.last_kernel_name() == kernel
+    # the sums are whole numbers below 2^31: exact in double
+    cols = torch.randint(0, n, (64,), generator=gen, device=DEV)
+    want = ((x.double() @ w[cols].double().T).float() * s2[cols] * s1[:, None]).to(torch.bfloat16)
+    assert bool(((y[:, cols].float() - want.float()).abs() <= want.float().abs() * 2.0 ** -7).all())
