@@ -513,18 +513,33 @@ constexpr uint32_t kMixPartBytes = 64u * 16u;
 // This CTA's sums (sixteen warps) to their owners. Within a part they lie in the order of the TMEM lanes (`lane`, of 128) and not of the columns, which in
 // (k,n) storage are permuted: in their order eight neighbouring lanes met in two of a shared memory's eight 16-byte banks (int4; in four, 8 bits):
 // us, graph replay, fetched / sent in the columns' order / in the lanes': 128 x 2048 x 12544 int4 15.7 / 16.3 / 15.6, 244 x 2560 x 8544 16.9 / 17.4 / 16.7.
-// Each CTA begins a quarter of its sums further on than the one before it: all beginning with the first rows, they were all sending to the same
-// few owners. fetched / from the first / further on and with four pieces on their way to an owner's registers instead of two: 128 rows, eight pieces,
-// 2048 x 4608 int4 12.8 / 13.0 / 12.2, seven, 339 x 1408 x 1696 11.9 / 12.2 / 11.4, five, 2048 x 7424 12.7 / 13.4 / 12.8 (112 rows 12.1 / 12.7 / 12.2), fourteen,
-// 2048 x 2560 13.0 / 12.2 / 11.5.
-template <bool kMany>
-__device__ __forceinline__ void mix_push(const MixArgs& a, uint32_t acc, uint32_t n_acc, uint32_t step, uint32_t smem, uint32_t live, uint32_t rank, uint32_t lane, uint32_t share)
+// With many rows (kTurn) each CTA begins a quarter of its sums further on than the one before it: all beginning with the first rows, they were all sending
+// to the same few owners. fetched / from the first / further on and with four pieces on their way to an owner's registers instead of two, where they
+// go worked out before the cluster meets: 128 rows, eight pieces, 2048 x 4608 int4 12.8 / 13.0 / 11.9, five, 2048 x 7424 12.7 / 13.4 / 12.6 (112 rows 12.1 / 12.8 /
+// 11.9), seven, 339 x 1408 x 1696 11.9 / 12.1 / 11.2, fourteen, 2048 x 2560 13.0 / 12.2 / 11.4. (16 rows do not need it, and its code cost them 1 %: 4 x 4096 x
+// 14336 int8 (n,k) 15.1 / 15.2, without it, worked out before the cluster meets, 15.0.)
+struct MixPush {
+    uint32_t live, per, inverse, mine, hc, left;
+};
+template <bool kTurn>
+__device__ __forceinline__ MixPush mix_push_plan(const MixArgs& a, uint32_t smem, uint32_t live, uint32_t rank, uint32_t lane, uint32_t share)
 {
-    const uint32_t rows = (uint32_t)a.rows, per = mix_share(live, a.split), inverse = 65535u / per + 1u;  // part * per < 2^16: the quotient is exact
-    const uint32_t mine = smem + rank * per * kMixPartBytes + (lane & 63u) * 16u;
+    MixPush q;
+    q.live = live;
+    q.per = mix_share(live, a.split);
+    q.inverse = 65535u / q.per + 1u;  // part * per < 2^16: the quotient is exact
+    q.mine = smem + rank * q.per * kMixPartBytes + (lane & 63u) * 16u;
+    q.hc = 16u * share + (kTurn ? 64u * (rank & 3u) : 0u);
+    q.left = (2u * (uint32_t)a.rows + 48u - 16u * share) / 64u;
+    return q;
+}
+template <bool kMany, bool kTurn>
+__device__ __forceinline__ void mix_push(const MixArgs& a, uint32_t acc, uint32_t n_acc, uint32_t step, const MixPush& q, uint32_t lane, uint32_t share)
+{
+    const uint32_t rows = (uint32_t)a.rows, live = q.live, per = q.per, inverse = q.inverse, mine = q.mine;
 #pragma unroll 1
-    for (uint32_t left = (2u * rows + 48u - 16u * share) / 64u, hc = 16u * share + 64u * (rank & 3u); left != 0u; --left, hc += 64u) {
-        if (hc >= 2u * rows) hc = 16u * share;  // (round to the first)
+    for (uint32_t left = q.left, hc = q.hc; kTurn ? left != 0u : hc < 2u * rows; --left, hc += 64u) {
+        if (kTurn && hc >= 2u * rows) hc = 16u * share;  // (round to the first)
         const uint32_t h = hc >= rows ? 1u : 0u, r0 = hc - h * rows;
         if (r0 >= live) continue;
         float f[16];
@@ -541,23 +556,39 @@ __device__ __forceinline__ void mix_push(const MixArgs& a, uint32_t acc, uint32_
     }
 }
 
-// This CTA's share of tile t: the pieces added in their order, + bias (s_bias: the tile's columns), stored (512 threads, one column of four rows each).
-template <MixW kW, bool kNK, bool kBf16>
-__device__ __forceinline__ void mix_sum_and_store(const MixArgs& a, uint32_t smem, uint32_t t, uint32_t live, uint32_t rank, uint32_t tid, const float* s_bias)
+// This CTA's share of its tile: the pieces added in their order, + bias (s_bias: the tile's columns), stored (512 threads, one column of four rows each).
+struct MixOwn {
+    uint32_t live, per, first, n0, col;  // first: of this CTA's parts; n0: the tile's first column; col: of a part, this thread's
+    uint16_t* out;                       // the tile's first row
+};
+template <MixW kW, bool kNK>
+__device__ __forceinline__ MixOwn mix_own(const MixArgs& a, uint32_t t, uint32_t live, uint32_t rank, uint32_t tid)
 {
-    const uint32_t tn = t / (uint32_t)a.t_tiles, tt = t - tn * (uint32_t)a.t_tiles, per = mix_share(live, a.split), parts = mix_parts(live);
-    const uint32_t col = (tid & 32u) + (uint32_t)mix_col_of_lane<kW, kNK>((int)(tid & 31u));  // of its part
-    uint16_t* out = reinterpret_cast<uint16_t*>(a.y) + (int64_t)(tt * (uint32_t)a.rows) * a.y_ld;
+    const uint32_t tn = t / (uint32_t)a.t_tiles, tt = t - tn * (uint32_t)a.t_tiles;
+    MixOwn q;
+    q.live = live;
+    q.per = mix_share(live, a.split);
+    q.first = rank * q.per;
+    q.n0 = tn * kMixTileN;
+    q.col = (tid & 32u) + (uint32_t)mix_col_of_lane<kW, kNK>((int)(tid & 31u));
+    q.out = reinterpret_cast<uint16_t*>(a.y) + (int64_t)(tt * (uint32_t)a.rows) * a.y_ld;
+    return q;
+}
+template <bool kBf16, int kAtOnce>
+__device__ __forceinline__ void mix_sum_and_store(const MixArgs& a, uint32_t smem, const MixOwn& q, uint32_t tid, const float* s_bias)
+{
+    const uint32_t live = q.live, per = q.per, parts = mix_parts(live), col = q.col;
+    uint16_t* out = q.out;
 #pragma unroll 1
     for (uint32_t slot = tid / 64u; slot < per; slot += kMixDqWarps * 32 / 64) {
-        const uint32_t part = rank * per + slot, row = part & ~3u, n = tn * kMixTileN + (part & 3u) * 64u + col;
+        const uint32_t part = q.first + slot, row = part & ~3u, n = q.n0 + (part & 3u) * 64u + col;
         if (part >= parts || n >= a.n) continue;
         float v[4] = {0.f, 0.f, 0.f, 0.f};
         uint32_t at = smem + slot * kMixPartBytes + tid % 64u * 16u;
-#pragma unroll 4
+#pragma unroll kAtOnce
         for (uint32_t j = 0; j < a.split; ++j, at += per * kMixPartBytes) {
-            const uint4 q = mix_lds128(at);
-            v[0] += __uint_as_float(q.x); v[1] += __uint_as_float(q.y); v[2] += __uint_as_float(q.z); v[3] += __uint_as_float(q.w);
+            const uint4 p = mix_lds128(at);
+            v[0] += __uint_as_float(p.x); v[1] += __uint_as_float(p.y); v[2] += __uint_as_float(p.z); v[3] += __uint_as_float(p.w);
         }
         uint16_t* y = out + (int64_t)row * a.y_ld + n;
 #pragma unroll
@@ -1067,7 +1098,7 @@ wqbmm_mixed_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
             mix_report(a, abort_flag, (3u << 8) | 3u);
             ok = false;
         }
-        constexpr bool kMany = kSum != MixSum::kChain;
+        constexpr bool kMany = kSum != MixSum::kChain, kTurn = kSum != MixSum::kCopies;
         const uint32_t acc = tmem + tlane + dbuf * d_set;
         // (with chunks: the last one and the sum of those before it)
         const uint32_t n_acc = kSum == MixSum::kCopies ? a.copies : (has_sum ? 2u : 1u), step = kSum == MixSum::kCopies ? d_one : tmem + tlane + d_sum - acc;
@@ -1078,8 +1109,9 @@ wqbmm_mixed_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
             ptx::tc_fence_after();
             __syncwarp();
             ptx::cluster_arrive();
+            const MixPush plan = mix_push_plan<kTurn>(a, smem0, rows_live(), ptx::cluster_ctarank(), (uint32_t)(qd * 32 + lane), (uint32_t)warp >> 2);
             ptx::cluster_wait();
-            mix_push<kMany>(a, acc, n_acc, step, smem0, rows_live(), ptx::cluster_ctarank(), (uint32_t)(qd * 32 + lane), (uint32_t)warp >> 2);
+            mix_push<kMany, kTurn>(a, acc, n_acc, step, plan, (uint32_t)(qd * 32 + lane), (uint32_t)warp >> 2);
         } else if (mix_all_ok<2, kMixDqWarps * 32>(ok)) {
             ptx::tc_fence_after();
             mix_finish<kBf16, 16, kMany>(a, acc, n_acc, step, t_last, last_cnt, col, qd, lane, warp >> 2, threadIdx.x == 0, &s_last[1], abort_flag);
@@ -1155,9 +1187,10 @@ wqbmm_mixed_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
         }
         __syncwarp();
         ptx::cluster_arrive();
+        const MixOwn own = mix_own<kW, kNK>(a, blockIdx.x / a.split, rows_live(), ptx::cluster_ctarank(), threadIdx.x);
         ptx::cluster_wait();
         // (nobody reaches into another CTA's shared memory from here on: they leave when they are done)
-        if (warp < kMixDqWarps && s_bad == 0u) mix_sum_and_store<kW, kNK, kBf16>(a, smem0, blockIdx.x / a.split, rows_live(), ptx::cluster_ctarank(), threadIdx.x, s_bias);
+        if (warp < kMixDqWarps && s_bad == 0u) mix_sum_and_store<kBf16, kSum == MixSum::kCopies ? 2 : 4>(a, smem0, own, threadIdx.x, s_bias);
     }
     // ---- teardown: everyone meets here, also after an aborted wait; then the allocating warp frees TMEM ----
     if (*abort_flag != 0u) __nanosleep(200000);  // lets bulk copies that are still in flight land before the CTA leaves
