@@ -755,7 +755,9 @@ int32_t mx_launch_one(const CUtensorMap& ma, const CUtensorMap& mb, UmmaArgs& a,
 
 // How many pieces a tile's k is cut into (kSplit), 1: none. In us: a stage of the chain 0.18, the two cluster barriers 0.9, a piece to add 0.15, a row to
 // send 0.018 (fitted; graph replay, by pieces, 12 x 9216 x 1408 fp8: one 20.0, two 13.4, four 9.9, eight 9.4, twelve 9.7; 128 x 4096 x 4096 one 12.5, two
-// 13.0, four 11.8; 2 x 300 x 2048 x 1024, which stays whole, one 9.4, three 11.4).
+// 13.0, four 11.8; 2 x 300 x 2048 x 1024, which stays whole, one 9.4, three 11.4). An fp4 stage is twice the k in the same time, so the same costs hold. us,
+// weights from HBM, whole / what this takes: 12 x 9216 x 1408 fp8 20.7 / 9.7, fp4 13.3 / 8.8; 100 x 16384 x 1024 33.6 / 13.8, 20.0 / 12.2; 20 x 14336 x 4096 29.8 / 16.8, 18.0 / 12.1;
+// 8 x 8192 x 9216 35.5 / 23.4, 21.2 / 15.7; 1 x 4096 x 4096 14.1 / 10.2, 9.1 / 8.4; 128 x 8192 x 4096 20.8 / 16.9, 13.9 / 14.0; 200 x 8192 x 1024 20.1 / 13.6, 13.4 / 12.5.
 template <bool kF4>
 int mx_pick_split(const UmmaArgs& a, size_t smem)
 {

@@ -2,8 +2,8 @@
 //
 // Why pairs. With one CTA per tile (128 x 256) every SM pulls 48 KB of operands from L2 per 512 tensor-core cycles; 148 SMs
 // at full rate ask for more than the L2 -> SM path delivers, so the tensor pipe waits for operands. Two CTAs of a cluster
-// that share one 256 x 256 tile each load their own 128 rows of A and only HALF of B (128 columns); the MMA, issued by the
-// even CTA, reads A and B from both CTAs' shared memory and writes rows 0-127 / 128-255 of the accumulator to the even / odd
+// that share one tile of 256 rows x 256 columns (or 224, 192: pair_tile) each load their own 128 rows of A and only HALF of B (128 columns); the MMA,
+// issued by the even CTA, reads A and B from both CTAs' shared memory and writes rows 0-127 / 128-255 of the accumulator to the even / odd
 // CTA's TMEM. Per SM that is 32 KB per 512 cycles: a third less traffic for the same arithmetic.
 //
 // Choreography (each CTA waits only on its own barriers):
@@ -162,7 +162,7 @@ qmm_umma_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_con
             }
         }
     } else {
-        // ======================= epilogue warps (both CTAs): own 128 rows x 256 columns =======================
+        // ======================= epilogue warps (both CTAs): own 128 rows x BN columns =======================
         const int quad = warp & 3;
         const uint32_t lane_addr = (uint32_t)(quad * 32) << 16;
         const uint32_t lead_tempty0 = tempty0 & ptx::kPeerBitMask;
@@ -215,9 +215,12 @@ qmm_umma_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_con
 
 // Columns of the pair kernel's tiles. All pairs run tiles of one size in waves, and a last wave that is nearly empty takes as long as a full one: 1024 rows
 // x 7168 columns are 1.5 waves of 256 columns and 1.7 of 224. A k-block is 2 BN clocks of tensor work and some 24 more; narrower tiles load A more often
-// per column, which costs 4 and 9 % under the power limit. us, 256 / 224 / 192 columns, back to back: 1024 x 4096 x 7168 int8 30.5 / 28.4 / 30.7,
-// 1300 x 8192 x 7168 16-bit after its pre-pass 190 / 182 / 194, 2048 x 8192 x 28672 876 / 869 / 888, 4096 x 4096 x 4096 fp8 61.2 / 62.8 / 62.3,
-// 2048 x 7168 x 4608 fp8 58.1 / 63.8 / 61.1. x2 stored along n keeps 256 columns, whole 128-byte rows a CTA. OPSNN_QMM_PAIR_BN fixes it.
+// per column, for which 4 and 9 % are counted. us, 256 / 224 / 192 columns, graph replay, weights from HBM (* the one that is taken): int8 and fp8
+// 1024 x 4096 x 7168 27.2 / 25.2* / 27.2, 640 x 2048 x 10240 21.1 / 18.8* / 22.3, 1300 x 256 x 16384 31.8 / 28.1* / 29.3, 2048 x 7168 x 4608 49.5* / 56.0 / 53.0, 482 x 2816 x 8928
+// 14.7* / 18.7 / 17.2, 4096 x 4096 x 4096 53.0 / 54.3 / 53.4*, 1036 x 2368 x 11376 33.4 / 33.6* / 33.5; 16-bit with its pre-pass 1559 x 7936 x 2688 95 / 84 / 75*, 1941 x 5888 x 2752
+// 75 / 66 / 60*, 1300 x 2048 x 7168 46.2 / 42.0* / 45.0, 2048 x 4096 x 4096 58 / 69 / 63*. Where a call lasts long enough for the power limit the width hardly shows:
+// 2048 x 8192 x 28672, which takes 224, in turn over seconds 873 with 256 and 861 - 867 with 224 (runs of one width differ by 0.3 - 1.2 %; on another GPU 891 and 891).
+// x2 stored along n keeps 256 columns, whole 128-byte rows a CTA. OPSNN_QMM_PAIR_BN fixes it.
 int pair_tile(const OpsnnQmmParams* p)
 {
     if (!p->trans_b) return 256;

@@ -320,7 +320,7 @@ qmm_umma_split_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_co
     // The out-of-line part of the waits, shared by all kernels of the file, is compiled to a convention that all of them can live with. Where the chain of
     // waits is most of a call it is worth a copy for the instance alone: us, graph replay, weights from HBM, shared / own, 128 x 4096 x 4096 int8 10.6 / 9.9,
     // 717 x 7168 x 2304 fp8 18.7 / 17.2, 14 x 8640 x 6048 fp8 17.9 / 16.0, 300 x 4096 x 2048 int8 11.6 / 10.8; per-block on weights stored (n,k)
-    // 5 x 8320 x 14080 27.6 / 24.9, 14 x 4480 x 15872 17.3 / 16.2, 24 x 7168 x 18432 25.4 / 25.3. Per-block on (k,n) it is not: 16 x 10368 x 3584 15.3 / 14.8, but
+    // 5 x 8320 x 14080 27.6 / 24.9 (25.8 since the forms are instances), 14 x 4480 x 15872 17.3 / 16.2, 24 x 7168 x 18432 25.4 / 25.3. Per-block on (k,n) it is not: 16 x 10368 x 3584 15.3 / 14.8, but
     // 5 x 8320 x 14080 28.3 / 28.8, 14 x 4480 x 15872 18.9 / 19.1, 100 x 7168 x 4096 15.9 / 16.2. That is why the order is a template argument there.
     // (The fused weight-only, pair and block-scaled kernels do not change.)
     constexpr int kMe = !kPerBlock ? 100 * kForm + (int)kKind * 2 + (int)kHalves : (kOrder == kOrderNK ? 1000 * kForm + kAcc + (int)kHalves : 0);

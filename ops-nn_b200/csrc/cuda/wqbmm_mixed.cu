@@ -29,7 +29,7 @@
 // Therefore buffers change hands by the stage and not by 64 rows of k, a warp arrives under a predicate instead of a branch, and scales that allow
 // it save the magic number (MixFast). Before / after, the same calls, weights from HBM (in brackets out of L2): 39.4 / 37.5, 27.9 / 24.5
 // (25.9 / 21.7), 17.7 / 15.7 (15.5 / 13.1), 9.5 / 9.2 (9.1 / 8.8).
-// Clocks, 16 x 8192 x 28672: 65000 a CTA, 3900 until the first stage is there, 6000 from the last sums to the end; the 16-bit pipe is busy for 37400. A
+// Clocks, 16 x 8192 x 28672: 65000 a CTA, 3900 until the first stage is there, 6000 from the last sums to the end; the busiest unit, the 16-bit pipe, works for 37400. A
 // warp waits for A buffers 7000, but others compute meanwhile: a third stage of buffers in place of the second accumulator set took 38.6 us, with
 // two 38.3 by the same code, 37.6 by this.
 // Every wait is bounded; a wait that gives up raises the CTA's abort flag, records a code and the CTA tears down (TMEM freed).
